@@ -1,0 +1,360 @@
+// Base conversions fused between the two halves of the 2^16 transforms (sm_100a).
+//
+// A base conversion (the lift of a key-switch digit, ModDown, the division by P * q_l, a rescale) works coefficient by
+// coefficient across limbs, and the column pass of a transform works column by column inside a limb.  So one CTA that owns
+// a strip of columns can finish the inverse transforms of the source limbs (their column pass), convert, and begin the
+// forward transforms of the target limbs, without the coefficients ever leaving shared memory:
+//
+//     inverse row pass (ntt16v2_inv_rows)  ->  conv_cols / lift_cols  ->  forward row pass (ntt16v2_fwd_rows*)
+//
+// replaces inverse columns, conversion and forward columns as three kernels: for a conversion of S limbs to T, S reads + T
+// writes instead of 3 S + S + 3 T limb transfers, and one launch instead of three.  Measured at S = 4, T = 6 (the division by
+// P * q_l at level 6) and 336 polynomials: see the launcher.
+//
+// A CTA is two groups of COLS * 16 threads.  Sources are dealt to the groups, then (one CTA barrier later) targets; inside a
+// group a radix-16 round exchanges through shared memory behind a named barrier of that group only, so one group's loads,
+// barriers and exchanges overlap the other's arithmetic.  Source residues stay in shared memory as two 30-bit pieces per
+// word: products with 26-bit (or 30-bit) pieces of the constants are single 32 x 32 multiply-adds into 64-bit sums, on the
+// integer pipe, which the FP64 butterflies around them leave idle.
+#pragma once
+#include "modarith.cuh"
+#include "ntt16.cuh"
+
+namespace hb {
+
+// One conversion: sources [ns] -> targets [nt].  scale: N^-1 * (D / d_s)^-1 mod d_s, as the last multiplication of the inverse transform.
+struct ConvPlan {
+    int ns, nt;
+    int src_limb, dst_limb;             // first limb of the sources / targets inside one instance of the arrays
+    unsigned char src_prime[8], dst_prime[kMaxPrimes];
+    u64 scale_w[8], scale_c[8];         // (ds_twiddle_word, w / q as a double) below 2^44, (w, Shoup companion) otherwise
+    uint4 c[kMaxPrimes][8];             // [target][source]: C = D / d_s mod target.  Target below 2^44: the 26-bit pieces of C
+                                        // and of C * 2^30; otherwise the 30-bit pieces of C, 0, 0
+};
+
+template <int COLS> struct StripIndex { // [256 rows][COLS] words in shared memory, COLS pad words per 16 rows: both access patterns are conflict-free
+    static constexpr int kWords = 256 * COLS + 16 * COLS;
+    static __device__ __forceinline__ int a(int e, int sub, int lane) { return e * 17 * COLS + sub * COLS + lane; }  // row e * 16 + sub
+    static __device__ __forceinline__ int b(int e, int sub, int lane) { return sub * 17 * COLS + e * COLS + lane; }  // row sub * 16 + e
+};
+template <int THREADS> __device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(THREADS) : "memory"); }
+
+// Inverse column pass of one limb strip into the registers of a group: on return v[e] is row e * 16 + sub, times the scale, canonical.
+template <int COLS>
+__device__ __forceinline__ void strip_inverse(u64 (&v)[16], const u64 *__restrict__ p /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, u64 sw, u64 sc,
+                                              int g, int sub, int lane) {
+    using I = StripIndex<COLS>;
+    if (m.small) {
+        const DsConst c = ds_const(m);
+        double *smd = reinterpret_cast<double *>(sm);
+        double d[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) d[e] = reinterpret_cast<const double *>(p)[(sub * 16 + e) * 256];
+        inv16_ds<1>(d, tab + Ntt16Layout::colsB(sub, 0), c);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) smd[I::b(e, sub, lane)] = d[e];
+        group_sync<COLS * 16>(g);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) d[e] = smd[I::a(e, sub, lane)];
+        inv16_ds<1>(d, tab + Ntt16Layout::colsA(0), c);
+        const double qinv_up = c.qinv * (1.0 + 0x1p-50), sf = __longlong_as_double((long long)sc);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = ds_store(ds_mul(d[e], sw, sf, c), c, c.qd, qinv_up);
+    } else {
+        const IntConst c = int_const(m);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = p[(sub * 16 + e) * 256];
+        inv16_int<1>(v, tab + Ntt16Layout::colsB(sub, 0), c);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) sm[I::b(e, sub, lane)] = v[e];
+        group_sync<COLS * 16>(g);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = sm[I::a(e, sub, lane)];
+        inv16_int<1>(v, tab + Ntt16Layout::colsA(0), c);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = canon_q(mul_shoup4(v[e], sw, sc, c.nq), c.q, c.sh);
+    }
+}
+// Forward column pass of one limb strip: v[e] holds row e * 16 + sub (double bits below 2^44, |v| < 2q; otherwise words below 4q).
+template <int COLS>
+__device__ __forceinline__ void strip_forward(u64 (&v)[16], u64 *__restrict__ o /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, int g, int sub, int lane) {
+    using I = StripIndex<COLS>;
+    if (m.small) {
+        const DsConst c = ds_const(m);
+        double *smd = reinterpret_cast<double *>(sm);
+        double d[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) d[e] = __longlong_as_double((long long)v[e]);
+        fwd16_ds<1>(d, tab + Ntt16Layout::colsA(0), c);
+        group_sync<COLS * 16>(g); // the strip of the previous target has been read
+#pragma unroll
+        for (int e = 0; e < 16; ++e) smd[I::a(e, sub, lane)] = d[e];
+        group_sync<COLS * 16>(g);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) d[e] = smd[I::b(e, sub, lane)];
+        fwd16_ds<1>(d, tab + Ntt16Layout::colsB(sub, 0), c);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) reinterpret_cast<double *>(o)[(sub * 16 + e) * 256] = d[e];
+    } else {
+        const IntConst c = int_const(m);
+        fwd16_int<1, kFoldColsA>(v, tab + Ntt16Layout::colsA(0), c);
+        group_sync<COLS * 16>(g);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) sm[I::a(e, sub, lane)] = v[e];
+        group_sync<COLS * 16>(g);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = sm[I::b(e, sub, lane)];
+        fwd16_int<1, kFoldColsB>(v, tab + Ntt16Layout::colsB(sub, 0), c);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) o[(sub * 16 + e) * 256] = v[e];
+    }
+}
+
+// a0 + a1 * 2^26 modulo a prime below 2^44 (a1 < 2^52, a0 < 2^61) as an integer-valued double within 2q of zero.  The quotient
+// comes from the FP64 pipe (both sums enter through the 2^52 exponent without a conversion, the offsets are folded into `base`,
+// off by at most 1.6), the remainder is exact in the low 64 bits.
+struct SmallFinish { double k1, k0, base; u32 n0, n1, hi0; };
+__device__ __forceinline__ SmallFinish small_finish(const PrimeConst &m) {
+    SmallFinish f;
+    f.k1 = 0x1p26 * m.q_inv_f; f.k0 = 0x1p32 * m.q_inv_f;
+    f.base = kMagic - kTwo52 * (f.k1 + f.k0);
+    const u64 nq = 0ull - m.q;
+    f.n0 = (u32)nq; f.n1 = (u32)(nq >> 32);
+    f.hi0 = 0x43380000u - 0x43380000u * f.n0; // exponent word of the result, minus what the exponent word of the quotient contributes
+    return f;
+}
+__device__ __forceinline__ double finish_small(u64 a0, u64 a1, const SmallFinish &f) {
+    const double d1 = __hiloint2double((int)((u32)(a1 >> 32) | 0x43300000u), (int)(u32)a1), d0 = __hiloint2double(0x43300000, (int)(u32)(a0 >> 32));
+    const double qh = __fma_rn(d1, f.k1, __fma_rn(d0, f.k0, f.base));
+    const u64 l = a0 + (a1 << 26);
+    const u32 q0 = (u32)__double2loint(qh), q1 = (u32)__double2hiint(qh);
+    const u64 r = mad_wide(q0, f.n0, l);
+    const u32 hi = q1 * f.n0 + (q0 * f.n1 + (u32)(r >> 32)) + f.hi0;
+    return __hiloint2double((int)hi, (int)(u32)r) - kMagic;
+}
+// a0 + a1 * 2^30 + a2 * 2^60 modulo a prime of 45 to 60 bits (a0, a1 + 2^34, a2 + 2^34 < 2^64): below 4q
+__device__ __forceinline__ u64 finish_wide(u64 a0, u64 a1, u64 a2, const PrimeConst &m) {
+    const u32 m30 = 0x3FFFFFFFu;
+    if (m.d60) { // 2^60 = d60 modulo q
+        const u64 u = a1 + (a0 >> 30), v = a2 + (u >> 30);
+        u64 r = mad_wide((u32)u & m30, 1u << 30, (u64)((u32)a0 & m30)); // < 2^60
+        r = mad_wide((u32)v, m.d60, r);                                 // + 2^58
+        const u64 t = (u64)(u32)(v >> 32) * m.d60;                      // < 2^58, weight 2^32
+        r = mad_wide((u32)(t >> 28), m.d60, r);                         // + 2^56
+        return r + ((u64)((u32)t & 0x0FFFFFFFu) << 32);                 // + 2^60
+    }
+    u64 lo = a0, hi = 0, x = a1 << 30;
+    lo += x; hi += (a1 >> 34) + (lo < x);
+    x = a2 << 60;
+    lo += x; hi += (a2 >> 4) + (lo < x);
+    return barrett128(hi, lo, m);
+}
+// the converted values of one target for this thread's sixteen coefficients.  NS > 0: compile-time source count, constants in registers.
+template <int NS, int COLS>
+__device__ __forceinline__ void convert_target(u64 (&v)[16], const u64 *ysm, const uint4 *__restrict__ cst, int ns_rt, const PrimeConst &m, int sub, int lane) {
+    using I = StripIndex<COLS>;
+    const int ns = NS > 0 ? NS : ns_rt;
+    uint4 k[NS > 0 ? NS : 1];
+    if (NS > 0) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) k[s] = __ldg(cst + s);
+    }
+    if (m.small) {
+        const SmallFinish f = small_finish(m);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            u64 a0 = 0, a1 = 0;
+#pragma unroll
+            for (int s = 0; s < ns; ++s) {
+                const uint4 c = NS > 0 ? k[s] : __ldg(cst + s);
+                const u64 y = ysm[s * I::kWords + I::a(e, sub, lane)];
+                a0 = mad_wide((u32)y, c.x, a0); a1 = mad_wide((u32)y, c.y, a1);
+                a0 = mad_wide((u32)(y >> 32), c.z, a0); a1 = mad_wide((u32)(y >> 32), c.w, a1);
+            }
+            v[e] = (u64)__double_as_longlong(finish_small(a0, a1, f));
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            u64 a0 = 0, a1 = 0, a2 = 0;
+#pragma unroll
+            for (int s = 0; s < ns; ++s) {
+                const uint4 c = NS > 0 ? k[s] : __ldg(cst + s);
+                const u64 y = ysm[s * I::kWords + I::a(e, sub, lane)];
+                a0 = mad_wide((u32)y, c.x, a0); a1 = mad_wide((u32)y, c.y, a1);
+                a1 = mad_wide((u32)(y >> 32), c.x, a1); a2 = mad_wide((u32)(y >> 32), c.y, a2);
+            }
+            v[e] = finish_wide(a0, a1, a2, m);
+        }
+    }
+}
+
+// src: half-inverse limbs (after the inverse row pass), instance b at src + b * src_outer; dst: half-forward limbs.
+// grid = (256 / COLS, plans * split, instances): a CTA takes every split-th target of its plan (small batches: more CTAs,
+// each repeating the source passes).  Dynamic shared memory: (largest ns + 2) strips.
+template <int COLS>
+__global__ void __launch_bounds__(COLS * 32, 512 / (COLS * 32)) conv_cols(const u64 *__restrict__ src, size_t src_outer, u64 *__restrict__ dst, size_t dst_outer, const ConvPlan *__restrict__ plans, int split,
+                                                                         const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
+    extern __shared__ __align__(16) u64 strips[];
+    using I = StripIndex<COLS>;
+    const ConvPlan *pl = plans + blockIdx.y / split;
+    const int part = blockIdx.y % split, ns = pl->ns, nt = pl->nt;
+    const int g = threadIdx.x / (COLS * 16), r = threadIdx.x % (COLS * 16), lane = r % COLS, sub = r / COLS;
+    const int col = blockIdx.x * COLS + lane;
+    const u64 *sp = src + (size_t)blockIdx.z * src_outer + (size_t)pl->src_limb * kN16 + col;
+    u64 *dp = dst + (size_t)blockIdx.z * dst_outer + (size_t)pl->dst_limb * kN16 + col;
+    u64 v[16];
+    for (int s = g; s < ns; s += 2) {
+        const int pi = pl->src_prime[s];
+        u64 *sm = strips + s * I::kWords;
+        strip_inverse<COLS>(v, sp + (size_t)s * kN16, sm, pc[pi], tb.inv + (size_t)pi * Ntt16Layout::kEntries, pl->scale_w[s], pl->scale_c[s], g, sub, lane);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) sm[I::a(e, sub, lane)] = ((v[e] >> 30) << 32) | ((u32)v[e] & 0x3FFFFFFFu); // the words this thread read itself
+    }
+    __syncthreads();
+    u64 *ex = strips + (ns + g) * I::kWords;
+    for (int t = part * 2 + g; t < nt; t += 2 * split) {
+        const int pi = pl->dst_prime[t];
+        const PrimeConst m = pc[pi];
+        const uint4 *cst = pl->c[t];
+        switch (ns) {
+        case 1: convert_target<1, COLS>(v, strips, cst, ns, m, sub, lane); break;
+        case 2: convert_target<2, COLS>(v, strips, cst, ns, m, sub, lane); break;
+        case 3: convert_target<3, COLS>(v, strips, cst, ns, m, sub, lane); break;
+        case 4: convert_target<4, COLS>(v, strips, cst, ns, m, sub, lane); break;
+        default: convert_target<0, COLS>(v, strips, cst, ns, m, sub, lane); break;
+        }
+        strip_forward<COLS>(v, dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)pi * Ntt16Layout::kEntries, g, sub, lane);
+    }
+}
+
+// Rescale: one source limb (prime index `level`), lifted centred to the limbs 0 .. level - 1.
+// grid = (256 / COLS, split, instances); dynamic shared memory: three strips.
+template <int COLS>
+__global__ void __launch_bounds__(COLS * 32, 512 / (COLS * 32)) lift_cols(const u64 *__restrict__ src, size_t src_outer, u64 *__restrict__ dst, size_t dst_outer, int level, int split,
+                                                                         const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
+    extern __shared__ __align__(16) u64 strips[];
+    using I = StripIndex<COLS>;
+    const int g = threadIdx.x / (COLS * 16), r = threadIdx.x % (COLS * 16), lane = r % COLS, sub = r / COLS;
+    const int col = blockIdx.x * COLS + lane;
+    const u64 ql = pc[level].q;
+    const bool src_small = pc[level].small;
+    u64 v[16];
+    if (g == 0) {
+        const PrimeConst m = pc[level];
+        const u64 sw = m.small ? ds_twiddle_word(m.n_inv) : m.n_inv, sc = m.small ? (u64)__double_as_longlong(m.n_inv_f) : m.n_inv_sh;
+        strip_inverse<COLS>(v, src + (size_t)blockIdx.z * src_outer + col, strips, m, tb.inv + (size_t)level * Ntt16Layout::kEntries, sw, sc, g, sub, lane);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) strips[I::a(e, sub, lane)] = v[e] > (ql >> 1) ? v[e] - ql : v[e]; // signed
+    }
+    __syncthreads();
+    u64 *dp = dst + (size_t)blockIdx.z * dst_outer + col, *ex = strips + (1 + g) * I::kWords;
+    for (int t = blockIdx.y * 2 + g; t < level; t += 2 * split) {
+        const PrimeConst m = pc[t];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            const i64 y = (i64)strips[I::a(e, sub, lane)];
+            if (m.small && src_small && (ql >> 1) < 2 * m.q) v[e] = (u64)__double_as_longlong(__longlong_as_double(y + 0x4338000000000000ll) - kMagic); // within 2q of zero
+            else if (m.small) v[e] = (u64)__double_as_longlong(u52_to_double(reduce_i64(y, m)));
+            else if ((ql >> 1) < m.q) v[e] = y < 0 ? (u64)(y + (i64)m.q) : (u64)y;
+            else v[e] = reduce_i64(y, m);
+        }
+        strip_forward<COLS>(v, dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)t * Ntt16Layout::kEntries, g, sub, lane);
+    }
+}
+
+// ---- forward row pass with the last step of a division ----
+//   out[b][p][l] = (x[b][p][l] - t[b][p][l]) * inv_l  (+ add_p[b][l] o perm_g)
+// t arrives half-forward (conv_cols / lift_cols).  grid = (16, n, instances), instance bp = b * np + p.  The operands of the last
+// step are read after the barrier of the final exchange, when the registers of the transform are free.
+struct RowsFin {
+    const u64 *x; size_t x_outer;            // instance stride of x; limb l at l * N
+    const u64 *add[3]; size_t add_outer;     // per polynomial, ciphertext stride; null: nothing to add
+    u32 g;                                   // Galois element of the addends, 0: none
+    u64 *out; size_t out_outer;              // ciphertext stride; polynomial p at p * n * N
+    int np;
+};
+struct InvScale { u64 w[kMaxPrimes], c[kMaxPrimes]; }; // per limb: (ds_twiddle_word, w / q as a double) below 2^44, (w, Shoup companion) otherwise
+template <int MINB>
+__global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *__restrict__ t, size_t t_outer, const __grid_constant__ RowsFin f, const __grid_constant__ InvScale sc, const PrimeConst *__restrict__ pc,
+                                                            Ntt16Tables tb) {
+    __shared__ u64 sm[16 * kRowStride];
+    const int l = blockIdx.y, bp = blockIdx.z, b = bp / f.np, p = bp % f.np, n = gridDim.y;
+    const PrimeConst m = pc[l];
+    const ulonglong2 *tab = tb.fwd + (size_t)l * Ntt16Layout::kEntries;
+    const int tid = threadIdx.x, clo = tid & 15, rl = tid >> 4;
+    const int row = blockIdx.x * 16 + rl;
+    const size_t pos = (size_t)row * 256 + clo, limb = (size_t)l * kN16;
+    const u64 *tp = t + (size_t)bp * t_outer + limb + pos;
+    const u64 *xp = f.x + (size_t)bp * f.x_outer + limb + pos;
+    const u64 *ap = f.add[p] ? f.add[p] + (size_t)b * f.add_outer + limb : nullptr;
+    u64 *o = f.out + (size_t)b * f.out_outer + ((size_t)p * n + l) * kN16 + pos;
+    u64 *smr = sm + rl * kRowStride;
+    if (m.small) {
+        const DsConst c = ds_const(m);
+        const double *td = reinterpret_cast<const double *>(tp);
+        double *smd = reinterpret_cast<double *>(smr);
+        double v[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = td[e * 16];
+        fwd16_ds<1>(v, tab + Ntt16Layout::rowsA(row, 0), c);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) smd[e * 17 + clo] = v[e];
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = smd[clo * 17 + e];
+        fwd16_ds8<16>(v, tb.fwdB8 + (size_t)l * kRowsB8 + (row * 15) * 16 + clo, c);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) smd[clo * 17 + e] = v[e]; // the words this thread read itself
+        u64 x[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) x[e] = xp[e * 16];
+        __syncthreads();
+        const double sf = __longlong_as_double((long long)sc.c[l]), qinv_up = c.qinv * (1.0 + 0x1p-50);
+        const u64 sw = sc.w[l];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            double r = ds_mul(ds_load(x[e]) - smd[e * 17 + clo], sw, sf, c); // within 0.52 q of zero
+            if (ap) r += ds_load(ap[f.g ? ntt_perm((u32)(pos + e * 16), f.g, 16) : (u32)(pos + e * 16)]);
+            o[e * 16] = ds_store(r, c, c.qd, qinv_up);
+        }
+    } else {
+        const IntConst c = int_const(m);
+        u64 v[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = tp[e * 16];
+        fwd16_int<1, kFoldRowsA>(v, tab + Ntt16Layout::rowsA(row, 0), c);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = v[e];
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
+        fwd16_int<16, kFoldRowsB>(v, tab + Ntt16Layout::rowsB(row, 0, clo), c); // below 5q
+#pragma unroll
+        for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = v[e];
+        u64 x[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) x[e] = xp[e * 16];
+        __syncthreads();
+        const u64 sw = sc.w[l], ss = sc.c[l];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            u64 r = mul_shoup4(x[e] + c.q8 - smr[e * 17 + clo], sw, ss, c.nq); // below 4q
+            if (ap) r += ap[f.g ? ntt_perm((u32)(pos + e * 16), f.g, 16) : (u32)(pos + e * 16)];
+            o[e * 16] = canon_q(r, c.q, c.sh);
+        }
+    }
+}
+
+// single passes, for the fused sequences
+inline void launch_inv_rows16(cudaStream_t st, const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
+    ntt16v2_inv_rows<4><<<dim3(16, count), 256, 0, st>>>(src, LimbAddr16{src_outer}, dst, LimbAddr16{dst_outer}, map, pc, tb);
+}
+inline void launch_fwd_rows16(cudaStream_t st, u64 *d, size_t outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
+    ntt16v2_fwd_rows<4><<<dim3(16, count), 256, 0, st>>>(d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb);
+}
+inline void launch_fwd_rows_fin16(cudaStream_t st, const u64 *t, size_t t_outer, int n, int instances, const RowsFin &f, const InvScale &sc, const PrimeConst *pc, const Ntt16Tables &tb) {
+    ntt16v2_fwd_rows_fin<4><<<dim3(16, n, instances), 256, 0, st>>>(t, t_outer, f, sc, pc, tb);
+}
+
+} // namespace hb

@@ -6,6 +6,7 @@
 #include "host_ctx.hpp"
 #include "kernels.cuh"
 #include "ntt.cuh"
+#include "convcols.cuh"
 
 #include <cstdio>
 #include <dlfcn.h>
@@ -118,7 +119,10 @@ struct hb_ctx {
     std::map<u64, Evk> gal_keys;
     std::map<int, KsPlan *> plans; // device copies
     std::map<int, DivPlan *> div_plans;
-    std::map<int, std::vector<u64>> div_hat_inv; // host copy of DivPlan::hat_inv per level (folded into the inverse transform)
+    std::map<int, ConvPlan *> conv_plans; // 2^16 rings, per level: one per key-switch digit, then ModDown, then the division by P * q_level (level >= 1)
+    InvScale p_inv_scale{};               // 2^16 rings: P^-1 mod q_l
+    std::map<int, InvScale> div_scale;    // (P * q_level)^-1 mod q_l per level
+    bool smem_opt_in_conv = false;
     u64 *pinned = nullptr; size_t pinned_bytes = 0; // host staging buffer of hb_decrypt_many
     ChaChaKey ckey{};
     std::map<std::pair<int, long long>, u32 *> gal_tables; // (copies, row_step) -> Galois elements of hb_matmul_acc, on the device
@@ -184,26 +188,16 @@ struct TmpBytes { // the same for a byte count (staging buffers of int64 coeffic
     TmpBytes(const TmpBytes &) = delete;
 };
 
-void ntt(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int count, const LimbMap &m, bool inv, const Ntt16Scale *scale = nullptr) {
+void ntt(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int count, const LimbMap &m, bool inv) {
     c->launches += (count == 0) ? 0 : (c->logn == 16 ? 2 : 1);
-    CK(launch_ntt(c->st, src, so, dst, dof, count, m, c->pc, c->tb, c->logn, inv, scale));
+    CK(launch_ntt(c->st, src, so, dst, dof, count, m, c->pc, c->tb, c->logn, inv));
 }
-// scale table of an inverse transform that also multiplies position k by f[k] (2^16 rings only): s_k = N^-1 * f[k] mod q
-Ntt16Scale ntt_scale(hb_ctx *c, const LimbMap &m, const u64 *f) {
-    Ntt16Scale sc{};
-    if (m.n > 8) fail(HB_E_LIMIT, "scaled inverse transform: at most 8 limb positions");
-    sc.on = 1;
-    for (int k = 0; k < m.n; ++k) {
-        const u64 q = c->h->q[m.prime[k]];
-        const u64 s = hbhost::mulmod(hbhost::invmod((u64)c->N % q, q), f[k] % q, q);
-        if (q >> 44) { sc.w[k] = s; sc.comp[k] = hbhost::shoup(s, q); }
-        else {
-            sc.w[k] = ds_twiddle_word(s);
-            const double sf = (double)s / (double)q;
-            std::memcpy(&sc.comp[k], &sf, 8);
-        }
-    }
-    return sc;
+// a constant v mod q in the form the 2^16 kernels multiply by: the value as a double and v / q, or the value and its Shoup companion
+void scale_words(u64 v, u64 q, u64 &w, u64 &comp) {
+    if (q >> 44) { w = v; comp = hbhost::shoup(v, q); return; }
+    w = ds_twiddle_word(v);
+    const double f = (double)v / (double)q;
+    std::memcpy(&comp, &f, 8);
 }
 void ntt_inplace(hb_ctx *c, u64 *d, int count, const LimbMap &m, bool inv) { ntt(c, d, (size_t)m.n * c->N, d, (size_t)m.n * c->N, count, m, inv); }
 
@@ -273,6 +267,110 @@ const KsPlan *get_plan(hb_ctx *c, int level) {
     c->plans[level] = d;
     return d;
 }
+// ---- conversions between the column passes (2^16 rings) ----
+void fill_conv(const HostCtx &h, ConvPlan &p, const std::vector<int> &src, const std::vector<int> &dst, int src_limb, int dst_limb) {
+    p.ns = (int)src.size(); p.nt = (int)dst.size(); p.src_limb = src_limb; p.dst_limb = dst_limb;
+    auto hat = [&](size_t s, u64 q) { u64 v = 1; for (size_t t = 0; t < src.size(); ++t) if (t != s) v = hbhost::mulmod(v, h.q[src[t]] % q, q); return v; };
+    for (size_t s = 0; s < src.size(); ++s) {
+        const u64 q = h.q[src[s]];
+        p.src_prime[s] = (unsigned char)src[s];
+        scale_words(hbhost::mulmod(hbhost::invmod((u64)h.N % q, q), hbhost::invmod(hat(s, q), q), q), q, p.scale_w[s], p.scale_c[s]);
+    }
+    for (size_t t = 0; t < dst.size(); ++t) {
+        const u64 q = h.q[dst[t]];
+        p.dst_prime[t] = (unsigned char)dst[t];
+        for (size_t s = 0; s < src.size(); ++s) {
+            const u64 v = hat(s, q), v30 = hbhost::mulmod(v, ((u64)1 << 30) % q, q), m26 = ((u64)1 << 26) - 1, m30 = ((u64)1 << 30) - 1;
+            p.c[t][s] = (q >> 44) ? make_uint4((u32)(v & m30), (u32)(v >> 30), 0, 0) : make_uint4((u32)(v & m26), (u32)(v >> 26), (u32)(v30 & m26), (u32)(v30 >> 26));
+        }
+    }
+}
+const ConvPlan *get_conv_plans(hb_ctx *c, int level) {
+    auto it = c->conv_plans.find(level);
+    if (it != c->conv_plans.end()) return it->second;
+    no_capture(c, "first key switch at this level");
+    const HostCtx &h = *c->h;
+    const int n = level + 1, K = h.K, ne = n + K, nd = h.digit_of(level) + 1;
+    auto prime_of = [&](int j) { return j < n ? j : h.L + 1 + (j - n); };
+    std::vector<ConvPlan> v((size_t)nd + 2);
+    std::memset(v.data(), 0, v.size() * sizeof(ConvPlan));
+    std::vector<int> special, q_all, q_low;
+    for (int k = 0; k < K; ++k) special.push_back(h.L + 1 + k);
+    for (int l = 0; l < n; ++l) { q_all.push_back(l); if (l < level) q_low.push_back(l); }
+    int entry = 0;
+    for (int dg = 0; dg < nd; ++dg) {
+        std::vector<int> src, dst;
+        for (int j = 0; j < ne; ++j) (j >= h.digit_lo(dg) && j < h.digit_hi(dg, n) ? src : dst).push_back(prime_of(j));
+        fill_conv(h, v[(size_t)dg], src, dst, h.digit_lo(dg), entry);
+        entry += (int)dst.size();
+    }
+    fill_conv(h, v[(size_t)nd], special, q_all, 0, 0);
+    if (level >= 1 && K < 8) {
+        std::vector<int> src{level};
+        src.insert(src.end(), special.begin(), special.end());
+        fill_conv(h, v[(size_t)nd + 1], src, q_low, 0, 0);
+        InvScale &sc = c->div_scale[level];
+        for (int l = 0; l < level; ++l) {
+            u64 d = h.q[level] % h.q[l];
+            for (int p : special) d = hbhost::mulmod(d, h.q[p] % h.q[l], h.q[l]);
+            scale_words(hbhost::invmod(d, h.q[l]), h.q[l], sc.w[l], sc.c[l]);
+        }
+    }
+    for (int l = 0; l < n; ++l) {
+        u64 d = 1;
+        for (int p : special) d = hbhost::mulmod(d, h.q[p] % h.q[l], h.q[l]);
+        scale_words(hbhost::invmod(d, h.q[l]), h.q[l], c->p_inv_scale.w[l], c->p_inv_scale.c[l]);
+    }
+    ConvPlan *d = nullptr;
+    CK(cudaMalloc(&d, v.size() * sizeof(ConvPlan)));
+    CK(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(ConvPlan), cudaMemcpyHostToDevice, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    c->conv_plans[level] = d;
+    return d;
+}
+template <int COLS> size_t strip_bytes(int strips) { return (size_t)strips * StripIndex<COLS>::kWords * 8; }
+void conv_opt_in(hb_ctx *c) {
+    if (c->smem_opt_in_conv) return;
+    CK(cudaFuncSetAttribute(conv_cols<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_bytes<8>(10)));
+    CK(cudaFuncSetAttribute(conv_cols<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_bytes<4>(10)));
+    CK(cudaFuncSetAttribute(lift_cols<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_bytes<8>(3)));
+    CK(cudaFuncSetAttribute(lift_cols<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_bytes<4>(3)));
+    c->smem_opt_in_conv = true;
+}
+// strip width and target split of a launch
+struct StripShape { int cols, split; };
+StripShape strip_shape(int instances, int targets) {
+    StripShape s{8, 1};
+    if (instances * 32 < 296) {
+        s.cols = 4;
+        while (s.split < 4 && instances * 64 * s.split * 2 <= 296 && targets > 2 * s.split) ++s.split;
+    }
+    if (const char *e = getenv("HB_COLS")) s.cols = atoi(e);
+    if (const char *e = getenv("HB_SPLIT")) s.split = atoi(e);
+    return s;
+}
+// `plans` conversions (the largest with max_ns sources and max_nt targets) of `instances` polynomials in one launch
+void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int max_nt, int instances) {
+    conv_opt_in(c);
+    const StripShape s = strip_shape(instances * count, max_nt);
+    if (s.cols == 8) LAUNCH(c), conv_cols<8><<<dim3(32, count * s.split, instances), 256, strip_bytes<8>(max_ns + 2), c->st>>>(src, so, dst, dof, plans, s.split, c->pc, c->tb.t16);
+    else LAUNCH(c), conv_cols<4><<<dim3(64, count * s.split, instances), 128, strip_bytes<4>(max_ns + 2), c->st>>>(src, so, dst, dof, plans, s.split, c->pc, c->tb.t16);
+}
+// half-inverse limbs of prime `level` (one per instance) -> half-forward lifts to the limbs below
+void launch_lift(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int level, int instances) {
+    conv_opt_in(c);
+    const StripShape s = strip_shape(instances, level);
+    if (s.cols == 8) LAUNCH(c), lift_cols<8><<<dim3(32, s.split, instances), 256, strip_bytes<8>(3), c->st>>>(src, so, dst, dof, level, s.split, c->pc, c->tb.t16);
+    else LAUNCH(c), lift_cols<4><<<dim3(64, s.split, instances), 128, strip_bytes<4>(3), c->st>>>(src, so, dst, dof, level, s.split, c->pc, c->tb.t16);
+}
+void inv_rows(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int count, const LimbMap &m) {
+    LAUNCH(c), launch_inv_rows16(c->st, src, so, dst, dof, count, m, c->pc, c->tb.t16);
+}
+void fwd_rows(hb_ctx *c, u64 *d, size_t outer, int count, const LimbMap &m) {
+    LAUNCH(c), launch_fwd_rows16(c->st, d, outer, count, m, c->pc, c->tb.t16);
+}
+LimbMap one_limb(int prime) { LimbMap m{}; m.n = 1; m.prime[0] = (unsigned char)prime; return m; }
+
 // host mirror of the few plan fields the launcher needs
 struct PlanDims { int n, ne, nd, K, dt_count; LimbMap dtmap; };
 PlanDims plan_dims(hb_ctx *c, int level) {
@@ -303,17 +401,35 @@ void ks_decompose(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch,
     const int N = c->N, n = d.n;
     const unsigned gx1 = (unsigned)((N + 255) / 256); // base-conversion kernels keep one coefficient per thread
     Tmp acoef(c, (size_t)batch * n);
+    if (c->logn == 16) {
+        inv_rows(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level));
+        launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.ne - 1, batch);
+        fwd_rows(c, dt, (size_t)d.dt_count * N, batch * d.dt_count, d.dtmap);
+        return;
+    }
     ntt(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level), true);
     LAUNCH(c), k_modup<<<dim3(gx1, d.nd, batch), 256, 0, c->st>>>(dt, acoef.p, pl, c->pc, N);
     ntt_inplace(c, dt, batch * d.dt_count, d.dtmap, false);
 }
 // ModDown of acc [batch*2][ne][N] into out: conversion of the special limbs, forward transform, final combination
-void moddown(hb_ctx *c, const u64 *acc, u64 *pco, u64 *tbuf, int level, int batch, u64 *out, size_t out_outer, const u64 *add0, const u64 *add1, size_t add_outer, u32 g) {
+void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int batch, u64 *out, size_t out_outer, const u64 *add0, const u64 *add1, size_t add_outer, u32 g) {
     const KsPlan *pl = get_plan(c, level);
     const PlanDims d = plan_dims(c, level);
     const int N = c->N, n = d.n, ne = d.ne, K = d.K;
     const unsigned gx1 = (unsigned)((N + 255) / 256), gx = c->gx();
     LimbMap pm{}; pm.n = K; for (int k = 0; k < K; ++k) pm.prime[k] = (unsigned char)(c->L + 1 + k);
+    if (c->logn == 16) { // the special limbs are transformed in place
+        const ConvPlan *cv = get_conv_plans(c, level);
+        u64 *sp = acc + (size_t)n * N;
+        inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, batch * 2 * K, pm);
+        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, n, batch * 2);
+        const RowsFin f{acc, (size_t)ne * N, {add0, add1}, add_outer, g, out, out_outer, 2};
+        LAUNCH(c), launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, batch * 2, f, c->p_inv_scale, c->pc, c->tb.t16);
+        CK(cudaGetLastError());
+        return;
+    }
+    Tmp pcob(c, (size_t)batch * 2 * K);
+    u64 *pco = pcob.p;
     ntt(c, acc + (size_t)n * N, (size_t)ne * N, pco, (size_t)K * N, batch * 2 * K, pm, true);
     LAUNCH(c), k_moddown_conv<<<dim3(gx1, 1, batch * 2), 256, 0, c->st>>>(tbuf, pco, pl, c->pc, c->L + 1, N);
     ntt_inplace(c, tbuf, batch * 2 * n, c->qmap(level), false);
@@ -326,11 +442,11 @@ void ks_apply(hb_ctx *c, const u64 *a, size_t a_outer, const u64 *dt, int level,
               const u64 *add1, size_t add_outer) {
     const KsPlan *pl = get_plan(c, level);
     const PlanDims d = plan_dims(c, level);
-    const int N = c->N, n = d.n, ne = d.ne, K = d.K;
+    const int N = c->N, n = d.n, ne = d.ne;
     const unsigned gx = c->gx();
-    Tmp acc(c, (size_t)batch * 2 * ne), pco(c, (size_t)batch * 2 * K), t(c, (size_t)batch * 2 * n);
+    Tmp acc(c, (size_t)batch * 2 * ne), t(c, (size_t)batch * 2 * n);
     LAUNCH(c), k_ks_inner<<<dim3(gx, batch, ne), 256, 0, c->st>>>(acc.p, a, a_outer, dt, key.d, c->nprimes, pl, c->pc, g, c->logn, N);
-    moddown(c, acc.p, pco.p, t.p, level, batch, out, out_outer, add0, add1, add_outer, g);
+    moddown(c, acc.p, t.p, level, batch, out, out_outer, add0, add1, add_outer, g);
 }
 // Hybrid key switch of polynomial a (NTT form, `n` limbs, per-batch stride a_outer) with key `key`
 void keyswitch(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch, const Evk &key, u32 g, u64 *out, size_t out_outer, const u64 *add0, const u64 *add1,
@@ -411,7 +527,6 @@ const DivPlan *get_div_plan(hb_ctx *c, int level) {
         for (int t = 0; t < ns; ++t) if (t != s) hat = hbhost::mulmod(hat, h.q[P->src_prime[t]] % ds, ds);
         const u64 hi_ = hbhost::invmod(hat, ds);
         P->hat_inv[s] = hi_; P->hat_inv_sh[s] = hbhost::shoup(hi_, ds);
-        c->div_hat_inv[level].push_back(hi_);
         for (int l = 0; l < level; ++l) {
             const u64 ql = h.q[l];
             u64 hm = 1;
@@ -437,22 +552,28 @@ const DivPlan *get_div_plan(hb_ctx *c, int level) {
     return d;
 }
 // E [batch][2][ne][N] over Q_level u P  ->  new ciphertext at level - 1:  (E - lift(E mod P*q_level)) / (P*q_level)
-hb_ct *divide_by_p_ql(hb_ctx *c, const u64 *E, int level, int batch) {
+hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch) {
     const DivPlan *dv = get_div_plan(c, level);
     const PlanDims d = plan_dims(c, level);
     const int N = c->N, n = d.n, ne = d.ne, ns = d.K + 1;
     hb_ct *r = new_ct(c, level - 1, 2, batch, 1);
     try {
         const unsigned gx1 = (unsigned)((N + 255) / 256), gx = c->gx();
-        Tmp sc(c, (size_t)batch * 2 * ns), t(c, (size_t)batch * 2 * level);
+        Tmp t(c, (size_t)batch * 2 * level);
         LimbMap sm{}; sm.n = ns; sm.prime[0] = (unsigned char)level; for (int k = 0; k < d.K; ++k) sm.prime[1 + k] = (unsigned char)(c->L + 1 + k);
-        // 2^16 rings: the inverse transform multiplies limb s by (D / d_s)^-1 on its way out, the conversion starts from there
-        const bool fold = c->logn == 16;
-        if (fold) {
-            const Ntt16Scale scale = ntt_scale(c, sm, c->div_hat_inv[level].data());
-            ntt(c, E + (size_t)(n - 1) * N, (size_t)ne * N, sc.p, (size_t)ns * N, batch * 2 * ns, sm, true, &scale);
-        } else ntt(c, E + (size_t)(n - 1) * N, (size_t)ne * N, sc.p, (size_t)ns * N, batch * 2 * ns, sm, true);
-        LAUNCH(c), k_div_conv<<<dim3(gx1, 1, batch * 2), 256, 0, c->st>>>(t.p, sc.p, dv, c->pc, N, fold ? 1 : 0);
+        u64 *src = E + (size_t)(n - 1) * N; // q_level and P sit side by side
+        if (c->logn == 16) {
+            const ConvPlan *cv = get_conv_plans(c, level);
+            inv_rows(c, src, (size_t)ne * N, src, (size_t)ne * N, batch * 2 * ns, sm);
+            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, level, batch * 2);
+            const RowsFin f{E, (size_t)ne * N, {nullptr, nullptr}, 0, 0u, r->d, (size_t)2 * level * N, 2};
+            LAUNCH(c), launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], c->pc, c->tb.t16);
+            CK(cudaGetLastError());
+            return r;
+        }
+        Tmp sc(c, (size_t)batch * 2 * ns);
+        ntt(c, src, (size_t)ne * N, sc.p, (size_t)ns * N, batch * 2 * ns, sm, true);
+        LAUNCH(c), k_div_conv<<<dim3(gx1, 1, batch * 2), 256, 0, c->st>>>(t.p, sc.p, dv, c->pc, N);
         ntt_inplace(c, t.p, batch * 2 * level, c->qmap(level - 1), false);
         LAUNCH(c), k_div_fin<<<dim3(gx, level, batch * 2), 256, 0, c->st>>>(r->d, E, t.p, ne, dv, c->pc, N);
         CK(cudaGetLastError());
@@ -535,6 +656,27 @@ void check_same(const hb_ct *a, const hb_ct *b, const char *what) {
     if (a->np != b->np || a->batch != b->batch || a->spow != b->spow) fail(HB_E_SHAPE, std::string(what) + ": shape mismatch");
 }
 
+// out[bp] = rescale of x[bp] (level + 1 limbs); scratch: nbp * (1 + level) limbs
+void rescale_core(hb_ctx *c, const u64 *x, u64 *out, int l, int np, int nbp, u64 *last, u64 *t) {
+    const int N = c->N;
+    const LimbMap lm = one_limb(l);
+    if (c->logn == 16) {
+        InvScale sc{};
+        for (int i = 0; i < l; ++i) scale_words(hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]), c->h->q[i], sc.w[i], sc.c[i]);
+        inv_rows(c, x + (size_t)l * N, (size_t)(l + 1) * N, last, (size_t)N, nbp, lm);
+        launch_lift(c, last, (size_t)N, t, (size_t)l * N, l, nbp);
+        const RowsFin f{x, (size_t)(l + 1) * N, {nullptr, nullptr, nullptr}, 0, 0u, out, (size_t)np * l * N, np};
+        LAUNCH(c), launch_fwd_rows_fin16(c->st, t, (size_t)l * N, l, nbp, f, sc, c->pc, c->tb.t16);
+    } else {
+        ntt(c, x + (size_t)l * N, (size_t)(l + 1) * N, last, (size_t)N, nbp, lm, true);
+        LAUNCH(c), k_rescale_prep<<<c->egrid(nbp * l), 256, 0, c->st>>>(t, last, l, c->pc, N);
+        ntt_inplace(c, t, nbp * l, c->qmap(l - 1), false);
+        Scalars qi{};
+        for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
+        LAUNCH(c), k_rescale_fin<<<c->egrid(nbp * l), 256, 0, c->st>>>(out, x, t, l, c->pc, N, qi);
+    }
+    CK(cudaGetLastError());
+}
 hb_ct *do_rescale(hb_ctx *c, const hb_ct *a) {
     own(c, a);
     if (a->level < 1) fail(HB_E_LEVEL, "rescale: level 0");
@@ -544,16 +686,24 @@ hb_ct *do_rescale(hb_ctx *c, const hb_ct *a) {
     ALG(c, (size_t)nbp * (2 * l + 1));
     try {
         Tmp last(c, (size_t)nbp), t(c, (size_t)nbp * l);
-        LimbMap lm{}; lm.n = 1; lm.prime[0] = (unsigned char)l;
-        ntt(c, a->d + (size_t)l * N, (size_t)(l + 1) * N, last.p, (size_t)N, nbp, lm, true);
-        LAUNCH(c), k_rescale_prep<<<c->egrid(nbp * l), 256, 0, c->st>>>(t.p, last.p, l, c->pc, N);
-        ntt_inplace(c, t.p, nbp * l, c->qmap(l - 1), false);
-        Scalars qi{};
-        for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
-        LAUNCH(c), k_rescale_fin<<<c->egrid(nbp * l), 256, 0, c->st>>>(r->d, a->d, t.p, l, c->pc, N, qi);
-        CK(cudaGetLastError());
+        rescale_core(c, a->d, r->d, l, a->np, nbp, last.p, t.p);
     } catch (...) { hb_ct_free(r); throw; }
     return r;
+}
+// last [groups][nbp][N], residues modulo q_l in NTT form -> t [nbp][l][N], NTT form: the sum over the groups of the centred lifts
+void lift_last(hb_ctx *c, u64 *last, int groups, int nbp, int l, u64 *t) {
+    const int N = c->N;
+    if (c->logn == 16 && groups == 1) {
+        inv_rows(c, last, (size_t)N, last, (size_t)N, nbp, one_limb(l));
+        launch_lift(c, last, (size_t)N, t, (size_t)l * N, l, nbp);
+        fwd_rows(c, t, (size_t)l * N, nbp * l, c->qmap(l - 1));
+        return;
+    }
+    Tmp S(c, (size_t)nbp);
+    ntt_inplace(c, last, groups * nbp, one_limb(l), true);
+    LAUNCH(c), k_centre_sum<<<dim3(c->gx(), nbp), 256, 0, c->st>>>((i64 *)S.p, last, groups, nbp, l, c->pc, N);
+    LAUNCH(c), k_lift_mod<<<c->egrid(nbp * l), 256, 0, c->st>>>(t, (const i64 *)S.p, l, c->pc, N);
+    ntt_inplace(c, t, nbp * l, c->qmap(l - 1), false);
 }
 // sum_j rescale(a_j (.) p_j)  (separate)  or  rescale(sum_j a_j (.) p_j)
 hb_ct *do_prod_rescale(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, int count, bool separate) {
@@ -573,13 +723,9 @@ hb_ct *do_prod_rescale(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, 
     hb_ct *r = new_ct(c, l - 1, a0->np, a0->batch, 1);
     ALG(c, (size_t)count * ((size_t)nbp * (l + 1) + (l + 1)) + (size_t)nbp * l);
     try {
-        Tmp last(c, (size_t)groups * nbp), S(c, (size_t)nbp), t(c, (size_t)nbp * l);
+        Tmp last(c, (size_t)groups * nbp), t(c, (size_t)nbp * l);
         LAUNCH(c), k_last_prod<<<dim3(gx, nbp, groups), 256, 0, c->st>>>(last.p, tl, separate ? 1 : 0, l, nbp, c->pc, N);
-        LimbMap lm{}; lm.n = 1; lm.prime[0] = (unsigned char)l;
-        ntt_inplace(c, last.p, groups * nbp, lm, true);
-        LAUNCH(c), k_centre_sum<<<dim3(gx, nbp), 256, 0, c->st>>>((i64 *)S.p, last.p, groups, nbp, l, c->pc, N);
-        LAUNCH(c), k_lift_mod<<<c->egrid(nbp * l), 256, 0, c->st>>>(t.p, (const i64 *)S.p, l, c->pc, N);
-        ntt_inplace(c, t.p, nbp * l, c->qmap(l - 1), false);
+        lift_last(c, last.p, groups, nbp, l, t.p);
         Scalars qi{};
         for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
         LAUNCH(c), k_prod_rescale_fin<<<c->egrid(nbp * l), 256, 0, c->st>>>(r->d, tl, t.p, l, nbp, c->pc, N, qi);
@@ -621,7 +767,7 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
     hb_ct *r = new_ct(c, l - 1, a0->np, parts * a0->batch, 1);
     ALG(c, (size_t)count * nbp * (l + 1) + used * (l + 1) + (size_t)gnbp * l);
     try {
-        Tmp last(c, (size_t)gnbp), S(c, (size_t)gnbp), t(c, (size_t)gnbp * l);
+        Tmp last(c, (size_t)gnbp), t(c, (size_t)gnbp * l);
         constexpr int G = 6; // parts per CTA: 6 x 17 mask chunks of 2 KB = 204 KB of shared memory
         const size_t smem = (size_t)G * count * 2048;
         const unsigned pg = (unsigned)((parts + G - 1) / G);
@@ -629,11 +775,7 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
         Scalars qi{};
         for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
         LAUNCH(c), k_prod_parts<G><<<dim3(gx1, 1, pg), 1024, smem, c->st>>>(last.p, pt, nullptr, l, nbp, c->pc, N, qi, c->dev_err);
-        LimbMap lm{}; lm.n = 1; lm.prime[0] = (unsigned char)l;
-        ntt_inplace(c, last.p, gnbp, lm, true);
-        LAUNCH(c), k_centre_sum<<<dim3(c->gx(), gnbp), 256, 0, c->st>>>((i64 *)S.p, last.p, 1, gnbp, l, c->pc, N);
-        LAUNCH(c), k_lift_mod<<<c->egrid(gnbp * l), 256, 0, c->st>>>(t.p, (const i64 *)S.p, l, c->pc, N);
-        ntt_inplace(c, t.p, gnbp * l, c->qmap(l - 1), false);
+        lift_last(c, last.p, 1, gnbp, l, t.p);
         LAUNCH(c), k_prod_parts<G><<<dim3(gx1, (unsigned)l, pg), 1024, smem, c->st>>>(r->d, pt, t.p, l, nbp, c->pc, N, qi, c->dev_err);
         CK(cudaGetLastError());
     } catch (...) { hb_ct_free(r); throw; }
@@ -819,6 +961,14 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             // the open-ended sum of k_matmul_acc folds at this count.
             p.lazy_terms = (u64)((((unsigned __int128)1 << 52) * 5) / ((unsigned __int128)q * 8));
             if (p.fp && p.lazy_terms < 160) throw std::invalid_argument("prime too large for the lazy FP64-assisted sums");
+            // primes of 45 bits and more: values are folded with shifts by the bit length b, which needs q close below 2^b; the
+            // primes of a context are the first ones below a power of two, at most a few hundred 2N-steps away from it
+            int bits = 0;
+            while (bits < 64 && (q >> bits)) ++bits;
+            p.fold_shift = bits > 32 ? (u32)(bits - 32) : 0;
+            if (!p.fp && (((u64)1 << bits) - q) >> (bits - 12)) throw std::invalid_argument("prime too far below its power of two");
+            const u64 below60 = q < ((u64)1 << 60) ? ((u64)1 << 60) - q : 0;
+            p.d60 = below60 < ((u64)1 << 26) ? (u32)below60 : 0;
             std::vector<u64> f, fs, iv, ivs;
             c->h->twiddles(i, f, fs, iv, ivs);
             if (p.small) { // companion words hold w/q as doubles instead of Shoup quotients
@@ -870,6 +1020,7 @@ void hb_ctx_destroy(hb_ctx *c) {
     if (c->st) cudaStreamSynchronize(c->st);
     for (auto &kv : c->plans) cudaFree(kv.second);
     for (auto &kv : c->div_plans) cudaFree(kv.second);
+    for (auto &kv : c->conv_plans) cudaFree(kv.second);
     for (auto &kv : c->gal_tables) cudaFree(kv.second);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->pc) cudaFree(c->pc);
@@ -1296,14 +1447,7 @@ int hb_rescale_noalloc(hb_ctx *c, const hb_ct *a, hb_ct *out) {
                                  " (one 2-poly ciphertext at level 12 and N = 2^16)");
         u64 *scratch = noalloc_scratch(c->device); // first call on a device resolves the address
         u64 *last = scratch, *t = scratch + (size_t)nbp * N;
-        LimbMap lm{}; lm.n = 1; lm.prime[0] = (unsigned char)l;
-        ntt(c, a->d + (size_t)l * N, (size_t)(l + 1) * N, last, (size_t)N, nbp, lm, true);
-        LAUNCH(c), k_rescale_prep<<<c->egrid(nbp * l), 256, 0, c->st>>>(t, last, l, c->pc, N);
-        ntt_inplace(c, t, nbp * l, c->qmap(l - 1), false);
-        Scalars qi{};
-        for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
-        LAUNCH(c), k_rescale_fin<<<c->egrid(nbp * l), 256, 0, c->st>>>(out->d, a->d, t, l, c->pc, N, qi);
-        CK(cudaGetLastError());
+        rescale_core(c, a->d, out->d, l, a->np, nbp, last, t);
         out->spow = 1;
     });
 }
@@ -1439,7 +1583,7 @@ static hb_ct *rotate_sum_core(hb_ctx *c, const u64 *const *base, const int64_t *
     const int N = c->N;
     const KsPlan *pl = get_plan(c, level);
     const PlanDims d = plan_dims(c, level);
-    const int n = d.n, ne = d.ne, K = d.K;
+    const int n = d.n, ne = d.ne;
     const size_t ct_outer = (size_t)2 * n * N;
     RotTermList rot{}; PlainTermList plain{};
     std::vector<u64 *> dts;
@@ -1471,9 +1615,9 @@ static hb_ct *rotate_sum_core(hb_ctx *c, const u64 *const *base, const int64_t *
         if (rot.count == 0) {
             CK(cudaMemcpyAsync(r->d, add.p, r->limbs() * N * 8, cudaMemcpyDeviceToDevice, c->st));
         } else {
-            Tmp acc(c, (size_t)batch * 2 * ne), pco(c, (size_t)batch * 2 * K), t(c, (size_t)batch * 2 * n);
+            Tmp acc(c, (size_t)batch * 2 * ne), t(c, (size_t)batch * 2 * n);
             LAUNCH(c), k_ks_inner_sum<<<dim3(gx, batch, ne), 256, 0, c->st>>>(acc.p, rot, ct_outer, c->nprimes, pl, c->pc, c->logn, N);
-            moddown(c, acc.p, pco.p, t.p, level, batch, r->d, ct_outer, add.p, add.p + (size_t)n * N, ct_outer, 0u);
+            moddown(c, acc.p, t.p, level, batch, r->d, ct_outer, add.p, add.p + (size_t)n * N, ct_outer, 0u);
         }
         CK(cudaGetLastError());
     } catch (...) { for (u64 *p : dts) c->pool.put(p); hb_ct_free(r); throw; }

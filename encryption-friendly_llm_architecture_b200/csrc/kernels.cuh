@@ -16,7 +16,7 @@ namespace hb {
 constexpr int kElems = 4;
 
 // out = a + b  (mode 0) | a - b (mode 1) | -a (mode 2)
-__global__ void k_addsub(u64 *__restrict__ out, const u64 *__restrict__ a, const u64 *__restrict__ b, LimbMap map, const PrimeConst *__restrict__ pc,
+__global__ void k_addsub(u64 *__restrict__ out, const u64 *__restrict__ a, const u64 *__restrict__ b, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc,
                          int N, int mode) {
     const int li = blockIdx.y;
 #pragma unroll
@@ -34,7 +34,7 @@ __global__ void k_addsub(u64 *__restrict__ out, const u64 *__restrict__ a, const
 
 struct Scalars { u64 v[kMaxPrimes]; };
 // out = a * s[prime]
-__global__ void k_scalar_mul(u64 *__restrict__ out, const u64 *__restrict__ a, size_t a_outer, LimbMap map, const PrimeConst *__restrict__ pc, int N, Scalars s) {
+__global__ void k_scalar_mul(u64 *__restrict__ out, const u64 *__restrict__ a, size_t a_outer, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N, const __grid_constant__ Scalars s) {
     const int li = blockIdx.y;
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
@@ -47,7 +47,7 @@ __global__ void k_scalar_mul(u64 *__restrict__ out, const u64 *__restrict__ a, s
     }
 }
 // multiplication by X^(N/2): +iu on the first half of an NTT-form limb, -iu on the second
-__global__ void k_mult_imag(u64 *__restrict__ out, const u64 *__restrict__ a, LimbMap map, const PrimeConst *__restrict__ pc, int N) {
+__global__ void k_mult_imag(u64 *__restrict__ out, const u64 *__restrict__ a, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N) {
     const int li = blockIdx.y;
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
@@ -61,7 +61,7 @@ __global__ void k_mult_imag(u64 *__restrict__ out, const u64 *__restrict__ a, Li
     }
 }
 // out = a (.) pt, pt limb = li % map.n
-__global__ void k_mul_pt(u64 *__restrict__ out, const u64 *__restrict__ a, const u64 *__restrict__ pt, LimbMap map, const PrimeConst *__restrict__ pc, int N) {
+__global__ void k_mul_pt(u64 *__restrict__ out, const u64 *__restrict__ a, const u64 *__restrict__ pt, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N) {
     const int li = blockIdx.y;
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
@@ -74,7 +74,7 @@ __global__ void k_mul_pt(u64 *__restrict__ out, const u64 *__restrict__ a, const
 }
 // out = a (.) pa + b (.) pb
 __global__ void k_mul2_add(u64 *__restrict__ out, const u64 *__restrict__ a, const u64 *__restrict__ pa, const u64 *__restrict__ b, const u64 *__restrict__ pb,
-                           LimbMap map, const PrimeConst *__restrict__ pc, int N) {
+                           const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N) {
     const int li = blockIdx.y;
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
@@ -91,7 +91,7 @@ __global__ void k_mul2_add(u64 *__restrict__ out, const u64 *__restrict__ a, con
 // tensor product, optional accumulation.  grid.y = batch * n; x, y: [groups][batch][2][n][N]; d: [batch][3][n][N]
 //   d[b] (+)= sum over the groups g of tensor(x[g][b], y[g][b])
 // (groups = 1 is the plain tensor product; several groups are several iterations of a product loop in one launch).
-__global__ void k_tensor(u64 *__restrict__ d, const u64 *__restrict__ x, const u64 *__restrict__ y, int n, LimbMap map, const PrimeConst *__restrict__ pc, int N,
+__global__ void k_tensor(u64 *__restrict__ d, const u64 *__restrict__ x, const u64 *__restrict__ y, int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N,
                          int accumulate, int groups, int batch) {
     const int bl = blockIdx.y, b = bl / n, l = bl % n;
     const size_t gstride = (size_t)batch * 2 * n * N;
@@ -136,7 +136,7 @@ __global__ void k_permute(u64 *__restrict__ out, const u64 *__restrict__ in, u32
     }
 }
 // int64 coefficients -> residues of every limb instance (coefficient form)
-__global__ void k_reduce_i64(u64 *__restrict__ out, const i64 *__restrict__ coef, LimbMap map, const PrimeConst *__restrict__ pc, int N) {
+__global__ void k_reduce_i64(u64 *__restrict__ out, const i64 *__restrict__ coef, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N) {
     const int li = blockIdx.y;
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
@@ -148,7 +148,7 @@ __global__ void k_reduce_i64(u64 *__restrict__ out, const i64 *__restrict__ coef
     }
 }
 // x mod q for lazily summed residues
-__global__ void k_mod_reduce(u64 *__restrict__ a, LimbMap map, const PrimeConst *__restrict__ pc, int N) {
+__global__ void k_mod_reduce(u64 *__restrict__ a, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N) {
     const int li = blockIdx.y;
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
@@ -161,7 +161,7 @@ __global__ void k_mod_reduce(u64 *__restrict__ a, LimbMap map, const PrimeConst 
 }
 // out = (x_0 + ... + x_{count-1}) mod q for canonical residues (count <= 16: the sum stays below 2^64)
 struct SumList { const u64 *x[16]; int count; };
-__global__ void k_sum_mod(u64 *__restrict__ out, SumList sl, LimbMap map, const PrimeConst *__restrict__ pc, int N) {
+__global__ void k_sum_mod(u64 *__restrict__ out, const __grid_constant__ SumList sl, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N) {
     const int li = blockIdx.y;
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
@@ -192,7 +192,7 @@ __global__ void k_rescale_prep(u64 *__restrict__ t, const u64 *__restrict__ last
 }
 // out[bp][l] = (x[bp][l] - t[bp][l]) * q_level^-1 ; x has level+1 limbs per poly
 __global__ void k_rescale_fin(u64 *__restrict__ out, const u64 *__restrict__ x, const u64 *__restrict__ t, int level, const PrimeConst *__restrict__ pc, int N,
-                              Scalars qlinv) {
+                              const __grid_constant__ Scalars qlinv) {
     const int w = blockIdx.y, bp = w / level, l = w % level;
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
@@ -215,7 +215,7 @@ constexpr int kMaxTerms = 24;
 struct TermList { const u64 *a[kMaxTerms]; const u64 *p[kMaxTerms]; int count; };
 // last[g][bp][x] = (sum over the terms of group g) a_j[bp][level][x] * p_j[level][x] mod q_level
 // grid = (N/256, nbp, groups)   groups = count (separate) or 1
-__global__ void k_last_prod(u64 *__restrict__ last, TermList tl, int separate, int level, int nbp, const PrimeConst *__restrict__ pc, int N) {
+__global__ void k_last_prod(u64 *__restrict__ last, const __grid_constant__ TermList tl, int separate, int level, int nbp, const PrimeConst *__restrict__ pc, int N) {
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
         const int x = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
@@ -268,7 +268,7 @@ __global__ void k_lift_mod(u64 *__restrict__ t, const i64 *__restrict__ S, int l
 // next) are in flight together: the kernel streams `count` ciphertexts per output and lives on memory parallelism.
 // Blocks are ordered limb-major (all batch members of limb 0, then of limb 1, ...): the plaintext limbs of a sum are
 // shared by every member, and in this order they stay in L2 while the members stream past.
-__global__ void k_prod_rescale_fin(u64 *__restrict__ out, TermList tl, const u64 *__restrict__ t, int level, int nbp, const PrimeConst *__restrict__ pc, int N, Scalars qlinv) {
+__global__ void k_prod_rescale_fin(u64 *__restrict__ out, const __grid_constant__ TermList tl, const u64 *__restrict__ t, int level, int nbp, const PrimeConst *__restrict__ pc, int N, const __grid_constant__ Scalars qlinv) {
     const int l = blockIdx.y / nbp, bp = blockIdx.y % nbp, w = bp * level + l;
     const PrimeConst m = pc[l];
     const u32 x0 = blockIdx.x * (blockDim.x * kElems) + threadIdx.x;
@@ -618,7 +618,7 @@ __global__ void k_moddown_fin(u64 *__restrict__ out, size_t out_outer, const u64
 struct RotTerm { const u64 *a_ntt; const u64 *dt; const u64 *key; u32 g; u32 pad; };
 struct RotTermList { RotTerm t[16]; int count; };
 //   acc[b][p][j][i] = sum_t sum_dg digit_t,dg[j][perm_t(i)] * key_t[dg][p][prime(j)][i]      grid = (N/(256*kElems), batch, ne)
-__global__ void k_ks_inner_sum(u64 *__restrict__ acc, RotTermList tl, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc,
+__global__ void k_ks_inner_sum(u64 *__restrict__ acc, const __grid_constant__ RotTermList tl, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc,
                                int logn, int N) {
     const int j = blockIdx.z, b = blockIdx.y;
     const int pj = pl->ext_prime[j], nd = pl->nd, ne = pl->ne;
@@ -685,7 +685,7 @@ __global__ void k_ks_inner_sum(u64 *__restrict__ acc, RotTermList tl, size_t a_o
 // add[b][p][l][i] = sum over the rotated terms of (p == 0) c0_t[b][l][perm_t(i)]  +  sum over the unrotated terms of x_t[b][p][l][i]
 // rot: terms with g != 1 (a_ntt - n limbs = c0); plain: terms added as they are.  grid = (N/(256*kElems), n, batch*2)
 struct PlainTermList { const u64 *x[16]; int count; };
-__global__ void k_rot_sum_addend(u64 *__restrict__ add, RotTermList rot, PlainTermList plain, int n, LimbMap map, const PrimeConst *__restrict__ pc, int logn, int N) {
+__global__ void k_rot_sum_addend(u64 *__restrict__ add, const __grid_constant__ RotTermList rot, const __grid_constant__ PlainTermList plain, int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int logn, int N) {
     const int l = blockIdx.y, bp = blockIdx.z, b = bp >> 1, p = bp & 1;
     const u64 q = pc[map.prime[l]].q;
     const size_t ct_outer = (size_t)2 * n * N;
@@ -722,7 +722,7 @@ struct RotPair {                       // the two rotations of one call
 // E[b][p][j][i] = sum_r mask_r[j][i] * (sum_dg digit_dg[j][perm_r(i)] * key_r[dg][p][prime(j)][i])
 //               + (p == 0 and j < n)  P * sum_r mask_r[j][i] * c0[b][j][perm_r(i)]
 // Every term is reduced to its canonical residue before the next operation uses it.  grid = (N/(256*kElems), ne, batch)
-__global__ void k_ks_inner_pair(u64 *__restrict__ E, const u64 *__restrict__ c0, const u64 *__restrict__ a_ntt, size_t a_outer, const u64 *__restrict__ dt, RotPair rp,
+__global__ void k_ks_inner_pair(u64 *__restrict__ E, const u64 *__restrict__ c0, const u64 *__restrict__ a_ntt, size_t a_outer, const u64 *__restrict__ dt, const __grid_constant__ RotPair rp,
                                 int key_primes, const KsPlan *__restrict__ pl, const DivPlan *__restrict__ dv, const PrimeConst *__restrict__ pc, int logn, int N) {
     const int j = blockIdx.y, b = blockIdx.z;
     const int pj = pl->ext_prime[j], nd = pl->nd, ne = pl->ne, n = pl->n;
@@ -843,7 +843,7 @@ struct MaskedRotList { MaskedRot r[kMaxRotGroups]; }; // one entry per wrapped c
 // grid = (N/(256*EL), groups * batch, ne); EL coefficients per thread.  Output member g * batch + b is wrapped copy
 // number g (its own pair of masked keys) of input member b: several iterations of a shift loop in one launch.
 template <int EL>
-__global__ void __launch_bounds__(256, EL == 2 ? 3 : 2) k_ks_inner_mk(u64 *__restrict__ E, const u64 *__restrict__ c0, const u64 *__restrict__ a_ntt, size_t a_outer, const u64 *__restrict__ dt, MaskedRotList mrl,
+__global__ void __launch_bounds__(256, EL == 2 ? 3 : 2) k_ks_inner_mk(u64 *__restrict__ E, const u64 *__restrict__ c0, const u64 *__restrict__ a_ntt, size_t a_outer, const u64 *__restrict__ dt, const __grid_constant__ MaskedRotList mrl,
                               int batch, const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, int logn, int N) {
     const int j = blockIdx.z, ob = blockIdx.y, b = ob % batch; // limb-major block order: the key limbs stay in L2 across the members
     const MaskedRot &mr = mrl.r[ob / batch];
@@ -1069,16 +1069,14 @@ __global__ void __launch_bounds__(256) k_ks_inner_mkb(u64 *__restrict__ E, const
 }
 // Base conversion of the division: src [bp][ns][N] (limbs q_level, P; coefficient form) -> t [bp][level][N]
 // grid = (N/256, 1, nbp)
-// prescaled: the inverse transform that produced src already multiplied limb k by hat_inv[k]
 template <int NS>
-__device__ __forceinline__ void div_conv_body(u64 *__restrict__ t, const u64 *__restrict__ src, const DivPlan *__restrict__ dv, const PrimeConst *__restrict__ pc, int N, int i, int bp,
-                                              int prescaled) {
+__device__ __forceinline__ void div_conv_body(u64 *__restrict__ t, const u64 *__restrict__ src, const DivPlan *__restrict__ dv, const PrimeConst *__restrict__ pc, int N, int i, int bp) {
     const int nl = dv->level;
     u64 y[NS];
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
         const u64 v = src[((size_t)bp * NS + k) * N + i];
-        y[k] = prescaled ? v : mul_shoup(v, dv->hat_inv[k], dv->hat_inv_sh[k], pc[dv->src_prime[k]].q);
+        y[k] = mul_shoup(v, dv->hat_inv[k], dv->hat_inv_sh[k], pc[dv->src_prime[k]].q);
     }
     u64 *o = t + (size_t)bp * nl * N + i;
     // targets below 2^44: y = y1 * 2^30 + y0 with both pieces as doubles, products on the FP64 pipe against the constants
@@ -1109,18 +1107,18 @@ __device__ __forceinline__ void div_conv_body(u64 *__restrict__ t, const u64 *__
         o += N;
     }
 }
-__global__ void k_div_conv(u64 *__restrict__ t, const u64 *__restrict__ src, const DivPlan *__restrict__ dv, const PrimeConst *__restrict__ pc, int N, int prescaled) {
+__global__ void k_div_conv(u64 *__restrict__ t, const u64 *__restrict__ src, const DivPlan *__restrict__ dv, const PrimeConst *__restrict__ pc, int N) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     const int bp = blockIdx.z;
     switch (dv->ns) {
-    case 2: div_conv_body<2>(t, src, dv, pc, N, i, bp, prescaled); break;
-    case 3: div_conv_body<3>(t, src, dv, pc, N, i, bp, prescaled); break;
-    case 4: div_conv_body<4>(t, src, dv, pc, N, i, bp, prescaled); break;
-    case 5: div_conv_body<5>(t, src, dv, pc, N, i, bp, prescaled); break;
-    case 6: div_conv_body<6>(t, src, dv, pc, N, i, bp, prescaled); break;
-    case 7: div_conv_body<7>(t, src, dv, pc, N, i, bp, prescaled); break;
-    default: div_conv_body<8>(t, src, dv, pc, N, i, bp, prescaled); break;
+    case 2: div_conv_body<2>(t, src, dv, pc, N, i, bp); break;
+    case 3: div_conv_body<3>(t, src, dv, pc, N, i, bp); break;
+    case 4: div_conv_body<4>(t, src, dv, pc, N, i, bp); break;
+    case 5: div_conv_body<5>(t, src, dv, pc, N, i, bp); break;
+    case 6: div_conv_body<6>(t, src, dv, pc, N, i, bp); break;
+    case 7: div_conv_body<7>(t, src, dv, pc, N, i, bp); break;
+    default: div_conv_body<8>(t, src, dv, pc, N, i, bp); break;
     }
 }
 // out[bp][l][i] = (E[bp][l][i] - t[bp][l][i]) * D^-1 for l < level.  grid = (N/(256*kElems), level, batch*2)
@@ -1159,7 +1157,7 @@ __device__ __forceinline__ void chacha_block(const ChaChaKey &key, u32 domain, u
 }
 // uniform residues: limb instance li (prime pi = map.prime[li]) coefficient c = (128-bit word (pi*N + c) of the stream) mod q.
 // One thread produces the four coefficients of one ChaCha block.  grid = (N/4/256, count)
-__global__ void k_uniform(u64 *__restrict__ out, LimbMap map, const PrimeConst *__restrict__ pc, int N, ChaChaKey key, u32 domain, u64 id) {
+__global__ void k_uniform(u64 *__restrict__ out, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N, ChaChaKey key, u32 domain, u64 id) {
     const int li = blockIdx.y;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t * 4 >= N) return;
@@ -1176,7 +1174,7 @@ __global__ void k_uniform(u64 *__restrict__ out, LimbMap map, const PrimeConst *
 
 // ---------------- encrypt / decrypt / key generation ----------------
 // b = e - a*s + msg   (all NTT form).  grid.y = n limbs
-__global__ void k_encrypt(u64 *__restrict__ b, const u64 *__restrict__ a, const u64 *__restrict__ e, const u64 *__restrict__ s, const u64 *__restrict__ msg, LimbMap map,
+__global__ void k_encrypt(u64 *__restrict__ b, const u64 *__restrict__ a, const u64 *__restrict__ e, const u64 *__restrict__ s, const u64 *__restrict__ msg, const __grid_constant__ LimbMap map,
                           const PrimeConst *__restrict__ pc, int N) {
     const int li = blockIdx.y;
 #pragma unroll
@@ -1207,7 +1205,7 @@ __global__ void k_decrypt(u64 *__restrict__ out, const u64 *__restrict__ ct, int
 // switching-key body: b = e - a*s + [prime in digit] * (P mod q) * s',  s' = s^2 (g == 0) or s o perm_g.
 // grid.y = nprimes; one digit per launch.
 __global__ void k_keygen(u64 *__restrict__ b, const u64 *__restrict__ a, const u64 *__restrict__ e, const u64 *__restrict__ s, const PrimeConst *__restrict__ pc, int N,
-                         int logn, u32 g, int dig_lo, int dig_hi, Scalars pmod) {
+                         int logn, u32 g, int dig_lo, int dig_hi, const __grid_constant__ Scalars pmod) {
     const int pi = blockIdx.y;
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
@@ -1231,8 +1229,8 @@ __global__ void k_keygen(u64 *__restrict__ b, const u64 *__restrict__ a, const u
 // (scale Delta^2, no rescale).  Shifted copies are stored k-major; the sum over b adds the partial products
 // of several K-groups in the same pass.  grid = (N/256, 2*n).  The 128-bit accumulator is folded every 64 terms.
 struct PtList { const u64 *p[16]; };
-__global__ void k_matmul_acc(u64 *__restrict__ out, const u64 *__restrict__ pre, int kcount, int btotal, int b0, int bcount, PtList pts, const u32 *__restrict__ gal,
-                             int n, LimbMap map, const PrimeConst *__restrict__ pc, int logn, int N) {
+__global__ void k_matmul_acc(u64 *__restrict__ out, const u64 *__restrict__ pre, int kcount, int btotal, int b0, int bcount, const __grid_constant__ PtList pts, const u32 *__restrict__ gal,
+                             int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int logn, int N) {
     const int pl = blockIdx.y, l = pl % n;
     const PrimeConst m = pc[map.prime[l]];
     const size_t estride = (size_t)2 * n * N;

@@ -22,11 +22,13 @@ struct PrimeConst {
     u64 mu_hi, mu_lo;   // floor(2^128 / q)
     u64 n_inv, n_inv_sh; // N^-1 mod q and its Shoup companion
     u64 iu, iu_sh;      // psi^(N/2): the image of the imaginary unit
-    u64 small;          // 1 when q < 2^44 and N = 2^16: the NTT tables hold w/q doubles (see mul_fp_lazy)
+    u64 small;          // 1 when q < 2^44 and N = 2^16: the transforms carry its residues as doubles
     double q_inv_f;     // 1/q
     double n_inv_f;     // n_inv / q
     u64 fp;             // 1 when q < 2^44: element-wise kernels take quotients from the FP64 pipe
     u64 lazy_terms;     // how many lazy products (each below 1.6 q) may be summed before the sum reaches 2^52
+    u32 fold_shift;     // primes of b >= 45 bits: b - 32 (every such prime of a context lies within 2^(b-12) below 2^b)
+    u32 d60;            // 2^60 - q when that is positive and below 2^26, else 0
 };
 
 // Limb instances of a launch: instance li (0 <= li < count) uses prime[li % n].
@@ -43,6 +45,40 @@ __device__ __forceinline__ u64 mul_shoup_lazy(u64 x, u64 w, u64 wsh, u64 q) {
 }
 __device__ __forceinline__ u64 mul_shoup(u64 x, u64 w, u64 wsh, u64 q) {
     u64 r = mul_shoup_lazy(x, w, wsh, q);
+    return r >= q ? r - q : r;
+}
+// ---- cheaper lazy forms for the primes of 45 to 60 bits --------------------------------------------------------
+// Every integer instruction except a 32-bit add costs two issue cycles on one 16-lane pipe here, and a full 64 x 64 high
+// product costs nineteen.  The quotient of a Shoup product does not need it: h = x1 s1 + hi(x0 s1) + hi(x1 s0) (three
+// 32 x 32 products) is low by less than three, so x*w - h*q lies in [0, 4q) for any x < 2^64.  A radix-16 round of
+// butterflies with it takes 36 (Cooley-Tukey) and 41 (Gentleman-Sande) cycles per warp butterfly, with the exact
+// high product and a conditional subtraction per butterfly 49.
+__device__ __forceinline__ u32 hi32_wide(u32 a, u32 b) { // the high word of the full product, kept in the two-cycle wide form
+    u32 h;
+    asm("{\n\t.reg .u32 l;\n\t.reg .u64 t;\n\tmul.wide.u32 t, %1, %2;\n\tmov.b64 {l, %0}, t;\n\t}" : "=r"(h) : "r"(a), "r"(b));
+    return h;
+}
+__device__ __forceinline__ u64 mul_shoup4(u64 x, u64 w, u64 wsh, u64 nq /* 2^64 - q */) {
+    const u32 x0 = (u32)x, x1 = (u32)(x >> 32), s0 = (u32)wsh, s1 = (u32)(wsh >> 32), w0 = (u32)w, w1 = (u32)(w >> 32), n0 = (u32)nq, n1 = (u32)(nq >> 32);
+    const u32 a = hi32_wide(x0, s1), b = hi32_wide(x1, s0);
+    u32 h0, h1, lo, hi;
+    asm("{\n\t.reg .u64 t;\n\tmul.wide.u32 t, %2, %3;\n\tmov.b64 {%0, %1}, t;\n\t"
+        "add.cc.u32 %0, %0, %4;\n\taddc.u32 %1, %1, 0;\n\tadd.cc.u32 %0, %0, %5;\n\taddc.u32 %1, %1, 0;\n\t}"
+        : "=&r"(h0), "=&r"(h1) : "r"(x1), "r"(s1), "r"(a), "r"(b));
+    asm("{\n\t.reg .u64 t;\n\tmul.wide.u32 t, %2, %3;\n\tmad.wide.u32 t, %4, %5, t;\n\tmov.b64 {%0, %1}, t;\n\t}"
+        : "=r"(lo), "=r"(hi) : "r"(x0), "r"(w0), "r"(h0), "r"(n0));
+    hi = x0 * w1 + hi; hi = x1 * w0 + hi; hi = h0 * n1 + hi; hi = h1 * n0 + hi;
+    return ((u64)hi << 32) | lo;
+}
+// x < 16 q  ->  congruent value below (1 + 2^-7) * 2^b: subtracts (x >> b) * q
+__device__ __forceinline__ u64 fold_q(u64 x, u64 nq, u32 fold_shift) {
+    const u32 k = (u32)(x >> 32) >> fold_shift;
+    u64 r;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(k), "r"((u32)nq), "l"(x));
+    return r + ((u64)(k * (u32)(nq >> 32)) << 32);
+}
+__device__ __forceinline__ u64 canon_q(u64 x, u64 q, u32 fold_shift) { // x < 16 q -> [0, q)
+    const u64 r = fold_q(x, 0ull - q, fold_shift);
     return r >= q ? r - q : r;
 }
 // (z1:z0) mod q, any 128-bit input.  The quotient estimate is low by at most 4.
@@ -90,10 +126,6 @@ __device__ __forceinline__ u64 mad2_lo64(u64 a, u64 b, u64 c, u64 d, u64 e) {
     asm("mad.lo.u32 %0, %1, %2, %0;" : "+r"(hi) : "r"(c0), "r"(d1));
     asm("mad.lo.u32 %0, %1, %2, %0;" : "+r"(hi) : "r"(c1), "r"(d0));
     return ((u64)hi << 32) | lo;
-}
-__device__ __forceinline__ u64 mul_fp_lazy(u64 y, u64 w, double w_over_q, u64 q) {
-    const u64 qh = mantissa52(__fma_rn(u52_to_double(y), w_over_q, kTwo52));
-    return mad2_lo64(y, w, qh, 0ull - q, q); // y*w - qh*q + q
 }
 // v < 2^52 -> residue in (0.4q, 1.6q)
 __device__ __forceinline__ u64 reduce_fp_lazy(u64 v, double q_inv, u64 q) {

@@ -16,18 +16,15 @@
 //
 //  * For primes below 2^44 the coefficients are carried as integer-valued doubles ("double storage") from the first
 //    load of a transform to its last store, signed and unreduced.  A butterfly is then
-//        qh = fma(y, w/q, M)                 quotient estimate, M = 2^52 + 2^51          (FP64)
-//        yb = y + M                          integer image of y in the mantissa           (FP64)
-//        r  = yb*w - qh*q + q  (low 48 bits)  six 32-bit multiply-adds                     (FMA pipe)
-//        t  = double(2^52 | r) - (2^52 + q)  exact remainder in (-0.52 q, 0.52 q)          (1 logic op + FP64)
-//        x' = x + t,  y' = x - t                                                          (FP64)
-//    twelve instructions, five of them on the FP64 pipe, six on the multiply-add pipe and one on the ALU, where the
-//    all-integer butterfly spends most of its issue slots on 64-bit adds, compares and selects.  Every step is exact:
-//    the quotient estimate is off by less than 0.02, so the remainder is the true residue class representative in
-//    (-0.52 q, 0.52 q); values grow by at most 0.52 q per forward stage (|x| < 9.4 q after 16 stages, far below 2^51).
+//        p  = y*w, e = fma(y, w, -p)              product and its rounding error
+//        qh = fma(y, w/q, M) - M                  quotient estimate, M = 2^52 + 2^51, off by less than 0.02
+//        t  = fma(-qh, q, p) + e                  exact remainder in (-0.52 q, 0.52 q)
+//        x' = x + t,  y' = x - t
+//    eight instructions, all on the FP64 pipe (which runs beside the integer pipe).  Values grow by at most 0.52 q per
+//    forward stage (|x| < 9.4 q after 16 stages from a canonical start, far below 2^51).
 //    The pass boundary stores the doubles as they are (the intermediate array is private to the transform); the last
 //    store reduces to the canonical residue, so the bits that reach memory are those of any other exact method.
-//    Primes of 44 bits and more use Shoup butterflies on integers in [0, 4q).
+//    Primes of 44 bits and more use Shoup butterflies on integers below 16 q.
 #pragma once
 #include "modarith.cuh"
 #include <cstring>
@@ -86,12 +83,6 @@ template <class F> inline void ntt16_fill_rows_b8(double *out, F w) {
         }
 }
 
-// Optional last multiplication of the inverse transform: position k = li % map.n gets scale s_k (which must already
-// contain N^-1) instead of N^-1 -- a base conversion that follows folds its first product (the inverse of a complementary
-// modulus) into the transform.  w: s_k (as ds_twiddle_word for primes below 2^44), comp: s_k / q as a double, or the
-// Shoup companion.
-struct Ntt16Scale { u64 w[8], comp[8]; int on; };
-
 // address of limb instance li: (li / period) * outer + (li % period) * N
 struct LimbAddr16 {
     size_t outer;
@@ -99,6 +90,7 @@ struct LimbAddr16 {
 };
 
 // ---------------- Shoup butterflies on integers (primes of 44 bits and more) ----------------
+// exact quotients, values in [0, 4q) and [0, 2q): the small-ring kernel
 __device__ __forceinline__ void ct_bfly(u64 &x, u64 &y, u64 w, u64 ws, u64 q, u64 q2) {
     x = x >= q2 ? x - q2 : x;
     u64 t = mul_shoup_lazy(y, w, ws, q);
@@ -111,9 +103,20 @@ __device__ __forceinline__ void gs_bfly(u64 &x, u64 &y, u64 w, u64 ws, u64 q, u6
     x = s >= q2 ? s - q2 : s;
     y = mul_shoup_lazy(d, w, ws, q);
 }
-// four Cooley-Tukey stages on 16 register values; twiddle j = (1 << s) - 1 + g of local stage s, group g, at tp[j * STRIDE]
-template <int STRIDE> __device__ __forceinline__ void fwd16_int(u64 (&v)[16], const ulonglong2 *__restrict__ tp, u64 q) {
-    const u64 q2 = q << 1;
+struct IntConst {
+    u64 q, nq, q4, q8;
+    u32 sh;
+};
+__device__ __forceinline__ IntConst int_const(const PrimeConst &m) {
+    IntConst c;
+    c.q = m.q; c.nq = 0ull - m.q; c.q4 = m.q << 2; c.q8 = m.q << 3; c.sh = m.fold_shift;
+    return c;
+}
+// Four Cooley-Tukey stages on 16 register values; twiddle j = (1 << s) - 1 + g of local stage s, group g, at tp[j * STRIDE].
+// Products are below 4q (mul_shoup4), so a stage adds 4q to the bound B of the values; x is folded below ~2^b before the
+// additions of the stages named by the bit mask FOLD.  The words hold 16 q: in units of q the four rounds of a transform
+// (masks 8, 4, 2, 9) run 3-7-11-15|5, 5-9-13|5-9, 9-13|5-9-13, 13|5-9-13|5 (| = a fold).
+template <int STRIDE, int FOLD> __device__ __forceinline__ void fwd16_int(u64 (&v)[16], const ulonglong2 *__restrict__ tp, const IntConst &c) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         const int half = 8 >> s;
@@ -121,13 +124,20 @@ template <int STRIDE> __device__ __forceinline__ void fwd16_int(u64 (&v)[16], co
         for (int g = 0; g < (1 << s); ++g) {
             const ulonglong2 tw = __ldg(tp + ((1 << s) - 1 + g) * STRIDE);
 #pragma unroll
-            for (int j = 0; j < half; ++j) ct_bfly(v[g * 2 * half + j], v[g * 2 * half + j + half], tw.x, tw.y, q, q2);
+            for (int j = 0; j < half; ++j) {
+                u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
+                const u64 t = mul_shoup4(y, tw.x, tw.y, c.nq);
+                if ((FOLD >> s) & 1) x = fold_q(x, c.nq, c.sh);
+                y = x + c.q4 - t;
+                x = x + t;
+            }
         }
     }
 }
-// four Gentleman-Sande stages, the mirror image
-template <int STRIDE> __device__ __forceinline__ void inv16_int(u64 (&v)[16], const ulonglong2 *__restrict__ tp, u64 q) {
-    const u64 q2 = q << 1;
+constexpr int kFoldColsA = 8, kFoldColsB = 4, kFoldRowsA = 2, kFoldRowsB = 9;
+// Four Gentleman-Sande stages, the mirror image.  Values enter and leave below 4q: sums reach 8q, then 16q, and are folded at
+// every second stage.
+template <int STRIDE> __device__ __forceinline__ void inv16_int(u64 (&v)[16], const ulonglong2 *__restrict__ tp, const IntConst &c) {
 #pragma unroll
     for (int s = 3; s >= 0; --s) {
         const int half = 8 >> s;
@@ -135,31 +145,27 @@ template <int STRIDE> __device__ __forceinline__ void inv16_int(u64 (&v)[16], co
         for (int g = 0; g < (1 << s); ++g) {
             const ulonglong2 tw = __ldg(tp + ((1 << s) - 1 + g) * STRIDE);
 #pragma unroll
-            for (int j = 0; j < half; ++j) gs_bfly(v[g * 2 * half + j], v[g * 2 * half + j + half], tw.x, tw.y, q, q2);
+            for (int j = 0; j < half; ++j) {
+                u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
+                const u64 d = x + ((s & 1) ? c.q4 : c.q8) - y, a = x + y;
+                x = (s & 1) ? a : fold_q(a, c.nq, c.sh);
+                y = mul_shoup4(d, tw.x, tw.y, c.nq);
+            }
         }
     }
 }
 
 // ---------------- double-storage butterflies (primes below 2^44) ----------------
 constexpr double kMagic = 6755399441055744.0; // 2^52 + 2^51: adding it leaves a signed integer |v| < 2^51 in the low mantissa bits
-struct DsConst {
-    u64 nq;      // 2^64 - q
-    u64 q;
-    double coff; // 2^52 + q
-    double qd, qinv;
-};
+struct DsConst { double qd, qinv; };
 __device__ __forceinline__ DsConst ds_const(const PrimeConst &m) {
     DsConst c;
-    c.nq = 0ull - m.q; c.q = m.q; c.coff = kTwo52 + (double)m.q; c.qd = (double)m.q; c.qinv = m.q_inv_f;
+    c.qd = (double)m.q; c.qinv = m.q_inv_f;
     return c;
 }
 // canonical residue -> double, exact for values below 2^52
 __device__ __forceinline__ double ds_load(u64 a) { return u52_to_double(a); }
 // t = y * w mod q as a signed double in (-0.52 q, 0.52 q); y integer-valued, |y| < 2^49; wf = w / q
-#ifndef HB_DS_FP
-#define HB_DS_FP 1
-#endif
-#if HB_DS_FP
 // wbits = bits of the double w.  Six FP64 instructions, every one exact: p + e = y * w (product and its rounding error),
 // qh = rint(y * w / q) up to 0.02, p - qh * q is an integer below 2^45 and so is its sum with e.
 __device__ __forceinline__ double ds_mul(double y, u64 wbits, double wf, const DsConst &c) {
@@ -170,15 +176,6 @@ __device__ __forceinline__ double ds_mul(double y, u64 wbits, double wf, const D
     const double t1 = __fma_rn(-qh, c.qd, p);
     return __dadd_rn(t1, e);
 }
-#else
-__device__ __forceinline__ double ds_mul(double y, u64 w, double wf, const DsConst &c) {
-    const double qh = __fma_rn(y, wf, kMagic);
-    const double yb = __dadd_rn(y, kMagic);
-    const u64 r = mad2_lo64((u64)__double_as_longlong(yb), w, (u64)__double_as_longlong(qh), c.nq, c.q); // y*w - qh*q + q, exact in its low 48 bits
-    const u32 hi = ((u32)(r >> 32) & 0xFFFFu) | 0x43300000u;
-    return __hiloint2double((int)hi, (int)(u32)r) - c.coff;
-}
-#endif
 // the same with the quotient estimated from the rounded product instead of from a precomputed w / q (one operand less to
 // fetch; the estimate is off by less than 0.07, so the result lies within 0.57 q of zero)
 __device__ __forceinline__ double ds_mul_w(double y, double wd, const DsConst &c) {
@@ -189,15 +186,11 @@ __device__ __forceinline__ double ds_mul_w(double y, double wd, const DsConst &c
 }
 // the form of a twiddle w that ds_mul takes as its second operand
 __host__ __device__ __forceinline__ u64 ds_twiddle_word(u64 w) {
-#if HB_DS_FP
     const double d = (double)w; // exact below 2^53
 #ifdef __CUDA_ARCH__
     return (u64)__double_as_longlong(d);
 #else
     u64 b; memcpy(&b, &d, 8); return b;
-#endif
-#else
-    return w;
 #endif
 }
 // x - rint(x / q) * q, |result| <= 0.52 q
@@ -319,13 +312,14 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_cols(const u64 *__restr
         u64 v[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = p[(e * 16 + sub) * 256];
-        fwd16_int<1>(v, tab + Ntt16Layout::colsA(0), m.q);
+        const IntConst c = int_const(m);
+        fwd16_int<1, kFoldColsA>(v, tab + Ntt16Layout::colsA(0), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[(e * 16 + sub) * 16 + lane] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[(sub * 16 + e) * 16 + lane];
-        fwd16_int<1>(v, tab + Ntt16Layout::colsB(sub, 0), m.q);
+        fwd16_int<1, kFoldColsB>(v, tab + Ntt16Layout::colsB(sub, 0), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) o[(sub * 16 + e) * 256] = v[e];
     }
@@ -362,23 +356,19 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows(const u64 *__restr
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = ds_store(v[e], c, shift, qinv_up); // the words this thread read itself
     } else {
-        const u64 q = m.q, q2 = q << 1;
+        const IntConst c = int_const(m);
         u64 v[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = p[e * 16];
-        fwd16_int<1>(v, tab + Ntt16Layout::rowsA(row, 0), q);
+        fwd16_int<1, kFoldRowsA>(v, tab + Ntt16Layout::rowsA(row, 0), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
-        fwd16_int<16>(v, tab + Ntt16Layout::rowsB(row, 0, clo), q);
+        fwd16_int<16, kFoldRowsB>(v, tab + Ntt16Layout::rowsB(row, 0, clo), c);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            u64 x = v[e];
-            x = x >= q2 ? x - q2 : x;
-            smr[clo * 17 + e] = x >= q ? x - q : x;
-        }
+        for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = canon_q(v[e], c.q, c.sh);
     }
     __syncthreads();
 #pragma unroll
@@ -421,13 +411,14 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_rows(const u64 *__restr
         u64 v[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
-        inv16_int<16>(v, tab + Ntt16Layout::rowsB(row, 0, clo), m.q);
+        const IntConst c = int_const(m);
+        inv16_int<16>(v, tab + Ntt16Layout::rowsB(row, 0, clo), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[e * 17 + clo];
-        inv16_int<1>(v, tab + Ntt16Layout::rowsA(row, 0), m.q);
+        inv16_int<1>(v, tab + Ntt16Layout::rowsA(row, 0), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) o[e * 16] = v[e];
     }
@@ -436,10 +427,9 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_rows(const u64 *__restr
 // ---- inverse, column pass: undoes stages 8..1, scales by N^-1, stores canonical residues ----
 template <int MINB>
 __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *__restrict__ src, LimbAddr16 sa, u64 *__restrict__ dst, LimbAddr16 da,
-                                                        const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, Ntt16Tables tb,
-                                                        const __grid_constant__ Ntt16Scale sc) {
+                                                        const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     __shared__ u64 sm[4096];
-    const int li = blockIdx.y, pos = li % map.n, pi = map.prime[pos];
+    const int li = blockIdx.y, pi = map.prime[li % map.n];
     const PrimeConst m = pc[pi];
     const ulonglong2 *tab = tb.inv + (size_t)pi * Ntt16Layout::kEntries;
     const int tid = threadIdx.x, lane = tid & 15, sub = tid >> 4;
@@ -460,28 +450,26 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *__restr
         for (int e = 0; e < 16; ++e) v[e] = smd[(e * 16 + sub) * 16 + lane];
         inv16_ds<1>(v, tab + Ntt16Layout::colsA(0), c);
         const double qinv_up = c.qinv * (1.0 + 0x1p-50);
-        const u64 sw = sc.on ? sc.w[pos] : ds_twiddle_word(m.n_inv);
-        const double sf = sc.on ? __longlong_as_double((long long)sc.comp[pos]) : m.n_inv_f;
+        const u64 sw = ds_twiddle_word(m.n_inv);
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-            const double t = ds_mul(v[e], sw, sf, c); // x * N^-1 (or x * scale) in (-0.52 q, 0.52 q)
+            const double t = ds_mul(v[e], sw, m.n_inv_f, c); // x * N^-1 in (-0.52 q, 0.52 q)
             o[(e * 16 + sub) * 256] = ds_store(t, c, c.qd, qinv_up);
         }
     } else {
         u64 v[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = p[(sub * 16 + e) * 256];
-        inv16_int<1>(v, tab + Ntt16Layout::colsB(sub, 0), m.q);
+        const IntConst c = int_const(m);
+        inv16_int<1>(v, tab + Ntt16Layout::colsB(sub, 0), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[(sub * 16 + e) * 16 + lane] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[(e * 16 + sub) * 16 + lane];
-        inv16_int<1>(v, tab + Ntt16Layout::colsA(0), m.q);
+        inv16_int<1>(v, tab + Ntt16Layout::colsA(0), c);
 #pragma unroll
-        const u64 sw = sc.on ? sc.w[pos] : m.n_inv, ss = sc.on ? sc.comp[pos] : m.n_inv_sh;
-#pragma unroll
-        for (int e = 0; e < 16; ++e) o[(e * 16 + sub) * 256] = mul_shoup(v[e], sw, ss, m.q);
+        for (int e = 0; e < 16; ++e) o[(e * 16 + sub) * 256] = canon_q(mul_shoup4(v[e], m.n_inv, m.n_inv_sh, c.nq), c.q, c.sh);
     }
 }
 
@@ -490,7 +478,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *__restr
 // are compiled for (register budget 65536 / (256 * MINB)); four measured fastest with the FP64 butterflies.
 template <int MINB = 4>
 inline cudaError_t launch_ntt16(cudaStream_t st, const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int count, const LimbMap &map,
-                                const PrimeConst *pc, const Ntt16Tables &tb, bool inverse, const Ntt16Scale *scale = nullptr) {
+                                const PrimeConst *pc, const Ntt16Tables &tb, bool inverse) {
     if (count == 0) return cudaSuccess;
     LimbAddr16 sa{src_outer}, da{dst_outer};
     dim3 grid(16, count);
@@ -499,8 +487,7 @@ inline cudaError_t launch_ntt16(cudaStream_t st, const u64 *src, size_t src_oute
         ntt16v2_fwd_rows<MINB><<<grid, 256, 0, st>>>(dst, da, dst, da, map, pc, tb);
     } else {
         ntt16v2_inv_rows<MINB><<<grid, 256, 0, st>>>(src, sa, dst, da, map, pc, tb);
-        Ntt16Scale none{};
-        ntt16v2_inv_cols<MINB><<<grid, 256, 0, st>>>(dst, da, dst, da, map, pc, tb, scale ? *scale : none);
+        ntt16v2_inv_cols<MINB><<<grid, 256, 0, st>>>(dst, da, dst, da, map, pc, tb);
     }
     return cudaGetLastError();
 }
