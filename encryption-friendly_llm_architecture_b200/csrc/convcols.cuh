@@ -11,14 +11,17 @@
 // writes instead of 3 S + S + 3 T limb transfers, and one launch instead of three.  Measured at S = 4, T = 6 (the division by
 // P * q_l at level 6) and 336 polynomials: see the launcher.
 //
-// A CTA is two groups of COLS * 16 threads.  Sources are dealt to the groups, then (one CTA barrier later) targets; inside a
+// A CTA is G groups of COLS * 16 threads.  Sources are dealt to the groups, then (one CTA barrier later) targets; inside a
 // group a radix-16 round exchanges through shared memory behind a named barrier of that group only, so one group's loads,
 // barriers and exchanges overlap the other's arithmetic.  Source residues stay in shared memory as two 30-bit pieces per
 // word: products with 26-bit (or 30-bit) pieces of the constants are single 32 x 32 multiply-adds into 64-bit sums, on the
 // integer pipe, which the FP64 butterflies around them leave idle.
 #pragma once
 #include "modarith.cuh"
+#include "pdl.cuh"
+#include "kernels.cuh"
 #include "ntt16.cuh"
+#include <type_traits>
 
 namespace hb {
 
@@ -41,7 +44,7 @@ template <int THREADS> __device__ __forceinline__ void group_sync(int g) { asm v
 
 // Inverse column pass of one limb strip into the registers of a group: on return v[e] is row e * 16 + sub, times the scale, canonical.
 template <int COLS>
-__device__ __forceinline__ void strip_inverse(u64 (&v)[16], const u64 *__restrict__ p /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, u64 sw, u64 sc,
+__device__ __forceinline__ void strip_inverse(u64 (&v)[16], const u64 *p /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, u64 sw, u64 sc,
                                               int g, int sub, int lane) {
     using I = StripIndex<COLS>;
     if (m.small) {
@@ -50,13 +53,13 @@ __device__ __forceinline__ void strip_inverse(u64 (&v)[16], const u64 *__restric
         double d[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) d[e] = reinterpret_cast<const double *>(p)[(sub * 16 + e) * 256];
-        inv16_ds<1>(d, tab + Ntt16Layout::colsB(sub, 0), c);
+        inv16_ds(d, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[I::b(e, sub, lane)] = d[e];
         group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) d[e] = smd[I::a(e, sub, lane)];
-        inv16_ds<1>(d, tab + Ntt16Layout::colsA(0), c);
+        inv16_ds(d, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
         const double qinv_up = c.qinv * (1.0 + 0x1p-50), sf = __longlong_as_double((long long)sc);
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = ds_store(ds_mul(d[e], sw, sf, c), c, c.qd, qinv_up);
@@ -64,20 +67,20 @@ __device__ __forceinline__ void strip_inverse(u64 (&v)[16], const u64 *__restric
         const IntConst c = int_const(m);
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = p[(sub * 16 + e) * 256];
-        inv16_int<1>(v, tab + Ntt16Layout::colsB(sub, 0), c);
+        inv16_int(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[I::b(e, sub, lane)] = v[e];
         group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[I::a(e, sub, lane)];
-        inv16_int<1>(v, tab + Ntt16Layout::colsA(0), c);
+        inv16_int(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = canon_q(mul_shoup4(v[e], sw, sc, c.nq), c.q, c.sh);
     }
 }
 // Forward column pass of one limb strip: v[e] holds row e * 16 + sub (double bits below 2^44, |v| < 2q; otherwise words below 4q).
 template <int COLS>
-__device__ __forceinline__ void strip_forward(u64 (&v)[16], u64 *__restrict__ o /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, int g, int sub, int lane) {
+__device__ __forceinline__ void strip_forward(u64 (&v)[16], u64 *o /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, int g, int sub, int lane) {
     using I = StripIndex<COLS>;
     if (m.small) {
         const DsConst c = ds_const(m);
@@ -85,26 +88,26 @@ __device__ __forceinline__ void strip_forward(u64 (&v)[16], u64 *__restrict__ o 
         double d[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) d[e] = __longlong_as_double((long long)v[e]);
-        fwd16_ds<1>(d, tab + Ntt16Layout::colsA(0), c);
+        fwd16_ds(d, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
         group_sync<COLS * 16>(g); // the strip of the previous target has been read
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[I::a(e, sub, lane)] = d[e];
         group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) d[e] = smd[I::b(e, sub, lane)];
-        fwd16_ds<1>(d, tab + Ntt16Layout::colsB(sub, 0), c);
+        fwd16_ds(d, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) reinterpret_cast<double *>(o)[(sub * 16 + e) * 256] = d[e];
     } else {
         const IntConst c = int_const(m);
-        fwd16_int<1, kFoldColsA>(v, tab + Ntt16Layout::colsA(0), c);
+        fwd16_int<kFoldColsA>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
         group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[I::a(e, sub, lane)] = v[e];
         group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[I::b(e, sub, lane)];
-        fwd16_int<1, kFoldColsB>(v, tab + Ntt16Layout::colsB(sub, 0), c);
+        fwd16_int<kFoldColsB>(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) o[(sub * 16 + e) * 256] = v[e];
     }
@@ -190,21 +193,21 @@ __device__ __forceinline__ void convert_target(u64 (&v)[16], const u64 *ysm, con
 }
 
 // src: half-inverse limbs (after the inverse row pass), instance b at src + b * src_outer; dst: half-forward limbs.
-// grid = (256 / COLS, plans * split, instances): a CTA takes every split-th target of its plan (small batches: more CTAs,
-// each repeating the source passes).  Dynamic shared memory: (largest ns + 2) strips.
-template <int COLS>
-__global__ void __launch_bounds__(COLS * 32, 512 / (COLS * 32)) conv_cols(const u64 *__restrict__ src, size_t src_outer, u64 *__restrict__ dst, size_t dst_outer, const ConvPlan *__restrict__ plans, int split,
+// grid = (256 / COLS, plans, instances).  Dynamic shared memory: (largest ns + G) strips.
+template <int COLS, int G>
+__global__ void __launch_bounds__(COLS * 16 * G, 512 / (COLS * 16 * G)) conv_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, const ConvPlan *__restrict__ plans,
                                                                          const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     extern __shared__ __align__(16) u64 strips[];
     using I = StripIndex<COLS>;
-    const ConvPlan *pl = plans + blockIdx.y / split;
-    const int part = blockIdx.y % split, ns = pl->ns, nt = pl->nt;
+    const ConvPlan *pl = plans + blockIdx.y;
+    const int ns = pl->ns, nt = pl->nt;
     const int g = threadIdx.x / (COLS * 16), r = threadIdx.x % (COLS * 16), lane = r % COLS, sub = r / COLS;
     const int col = blockIdx.x * COLS + lane;
     const u64 *sp = src + (size_t)blockIdx.z * src_outer + (size_t)pl->src_limb * kN16 + col;
     u64 *dp = dst + (size_t)blockIdx.z * dst_outer + (size_t)pl->dst_limb * kN16 + col;
     u64 v[16];
-    for (int s = g; s < ns; s += 2) {
+    pdl_wait();
+    for (int s = g; s < ns; s += G) {
         const int pi = pl->src_prime[s];
         u64 *sm = strips + s * I::kWords;
         strip_inverse<COLS>(v, sp + (size_t)s * kN16, sm, pc[pi], tb.inv + (size_t)pi * Ntt16Layout::kEntries, pl->scale_w[s], pl->scale_c[s], g, sub, lane);
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(COLS * 32, 512 / (COLS * 32)) conv_cols(const 
     }
     __syncthreads();
     u64 *ex = strips + (ns + g) * I::kWords;
-    for (int t = part * 2 + g; t < nt; t += 2 * split) {
+    for (int t = g; t < nt; t += G) {
         const int pi = pl->dst_prime[t];
         const PrimeConst m = pc[pi];
         const uint4 *cst = pl->c[t];
@@ -229,9 +232,9 @@ __global__ void __launch_bounds__(COLS * 32, 512 / (COLS * 32)) conv_cols(const 
 }
 
 // Rescale: one source limb (prime index `level`), lifted centred to the limbs 0 .. level - 1.
-// grid = (256 / COLS, split, instances); dynamic shared memory: three strips.
-template <int COLS>
-__global__ void __launch_bounds__(COLS * 32, 512 / (COLS * 32)) lift_cols(const u64 *__restrict__ src, size_t src_outer, u64 *__restrict__ dst, size_t dst_outer, int level, int split,
+// grid = (256 / COLS, instances); dynamic shared memory: 1 + G strips.
+template <int COLS, int G>
+__global__ void __launch_bounds__(COLS * 16 * G, 512 / (COLS * 16 * G)) lift_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int level,
                                                                          const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     extern __shared__ __align__(16) u64 strips[];
     using I = StripIndex<COLS>;
@@ -240,16 +243,17 @@ __global__ void __launch_bounds__(COLS * 32, 512 / (COLS * 32)) lift_cols(const 
     const u64 ql = pc[level].q;
     const bool src_small = pc[level].small;
     u64 v[16];
+    pdl_wait();
     if (g == 0) {
         const PrimeConst m = pc[level];
         const u64 sw = m.small ? ds_twiddle_word(m.n_inv) : m.n_inv, sc = m.small ? (u64)__double_as_longlong(m.n_inv_f) : m.n_inv_sh;
-        strip_inverse<COLS>(v, src + (size_t)blockIdx.z * src_outer + col, strips, m, tb.inv + (size_t)level * Ntt16Layout::kEntries, sw, sc, g, sub, lane);
+        strip_inverse<COLS>(v, src + (size_t)blockIdx.y * src_outer + col, strips, m, tb.inv + (size_t)level * Ntt16Layout::kEntries, sw, sc, g, sub, lane);
 #pragma unroll
         for (int e = 0; e < 16; ++e) strips[I::a(e, sub, lane)] = v[e] > (ql >> 1) ? v[e] - ql : v[e]; // signed
     }
     __syncthreads();
-    u64 *dp = dst + (size_t)blockIdx.z * dst_outer + col, *ex = strips + (1 + g) * I::kWords;
-    for (int t = blockIdx.y * 2 + g; t < level; t += 2 * split) {
+    u64 *dp = dst + (size_t)blockIdx.y * dst_outer + col, *ex = strips + (1 + g) * I::kWords;
+    for (int t = g; t < level; t += G) {
         const PrimeConst m = pc[t];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
@@ -264,20 +268,19 @@ __global__ void __launch_bounds__(COLS * 32, 512 / (COLS * 32)) lift_cols(const 
 }
 
 // ---- forward row pass with the last step of a division ----
-//   out[b][p][l] = (x[b][p][l] - t[b][p][l]) * inv_l  (+ add_p[b][l] o perm_g)
+//   out[b][p][l] = (x[b][p][l] - t[b][p][l]) * inv_l  (+ add_p[b][l] o perm_g, ADD: addends and g of the member's group)
 // t arrives half-forward (conv_cols / lift_cols).  grid = (16, n, instances), instance bp = b * np + p.  The operands of the last
 // step are read after the barrier of the final exchange, when the registers of the transform are free.
 struct RowsFin {
     const u64 *x; size_t x_outer;            // instance stride of x; limb l at l * N
-    const u64 *add[3]; size_t add_outer;     // per polynomial, ciphertext stride; null: nothing to add
-    u32 g;                                   // Galois element of the addends, 0: none
     u64 *out; size_t out_outer;              // ciphertext stride; polynomial p at p * n * N
-    int np;
+    int np, batch; size_t add_outer;         // ciphertexts per group, ciphertext stride of the addends
 };
 struct InvScale { u64 w[kMaxPrimes], c[kMaxPrimes]; }; // per limb: (ds_twiddle_word, w / q as a double) below 2^44, (w, Shoup companion) otherwise
-template <int MINB>
-__global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *__restrict__ t, size_t t_outer, const __grid_constant__ RowsFin f, const __grid_constant__ InvScale sc, const PrimeConst *__restrict__ pc,
-                                                            Ntt16Tables tb) {
+struct NoAddends {};
+template <int MINB, class ADD /* SwitchList or NoAddends */>
+__global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, size_t t_outer, const __grid_constant__ RowsFin f, const __grid_constant__ InvScale sc, const __grid_constant__ ADD add,
+                                                            const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     __shared__ u64 sm[16 * kRowStride];
     const int l = blockIdx.y, bp = blockIdx.z, b = bp / f.np, p = bp % f.np, n = gridDim.y;
     const PrimeConst m = pc[l];
@@ -287,7 +290,13 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *__r
     const size_t pos = (size_t)row * 256 + clo, limb = (size_t)l * kN16;
     const u64 *tp = t + (size_t)bp * t_outer + limb + pos;
     const u64 *xp = f.x + (size_t)bp * f.x_outer + limb + pos;
-    const u64 *ap = f.add[p] ? f.add[p] + (size_t)b * f.add_outer + limb : nullptr;
+    const u64 *ap = nullptr;
+    u32 g = 0;
+    if constexpr (!std::is_same_v<ADD, NoAddends>) {
+        const SwitchGroup &sg = add.s[b / f.batch];
+        g = sg.g;
+        if (sg.add[p]) ap = sg.add[p] + (size_t)(b % f.batch) * f.add_outer + limb;
+    }
     u64 *o = f.out + (size_t)b * f.out_outer + ((size_t)p * n + l) * kN16 + pos;
     u64 *smr = sm + rl * kRowStride;
     if (m.small) {
@@ -295,15 +304,17 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *__r
         const double *td = reinterpret_cast<const double *>(tp);
         double *smd = reinterpret_cast<double *>(smr);
         double v[16];
+        const TwiddlesB<double, MINB <= 2> tw(tb.fwdB8 + (size_t)l * kRowsB8 + (row * 15) * 16 + clo);
+        pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = td[e * 16];
-        fwd16_ds<1>(v, tab + Ntt16Layout::rowsA(row, 0), c);
+        fwd16_ds(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[e * 17 + clo] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smd[clo * 17 + e];
-        fwd16_ds8<16>(v, tb.fwdB8 + (size_t)l * kRowsB8 + (row * 15) * 16 + clo, c);
+        fwd16_ds8(v, tw, c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[clo * 17 + e] = v[e]; // the words this thread read itself
         u64 x[16];
@@ -315,21 +326,23 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *__r
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
             double r = ds_mul(ds_load(x[e]) - smd[e * 17 + clo], sw, sf, c); // within 0.52 q of zero
-            if (ap) r += ds_load(ap[f.g ? ntt_perm((u32)(pos + e * 16), f.g, 16) : (u32)(pos + e * 16)]);
+            if (ap) r += ds_load(ap[g ? ntt_perm((u32)(pos + e * 16), g, 16) : (u32)(pos + e * 16)]);
             o[e * 16] = ds_store(r, c, c.qd, qinv_up);
         }
     } else {
         const IntConst c = int_const(m);
         u64 v[16];
+        const TwiddlesB<ulonglong2, MINB <= 2> tw(tab + Ntt16Layout::rowsB(row, 0, clo));
+        pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = tp[e * 16];
-        fwd16_int<1, kFoldRowsA>(v, tab + Ntt16Layout::rowsA(row, 0), c);
+        fwd16_int<kFoldRowsA>(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
-        fwd16_int<16, kFoldRowsB>(v, tab + Ntt16Layout::rowsB(row, 0, clo), c); // below 5q
+        fwd16_int<kFoldRowsB>(v, tw, c); // below 5q
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = v[e];
         u64 x[16];
@@ -340,21 +353,24 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *__r
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
             u64 r = mul_shoup4(x[e] + c.q8 - smr[e * 17 + clo], sw, ss, c.nq); // below 4q
-            if (ap) r += ap[f.g ? ntt_perm((u32)(pos + e * 16), f.g, 16) : (u32)(pos + e * 16)];
+            if (ap) r += ap[g ? ntt_perm((u32)(pos + e * 16), g, 16) : (u32)(pos + e * 16)];
             o[e * 16] = canon_q(r, c.q, c.sh);
         }
     }
 }
 
-// single passes, for the fused sequences
+// Single passes, for the fused sequences.  A grid of one or two CTAs per SM takes the kernels that may use 128 registers and
+// fetch the twiddles of the second round (which nobody shares) before anything else, under the tail of the predecessor.
+constexpr int kSmallGrid = 2 * 148;
 inline void launch_inv_rows16(cudaStream_t st, const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
-    ntt16v2_inv_rows<4><<<dim3(16, count), 256, 0, st>>>(src, LimbAddr16{src_outer}, dst, LimbAddr16{dst_outer}, map, pc, tb);
+    launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_inv_rows<2> : ntt16v2_inv_rows<4>, dim3(16, count), 256, 0, src, LimbAddr16{src_outer}, dst, LimbAddr16{dst_outer}, map, pc, tb);
 }
 inline void launch_fwd_rows16(cudaStream_t st, u64 *d, size_t outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
-    ntt16v2_fwd_rows<4><<<dim3(16, count), 256, 0, st>>>(d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb);
+    launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_fwd_rows<2> : ntt16v2_fwd_rows<4>, dim3(16, count), 256, 0, d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb);
 }
-inline void launch_fwd_rows_fin16(cudaStream_t st, const u64 *t, size_t t_outer, int n, int instances, const RowsFin &f, const InvScale &sc, const PrimeConst *pc, const Ntt16Tables &tb) {
-    ntt16v2_fwd_rows_fin<4><<<dim3(16, n, instances), 256, 0, st>>>(t, t_outer, f, sc, pc, tb);
+template <class ADD>
+inline void launch_fwd_rows_fin16(cudaStream_t st, const u64 *t, size_t t_outer, int n, int instances, const RowsFin &f, const InvScale &sc, const ADD &add, const PrimeConst *pc, const Ntt16Tables &tb) {
+    launch_pdl(st, 16 * n * instances <= kSmallGrid ? ntt16v2_fwd_rows_fin<2, ADD> : ntt16v2_fwd_rows_fin<4, ADD>, dim3(16, n, instances), 256, 0, t, t_outer, f, sc, add, pc, tb);
 }
 
 } // namespace hb

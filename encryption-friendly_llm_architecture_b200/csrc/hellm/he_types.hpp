@@ -5,6 +5,7 @@
 #pragma once
 #include "hemmer_b200.h"
 
+#include <algorithm>
 #include <complex>
 #include <cstdint>
 #include <memory>
@@ -156,6 +157,49 @@ class Evaluator {
         check(c_, hb_gen_rot_keys(c_, &steps, 1));
         hb_ct *o = nullptr; check(c_, hb_rotate_hoisted(c_, a.raw(), h.raw(), steps, &o)); return Ciphertext(c_, o);
     }
+    // all rotations of one ciphertext by `steps` in one launch sequence: member k * batch + b = rotation k of member b
+    Ciphertext leftRotateMulti(const Ciphertext &a, const Hoisted &h, const std::vector<i64> &steps) const {
+        check(c_, hb_gen_rot_keys(c_, steps.data(), (int)steps.size()));
+        hb_ct *o = nullptr; check(c_, hb_rotate_hoisted_multi(c_, a.raw(), h.raw(), steps.data(), (int)steps.size(), &o)); return Ciphertext(c_, o);
+    }
+    // member group k of x rotated by steps[k], one launch sequence
+    Ciphertext leftRotateGroups(const Ciphertext &x, const std::vector<i64> &steps) const {
+        check(c_, hb_gen_rot_keys(c_, steps.data(), (int)steps.size()));
+        hb_ct *o = nullptr; check(c_, hb_rotate_grouped(c_, x.raw(), steps.data(), (int)steps.size(), &o)); return Ciphertext(c_, o);
+    }
+    // member group k of `groups`, without a copy; x must stay alive
+    Ciphertext group(const Ciphertext &x, int k, int groups) const {
+        const int b = x.getBatch() / groups;
+        hb_ct *o = nullptr; check(c_, hb_batch_view(c_, x.raw(), k * b, b, &o)); return Ciphertext(c_, o);
+    }
+    Ciphertext copyGroup(const Ciphertext &x, int k, int groups) const {
+        const int b = x.getBatch() / groups;
+        hb_ct *o = nullptr; check(c_, hb_batch_slice(c_, x.raw(), k * b, b, &o)); return Ciphertext(c_, o);
+    }
+    Ciphertext view(const Ciphertext &x, int start, int count) const { hb_ct *o = nullptr; check(c_, hb_batch_view(c_, x.raw(), start, count, &o)); return Ciphertext(c_, o); }
+    // sum of the member groups of x
+    Ciphertext sumGroups(const Ciphertext &x, int groups) const {
+        std::vector<Ciphertext> v;
+        std::vector<const hb_ct *> raw;
+        for (int k = 0; k < groups; ++k) { v.push_back(group(x, k, groups)); raw.push_back(v.back().raw()); }
+        hb_ct *o = nullptr; check(c_, hb_sum_mod_reduce(c_, raw.data(), std::min(groups, 16), &o));
+        Ciphertext r(c_, o);
+        for (int k = 16; k < groups; ++k) r = add(r, v[(size_t)k]);
+        return r;
+    }
+    // sum k = rescale(sum_j x_{k * count + j} (.) p[k * count + j]) over the member groups x_i of x; sums member groups
+    Ciphertext multSumGrouped(const Ciphertext &x, const std::vector<const Plaintext *> &p, int count, int sums) const {
+        std::vector<const hb_pt *> rp;
+        for (auto *q : p) rp.push_back(q->raw());
+        hb_ct *o = nullptr; check(c_, hb_sum_mul_pt_rescale_grouped(c_, x.raw(), rp.data(), count, sums, &o)); return Ciphertext(c_, o);
+    }
+    // acc += tensor(first half of x's members, second half)
+    void tensorAccumulateHalves(Ciphertext &acc, const Ciphertext &x) const {
+        hb_ct *p = acc.release();
+        int rc = hb_tensor_acc_halves(c_, x.raw(), &p);
+        acc = Ciphertext(c_, p);
+        check(c_, rc);
+    }
     // sum_t leftRotate(x[t], steps[t]) with one ModDown for the whole sum
     Ciphertext rotateSum(const std::vector<Ciphertext> &x, const std::vector<i64> &steps) const {
         check(c_, hb_gen_rot_keys(c_, steps.data(), (int)steps.size()));
@@ -220,12 +264,13 @@ class Evaluator {
     // all giant-step parts of a baby-step / giant-step transform in one pass over the shared terms:
     // part g = rescale(sum_j multWithoutRescale(a[j], p[g][j])), null entries skipped; members part-major in the result
     static constexpr size_t kMaxPartTerms = 17, kMaxParts = 17;
-    Ciphertext multSumRescaledOnceParts(const std::vector<const Ciphertext *> &a, const std::vector<std::vector<const Plaintext *>> &p) const {
+    // (each: every product is rescaled on its own before the sum, the residues of multSum)
+    Ciphertext multSumParts(const std::vector<const Ciphertext *> &a, const std::vector<std::vector<const Plaintext *>> &p, bool each) const {
         std::vector<const hb_ct *> ra; std::vector<const hb_pt *> rp;
         for (auto *x : a) ra.push_back(x->raw());
         for (const auto &row : p)
             for (size_t j = 0; j < a.size(); ++j) rp.push_back(j < row.size() && row[j] ? row[j]->raw() : nullptr);
-        hb_ct *o = nullptr; check(c_, hb_mul_pt_sum_parts(c_, ra.data(), rp.data(), (int)ra.size(), (int)p.size(), &o)); return Ciphertext(c_, o);
+        hb_ct *o = nullptr; check(c_, (each ? hb_mul_pt_sum_parts_each : hb_mul_pt_sum_parts)(c_, ra.data(), rp.data(), (int)ra.size(), (int)p.size(), &o)); return Ciphertext(c_, o);
     }
     // sum_t leftRotate(member group t of x, steps[t]) with one lift of the digits and one ModDown
     Ciphertext rotateSumGrouped(const Ciphertext &x, const std::vector<i64> &steps) const {

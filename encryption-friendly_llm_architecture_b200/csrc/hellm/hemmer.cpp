@@ -162,38 +162,42 @@ void HEMMer::transposeComplexPackingInplace(CtxtTensor &t, int target_level) {
     transposeInplace(t, 0);
 }
 void HEMMer::complexPackingRowInplace(CtxtTensor &t) { t.get() = fold_odd(*this, t.get(), kRowEven, t.getBlockWidth(), true, true); }
-// HEMMer::oneMatRotSumInplace -- HEMMer.cpp:882-919 with ModelArgs::HEAD_DIM equal to the tile side
-void HEMMer::oneMatRotSumInplace(CtxtTensor &a, CtxtTensor &b) {
-    const i64 d = tile_;
-    for (i64 rot = 1; rot < d / 2; rot <<= 1) {
-        a.get() = eval_.add(a.get(), eval_.leftRotate(a.get(), rot));
-        b.get() = eval_.add(b.get(), eval_.rightRotate(b.get(), rot));
-    }
-    a.get() = eval_.mult(a.get(), hemmer_mask(*this, kFirstCol, a.getLevel()));
-    b.get() = eval_.mult(b.get(), hemmer_mask(*this, kLastCol, b.getLevel()));
-    for (i64 rot = 1; rot < d; rot <<= 1) {
-        a.get() = eval_.add(a.get(), eval_.rightRotate(a.get(), rot));
-        b.get() = eval_.add(b.get(), eval_.leftRotate(b.get(), rot));
-    }
+// The rotate-and-add row sums of oneMatRotSumInplace / trOneMatRotSumInplace on the member groups of x: a group of direction +1 sums
+// to the left over `in_end` columns, keeps the first column and spreads it to the right over `out_end`; a group of direction -1
+// does the mirror image with the last column.
+static Ciphertext row_sums(HEMMer &h, Ciphertext x, const std::vector<int> &dir, i64 in_end, i64 out_end) {
+    const Evaluator &ev = h.eval();
+    auto steps = [&](i64 rot) { std::vector<i64> s; for (int d : dir) s.push_back(d * rot); return s; };
+    for (i64 rot = 1; rot < in_end; rot <<= 1) x = ev.add(x, ev.leftRotateGroups(x, steps(rot)));
+    std::vector<const Plaintext *> masks;
+    for (int d : dir) masks.push_back(&hemmer_mask(h, d > 0 ? kFirstCol : kLastCol, x.getLevel()));
+    x = ev.multSumGrouped(x, masks, 1, (int)dir.size());
+    for (i64 rot = 1; rot < out_end; rot <<= 1) x = ev.add(x, ev.leftRotateGroups(x, steps(-rot)));
+    return x;
 }
+static void row_sums_pair(HEMMer &h, CtxtTensor &a, CtxtTensor &b, i64 in_end, i64 out_end) {
+    const Evaluator &ev = h.eval();
+    if (a.getLevel() != b.getLevel() || a.get().getBatch() != b.get().getBatch()) {
+        a.get() = row_sums(h, std::move(a.get()), {1}, in_end, out_end);
+        b.get() = row_sums(h, std::move(b.get()), {-1}, in_end, out_end);
+        return;
+    }
+    std::vector<Ciphertext> two;
+    two.push_back(std::move(a.get())); two.push_back(std::move(b.get()));
+    const Ciphertext x = row_sums(h, ev.concat(two), {1, -1}, in_end, out_end);
+    a.get() = ev.copyGroup(x, 0, 2);
+    b.get() = ev.copyGroup(x, 1, 2);
+}
+// HEMMer::oneMatRotSumInplace -- HEMMer.cpp:882-919 with ModelArgs::HEAD_DIM equal to the tile side
+void HEMMer::oneMatRotSumInplace(CtxtTensor &a, CtxtTensor &b) { row_sums_pair(*this, a, b, tile_ / 2, tile_); }
 // HEMMer::tr_oneMatRotSumInplace -- HEMMer.cpp:921-962 with ModelArgs::HEAD_DIM equal to the tile side: the sums run over a
 // whole row of a tile and come back on half of it (a: left half, b: right half), after an optional level-down
 void HEMMer::trOneMatRotSumInplace(CtxtTensor &a, CtxtTensor &b, int target_level) {
-    const i64 d = tile_;
     if (target_level > 0) {
         a.get() = eval_.levelDown(a.get(), target_level + 1);
         b.get() = eval_.levelDown(b.get(), target_level + 1);
     }
-    for (i64 rot = 1; rot < d; rot <<= 1) {
-        a.get() = eval_.add(a.get(), eval_.leftRotate(a.get(), rot));
-        b.get() = eval_.add(b.get(), eval_.rightRotate(b.get(), rot));
-    }
-    a.get() = eval_.mult(a.get(), hemmer_mask(*this, kFirstCol, a.getLevel()));
-    b.get() = eval_.mult(b.get(), hemmer_mask(*this, kLastCol, b.getLevel()));
-    for (i64 rot = 1; rot < d / 2; rot <<= 1) {
-        a.get() = eval_.add(a.get(), eval_.rightRotate(a.get(), rot));
-        b.get() = eval_.add(b.get(), eval_.leftRotate(b.get(), rot));
-    }
+    row_sums_pair(*this, a, b, tile_, tile_ / 2);
 }
 // HEMMer::maskFirstRowInplace / maskFirstColOnlyInplace -- HEMMer.cpp:1255-1261, masks :2384-2388, :2418
 void HEMMer::maskFirstRowInplace(CtxtTensor &t) { t.get() = eval_.mult(t.get(), hemmer_mask(*this, kFirstRow, t.getLevel())); }
@@ -222,30 +226,35 @@ void HEMMer::maskRightLeft(const CtxtTensor &t, CtxtTensor &left, CtxtTensor &ri
     left = CtxtTensor(t.getShape(), eval_.mult(t.get(), hemmer_mask(*this, kHeadLeft, t.getLevel())));
     right = CtxtTensor(t.getShape(), eval_.mult(t.get(), hemmer_mask(*this, kHeadRight, t.getLevel())));
 }
-// Gaussian-kernel score assembly -- TransformerBlock.cpp:2420-2482 (one query / key pair; the reference loops over three)
+// Gaussian-kernel score assembly -- TransformerBlock.cpp:2420-2482 (one query / key pair; the reference loops over three).  The two heads
+// go through the same operations, so they travel as the two member groups [left | right] of one ciphertext.
 std::vector<CtxtTensor> HEMMer::gaussianKernelScores(const CtxtTensor &query, const CtxtTensor &key, int target_level) {
-    std::vector<CtxtTensor> mq(2), mk(2);
-    maskRightLeft(query, mq[0], mq[1]);
-    maskRightLeft(key, mk[0], mk[1]);
-    std::vector<CtxtTensor> oq, ok;
-    for (int j = 0; j < 2; ++j) {
-        oq.emplace_back(query.getShape(), eval_.square(mq[(size_t)j].get()));
-        ok.emplace_back(key.getShape(), eval_.square(mk[(size_t)j].get()));
+    auto heads = [&](const CtxtTensor &t) { // maskRightLeft
+        return CtxtTensor(t.getShape(), eval_.multSumParts({&t.get()}, {{&hemmer_mask(*this, kHeadLeft, t.getLevel())}, {&hemmer_mask(*this, kHeadRight, t.getLevel())}}, false));
+    };
+    CtxtTensor mq = heads(query), mk = heads(key);
+    Ciphertext oq = eval_.square(mq.get()), ok = eval_.square(mk.get());
+    if (oq.getLevel() == ok.getLevel() && oq.getBatch() == ok.getBatch()) {
+        std::vector<Ciphertext> both;
+        both.push_back(std::move(oq)); both.push_back(std::move(ok));
+        const Ciphertext x = row_sums(*this, eval_.concat(both), {1, -1, 1, -1}, tile_ / 2, tile_);
+        oq = eval_.copyGroup(x, 0, 2);
+        ok = eval_.copyGroup(x, 1, 2);
+    } else {
+        oq = row_sums(*this, std::move(oq), {1, -1}, tile_ / 2, tile_);
+        ok = row_sums(*this, std::move(ok), {1, -1}, tile_ / 2, tile_);
     }
-    oneMatRotSumInplace(oq[0], oq[1]);
-    oneMatRotSumInplace(ok[0], ok[1]);
-    for (auto &t : ok) transposeInplace(t, target_level);
+    CtxtTensor okt(key.getShape(), std::move(ok));
+    transposeInplace(okt, target_level);
+    complexPackingInplace(mq);
+    transposeInplace(mk);
+    complexPackingRowInplace(mk);
+    CtxtTensor s = repackCC(packedMatMul(mq, mk, target_level));
+    s.get() = eval_.multInteger(s.get(), -2);
+    s.get() = eval_.add(s.get(), oq);
+    s.get() = eval_.add(s.get(), okt.get());
     std::vector<CtxtTensor> out;
-    for (size_t j = 0; j < 2; ++j) {
-        complexPackingInplace(mq[j]);
-        transposeInplace(mk[j]);
-        complexPackingRowInplace(mk[j]);
-        CtxtTensor s = repackCC(packedMatMul(mq[j], mk[j], target_level));
-        s.get() = eval_.multInteger(s.get(), -2);
-        s.get() = eval_.add(s.get(), oq[j].get());
-        s.get() = eval_.add(s.get(), ok[j].get());
-        out.push_back(std::move(s));
-    }
+    for (int j = 0; j < 2; ++j) out.emplace_back(s.getShape(), eval_.copyGroup(s.get(), j, 2));
     return out;
 }
 // the rank-2 LoRA branch of TransformerBlock::attention2_bert_loraOpti -- TransformerBlock.cpp:2199-2365

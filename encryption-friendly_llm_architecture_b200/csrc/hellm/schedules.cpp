@@ -10,6 +10,7 @@
 // mask-mask-add-rescale "assemble" step and the tensor accumulation are single fused launches.
 #include "schedules.hpp"
 
+#include <algorithm>
 #include <cmath>
 #include <functional>
 
@@ -101,6 +102,36 @@ Message diag_family_mask(const Env &e, const TileTensorShape &s, const DiagFamil
     return m.rotated_right(idx > 0 ? rot_num : rot_num - main * f.gap);
 }
 
+// Iterations of a shift loop handled by one launch sequence: batches are stacked until about 168 ciphertexts are in
+// flight.  A batch of 40 fills the GPU on its own; beyond that the gain is the accumulator of the product loop, which is
+// read and written once per launch sequence instead of once per iteration.  The stored residues do not depend on the grouping.
+i64 loop_group(const Ciphertext &x) { return std::max<i64>(1, std::min<i64>(16, 168 / std::max(1, x.getBatch()))); }
+
+// Rotations of x by all `steps` (sharing its decomposition), several per launch sequence: one ciphertext has work for a fraction of
+// the GPU.  The rotations are handed out as views of the batches that hold them.
+struct Rotations { std::vector<Ciphertext> stacks, each; };
+Rotations rotate_all(Env &e, const Ciphertext &x, const Hoisted &h, const std::vector<i64> &steps) {
+    Rotations r;
+    const size_t group = (size_t)loop_group(x);
+    for (size_t k = 0; k < steps.size(); k += group) {
+        const std::vector<i64> some(steps.begin() + (std::ptrdiff_t)k, steps.begin() + (std::ptrdiff_t)std::min(steps.size(), k + group));
+        r.stacks.push_back(e.ev.leftRotateMulti(x, h, some));
+        for (size_t j = 0; j < some.size(); ++j) r.each.push_back(e.ev.group(r.stacks.back(), (int)j, (int)some.size()));
+    }
+    return r;
+}
+// The masked sums of a baby-step / giant-step transform, all parts at once, rotated by their giant steps and added up: in kLazy the
+// sums are rescaled once and share a ModDown, otherwise every product is rescaled and every rotation is complete (the
+// residues of the reference's order of operations; sums modulo q do not depend on the order).
+bool parts_fit(const Env &e, size_t terms, size_t parts, int batch) {
+    if (terms > Evaluator::kMaxPartTerms || parts > Evaluator::kMaxParts) return false;
+    return e.mode == kLazy || terms * parts * (size_t)batch * 2 <= 4096; // one limb per product of the unlazy form: at most 2 GB of them
+}
+Ciphertext giant_steps(Env &e, const std::vector<const Ciphertext *> &terms, const std::vector<std::vector<const Plaintext *>> &rows, const std::vector<i64> &steps) {
+    if (e.mode == kLazy) return e.ev.rotateSumGrouped(e.ev.multSumParts(terms, rows, false), steps);
+    return e.ev.sumGroups(e.ev.leftRotateGroups(e.ev.multSumParts(terms, rows, true), steps), (int)steps.size());
+}
+
 // Baby-step / giant-step evaluation shared by diagonalToColumn (MatrixUtils.cpp:776-848), diagonalToRow
 // (:924-996), packedDiagonalToColumn (:850-922) and packedDiagonalToRow (:998-1070).
 Ciphertext bsgs_diagonals(Env &e, const Ciphertext &op, const TileTensorShape &s, bool vertical, bool packed) {
@@ -108,18 +139,18 @@ Ciphertext bsgs_diagonals(Env &e, const Ciphertext &op, const TileTensorShape &s
     const int kind = packed ? (vertical ? kPackedVertical : kPackedHorizontal) : (vertical ? kVertical : kHorizontal);
     const int level = op.getLevel();
     auto mask = [&](i64 idx) -> const Plaintext & { return cached(e, kind, s, idx, level, [&] { return diag_family_mask(e, s, f, idx); }); };
-    std::vector<Ciphertext> baby;
-    baby.reserve((size_t)f.bs);
+    Rotations rot;
+    std::vector<Ciphertext> &baby = rot.each;
     if (e.mode >= kDirect) {
-        const Hoisted h = e.ev.decompose(op);
-        for (i64 j = 0; j < f.bs; ++j) baby.push_back(e.ev.leftRotate(op, h, (j + 1) * f.gap));
+        std::vector<i64> steps;
+        for (i64 j = 0; j < f.bs; ++j) steps.push_back((j + 1) * f.gap);
+        rot = rotate_all(e, op, e.ev.decompose(op), steps);
     } else {
         baby.push_back(e.ev.leftRotate(op, f.gap));
         for (i64 j = 1; j < f.bs; ++j) baby.push_back(e.ev.leftRotate(baby.back(), f.gap));
     }
-    // kLazy: the parts and their giant steps are collected and rotated by ONE call that shares the ModDown; when they
-    // fit its limits, all parts are also formed by one pass over the baby steps (terms: op, baby[0], baby[1], ...)
-    if (e.mode == kLazy && (size_t)f.bs + 1 <= Evaluator::kMaxPartTerms && (size_t)(2 * f.gs + 1) <= Evaluator::kMaxParts) {
+    // all parts by one pass over the baby steps (terms: op, baby[0], baby[1], ...) when they fit its limits
+    if (parts_fit(e, (size_t)f.bs + 1, (size_t)(2 * f.gs + 1), op.getBatch())) {
         std::vector<const Ciphertext *> terms{&op};
         for (i64 j = 0; j < f.bs; ++j) terms.push_back(&baby[(size_t)j]);
         std::vector<std::vector<const Plaintext *>> rows;
@@ -140,7 +171,7 @@ Ciphertext bsgs_diagonals(Env &e, const Ciphertext &op, const TileTensorShape &s
                 steps.push_back(sign < 0 ? -(f.main * f.gap - rot_num) : rot_num);
             }
         }
-        return e.ev.rotateSumGrouped(e.ev.multSumRescaledOnceParts(terms, rows), steps);
+        return giant_steps(e, terms, rows, steps);
     }
     std::vector<Ciphertext> parts; std::vector<i64> part_steps;
     Ciphertext res = e.ev.mult(op, mask(0));
@@ -218,10 +249,49 @@ Ciphertext assemble_lazy(Env &e, const Ciphertext &x, const Hoisted &h, const st
     for (const auto &c : w) { ka.push_back(c.main); kb.push_back(c.wrapped); }
     return e.ev.assembleRotationsMulti(x, h, ka, kb);
 }
-// Iterations of a shift loop handled by one launch sequence: batches are stacked until about 168 ciphertexts are in
-// flight.  A batch of 40 fills the GPU on its own; beyond that the gain is the accumulator of the product loop, which is
-// read and written once per launch sequence instead of once per iteration.  The stored residues do not depend on the grouping.
-i64 loop_group(const Ciphertext &x) { return std::max<i64>(1, std::min<i64>(16, 168 / std::max(1, x.getBatch()))); }
+// ---- shift loops of the other two schedules ----
+// Copies first .. first + count - 1 of one operand in kDirect: rescale(wrap[2i+1] (.) rot(x, step_i) + wrap[2i] (.) rot(x, wrapped_i)), all
+// rotations and all sums of the group in one launch sequence each; group-major batch.
+using Steps = std::function<std::pair<i64, i64>(i64)>;
+using Wraps = std::function<const Plaintext &(i64)>;
+Ciphertext direct_copies(Env &e, const Ciphertext &x, const Hoisted &h, i64 first, i64 count, const Steps &steps, const Wraps &wrap) {
+    std::vector<i64> s;
+    std::vector<const Plaintext *> m;
+    for (i64 i = first; i < first + count; ++i) {
+        const auto st = steps(i);
+        s.push_back(st.first); s.push_back(st.second);
+        m.push_back(&wrap(2 * i + 1)); m.push_back(&wrap(2 * i));
+    }
+    return e.ev.multSumGrouped(e.ev.leftRotateMulti(x, h, s), m, 2, (int)count);
+}
+// a group's 2 * count rotations and masked terms stay within 16 member groups per call
+i64 direct_group(const Ciphertext &x) { return std::max<i64>(1, std::min<i64>(8, loop_group(x) / 2)); }
+// In kFaithful every shifted copy is the previous one rotated once more: the chains of one loop (an operand and its wrapped copy,
+// of one or both operands) advance side by side as the member groups of one ciphertext.
+struct Chains {
+    Ciphertext x;
+    std::vector<i64> steps;
+    void advance(Env &e) { x = e.ev.leftRotateGroups(x, steps); }
+    int count() const { return (int)steps.size(); }
+};
+// operand k: groups 2k (rotated by step[k]) and 2k + 1 (that, rotated by -back[k])
+Chains start_chains(Env &e, const std::vector<const Ciphertext *> &ops, const std::vector<i64> &step, const std::vector<i64> &back) {
+    const int n = (int)ops.size();
+    auto stack = [&](std::vector<Ciphertext> v) { return e.ev.concat(v); };
+    std::vector<Ciphertext> in;
+    for (auto *o : ops) in.push_back(e.ev.view(*o, 0, o->getBatch()));
+    std::vector<i64> minus;
+    for (i64 b : back) minus.push_back(-b);
+    const Ciphertext main = e.ev.leftRotateGroups(stack(std::move(in)), step), wrapped = e.ev.leftRotateGroups(main, minus);
+    std::vector<Ciphertext> all;
+    Chains c;
+    for (int k = 0; k < n; ++k) {
+        all.push_back(e.ev.group(main, k, n)); all.push_back(e.ev.group(wrapped, k, n));
+        c.steps.push_back(step[(size_t)k]); c.steps.push_back(step[(size_t)k]);
+    }
+    c.x = stack(std::move(all));
+    return c;
+}
 
 void require_product_shapes(const CtxtTensor &a, const CtxtTensor &b) {
     if (a.getWidth() != b.getHeight()) throw std::invalid_argument("[getCommonInsideLength] different inside length.");
@@ -247,17 +317,18 @@ CtxtTensor transpose(Env &e, const CtxtTensor &op) {
             return m.rotated_right(i * bs * gap);
         });
     };
-    std::vector<Ciphertext> baby;
-    baby.reserve((size_t)bs);
+    Rotations rot;
+    std::vector<Ciphertext> &baby = rot.each;
     if (e.mode >= kDirect) {
-        const Hoisted h = e.ev.decompose(op.get());
-        for (i64 j = 0; j < bs; ++j) baby.push_back(e.ev.leftRotate(op.get(), h, (j - (num_rows - 1)) * gap));
+        std::vector<i64> steps;
+        for (i64 j = 0; j < bs; ++j) steps.push_back((j - (num_rows - 1)) * gap);
+        rot = rotate_all(e, op.get(), e.ev.decompose(op.get()), steps);
     } else {
         baby.push_back(e.ev.rightRotate(op.get(), (num_rows - 1) * gap));
         for (i64 j = 1; j < bs; ++j) baby.push_back(e.ev.leftRotate(baby.back(), gap));
     }
     Ciphertext res;
-    if (e.mode == kLazy && (size_t)bs <= Evaluator::kMaxPartTerms && (size_t)gs <= Evaluator::kMaxParts) { // all parts by one pass over the baby steps
+    if (parts_fit(e, (size_t)bs, (size_t)gs, op.get().getBatch())) { // all parts by one pass over the baby steps
         std::vector<const Ciphertext *> terms;
         for (i64 j = 0; j < bs; ++j) terms.push_back(&baby[(size_t)j]);
         std::vector<std::vector<const Plaintext *>> rows;
@@ -273,7 +344,7 @@ CtxtTensor transpose(Env &e, const CtxtTensor &op) {
             rows.push_back(std::move(row));
             steps.push_back(i * bs * gap);
         }
-        return CtxtTensor(s, e.ev.rotateSumGrouped(e.ev.multSumRescaledOnceParts(terms, rows), steps));
+        return CtxtTensor(s, giant_steps(e, terms, rows, steps));
     }
     std::vector<Ciphertext> parts; std::vector<i64> part_steps; // kLazy: all giant steps in one call
     for (i64 i = 0; i < gs; ++i) {
@@ -345,25 +416,18 @@ CtxtTensor ccmmCore(Env &e, Ciphertext a, Ciphertext b, i64 num_rows, i64 inner,
         }
     } else if (e.mode >= kDirect) {
         const Hoisted ha = e.ev.decompose(a), hb = e.ev.decompose(b);
-        for (i64 i = 1; i < num_k; ++i) {
-            Ciphertext ai = e.ev.leftRotate(a, ha, i), aw = e.ev.leftRotate(a, ha, i - cols_tmp);
-            Ciphertext bi = e.ev.leftRotate(b, hb, i * width), bw = e.ev.leftRotate(b, hb, (i - rows_tmp) * width);
-            Ciphertext ak = e.ev.assemble(ai, col_wrap(e, sa, 2 * i + 1, lvl), aw, col_wrap(e, sa, 2 * i, lvl));
-            Ciphertext bk = e.ev.assemble(bi, row_wrap(e, sb, 2 * i + 1, lvl), bw, row_wrap(e, sb, 2 * i, lvl));
-            e.ev.tensorAccumulate(acc, ak, bk);
+        const i64 group = direct_group(a);
+        for (i64 i0 = 1; i0 < num_k; i0 += group) {
+            const i64 count = std::min(num_k - i0, group);
+            Ciphertext ak = direct_copies(e, a, ha, i0, count, [&](i64 i) { return std::make_pair(i, i - cols_tmp); }, [&](i64 w) -> const Plaintext & { return col_wrap(e, sa, w, lvl); });
+            Ciphertext bk = direct_copies(e, b, hb, i0, count, [&](i64 i) { return std::make_pair(i * width, (i - rows_tmp) * width); }, [&](i64 w) -> const Plaintext & { return row_wrap(e, sb, w, lvl); });
+            e.ev.tensorAccumulateGroups(acc, ak, bk, (int)count);
         }
     } else {
-        a = e.ev.leftRotate(a, 1);
-        b = e.ev.leftRotate(b, width);
-        Ciphertext a_wrap = e.ev.rightRotate(a, cols_tmp), b_wrap = e.ev.rightRotate(b, rows_tmp * width);
+        Chains c = start_chains(e, {&a, &b}, {1, width}, {cols_tmp, rows_tmp * width});
         for (i64 i = 1; i < num_k; ++i) {
-            if (i > 1) {
-                a = e.ev.leftRotate(a, 1); a_wrap = e.ev.leftRotate(a_wrap, 1);
-                b = e.ev.leftRotate(b, width); b_wrap = e.ev.leftRotate(b_wrap, width);
-            }
-            Ciphertext ak = e.ev.assemble(a, col_wrap(e, sa, 2 * i + 1, lvl), a_wrap, col_wrap(e, sa, 2 * i, lvl));
-            Ciphertext bk = e.ev.assemble(b, row_wrap(e, sb, 2 * i + 1, lvl), b_wrap, row_wrap(e, sb, 2 * i, lvl));
-            e.ev.tensorAccumulate(acc, ak, bk);
+            if (i > 1) c.advance(e);
+            e.ev.tensorAccumulateHalves(acc, e.ev.multSumGrouped(c.x, {&col_wrap(e, sa, 2 * i + 1, lvl), &col_wrap(e, sa, 2 * i, lvl), &row_wrap(e, sb, 2 * i + 1, lvl), &row_wrap(e, sb, 2 * i, lvl)}, 2, 2));
         }
     }
     res = e.ev.add(res, e.ev.rescale(e.ev.relinearize(acc)));
@@ -398,17 +462,16 @@ CtxtTensor multMatMatCP(Env &e, const CtxtTensor &op1, const PtxtTensor &op2, in
     Plaintext b = e.ev.encode(tau, lvl);
     const i64 rows_tmp = num_k > num_rows ? num_k : ceil_pow2(num_rows), cols_tmp = num_k > num_cols ? num_k : ceil_pow2(num_cols);
     Ciphertext res = e.ev.mult(a, b);
-    a = e.ev.leftRotate(a, 1);
+    Chains c = start_chains(e, {&a}, {1}, {cols_tmp});
     b = e.ev.leftRotate(b, width);
-    Ciphertext a_wrap = e.ev.rightRotate(a, cols_tmp);
     Plaintext b_wrap = e.ev.leftRotate(b, -rows_tmp * width);
     Ciphertext acc;
     for (i64 i = 1; i < num_k; ++i) {
         if (i > 1) {
-            a = e.ev.leftRotate(a, 1); a_wrap = e.ev.leftRotate(a_wrap, 1);
+            c.advance(e);
             b = e.ev.leftRotate(b, width); b_wrap = e.ev.leftRotate(b_wrap, width);
         }
-        Ciphertext ak = e.ev.assemble(a, col_wrap(e, sa, 2 * i + 1, lvl), a_wrap, col_wrap(e, sa, 2 * i, lvl));
+        Ciphertext ak = e.ev.multSumGrouped(c.x, {&col_wrap(e, sa, 2 * i + 1, lvl), &col_wrap(e, sa, 2 * i, lvl)}, 2, 1);
         Plaintext bk = e.ev.add(e.ev.mult(b, row_wrap(e, sb, 2 * i + 1, lvl)), e.ev.mult(b_wrap, row_wrap(e, sb, 2 * i, lvl)));
         Ciphertext term = e.ev.mult(ak, bk);
         acc = acc.empty() ? std::move(term) : e.ev.add(acc, term);
@@ -431,23 +494,20 @@ CtxtTensor multPackedMatMat(Env &e, const CtxtTensor &op1, const CtxtTensor &op2
     Ciphertext acc;
     if (e.mode >= kDirect) {
         const Hoisted ha = e.ev.decompose(a), hb = e.ev.decompose(b);
-        for (i64 i = 1; i < num_k / 2; ++i) {
-            Ciphertext ai = e.ev.leftRotate(a, ha, 2 * i), aw = e.ev.leftRotate(a, ha, 2 * i - cols_tmp);
-            Ciphertext bi = e.ev.leftRotate(b, hb, 2 * i * width);
-            Ciphertext ak = e.ev.assemble(ai, col_wrap(e, sa, 4 * i + 1, lvl), aw, col_wrap(e, sa, 4 * i, lvl));
-            e.ev.tensorAccumulate(acc, ak, bi);
+        const i64 group = direct_group(a);
+        for (i64 i0 = 1; i0 < num_k / 2; i0 += group) {
+            const i64 count = std::min(num_k / 2 - i0, group);
+            std::vector<i64> bs;
+            for (i64 i = i0; i < i0 + count; ++i) bs.push_back(2 * i * width);
+            Ciphertext ak = direct_copies(e, a, ha, i0, count, [&](i64 i) { return std::make_pair(2 * i, 2 * i - cols_tmp); }, [&](i64 w) -> const Plaintext & { return col_wrap(e, sa, 2 * w - (w % 2), lvl); });
+            e.ev.tensorAccumulateGroups(acc, ak, e.ev.leftRotateMulti(b, hb, bs), (int)count);
         }
-    } else {
-        a = e.ev.leftRotate(a, 2);
+    } else { // b sits one level below a
+        Chains c = start_chains(e, {&a}, {2}, {cols_tmp});
         b = e.ev.leftRotate(b, 2 * width);
-        Ciphertext a_wrap = e.ev.rightRotate(a, cols_tmp);
         for (i64 i = 1; i < num_k / 2; ++i) {
-            if (i > 1) {
-                a = e.ev.leftRotate(a, 2); a_wrap = e.ev.leftRotate(a_wrap, 2);
-                b = e.ev.leftRotate(b, 2 * width);
-            }
-            Ciphertext ak = e.ev.assemble(a, col_wrap(e, sa, 4 * i + 1, lvl), a_wrap, col_wrap(e, sa, 4 * i, lvl));
-            e.ev.tensorAccumulate(acc, ak, b);
+            if (i > 1) { c.advance(e); b = e.ev.leftRotate(b, 2 * width); }
+            e.ev.tensorAccumulate(acc, e.ev.multSumGrouped(c.x, {&col_wrap(e, sa, 4 * i + 1, lvl), &col_wrap(e, sa, 4 * i, lvl)}, 2, 1), b);
         }
     }
     res = e.ev.add(res, e.ev.rescale(e.ev.relinearize(acc)));
@@ -463,19 +523,19 @@ Ciphertext multPackedMatMatPreRot(Env &e, const CtxtTensor &in, int target_level
     const int lvl = target_level + 2;
     std::vector<Ciphertext> copies;
     copies.push_back(e.ev.levelDownOne(in.get()));
+    const TileTensorShape shp = in.getShape();
     if (e.mode >= kDirect) {
         const Hoisted h = e.ev.decompose(in.get());
-        for (i64 i = 1; i < num_rows / 2; ++i) {
-            Ciphertext ai = e.ev.leftRotate(in.get(), h, 2 * i), aw = e.ev.leftRotate(in.get(), h, 2 * i - num_rows);
-            copies.push_back(e.ev.assemble(ai, col_wrap(e, in.getShape(), 4 * i + 1, lvl), aw, col_wrap(e, in.getShape(), 4 * i, lvl)));
-        }
-        return e.ev.stack(copies);
+        const i64 group = direct_group(in.get());
+        for (i64 i0 = 1; i0 < num_rows / 2; i0 += group)
+            copies.push_back(direct_copies(e, in.get(), h, i0, std::min(num_rows / 2 - i0, group), [&](i64 i) { return std::make_pair(2 * i, 2 * i - num_rows); },
+                                           [&](i64 w) -> const Plaintext & { return col_wrap(e, shp, 2 * w - (w % 2), lvl); }));
+        return e.ev.concat(copies);
     }
-    Ciphertext a = e.ev.leftRotate(in.get(), 2);
-    Ciphertext a_wrap = e.ev.rightRotate(a, num_rows);
+    Chains c = start_chains(e, {&in.get()}, {2}, {num_rows});
     for (i64 i = 1; i < num_rows / 2; ++i) {
-        if (i > 1) { a = e.ev.leftRotate(a, 2); a_wrap = e.ev.leftRotate(a_wrap, 2); }
-        copies.push_back(e.ev.assemble(a, col_wrap(e, in.getShape(), 4 * i + 1, lvl), a_wrap, col_wrap(e, in.getShape(), 4 * i, lvl)));
+        if (i > 1) c.advance(e);
+        copies.push_back(e.ev.multSumGrouped(c.x, {&col_wrap(e, shp, 4 * i + 1, lvl), &col_wrap(e, shp, 4 * i, lvl)}, 2, 1));
     }
     return e.ev.stack(copies);
 }
@@ -487,11 +547,21 @@ CtxtTensor multPackedMatMatPreRev(Env &e, const CtxtTensor &b, int target_level)
 CtxtTensor multPackedMatMatCCReuse(Env &e, const Ciphertext &pre, const CtxtTensor &tb) {
     const i64 width = tb.getBlockWidth();
     Ciphertext b = tb.get(), acc;
-    const int count = pre.getBatch();
-    const Hoisted h = e.mode >= kDirect ? e.ev.decompose(tb.get()) : Hoisted();
-    for (int i = 0; i < count; ++i) {
-        if (i > 0) b = e.mode >= kDirect ? e.ev.leftRotate(tb.get(), h, (i64)i * 2 * width) : e.ev.leftRotate(b, 2 * width);
-        e.ev.tensorAccumulate(acc, e.ev.slice(pre, i), b);
+    const int count = pre.getBatch() / tb.get().getBatch();
+    if (e.mode >= kDirect) {
+        const Hoisted h = e.ev.decompose(tb.get());
+        const i64 group = loop_group(tb.get());
+        for (i64 i0 = 0; i0 < count; i0 += group) {
+            std::vector<i64> steps;
+            for (i64 i = i0; i < std::min<i64>(count, i0 + group); ++i) steps.push_back(i * 2 * width);
+            const int bt = tb.get().getBatch(), n = (int)steps.size();
+            e.ev.tensorAccumulateGroups(acc, e.ev.view(pre, (int)i0 * bt, n * bt), e.ev.leftRotateMulti(tb.get(), h, steps), n);
+        }
+    } else {
+        for (int i = 0; i < count; ++i) {
+            if (i > 0) b = e.ev.leftRotate(b, 2 * width);
+            e.ev.tensorAccumulate(acc, e.ev.group(pre, i, count), b);
+        }
     }
     return CtxtTensor(tb.getShape(), e.ev.rescale(e.ev.relinearize(acc)));
 }
@@ -513,19 +583,19 @@ Ciphertext multMatMatPre(Env &e, const CtxtTensor &in, int target_level) {
         }
         return e.ev.concat(copies);
     }
+    const TileTensorShape shp = s.getShape();
     if (e.mode >= kDirect) {
         const Hoisted h = e.ev.decompose(s.get());
-        for (i64 i = 1; i < num_rows; ++i) {
-            Ciphertext ai = e.ev.leftRotate(s.get(), h, i), aw = e.ev.leftRotate(s.get(), h, i - num_rows);
-            copies.push_back(e.ev.assemble(ai, col_wrap(e, s.getShape(), 2 * i + 1, lvl), aw, col_wrap(e, s.getShape(), 2 * i, lvl)));
-        }
-        return e.ev.stack(copies);
+        const i64 group = direct_group(s.get());
+        for (i64 i0 = 1; i0 < num_rows; i0 += group)
+            copies.push_back(direct_copies(e, s.get(), h, i0, std::min(num_rows - i0, group), [&](i64 i) { return std::make_pair(i, i - num_rows); },
+                                           [&](i64 w) -> const Plaintext & { return col_wrap(e, shp, w, lvl); }));
+        return e.ev.concat(copies);
     }
-    Ciphertext a = e.ev.leftRotate(s.get(), 1);
-    Ciphertext a_wrap = e.ev.rightRotate(a, num_rows);
+    Chains c = start_chains(e, {&s.get()}, {1}, {num_rows});
     for (i64 i = 1; i < num_rows; ++i) {
-        if (i > 1) { a = e.ev.leftRotate(a, 1); a_wrap = e.ev.leftRotate(a_wrap, 1); }
-        copies.push_back(e.ev.assemble(a, col_wrap(e, s.getShape(), 2 * i + 1, lvl), a_wrap, col_wrap(e, s.getShape(), 2 * i, lvl)));
+        if (i > 1) c.advance(e);
+        copies.push_back(e.ev.multSumGrouped(c.x, {&col_wrap(e, shp, 2 * i + 1, lvl), &col_wrap(e, shp, 2 * i, lvl)}, 2, 1));
     }
     return e.ev.stack(copies);
 }
@@ -542,11 +612,21 @@ CtxtTensor multMatMatPreRev(Env &e, const CtxtTensor &b, int target_level) {
 CtxtTensor multMatMatCCReUse(Env &e, const Ciphertext &pre, const CtxtTensor &tb) {
     const i64 width = tb.getBlockWidth();
     Ciphertext b = tb.get(), acc;
-    const int count = pre.getBatch();
-    const Hoisted h = e.mode >= kDirect ? e.ev.decompose(tb.get()) : Hoisted();
-    for (int i = 0; i < count; ++i) {
-        if (i > 0) b = e.mode >= kDirect ? e.ev.leftRotate(tb.get(), h, (i64)i * width) : e.ev.leftRotate(b, width);
-        e.ev.tensorAccumulate(acc, e.ev.slice(pre, i), b);
+    const int count = pre.getBatch() / tb.get().getBatch();
+    if (e.mode >= kDirect) {
+        const Hoisted h = e.ev.decompose(tb.get());
+        const i64 group = loop_group(tb.get());
+        for (i64 i0 = 0; i0 < count; i0 += group) {
+            std::vector<i64> steps;
+            for (i64 i = i0; i < std::min<i64>(count, i0 + group); ++i) steps.push_back(i * width);
+            const int bt = tb.get().getBatch(), n = (int)steps.size();
+            e.ev.tensorAccumulateGroups(acc, e.ev.view(pre, (int)i0 * bt, n * bt), e.ev.leftRotateMulti(tb.get(), h, steps), n);
+        }
+    } else {
+        for (int i = 0; i < count; ++i) {
+            if (i > 0) b = e.ev.leftRotate(b, width);
+            e.ev.tensorAccumulate(acc, e.ev.group(pre, i, count), b);
+        }
     }
     return CtxtTensor(tb.getShape(), e.ev.relinearize(acc));
 }
@@ -575,18 +655,11 @@ CtxtTensor low_rank_tail(Env &e, Ciphertext a, Ciphertext b, const TileTensorSha
     const i64 num_rows = s1.getNumRows();
     Ciphertext res = e.ev.mult(a, b);
     if (low_dim > 1) {
-        a = e.ev.leftRotate(a, 1);
-        b = e.ev.leftRotate(b, width);
-        Ciphertext a_wrap = e.ev.rightRotate(a, width / 2), b_wrap = e.ev.rightRotate(b, num_rows * width);
+        Chains c = start_chains(e, {&a, &b}, {1, width}, {width / 2, num_rows * width});
         Ciphertext acc;
         for (i64 i = 1; i < low_dim; ++i) {
-            if (i > 1) {
-                a = e.ev.leftRotate(a, 1); a_wrap = e.ev.leftRotate(a_wrap, 1);
-                b = e.ev.leftRotate(b, width); b_wrap = e.ev.leftRotate(b_wrap, width);
-            }
-            Ciphertext ak = e.ev.assemble(a, col_wrap(e, s1, 2 * i + 1, lvl), a_wrap, col_wrap(e, s1, 2 * i, lvl));
-            Ciphertext bk = e.ev.assemble(b, row_wrap(e, s2, 2 * i + 1, lvl), b_wrap, row_wrap(e, s2, 2 * i, lvl));
-            e.ev.tensorAccumulate(acc, ak, bk);
+            if (i > 1) c.advance(e);
+            e.ev.tensorAccumulateHalves(acc, e.ev.multSumGrouped(c.x, {&col_wrap(e, s1, 2 * i + 1, lvl), &col_wrap(e, s1, 2 * i, lvl), &row_wrap(e, s2, 2 * i + 1, lvl), &row_wrap(e, s2, 2 * i, lvl)}, 2, 2));
         }
         res = e.ev.add(res, e.ev.rescale(e.ev.relinearize(acc)));
     }

@@ -147,7 +147,7 @@ struct hb_ctx {
 
 #define LAUNCH(c) ((c)->launches++, 0)
 #define ALG(c, limbs) ((c)->alg_limbs += (unsigned long long)(limbs))
-struct hb_ct { hb_ctx *ctx; int level, np, batch, spow; u64 *d; size_t limbs() const { return (size_t)batch * np * (level + 1); } };
+struct hb_ct { hb_ctx *ctx; int level, np, batch, spow; u64 *d; bool borrowed = false; /* a view: the buffer belongs to another handle */ size_t limbs() const { return (size_t)batch * np * (level + 1); } };
 struct hb_pt { hb_ctx *ctx; int level, spow; u64 *d; int ext = 0; }; // ext: K further limbs modulo the special primes follow the level+1 limbs
 // lifted digits of the a-part of a ciphertext batch, NTT form: what all rotations of that ciphertext share
 struct hb_digits { hb_ctx *ctx; int level, batch; u64 *d; };
@@ -331,37 +331,34 @@ const ConvPlan *get_conv_plans(hb_ctx *c, int level) {
 template <int COLS> size_t strip_bytes(int strips) { return (size_t)strips * StripIndex<COLS>::kWords * 8; }
 void conv_opt_in(hb_ctx *c) {
     if (c->smem_opt_in_conv) return;
-    CK(cudaFuncSetAttribute(conv_cols<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_bytes<8>(10)));
-    CK(cudaFuncSetAttribute(conv_cols<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_bytes<4>(10)));
-    CK(cudaFuncSetAttribute(lift_cols<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_bytes<8>(3)));
-    CK(cudaFuncSetAttribute(lift_cols<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_bytes<4>(3)));
+    auto allow = [](auto *kernel, size_t bytes) { CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); };
+    allow(conv_cols<8, 2>, strip_bytes<8>(10)); allow(conv_cols<4, 4>, strip_bytes<4>(12)); allow(conv_cols<4, 8>, strip_bytes<4>(16));
+    allow(lift_cols<8, 2>, strip_bytes<8>(3)); allow(lift_cols<4, 4>, strip_bytes<4>(5)); allow(lift_cols<4, 8>, strip_bytes<4>(9));
     c->smem_opt_in_conv = true;
 }
-// strip width and target split of a launch
-struct StripShape { int cols, split; };
-StripShape strip_shape(int instances, int targets) {
-    StripShape s{8, 1};
-    if (instances * 32 < 296) {
-        s.cols = 4;
-        while (s.split < 4 && instances * 64 * s.split * 2 <= 296 && targets > 2 * s.split) ++s.split;
-    }
-    if (const char *e = getenv("HB_COLS")) s.cols = atoi(e);
-    if (const char *e = getenv("HB_SPLIT")) s.split = atoi(e);
-    return s;
+// Strip width and groups of a launch over `units` (polynomial, conversion) pairs: wide strips when they fill the GPU; otherwise narrow
+// ones with more groups, so that more sources and targets of a unit are worked on at once.
+enum StripShape { kStrip8x2, kStrip4x4, kStrip4x8 };
+StripShape strip_shape(int units) {
+    return units * 64 <= 148 ? kStrip4x8 : units * 64 <= 2 * 148 ? kStrip4x4 : kStrip8x2;
 }
-// `plans` conversions (the largest with max_ns sources and max_nt targets) of `instances` polynomials in one launch
-void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int max_nt, int instances) {
+// `plans` conversions (the largest with max_ns sources) of `instances` polynomials in one launch
+void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int instances) {
     conv_opt_in(c);
-    const StripShape s = strip_shape(instances * count, max_nt);
-    if (s.cols == 8) LAUNCH(c), conv_cols<8><<<dim3(32, count * s.split, instances), 256, strip_bytes<8>(max_ns + 2), c->st>>>(src, so, dst, dof, plans, s.split, c->pc, c->tb.t16);
-    else LAUNCH(c), conv_cols<4><<<dim3(64, count * s.split, instances), 128, strip_bytes<4>(max_ns + 2), c->st>>>(src, so, dst, dof, plans, s.split, c->pc, c->tb.t16);
+    LAUNCH(c);
+    const StripShape s = strip_shape(instances * count);
+    if (s == kStrip8x2) launch_pdl(c->st, conv_cols<8, 2>, dim3(32, count, instances), 256, strip_bytes<8>(max_ns + 2), src, so, dst, dof, plans, c->pc, c->tb.t16);
+    else if (s == kStrip4x4) launch_pdl(c->st, conv_cols<4, 4>, dim3(64, count, instances), 256, strip_bytes<4>(max_ns + 4), src, so, dst, dof, plans, c->pc, c->tb.t16);
+    else launch_pdl(c->st, conv_cols<4, 8>, dim3(64, count, instances), 512, strip_bytes<4>(max_ns + 8), src, so, dst, dof, plans, c->pc, c->tb.t16);
 }
 // half-inverse limbs of prime `level` (one per instance) -> half-forward lifts to the limbs below
 void launch_lift(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int level, int instances) {
     conv_opt_in(c);
-    const StripShape s = strip_shape(instances, level);
-    if (s.cols == 8) LAUNCH(c), lift_cols<8><<<dim3(32, s.split, instances), 256, strip_bytes<8>(3), c->st>>>(src, so, dst, dof, level, s.split, c->pc, c->tb.t16);
-    else LAUNCH(c), lift_cols<4><<<dim3(64, s.split, instances), 128, strip_bytes<4>(3), c->st>>>(src, so, dst, dof, level, s.split, c->pc, c->tb.t16);
+    LAUNCH(c);
+    const StripShape s = strip_shape(instances);
+    if (s == kStrip8x2) launch_pdl(c->st, lift_cols<8, 2>, dim3(32, instances), 256, strip_bytes<8>(3), src, so, dst, dof, level, c->pc, c->tb.t16);
+    else if (s == kStrip4x4) launch_pdl(c->st, lift_cols<4, 4>, dim3(64, instances), 256, strip_bytes<4>(5), src, so, dst, dof, level, c->pc, c->tb.t16);
+    else launch_pdl(c->st, lift_cols<4, 8>, dim3(64, instances), 512, strip_bytes<4>(9), src, so, dst, dof, level, c->pc, c->tb.t16);
 }
 void inv_rows(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int count, const LimbMap &m) {
     LAUNCH(c), launch_inv_rows16(c->st, src, so, dst, dof, count, m, c->pc, c->tb.t16);
@@ -403,7 +400,7 @@ void ks_decompose(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch,
     Tmp acoef(c, (size_t)batch * n);
     if (c->logn == 16) {
         inv_rows(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level));
-        launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.ne - 1, batch);
+        launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), batch);
         fwd_rows(c, dt, (size_t)d.dt_count * N, batch * d.dt_count, d.dtmap);
         return;
     }
@@ -412,7 +409,8 @@ void ks_decompose(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch,
     ntt_inplace(c, dt, batch * d.dt_count, d.dtmap, false);
 }
 // ModDown of acc [batch*2][ne][N] into out: conversion of the special limbs, forward transform, final combination
-void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int batch, u64 *out, size_t out_outer, const u64 *add0, const u64 *add1, size_t add_outer, u32 g) {
+// (`total` members; addends per group of sl, `batch` members each)
+void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, size_t out_outer, const SwitchList &sl, int batch, size_t add_outer) {
     const KsPlan *pl = get_plan(c, level);
     const PlanDims d = plan_dims(c, level);
     const int N = c->N, n = d.n, ne = d.ne, K = d.K;
@@ -421,32 +419,30 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int batch, u64 *out, siz
     if (c->logn == 16) { // the special limbs are transformed in place
         const ConvPlan *cv = get_conv_plans(c, level);
         u64 *sp = acc + (size_t)n * N;
-        inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, batch * 2 * K, pm);
-        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, n, batch * 2);
-        const RowsFin f{acc, (size_t)ne * N, {add0, add1}, add_outer, g, out, out_outer, 2};
-        LAUNCH(c), launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, batch * 2, f, c->p_inv_scale, c->pc, c->tb.t16);
+        inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, total * 2 * K, pm);
+        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, total * 2);
+        const RowsFin f{acc, (size_t)ne * N, out, out_outer, 2, batch, add_outer};
+        LAUNCH(c), launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, total * 2, f, c->p_inv_scale, sl, c->pc, c->tb.t16);
         CK(cudaGetLastError());
         return;
     }
-    Tmp pcob(c, (size_t)batch * 2 * K);
+    Tmp pcob(c, (size_t)total * 2 * K);
     u64 *pco = pcob.p;
-    ntt(c, acc + (size_t)n * N, (size_t)ne * N, pco, (size_t)K * N, batch * 2 * K, pm, true);
-    LAUNCH(c), k_moddown_conv<<<dim3(gx1, 1, batch * 2), 256, 0, c->st>>>(tbuf, pco, pl, c->pc, c->L + 1, N);
-    ntt_inplace(c, tbuf, batch * 2 * n, c->qmap(level), false);
-    LAUNCH(c), k_moddown_fin<<<dim3(gx, n, batch * 2), 256, 0, c->st>>>(out, out_outer, acc, tbuf, add0, add1, add_outer, pl, c->pc, g, c->logn, N);
+    ntt(c, acc + (size_t)n * N, (size_t)ne * N, pco, (size_t)K * N, total * 2 * K, pm, true);
+    LAUNCH(c), k_moddown_conv<<<dim3(gx1, 1, total * 2), 256, 0, c->st>>>(tbuf, pco, pl, c->pc, c->L + 1, N);
+    ntt_inplace(c, tbuf, total * 2 * n, c->qmap(level), false);
+    LAUNCH(c), k_moddown_fin<<<dim3(gx, n, total * 2), 256, 0, c->st>>>(out, out_outer, acc, tbuf, sl, batch, add_outer, pl, c->pc, c->logn, N);
     CK(cudaGetLastError());
 }
-// Phase 2: inner product of the (permuted) digits with the key over Q_level u P, then ModDown:
-//   out[b][p][l] = ModDown(sum_dg perm_g(digit_dg) (.) key_dg)[p][l] + add_p[b][l] o perm_g
-void ks_apply(hb_ctx *c, const u64 *a, size_t a_outer, const u64 *dt, int level, int batch, const Evk &key, u32 g, u64 *out, size_t out_outer, const u64 *add0,
-              const u64 *add1, size_t add_outer) {
+// Phase 2: inner products of the (permuted) digits with the keys over Q_level u P, then ModDown, for every group of `sl`:
+//   out[ob][p][l] = ModDown(sum_dg perm_g(digit_dg) (.) key_dg)[p][l] + add_p[b][l] o perm_g,   ob = group * batch + b
+void ks_apply(hb_ctx *c, const SwitchList &sl, size_t a_outer, int level, int batch, u64 *out, size_t out_outer, size_t add_outer) {
     const KsPlan *pl = get_plan(c, level);
     const PlanDims d = plan_dims(c, level);
-    const int N = c->N, n = d.n, ne = d.ne;
-    const unsigned gx = c->gx();
-    Tmp acc(c, (size_t)batch * 2 * ne), t(c, (size_t)batch * 2 * n);
-    LAUNCH(c), k_ks_inner<<<dim3(gx, batch, ne), 256, 0, c->st>>>(acc.p, a, a_outer, dt, key.d, c->nprimes, pl, c->pc, g, c->logn, N);
-    moddown(c, acc.p, t.p, level, batch, out, out_outer, add0, add1, add_outer, g);
+    const int N = c->N, n = d.n, ne = d.ne, total = sl.count * batch;
+    Tmp acc(c, (size_t)total * 2 * ne), t(c, (size_t)total * 2 * n);
+    LAUNCH(c), launch_pdl(c->st, k_ks_inner, dim3(c->gx(), total, ne), 256, 0, acc.p, sl, batch, a_outer, c->nprimes, pl, c->pc, c->logn, N);
+    moddown(c, acc.p, t.p, level, total, out, out_outer, sl, batch, add_outer);
 }
 // Hybrid key switch of polynomial a (NTT form, `n` limbs, per-batch stride a_outer) with key `key`
 void keyswitch(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch, const Evk &key, u32 g, u64 *out, size_t out_outer, const u64 *add0, const u64 *add1,
@@ -454,7 +450,10 @@ void keyswitch(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch, co
     const PlanDims d = plan_dims(c, level);
     Tmp dt(c, (size_t)batch * d.dt_count);
     ks_decompose(c, a, a_outer, level, batch, dt.p);
-    ks_apply(c, a, a_outer, dt.p, level, batch, key, g, out, out_outer, add0, add1, add_outer);
+    SwitchList sl{};
+    sl.count = 1;
+    sl.s[0] = SwitchGroup{a, dt.p, key.d, {add0, add1}, g, 0u};
+    ks_apply(c, sl, a_outer, level, batch, out, out_outer, add_outer);
 }
 
 // Galois elements of the row shifts k * row_step, k < copies, kept on the device per (copies, row_step): the fused
@@ -565,9 +564,9 @@ hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch) {
         if (c->logn == 16) {
             const ConvPlan *cv = get_conv_plans(c, level);
             inv_rows(c, src, (size_t)ne * N, src, (size_t)ne * N, batch * 2 * ns, sm);
-            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, level, batch * 2);
-            const RowsFin f{E, (size_t)ne * N, {nullptr, nullptr}, 0, 0u, r->d, (size_t)2 * level * N, 2};
-            LAUNCH(c), launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], c->pc, c->tb.t16);
+            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, batch * 2);
+            const RowsFin f{E, (size_t)ne * N, r->d, (size_t)2 * level * N, 2, 1, 0};
+            LAUNCH(c), launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], NoAddends{}, c->pc, c->tb.t16);
             CK(cudaGetLastError());
             return r;
         }
@@ -665,8 +664,8 @@ void rescale_core(hb_ctx *c, const u64 *x, u64 *out, int l, int np, int nbp, u64
         for (int i = 0; i < l; ++i) scale_words(hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]), c->h->q[i], sc.w[i], sc.c[i]);
         inv_rows(c, x + (size_t)l * N, (size_t)(l + 1) * N, last, (size_t)N, nbp, lm);
         launch_lift(c, last, (size_t)N, t, (size_t)l * N, l, nbp);
-        const RowsFin f{x, (size_t)(l + 1) * N, {nullptr, nullptr, nullptr}, 0, 0u, out, (size_t)np * l * N, np};
-        LAUNCH(c), launch_fwd_rows_fin16(c->st, t, (size_t)l * N, l, nbp, f, sc, c->pc, c->tb.t16);
+        const RowsFin f{x, (size_t)(l + 1) * N, out, (size_t)np * l * N, np, 1, 0};
+        LAUNCH(c), launch_fwd_rows_fin16(c->st, t, (size_t)l * N, l, nbp, f, sc, NoAddends{}, c->pc, c->tb.t16);
     } else {
         ntt(c, x + (size_t)l * N, (size_t)(l + 1) * N, last, (size_t)N, nbp, lm, true);
         LAUNCH(c), k_rescale_prep<<<c->egrid(nbp * l), 256, 0, c->st>>>(t, last, l, c->pc, N);
@@ -690,51 +689,53 @@ hb_ct *do_rescale(hb_ctx *c, const hb_ct *a) {
     } catch (...) { hb_ct_free(r); throw; }
     return r;
 }
-// last [groups][nbp][N], residues modulo q_l in NTT form -> t [nbp][l][N], NTT form: the sum over the groups of the centred lifts
-void lift_last(hb_ctx *c, u64 *last, int groups, int nbp, int l, u64 *t) {
-    const int N = c->N;
+// last [sums][groups][nbp][N], residues modulo q_l in NTT form -> t [sums][nbp][l][N], NTT form: the sum over the groups of the centred lifts
+void lift_last(hb_ctx *c, u64 *last, int sums, int groups, int nbp, int l, u64 *t) {
+    const int N = c->N, total = sums * nbp;
     if (c->logn == 16 && groups == 1) {
-        inv_rows(c, last, (size_t)N, last, (size_t)N, nbp, one_limb(l));
-        launch_lift(c, last, (size_t)N, t, (size_t)l * N, l, nbp);
-        fwd_rows(c, t, (size_t)l * N, nbp * l, c->qmap(l - 1));
+        inv_rows(c, last, (size_t)N, last, (size_t)N, total, one_limb(l));
+        launch_lift(c, last, (size_t)N, t, (size_t)l * N, l, total);
+        fwd_rows(c, t, (size_t)l * N, total * l, c->qmap(l - 1));
         return;
     }
-    Tmp S(c, (size_t)nbp);
-    ntt_inplace(c, last, groups * nbp, one_limb(l), true);
-    LAUNCH(c), k_centre_sum<<<dim3(c->gx(), nbp), 256, 0, c->st>>>((i64 *)S.p, last, groups, nbp, l, c->pc, N);
-    LAUNCH(c), k_lift_mod<<<c->egrid(nbp * l), 256, 0, c->st>>>(t, (const i64 *)S.p, l, c->pc, N);
-    ntt_inplace(c, t, nbp * l, c->qmap(l - 1), false);
+    Tmp S(c, (size_t)total);
+    ntt_inplace(c, last, groups * total, one_limb(l), true);
+    LAUNCH(c), k_centre_sum<<<dim3(c->gx(), total), 256, 0, c->st>>>((i64 *)S.p, last, groups, nbp, l, c->pc, N);
+    LAUNCH(c), k_lift_mod<<<c->egrid(total * l), 256, 0, c->st>>>(t, (const i64 *)S.p, l, c->pc, N);
+    ntt_inplace(c, t, total * l, c->qmap(l - 1), false);
 }
-// sum_j rescale(a_j (.) p_j)  (separate)  or  rescale(sum_j a_j (.) p_j)
-hb_ct *do_prod_rescale(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, int count, bool separate) {
-    if (count < 1 || count > kMaxTerms) fail(HB_E_LIMIT, "product sum: between 1 and " + std::to_string(kMaxTerms) + " terms");
+// sum_j rescale(a_j (.) p_j)  (separate)  or  rescale(sum_j a_j (.) p_j); `sums` such sums of `count` terms each, sum k from the terms
+// k * count ..., one member group of the result per sum
+hb_ct *do_prod_rescale(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, int count, bool separate, int sums = 1) {
+    if (count < 1 || sums < 1 || count * sums > kMaxTerms) fail(HB_E_LIMIT, "product sum: between 1 and " + std::to_string(kMaxTerms) + " terms");
     const hb_ct *a0 = a[0];
     if (a0->level < 1) fail(HB_E_LEVEL, "rescale: level 0");
     TermList tl{}; tl.count = count;
-    for (int j = 0; j < count; ++j) {
+    for (int j = 0; j < count * sums; ++j) {
         if (a[j]->level != a0->level || p[j]->level != a0->level) fail(HB_E_LEVEL, "mul_pt: level mismatch");
         own(c, a[j]); own(c, p[j]);
         if (a[j]->np != a0->np || a[j]->batch != a0->batch) fail(HB_E_SHAPE, "product sum: shape mismatch");
         if (a[j]->spow != 1 || p[j]->spow != 1) fail(HB_E_SHAPE, "mul_pt: operand not rescaled");
         tl.a[j] = a[j]->d; tl.p[j] = p[j]->d;
     }
-    const int l = a0->level, N = c->N, nbp = a0->batch * a0->np, groups = separate ? count : 1;
+    const int l = a0->level, N = c->N, nbp = a0->batch * a0->np, total = sums * nbp, groups = separate ? count : 1;
     const unsigned gx = c->gx();
-    hb_ct *r = new_ct(c, l - 1, a0->np, a0->batch, 1);
-    ALG(c, (size_t)count * ((size_t)nbp * (l + 1) + (l + 1)) + (size_t)nbp * l);
+    hb_ct *r = new_ct(c, l - 1, a0->np, sums * a0->batch, 1);
+    ALG(c, (size_t)count * sums * ((size_t)nbp * (l + 1) + (l + 1)) + (size_t)total * l);
     try {
-        Tmp last(c, (size_t)groups * nbp), t(c, (size_t)nbp * l);
-        LAUNCH(c), k_last_prod<<<dim3(gx, nbp, groups), 256, 0, c->st>>>(last.p, tl, separate ? 1 : 0, l, nbp, c->pc, N);
-        lift_last(c, last.p, groups, nbp, l, t.p);
+        Tmp last(c, (size_t)groups * total), t(c, (size_t)total * l);
+        LAUNCH(c), launch_pdl(c->st, k_last_prod, dim3(gx, total, groups), 256, 0, last.p, tl, separate ? 1 : 0, l, nbp, c->pc, N);
+        lift_last(c, last.p, 1, groups, total, l, t.p);
         Scalars qi{};
         for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
-        LAUNCH(c), k_prod_rescale_fin<<<c->egrid(nbp * l), 256, 0, c->st>>>(r->d, tl, t.p, l, nbp, c->pc, N, qi);
+        LAUNCH(c), launch_pdl(c->st, k_prod_rescale_fin, c->egrid(total * l), 256, 0, r->d, tl, t.p, l, nbp, c->pc, N, qi);
         CK(cudaGetLastError());
     } catch (...) { hb_ct_free(r); throw; }
     return r;
 }
 // out_g = rescale(sum_j a_j (.) p[g * count + j]) for every part g in one pass over the a_j; out holds parts * batch members, part-major
-hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, int count, int parts) {
+// separate: every product is rescaled on its own, then the parts' products are added
+hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, int count, int parts, bool separate) {
     if (count < 1 || count > kMaxPartTerms || parts < 1 || parts > kMaxParts) fail(HB_E_LIMIT, "product sums: 1 to 17 terms, 1 to 17 parts");
     const hb_ct *a0 = a[0];
     if (!a0) fail(HB_E_ARG, "product sums: null ciphertext");
@@ -767,15 +768,16 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
     hb_ct *r = new_ct(c, l - 1, a0->np, parts * a0->batch, 1);
     ALG(c, (size_t)count * nbp * (l + 1) + used * (l + 1) + (size_t)gnbp * l);
     try {
-        Tmp last(c, (size_t)gnbp), t(c, (size_t)gnbp * l);
+        Tmp last(c, (size_t)gnbp * (separate ? count : 1)), t(c, (size_t)gnbp * l);
         constexpr int G = 6; // parts per CTA: 6 x 17 mask chunks of 2 KB = 204 KB of shared memory
         const size_t smem = (size_t)G * count * 2048;
         const unsigned pg = (unsigned)((parts + G - 1) / G);
         if (!c->smem_opt_in_parts) { CK(cudaFuncSetAttribute(k_prod_parts<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, G * kMaxPartTerms * 2048)); c->smem_opt_in_parts = true; }
         Scalars qi{};
         for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
-        LAUNCH(c), k_prod_parts<G><<<dim3(gx1, 1, pg), 1024, smem, c->st>>>(last.p, pt, nullptr, l, nbp, c->pc, N, qi, c->dev_err);
-        lift_last(c, last.p, 1, gnbp, l, t.p);
+        if (separate) LAUNCH(c), launch_pdl(c->st, k_last_prod_parts, dim3(c->gx(), nbp, parts * count), 256, 0, last.p, pt, l, nbp, c->pc, N);
+        else LAUNCH(c), k_prod_parts<G><<<dim3(gx1, 1, pg), 1024, smem, c->st>>>(last.p, pt, nullptr, l, nbp, c->pc, N, qi, c->dev_err);
+        lift_last(c, last.p, parts, separate ? count : 1, nbp, l, t.p);
         LAUNCH(c), k_prod_parts<G><<<dim3(gx1, (unsigned)l, pg), 1024, smem, c->st>>>(r->d, pt, t.p, l, nbp, c->pc, N, qi, c->dev_err);
         CK(cudaGetLastError());
     } catch (...) { hb_ct_free(r); throw; }
@@ -839,7 +841,7 @@ hb_ct *do_tensor(hb_ctx *c, const hb_ct *a, const hb_ct *b, hb_ct *acc, int grou
     else r = new_ct(c, a->level, 3, batch, 2);
     const int n = a->level + 1;
     ALG(c, 2 * a->limbs() + (size_t)(acc ? 2 : 1) * batch * 3 * n);
-    LAUNCH(c), k_tensor<<<c->egrid(batch * n), 256, 0, c->st>>>(r->d, a->d, b->d, n, c->qmap(a->level), c->pc, c->N, acc ? 1 : 0, groups, batch);
+    LAUNCH(c), launch_pdl(c->st, k_tensor, c->egrid(batch * n), 256, 0, r->d, (const u64 *)a->d, (const u64 *)b->d, n, c->qmap(a->level), c->pc, c->N, acc ? 1 : 0, groups, batch);
     return r;
 }
 hb_ct *do_relin(hb_ctx *c, const hb_ct *a) {
@@ -1333,7 +1335,7 @@ int hb_ct_clone(hb_ctx *c, const hb_ct *s, hb_ct **out) {
     });
 }
 int hb_ct_zero(hb_ctx *c, hb_ct *x) { return guard(c, [&] { own(c, x); CK(cudaMemsetAsync(x->d, 0, x->limbs() * c->N * 8, c->st)); }); }
-void hb_ct_free(hb_ct *x) { if (x) { x->ctx->pool.put(x->d); delete x; } }
+void hb_ct_free(hb_ct *x) { if (x) { if (!x->borrowed) x->ctx->pool.put(x->d); delete x; } }
 void hb_pt_free(hb_pt *x) { if (x) { x->ctx->pool.put(x->d); delete x; } }
 int hb_ct_meta(const hb_ct *x, int *level, int *np, int *batch, int *spow) {
     if (!x) return HB_E_ARG;
@@ -1385,6 +1387,13 @@ int hb_batch_concat(hb_ctx *c, const hb_ct *const *parts, int n, hb_ct **out) {
             off += words;
         }
         *out = r;
+    });
+}
+int hb_batch_view(hb_ctx *c, const hb_ct *src, int start, int count, hb_ct **out) {
+    return guard(c, [&] {
+        own(c, src);
+        if (start < 0 || count < 1 || start + count > src->batch) fail(HB_E_ARG, "batch_view: bad range");
+        *out = new hb_ct{c, src->level, src->np, count, src->spow, src->d + (size_t)start * src->np * (src->level + 1) * c->N, true};
     });
 }
 int hb_batch_slice(hb_ctx *c, const hb_ct *src, int start, int count, hb_ct **out) {
@@ -1507,20 +1516,51 @@ int hb_decompose(hb_ctx *c, const hb_ct *a, hb_digits **out) {
     });
 }
 void hb_digits_free(hb_digits *h) { if (h) { h->ctx->pool.put(h->d); delete h; } }
-int hb_rotate_hoisted(hb_ctx *c, const hb_ct *a, const hb_digits *dg, int64_t steps, hb_ct **out) {
+// rotations of `groups` member groups of x (group k = members k * batch ... ; shared: every group is the whole of x) by their own steps
+static hb_ct *rotate_groups(hb_ctx *c, const hb_ct *x, const u64 *dt, bool shared, const int64_t *steps, int groups) {
+    const int N = c->N, level = x->level, n = level + 1, batch = shared ? x->batch : x->batch / groups;
+    const size_t ct_outer = (size_t)2 * n * N, dt_count = (size_t)plan_dims(c, level).dt_count;
+    hb_ct *r = new_ct(c, level, 2, groups * batch, x->spow);
+    try {
+        for (int k0 = 0; k0 < groups;) { // runs of up to 16 rotated groups; an unrotated group is a copy
+            SwitchList sl{};
+            int k = k0;
+            for (; k < groups && sl.count < kMaxSwitchGroups; ++k) {
+                const u64 g = c->h->galois_rot(steps[k]);
+                if (g == 1) break;
+                const size_t first = shared ? 0 : (size_t)k * batch;
+                const u64 *a = x->d + first * ct_outer;
+                sl.s[sl.count++] = SwitchGroup{a + (size_t)n * N, dt + first * dt_count * N, galois_key(c, g).d, {a, nullptr}, (u32)g, 0u};
+            }
+            ALG(c, (size_t)sl.count * ((size_t)batch * (4 * n + dt_count) + key_limbs(c, level)));
+            if (sl.count) ks_apply(c, sl, ct_outer, level, batch, r->d + (size_t)k0 * batch * ct_outer, ct_outer, ct_outer);
+            if (k < groups && sl.count < kMaxSwitchGroups) {
+                CK(cudaMemcpyAsync(r->d + (size_t)k * batch * ct_outer, x->d + (shared ? 0 : (size_t)k * batch * ct_outer), (size_t)batch * ct_outer * 8, cudaMemcpyDeviceToDevice, c->st));
+                ++k;
+            }
+            k0 = k;
+        }
+    } catch (...) { hb_ct_free(r); throw; }
+    return r;
+}
+int hb_rotate_hoisted(hb_ctx *c, const hb_ct *a, const hb_digits *dg, int64_t steps, hb_ct **out) { return hb_rotate_hoisted_multi(c, a, dg, &steps, 1, out); }
+int hb_rotate_hoisted_multi(hb_ctx *c, const hb_ct *a, const hb_digits *dg, const int64_t *steps, int count, hb_ct **out) {
     return guard(c, [&] {
+        if (count < 1 || !steps) fail(HB_E_ARG, "rotate_hoisted: no steps");
         if (a->np != 2 || dg->level != a->level || dg->batch != a->batch) fail(HB_E_SHAPE, "rotate_hoisted: digits do not belong to this ciphertext");
         own(c, a); own(c, dg);
-        const u64 g = c->h->galois_rot(steps);
-        const int n = a->level + 1, N = c->N;
-        hb_ct *r = new_ct(c, a->level, 2, a->batch, a->spow);
-        if (g == 1) { CK(cudaMemcpyAsync(r->d, a->d, a->limbs() * N * 8, cudaMemcpyDeviceToDevice, c->st)); *out = r; return; }
-        try {
-            const Evk &key = galois_key(c, g);
-            ALG(c, (size_t)a->batch * (4 * n + plan_dims(c, a->level).dt_count) + key_limbs(c, a->level));
-            ks_apply(c, a->d + (size_t)n * N, (size_t)2 * n * N, dg->d, a->level, a->batch, key, (u32)g, r->d, (size_t)2 * n * N, a->d, nullptr, (size_t)2 * n * N);
-        } catch (...) { hb_ct_free(r); throw; }
-        *out = r;
+        *out = rotate_groups(c, a, dg->d, true, steps, count);
+    });
+}
+int hb_rotate_grouped(hb_ctx *c, const hb_ct *x, const int64_t *steps, int groups, hb_ct **out) {
+    return guard(c, [&] {
+        if (groups < 1 || !steps) fail(HB_E_ARG, "rotate: no steps");
+        own(c, x);
+        if (x->np != 2 || x->batch % groups) fail(HB_E_SHAPE, "rotate: the batch does not split into that many groups");
+        const PlanDims d = plan_dims(c, x->level);
+        Tmp dt(c, (size_t)x->batch * d.dt_count);
+        ks_decompose(c, x->d + (size_t)d.n * c->N, (size_t)2 * d.n * c->N, x->level, x->batch, dt.p);
+        *out = rotate_groups(c, x, dt.p, false, steps, groups);
     });
 }
 int hb_assemble_hoisted(hb_ctx *c, const hb_ct *a, const hb_digits *dg, int64_t s1, const hb_pt *p1, int64_t s2, const hb_pt *p2, hb_ct **out) {
@@ -1617,7 +1657,10 @@ static hb_ct *rotate_sum_core(hb_ctx *c, const u64 *const *base, const int64_t *
         } else {
             Tmp acc(c, (size_t)batch * 2 * ne), t(c, (size_t)batch * 2 * n);
             LAUNCH(c), k_ks_inner_sum<<<dim3(gx, batch, ne), 256, 0, c->st>>>(acc.p, rot, ct_outer, c->nprimes, pl, c->pc, c->logn, N);
-            moddown(c, acc.p, t.p, level, batch, r->d, ct_outer, add.p, add.p + (size_t)n * N, ct_outer, 0u);
+            SwitchList sl{};
+            sl.count = 1;
+            sl.s[0].add[0] = add.p; sl.s[0].add[1] = add.p + (size_t)n * N;
+            moddown(c, acc.p, t.p, level, batch, r->d, ct_outer, sl, batch, ct_outer);
         }
         CK(cudaGetLastError());
     } catch (...) { for (u64 *p : dts) c->pool.put(p); hb_ct_free(r); throw; }
@@ -1659,7 +1702,37 @@ int hb_ntt(hb_ctx *c, hb_ct *a, int inverse) { return guard(c, [&] { own(c, a); 
 int hb_mul_pt_sum_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, int count, int parts, hb_ct **out) {
     return guard(c, [&] {
         if (!a || !p) fail(HB_E_ARG, "product sums: null argument");
-        *out = do_prod_rescale_parts(c, a, p, count, parts);
+        *out = do_prod_rescale_parts(c, a, p, count, parts, false);
+    });
+}
+int hb_mul_pt_sum_parts_each(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, int count, int parts, hb_ct **out) {
+    return guard(c, [&] {
+        if (!a || !p) fail(HB_E_ARG, "product sums: null argument");
+        *out = do_prod_rescale_parts(c, a, p, count, parts, true);
+    });
+}
+// views of the member groups of one ciphertext
+static std::vector<hb_ct> group_views(hb_ctx *c, const hb_ct *x, int groups) {
+    own(c, x);
+    if (groups < 1 || x->batch % groups) fail(HB_E_SHAPE, "the batch does not split into that many groups");
+    const int batch = x->batch / groups;
+    std::vector<hb_ct> v;
+    for (int k = 0; k < groups; ++k) v.push_back(hb_ct{c, x->level, x->np, batch, x->spow, x->d + (size_t)k * batch * x->np * (x->level + 1) * c->N, true});
+    return v;
+}
+int hb_sum_mul_pt_rescale_grouped(hb_ctx *c, const hb_ct *x, const hb_pt *const *p, int count, int sums, hb_ct **out) {
+    return guard(c, [&] {
+        if (!x || !p || count < 1 || sums < 1) fail(HB_E_ARG, "product sums: bad arguments");
+        const std::vector<hb_ct> v = group_views(c, x, count * sums);
+        std::vector<const hb_ct *> a;
+        for (const hb_ct &y : v) a.push_back(&y);
+        *out = do_prod_rescale(c, a.data(), p, count, false, sums);
+    });
+}
+int hb_tensor_acc_halves(hb_ctx *c, const hb_ct *x, hb_ct **acc) {
+    return guard(c, [&] {
+        const std::vector<hb_ct> v = group_views(c, x, 2);
+        *acc = do_tensor(c, &v[0], &v[1], *acc);
     });
 }
 int hb_mul2_add_rescale(hb_ctx *c, const hb_ct *a, const hb_pt *pa, const hb_ct *b, const hb_pt *pb, hb_ct **out) {
@@ -1741,7 +1814,7 @@ int hb_pt_rotate(hb_ctx *c, const hb_pt *p, int64_t steps, hb_pt **out) {
 // plaintext x plaintext with rescale, and plaintext + plaintext: a plaintext is handled as a one-polynomial ciphertext
 int hb_pt_mul(hb_ctx *c, const hb_pt *a, const hb_pt *b, hb_pt **out) {
     return guard(c, [&] {
-        hb_ct view{c, a->level, 1, 1, a->spow, a->d};
+        hb_ct view{c, a->level, 1, 1, a->spow, a->d, true};
         const hb_ct *vp = &view;
         hb_ct *r = do_prod_rescale(c, &vp, &b, 1, true);
         hb_pt *p = new hb_pt{c, r->level, 1, r->d};

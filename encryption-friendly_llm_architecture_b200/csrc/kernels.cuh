@@ -7,6 +7,7 @@
 #pragma once
 #include "modarith.cuh"
 #include "bulk.cuh"
+#include "pdl.cuh"
 
 namespace hb {
 
@@ -91,10 +92,11 @@ __global__ void k_mul2_add(u64 *__restrict__ out, const u64 *__restrict__ a, con
 // tensor product, optional accumulation.  grid.y = batch * n; x, y: [groups][batch][2][n][N]; d: [batch][3][n][N]
 //   d[b] (+)= sum over the groups g of tensor(x[g][b], y[g][b])
 // (groups = 1 is the plain tensor product; several groups are several iterations of a product loop in one launch).
-__global__ void k_tensor(u64 *__restrict__ d, const u64 *__restrict__ x, const u64 *__restrict__ y, int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N,
+__global__ void k_tensor(u64 *d, const u64 *x, const u64 *y, int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N,
                          int accumulate, int groups, int batch) {
     const int bl = blockIdx.y, b = bl / n, l = bl % n;
     const size_t gstride = (size_t)batch * 2 * n * N;
+    pdl_wait();
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
         const int i = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
@@ -212,18 +214,19 @@ __global__ void k_rescale_fin(u64 *__restrict__ out, const u64 *__restrict__ x, 
 // centred lifts of all terms are summed as integers first and ONE transform per limb serves the whole
 // sum.  The stored residues equal those of the term-by-term sequence.
 constexpr int kMaxTerms = 24;
-struct TermList { const u64 *a[kMaxTerms]; const u64 *p[kMaxTerms]; int count; };
-// last[g][bp][x] = (sum over the terms of group g) a_j[bp][level][x] * p_j[level][x] mod q_level
-// grid = (N/256, nbp, groups)   groups = count (separate) or 1
-__global__ void k_last_prod(u64 *__restrict__ last, const __grid_constant__ TermList tl, int separate, int level, int nbp, const PrimeConst *__restrict__ pc, int N) {
+struct TermList { const u64 *a[kMaxTerms]; const u64 *p[kMaxTerms]; int count; }; // `count` terms per sum; sum k takes terms k * count ...
+// last[g][k * nbp + bp][x] = (the terms of group g of sum k) a_j[bp][level][x] * p_j[level][x] mod q_level
+// grid = (N/256, sums * nbp, groups)   groups = count (separate) or 1
+__global__ void k_last_prod(u64 *last, const __grid_constant__ TermList tl, int separate, int level, int nbp, const PrimeConst *__restrict__ pc, int N) {
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
         const int x = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
+        if (u_ == 0) pdl_wait();
         if (x >= N) break;
-        const int bp = blockIdx.y, g = blockIdx.z;
+        const int bp = blockIdx.y % nbp, first = (blockIdx.y / nbp) * tl.count, g = blockIdx.z;
         const PrimeConst m = pc[level];
         const size_t ao = ((size_t)bp * (level + 1) + level) * N + x, po = (size_t)level * N + x;
-        const int j0 = separate ? g : 0, j1 = separate ? g + 1 : tl.count;
+        const int j0 = first + (separate ? g : 0), j1 = separate ? j0 + 1 : first + tl.count;
         u64 r;
         if (m.fp) {
             u64 acc = 0;
@@ -234,23 +237,24 @@ __global__ void k_last_prod(u64 *__restrict__ last, const __grid_constant__ Term
             for (int j = j0; j < j1; ++j) s.mad(tl.a[j][ao], tl.p[j][po]);
             r = barrett128(s.hi, s.lo, m);
         }
-        last[((size_t)g * nbp + bp) * N + x] = r;
+        last[((size_t)g * gridDim.y + blockIdx.y) * N + x] = r;
     }
 }
-// S[bp][x] = sum_g centred(last[g][bp][x]) as a signed integer (|S| <= groups * q_level / 2)
+// S[k * nbp + bp][x] = sum_g centred(last[(k * groups + g) * nbp + bp][x]) as a signed integer (|S| <= groups * q_level / 2)
+// grid = (N/(256*kElems), sums * nbp)
 __global__ void k_centre_sum(i64 *__restrict__ S, const u64 *__restrict__ last, int groups, int nbp, int level, const PrimeConst *__restrict__ pc, int N) {
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
         const int x = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
         if (x >= N) break;
-        const int bp = blockIdx.y;
+        const int bp = blockIdx.y % nbp, k = blockIdx.y / nbp;
         const u64 ql = pc[level].q, half = ql >> 1;
         i64 acc = 0;
         for (int g = 0; g < groups; ++g) {
-            const u64 r = last[((size_t)g * nbp + bp) * N + x];
+            const u64 r = last[((size_t)(k * groups + g) * nbp + bp) * N + x];
             acc += r > half ? (i64)r - (i64)ql : (i64)r;
         }
-        S[(size_t)bp * N + x] = acc;
+        S[(size_t)blockIdx.y * N + x] = acc;
     }
 }
 // t[bp][l][x] = S[bp][x] mod q_l.  grid.y = nbp * level
@@ -263,14 +267,15 @@ __global__ void k_lift_mod(u64 *__restrict__ t, const i64 *__restrict__ S, int l
         t[(size_t)w * N + x] = reduce_i64_any(S[(size_t)bp * N + x], pc[l]);
     }
 }
-// out[bp][l][x] = (sum_j a_j[bp][l][x] * p_j[l][x] - t[bp][l][x]) * q_level^-1.  grid = (N/(256*kElems), nbp * level).
+// out[bp][l][x] = (sum_j a_j[bp][l][x] * p_j[l][x] - t[bp][l][x]) * q_level^-1.  grid = (N/(256*kElems), sums * nbp * level); instance k * nbp + bp.
 // The four coefficients of a thread sit in the inner loop so that eight loads of one term (and, unrolled, of the
 // next) are in flight together: the kernel streams `count` ciphertexts per output and lives on memory parallelism.
 // Blocks are ordered limb-major (all batch members of limb 0, then of limb 1, ...): the plaintext limbs of a sum are
 // shared by every member, and in this order they stay in L2 while the members stream past.
-__global__ void k_prod_rescale_fin(u64 *__restrict__ out, const __grid_constant__ TermList tl, const u64 *__restrict__ t, int level, int nbp, const PrimeConst *__restrict__ pc, int N, const __grid_constant__ Scalars qlinv) {
-    const int l = blockIdx.y / nbp, bp = blockIdx.y % nbp, w = bp * level + l;
+__global__ void k_prod_rescale_fin(u64 *out, const __grid_constant__ TermList tl, const u64 *t, int level, int nbp, const PrimeConst *__restrict__ pc, int N, const __grid_constant__ Scalars qlinv) {
+    const int total = gridDim.y / level, l = blockIdx.y / total, inst = blockIdx.y % total, bp = inst % nbp, first = (inst / nbp) * tl.count, w = inst * level + l;
     const PrimeConst m = pc[l];
+    pdl_wait();
     const u32 x0 = blockIdx.x * (blockDim.x * kElems) + threadIdx.x;
     const size_t ao = ((size_t)bp * (level + 1) + l) * N + x0, po = (size_t)l * N + x0;
     u64 v[kElems];
@@ -279,7 +284,7 @@ __global__ void k_prod_rescale_fin(u64 *__restrict__ out, const __grid_constant_
 #pragma unroll
         for (int u = 0; u < kElems; ++u) acc[u] = 0;
 #pragma unroll 2
-        for (int j = 0; j < tl.count; ++j) {
+        for (int j = first; j < first + tl.count; ++j) {
             const u64 *a = tl.a[j] + ao, *p = tl.p[j] + po;
 #pragma unroll
             for (int u = 0; u < kElems; ++u) acc[u] += mul_small_lazy(a[u * blockDim.x], p[u * blockDim.x], m.q_inv_f, m.q);
@@ -291,7 +296,7 @@ __global__ void k_prod_rescale_fin(u64 *__restrict__ out, const __grid_constant_
 #pragma unroll
         for (int u = 0; u < kElems; ++u) s[u].zero();
 #pragma unroll 2
-        for (int j = 0; j < tl.count; ++j) {
+        for (int j = first; j < first + tl.count; ++j) {
             const u64 *a = tl.a[j] + ao, *p = tl.p[j] + po;
 #pragma unroll
             for (int u = 0; u < kElems; ++u) s[u].mad(a[u * blockDim.x], p[u * blockDim.x]);
@@ -312,6 +317,20 @@ __global__ void k_prod_rescale_fin(u64 *__restrict__ out, const __grid_constant_
 // from L2.  Absent terms of a part are null pointers.
 constexpr int kMaxParts = 17, kMaxPartTerms = 17;
 struct PartTerms { const u64 *a[kMaxPartTerms]; const u64 *p[kMaxParts][kMaxPartTerms]; int count, parts; };
+// last[(g * count + j) * nbp + bp][x] = a_j[bp][level][x] * p_gj[level][x] mod q_level, zero for an absent term: every product is
+// rescaled on its own (as eval.mult(ct, mask) does).  grid = (N/256, nbp, parts * count)
+__global__ void k_last_prod_parts(u64 *last, const __grid_constant__ PartTerms pt, int level, int nbp, const PrimeConst *__restrict__ pc, int N) {
+    const int bp = blockIdx.y, g = blockIdx.z / pt.count, j = blockIdx.z % pt.count;
+    const PrimeConst m = pc[level];
+    const u64 *p = pt.p[g][j];
+    pdl_wait();
+#pragma unroll
+    for (int u_ = 0; u_ < kElems; ++u_) {
+        const int x = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
+        if (x >= N) break;
+        last[((size_t)blockIdx.z * nbp + bp) * N + x] = p ? mul_mod_any(pt.a[j][((size_t)bp * (level + 1) + level) * N + x], p[(size_t)level * N + x], m) : 0;
+    }
+}
 // A CTA of 1024 threads keeps the mask chunks of G parts for its 256 coefficients of one limb in shared memory (bulk
 // copies, up to G * 17 chunks of 2 KB, one mbarrier, bounded wait) and walks over the batch members, four at a time
 // (thread = coefficient + 256 * member slot): the masks cross L2 once per CTA instead of once per member, the a_j of a
@@ -482,22 +501,30 @@ __global__ void k_modup(u64 *__restrict__ dt, const u64 *__restrict__ a_coef, co
     }
 }
 
+// Up to 16 groups of `batch` members, each group with its own key switch: operand (limbs of the switched polynomial in NTT form and
+// its lifted digits), key, Galois element (0: no automorphism) and addends (null: none).
+struct SwitchGroup { const u64 *a_ntt, *dt, *key, *add[2]; u32 g, pad; };
+constexpr int kMaxSwitchGroups = 16;
+struct SwitchList { SwitchGroup s[kMaxSwitchGroups]; int count; };
 // Inner product with the switching key over Q_level u P.
-//   acc[b][p][j][i] = sum_dg digit_dg[j][perm_g(i)] * key[dg][p][prime(j)][i]
-// digit_dg[j] is a_ntt[j] for own limbs and dt[...] otherwise.  grid = (N/(256*kElems), batch, ne)
-__global__ void k_ks_inner(u64 *__restrict__ acc, const u64 *__restrict__ a_ntt, size_t a_outer, const u64 *__restrict__ dt, const u64 *__restrict__ key, int key_primes,
-                           const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, u32 g, int logn, int N) {
-    const int j = blockIdx.z, b = blockIdx.y; // limb-major block order: the key limbs stay in L2 across the members
+//   acc[ob][p][j][i] = sum_dg digit_dg[j][perm_g(i)] * key[dg][p][prime(j)][i],   member ob = group * batch + b
+// digit_dg[j] is a_ntt[j] for own limbs and dt[...] otherwise.  grid = (N/(256*kElems), groups * batch, ne)
+__global__ void k_ks_inner(u64 *acc, const __grid_constant__ SwitchList sl, int batch, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, int logn,
+                           int N) {
+    const int j = blockIdx.z, ob = blockIdx.y, b = ob % batch; // limb-major block order: the key limbs stay in L2 across the members
+    const SwitchGroup &sg = sl.s[ob / batch];
+    const u32 g = sg.g;
     const int pj = pl->ext_prime[j], nd = pl->nd, ne = pl->ne;
     const PrimeConst m = pc[pj];
     const u32 x0 = blockIdx.x * (blockDim.x * kElems) + threadIdx.x;
     u32 src[kElems];
 #pragma unroll
     for (int u = 0; u < kElems; ++u) { const u32 i = x0 + u * blockDim.x; src[u] = g ? ntt_perm(i, g, logn) : i; }
-    const u64 *abase = a_ntt + (size_t)b * a_outer + (size_t)j * N;
-    const u64 *dbase = dt + (size_t)b * pl->dt_count * N;
-    const u64 *kbase = key + (size_t)pj * N + x0;
+    const u64 *abase = sg.a_ntt + (size_t)b * a_outer + (size_t)j * N;
+    const u64 *dbase = sg.dt + (size_t)b * pl->dt_count * N;
+    const u64 *kbase = sg.key + (size_t)pj * N + x0;
     const size_t kpoly = (size_t)key_primes * N;
+    pdl_wait();
     u64 r0[kElems], r1[kElems];
     if (m.fp) { // products on the FP64 pipe, signed double sums
         const double qd = (double)m.q;
@@ -535,7 +562,7 @@ __global__ void k_ks_inner(u64 *__restrict__ acc, const u64 *__restrict__ a_ntt,
 #pragma unroll
         for (int u = 0; u < kElems; ++u) { r0[u] = barrett128(s0[u].hi, s0[u].lo, m); r1[u] = barrett128(s1[u].hi, s1[u].lo, m); }
     }
-    u64 *o0 = acc + (((size_t)b * 2) * ne + j) * N + x0, *o1 = o0 + (size_t)ne * N;
+    u64 *o0 = acc + (((size_t)ob * 2) * ne + j) * N + x0, *o1 = o0 + (size_t)ne * N;
 #pragma unroll
     for (int u = 0; u < kElems; ++u) { o0[u * blockDim.x] = r0[u]; o1[u * blockDim.x] = r1[u]; }
 }
@@ -591,25 +618,26 @@ __global__ void k_moddown_conv(u64 *__restrict__ t, const u64 *__restrict__ pcoe
     default: moddown_conv_body<8>(t, pcoef, pl, pc, Lp1, N, i, bp); break;
     }
 }
-// out[b][p][l][i] = (acc[b][p][l][i] - t[b][p][l][i]) * P^-1 + add_p[b][l][perm_g(i)]
-// add0 / add1 may be null; perm applies when g != 0.  grid = (N/256, n, batch*2)
-__global__ void k_moddown_fin(u64 *__restrict__ out, size_t out_outer, const u64 *__restrict__ acc, const u64 *__restrict__ t, const u64 *__restrict__ add0,
-                              const u64 *__restrict__ add1, size_t add_outer, const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, u32 g, int logn, int N) {
+// out[ob][p][l][i] = (acc[ob][p][l][i] - t[ob][p][l][i]) * P^-1 + add_p[b][l][perm_g(i)],  addends and g of ob's group
+// grid = (N/256, n, groups*batch*2)
+__global__ void k_moddown_fin(u64 *out, size_t out_outer, const u64 *acc, const u64 *t, const __grid_constant__ SwitchList sl, int batch, size_t add_outer, const KsPlan *__restrict__ pl,
+                              const PrimeConst *__restrict__ pc, int logn, int N) {
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
         const int i = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
         if (i >= N) break;
-        const int l = blockIdx.y, bp = blockIdx.z, b = bp >> 1, p = bp & 1;
+        const int l = blockIdx.y, bp = blockIdx.z, ob = bp >> 1, b = ob % batch, p = bp & 1;
+        const SwitchGroup &sg = sl.s[ob / batch];
         const int n = pl->n, ne = pl->ne;
         const PrimeConst m = pc[l];
         u64 v = sub_mod(acc[((size_t)bp * ne + l) * N + i], t[((size_t)bp * n + l) * N + i], m.q);
         v = mul_mod_any(v, pl->p_inv[l], m);
-        const u64 *ad = p ? add1 : add0;
+        const u64 *ad = sg.add[p];
         if (ad) {
-            const u32 s = g ? ntt_perm((u32)i, g, logn) : (u32)i;
+            const u32 s = sg.g ? ntt_perm((u32)i, sg.g, logn) : (u32)i;
             v = add_mod(v, ad[(size_t)b * add_outer + (size_t)l * N + s], m.q);
         }
-        out[(size_t)b * out_outer + ((size_t)p * n + l) * N + i] = v;
+        out[(size_t)ob * out_outer + ((size_t)p * n + l) * N + i] = v;
     }
 }
 

@@ -27,6 +27,7 @@
 //    Primes of 44 bits and more use Shoup butterflies on integers below 16 q.
 #pragma once
 #include "modarith.cuh"
+#include "pdl.cuh"
 #include <cstring>
 
 namespace hb {
@@ -89,6 +90,28 @@ struct LimbAddr16 {
     __device__ __forceinline__ size_t off(int li, int period) const { return (size_t)(li / period) * outer + (size_t)(li % period) * kN16; }
 };
 
+// The fifteen twiddles of a radix-16 round, j = (1 << s) - 1 + g of local stage s, group g.
+struct TwiddlesA { // shared by many threads: (w, companion), consecutive
+    const ulonglong2 *p;
+    __device__ __forceinline__ explicit TwiddlesA(const ulonglong2 *q) : p(q) {}
+    __device__ __forceinline__ ulonglong2 operator[](int j) const { return __ldg(p + j); }
+};
+// owned by one thread, 16 entries apart; EARLY: fetched when the object is made instead of when they are used
+template <class T, bool EARLY> struct TwiddlesB;
+template <class T> struct TwiddlesB<T, false> {
+    const T *p;
+    __device__ __forceinline__ explicit TwiddlesB(const T *q) : p(q) {}
+    __device__ __forceinline__ T operator[](int j) const { return __ldg(p + j * 16); }
+};
+template <class T> struct TwiddlesB<T, true> {
+    T w[15];
+    __device__ __forceinline__ explicit TwiddlesB(const T *q) {
+#pragma unroll
+        for (int j = 0; j < 15; ++j) w[j] = __ldg(q + j * 16);
+    }
+    __device__ __forceinline__ T operator[](int j) const { return w[j]; }
+};
+
 // ---------------- Shoup butterflies on integers (primes of 44 bits and more) ----------------
 // exact quotients, values in [0, 4q) and [0, 2q): the small-ring kernel
 __device__ __forceinline__ void ct_bfly(u64 &x, u64 &y, u64 w, u64 ws, u64 q, u64 q2) {
@@ -112,17 +135,17 @@ __device__ __forceinline__ IntConst int_const(const PrimeConst &m) {
     c.q = m.q; c.nq = 0ull - m.q; c.q4 = m.q << 2; c.q8 = m.q << 3; c.sh = m.fold_shift;
     return c;
 }
-// Four Cooley-Tukey stages on 16 register values; twiddle j = (1 << s) - 1 + g of local stage s, group g, at tp[j * STRIDE].
+// Four Cooley-Tukey stages on 16 register values; twiddles tp[j].
 // Products are below 4q (mul_shoup4), so a stage adds 4q to the bound B of the values; x is folded below ~2^b before the
 // additions of the stages named by the bit mask FOLD.  The words hold 16 q: in units of q the four rounds of a transform
 // (masks 8, 4, 2, 9) run 3-7-11-15|5, 5-9-13|5-9, 9-13|5-9-13, 13|5-9-13|5 (| = a fold).
-template <int STRIDE, int FOLD> __device__ __forceinline__ void fwd16_int(u64 (&v)[16], const ulonglong2 *__restrict__ tp, const IntConst &c) {
+template <int FOLD, class TW> __device__ __forceinline__ void fwd16_int(u64 (&v)[16], const TW &tp, const IntConst &c) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         const int half = 8 >> s;
 #pragma unroll
         for (int g = 0; g < (1 << s); ++g) {
-            const ulonglong2 tw = __ldg(tp + ((1 << s) - 1 + g) * STRIDE);
+            const ulonglong2 tw = tp[(1 << s) - 1 + g];
 #pragma unroll
             for (int j = 0; j < half; ++j) {
                 u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
@@ -137,13 +160,13 @@ template <int STRIDE, int FOLD> __device__ __forceinline__ void fwd16_int(u64 (&
 constexpr int kFoldColsA = 8, kFoldColsB = 4, kFoldRowsA = 2, kFoldRowsB = 9;
 // Four Gentleman-Sande stages, the mirror image.  Values enter and leave below 4q: sums reach 8q, then 16q, and are folded at
 // every second stage.
-template <int STRIDE> __device__ __forceinline__ void inv16_int(u64 (&v)[16], const ulonglong2 *__restrict__ tp, const IntConst &c) {
+template <class TW> __device__ __forceinline__ void inv16_int(u64 (&v)[16], const TW &tp, const IntConst &c) {
 #pragma unroll
     for (int s = 3; s >= 0; --s) {
         const int half = 8 >> s;
 #pragma unroll
         for (int g = 0; g < (1 << s); ++g) {
-            const ulonglong2 tw = __ldg(tp + ((1 << s) - 1 + g) * STRIDE);
+            const ulonglong2 tw = tp[(1 << s) - 1 + g];
 #pragma unroll
             for (int j = 0; j < half; ++j) {
                 u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
@@ -205,13 +228,13 @@ __device__ __forceinline__ u64 ds_store(double v, const DsConst &c, double shift
     const double rb = __fma_rn(-k, c.qd, v2 + kTwo52);                   // 2^52 + (v2 - k q), exact
     return (u64)__double_as_longlong(rb) & 0x000FFFFFFFFFFFFFull;
 }
-template <int STRIDE> __device__ __forceinline__ void fwd16_ds(double (&v)[16], const ulonglong2 *__restrict__ tp, const DsConst &c) {
+template <class TW> __device__ __forceinline__ void fwd16_ds(double (&v)[16], const TW &tp, const DsConst &c) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         const int half = 8 >> s;
 #pragma unroll
         for (int g = 0; g < (1 << s); ++g) {
-            const ulonglong2 tw = __ldg(tp + ((1 << s) - 1 + g) * STRIDE);
+            const ulonglong2 tw = tp[(1 << s) - 1 + g];
             const double wf = __longlong_as_double((long long)tw.y);
 #pragma unroll
             for (int j = 0; j < half; ++j) {
@@ -223,13 +246,13 @@ template <int STRIDE> __device__ __forceinline__ void fwd16_ds(double (&v)[16], 
         }
     }
 }
-template <int STRIDE> __device__ __forceinline__ void fwd16_ds8(double (&v)[16], const double *__restrict__ tp, const DsConst &c) {
+template <class TW> __device__ __forceinline__ void fwd16_ds8(double (&v)[16], const TW &tp, const DsConst &c) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         const int half = 8 >> s;
 #pragma unroll
         for (int g = 0; g < (1 << s); ++g) {
-            const double wd = __ldg(tp + ((1 << s) - 1 + g) * STRIDE);
+            const double wd = tp[(1 << s) - 1 + g];
 #pragma unroll
             for (int j = 0; j < half; ++j) {
                 double &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
@@ -240,13 +263,13 @@ template <int STRIDE> __device__ __forceinline__ void fwd16_ds8(double (&v)[16],
         }
     }
 }
-template <int STRIDE> __device__ __forceinline__ void inv16_ds8(double (&v)[16], const double *__restrict__ tp, const DsConst &c) {
+template <class TW> __device__ __forceinline__ void inv16_ds8(double (&v)[16], const TW &tp, const DsConst &c) {
 #pragma unroll
     for (int s = 3; s >= 0; --s) {
         const int half = 8 >> s;
 #pragma unroll
         for (int g = 0; g < (1 << s); ++g) {
-            const double wd = __ldg(tp + ((1 << s) - 1 + g) * STRIDE);
+            const double wd = tp[(1 << s) - 1 + g];
 #pragma unroll
             for (int j = 0; j < half; ++j) {
                 double &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
@@ -261,13 +284,13 @@ template <int STRIDE> __device__ __forceinline__ void inv16_ds8(double (&v)[16],
 // Gentleman-Sande round.  The sum path doubles per stage; only v[0] takes the sum at all four stages (16 x its
 // inputs), v[1] ends below 4.2 q whatever came in, the others lower: the caller reduces v[0] after each round, so
 // every round starts from values below 4.2 q and stays below 68 q.
-template <int STRIDE> __device__ __forceinline__ void inv16_ds(double (&v)[16], const ulonglong2 *__restrict__ tp, const DsConst &c) {
+template <class TW> __device__ __forceinline__ void inv16_ds(double (&v)[16], const TW &tp, const DsConst &c) {
 #pragma unroll
     for (int s = 3; s >= 0; --s) {
         const int half = 8 >> s;
 #pragma unroll
         for (int g = 0; g < (1 << s); ++g) {
-            const ulonglong2 tw = __ldg(tp + ((1 << s) - 1 + g) * STRIDE);
+            const ulonglong2 tw = tp[(1 << s) - 1 + g];
             const double wf = __longlong_as_double((long long)tw.y);
 #pragma unroll
             for (int j = 0; j < half; ++j) {
@@ -283,7 +306,7 @@ template <int STRIDE> __device__ __forceinline__ void inv16_ds(double (&v)[16], 
 
 // ---- forward, column pass: stages 1..8 ----
 template <int MINB>
-__global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_cols(const u64 *__restrict__ src, LimbAddr16 sa, u64 *__restrict__ dst, LimbAddr16 da,
+__global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_cols(const u64 *src, LimbAddr16 sa, u64 *dst, LimbAddr16 da,
                                                         const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     __shared__ u64 sm[4096];
     const int li = blockIdx.y, pi = map.prime[li % map.n];
@@ -295,31 +318,33 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_cols(const u64 *__restr
     if (m.small) {
         const DsConst c = ds_const(m);
         double v[16];
+        pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = ds_load(p[(e * 16 + sub) * 256]);
-        fwd16_ds<1>(v, tab + Ntt16Layout::colsA(0), c);
+        fwd16_ds(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
         double *smd = reinterpret_cast<double *>(sm);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[(e * 16 + sub) * 16 + lane] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smd[(sub * 16 + e) * 16 + lane];
-        fwd16_ds<1>(v, tab + Ntt16Layout::colsB(sub, 0), c);
+        fwd16_ds(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
         double *od = reinterpret_cast<double *>(o);
 #pragma unroll
         for (int e = 0; e < 16; ++e) od[(sub * 16 + e) * 256] = v[e];
     } else {
         u64 v[16];
+        pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = p[(e * 16 + sub) * 256];
         const IntConst c = int_const(m);
-        fwd16_int<1, kFoldColsA>(v, tab + Ntt16Layout::colsA(0), c);
+        fwd16_int<kFoldColsA>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[(e * 16 + sub) * 16 + lane] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[(sub * 16 + e) * 16 + lane];
-        fwd16_int<1, kFoldColsB>(v, tab + Ntt16Layout::colsB(sub, 0), c);
+        fwd16_int<kFoldColsB>(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) o[(sub * 16 + e) * 256] = v[e];
     }
@@ -327,7 +352,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_cols(const u64 *__restr
 
 // ---- forward, row pass: stages 9..16; stores canonical residues ----
 template <int MINB>
-__global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows(const u64 *__restrict__ src, LimbAddr16 sa, u64 *__restrict__ dst, LimbAddr16 da,
+__global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows(const u64 *src, LimbAddr16 sa, u64 *dst, LimbAddr16 da,
                                                         const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     __shared__ u64 sm[16 * kRowStride];
     const int li = blockIdx.y, pi = map.prime[li % map.n];
@@ -343,30 +368,34 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows(const u64 *__restr
         const double *pd = reinterpret_cast<const double *>(p);
         double *smd = reinterpret_cast<double *>(smr);
         double v[16];
+        const TwiddlesB<double, MINB <= 2> tw(tb.fwdB8 + (size_t)pi * kRowsB8 + (row * 15) * 16 + clo);
+        pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = pd[e * 16];
-        fwd16_ds<1>(v, tab + Ntt16Layout::rowsA(row, 0), c);
+        fwd16_ds(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[e * 17 + clo] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smd[clo * 17 + e];
-        fwd16_ds8<16>(v, tb.fwdB8 + (size_t)pi * kRowsB8 + (row * 15) * 16 + clo, c);
+        fwd16_ds8(v, tw, c);
         const double shift = 16.0 * c.qd, qinv_up = c.qinv * (1.0 + 0x1p-50);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = ds_store(v[e], c, shift, qinv_up); // the words this thread read itself
     } else {
         const IntConst c = int_const(m);
         u64 v[16];
+        const TwiddlesB<ulonglong2, MINB <= 2> tw(tab + Ntt16Layout::rowsB(row, 0, clo));
+        pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = p[e * 16];
-        fwd16_int<1, kFoldRowsA>(v, tab + Ntt16Layout::rowsA(row, 0), c);
+        fwd16_int<kFoldRowsA>(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
-        fwd16_int<16, kFoldRowsB>(v, tab + Ntt16Layout::rowsB(row, 0, clo), c);
+        fwd16_int<kFoldRowsB>(v, tw, c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = canon_q(v[e], c.q, c.sh);
     }
@@ -377,7 +406,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows(const u64 *__restr
 
 // ---- inverse, row pass: undoes stages 16..9 ----
 template <int MINB>
-__global__ void __launch_bounds__(256, MINB) ntt16v2_inv_rows(const u64 *__restrict__ src, LimbAddr16 sa, u64 *__restrict__ dst, LimbAddr16 da,
+__global__ void __launch_bounds__(256, MINB) ntt16v2_inv_rows(const u64 *src, LimbAddr16 sa, u64 *dst, LimbAddr16 da,
                                                         const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     __shared__ u64 sm[16 * kRowStride];
     const int li = blockIdx.y, pi = map.prime[li % map.n];
@@ -388,37 +417,44 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_rows(const u64 *__restr
     const u64 *p = src + sa.off(li, map.n) + (size_t)row * 256 + clo;
     u64 *o = dst + da.off(li, map.n) + (size_t)row * 256 + clo;
     u64 *smr = sm + rl * kRowStride;
+    const auto exchange_in = [&] { // the coefficients, row-major into shared memory
+        pdl_wait();
 #pragma unroll
-    for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = p[e * 16];
-    __syncthreads();
+        for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = p[e * 16];
+        __syncthreads();
+    };
     if (m.small) {
+        const TwiddlesB<double, MINB <= 2> tw(tb.invB8 + (size_t)pi * kRowsB8 + (row * 15) * 16 + clo);
+        exchange_in();
         const DsConst c = ds_const(m);
         double *smd = reinterpret_cast<double *>(smr);
         double v[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = ds_load(smr[clo * 17 + e]);
-        inv16_ds8<16>(v, tb.invB8 + (size_t)pi * kRowsB8 + (row * 15) * 16 + clo, c);
+        inv16_ds8(v, tw, c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[clo * 17 + e] = v[e]; // the words this thread read itself
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smd[e * 17 + clo];
-        inv16_ds<1>(v, tab + Ntt16Layout::rowsA(row, 0), c);
+        inv16_ds(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
         double *od = reinterpret_cast<double *>(o);
 #pragma unroll
         for (int e = 0; e < 16; ++e) od[e * 16] = v[e];
     } else {
+        const TwiddlesB<ulonglong2, MINB <= 2> tw(tab + Ntt16Layout::rowsB(row, 0, clo));
+        exchange_in();
         u64 v[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
         const IntConst c = int_const(m);
-        inv16_int<16>(v, tab + Ntt16Layout::rowsB(row, 0, clo), c);
+        inv16_int(v, tw, c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[e * 17 + clo];
-        inv16_int<1>(v, tab + Ntt16Layout::rowsA(row, 0), c);
+        inv16_int(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) o[e * 16] = v[e];
     }
@@ -426,7 +462,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_rows(const u64 *__restr
 
 // ---- inverse, column pass: undoes stages 8..1, scales by N^-1, stores canonical residues ----
 template <int MINB>
-__global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *__restrict__ src, LimbAddr16 sa, u64 *__restrict__ dst, LimbAddr16 da,
+__global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *src, LimbAddr16 sa, u64 *dst, LimbAddr16 da,
                                                         const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     __shared__ u64 sm[4096];
     const int li = blockIdx.y, pi = map.prime[li % map.n];
@@ -440,15 +476,16 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *__restr
         const double *pd = reinterpret_cast<const double *>(p);
         double *smd = reinterpret_cast<double *>(sm);
         double v[16];
+        pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = pd[(sub * 16 + e) * 256];
-        inv16_ds<1>(v, tab + Ntt16Layout::colsB(sub, 0), c);
+        inv16_ds(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[(sub * 16 + e) * 16 + lane] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smd[(e * 16 + sub) * 16 + lane];
-        inv16_ds<1>(v, tab + Ntt16Layout::colsA(0), c);
+        inv16_ds(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
         const double qinv_up = c.qinv * (1.0 + 0x1p-50);
         const u64 sw = ds_twiddle_word(m.n_inv);
 #pragma unroll
@@ -458,16 +495,17 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *__restr
         }
     } else {
         u64 v[16];
+        pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = p[(sub * 16 + e) * 256];
         const IntConst c = int_const(m);
-        inv16_int<1>(v, tab + Ntt16Layout::colsB(sub, 0), c);
+        inv16_int(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[(sub * 16 + e) * 16 + lane] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[(e * 16 + sub) * 16 + lane];
-        inv16_int<1>(v, tab + Ntt16Layout::colsA(0), c);
+        inv16_int(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) o[(e * 16 + sub) * 256] = canon_q(mul_shoup4(v[e], m.n_inv, m.n_inv_sh, c.nq), c.q, c.sh);
     }
@@ -483,11 +521,11 @@ inline cudaError_t launch_ntt16(cudaStream_t st, const u64 *src, size_t src_oute
     LimbAddr16 sa{src_outer}, da{dst_outer};
     dim3 grid(16, count);
     if (!inverse) {
-        ntt16v2_fwd_cols<MINB><<<grid, 256, 0, st>>>(src, sa, dst, da, map, pc, tb);
-        ntt16v2_fwd_rows<MINB><<<grid, 256, 0, st>>>(dst, da, dst, da, map, pc, tb);
+        launch_pdl(st, ntt16v2_fwd_cols<MINB>, grid, 256, 0, src, sa, dst, da, map, pc, tb);
+        launch_pdl(st, ntt16v2_fwd_rows<MINB>, grid, 256, 0, dst, da, dst, da, map, pc, tb);
     } else {
-        ntt16v2_inv_rows<MINB><<<grid, 256, 0, st>>>(src, sa, dst, da, map, pc, tb);
-        ntt16v2_inv_cols<MINB><<<grid, 256, 0, st>>>(dst, da, dst, da, map, pc, tb);
+        launch_pdl(st, ntt16v2_inv_rows<MINB>, grid, 256, 0, src, sa, dst, da, map, pc, tb);
+        launch_pdl(st, ntt16v2_inv_cols<MINB>, grid, 256, 0, dst, da, dst, da, map, pc, tb);
     }
     return cudaGetLastError();
 }

@@ -145,6 +145,8 @@ int hb_batch_get(hb_ctx *ctx, const hb_ct *src, int index, hb_ct **out);
 /* join batches end to end / copy out a run of entries (device-to-device copies) */
 int hb_batch_concat(hb_ctx *ctx, const hb_ct *const *parts, int n, hb_ct **out);
 int hb_batch_slice(hb_ctx *ctx, const hb_ct *src, int start, int count, hb_ct **out);
+/* the same run of entries as a handle on src's own buffer: no copy; src must outlive every use of the view.  Freed with hb_ct_free. */
+int hb_batch_view(hb_ctx *ctx, const hb_ct *src, int start, int count, hb_ct **out);
 
 /* HomEvaluator primitives; `out` receives a new handle unless stated otherwise. */
 int hb_add(hb_ctx *ctx, const hb_ct *a, const hb_ct *b, hb_ct **out);           /* HomEvaluator.hpp:143-146 */
@@ -181,6 +183,11 @@ int hb_conjugate(hb_ctx *ctx, const hb_ct *a, hb_ct **out);                     
 int hb_decompose(hb_ctx *ctx, const hb_ct *a, hb_digits **out);
 int hb_rotate_hoisted(hb_ctx *ctx, const hb_ct *a, const hb_digits *digits, int64_t left_steps, hb_ct **out);
 void hb_digits_free(hb_digits *digits);
+/* Several rotations in one launch sequence, member for member the residues of hb_rotate: hb_rotate_hoisted_multi gives rot(a, steps[k])
+ * for every k (count * batch(a) members, step-major); hb_rotate_grouped rotates the member groups of x (group k = members
+ * k * batch / groups onwards) by steps[k] each. */
+int hb_rotate_hoisted_multi(hb_ctx *ctx, const hb_ct *a, const hb_digits *digits, const int64_t *left_steps, int count, hb_ct **out);
+int hb_rotate_grouped(hb_ctx *ctx, const hb_ct *x, const int64_t *left_steps, int groups, hb_ct **out);
 /* out = sum_t rot(xs[t], left_steps[t]) for ciphertexts of equal level (at most 16 rotated and 16 unrotated terms): the key-switch inner products of
  * all terms are added up in the extended basis and ONE ModDown serves the sum (a step of 0 adds its operand as it is).
  * The giant-step half of a baby-step / giant-step transform in schedule 2.  Same slots as the sum of hb_rotate
@@ -230,6 +237,11 @@ int hb_mul_pt_sum(hb_ctx *ctx, const hb_ct *const *a, const hb_pt *const *p, int
  * transform (MatrixUtils.cpp:776-1070) share their baby-step rotations.  out holds parts * batch members, part-major;
  * every part has the residues hb_sum_mul_pt_rescale gives for its terms. */
 int hb_mul_pt_sum_parts(hb_ctx *ctx, const hb_ct *const *a, const hb_pt *const *p, int count, int parts, hb_ct **out);
+/* the same with every product rescaled on its own before the sum, as hb_mul_pt_sum does */
+int hb_mul_pt_sum_parts_each(hb_ctx *ctx, const hb_ct *const *a, const hb_pt *const *p, int count, int parts, hb_ct **out);
+/* out_k = rescale(sum_{j < count} x_{k * count + j} (.) p[k * count + j]) for k < sums, where x_i is member group i of x (count * sums
+ * groups, at most 24); out holds sums * batch / (count * sums) members, sum-major */
+int hb_sum_mul_pt_rescale_grouped(hb_ctx *ctx, const hb_ct *x, const hb_pt *const *p, int count, int sums, hb_ct **out);
 /* out = rescale(sum_j a[j] (.) p[j]): the products are added un-rescaled and the sum is rescaled once (one inverse
  * transform of the last limb instead of one per term).  The masked sums of the linear transforms in schedule 2. */
 int hb_sum_mul_pt_rescale(hb_ctx *ctx, const hb_ct *const *a, const hb_pt *const *p, int count, hb_ct **out);
@@ -238,6 +250,8 @@ int hb_tensor_acc(hb_ctx *ctx, const hb_ct *a, const hb_ct *b, hb_ct **acc);
 /* *acc (+)= sum over g < groups of tensor(a[g], b[g]); a and b hold groups * batch members (group-major), *acc holds
  * batch members (NULL: created).  Same residues as `groups` calls of hb_tensor_acc. */
 int hb_tensor_acc_groups(hb_ctx *ctx, const hb_ct *a, const hb_ct *b, int groups, hb_ct **acc);
+/* acc += tensor(first half of the members of x, second half); *acc may be NULL on entry */
+int hb_tensor_acc_halves(hb_ctx *ctx, const hb_ct *x, hb_ct **acc);
 /* out = sum_k pre[k] (.) rot_rows(pt, k * row_step), un-rescaled -- HomEvaluator::matmul :595-601 */
 int hb_matmul_acc(hb_ctx *ctx, const hb_ct *pre, const hb_pt *pt, int64_t row_step, hb_ct **out);
 /* the same over several K-groups at once: `pre` holds the shifted copies of `btotal` independent inputs, copy k of
