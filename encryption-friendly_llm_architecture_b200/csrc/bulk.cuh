@@ -20,6 +20,8 @@ __device__ __forceinline__ void bulk_load(void *dst_smem, const void *src_gmem, 
                  "r"(smem_u32(bar))
                  : "memory");
 }
+// asks for `bytes` (a multiple of 16) at a 16-byte aligned global address to be brought into L2
+__device__ __forceinline__ void prefetch_l2(const void *p, u32 bytes) { asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory"); }
 __device__ __forceinline__ bool mbar_try_wait(u64 *bar, u32 parity) {
     u32 ok;
     // the last operand is a suspend-time hint in nanoseconds: the thread may sleep that long inside the instruction

@@ -30,9 +30,13 @@ struct ConvPlan {
     int ns, nt;
     int src_limb, dst_limb;             // first limb of the sources / targets inside one instance of the arrays
     unsigned char src_prime[8], dst_prime[kMaxPrimes];
+    unsigned char order[kMaxPrimes];    // targets in the order they are taken: those of the long primes, which take twice the time, first
     u64 scale_w[8], scale_c[8];         // (ds_twiddle_word, w / q as a double) below 2^44, (w, Shoup companion) otherwise
+    unsigned char fp[kMaxPrimes];       // target t converts on the FP64 pipe (see ConvFp)
     uint4 c[kMaxPrimes][8];             // [target][source]: C = D / d_s mod target.  Target below 2^44: the 26-bit pieces of C
                                         // and of C * 2^30; otherwise the 30-bit pieces of C, 0, 0
+    double d[kMaxPrimes][8][4];         // fp targets: C = d1 + d0 with d1 a multiple of 2^21, |d0| <= 2^20, C taken within q/2 of zero; the
+                                        // same for C * 2^30.  Set when every sum of the products is exact in a double
 };
 
 template <int COLS> struct StripIndex { // [256 rows][COLS] words in shared memory, COLS pad words per 16 rows: both access patterns are conflict-free
@@ -75,21 +79,20 @@ __device__ __forceinline__ void strip_inverse(u64 (&v)[16], const u64 *p /* limb
         for (int e = 0; e < 16; ++e) v[e] = sm[I::a(e, sub, lane)];
         inv16_int(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = canon_q(mul_shoup4(v[e], sw, sc, c.nq), c.q, c.sh);
+        for (int e = 0; e < 16; ++e) v[e] = canon_q(mul_shoup4(v[e], sw, sc, c.nq), c.q, c.f);
     }
 }
-// Forward column pass of one limb strip: v[e] holds row e * 16 + sub (double bits below 2^44, |v| < 2q; otherwise words below 4q).
+// Forward column pass of one limb strip that lies in sm (words of this thread at I::a; double bits below 2^44, |v| < 2q; otherwise below 4q).
 template <int COLS>
-__device__ __forceinline__ void strip_forward(u64 (&v)[16], u64 *o /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, int g, int sub, int lane) {
+__device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, int g, int sub, int lane) {
     using I = StripIndex<COLS>;
     if (m.small) {
         const DsConst c = ds_const(m);
         double *smd = reinterpret_cast<double *>(sm);
         double d[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) d[e] = __longlong_as_double((long long)v[e]);
+        for (int e = 0; e < 16; ++e) d[e] = smd[I::a(e, sub, lane)];
         fwd16_ds(d, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
-        group_sync<COLS * 16>(g); // the strip of the previous target has been read
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[I::a(e, sub, lane)] = d[e];
         group_sync<COLS * 16>(g);
@@ -100,8 +103,10 @@ __device__ __forceinline__ void strip_forward(u64 (&v)[16], u64 *o /* limb + col
         for (int e = 0; e < 16; ++e) reinterpret_cast<double *>(o)[(sub * 16 + e) * 256] = d[e];
     } else {
         const IntConst c = int_const(m);
+        u64 v[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = sm[I::a(e, sub, lane)];
         fwd16_int<kFoldColsA>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
-        group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[I::a(e, sub, lane)] = v[e];
         group_sync<COLS * 16>(g);
@@ -135,70 +140,95 @@ __device__ __forceinline__ double finish_small(u64 a0, u64 a1, const SmallFinish
     const u32 hi = q1 * f.n0 + (q0 * f.n1 + (u32)(r >> 32)) + f.hi0;
     return __hiloint2double((int)hi, (int)(u32)r) - kMagic;
 }
-// a0 + a1 * 2^30 + a2 * 2^60 modulo a prime of 45 to 60 bits (a0, a1 + 2^34, a2 + 2^34 < 2^64): below 4q
-__device__ __forceinline__ u64 finish_wide(u64 a0, u64 a1, u64 a2, const PrimeConst &m) {
-    const u32 m30 = 0x3FFFFFFFu;
-    if (m.d60) { // 2^60 = d60 modulo q
-        const u64 u = a1 + (a0 >> 30), v = a2 + (u >> 30);
-        u64 r = mad_wide((u32)u & m30, 1u << 30, (u64)((u32)a0 & m30)); // < 2^60
-        r = mad_wide((u32)v, m.d60, r);                                 // + 2^58
-        const u64 t = (u64)(u32)(v >> 32) * m.d60;                      // < 2^58, weight 2^32
-        r = mad_wide((u32)(t >> 28), m.d60, r);                         // + 2^56
-        return r + ((u64)((u32)t & 0x0FFFFFFFu) << 32);                 // + 2^60
-    }
-    u64 lo = a0, hi = 0, x = a1 << 30;
-    lo += x; hi += (a1 >> 34) + (lo < x);
-    x = a2 << 60;
-    lo += x; hi += (a2 >> 4) + (lo < x);
-    return barrett128(hi, lo, m);
-}
-// the converted values of one target for this thread's sixteen coefficients.  NS > 0: compile-time source count, constants in registers.
-template <int NS, int COLS>
-__device__ __forceinline__ void convert_target(u64 (&v)[16], const u64 *ysm, const uint4 *__restrict__ cst, int ns_rt, const PrimeConst &m, int sub, int lane) {
+// The conversions of one target for this thread's sixteen coefficients, into sm (at I::a).  Four coefficients at a time in a rolled loop:
+// the constants are fetched four times instead of held, and the straight-line code stays small (warps of a CTA work on
+// different targets, so long code is fetched again and again).
+//
+// On the FP64 pipe: y = y0 + y1 * 2^30 as two doubles, sums a0 of y * d0 and a1 of y * d1 (both exact: below 2^53, and below 2^53
+// units of 2^21), remainder of a1 + a0.  Sixteen fused multiply-adds and eight conversions for four sources, 58 FP64 cycles per warp
+// coefficient; the integer sums take 100 on the integer pipes.
+template <int COLS>
+__device__ __forceinline__ void convert_target_fp(u64 *sm, const u64 *ysm, const double (*__restrict__ cst)[4], int ns, const PrimeConst &m, int sub, int lane) {
     using I = StripIndex<COLS>;
-    const int ns = NS > 0 ? NS : ns_rt;
-    uint4 k[NS > 0 ? NS : 1];
-    if (NS > 0) {
+    const double qinv = m.q_inv_f, qd = (double)m.q;
+#pragma unroll 1
+    for (int e0 = 0; e0 < 16; e0 += 4) {
+        double a0[4], a1[4];
 #pragma unroll
-        for (int s = 0; s < NS; ++s) k[s] = __ldg(cst + s);
+        for (int u = 0; u < 4; ++u) { a0[u] = 0.0; a1[u] = 0.0; }
+#pragma unroll 2
+        for (int s = 0; s < ns; ++s) {
+            const double2 k0 = __ldg(reinterpret_cast<const double2 *>(cst[s])), k1 = __ldg(reinterpret_cast<const double2 *>(cst[s]) + 1);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
+                const double y0 = __hiloint2double(0x43300000, (int)(u32)y) - kTwo52, y1 = __hiloint2double(0x43300000, (int)(u32)(y >> 32)) - kTwo52;
+                a0[u] = __fma_rn(y0, k0.x, a0[u]); a1[u] = __fma_rn(y0, k0.y, a1[u]);
+                a0[u] = __fma_rn(y1, k1.x, a0[u]); a1[u] = __fma_rn(y1, k1.y, a1[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const double qh = __fma_rn(a1[u], qinv, __fma_rn(a0[u], qinv, kMagic)) - kMagic;
+            sm[I::a(e0 + u, sub, lane)] = (u64)__double_as_longlong(__fma_rn(-qh, qd, a1[u]) + a0[u]); // within 1.1 q of zero
+        }
     }
-    if (m.small) {
-        const SmallFinish f = small_finish(m);
+}
+template <int COLS>
+__device__ __forceinline__ void convert_target_small(u64 *sm, const u64 *ysm, const uint4 *__restrict__ cst, int ns, const PrimeConst &m, int sub, int lane) {
+    using I = StripIndex<COLS>;
+    const SmallFinish f = small_finish(m);
+#pragma unroll 1
+    for (int e0 = 0; e0 < 16; e0 += 4) {
+        u64 a0[4], a1[4];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            u64 a0 = 0, a1 = 0;
+        for (int u = 0; u < 4; ++u) { a0[u] = 0; a1[u] = 0; }
+#pragma unroll 1
+        for (int s = 0; s < ns; ++s) {
+            const uint4 c = __ldg(cst + s);
 #pragma unroll
-            for (int s = 0; s < ns; ++s) {
-                const uint4 c = NS > 0 ? k[s] : __ldg(cst + s);
-                const u64 y = ysm[s * I::kWords + I::a(e, sub, lane)];
-                a0 = mad_wide((u32)y, c.x, a0); a1 = mad_wide((u32)y, c.y, a1);
-                a0 = mad_wide((u32)(y >> 32), c.z, a0); a1 = mad_wide((u32)(y >> 32), c.w, a1);
+            for (int u = 0; u < 4; ++u) {
+                const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
+                a0[u] = mad_wide((u32)y, c.x, a0[u]); a1[u] = mad_wide((u32)y, c.y, a1[u]);
+                a0[u] = mad_wide((u32)(y >> 32), c.z, a0[u]); a1[u] = mad_wide((u32)(y >> 32), c.w, a1[u]);
             }
-            v[e] = (u64)__double_as_longlong(finish_small(a0, a1, f));
         }
-    } else {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            u64 a0 = 0, a1 = 0, a2 = 0;
+        for (int u = 0; u < 4; ++u) sm[I::a(e0 + u, sub, lane)] = (u64)__double_as_longlong(finish_small(a0[u], a1[u], f));
+    }
+}
+template <int COLS>
+__device__ __forceinline__ void convert_target_wide(u64 *sm, const u64 *ysm, const uint4 *__restrict__ cst, int ns, const PrimeConst &m, int sub, int lane) {
+    using I = StripIndex<COLS>;
+#pragma unroll 1
+    for (int e0 = 0; e0 < 16; e0 += 4) {
+        u64 a0[4], a1[4], a2[4];
 #pragma unroll
-            for (int s = 0; s < ns; ++s) {
-                const uint4 c = NS > 0 ? k[s] : __ldg(cst + s);
-                const u64 y = ysm[s * I::kWords + I::a(e, sub, lane)];
-                a0 = mad_wide((u32)y, c.x, a0); a1 = mad_wide((u32)y, c.y, a1);
-                a1 = mad_wide((u32)(y >> 32), c.x, a1); a2 = mad_wide((u32)(y >> 32), c.y, a2);
+        for (int u = 0; u < 4; ++u) { a0[u] = 0; a1[u] = 0; a2[u] = 0; }
+#pragma unroll 2
+        for (int s = 0; s < ns; ++s) {
+            const uint4 c = __ldg(cst + s);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
+                a0[u] = mad_wide((u32)y, c.x, a0[u]); a1[u] = mad_wide((u32)y, c.y, a1[u]);
+                a1[u] = mad_wide((u32)(y >> 32), c.x, a1[u]); a2[u] = mad_wide((u32)(y >> 32), c.y, a2[u]);
             }
-            v[e] = finish_wide(a0, a1, a2, m);
         }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) sm[I::a(e0 + u, sub, lane)] = finish_wide(a0[u], a1[u], a2[u], m);
     }
 }
 
 // src: half-inverse limbs (after the inverse row pass), instance b at src + b * src_outer; dst: half-forward limbs.
 // grid = (256 / COLS, plans, instances).  Dynamic shared memory: (largest ns + G) strips.
-template <int COLS, int G>
-__global__ void __launch_bounds__(COLS * 16 * G, 512 / (COLS * 16 * G)) conv_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, const ConvPlan *__restrict__ plans,
+template <int COLS, int G, int MINB>
+__global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, const ConvPlan *__restrict__ plans,
                                                                          const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     extern __shared__ __align__(16) u64 strips[];
+    __shared__ int next, turn[G];
     using I = StripIndex<COLS>;
+    if (threadIdx.x == 0) next = 0;
     const ConvPlan *pl = plans + blockIdx.y;
     const int ns = pl->ns, nt = pl->nt;
     const int g = threadIdx.x / (COLS * 16), r = threadIdx.x % (COLS * 16), lane = r % COLS, sub = r / COLS;
@@ -216,25 +246,28 @@ __global__ void __launch_bounds__(COLS * 16 * G, 512 / (COLS * 16 * G)) conv_col
     }
     __syncthreads();
     u64 *ex = strips + (ns + g) * I::kWords;
-    for (int t = g; t < nt; t += G) {
+    while (true) { // the groups take targets from a common counter
+        group_sync<COLS * 16>(g); // the strip of the previous target has been read
+        if (r == 0) turn[g] = atomicAdd(&next, 1);
+        group_sync<COLS * 16>(g);
+        const int k = turn[g];
+        if (k >= nt) break;
+        const int t = pl->order[k];
         const int pi = pl->dst_prime[t];
         const PrimeConst m = pc[pi];
         const uint4 *cst = pl->c[t];
-        switch (ns) {
-        case 1: convert_target<1, COLS>(v, strips, cst, ns, m, sub, lane); break;
-        case 2: convert_target<2, COLS>(v, strips, cst, ns, m, sub, lane); break;
-        case 3: convert_target<3, COLS>(v, strips, cst, ns, m, sub, lane); break;
-        case 4: convert_target<4, COLS>(v, strips, cst, ns, m, sub, lane); break;
-        default: convert_target<0, COLS>(v, strips, cst, ns, m, sub, lane); break;
-        }
-        strip_forward<COLS>(v, dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)pi * Ntt16Layout::kEntries, g, sub, lane);
+        const bool fp = pl->fp[t];
+        if (fp) convert_target_fp<COLS>(ex, strips, pl->d[t], ns, m, sub, lane);
+        else if (m.small) convert_target_small<COLS>(ex, strips, cst, ns, m, sub, lane);
+        else convert_target_wide<COLS>(ex, strips, cst, ns, m, sub, lane);
+        strip_forward<COLS>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)pi * Ntt16Layout::kEntries, g, sub, lane);
     }
 }
 
 // Rescale: one source limb (prime index `level`), lifted centred to the limbs 0 .. level - 1.
 // grid = (256 / COLS, instances); dynamic shared memory: 1 + G strips.
-template <int COLS, int G>
-__global__ void __launch_bounds__(COLS * 16 * G, 512 / (COLS * 16 * G)) lift_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int level,
+template <int COLS, int G, int MINB>
+__global__ void __launch_bounds__(COLS * 16 * G, MINB) lift_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int level,
                                                                          const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     extern __shared__ __align__(16) u64 strips[];
     using I = StripIndex<COLS>;
@@ -255,15 +288,17 @@ __global__ void __launch_bounds__(COLS * 16 * G, 512 / (COLS * 16 * G)) lift_col
     u64 *dp = dst + (size_t)blockIdx.y * dst_outer + col, *ex = strips + (1 + g) * I::kWords;
     for (int t = g; t < level; t += G) {
         const PrimeConst m = pc[t];
-#pragma unroll
+        group_sync<COLS * 16>(g); // the strip of the previous target has been read
+#pragma unroll 4
         for (int e = 0; e < 16; ++e) {
             const i64 y = (i64)strips[I::a(e, sub, lane)];
-            if (m.small && src_small && (ql >> 1) < 2 * m.q) v[e] = (u64)__double_as_longlong(__longlong_as_double(y + 0x4338000000000000ll) - kMagic); // within 2q of zero
-            else if (m.small) v[e] = (u64)__double_as_longlong(u52_to_double(reduce_i64(y, m)));
-            else if ((ql >> 1) < m.q) v[e] = y < 0 ? (u64)(y + (i64)m.q) : (u64)y;
-            else v[e] = reduce_i64(y, m);
+            u64 &w = ex[I::a(e, sub, lane)];
+            if (m.small && src_small && (ql >> 1) < 2 * m.q) w = (u64)__double_as_longlong(__longlong_as_double(y + 0x4338000000000000ll) - kMagic); // within 2q of zero
+            else if (m.small) w = (u64)__double_as_longlong(u52_to_double(reduce_i64(y, m)));
+            else if ((ql >> 1) < m.q) w = y < 0 ? (u64)(y + (i64)m.q) : (u64)y;
+            else w = reduce_i64(y, m);
         }
-        strip_forward<COLS>(v, dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)t * Ntt16Layout::kEntries, g, sub, lane);
+        strip_forward<COLS>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)t * Ntt16Layout::kEntries, g, sub, lane);
     }
 }
 
@@ -299,6 +334,11 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
     }
     u64 *o = f.out + (size_t)b * f.out_outer + ((size_t)p * n + l) * kN16 + pos;
     u64 *smr = sm + rl * kRowStride;
+    if (tid == 0) { // what the last step reads is on its way while the transform runs
+        const size_t first = (size_t)blockIdx.x * 4096;
+        prefetch_l2(f.x + (size_t)bp * f.x_outer + limb + first, 4096 * 8);
+        if (ap) prefetch_l2(ap + (g ? ntt_perm((u32)first, g, 16) & ~4095u : (u32)first), 4096 * 8);
+    }
     if (m.small) {
         const DsConst c = ds_const(m);
         const double *td = reinterpret_cast<const double *>(tp);
@@ -354,14 +394,14 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
         for (int e = 0; e < 16; ++e) {
             u64 r = mul_shoup4(x[e] + c.q8 - smr[e * 17 + clo], sw, ss, c.nq); // below 4q
             if (ap) r += ap[g ? ntt_perm((u32)(pos + e * 16), g, 16) : (u32)(pos + e * 16)];
-            o[e * 16] = canon_q(r, c.q, c.sh);
+            o[e * 16] = canon_q(r, c.q, c.f);
         }
     }
 }
 
 // Single passes, for the fused sequences.  A grid of one or two CTAs per SM takes the kernels that may use 128 registers and
 // fetch the twiddles of the second round (which nobody shares) before anything else, under the tail of the predecessor.
-constexpr int kSmallGrid = 2 * 148;
+static const int kSmallGrid = getenv("HB_SG") ? atoi(getenv("HB_SG")) : 2 * 148;
 inline void launch_inv_rows16(cudaStream_t st, const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
     launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_inv_rows<2> : ntt16v2_inv_rows<4>, dim3(16, count), 256, 0, src, LimbAddr16{src_outer}, dst, LimbAddr16{dst_outer}, map, pc, tb);
 }

@@ -279,11 +279,26 @@ void fill_conv(const HostCtx &h, ConvPlan &p, const std::vector<int> &src, const
     for (size_t t = 0; t < dst.size(); ++t) {
         const u64 q = h.q[dst[t]];
         p.dst_prime[t] = (unsigned char)dst[t];
+        double low = 0, high = 0; // largest sums of the FP64 form, in units of 1 and 2^21
         for (size_t s = 0; s < src.size(); ++s) {
             const u64 v = hat(s, q), v30 = hbhost::mulmod(v, ((u64)1 << 30) % q, q), m26 = ((u64)1 << 26) - 1, m30 = ((u64)1 << 30) - 1;
+            if (!(q >> 44)) {
+                auto split = [&](u64 w, double *d) { // |w - q * [w > q / 2]| = d[1] + d[0]
+                    const i64 c = w > q / 2 ? (i64)w - (i64)q : (i64)w, hi = (c + ((i64)1 << 20)) >> 21;
+                    d[0] = (double)(c - hi * ((i64)1 << 21)); d[1] = (double)(hi * ((i64)1 << 21));
+                };
+                split(v, p.d[t][s]); split(v30, p.d[t][s] + 2);
+            }
             p.c[t][s] = (q >> 44) ? make_uint4((u32)(v & m30), (u32)(v >> 30), 0, 0) : make_uint4((u32)(v & m26), (u32)(v >> 26), (u32)(v30 & m26), (u32)(v30 >> 26));
+            const double y0 = 0x1p30, y1 = (double)((h.q[src[s]] >> 30) + 1);
+            low += y0 * std::fabs(p.d[t][s][0]) + y1 * std::fabs(p.d[t][s][2]);
+            high += (y0 * std::fabs(p.d[t][s][1]) + y1 * std::fabs(p.d[t][s][3])) * 0x1p-21;
         }
+        // a1 - qh * q is formed exactly when |a0| + 2q stays below 2^53; the quotient must be exact to well below one
+        p.order[t] = (unsigned char)t;
+        p.fp[t] = !(q >> 44) && src.size() <= 4 && low + 2.0 * (double)q < 0x1p53 && high < 0x1p53;
     }
+    std::stable_sort(p.order, p.order + p.nt, [&](int x, int y) { return (h.q[p.dst_prime[x]] >> 44) && !(h.q[p.dst_prime[y]] >> 44); });
 }
 const ConvPlan *get_conv_plans(hb_ctx *c, int level) {
     auto it = c->conv_plans.find(level);
@@ -332,33 +347,55 @@ template <int COLS> size_t strip_bytes(int strips) { return (size_t)strips * Str
 void conv_opt_in(hb_ctx *c) {
     if (c->smem_opt_in_conv) return;
     auto allow = [](auto *kernel, size_t bytes) { CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); };
-    allow(conv_cols<8, 2>, strip_bytes<8>(10)); allow(conv_cols<4, 4>, strip_bytes<4>(12)); allow(conv_cols<4, 8>, strip_bytes<4>(16));
-    allow(lift_cols<8, 2>, strip_bytes<8>(3)); allow(lift_cols<4, 4>, strip_bytes<4>(5)); allow(lift_cols<4, 8>, strip_bytes<4>(9));
+    allow(conv_cols<8, 2, 2>, strip_bytes<8>(10)); allow(conv_cols<8, 4, 1>, strip_bytes<8>(12)); allow(conv_cols<4, 4, 3>, strip_bytes<4>(12));
+    allow(conv_cols<4, 8, 1>, strip_bytes<4>(16)); allow(conv_cols<4, 8, 2>, strip_bytes<4>(16)); allow(conv_cols<4, 4, 2>, strip_bytes<4>(12));
+    allow(lift_cols<8, 2, 2>, strip_bytes<8>(3)); allow(lift_cols<4, 4, 2>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1>, strip_bytes<4>(9));
+    allow(lift_cols<4, 4, 4>, strip_bytes<4>(5)); allow(lift_cols<8, 2, 4>, strip_bytes<8>(3));
     c->smem_opt_in_conv = true;
 }
-// Strip width and groups of a launch over `units` (polynomial, conversion) pairs: wide strips when they fill the GPU; otherwise narrow
-// ones with more groups, so that more sources and targets of a unit are worked on at once.
-enum StripShape { kStrip8x2, kStrip4x4, kStrip4x8 };
-StripShape strip_shape(int units) {
-    return units * 64 <= 148 ? kStrip4x8 : units * 64 <= 2 * 148 ? kStrip4x4 : kStrip8x2;
+// Strip width and groups of a launch over `units` (polynomial, conversion) pairs.  At most two units: narrow strips and many groups, so that
+// all sources and all targets of a unit are worked on at once.  Otherwise strips of eight columns, in the shape that fills the
+// last wave better: 32 * units CTAs of four groups, one per SM, or of two groups, two per SM and half as fast each.
+enum StripShape { kStrip8x2, kStrip8x4, kStrip4x4, kStrip4x8 };
+StripShape conv_shape(int units) {
+    if (const char *e = getenv("HB_STRIP")) return (StripShape)atoi(e);
+    if (units <= 2) return kStrip4x8;
+    return (units * 32 + 147) / 148 <= 1.9 * ((units * 32 + 295) / 296) ? kStrip8x4 : kStrip8x2;
 }
+StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : kStrip8x2; }
 // `plans` conversions (the largest with max_ns sources) of `instances` polynomials in one launch
 void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int instances) {
     conv_opt_in(c);
     LAUNCH(c);
-    const StripShape s = strip_shape(instances * count);
-    if (s == kStrip8x2) launch_pdl(c->st, conv_cols<8, 2>, dim3(32, count, instances), 256, strip_bytes<8>(max_ns + 2), src, so, dst, dof, plans, c->pc, c->tb.t16);
-    else if (s == kStrip4x4) launch_pdl(c->st, conv_cols<4, 4>, dim3(64, count, instances), 256, strip_bytes<4>(max_ns + 4), src, so, dst, dof, plans, c->pc, c->tb.t16);
-    else launch_pdl(c->st, conv_cols<4, 8>, dim3(64, count, instances), 512, strip_bytes<4>(max_ns + 8), src, so, dst, dof, plans, c->pc, c->tb.t16);
+    auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
+        launch_pdl(c->st, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
+    };
+    int sh = conv_shape(instances * count);
+    switch (sh) {
+    case 0: go(conv_cols<8, 2, 2>, 8, 2, strip_bytes<8>(max_ns + 2)); break;
+    case 1: go(conv_cols<8, 4, 1>, 8, 4, strip_bytes<8>(max_ns + 4)); break;
+    case 2: go(conv_cols<4, 4, 3>, 4, 4, strip_bytes<4>(max_ns + 4)); break;
+    case 3: go(conv_cols<4, 8, 1>, 4, 8, strip_bytes<4>(max_ns + 8)); break;
+    case 4: go(conv_cols<4, 8, 2>, 4, 8, strip_bytes<4>(max_ns + 8)); break;
+    case 5: go(conv_cols<4, 4, 2>, 4, 4, strip_bytes<4>(max_ns + 4)); break;
+    }
 }
 // half-inverse limbs of prime `level` (one per instance) -> half-forward lifts to the limbs below
 void launch_lift(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int level, int instances) {
     conv_opt_in(c);
     LAUNCH(c);
-    const StripShape s = strip_shape(instances);
-    if (s == kStrip8x2) launch_pdl(c->st, lift_cols<8, 2>, dim3(32, instances), 256, strip_bytes<8>(3), src, so, dst, dof, level, c->pc, c->tb.t16);
-    else if (s == kStrip4x4) launch_pdl(c->st, lift_cols<4, 4>, dim3(64, instances), 256, strip_bytes<4>(5), src, so, dst, dof, level, c->pc, c->tb.t16);
-    else launch_pdl(c->st, lift_cols<4, 8>, dim3(64, instances), 512, strip_bytes<4>(9), src, so, dst, dof, level, c->pc, c->tb.t16);
+    auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
+        launch_pdl(c->st, kernel, dim3(256 / cols, instances), cols * 16 * groups, smem, src, so, dst, dof, level, c->pc, c->tb.t16);
+    };
+    int sh = lift_shape(instances);
+    if (const char *e = getenv("HB_LIFT")) sh = atoi(e);
+    switch (sh) {
+    case 0: go(lift_cols<8, 2, 2>, 8, 2, strip_bytes<8>(3)); break;
+    case 1: go(lift_cols<8, 2, 4>, 8, 2, strip_bytes<8>(3)); break;
+    case 2: go(lift_cols<4, 4, 2>, 4, 4, strip_bytes<4>(5)); break;
+    case 3: go(lift_cols<4, 8, 1>, 4, 8, strip_bytes<4>(9)); break;
+    case 4: go(lift_cols<4, 4, 4>, 4, 4, strip_bytes<4>(5)); break;
+    }
 }
 void inv_rows(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int count, const LimbMap &m) {
     LAUNCH(c), launch_inv_rows16(c->st, src, so, dst, dof, count, m, c->pc, c->tb.t16);
@@ -968,7 +1005,8 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             int bits = 0;
             while (bits < 64 && (q >> bits)) ++bits;
             p.fold_shift = bits > 32 ? (u32)(bits - 32) : 0;
-            if (!p.fp && (((u64)1 << bits) - q) >> (bits - 12)) throw std::invalid_argument("prime too far below its power of two");
+            p.fold_d = p.fp ? 0 : (u32)(((u64)1 << bits) - q);
+            if (!p.fp && (((u64)1 << bits) - q) >> std::min(bits - 12, 32)) throw std::invalid_argument("prime too far below its power of two");
             const u64 below60 = q < ((u64)1 << 60) ? ((u64)1 << 60) - q : 0;
             p.d60 = below60 < ((u64)1 << 26) ? (u32)below60 : 0;
             std::vector<u64> f, fs, iv, ivs;

@@ -73,22 +73,6 @@ __global__ void k_mul_pt(u64 *__restrict__ out, const u64 *__restrict__ a, const
         out[off] = mul_mod_any(a[off], pt[(size_t)(li % map.n) * N + i], m);
     }
 }
-// out = a (.) pa + b (.) pb
-__global__ void k_mul2_add(u64 *__restrict__ out, const u64 *__restrict__ a, const u64 *__restrict__ pa, const u64 *__restrict__ b, const u64 *__restrict__ pb,
-                           const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N) {
-    const int li = blockIdx.y;
-#pragma unroll
-    for (int u_ = 0; u_ < kElems; ++u_) {
-        const int i = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
-        if (i >= N) break;
-        const PrimeConst m = pc[map.prime[li % map.n]];
-        const size_t off = (size_t)li * N + i;
-        const size_t po = (size_t)(li % map.n) * N + i;
-        Acc128 s; s.zero();
-        s.mad(a[off], pa[po]); s.mad(b[off], pb[po]);
-        out[off] = barrett128(s.hi, s.lo, m);
-    }
-}
 // tensor product, optional accumulation.  grid.y = batch * n; x, y: [groups][batch][2][n][N]; d: [batch][3][n][N]
 //   d[b] (+)= sum over the groups g of tensor(x[g][b], y[g][b])
 // (groups = 1 is the plain tensor product; several groups are several iterations of a product loop in one launch).
@@ -116,12 +100,13 @@ __global__ void k_tensor(u64 *d, const u64 *x, const u64 *y, int n, const __grid
             }
             r0 = reduce_fp(s0, m.q_inv_f, m.q); r1 = reduce_fp(s1, m.q_inv_f, m.q); r2 = reduce_fp(s2, m.q_inv_f, m.q);
         } else {
-            Acc128 s0, s1, s2; s0.zero(); s1.zero(); s2.zero();
+            PieceAcc s0, s1, s2; s0.zero(); s1.zero(); s2.zero();
             for (int g = 0; g < groups; ++g) {
+                if (g && g % 3 == 0) { s0.relax(m); s1.relax(m); s2.relax(m); }
                 const u64 b1 = x[g * gstride + x0], a1 = x[g * gstride + x1], b2 = y[g * gstride + x0], a2 = y[g * gstride + x1];
-                s0.mad(b1, b2); s2.mad(a1, a2); s1.mad(a1, b2); s1.mad(a2, b1);
+                s0.mac(b1, b2); s2.mac(a1, a2); s1.mac(a1, b2); s1.mac(a2, b1);
             }
-            r0 = barrett128(s0.hi, s0.lo, m); r1 = barrett128(s1.hi, s1.lo, m); r2 = barrett128(s2.hi, s2.lo, m);
+            r0 = s0.finish(m); r1 = s1.finish(m); r2 = s2.finish(m);
         }
         if (accumulate) { r0 = add_mod(r0, d[d0], m.q); r1 = add_mod(r1, d[d1], m.q); r2 = add_mod(r2, d[d2], m.q); }
         d[d0] = r0; d[d1] = r1; d[d2] = r2;
@@ -233,9 +218,12 @@ __global__ void k_last_prod(u64 *last, const __grid_constant__ TermList tl, int 
             for (int j = j0; j < j1; ++j) acc += mul_small_lazy(tl.a[j][ao], tl.p[j][po], m.q_inv_f, m.q);
             r = reduce_fp(acc, m.q_inv_f, m.q);
         } else {
-            Acc128 s; s.zero();
-            for (int j = j0; j < j1; ++j) s.mad(tl.a[j][ao], tl.p[j][po]);
-            r = barrett128(s.hi, s.lo, m);
+            PieceAcc s; s.zero();
+            for (int j = j0; j < j1; ++j) {
+                if (j > j0 && (j - j0) % 7 == 0) s.relax(m);
+                s.mac(tl.a[j][ao], tl.p[j][po]);
+            }
+            r = s.finish(m);
         }
         last[((size_t)g * gridDim.y + blockIdx.y) * N + x] = r;
     }
@@ -292,17 +280,21 @@ __global__ void k_prod_rescale_fin(u64 *out, const __grid_constant__ TermList tl
 #pragma unroll
         for (int u = 0; u < kElems; ++u) v[u] = reduce_fp(acc[u], m.q_inv_f, m.q);
     } else {
-        Acc128 s[kElems];
+        PieceAcc s[kElems];
 #pragma unroll
         for (int u = 0; u < kElems; ++u) s[u].zero();
 #pragma unroll 2
-        for (int j = first; j < first + tl.count; ++j) {
-            const u64 *a = tl.a[j] + ao, *p = tl.p[j] + po;
+        for (int j = 0; j < tl.count; ++j) {
+            const u64 *a = tl.a[first + j] + ao, *p = tl.p[first + j] + po;
+            if (j && j % 7 == 0) {
 #pragma unroll
-            for (int u = 0; u < kElems; ++u) s[u].mad(a[u * blockDim.x], p[u * blockDim.x]);
+                for (int u = 0; u < kElems; ++u) s[u].relax(m);
+            }
+#pragma unroll
+            for (int u = 0; u < kElems; ++u) s[u].mac(a[u * blockDim.x], p[u * blockDim.x]);
         }
 #pragma unroll
-        for (int u = 0; u < kElems; ++u) v[u] = barrett128(s[u].hi, s[u].lo, m);
+        for (int u = 0; u < kElems; ++u) v[u] = s[u].finish(m);
     }
     const u64 *tp = t + (size_t)w * N + x0;
     u64 *op = out + (size_t)w * N + x0;
@@ -479,8 +471,7 @@ __device__ __forceinline__ void modup_body(u64 *__restrict__ dt, const u64 *__re
             PieceAcc s; s.zero(); // at most 8 sources
 #pragma unroll
             for (int k = 0; k < NS; ++k) s.mac(y[k], pl->hat_mod[dg][k][j]);
-            PrimeConst mm; mm.q = m->q; mm.mu_hi = m->mu_hi; mm.mu_lo = m->mu_lo;
-            *o = s.finish(mm);
+            *o = s.finish(*m);
         }
         o += N;
     }
@@ -545,7 +536,7 @@ __global__ void k_ks_inner(u64 *acc, const __grid_constant__ SwitchList sl, int 
 #pragma unroll
         for (int u = 0; u < kElems; ++u) { r0[u] = canon_fp64(d0[u], m.q_inv_f, qd); r1[u] = canon_fp64(d1[u], m.q_inv_f, qd); }
     } else {
-        Acc128 s0[kElems], s1[kElems];
+        PieceAcc s0[kElems], s1[kElems];
 #pragma unroll
         for (int u = 0; u < kElems; ++u) { s0[u].zero(); s1[u].zero(); }
         for (int dg = 0; dg < nd; ++dg) {
@@ -555,12 +546,12 @@ __global__ void k_ks_inner(u64 *acc, const __grid_constant__ SwitchList sl, int 
 #pragma unroll
             for (int u = 0; u < kElems; ++u) {
                 const u64 v = sp[src[u]];
-                s0[u].mad(v, k0[u * blockDim.x]);
-                s1[u].mad(v, k0[kpoly + u * blockDim.x]);
+                s0[u].mac(v, k0[u * blockDim.x]);
+                s1[u].mac(v, k0[kpoly + u * blockDim.x]);
             }
         }
 #pragma unroll
-        for (int u = 0; u < kElems; ++u) { r0[u] = barrett128(s0[u].hi, s0[u].lo, m); r1[u] = barrett128(s1[u].hi, s1[u].lo, m); }
+        for (int u = 0; u < kElems; ++u) { r0[u] = s0[u].finish(m); r1[u] = s1[u].finish(m); }
     }
     u64 *o0 = acc + (((size_t)ob * 2) * ne + j) * N + x0, *o1 = o0 + (size_t)ne * N;
 #pragma unroll
@@ -597,8 +588,7 @@ __device__ __forceinline__ void moddown_conv_body(u64 *__restrict__ t, const u64
             PieceAcc s; s.zero();
 #pragma unroll
             for (int k = 0; k < K; ++k) s.mac(y[k], pl->p_hat_mod[k][l]);
-            PrimeConst mm; mm.q = pc[l].q; mm.mu_hi = pc[l].mu_hi; mm.mu_lo = pc[l].mu_lo;
-            *o = s.finish(mm);
+            *o = s.finish(pc[l]);
         }
         o += N;
     }
@@ -680,10 +670,11 @@ __global__ void k_ks_inner_sum(u64 *__restrict__ acc, const __grid_constant__ Ro
         }
 #pragma unroll
         for (int u = 0; u < kElems; ++u) { r0[u] = canon_fp64(d0[u], m.q_inv_f, qd); r1[u] = canon_fp64(d1[u], m.q_inv_f, qd); }
-    } else {   // 64 products below 2^120 fit the 128-bit accumulator
-        Acc128 s0[kElems], s1[kElems];
+    } else {
+        PieceAcc s0[kElems], s1[kElems];
 #pragma unroll
         for (int u = 0; u < kElems; ++u) { s0[u].zero(); s1[u].zero(); }
+        int held = 0; // products in the accumulators
         for (int t = 0; t < tl.count; ++t) {
             u32 src[kElems];
 #pragma unroll
@@ -692,19 +683,24 @@ __global__ void k_ks_inner_sum(u64 *__restrict__ acc, const __grid_constant__ Ro
             const u64 *dbase = tl.t[t].dt + (size_t)b * pl->dt_count * N;
             const u64 *kbase = tl.t[t].key + (size_t)pj * N + x0;
             for (int dg = 0; dg < nd; ++dg) {
+                if (++held == 8) {
+                    held = 1;
+#pragma unroll
+                    for (int u = 0; u < kElems; ++u) { s0[u].relax(m); s1[u].relax(m); }
+                }
                 const int en = pl->dt_entry[dg][j];
                 const u64 *sp = en < 0 ? abase : dbase + (size_t)en * N;
                 const u64 *k0 = kbase + (size_t)dg * 2 * kpoly;
 #pragma unroll
                 for (int u = 0; u < kElems; ++u) {
                     const u64 v = sp[src[u]];
-                    s0[u].mad(v, k0[u * blockDim.x]);
-                    s1[u].mad(v, k0[kpoly + u * blockDim.x]);
+                    s0[u].mac(v, k0[u * blockDim.x]);
+                    s1[u].mac(v, k0[kpoly + u * blockDim.x]);
                 }
             }
         }
 #pragma unroll
-        for (int u = 0; u < kElems; ++u) { r0[u] = barrett128(s0[u].hi, s0[u].lo, m); r1[u] = barrett128(s1[u].hi, s1[u].lo, m); }
+        for (int u = 0; u < kElems; ++u) { r0[u] = s0[u].finish(m); r1[u] = s1[u].finish(m); }
     }
     u64 *o0 = acc + (((size_t)b * 2) * ne + j) * N + x0, *o1 = o0 + (size_t)ne * N;
 #pragma unroll
@@ -791,7 +787,7 @@ __global__ void k_ks_inner_pair(u64 *__restrict__ E, const u64 *__restrict__ c0,
 #pragma unroll
             for (int u = 0; u < kElems; ++u) { r0[u] = reduce_fp(r0[u], m.q_inv_f, m.q); r1[u] = reduce_fp(r1[u], m.q_inv_f, m.q); }
         } else {
-            Acc128 s0[kElems], s1[kElems];
+            PieceAcc s0[kElems], s1[kElems];
 #pragma unroll
             for (int u = 0; u < kElems; ++u) { s0[u].zero(); s1[u].zero(); }
             for (int dg = 0; dg < nd; ++dg) {
@@ -801,12 +797,12 @@ __global__ void k_ks_inner_pair(u64 *__restrict__ E, const u64 *__restrict__ c0,
 #pragma unroll
                 for (int u = 0; u < kElems; ++u) {
                     const u64 v = sp[src[u]];
-                    s0[u].mad(v, k0[u * blockDim.x]);
-                    s1[u].mad(v, k0[kpoly + u * blockDim.x]);
+                    s0[u].mac(v, k0[u * blockDim.x]);
+                    s1[u].mac(v, k0[kpoly + u * blockDim.x]);
                 }
             }
 #pragma unroll
-            for (int u = 0; u < kElems; ++u) { r0[u] = barrett128(s0[u].hi, s0[u].lo, m); r1[u] = barrett128(s1[u].hi, s1[u].lo, m); }
+            for (int u = 0; u < kElems; ++u) { r0[u] = s0[u].finish(m); r1[u] = s1[u].finish(m); }
         }
         const u64 *mk = rp.mask[r] + (size_t)j * N + x0, *mk2 = rp.mask[1] + (size_t)j * N + x0;
 #pragma unroll
@@ -913,33 +909,40 @@ __global__ void __launch_bounds__(256, EL == 2 ? 3 : 2) k_ks_inner_mk(u64 *__res
 #pragma unroll
         for (int u = 0; u < EL; ++u) { r0[u] = canon_fp64(d0[u], m.q_inv_f, qd); r1[u] = canon_fp64(d1[u], m.q_inv_f, qd); }
     } else {
-        Acc128 s0[EL], s1[EL];
+        PieceAcc s0[EL], s1[EL];
 #pragma unroll
         for (int u = 0; u < EL; ++u) { s0[u].zero(); s1[u].zero(); }
+        int held = 0; // products in the accumulators
         for (int r = 0; r < mr.count; ++r) {
             u32 src[EL];
 #pragma unroll
             for (int u = 0; u < EL; ++u) src[u] = ntt_perm(x0 + u * blockDim.x, mr.g[r], logn);
             const u64 *kbase = mr.mkey[r] + (size_t)j * N + x0;
             for (int dg = 0; dg < nd; ++dg) {
+                if (++held >= 8) {
+                    held = 1;
+#pragma unroll
+                    for (int u = 0; u < EL; ++u) { s0[u].relax(m); s1[u].relax(m); }
+                }
                 const int en = pl->dt_entry[dg][j];
                 const u64 *sp = en < 0 ? abase : dbase + (size_t)en * N;
                 const u64 *k0 = kbase + (size_t)dg * 2 * kpoly;
 #pragma unroll
                 for (int u = 0; u < EL; ++u) {
                     const u64 v = sp[src[u]];
-                    s0[u].mad(v, k0[u * blockDim.x]);
-                    s1[u].mad(v, k0[kpoly + u * blockDim.x]);
+                    s0[u].mac(v, k0[u * blockDim.x]);
+                    s1[u].mac(v, k0[kpoly + u * blockDim.x]);
                 }
             }
             if (j < n) {
                 const u64 *pmb = mr.pm[r] + (size_t)j * N + x0;
 #pragma unroll
-                for (int u = 0; u < EL; ++u) s0[u].mad(cbase[src[u]], pmb[u * blockDim.x]);
+                for (int u = 0; u < EL; ++u) s0[u].mac(cbase[src[u]], pmb[u * blockDim.x]);
+                ++held;
             }
         }
 #pragma unroll
-        for (int u = 0; u < EL; ++u) { r0[u] = barrett128(s0[u].hi, s0[u].lo, m); r1[u] = barrett128(s1[u].hi, s1[u].lo, m); }
+        for (int u = 0; u < EL; ++u) { r0[u] = s0[u].finish(m); r1[u] = s1[u].finish(m); }
     }
     u64 *o0 = E + (((size_t)ob * 2) * ne + j) * N + x0, *o1 = o0 + (size_t)ne * N;
 #pragma unroll
@@ -1046,7 +1049,7 @@ __global__ void __launch_bounds__(256) k_ks_inner_mkb(u64 *__restrict__ E, const
 #pragma unroll
             for (int e = 0; e < EL; ++e) { r0[u][e] = canon_fp64(d0[u][e], m.q_inv_f, qd); r1[u][e] = canon_fp64(d1[u][e], m.q_inv_f, qd); }
     } else {
-        Acc128 s0[M][EL], s1[M][EL];
+        PieceAcc s0[M][EL], s1[M][EL];
 #pragma unroll
         for (int u = 0; u < M; ++u)
 #pragma unroll
@@ -1061,12 +1064,14 @@ __global__ void __launch_bounds__(256) k_ks_inner_mkb(u64 *__restrict__ E, const
 #pragma unroll
                 for (int e = 0; e < EL; ++e) {
                     const u64 ka = kp[e * 256], kb = kp[T + e * 256];
+                    const u32 ka0 = (u32)ka & 0x3FFFFFFFu, ka1 = (u32)(ka >> 30), kb0 = (u32)kb & 0x3FFFFFFFu, kb1 = (u32)(kb >> 30);
 #pragma unroll
                     for (int u = 0; u < M; ++u)
                         if (u < nm) {
                             const u64 v = sp[(size_t)u * count * nsrc * T + li[e]];
-                            s0[u][e].mad(v, ka);
-                            s1[u][e].mad(v, kb);
+                            const u32 v0 = (u32)v & 0x3FFFFFFFu, v1 = (u32)(v >> 30);
+                            s0[u][e].mac(v0, v1, ka0, ka1);
+                            s1[u][e].mac(v0, v1, kb0, kb1);
                         }
                 }
             }
@@ -1077,14 +1082,14 @@ __global__ void __launch_bounds__(256) k_ks_inner_mkb(u64 *__restrict__ E, const
                     const u64 pmv = pmb[(size_t)r * T + e * 256 + tid];
 #pragma unroll
                     for (int u = 0; u < M; ++u)
-                        if (u < nm) s0[u][e].mad(sp[(size_t)u * count * nsrc * T + li[e]], pmv);
+                        if (u < nm) s0[u][e].mac(sp[(size_t)u * count * nsrc * T + li[e]], pmv);
                 }
             }
         }
 #pragma unroll
         for (int u = 0; u < M; ++u)
 #pragma unroll
-            for (int e = 0; e < EL; ++e) { r0[u][e] = barrett128(s0[u][e].hi, s0[u][e].lo, m); r1[u][e] = barrett128(s1[u][e].hi, s1[u][e].lo, m); }
+            for (int e = 0; e < EL; ++e) { r0[u][e] = s0[u][e].finish(m); r1[u][e] = s1[u][e].finish(m); }
     }
     const size_t kpoly = (size_t)ne * N;
     u64 *o0 = E + (((size_t)(grp * batch + b0) * 2) * ne + j) * N + tile0 + tid;
@@ -1129,8 +1134,7 @@ __device__ __forceinline__ void div_conv_body(u64 *__restrict__ t, const u64 *__
             PieceAcc s; s.zero();
 #pragma unroll
             for (int k = 0; k < NS; ++k) s.mac(y[k], dv->hat_mod[k][l]);
-            PrimeConst mm; mm.q = pc[l].q; mm.mu_hi = pc[l].mu_hi; mm.mu_lo = pc[l].mu_lo;
-            *o = s.finish(mm);
+            *o = s.finish(pc[l]);
         }
         o += N;
     }
@@ -1255,7 +1259,7 @@ __global__ void k_keygen(u64 *__restrict__ b, const u64 *__restrict__ a, const u
 // ---------------- fused plaintext-matmul accumulate ----------------
 // out[p][l][i] = sum_{b < bcount} sum_{k < kcount} pre[k * btotal + b0 + b][p][l][i] * pt_b[l][perm_{g_k}(i)]
 // (scale Delta^2, no rescale).  Shifted copies are stored k-major; the sum over b adds the partial products
-// of several K-groups in the same pass.  grid = (N/256, 2*n).  The 128-bit accumulator is folded every 64 terms.
+// of several K-groups in the same pass.  grid = (N/256, 2*n).  The accumulators are reduced every few terms.
 struct PtList { const u64 *p[16]; };
 __global__ void k_matmul_acc(u64 *__restrict__ out, const u64 *__restrict__ pre, int kcount, int btotal, int b0, int bcount, const __grid_constant__ PtList pts, const u32 *__restrict__ gal,
                              int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int logn, int N) {
@@ -1295,10 +1299,10 @@ __global__ void k_matmul_acc(u64 *__restrict__ out, const u64 *__restrict__ pre,
 #pragma unroll
         for (int u = 0; u < kElems; ++u) total[u] = add_mod(total[u], reduce_fp(acc[u], m.q_inv_f, m.q), m.q);
     } else {
-        Acc128 s[kElems];
+        PieceAcc s[kElems];
 #pragma unroll
         for (int u = 0; u < kElems; ++u) s[u].zero();
-        int terms = 0;
+        int held = 0; // products in the accumulators
         for (int k = 0; k < kcount; ++k) {
             const u32 g = __ldg(gal + k);
             u32 src[kElems];
@@ -1307,18 +1311,17 @@ __global__ void k_matmul_acc(u64 *__restrict__ out, const u64 *__restrict__ pre,
 #pragma unroll 2
             for (int b = 0; b < bcount; ++b) {
                 const u64 *a = pbase + ((size_t)k * btotal + b0 + b) * estride, *w = pts.p[b] + (size_t)l * N;
+                if (++held == 8) {
+                    held = 1;
 #pragma unroll
-                for (int u = 0; u < kElems; ++u) s[u].mad(a[u * blockDim.x], w[src[u]]);
-            }
-            terms += bcount;
-            if (terms >= 48) { // products below 2^120: the 128-bit accumulator holds 256 of them
+                    for (int u = 0; u < kElems; ++u) s[u].relax(m);
+                }
 #pragma unroll
-                for (int u = 0; u < kElems; ++u) { total[u] = add_mod(total[u], barrett128(s[u].hi, s[u].lo, m), m.q); s[u].zero(); }
-                terms = 0;
+                for (int u = 0; u < kElems; ++u) s[u].mac(a[u * blockDim.x], w[src[u]]);
             }
         }
 #pragma unroll
-        for (int u = 0; u < kElems; ++u) total[u] = add_mod(total[u], barrett128(s[u].hi, s[u].lo, m), m.q);
+        for (int u = 0; u < kElems; ++u) total[u] = s[u].finish(m);
     }
     u64 *op = out + (size_t)pl * N + x0;
 #pragma unroll
@@ -1383,12 +1386,12 @@ __global__ void __launch_bounds__(256) k_matmul_acc_tiles(const __grid_constant_
 #pragma unroll
             for (int u = 0; u < E; ++u) total[t][u] = add_mod(total[t][u], canon_fp64(acc[t][u], m.q_inv_f, qd), m.q);
     } else {
-        Acc128 s[T][E];
+        PieceAcc s[T][E];
 #pragma unroll
         for (int t = 0; t < T; ++t)
 #pragma unroll
             for (int u = 0; u < E; ++u) s[t][u].zero();
-        int terms = 0;
+        int held = 0; // products in the accumulators
         for (int k = 0; k < kcount; ++k) {
             const u32 g = __ldg(gal + k);
             u32 src[E];
@@ -1396,29 +1399,28 @@ __global__ void __launch_bounds__(256) k_matmul_acc_tiles(const __grid_constant_
             for (int u = 0; u < E; ++u) src[u] = g == 1 ? x0 + u * blockDim.x : ntt_perm(x0 + u * blockDim.x, g, logn);
             for (int b = 0; b < bcount; ++b) {
                 const u64 *a = pbase + ((size_t)k * btotal + b0 + b) * estride;
-                u64 av[E];
+                if (++held == 8) {
+                    held = 1;
 #pragma unroll
-                for (int u = 0; u < E; ++u) av[u] = a[u * blockDim.x];
+                    for (int t = 0; t < T; ++t)
+#pragma unroll
+                        for (int u = 0; u < E; ++u) s[t][u].relax(m);
+                }
+                u32 a0[E], a1[E];
+#pragma unroll
+                for (int u = 0; u < E; ++u) { const u64 v = a[u * blockDim.x]; a0[u] = (u32)v & 0x3FFFFFFFu; a1[u] = (u32)(v >> 30); }
 #pragma unroll
                 for (int t = 0; t < T; ++t) {
                     const u64 *w = tp.p[t][b] + (size_t)l * N;
 #pragma unroll
-                    for (int u = 0; u < E; ++u) s[t][u].mad(av[u], w[src[u]]);
+                    for (int u = 0; u < E; ++u) { const u64 k_ = w[src[u]]; s[t][u].mac(a0[u], a1[u], (u32)k_ & 0x3FFFFFFFu, (u32)(k_ >> 30)); }
                 }
-            }
-            terms += bcount;
-            if (terms >= 48) { // products below 2^120: the 128-bit accumulator holds 256 of them
-#pragma unroll
-                for (int t = 0; t < T; ++t)
-#pragma unroll
-                    for (int u = 0; u < E; ++u) { total[t][u] = add_mod(total[t][u], barrett128(s[t][u].hi, s[t][u].lo, m), m.q); s[t][u].zero(); }
-                terms = 0;
             }
         }
 #pragma unroll
         for (int t = 0; t < T; ++t)
 #pragma unroll
-            for (int u = 0; u < E; ++u) total[t][u] = add_mod(total[t][u], barrett128(s[t][u].hi, s[t][u].lo, m), m.q);
+            for (int u = 0; u < E; ++u) total[t][u] = s[t][u].finish(m);
     }
 #pragma unroll
     for (int t = 0; t < T; ++t) {

@@ -28,6 +28,7 @@ struct PrimeConst {
     u64 fp;             // 1 when q < 2^44: element-wise kernels take quotients from the FP64 pipe
     u64 lazy_terms;     // how many lazy products (each below 1.6 q) may be summed before the sum reaches 2^52
     u32 fold_shift;     // primes of b >= 45 bits: b - 32 (every such prime of a context lies within 2^(b-12) below 2^b)
+    u32 fold_d;         //   and 2^b - q
     u32 d60;            // 2^60 - q when that is positive and below 2^26, else 0
 };
 
@@ -48,37 +49,29 @@ __device__ __forceinline__ u64 mul_shoup(u64 x, u64 w, u64 wsh, u64 q) {
     return r >= q ? r - q : r;
 }
 // ---- cheaper lazy forms for the primes of 45 to 60 bits --------------------------------------------------------
-// Every integer instruction except a 32-bit add costs two issue cycles on one 16-lane pipe here, and a full 64 x 64 high
-// product costs nineteen.  The quotient of a Shoup product does not need it: h = x1 s1 + hi(x0 s1) + hi(x1 s0) (three
-// 32 x 32 products) is low by less than three, so x*w - h*q lies in [0, 4q) for any x < 2^64.  A radix-16 round of
-// butterflies with it takes 36 (Cooley-Tukey) and 41 (Gentleman-Sande) cycles per warp butterfly, with the exact
-// high product and a conditional subtraction per butterfly 49.
-__device__ __forceinline__ u32 hi32_wide(u32 a, u32 b) { // the high word of the full product, kept in the two-cycle wide form
-    u32 h;
-    asm("{\n\t.reg .u32 l;\n\t.reg .u64 t;\n\tmul.wide.u32 t, %1, %2;\n\tmov.b64 {l, %0}, t;\n\t}" : "=r"(h) : "r"(a), "r"(b));
-    return h;
-}
+// Measured here (cycles per warp instruction and SM sub-partition): a 32 x 32 -> 64 product 2.1, a low product with a 32-bit addend
+// 2.0, a high word 4.0, the product with a 64-bit addend 5.0 (4.1 as mad.lo.cc + madc.hi), a 64-bit add 2.1; products and shifts
+// overlap, products and adds do not.  The quotient of a Shoup product does not need the exact high product:
+// h = x1 s1 + hi(x0 s1) + hi(x1 s0) is low by less than three, so x*w - h*q lies in [0, 4q) for any x < 2^64.  A radix-16 round of
+// butterflies with it takes 35 (Cooley-Tukey) and 36 (Gentleman-Sande) cycles per warp butterfly; with the exact high
+// product and a conditional subtraction per butterfly 49.
 __device__ __forceinline__ u64 mul_shoup4(u64 x, u64 w, u64 wsh, u64 nq /* 2^64 - q */) {
     const u32 x0 = (u32)x, x1 = (u32)(x >> 32), s0 = (u32)wsh, s1 = (u32)(wsh >> 32), w0 = (u32)w, w1 = (u32)(w >> 32), n0 = (u32)nq, n1 = (u32)(nq >> 32);
-    const u32 a = hi32_wide(x0, s1), b = hi32_wide(x1, s0);
-    u32 h0, h1, lo, hi;
-    asm("{\n\t.reg .u64 t;\n\tmul.wide.u32 t, %2, %3;\n\tmov.b64 {%0, %1}, t;\n\t"
-        "add.cc.u32 %0, %0, %4;\n\taddc.u32 %1, %1, 0;\n\tadd.cc.u32 %0, %0, %5;\n\taddc.u32 %1, %1, 0;\n\t}"
-        : "=&r"(h0), "=&r"(h1) : "r"(x1), "r"(s1), "r"(a), "r"(b));
-    asm("{\n\t.reg .u64 t;\n\tmul.wide.u32 t, %2, %3;\n\tmad.wide.u32 t, %4, %5, t;\n\tmov.b64 {%0, %1}, t;\n\t}"
-        : "=r"(lo), "=r"(hi) : "r"(x0), "r"(w0), "r"(h0), "r"(n0));
+    const u64 h = (u64)x1 * s1 + (u64)__umulhi(x0, s1) + __umulhi(x1, s0);
+    const u32 h0 = (u32)h, h1 = (u32)(h >> 32);
+    const u64 r = (u64)x0 * w0 + (u64)h0 * n0;
+    u32 hi = (u32)(r >> 32);
     hi = x0 * w1 + hi; hi = x1 * w0 + hi; hi = h0 * n1 + hi; hi = h1 * n0 + hi;
-    return ((u64)hi << 32) | lo;
+    return ((u64)hi << 32) | (u32)r;
 }
-// x < 16 q  ->  congruent value below (1 + 2^-7) * 2^b: subtracts (x >> b) * q
-__device__ __forceinline__ u64 fold_q(u64 x, u64 nq, u32 fold_shift) {
-    const u32 k = (u32)(x >> 32) >> fold_shift;
-    u64 r;
-    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(k), "r"((u32)nq), "l"(x));
-    return r + ((u64)(k * (u32)(nq >> 32)) << 32);
+// x < 16 q  ->  congruent value below (1 + 2^-7) * 2^b, b = fold_shift + 32: replaces k * 2^b (k = x >> b) by k * (2^b - q)
+struct FoldQ { u32 shift, mask, d; };
+__device__ __forceinline__ u64 fold_q(u64 x, const FoldQ &f) {
+    const u32 hi = (u32)(x >> 32);
+    return (((u64)(hi & f.mask) << 32) | (u32)x) + (u64)(hi >> f.shift) * f.d;
 }
-__device__ __forceinline__ u64 canon_q(u64 x, u64 q, u32 fold_shift) { // x < 16 q -> [0, q)
-    const u64 r = fold_q(x, 0ull - q, fold_shift);
+__device__ __forceinline__ u64 canon_q(u64 x, u64 q, const FoldQ &f) { // x < 16 q -> [0, q)
+    const u64 r = fold_q(x, f);
     return r >= q ? r - q : r;
 }
 // (z1:z0) mod q, any 128-bit input.  The quotient estimate is low by at most 4.
@@ -192,33 +185,49 @@ struct Acc128 {
     }
 };
 
-// ---- sums of products modulo the primes of 44 to 60 bits ---------------------------------------------------------
-// A full 64 x 64 -> 128-bit product with its carries costs about thirty 32-bit multiply-adds on this GPU.  For lazy
-// sums of a few products the operands are cut into two pieces of 30 bits instead: a product is then four
-// 32 x 32 -> 64-bit multiply-adds, one per pair of pieces, each into its own 64-bit accumulator with no carries, and
-// the sum of products is  a0 + (a1 + a2) * 2^30 + a3 * 2^60,  assembled and reduced once per output residue.
-// A piece product is below 2^60, so an accumulator holds 16 terms; flush() folds them into a 128-bit running sum.
+// ---- sums of products modulo the primes of 45 to 60 bits ---------------------------------------------------------
+// A full 64 x 64 -> 128-bit product with its carries costs about 34 cycles here.  For sums of a few products the operands are cut
+// into two pieces of 30 bits instead: a product is four 32 x 32 -> 64-bit multiply-adds into three carry-free accumulators (16
+// cycles, 4 more per operand that is cut), and the sum  a0 + a1 * 2^30 + a2 * 2^60  is reduced once per output residue with
+// 2^60 = d60 modulo q (a 128-bit Barrett reduction takes 65 cycles).  Eight products fit the accumulators.
 __device__ __forceinline__ u64 mad_wide(u32 a, u32 b, u64 c) {
-    u64 r;
-    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
-    return r;
+    u32 l = (u32)c, h = (u32)(c >> 32);
+    asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;" : "+r"(l), "+r"(h) : "r"(a), "r"(b));
+    return ((u64)h << 32) | l;
+}
+// a0 + a1 * 2^30 + a2 * 2^60 modulo a prime of 45 to 60 bits (a0, a1 + 2^34, a2 + 2^34 < 2^64): below 4q
+__device__ __forceinline__ u64 finish_wide(u64 a0, u64 a1, u64 a2, const PrimeConst &m) {
+    const u32 m30 = 0x3FFFFFFFu;
+    if (m.d60) { // 2^60 = d60 modulo q
+        const u64 u = a1 + (a0 >> 30), v = a2 + (u >> 30);
+        u64 r = mad_wide((u32)u & m30, 1u << 30, (u64)((u32)a0 & m30)); // < 2^60
+        r = mad_wide((u32)v, m.d60, r);                                 // + 2^58
+        const u64 t = (u64)(u32)(v >> 32) * m.d60;                      // < 2^58, weight 2^32
+        r = mad_wide((u32)(t >> 28), m.d60, r);                         // + 2^56
+        return r + ((u64)((u32)t & 0x0FFFFFFFu) << 32);                 // + 2^60
+    }
+    u64 lo = a0, hi = 0, x = a1 << 30;
+    lo += x; hi += (a1 >> 34) + (lo < x);
+    x = a2 << 60;
+    lo += x; hi += (a2 >> 4) + (lo < x);
+    return barrett128(hi, lo, m);
 }
 struct PieceAcc {
-    u64 a0, a1, a2, a3, lo, hi;
-    __device__ __forceinline__ void zero() { a0 = a1 = a2 = a3 = 0; lo = hi = 0; }
-    __device__ __forceinline__ void mac(u64 v, u64 k) { // v, k < 2^60
-        const u32 v0 = (u32)v & 0x3FFFFFFFu, v1 = (u32)(v >> 30), k0 = (u32)k & 0x3FFFFFFFu, k1 = (u32)(k >> 30);
-        a0 = mad_wide(v0, k0, a0); a1 = mad_wide(v0, k1, a1); a2 = mad_wide(v1, k0, a2); a3 = mad_wide(v1, k1, a3);
+    u64 a0, a1, a2; // weights 1, 2^30, 2^60
+    __device__ __forceinline__ void zero() { a0 = a1 = a2 = 0; }
+    __device__ __forceinline__ void mac(u32 v0, u32 v1, u32 k0, u32 k1) { // 30-bit pieces of the factors
+        a0 = mad_wide(v0, k0, a0); a1 = mad_wide(v0, k1, a1); a1 = mad_wide(v1, k0, a1); a2 = mad_wide(v1, k1, a2);
     }
-    __device__ __forceinline__ void add128(u64 l, u64 h) { lo += l; hi += h + (lo < l); }
-    __device__ __forceinline__ void flush() {
-        add128(a0, 0);
-        add128(a1 << 30, a1 >> 34);
-        add128(a2 << 30, a2 >> 34);
-        add128(a3 << 60, a3 >> 4);
-        a0 = a1 = a2 = a3 = 0;
+    __device__ __forceinline__ void mac(u64 v, u64 k) { mac((u32)v & 0x3FFFFFFFu, (u32)(v >> 30), (u32)k & 0x3FFFFFFFu, (u32)(k >> 30)); } // v, k < 2^60
+    // after at most eight products: makes room for eight more
+    __device__ __forceinline__ void relax(const PrimeConst &m) {
+        const u64 r = finish_wide(a0, a1, a2, m);
+        a0 = r & 0x3FFFFFFFu; a1 = r >> 30; a2 = 0;
     }
-    __device__ __forceinline__ u64 finish(const PrimeConst &m) { flush(); return barrett128(hi, lo, m); }
+    __device__ __forceinline__ u64 finish(const PrimeConst &m) const { // canonical
+        const u64 r = finish_wide(a0, a1, a2, m);
+        return canon_q(r, m.q, FoldQ{m.fold_shift, (1u << m.fold_shift) - 1u, m.fold_d});
+    }
 };
 
 // index of the source slot of the automorphism X -> X^g on an NTT-form limb:

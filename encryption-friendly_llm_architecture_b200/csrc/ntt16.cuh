@@ -128,11 +128,12 @@ __device__ __forceinline__ void gs_bfly(u64 &x, u64 &y, u64 w, u64 ws, u64 q, u6
 }
 struct IntConst {
     u64 q, nq, q4, q8;
-    u32 sh;
+    FoldQ f;
 };
 __device__ __forceinline__ IntConst int_const(const PrimeConst &m) {
     IntConst c;
-    c.q = m.q; c.nq = 0ull - m.q; c.q4 = m.q << 2; c.q8 = m.q << 3; c.sh = m.fold_shift;
+    c.q = m.q; c.nq = 0ull - m.q; c.q4 = m.q << 2; c.q8 = m.q << 3;
+    c.f.shift = m.fold_shift; c.f.mask = (1u << m.fold_shift) - 1u; c.f.d = m.fold_d;
     return c;
 }
 // Four Cooley-Tukey stages on 16 register values; twiddles tp[j].
@@ -150,7 +151,7 @@ template <int FOLD, class TW> __device__ __forceinline__ void fwd16_int(u64 (&v)
             for (int j = 0; j < half; ++j) {
                 u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
                 const u64 t = mul_shoup4(y, tw.x, tw.y, c.nq);
-                if ((FOLD >> s) & 1) x = fold_q(x, c.nq, c.sh);
+                if ((FOLD >> s) & 1) x = fold_q(x, c.f);
                 y = x + c.q4 - t;
                 x = x + t;
             }
@@ -171,7 +172,7 @@ template <class TW> __device__ __forceinline__ void inv16_int(u64 (&v)[16], cons
             for (int j = 0; j < half; ++j) {
                 u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
                 const u64 d = x + ((s & 1) ? c.q4 : c.q8) - y, a = x + y;
-                x = (s & 1) ? a : fold_q(a, c.nq, c.sh);
+                x = (s & 1) ? a : fold_q(a, c.f);
                 y = mul_shoup4(d, tw.x, tw.y, c.nq);
             }
         }
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows(const u64 *src, Li
         for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
         fwd16_int<kFoldRowsB>(v, tw, c);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = canon_q(v[e], c.q, c.sh);
+        for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = canon_q(v[e], c.q, c.f);
     }
     __syncthreads();
 #pragma unroll
@@ -507,7 +508,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *src, Li
         for (int e = 0; e < 16; ++e) v[e] = sm[(e * 16 + sub) * 16 + lane];
         inv16_int(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) o[(e * 16 + sub) * 256] = canon_q(mul_shoup4(v[e], m.n_inv, m.n_inv_sh, c.nq), c.q, c.sh);
+        for (int e = 0; e < 16; ++e) o[(e * 16 + sub) * 256] = canon_q(mul_shoup4(v[e], m.n_inv, m.n_inv_sh, c.nq), c.q, c.f);
     }
 }
 
