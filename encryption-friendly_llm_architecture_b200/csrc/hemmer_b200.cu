@@ -132,7 +132,7 @@ struct hb_ctx {
     int N = 0, logn = 0, L = 0, K = 0, nprimes = 0;
     unsigned long long launches = 0; // kernels launched by this context
     int *dev_err = nullptr;          // raised by a kernel whose bounded wait ran out; read by hb_sync
-    bool smem_opt_in_mkb = false, smem_opt_in_parts = false; // the opt-in to more than 48 KB of shared memory is per kernel and per device: once per context
+    bool smem_opt_in_parts = false; // the opt-in to more than 48 KB of shared memory is per kernel and per device: once per context
     // Compulsory HBM traffic of the primitives called so far, in limbs of N words: every input of a primitive read once,
     // every output written once, a switching key or plaintext once per batch (temporaries and transforms inside a
     // primitive do not count).  Divided by the HBM peak this is the time the call sequence cannot go below.
@@ -347,21 +347,16 @@ template <int COLS> size_t strip_bytes(int strips) { return (size_t)strips * Str
 void conv_opt_in(hb_ctx *c) {
     if (c->smem_opt_in_conv) return;
     auto allow = [](auto *kernel, size_t bytes) { CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); };
-    allow(conv_cols<8, 2, 2>, strip_bytes<8>(10)); allow(conv_cols<8, 4, 1>, strip_bytes<8>(12)); allow(conv_cols<4, 4, 3>, strip_bytes<4>(12));
-    allow(conv_cols<4, 8, 1>, strip_bytes<4>(16)); allow(conv_cols<4, 8, 2>, strip_bytes<4>(16)); allow(conv_cols<4, 4, 2>, strip_bytes<4>(12));
+    allow(conv_cols<8, 4, 1>, strip_bytes<8>(12)); allow(conv_cols<4, 4, 2>, strip_bytes<4>(12)); allow(conv_cols<4, 8, 1>, strip_bytes<4>(16));
     allow(lift_cols<8, 2, 2>, strip_bytes<8>(3)); allow(lift_cols<4, 4, 2>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1>, strip_bytes<4>(9));
-    allow(lift_cols<4, 4, 4>, strip_bytes<4>(5)); allow(lift_cols<8, 2, 4>, strip_bytes<8>(3));
     c->smem_opt_in_conv = true;
 }
 // Strip width and groups of a launch over `units` (polynomial, conversion) pairs.  At most two units: narrow strips and many groups, so that
-// all sources and all targets of a unit are worked on at once.  Otherwise strips of eight columns, in the shape that fills the
-// last wave better: 32 * units CTAs of four groups, one per SM, or of two groups, two per SM and half as fast each.
+// all sources and all targets of a unit are worked on at once.  Up to 32: narrow strips, two CTAs per SM, for the last wave.
+// Beyond: strips of eight columns (64-byte runs).  Rotations at level 6, us, (4 cols x 8 groups) / (4 x 4) / (8 x 4): one ciphertext
+// 88 / 103 / 98, eight 397 / 363 / 378, 64 2773 / 2524 / 2494.
 enum StripShape { kStrip8x2, kStrip8x4, kStrip4x4, kStrip4x8 };
-StripShape conv_shape(int units) {
-    if (const char *e = getenv("HB_STRIP")) return (StripShape)atoi(e);
-    if (units <= 2) return kStrip4x8;
-    return (units * 32 + 147) / 148 <= 1.9 * ((units * 32 + 295) / 296) ? kStrip8x4 : kStrip8x2;
-}
+StripShape conv_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 32 ? kStrip4x4 : kStrip8x4; }
 StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : kStrip8x2; }
 // `plans` conversions (the largest with max_ns sources) of `instances` polynomials in one launch
 void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int instances) {
@@ -370,14 +365,10 @@ void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, con
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
         launch_pdl(c->st, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
     };
-    int sh = conv_shape(instances * count);
-    switch (sh) {
-    case 0: go(conv_cols<8, 2, 2>, 8, 2, strip_bytes<8>(max_ns + 2)); break;
-    case 1: go(conv_cols<8, 4, 1>, 8, 4, strip_bytes<8>(max_ns + 4)); break;
-    case 2: go(conv_cols<4, 4, 3>, 4, 4, strip_bytes<4>(max_ns + 4)); break;
-    case 3: go(conv_cols<4, 8, 1>, 4, 8, strip_bytes<4>(max_ns + 8)); break;
-    case 4: go(conv_cols<4, 8, 2>, 4, 8, strip_bytes<4>(max_ns + 8)); break;
-    case 5: go(conv_cols<4, 4, 2>, 4, 4, strip_bytes<4>(max_ns + 4)); break;
+    switch (conv_shape(instances * count)) {
+    case kStrip8x4: go(conv_cols<8, 4, 1>, 8, 4, strip_bytes<8>(max_ns + 4)); break;
+    case kStrip4x4: go(conv_cols<4, 4, 2>, 4, 4, strip_bytes<4>(max_ns + 4)); break;
+    default: go(conv_cols<4, 8, 1>, 4, 8, strip_bytes<4>(max_ns + 8)); break;
     }
 }
 // half-inverse limbs of prime `level` (one per instance) -> half-forward lifts to the limbs below
@@ -387,14 +378,10 @@ void launch_lift(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
         launch_pdl(c->st, kernel, dim3(256 / cols, instances), cols * 16 * groups, smem, src, so, dst, dof, level, c->pc, c->tb.t16);
     };
-    int sh = lift_shape(instances);
-    if (const char *e = getenv("HB_LIFT")) sh = atoi(e);
-    switch (sh) {
-    case 0: go(lift_cols<8, 2, 2>, 8, 2, strip_bytes<8>(3)); break;
-    case 1: go(lift_cols<8, 2, 4>, 8, 2, strip_bytes<8>(3)); break;
-    case 2: go(lift_cols<4, 4, 2>, 4, 4, strip_bytes<4>(5)); break;
-    case 3: go(lift_cols<4, 8, 1>, 4, 8, strip_bytes<4>(9)); break;
-    case 4: go(lift_cols<4, 4, 4>, 4, 4, strip_bytes<4>(5)); break;
+    switch (lift_shape(instances)) {
+    case kStrip4x8: go(lift_cols<4, 8, 1>, 4, 8, strip_bytes<4>(9)); break;
+    case kStrip4x4: go(lift_cols<4, 4, 2>, 4, 4, strip_bytes<4>(5)); break;
+    default: go(lift_cols<8, 2, 2>, 8, 2, strip_bytes<8>(3)); break;
     }
 }
 void inv_rows(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int count, const LimbMap &m) {
@@ -471,6 +458,11 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, siz
     LAUNCH(c), k_moddown_fin<<<dim3(gx, n, total * 2), 256, 0, c->st>>>(out, out_outer, acc, tbuf, sl, batch, add_outer, pl, c->pc, c->logn, N);
     CK(cudaGetLastError());
 }
+// Members that one CTA of a key-stationary kernel walks over: as many as leave about eight CTAs per SM
+int members_per_cta(int batch, int ctas_per_chunk) {
+    const int chunks = std::max(1, std::min(batch, (8 * 148 + ctas_per_chunk - 1) / ctas_per_chunk));
+    return (batch + chunks - 1) / chunks;
+}
 // Phase 2: inner products of the (permuted) digits with the keys over Q_level u P, then ModDown, for every group of `sl`:
 //   out[ob][p][l] = ModDown(sum_dg perm_g(digit_dg) (.) key_dg)[p][l] + add_p[b][l] o perm_g,   ob = group * batch + b
 void ks_apply(hb_ctx *c, const SwitchList &sl, size_t a_outer, int level, int batch, u64 *out, size_t out_outer, size_t add_outer) {
@@ -478,7 +470,18 @@ void ks_apply(hb_ctx *c, const SwitchList &sl, size_t a_outer, int level, int ba
     const PlanDims d = plan_dims(c, level);
     const int N = c->N, n = d.n, ne = d.ne, total = sl.count * batch;
     Tmp acc(c, (size_t)total * 2 * ne), t(c, (size_t)total * 2 * n);
-    LAUNCH(c), launch_pdl(c->st, k_ks_inner, dim3(c->gx(), total, ne), 256, 0, acc.p, sl, batch, a_outer, c->nprimes, pl, c->pc, c->logn, N);
+    const int per = members_per_cta(batch, N / 512 * ne * sl.count), chunks = (batch + per - 1) / per;
+    auto inner = [&](auto *kernel) { LAUNCH(c), launch_pdl(c->st, kernel, dim3((unsigned)(N / 512), sl.count * chunks, ne), 256, 0, acc.p, sl, batch, per, a_outer, c->nprimes, pl, c->pc, c->logn, N); };
+    switch (d.nd) {
+    case 1: inner(k_ks_inner<1>); break;
+    case 2: inner(k_ks_inner<2>); break;
+    case 3: inner(k_ks_inner<3>); break;
+    case 4: inner(k_ks_inner<4>); break;
+    case 5: inner(k_ks_inner<5>); break;
+    case 6: inner(k_ks_inner<6>); break;
+    case 7: inner(k_ks_inner<7>); break;
+    default: inner(k_ks_inner<8>); break;
+    }
     moddown(c, acc.p, t.p, level, total, out, out_outer, sl, batch, add_outer);
 }
 // Hybrid key switch of polynomial a (NTT form, `n` limbs, per-batch stride a_outer) with key `key`
@@ -667,23 +670,15 @@ hb_ct *do_assemble_mk(hb_ctx *c, const hb_ct *a, const u64 *dt, const hb_mkey *c
     Tmp E(c, (size_t)groups * batch * 2 * ne);
     for (int g = 0; g < groups; ++g) ALG(c, (size_t)mrl.r[g].count * ((size_t)d.nd * 2 * ne + n) + (size_t)batch * 2 * (n - 1));
     ALG(c, (size_t)batch * (2 * n + d.dt_count));
-    // Up to two digits: the bulk-copy kernel (three members per CTA, 512 coefficients; 112 KB of shared memory, two CTAs
-    // per SM).  With more digits its staging buffers leave room for one CTA per SM only and the register kernel is faster.
-    if (d.nd <= 2 && N % 512 == 0) {
-        constexpr int M = 3, EL = 2, T = 256 * EL;
-        const int chunks = (batch + M - 1) / M;
-        int maxcount = 1;
-        for (int g = 0; g < groups; ++g) maxcount = std::max(maxcount, mrl.r[g].count);
-        const size_t smem = ((size_t)maxcount * d.nd * 2 + maxcount + (size_t)M * maxcount * (d.nd + 1)) * T * 8;
-        if (!c->smem_opt_in_mkb) { CK(cudaFuncSetAttribute(k_ks_inner_mkb<M, EL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 28 * T * 8)); c->smem_opt_in_mkb = true; }
-        LAUNCH(c), k_ks_inner_mkb<M, EL><<<dim3((unsigned)(N / T), (unsigned)(groups * chunks), (unsigned)ne), 256, smem, c->st>>>(E.p, a->d, a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch,
-                                                                                                                              maxcount, pl, c->pc, c->logn, N, c->dev_err);
-        CK(cudaGetLastError());
-        return divide_by_p_ql(c, E.p, level, groups * batch);
+    if (d.nd <= 2) {
+        const int per = members_per_cta(batch, N / 512 * ne * groups), chunks = (batch + per - 1) / per;
+        LAUNCH(c), launch_pdl(c->st, d.nd == 1 ? k_ks_inner_mkr<1> : k_ks_inner_mkr<2>, dim3((unsigned)(N / 512), (unsigned)(groups * chunks), (unsigned)ne), 256, 0, E.p, (const u64 *)a->d,
+                              (const u64 *)a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch, per, pl, c->pc, c->logn, N);
+    } else {
+        LAUNCH(c), launch_pdl(c->st, k_ks_inner_mk, dim3((unsigned)((N + 1023) / 1024), groups * batch, ne), 256, 0, E.p, (const u64 *)a->d, (const u64 *)a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch, pl,
+                              c->pc, c->logn, N);
     }
-    constexpr int kEl = 4; // coefficients per thread (2, with three CTAs resident per SM, measured no faster)
-    LAUNCH(c), k_ks_inner_mk<kEl><<<dim3((unsigned)((N + 256 * kEl - 1) / (256 * kEl)), groups * batch, ne), 256, 0, c->st>>>(E.p, a->d, a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch, pl, c->pc,
-                                                                                                                        c->logn, N);
+    CK(cudaGetLastError());
     return divide_by_p_ql(c, E.p, level, groups * batch);
 }
 

@@ -499,63 +499,109 @@ constexpr int kMaxSwitchGroups = 16;
 struct SwitchList { SwitchGroup s[kMaxSwitchGroups]; int count; };
 // Inner product with the switching key over Q_level u P.
 //   acc[ob][p][j][i] = sum_dg digit_dg[j][perm_g(i)] * key[dg][p][prime(j)][i],   member ob = group * batch + b
-// digit_dg[j] is a_ntt[j] for own limbs and dt[...] otherwise.  grid = (N/(256*kElems), groups * batch, ne)
-__global__ void k_ks_inner(u64 *acc, const __grid_constant__ SwitchList sl, int batch, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, int logn,
-                           int N) {
-    const int j = blockIdx.z, ob = blockIdx.y, b = ob % batch; // limb-major block order: the key limbs stay in L2 across the members
-    const SwitchGroup &sg = sl.s[ob / batch];
+// digit_dg[j] is a_ntt[j] for own limbs and dt[...] otherwise.  A CTA owns 512 coefficients of one limb for `per` members of a group:
+// a thread keeps the key words of its two coefficients in registers (as doubles, or cut into pieces) and walks over the
+// members with the next member's digits in flight, so the keys -- two thirds of the words a member needs -- are read once.
+// One member per CTA read and converted them every time: 517 us for 64 members at level 6.
+// grid = (N/512, groups * ceil(batch/per), ne); ND = digits in use
+template <int ND>
+__global__ void __launch_bounds__(256, ND <= 2 ? 3 : 2) k_ks_inner(u64 *acc, const __grid_constant__ SwitchList sl, int batch, int per, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl,
+                                                                   const PrimeConst *__restrict__ pc, int logn, int N) {
+    constexpr int EL = 2;
+    const int chunks = (batch + per - 1) / per, grp = blockIdx.y / chunks, b0 = (blockIdx.y % chunks) * per, b1 = min(batch, b0 + per);
+    const int j = blockIdx.z; // limb-major block order
+    const SwitchGroup &sg = sl.s[grp];
     const u32 g = sg.g;
-    const int pj = pl->ext_prime[j], nd = pl->nd, ne = pl->ne;
+    const int pj = pl->ext_prime[j], ne = pl->ne;
     const PrimeConst m = pc[pj];
-    const u32 x0 = blockIdx.x * (blockDim.x * kElems) + threadIdx.x;
-    u32 src[kElems];
+    const u32 x0 = blockIdx.x * (256 * EL) + threadIdx.x;
+    u32 src[EL];
 #pragma unroll
-    for (int u = 0; u < kElems; ++u) { const u32 i = x0 + u * blockDim.x; src[u] = g ? ntt_perm(i, g, logn) : i; }
-    const u64 *abase = sg.a_ntt + (size_t)b * a_outer + (size_t)j * N;
-    const u64 *dbase = sg.dt + (size_t)b * pl->dt_count * N;
+    for (int u = 0; u < EL; ++u) { const u32 i = x0 + u * 256; src[u] = g ? ntt_perm(i, g, logn) : i; }
+    const u64 *sp[ND];
+    size_t stride[ND];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        const int en = pl->dt_entry[d][j];
+        stride[d] = en < 0 ? a_outer : (size_t)pl->dt_count * N;
+        sp[d] = (en < 0 ? sg.a_ntt + (size_t)j * N : sg.dt + (size_t)en * N) + (size_t)b0 * stride[d];
+    }
     const u64 *kbase = sg.key + (size_t)pj * N + x0;
     const size_t kpoly = (size_t)key_primes * N;
+    u64 *o = acc + (((size_t)(grp * batch + b0) * 2) * ne + j) * N + x0;
+    const size_t opoly = (size_t)ne * N;
     pdl_wait();
-    u64 r0[kElems], r1[kElems];
-    if (m.fp) { // products on the FP64 pipe, signed double sums
+    u64 cur[ND][EL];
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+#pragma unroll
+        for (int u = 0; u < EL; ++u) cur[d][u] = sp[d][src[u]];
+    if (m.fp) {
         const double qd = (double)m.q;
-        double d0[kElems], d1[kElems];
+        double k[ND][2][EL];
 #pragma unroll
-        for (int u = 0; u < kElems; ++u) { d0[u] = 0.0; d1[u] = 0.0; }
-        for (int dg = 0; dg < nd; ++dg) {
-            const int en = pl->dt_entry[dg][j];
-            const u64 *sp = en < 0 ? abase : dbase + (size_t)en * N;
-            const u64 *k0 = kbase + (size_t)dg * 2 * kpoly;
+        for (int d = 0; d < ND; ++d)
 #pragma unroll
-            for (int u = 0; u < kElems; ++u) {
-                const double vd = u52_to_double(sp[src[u]]);
-                d0[u] = __dadd_rn(d0[u], mul_fp64_lazy(vd, u52_to_double(k0[u * blockDim.x]), m.q_inv_f, qd));
-                d1[u] = __dadd_rn(d1[u], mul_fp64_lazy(vd, u52_to_double(k0[kpoly + u * blockDim.x]), m.q_inv_f, qd));
+            for (int p = 0; p < 2; ++p)
+#pragma unroll
+                for (int u = 0; u < EL; ++u) k[d][p][u] = u52_to_double(kbase[(size_t)(d * 2 + p) * kpoly + u * 256]);
+        for (int b = b0; b < b1; ++b) {
+            double v[ND][EL];
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+                sp[d] += stride[d];
+#pragma unroll
+                for (int u = 0; u < EL; ++u) {
+                    v[d][u] = u52_to_double(cur[d][u]);
+                    if (b + 1 < b1) cur[d][u] = sp[d][src[u]];
+                }
             }
-        }
 #pragma unroll
-        for (int u = 0; u < kElems; ++u) { r0[u] = canon_fp64(d0[u], m.q_inv_f, qd); r1[u] = canon_fp64(d1[u], m.q_inv_f, qd); }
+            for (int u = 0; u < EL; ++u)
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    FpAcc s;
+                    s.first(v[0][u], k[0][p][u]);
+#pragma unroll
+                    for (int d = 1; d < ND; ++d) s.mac(v[d][u], k[d][p][u]);
+                    o[(size_t)p * opoly + u * 256] = s.finish(m.q_inv_f, qd);
+                }
+            o += 2 * opoly;
+        }
     } else {
-        PieceAcc s0[kElems], s1[kElems];
+        u32 k0[ND][2][EL], k1[ND][2][EL];
 #pragma unroll
-        for (int u = 0; u < kElems; ++u) { s0[u].zero(); s1[u].zero(); }
-        for (int dg = 0; dg < nd; ++dg) {
-            const int en = pl->dt_entry[dg][j];
-            const u64 *sp = en < 0 ? abase : dbase + (size_t)en * N;
-            const u64 *k0 = kbase + (size_t)dg * 2 * kpoly;
+        for (int d = 0; d < ND; ++d)
 #pragma unroll
-            for (int u = 0; u < kElems; ++u) {
-                const u64 v = sp[src[u]];
-                s0[u].mac(v, k0[u * blockDim.x]);
-                s1[u].mac(v, k0[kpoly + u * blockDim.x]);
+            for (int p = 0; p < 2; ++p)
+#pragma unroll
+                for (int u = 0; u < EL; ++u) {
+                    const u64 w = kbase[(size_t)(d * 2 + p) * kpoly + u * 256];
+                    k0[d][p][u] = (u32)w & 0x3FFFFFFFu; k1[d][p][u] = (u32)(w >> 30);
+                }
+        for (int b = b0; b < b1; ++b) {
+            u32 v0[ND][EL], v1[ND][EL];
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+                sp[d] += stride[d];
+#pragma unroll
+                for (int u = 0; u < EL; ++u) {
+                    v0[d][u] = (u32)cur[d][u] & 0x3FFFFFFFu; v1[d][u] = (u32)(cur[d][u] >> 30);
+                    if (b + 1 < b1) cur[d][u] = sp[d][src[u]];
+                }
             }
+#pragma unroll
+            for (int u = 0; u < EL; ++u)
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    PieceAcc s; s.zero(); // at most eight digits
+#pragma unroll
+                    for (int d = 0; d < ND; ++d) s.mac(v0[d][u], v1[d][u], k0[d][p][u], k1[d][p][u]);
+                    o[(size_t)p * opoly + u * 256] = s.finish(m);
+                }
+            o += 2 * opoly;
         }
-#pragma unroll
-        for (int u = 0; u < kElems; ++u) { r0[u] = s0[u].finish(m); r1[u] = s1[u].finish(m); }
     }
-    u64 *o0 = acc + (((size_t)ob * 2) * ne + j) * N + x0, *o1 = o0 + (size_t)ne * N;
-#pragma unroll
-    for (int u = 0; u < kElems; ++u) { o0[u * blockDim.x] = r0[u]; o1[u * blockDim.x] = r1[u]; }
 }
 
 // ModDown conversion: pcoef [bp][K][N] (special limbs, coefficient form) -> t [bp][n][N] (coefficient form)
@@ -827,6 +873,9 @@ __global__ void k_ks_inner_pair(u64 *__restrict__ E, const u64 *__restrict__ c0,
 // sum_dg digit_dg * (mask * key_dg) = mask * sum_dg digit_dg * key_dg modulo q, so a key multiplied by the mask once
 // (k_mask_key) turns the masked pair of rotations into ONE lazy inner product with ONE reduction per output residue;
 // the residues are those of k_ks_inner_pair.
+// Stored form of a masked-key word (nothing outside the kernels below sees it): an integer-valued double for primes below 2^44, the two
+// 30-bit pieces in the halves of the word otherwise.
+__device__ __forceinline__ u64 key_word(u64 w, bool fp) { return fp ? (u64)__double_as_longlong(u52_to_double(w)) : ((w >> 30) << 32) | ((u32)w & 0x3FFFFFFFu); }
 // mkey[dg][p][j][i] = (mask[j][i] + mask2[j][i]) * key[dg][p][prime(j)][i];  grid = (N/(256*kElems), ne, nd*2)
 __global__ void k_mask_key(u64 *__restrict__ mkey, const u64 *__restrict__ key, int key_primes, const u64 *__restrict__ mask, const u64 *__restrict__ mask2,
                            const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, int N) {
@@ -839,7 +888,7 @@ __global__ void k_mask_key(u64 *__restrict__ mkey, const u64 *__restrict__ key, 
         if (i >= N) break;
         u64 w = mask[(size_t)j * N + i];
         if (mask2) w = add_mod(w, mask2[(size_t)j * N + i], m.q);
-        mkey[((size_t)dgp * ne + j) * N + i] = mul_mod_any(w, key[((size_t)dgp * key_primes + pj) * N + i], m);
+        mkey[((size_t)dgp * ne + j) * N + i] = key_word(mul_mod_any(w, key[((size_t)dgp * key_primes + pj) * N + i], m), m.fp);
     }
 }
 // pm[j][i] = P * (mask[j][i] + mask2[j][i]) mod q_j for the Q limbs;  grid = (N/(256*kElems), n)
@@ -852,7 +901,7 @@ __global__ void k_mask_p(u64 *__restrict__ pm, const u64 *__restrict__ mask, con
         if (i >= N) break;
         u64 w = mask[(size_t)j * N + i];
         if (mask2) w = add_mod(w, mask2[(size_t)j * N + i], m.q);
-        pm[(size_t)j * N + i] = mul_mod_any(w, dv->p_mod[j], m);
+        pm[(size_t)j * N + i] = key_word(mul_mod_any(w, dv->p_mod[j], m), m.fp);
     }
 }
 struct MaskedRot {
@@ -864,11 +913,13 @@ struct MaskedRot {
 constexpr int kMaxRotGroups = 16;
 struct MaskedRotList { MaskedRot r[kMaxRotGroups]; }; // one entry per wrapped copy made by the same launch
 // E[b][p][j][i] = sum_r sum_dg digit_dg[j][perm_r(i)] * mkey_r[dg][p][j][i]  +  (p == 0, j < n) sum_r c0[b][j][perm_r(i)] * pm_r[j][i]
-// grid = (N/(256*EL), groups * batch, ne); EL coefficients per thread.  Output member g * batch + b is wrapped copy
-// number g (its own pair of masked keys) of input member b: several iterations of a shift loop in one launch.
-template <int EL>
-__global__ void __launch_bounds__(256, EL == 2 ? 3 : 2) k_ks_inner_mk(u64 *__restrict__ E, const u64 *__restrict__ c0, const u64 *__restrict__ a_ntt, size_t a_outer, const u64 *__restrict__ dt, const __grid_constant__ MaskedRotList mrl,
-                              int batch, const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, int logn, int N) {
+// Output member g * batch + b is wrapped copy number g (its own one or two masked keys) of input member b: several iterations
+// of a shift loop in one launch.
+//
+// Any number of digits: one member and four coefficients per thread.  grid = (N/1024, groups * batch, ne)
+__global__ void __launch_bounds__(256, 2) k_ks_inner_mk(u64 *E, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const __grid_constant__ MaskedRotList mrl, int batch,
+                                                        const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, int logn, int N) {
+    constexpr int EL = 4;
     const int j = blockIdx.z, ob = blockIdx.y, b = ob % batch; // limb-major block order: the key limbs stay in L2 across the members
     const MaskedRot &mr = mrl.r[ob / batch];
     const int pj = pl->ext_prime[j], nd = pl->nd, ne = pl->ne, n = pl->n;
@@ -879,7 +930,8 @@ __global__ void __launch_bounds__(256, EL == 2 ? 3 : 2) k_ks_inner_mk(u64 *__res
     const u64 *dbase = dt + (size_t)b * pl->dt_count * N;
     const size_t kpoly = (size_t)ne * N;
     u64 r0[EL], r1[EL];
-    if (m.fp) { // products on the FP64 pipe, signed double sums
+    pdl_wait();
+    if (m.fp) { // products reduced one by one, signed double sums (up to 18 of them)
         const double qd = (double)m.q;
         double d0[EL], d1[EL];
 #pragma unroll
@@ -888,22 +940,22 @@ __global__ void __launch_bounds__(256, EL == 2 ? 3 : 2) k_ks_inner_mk(u64 *__res
             u32 src[EL];
 #pragma unroll
             for (int u = 0; u < EL; ++u) src[u] = ntt_perm(x0 + u * blockDim.x, mr.g[r], logn);
-            const u64 *kbase = mr.mkey[r] + (size_t)j * N + x0;
+            const double *kbase = reinterpret_cast<const double *>(mr.mkey[r]) + (size_t)j * N + x0;
             for (int dg = 0; dg < nd; ++dg) {
                 const int en = pl->dt_entry[dg][j];
                 const u64 *sp = en < 0 ? abase : dbase + (size_t)en * N;
-                const u64 *k0 = kbase + (size_t)dg * 2 * kpoly;
+                const double *k0 = kbase + (size_t)dg * 2 * kpoly;
 #pragma unroll
                 for (int u = 0; u < EL; ++u) {
                     const double vd = u52_to_double(sp[src[u]]);
-                    d0[u] = __dadd_rn(d0[u], mul_fp64_lazy(vd, u52_to_double(k0[u * blockDim.x]), m.q_inv_f, qd));
-                    d1[u] = __dadd_rn(d1[u], mul_fp64_lazy(vd, u52_to_double(k0[kpoly + u * blockDim.x]), m.q_inv_f, qd));
+                    d0[u] = __dadd_rn(d0[u], mul_fp64_lazy(vd, k0[u * blockDim.x], m.q_inv_f, qd));
+                    d1[u] = __dadd_rn(d1[u], mul_fp64_lazy(vd, k0[kpoly + u * blockDim.x], m.q_inv_f, qd));
                 }
             }
             if (j < n) {
-                const u64 *pmb = mr.pm[r] + (size_t)j * N + x0;
+                const double *pmb = reinterpret_cast<const double *>(mr.pm[r]) + (size_t)j * N + x0;
 #pragma unroll
-                for (int u = 0; u < EL; ++u) d0[u] = __dadd_rn(d0[u], mul_fp64_lazy(u52_to_double(cbase[src[u]]), u52_to_double(pmb[u * blockDim.x]), m.q_inv_f, qd));
+                for (int u = 0; u < EL; ++u) d0[u] = __dadd_rn(d0[u], mul_fp64_lazy(u52_to_double(cbase[src[u]]), pmb[u * blockDim.x], m.q_inv_f, qd));
             }
         }
 #pragma unroll
@@ -929,15 +981,19 @@ __global__ void __launch_bounds__(256, EL == 2 ? 3 : 2) k_ks_inner_mk(u64 *__res
                 const u64 *k0 = kbase + (size_t)dg * 2 * kpoly;
 #pragma unroll
                 for (int u = 0; u < EL; ++u) {
-                    const u64 v = sp[src[u]];
-                    s0[u].mac(v, k0[u * blockDim.x]);
-                    s1[u].mac(v, k0[kpoly + u * blockDim.x]);
+                    const u64 v = sp[src[u]], ka = k0[u * blockDim.x], kb = k0[kpoly + u * blockDim.x];
+                    const u32 v0 = (u32)v & 0x3FFFFFFFu, v1 = (u32)(v >> 30);
+                    s0[u].mac(v0, v1, (u32)ka, (u32)(ka >> 32));
+                    s1[u].mac(v0, v1, (u32)kb, (u32)(kb >> 32));
                 }
             }
             if (j < n) {
                 const u64 *pmb = mr.pm[r] + (size_t)j * N + x0;
 #pragma unroll
-                for (int u = 0; u < EL; ++u) s0[u].mac(cbase[src[u]], pmb[u * blockDim.x]);
+                for (int u = 0; u < EL; ++u) {
+                    const u64 v = cbase[src[u]], k = pmb[u * blockDim.x];
+                    s0[u].mac((u32)v & 0x3FFFFFFFu, (u32)(v >> 30), (u32)k, (u32)(k >> 32));
+                }
                 ++held;
             }
         }
@@ -948,157 +1004,111 @@ __global__ void __launch_bounds__(256, EL == 2 ? 3 : 2) k_ks_inner_mk(u64 *__res
 #pragma unroll
     for (int u = 0; u < EL; ++u) { o0[u * blockDim.x] = r0[u]; o1[u * blockDim.x] = r1[u]; }
 }
-// The same sums fed by bulk copies.  The automorphism maps every aligned block of 2^k outputs onto one aligned block
-// of 2^k inputs, so a CTA that owns T consecutive coefficients of limb j needs, per (member, rotation, digit), exactly
-// one contiguous chunk of T words -- and one chunk per key word.  One warp issues all those copies at once (tens of KB
-// per CTA in flight from its first instruction on, which 8-byte register loads cannot keep up), every thread then
-// waits on the mbarrier and works from shared memory: the permutation becomes an index into the staged chunk, key
-// words are read once and meet M members.  Other resident CTAs of the SM compute while this one's copies land.
-// Dynamic shared memory: (count*nd*2 + count + M*count*(nd+1)) * T words, count = most rotations of any group.
-// grid = (N / T, groups * ceil(batch / M), ne), T = 256 * EL
-template <int M, int EL>
-__global__ void __launch_bounds__(256) k_ks_inner_mkb(u64 *__restrict__ E, const u64 *__restrict__ c0, const u64 *__restrict__ a_ntt, size_t a_outer, const u64 *__restrict__ dt,
-                                                      const __grid_constant__ MaskedRotList mrl, int batch, int maxcount, const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, int logn,
-                                                      int N, int *__restrict__ err) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ __align__(8) u64 bar;
-    constexpr int T = 256 * EL;
-    const int chunks = (batch + M - 1) / M;
-    const int j = blockIdx.z, grp = blockIdx.y / chunks, b0 = (blockIdx.y % chunks) * M;
-    const int nm = min(M, batch - b0);
-    const MaskedRot &mr = mrl.r[grp];
-    const int pj = pl->ext_prime[j], nd = pl->nd, ne = pl->ne, n = pl->n, count = mr.count;
-    const bool has_c0 = j < n;
-    const int nsrc = nd + 1; // chunks per (member, rotation): the digits, then c0 (left empty on the limbs of P)
-    u64 *keyb = reinterpret_cast<u64 *>(smem_raw), *pmb = keyb + (size_t)maxcount * nd * 2 * T, *srcb = pmb + (size_t)maxcount * T;
-    const u32 tile0 = blockIdx.x * T;
-    const int tid = threadIdx.x;
-    if (tid == 0) { mbar_init(&bar, 1); mbar_fence_init(); }
-    __syncthreads();
-    if (tid < 32) {
-        const int nkey = count * nd * 2, npm = has_c0 ? count : 0, per_member = count * (nd + (has_c0 ? 1 : 0));
-        const int total = nkey + npm + nm * per_member;
-        if (tid == 0) mbar_arrive_expect_tx(&bar, (u32)total * T * 8);
-        __syncwarp();
-        for (int ci = tid; ci < total; ci += 32) {
-            const u64 *src;
-            u64 *dst;
-            if (ci < nkey) {
-                const int r = ci / (nd * 2), rem = ci % (nd * 2); // rem = digit * 2 + poly
-                src = mr.mkey[r] + ((size_t)rem * ne + j) * N + tile0;
-                dst = keyb + (size_t)ci * T;
-            } else if (ci < nkey + npm) {
-                const int r = ci - nkey;
-                src = mr.pm[r] + (size_t)j * N + tile0;
-                dst = pmb + (size_t)r * T;
-            } else {
-                const int k = ci - nkey - npm, u = k / per_member, rem = k % per_member, r = rem % count, dg = rem / count;
-                const u32 st0 = ntt_perm(tile0, mr.g[r], logn) & ~(u32)(T - 1);
-                if (dg < nd) {
-                    const int en = pl->dt_entry[dg][j];
-                    src = en < 0 ? a_ntt + (size_t)(b0 + u) * a_outer + (size_t)j * N : dt + ((size_t)(b0 + u) * pl->dt_count + en) * N;
-                } else src = c0 + (size_t)(b0 + u) * a_outer + (size_t)j * N;
-                src += st0;
-                dst = srcb + ((size_t)(u * count + r) * nsrc + dg) * T;
-            }
-            bulk_load(dst, src, T * 8, &bar);
-        }
-    }
-    mbar_wait_bounded(&bar, 0, err);
-    const PrimeConst m = pc[pj];
-    u64 r0[M][EL], r1[M][EL];
-    if (m.fp) { // products on the FP64 pipe, signed double sums of at most 2 * (nd + 1) terms
-        const double qd = (double)m.q;
-        double d0[M][EL], d1[M][EL];
-#pragma unroll
-        for (int u = 0; u < M; ++u)
-#pragma unroll
-            for (int e = 0; e < EL; ++e) { d0[u][e] = 0.0; d1[u][e] = 0.0; }
-        for (int r = 0; r < count; ++r) {
-            u32 li[EL];
-#pragma unroll
-            for (int e = 0; e < EL; ++e) li[e] = ntt_perm(tile0 + e * 256 + tid, mr.g[r], logn) & (u32)(T - 1);
-            for (int dg = 0; dg < nd; ++dg) {
-                const u64 *kp = keyb + (size_t)((r * nd + dg) * 2) * T + tid;
-                const u64 *sp = srcb + (size_t)(r * nsrc + dg) * T;
-#pragma unroll
-                for (int e = 0; e < EL; ++e) {
-                    const double kad = u52_to_double(kp[e * 256]), kbd = u52_to_double(kp[T + e * 256]);
-#pragma unroll
-                    for (int u = 0; u < M; ++u)
-                        if (u < nm) {
-                            const double vd = u52_to_double(sp[(size_t)u * count * nsrc * T + li[e]]);
-                            d0[u][e] = __dadd_rn(d0[u][e], mul_fp64_lazy(vd, kad, m.q_inv_f, qd));
-                            d1[u][e] = __dadd_rn(d1[u][e], mul_fp64_lazy(vd, kbd, m.q_inv_f, qd));
-                        }
-                }
-            }
-            if (has_c0) {
-                const u64 *sp = srcb + (size_t)(r * nsrc + nd) * T;
-#pragma unroll
-                for (int e = 0; e < EL; ++e) {
-                    const double pmd = u52_to_double(pmb[(size_t)r * T + e * 256 + tid]);
-#pragma unroll
-                    for (int u = 0; u < M; ++u)
-                        if (u < nm) d0[u][e] = __dadd_rn(d0[u][e], mul_fp64_lazy(u52_to_double(sp[(size_t)u * count * nsrc * T + li[e]]), pmd, m.q_inv_f, qd));
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < M; ++u)
-#pragma unroll
-            for (int e = 0; e < EL; ++e) { r0[u][e] = canon_fp64(d0[u][e], m.q_inv_f, qd); r1[u][e] = canon_fp64(d1[u][e], m.q_inv_f, qd); }
-    } else {
-        PieceAcc s0[M][EL], s1[M][EL];
-#pragma unroll
-        for (int u = 0; u < M; ++u)
-#pragma unroll
-            for (int e = 0; e < EL; ++e) { s0[u][e].zero(); s1[u][e].zero(); }
-        for (int r = 0; r < count; ++r) {
-            u32 li[EL];
-#pragma unroll
-            for (int e = 0; e < EL; ++e) li[e] = ntt_perm(tile0 + e * 256 + tid, mr.g[r], logn) & (u32)(T - 1);
-            for (int dg = 0; dg < nd; ++dg) {
-                const u64 *kp = keyb + (size_t)((r * nd + dg) * 2) * T + tid;
-                const u64 *sp = srcb + (size_t)(r * nsrc + dg) * T;
-#pragma unroll
-                for (int e = 0; e < EL; ++e) {
-                    const u64 ka = kp[e * 256], kb = kp[T + e * 256];
-                    const u32 ka0 = (u32)ka & 0x3FFFFFFFu, ka1 = (u32)(ka >> 30), kb0 = (u32)kb & 0x3FFFFFFFu, kb1 = (u32)(kb >> 30);
-#pragma unroll
-                    for (int u = 0; u < M; ++u)
-                        if (u < nm) {
-                            const u64 v = sp[(size_t)u * count * nsrc * T + li[e]];
-                            const u32 v0 = (u32)v & 0x3FFFFFFFu, v1 = (u32)(v >> 30);
-                            s0[u][e].mac(v0, v1, ka0, ka1);
-                            s1[u][e].mac(v0, v1, kb0, kb1);
-                        }
-                }
-            }
-            if (has_c0) {
-                const u64 *sp = srcb + (size_t)(r * nsrc + nd) * T;
-#pragma unroll
-                for (int e = 0; e < EL; ++e) {
-                    const u64 pmv = pmb[(size_t)r * T + e * 256 + tid];
-#pragma unroll
-                    for (int u = 0; u < M; ++u)
-                        if (u < nm) s0[u][e].mac(sp[(size_t)u * count * nsrc * T + li[e]], pmv);
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < M; ++u)
-#pragma unroll
-            for (int e = 0; e < EL; ++e) { r0[u][e] = s0[u][e].finish(m); r1[u][e] = s1[u][e].finish(m); }
-    }
+// At most two digits: a thread keeps the words of the one or two masked keys for its two coefficients in registers and walks over `per`
+// input members with the next member's words in flight.  Up to eleven masked-key words meet six words per member and coefficient;
+// staging both in shared memory by bulk copies for three members at a time took 1.6 times as long (they crossed L2 for every
+// third member, and a CTA's copies, sums and stores did not overlap).
+// grid = (N/512, groups * ceil(batch/per), ne)
+template <int ND, int CNT>
+__device__ __forceinline__ void ks_inner_mkr_body(u64 *o, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const MaskedRot &mr, int b0, int b1, const KsPlan *__restrict__ pl,
+                                                  const PrimeConst &m, int j, u32 x0, int logn, int N) {
+    constexpr int EL = 2;
+    const int ne = pl->ne;
+    const bool has_c0 = j < pl->n;
     const size_t kpoly = (size_t)ne * N;
-    u64 *o0 = E + (((size_t)(grp * batch + b0) * 2) * ne + j) * N + tile0 + tid;
+    u32 src[CNT][EL];
 #pragma unroll
-    for (int u = 0; u < M; ++u)
-        if (u < nm) {
+    for (int r = 0; r < CNT; ++r)
 #pragma unroll
-            for (int e = 0; e < EL; ++e) { o0[(size_t)u * 2 * kpoly + e * 256] = r0[u][e]; o0[(size_t)u * 2 * kpoly + kpoly + e * 256] = r1[u][e]; }
+        for (int u = 0; u < EL; ++u) src[r][u] = ntt_perm(x0 + u * 256, mr.g[r], logn);
+    const u64 *sp[ND];
+    size_t stride[ND];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        const int en = pl->dt_entry[d][j];
+        stride[d] = en < 0 ? a_outer : (size_t)pl->dt_count * N;
+        sp[d] = (en < 0 ? a_ntt + (size_t)j * N : dt + (size_t)en * N) + (size_t)b0 * stride[d];
+    }
+    const u64 *cp = c0 + (size_t)b0 * a_outer + (size_t)j * N;
+    u64 cur[CNT][ND][EL], cc[CNT][EL], k[CNT][ND][2][EL], pm[CNT][EL];
+#pragma unroll
+    for (int r = 0; r < CNT; ++r)
+#pragma unroll
+        for (int u = 0; u < EL; ++u) {
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+                cur[r][d][u] = sp[d][src[r][u]];
+                k[r][d][0][u] = mr.mkey[r][(size_t)(d * 2) * kpoly + (size_t)j * N + x0 + u * 256];
+                k[r][d][1][u] = mr.mkey[r][(size_t)(d * 2 + 1) * kpoly + (size_t)j * N + x0 + u * 256];
+            }
+            cc[r][u] = has_c0 ? cp[src[r][u]] : 0;
+            pm[r][u] = has_c0 ? mr.pm[r][(size_t)j * N + x0 + u * 256] : 0;
         }
+    const double qd = (double)m.q;
+    for (int b = b0; b < b1; ++b) {
+        u64 v[CNT][ND][EL], w[CNT][EL];
+        cp += a_outer;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) sp[d] += stride[d];
+#pragma unroll
+        for (int r = 0; r < CNT; ++r)
+#pragma unroll
+            for (int u = 0; u < EL; ++u) {
+#pragma unroll
+                for (int d = 0; d < ND; ++d) { v[r][d][u] = cur[r][d][u]; if (b + 1 < b1) cur[r][d][u] = sp[d][src[r][u]]; }
+                w[r][u] = cc[r][u];
+                if (has_c0 && b + 1 < b1) cc[r][u] = cp[src[r][u]];
+            }
+        if (m.fp) {
+#pragma unroll
+            for (int u = 0; u < EL; ++u) {
+                FpAcc s0, s1;
+#pragma unroll
+                for (int r = 0; r < CNT; ++r) {
+#pragma unroll
+                    for (int d = 0; d < ND; ++d) {
+                        const double x = u52_to_double(v[r][d][u]), k0 = __longlong_as_double((long long)k[r][d][0][u]), k1 = __longlong_as_double((long long)k[r][d][1][u]);
+                        if (r == 0 && d == 0) { s0.first(x, k0); s1.first(x, k1); }
+                        else { s0.mac(x, k0); s1.mac(x, k1); }
+                    }
+                    if (has_c0) s0.mac(u52_to_double(w[r][u]), __longlong_as_double((long long)pm[r][u]));
+                }
+                o[u * 256] = s0.finish(m.q_inv_f, qd);
+                o[kpoly + u * 256] = s1.finish(m.q_inv_f, qd);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < EL; ++u) {
+                PieceAcc s0, s1; s0.zero(); s1.zero(); // at most six products
+#pragma unroll
+                for (int r = 0; r < CNT; ++r) {
+#pragma unroll
+                    for (int d = 0; d < ND; ++d) {
+                        const u32 v0 = (u32)v[r][d][u] & 0x3FFFFFFFu, v1 = (u32)(v[r][d][u] >> 30);
+                        s0.mac(v0, v1, (u32)k[r][d][0][u], (u32)(k[r][d][0][u] >> 32));
+                        s1.mac(v0, v1, (u32)k[r][d][1][u], (u32)(k[r][d][1][u] >> 32));
+                    }
+                    if (has_c0) s0.mac((u32)w[r][u] & 0x3FFFFFFFu, (u32)(w[r][u] >> 30), (u32)pm[r][u], (u32)(pm[r][u] >> 32));
+                }
+                o[u * 256] = s0.finish(m);
+                o[kpoly + u * 256] = s1.finish(m);
+            }
+        }
+        o += 2 * kpoly;
+    }
+}
+template <int ND>
+__global__ void __launch_bounds__(256, 2) k_ks_inner_mkr(u64 *E, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const __grid_constant__ MaskedRotList mrl, int batch, int per,
+                                                         const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, int logn, int N) {
+    const int chunks = (batch + per - 1) / per, grp = blockIdx.y / chunks, b0 = (blockIdx.y % chunks) * per, b1 = min(batch, b0 + per);
+    const int j = blockIdx.z; // limb-major block order: the digits of one limb stay in L2 across the copies
+    const MaskedRot &mr = mrl.r[grp];
+    const PrimeConst m = pc[pl->ext_prime[j]];
+    const u32 x0 = blockIdx.x * 512 + threadIdx.x;
+    u64 *o = E + (((size_t)(grp * batch + b0) * 2) * pl->ne + j) * N + x0;
+    pdl_wait();
+    if (mr.count == 1) ks_inner_mkr_body<ND, 1>(o, c0, a_ntt, a_outer, dt, mr, b0, b1, pl, m, j, x0, logn, N);
+    else ks_inner_mkr_body<ND, 2>(o, c0, a_ntt, a_outer, dt, mr, b0, b1, pl, m, j, x0, logn, N);
 }
 // Base conversion of the division: src [bp][ns][N] (limbs q_level, P; coefficient form) -> t [bp][level][N]
 // grid = (N/256, 1, nbp)

@@ -175,6 +175,31 @@ __device__ __forceinline__ u64 canon_fp64(double v, double q_inv, double qd) {
     return mantissa52(__dadd_rn(r, kTwo52));
 }
 
+// ---- exact sums of a few such products -------------------------------------------------------------------------
+// h collects the products rounded to multiples of 2^40 (it starts at 1.5 * 2^92, whose ulp that is), l the remainders: four FP64
+// instructions per product instead of seven, one quotient for the sum.  a, w >= 0; the products must add up to less than 2^91:
+// 2^7 of them for primes below 2^42, eight below 2^44.
+constexpr double kGrid40 = 1.5 * 0x1p92;
+struct FpAcc {
+    double h, l;
+    __device__ __forceinline__ void first(double a, double w) {
+        h = __fma_rn(a, w, kGrid40);
+        l = __fma_rn(a, w, -__dadd_rn(h, -kGrid40));
+    }
+    __device__ __forceinline__ void mac(double a, double w) {
+        const double t = __fma_rn(a, w, h), d = __dadd_rn(t, -h);
+        h = t;
+        l = __dadd_rn(l, __fma_rn(a, w, -d));
+    }
+    __device__ __forceinline__ u64 finish(double q_inv, double qd) const { // canonical
+        const double t = __dadd_rn(h, -kGrid40);
+        const double k = __dadd_rn(__dadd_rn(__fma_rn(t, q_inv, __dmul_rn(l, q_inv)), kMagicS), -kMagicS);
+        double r = __dadd_rn(__fma_rn(-k, qd, t), l); // within 0.51 q of zero
+        if (r < 0.0) r = __dadd_rn(r, qd);
+        return mantissa52(__dadd_rn(r, kTwo52));
+    }
+};
+
 // 128-bit accumulator for lazy sums of products
 struct Acc128 {
     u64 lo, hi;
