@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
 
 // Single passes, for the fused sequences.  A grid of one or two CTAs per SM takes the kernels that may use 128 registers and
 // fetch the twiddles of the second round (which nobody shares) before anything else, under the tail of the predecessor.
-static const int kSmallGrid = getenv("HB_SG") ? atoi(getenv("HB_SG")) : 2 * 148;
+constexpr int kSmallGrid = 2 * 148;
 inline void launch_inv_rows16(cudaStream_t st, const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
     launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_inv_rows<2> : ntt16v2_inv_rows<4>, dim3(16, count), 256, 0, src, LimbAddr16{src_outer}, dst, LimbAddr16{dst_outer}, map, pc, tb);
 }

@@ -712,7 +712,7 @@ hb_ct *do_rescale(hb_ctx *c, const hb_ct *a) {
     own(c, a);
     if (a->level < 1) fail(HB_E_LEVEL, "rescale: level 0");
     if (a->spow != 2) fail(HB_E_SHAPE, "rescale: nothing to rescale");
-    const int l = a->level, N = c->N, nbp = a->batch * a->np;
+    const int l = a->level, nbp = a->batch * a->np;
     hb_ct *r = new_ct(c, l - 1, a->np, a->batch, 1);
     ALG(c, (size_t)nbp * (2 * l + 1));
     try {
