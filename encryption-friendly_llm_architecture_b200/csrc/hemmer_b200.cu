@@ -1689,7 +1689,13 @@ static hb_ct *rotate_sum_core(hb_ctx *c, const u64 *const *base, const int64_t *
             CK(cudaMemcpyAsync(r->d, add.p, r->limbs() * N * 8, cudaMemcpyDeviceToDevice, c->st));
         } else {
             Tmp acc(c, (size_t)batch * 2 * ne), t(c, (size_t)batch * 2 * n);
-            LAUNCH(c), k_ks_inner_sum<<<dim3(gx, batch, ne), 256, 0, c->st>>>(acc.p, rot, ct_outer, c->nprimes, pl, c->pc, c->logn, N);
+            auto inner = [&](auto *kernel, int el, int members) {
+                LAUNCH(c), kernel<<<dim3((unsigned)(N / (256 * el)), (unsigned)((batch + members - 1) / members), (unsigned)ne), 256, 0, c->st>>>(acc.p, rot, batch, ct_outer, c->nprimes, pl, c->pc,
+                                                                                                                                         c->logn, N);
+            };
+            if (batch == 1) inner(k_ks_inner_sum<2, 1>, 2, 1);
+            else if (batch < 4) inner(k_ks_inner_sum<2, 2>, 2, 2);
+            else inner(k_ks_inner_sum<1, 4>, 1, 4);
             SwitchList sl{};
             sl.count = 1;
             sl.s[0].add[0] = add.p; sl.s[0].add[1] = add.p + (size_t)n * N;

@@ -681,76 +681,124 @@ __global__ void k_moddown_fin(u64 *out, size_t out_outer, const u64 *acc, const 
 // Up to 16 terms (ciphertext batch x_t rotated by g_t): the inner products of all terms are added up in Q_level u P.
 struct RotTerm { const u64 *a_ntt; const u64 *dt; const u64 *key; u32 g; u32 pad; };
 struct RotTermList { RotTerm t[16]; int count; };
-//   acc[b][p][j][i] = sum_t sum_dg digit_t,dg[j][perm_t(i)] * key_t[dg][p][prime(j)][i]      grid = (N/(256*kElems), batch, ne)
-__global__ void k_ks_inner_sum(u64 *__restrict__ acc, const __grid_constant__ RotTermList tl, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc,
-                               int logn, int N) {
-    const int j = blockIdx.z, b = blockIdx.y;
+//   acc[b][p][j][i] = sum_t sum_dg digit_t,dg[j][perm_t(i)] * key_t[dg][p][prime(j)][i]
+// A thread works on EL coefficients of M members: a key word is read (and converted or cut) once for M products, and the sums take
+// one reduction each.  One member per thread, every product reduced: 1068 us a launch in the layer pass, now 907 us (four members);
+// a single ciphertext 107 -> 100 us.  Bound by instruction issue, half of it on the 60-bit limbs.
+// grid = (N/(256*EL), ceil(batch/M), ne); members beyond the batch repeat the last one and are not stored
+template <int EL, int M>
+__global__ void __launch_bounds__(256, 2) k_ks_inner_sum(u64 *acc, const __grid_constant__ RotTermList tl, int batch, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl,
+                                                         const PrimeConst *__restrict__ pc, int logn, int N) {
+    const int j = blockIdx.z, b0 = blockIdx.y * M;
     const int pj = pl->ext_prime[j], nd = pl->nd, ne = pl->ne;
     const PrimeConst m = pc[pj];
-    const u32 x0 = blockIdx.x * (blockDim.x * kElems) + threadIdx.x;
-    const size_t kpoly = (size_t)key_primes * N;
-    u64 r0[kElems], r1[kElems];
-    if (m.fp) { // at most 16 terms x 8 digits of products within 0.51 q of zero: signed double sums far below 2^53
+    const u32 x0 = blockIdx.x * (256 * EL) + threadIdx.x;
+    const size_t kpoly = (size_t)key_primes * N, d_outer = (size_t)pl->dt_count * N;
+    u64 r[2][M][EL];
+    // every term meets EL * (M digit words + 2 key words) per digit
+    auto terms = [&](auto &&product) {
+        for (int t = 0; t < tl.count; ++t) {
+            const RotTerm &rt = tl.t[t];
+            u32 src[EL];
+#pragma unroll
+            for (int u = 0; u < EL; ++u) src[u] = ntt_perm(x0 + u * 256, rt.g, logn);
+            const u64 *kbase = rt.key + (size_t)pj * N + x0;
+#pragma unroll 2
+            for (int dg = 0; dg < nd; ++dg) {
+                const int en = pl->dt_entry[dg][j];
+                const u64 *sp = en < 0 ? rt.a_ntt + (size_t)j * N : rt.dt + (size_t)en * N;
+                const size_t outer = en < 0 ? a_outer : d_outer;
+                u64 v[M][EL], k[2][EL];
+#pragma unroll
+                for (int u = 0; u < EL; ++u) {
+#pragma unroll
+                    for (int i = 0; i < M; ++i) v[i][u] = sp[(size_t)min(b0 + i, batch - 1) * outer + src[u]];
+                    k[0][u] = kbase[(size_t)(dg * 2) * kpoly + u * 256];
+                    k[1][u] = kbase[(size_t)(dg * 2 + 1) * kpoly + u * 256];
+                }
+                product(v, k);
+            }
+        }
+    };
+    if (m.fp) { // exact sums (see FpAcc): 128 products of primes below 2^42, eight below 2^44, before they are reduced
         const double qd = (double)m.q;
-        double d0[kElems], d1[kElems];
+        const int room = m.q < (1ull << 42) ? 128 : 8;
+        FpAcc s[2][M][EL];
+        int held = 0;
 #pragma unroll
-        for (int u = 0; u < kElems; ++u) { d0[u] = 0.0; d1[u] = 0.0; }
-        for (int t = 0; t < tl.count; ++t) {
-            u32 src[kElems];
+        for (int p = 0; p < 2; ++p)
 #pragma unroll
-            for (int u = 0; u < kElems; ++u) src[u] = ntt_perm(x0 + u * blockDim.x, tl.t[t].g, logn);
-            const u64 *abase = tl.t[t].a_ntt + (size_t)b * a_outer + (size_t)j * N;
-            const u64 *dbase = tl.t[t].dt + (size_t)b * pl->dt_count * N;
-            const u64 *kbase = tl.t[t].key + (size_t)pj * N + x0;
-            for (int dg = 0; dg < nd; ++dg) {
-                const int en = pl->dt_entry[dg][j];
-                const u64 *sp = en < 0 ? abase : dbase + (size_t)en * N;
-                const u64 *k0 = kbase + (size_t)dg * 2 * kpoly;
+            for (int i = 0; i < M; ++i)
 #pragma unroll
-                for (int u = 0; u < kElems; ++u) {
-                    const double vd = u52_to_double(sp[src[u]]);
-                    d0[u] = __dadd_rn(d0[u], mul_fp64_lazy(vd, u52_to_double(k0[u * blockDim.x]), m.q_inv_f, qd));
-                    d1[u] = __dadd_rn(d1[u], mul_fp64_lazy(vd, u52_to_double(k0[kpoly + u * blockDim.x]), m.q_inv_f, qd));
+                for (int u = 0; u < EL; ++u) s[p][i][u].zero();
+        terms([&](const u64 (&v)[M][EL], const u64 (&k)[2][EL]) {
+            if (++held > room) {
+                held = 1;
+#pragma unroll
+                for (int p = 0; p < 2; ++p)
+#pragma unroll
+                    for (int i = 0; i < M; ++i)
+#pragma unroll
+                        for (int u = 0; u < EL; ++u) s[p][i][u].relax(m.q_inv_f, qd);
+            }
+#pragma unroll
+            for (int u = 0; u < EL; ++u) {
+                const double k0 = u52_to_double(k[0][u]), k1 = u52_to_double(k[1][u]);
+#pragma unroll
+                for (int i = 0; i < M; ++i) {
+                    const double vd = u52_to_double(v[i][u]);
+                    s[0][i][u].mac(vd, k0);
+                    s[1][i][u].mac(vd, k1);
                 }
             }
-        }
+        });
 #pragma unroll
-        for (int u = 0; u < kElems; ++u) { r0[u] = canon_fp64(d0[u], m.q_inv_f, qd); r1[u] = canon_fp64(d1[u], m.q_inv_f, qd); }
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int i = 0; i < M; ++i)
+#pragma unroll
+                for (int u = 0; u < EL; ++u) r[p][i][u] = s[p][i][u].finish(m.q_inv_f, qd);
     } else {
-        PieceAcc s0[kElems], s1[kElems];
-#pragma unroll
-        for (int u = 0; u < kElems; ++u) { s0[u].zero(); s1[u].zero(); }
+        PieceAcc s[2][M][EL];
         int held = 0; // products in the accumulators
-        for (int t = 0; t < tl.count; ++t) {
-            u32 src[kElems];
 #pragma unroll
-            for (int u = 0; u < kElems; ++u) src[u] = ntt_perm(x0 + u * blockDim.x, tl.t[t].g, logn);
-            const u64 *abase = tl.t[t].a_ntt + (size_t)b * a_outer + (size_t)j * N;
-            const u64 *dbase = tl.t[t].dt + (size_t)b * pl->dt_count * N;
-            const u64 *kbase = tl.t[t].key + (size_t)pj * N + x0;
-            for (int dg = 0; dg < nd; ++dg) {
-                if (++held == 8) {
-                    held = 1;
+        for (int p = 0; p < 2; ++p)
 #pragma unroll
-                    for (int u = 0; u < kElems; ++u) { s0[u].relax(m); s1[u].relax(m); }
-                }
-                const int en = pl->dt_entry[dg][j];
-                const u64 *sp = en < 0 ? abase : dbase + (size_t)en * N;
-                const u64 *k0 = kbase + (size_t)dg * 2 * kpoly;
+            for (int i = 0; i < M; ++i)
 #pragma unroll
-                for (int u = 0; u < kElems; ++u) {
-                    const u64 v = sp[src[u]];
-                    s0[u].mac(v, k0[u * blockDim.x]);
-                    s1[u].mac(v, k0[kpoly + u * blockDim.x]);
-                }
+                for (int u = 0; u < EL; ++u) s[p][i][u].zero();
+        terms([&](const u64 (&v)[M][EL], const u64 (&k)[2][EL]) {
+            if (++held > 8) {
+                held = 1;
+#pragma unroll
+                for (int p = 0; p < 2; ++p)
+#pragma unroll
+                    for (int i = 0; i < M; ++i)
+#pragma unroll
+                        for (int u = 0; u < EL; ++u) s[p][i][u].relax(m);
             }
-        }
 #pragma unroll
-        for (int u = 0; u < kElems; ++u) { r0[u] = s0[u].finish(m); r1[u] = s1[u].finish(m); }
+            for (int u = 0; u < EL; ++u)
+#pragma unroll
+                for (int i = 0; i < M; ++i) {
+                    s[0][i][u].mac(v[i][u], k[0][u]);
+                    s[1][i][u].mac(v[i][u], k[1][u]);
+                }
+        });
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int i = 0; i < M; ++i)
+#pragma unroll
+                for (int u = 0; u < EL; ++u) r[p][i][u] = s[p][i][u].finish(m);
     }
-    u64 *o0 = acc + (((size_t)b * 2) * ne + j) * N + x0, *o1 = o0 + (size_t)ne * N;
 #pragma unroll
-    for (int u = 0; u < kElems; ++u) { o0[u * blockDim.x] = r0[u]; o1[u * blockDim.x] = r1[u]; }
+    for (int i = 0; i < M; ++i)
+        if (b0 + i < batch) {
+            u64 *o = acc + (((size_t)(b0 + i) * 2) * ne + j) * N + x0;
+#pragma unroll
+            for (int u = 0; u < EL; ++u) { o[u * 256] = r[0][i][u]; o[(size_t)ne * N + u * 256] = r[1][i][u]; }
+        }
 }
 // add[b][p][l][i] = sum over the rotated terms of (p == 0) c0_t[b][l][perm_t(i)]  +  sum over the unrotated terms of x_t[b][p][l][i]
 // rot: terms with g != 1 (a_ntt - n limbs = c0); plain: terms added as they are.  grid = (N/(256*kElems), n, batch*2)

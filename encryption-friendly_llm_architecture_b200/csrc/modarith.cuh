@@ -182,6 +182,7 @@ __device__ __forceinline__ u64 canon_fp64(double v, double q_inv, double qd) {
 constexpr double kGrid40 = 1.5 * 0x1p92;
 struct FpAcc {
     double h, l;
+    __device__ __forceinline__ void zero() { h = kGrid40; l = 0.0; }
     __device__ __forceinline__ void first(double a, double w) {
         h = __fma_rn(a, w, kGrid40);
         l = __fma_rn(a, w, -__dadd_rn(h, -kGrid40));
@@ -191,10 +192,15 @@ struct FpAcc {
         h = t;
         l = __dadd_rn(l, __fma_rn(a, w, -d));
     }
-    __device__ __forceinline__ u64 finish(double q_inv, double qd) const { // canonical
+    // The quotient is below 2^49 and off by less than 0.2 beyond its rounding; t - k q is an integer below 2^48, so exact.
+    __device__ __forceinline__ double reduced(double q_inv, double qd) const { // within 0.7 q of zero
         const double t = __dadd_rn(h, -kGrid40);
         const double k = __dadd_rn(__dadd_rn(__fma_rn(t, q_inv, __dmul_rn(l, q_inv)), kMagicS), -kMagicS);
-        double r = __dadd_rn(__fma_rn(-k, qd, t), l); // within 0.51 q of zero
+        return __dadd_rn(__fma_rn(-k, qd, t), l);
+    }
+    __device__ __forceinline__ void relax(double q_inv, double qd) { l = reduced(q_inv, qd); h = kGrid40; } // makes room for as many products again
+    __device__ __forceinline__ u64 finish(double q_inv, double qd) const { // canonical
+        double r = reduced(q_inv, qd);
         if (r < 0.0) r = __dadd_rn(r, qd);
         return mantissa52(__dadd_rn(r, kTwo52));
     }
