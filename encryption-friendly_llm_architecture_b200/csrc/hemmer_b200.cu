@@ -823,7 +823,8 @@ void launch_matmul_tiles(hb_ctx *c, const hb_ct *pre, int btotal, int b0, const 
         tp.out[t] = outs[t]->d;
     }
     const int n = pre->level + 1;
-    LAUNCH(c), k_matmul_acc_tiles<T><<<dim3((unsigned)(c->N / 512), (unsigned)(2 * n)), 256, 0, c->st>>>(tp, pre->d, kc, btotal, b0, bcount, dg, n, c->qmap(pre->level), c->pc, c->logn, c->N);
+    constexpr int E = T >= 3 ? 1 : 2;
+    LAUNCH(c), k_matmul_acc<T, E><<<dim3((unsigned)(c->N / (256 * E)), (unsigned)n), 256, 0, c->st>>>(tp, pre->d, kc, btotal, b0, bcount, dg, n, c->qmap(pre->level), c->pc, c->logn, c->N);
 }
 hb_ct *do_level_down(hb_ctx *c, const hb_ct *a, int target) {
     own(c, a);
@@ -991,8 +992,7 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             p.n_inv_f = (double)p.n_inv / (double)q;
             p.fp = q < ((u64)1 << 44) ? 1 : 0;
             // lazy FP64-assisted products are below 1.6 q; reduce_fp takes sums below 2^52.  Every fixed-length lazy sum in
-            // the kernels has at most 128 terms (16 rotated terms x 8 digits), which any prime below 2^44 allows (>= 160);
-            // the open-ended sum of k_matmul_acc folds at this count.
+            // the kernels has at most 128 terms (16 rotated terms x 8 digits), which any prime below 2^44 allows (>= 160).
             p.lazy_terms = (u64)((((unsigned __int128)1 << 52) * 5) / ((unsigned __int128)q * 8));
             if (p.fp && p.lazy_terms < 160) throw std::invalid_argument("prime too large for the lazy FP64-assisted sums");
             // primes of 45 bits and more: values are folded with shifts by the bit length b, which needs q close below 2^b; the
@@ -1786,18 +1786,16 @@ int hb_matmul_acc_multi(hb_ctx *c, const hb_ct *pre, int btotal, int b0, const h
         if (btotal < 1 || pre->batch % btotal || b0 < 0 || bcount < 1 || b0 + bcount > btotal || bcount > 16) fail(HB_E_SHAPE, "matmul_acc: group selection");
         if (pre->np != 2 || pre->spow != 1) fail(HB_E_SHAPE, "matmul_acc: operands");
         own(c, pre);
-        PtList pl{};
         for (int b = 0; b < bcount; ++b) {
             if (pre->level != pts[b]->level) fail(HB_E_LEVEL, "matmul_acc: plaintext level differs from the ciphertexts'");
             own(c, pts[b]);
             if (pts[b]->spow != 1) fail(HB_E_SHAPE, "matmul_acc: operands");
-            pl.p[b] = pts[b]->d;
         }
         const int n = pre->level + 1, kc = pre->batch / btotal;
         const u32 *dg = galois_table(c, kc, row_step);
         hb_ct *r = new_ct(c, pre->level, 2, 1, 2);
         ALG(c, (size_t)kc * bcount * 2 * n + (size_t)bcount * n + 2 * n);
-        LAUNCH(c), k_matmul_acc<<<c->egrid(2 * n), 256, 0, c->st>>>(r->d, pre->d, kc, btotal, b0, bcount, pl, dg, n, c->qmap(pre->level), c->pc, c->logn, c->N);
+        launch_matmul_tiles<1>(c, pre, btotal, b0, pts, bcount, kc, dg, &r);
         *out = r;
     });
 }

@@ -1315,176 +1315,106 @@ __global__ void k_keygen(u64 *__restrict__ b, const u64 *__restrict__ a, const u
 }
 
 // ---------------- fused plaintext-matmul accumulate ----------------
-// out[p][l][i] = sum_{b < bcount} sum_{k < kcount} pre[k * btotal + b0 + b][p][l][i] * pt_b[l][perm_{g_k}(i)]
-// (scale Delta^2, no rescale).  Shifted copies are stored k-major; the sum over b adds the partial products
-// of several K-groups in the same pass.  grid = (N/256, 2*n).  The accumulators are reduced every few terms.
-struct PtList { const u64 *p[16]; };
-__global__ void k_matmul_acc(u64 *__restrict__ out, const u64 *__restrict__ pre, int kcount, int btotal, int b0, int bcount, const __grid_constant__ PtList pts, const u32 *__restrict__ gal,
-                             int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int logn, int N) {
-    const int pl = blockIdx.y, l = pl % n;
-    const PrimeConst m = pc[map.prime[l]];
-    const size_t estride = (size_t)2 * n * N;
-    const u32 x0 = blockIdx.x * (blockDim.x * kElems) + threadIdx.x;
-    const u64 *pbase = pre + (size_t)pl * N + x0;
-    u64 total[kElems];
-#pragma unroll
-    for (int u = 0; u < kElems; ++u) total[u] = 0;
-    // the four coefficients of a thread sit in the inner loop: their loads (and those of the next K-group) overlap
-    if (m.fp) { // lazy terms below 1.6q: the running sum is folded before it can reach 2^52 (reduce_fp's input range)
-        u64 acc[kElems];
-#pragma unroll
-        for (int u = 0; u < kElems; ++u) acc[u] = 0;
-        int terms = 0;
-        const int fold_at = (int)m.lazy_terms - 16; // a round of the inner loop adds at most 16 terms (bcount <= 16)
-        for (int k = 0; k < kcount; ++k) {
-            const u32 g = __ldg(gal + k);
-            u32 src[kElems];
-#pragma unroll
-            for (int u = 0; u < kElems; ++u) src[u] = g == 1 ? x0 + u * blockDim.x : ntt_perm(x0 + u * blockDim.x, g, logn);
-#pragma unroll 2
-            for (int b = 0; b < bcount; ++b) {
-                const u64 *a = pbase + ((size_t)k * btotal + b0 + b) * estride, *w = pts.p[b] + (size_t)l * N;
-#pragma unroll
-                for (int u = 0; u < kElems; ++u) acc[u] += mul_small_lazy(a[u * blockDim.x], w[src[u]], m.q_inv_f, m.q);
-            }
-            terms += bcount;
-            if (terms > fold_at) {
-#pragma unroll
-                for (int u = 0; u < kElems; ++u) { total[u] = add_mod(total[u], reduce_fp(acc[u], m.q_inv_f, m.q), m.q); acc[u] = 0; }
-                terms = 0;
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kElems; ++u) total[u] = add_mod(total[u], reduce_fp(acc[u], m.q_inv_f, m.q), m.q);
-    } else {
-        PieceAcc s[kElems];
-#pragma unroll
-        for (int u = 0; u < kElems; ++u) s[u].zero();
-        int held = 0; // products in the accumulators
-        for (int k = 0; k < kcount; ++k) {
-            const u32 g = __ldg(gal + k);
-            u32 src[kElems];
-#pragma unroll
-            for (int u = 0; u < kElems; ++u) src[u] = g == 1 ? x0 + u * blockDim.x : ntt_perm(x0 + u * blockDim.x, g, logn);
-#pragma unroll 2
-            for (int b = 0; b < bcount; ++b) {
-                const u64 *a = pbase + ((size_t)k * btotal + b0 + b) * estride, *w = pts.p[b] + (size_t)l * N;
-                if (++held == 8) {
-                    held = 1;
-#pragma unroll
-                    for (int u = 0; u < kElems; ++u) s[u].relax(m);
-                }
-#pragma unroll
-                for (int u = 0; u < kElems; ++u) s[u].mac(a[u * blockDim.x], w[src[u]]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kElems; ++u) total[u] = s[u].finish(m);
-    }
-    u64 *op = out + (size_t)pl * N + x0;
-#pragma unroll
-    for (int u = 0; u < kElems; ++u) op[u * blockDim.x] = total[u];
-}
-
-// The same for T output tiles that share the shifted copies: a copy word is read once and meets the weights of T tiles
-// (all output tiles of a sublayer multiply the same copies of x), so the copies -- the bulk of the traffic -- cross HBM
-// once per T tiles.  Two coefficients per thread.  Primes below 2^44: products on the FP64 pipe, signed double sums folded
-// every 512 terms (512 * 0.51 q stays far below 2^53).  grid = (N/512, 2*n)
+// out_t[p][l][i] = sum_{b < bcount} sum_{k < kcount} pre[k * btotal + b0 + b][p][l][i] * pt_tb[l][perm_{g_k}(i)]
+// (scale Delta^2, no rescale) for T output tiles t that share the shifted copies, which are stored k-major; the sum over b adds the
+// partial products of several K-groups in the same pass.  A thread works on E coefficients of both polynomials: a copy word is
+// read once for T tiles and a weight word once (and converted or cut once) for two polynomials.  Four tiles a launch in the layer
+// pass: one polynomial per thread with every product reduced 840 us, this 675 us; bound by the 60-bit limb's integer products and
+// by HBM on the copies.  grid = (N/(256*E), n)
 template <int T> struct TilePts { const u64 *p[T][16]; u64 *out[T]; };
-template <int T>
-__global__ void __launch_bounds__(256) k_matmul_acc_tiles(const __grid_constant__ TilePts<T> tp, const u64 *__restrict__ pre, int kcount, int btotal, int b0, int bcount,
-                                                          const u32 *__restrict__ gal, int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int logn, int N) {
-    constexpr int E = 2;
-    const int pl = blockIdx.y, l = pl % n;
+template <int T, int E>
+__global__ void __launch_bounds__(256, 2) k_matmul_acc(const __grid_constant__ TilePts<T> tp, const u64 *__restrict__ pre, int kcount, int btotal, int b0, int bcount, const u32 *__restrict__ gal,
+                                                       int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int logn, int N) {
+    const int l = blockIdx.y;
     const PrimeConst m = pc[map.prime[l]];
-    const size_t estride = (size_t)2 * n * N;
-    const u32 x0 = blockIdx.x * (blockDim.x * E) + threadIdx.x;
-    const u64 *pbase = pre + (size_t)pl * N + x0;
-    u64 total[T][E];
-#pragma unroll
-    for (int t = 0; t < T; ++t)
-#pragma unroll
-        for (int u = 0; u < E; ++u) total[t][u] = 0;
-    if (m.fp) {
-        const double qd = (double)m.q;
-        double acc[T][E];
-#pragma unroll
-        for (int t = 0; t < T; ++t)
-#pragma unroll
-            for (int u = 0; u < E; ++u) acc[t][u] = 0.0;
-        int terms = 0;
+    const size_t poly = (size_t)n * N, limb = (size_t)l * N;
+    const u32 x0 = blockIdx.x * (256 * E) + threadIdx.x;
+    u64 r[T][2][E];
+    auto terms = [&](auto &&product) {
         for (int k = 0; k < kcount; ++k) {
             const u32 g = __ldg(gal + k);
             u32 src[E];
 #pragma unroll
-            for (int u = 0; u < E; ++u) src[u] = g == 1 ? x0 + u * blockDim.x : ntt_perm(x0 + u * blockDim.x, g, logn);
-            for (int b = 0; b < bcount; ++b) {
-                const u64 *a = pbase + ((size_t)k * btotal + b0 + b) * estride;
-                double ad[E];
+            for (int u = 0; u < E; ++u) src[u] = g == 1 ? x0 + u * 256 : ntt_perm(x0 + u * 256, g, logn);
+            const u64 *a = pre + ((size_t)k * btotal + b0) * 2 * poly + limb + x0;
+#pragma unroll 2
+            for (int b = 0; b < bcount; ++b, a += 2 * poly) {
+                u64 v[2][E], w[T][E];
 #pragma unroll
-                for (int u = 0; u < E; ++u) ad[u] = u52_to_double(a[u * blockDim.x]);
+                for (int u = 0; u < E; ++u) {
+                    v[0][u] = a[u * 256]; v[1][u] = a[poly + u * 256];
 #pragma unroll
-                for (int t = 0; t < T; ++t) {
-                    const u64 *w = tp.p[t][b] + (size_t)l * N;
-#pragma unroll
-                    for (int u = 0; u < E; ++u) acc[t][u] = __dadd_rn(acc[t][u], mul_fp64_lazy(ad[u], u52_to_double(w[src[u]]), m.q_inv_f, qd));
+                    for (int t = 0; t < T; ++t) w[t][u] = (tp.p[t][b] + limb)[src[u]];
                 }
+                product(v, w);
             }
-            terms += bcount;
-            if (terms >= 496) {
+        }
+    };
+    if (m.fp) { // exact sums (see FpAcc): 128 products of primes below 2^42, eight below 2^44, before they are reduced
+        const double qd = (double)m.q;
+        const int room = m.q < (1ull << 42) ? 128 : 8;
+        FpAcc s[T][2][E];
+        int held = 0;
+#pragma unroll
+        for (int t = 0; t < T; ++t)
+#pragma unroll
+            for (int u = 0; u < E; ++u) { s[t][0][u].zero(); s[t][1][u].zero(); }
+        terms([&](const u64 (&v)[2][E], const u64 (&w)[T][E]) {
+            if (++held > room) {
+                held = 1;
 #pragma unroll
                 for (int t = 0; t < T; ++t)
 #pragma unroll
-                    for (int u = 0; u < E; ++u) { total[t][u] = add_mod(total[t][u], canon_fp64(acc[t][u], m.q_inv_f, qd), m.q); acc[t][u] = 0.0; }
-                terms = 0;
+                    for (int u = 0; u < E; ++u) { s[t][0][u].relax(m.q_inv_f, qd); s[t][1][u].relax(m.q_inv_f, qd); }
             }
-        }
 #pragma unroll
-        for (int t = 0; t < T; ++t)
-#pragma unroll
-            for (int u = 0; u < E; ++u) total[t][u] = add_mod(total[t][u], canon_fp64(acc[t][u], m.q_inv_f, qd), m.q);
-    } else {
-        PieceAcc s[T][E];
-#pragma unroll
-        for (int t = 0; t < T; ++t)
-#pragma unroll
-            for (int u = 0; u < E; ++u) s[t][u].zero();
-        int held = 0; // products in the accumulators
-        for (int k = 0; k < kcount; ++k) {
-            const u32 g = __ldg(gal + k);
-            u32 src[E];
-#pragma unroll
-            for (int u = 0; u < E; ++u) src[u] = g == 1 ? x0 + u * blockDim.x : ntt_perm(x0 + u * blockDim.x, g, logn);
-            for (int b = 0; b < bcount; ++b) {
-                const u64 *a = pbase + ((size_t)k * btotal + b0 + b) * estride;
-                if (++held == 8) {
-                    held = 1;
-#pragma unroll
-                    for (int t = 0; t < T; ++t)
-#pragma unroll
-                        for (int u = 0; u < E; ++u) s[t][u].relax(m);
-                }
-                u32 a0[E], a1[E];
-#pragma unroll
-                for (int u = 0; u < E; ++u) { const u64 v = a[u * blockDim.x]; a0[u] = (u32)v & 0x3FFFFFFFu; a1[u] = (u32)(v >> 30); }
+            for (int u = 0; u < E; ++u) {
+                const double v0 = u52_to_double(v[0][u]), v1 = u52_to_double(v[1][u]);
 #pragma unroll
                 for (int t = 0; t < T; ++t) {
-                    const u64 *w = tp.p[t][b] + (size_t)l * N;
-#pragma unroll
-                    for (int u = 0; u < E; ++u) { const u64 k_ = w[src[u]]; s[t][u].mac(a0[u], a1[u], (u32)k_ & 0x3FFFFFFFu, (u32)(k_ >> 30)); }
+                    const double wd = u52_to_double(w[t][u]);
+                    s[t][0][u].mac(v0, wd);
+                    s[t][1][u].mac(v1, wd);
                 }
             }
-        }
+        });
 #pragma unroll
         for (int t = 0; t < T; ++t)
 #pragma unroll
-            for (int u = 0; u < E; ++u) total[t][u] = s[t][u].finish(m);
+            for (int u = 0; u < E; ++u) { r[t][0][u] = s[t][0][u].finish(m.q_inv_f, qd); r[t][1][u] = s[t][1][u].finish(m.q_inv_f, qd); }
+    } else {
+        PieceAcc s[T][2][E];
+        int held = 0; // products in the accumulators
+#pragma unroll
+        for (int t = 0; t < T; ++t)
+#pragma unroll
+            for (int u = 0; u < E; ++u) { s[t][0][u].zero(); s[t][1][u].zero(); }
+        terms([&](const u64 (&v)[2][E], const u64 (&w)[T][E]) {
+            if (++held > 8) {
+                held = 1;
+#pragma unroll
+                for (int t = 0; t < T; ++t)
+#pragma unroll
+                    for (int u = 0; u < E; ++u) { s[t][0][u].relax(m); s[t][1][u].relax(m); }
+            }
+#pragma unroll
+            for (int u = 0; u < E; ++u)
+#pragma unroll
+                for (int t = 0; t < T; ++t) {
+                    s[t][0][u].mac(v[0][u], w[t][u]);
+                    s[t][1][u].mac(v[1][u], w[t][u]);
+                }
+        });
+#pragma unroll
+        for (int t = 0; t < T; ++t)
+#pragma unroll
+            for (int u = 0; u < E; ++u) { r[t][0][u] = s[t][0][u].finish(m); r[t][1][u] = s[t][1][u].finish(m); }
     }
 #pragma unroll
     for (int t = 0; t < T; ++t) {
-        u64 *op = tp.out[t] + (size_t)pl * N + x0;
+        u64 *o = tp.out[t] + limb + x0;
 #pragma unroll
-        for (int u = 0; u < E; ++u) op[u * blockDim.x] = total[t][u];
+        for (int u = 0; u < E; ++u) { o[u * 256] = r[t][0][u]; o[poly + u * 256] = r[t][1][u]; }
     }
 }
 
