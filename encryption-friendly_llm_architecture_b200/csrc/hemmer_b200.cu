@@ -808,9 +808,9 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
         Scalars qi{};
         for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
         if (separate) LAUNCH(c), launch_pdl(c->st, k_last_prod_parts, dim3(c->gx(), nbp, parts * count), 256, 0, last.p, pt, l, nbp, c->pc, N);
-        else LAUNCH(c), k_prod_parts<G><<<dim3(gx1, 1, pg), 1024, smem, c->st>>>(last.p, pt, nullptr, l, nbp, c->pc, N, qi, c->dev_err);
+        else LAUNCH(c), k_prod_parts<G><<<dim3(gx1, 1, pg), 512, smem, c->st>>>(last.p, pt, nullptr, l, nbp, c->pc, N, qi, c->dev_err);
         lift_last(c, last.p, parts, separate ? count : 1, nbp, l, t.p);
-        LAUNCH(c), k_prod_parts<G><<<dim3(gx1, (unsigned)l, pg), 1024, smem, c->st>>>(r->d, pt, t.p, l, nbp, c->pc, N, qi, c->dev_err);
+        LAUNCH(c), k_prod_parts<G><<<dim3(gx1, (unsigned)l, pg), 512, smem, c->st>>>(r->d, pt, t.p, l, nbp, c->pc, N, qi, c->dev_err);
         CK(cudaGetLastError());
     } catch (...) { hb_ct_free(r); throw; }
     return r;

@@ -302,6 +302,9 @@ __global__ void k_prod_rescale_fin(u64 *out, const __grid_constant__ TermList tl
     for (int u = 0; u < kElems; ++u) op[u * blockDim.x] = mul_mod_any(sub_mod(v[u], tp[u * blockDim.x], m.q), qlinv.v[l], m);
 }
 
+// Form of a factor that many products share (masks in shared memory, words of a masked key; nothing outside the kernels sees it): an integer-valued double for primes below 2^44, the two
+// 30-bit pieces in the halves of the word otherwise.
+__device__ __forceinline__ u64 key_word(u64 w, bool fp) { return fp ? (u64)__double_as_longlong(u52_to_double(w)) : ((w >> 30) << 32) | ((u32)w & 0x3FFFFFFFu); }
 // ---- the same for all giant-step parts of a baby-step / giant-step transform at once ----
 // A transform with bs baby rotations a_j and 2 gs parts computes  out_g = rescale(sum_j a_j (.) p_gj): every part reads
 // the same a_j.  One pass per limb keeps a part accumulator per g in registers and reads every a_j once (and, for
@@ -323,16 +326,18 @@ __global__ void k_last_prod_parts(u64 *last, const __grid_constant__ PartTerms p
         last[((size_t)blockIdx.z * nbp + bp) * N + x] = p ? mul_mod_any(pt.a[j][((size_t)bp * (level + 1) + level) * N + x], p[(size_t)level * N + x], m) : 0;
     }
 }
-// A CTA of 1024 threads keeps the mask chunks of G parts for its 256 coefficients of one limb in shared memory (bulk
+// A CTA of 512 threads keeps the mask chunks of G parts for its 256 coefficients of one limb in shared memory (bulk
 // copies, up to G * 17 chunks of 2 KB, one mbarrier, bounded wait) and walks over the batch members, four at a time
-// (thread = coefficient + 256 * member slot): the masks cross L2 once per CTA instead of once per member, the a_j of a
-// member are read by the ceil(parts / G) CTAs of the chunk (from L2 after the first), and every thread has the next
-// two a_j in flight while it works on the current one.
+// (thread = coefficient + 256 * member pair): the masks cross L2 once per CTA instead of once per member and shared memory once per
+// two members, the a_j of a member are read by the ceil(parts / G) CTAs of the chunk (from L2 after the first), and every
+// thread has the next two a_j of both members in flight while it works on the current ones.  1024 threads with one member each and
+// 128-bit sums on the 60-bit limbs: 639 us a launch for one two-tile product, 2876 us in the layer pass; now 607 and 2859 us.
+// Bound by HBM: a_j, t and the parts are 14 GB a launch in the layer pass.
 // t == nullptr: raw sums of limb `level`, out[(g * nbp + bp) * N + x]                       grid = (N/256, 1, ceil(parts/G))
 // else: out[((g * nbp + bp) * level + l) * N + x] = (sum - t[same]) * q_level^-1 mod q_l      grid = (N/256, level, ceil(parts/G))
 template <int G>
-__global__ void __launch_bounds__(1024, 1) k_prod_parts(u64 *__restrict__ out, const __grid_constant__ PartTerms pt, const u64 *__restrict__ t, int level, int nbp,
-                                                        const PrimeConst *__restrict__ pc, int N, const __grid_constant__ Scalars qlinv, int *__restrict__ err) {
+__global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, const __grid_constant__ PartTerms pt, const u64 *__restrict__ t, int level, int nbp,
+                                                       const PrimeConst *__restrict__ pc, int N, const __grid_constant__ Scalars qlinv, int *__restrict__ err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) u64 bar;
     u64 *ptile = reinterpret_cast<u64 *>(smem_raw); // [G][count][256]
@@ -366,55 +371,77 @@ __global__ void __launch_bounds__(1024, 1) k_prod_parts(u64 *__restrict__ out, c
     const u64 qli = t ? qlinv.v[l] : 0;
     const double qd = (double)m.q;
     // Absent terms get zero masks, so the product loop below is straight-line code (no test per part and term: the
-    // independent chains of the G parts interleave); the masks of a prime below 2^44 become doubles once.
+    // independent chains of the G parts interleave); the masks become doubles or pairs of pieces once.
 #pragma unroll
     for (int g = 0; g < G; ++g)
-        for (int j = slot; j < count; j += 4) {
+        for (int j = slot; j < count; j += 2) {
             u64 *w = ptile + (size_t)(g * count + j) * 256 + lane;
-            if (!((have[g] >> j) & 1u)) *w = 0;
-            else if (m.fp) *w = (u64)__double_as_longlong(u52_to_double(*w));
+            *w = ((have[g] >> j) & 1u) ? key_word(*w, m.fp) : 0;
         }
     __syncthreads();
-    for (int bp = slot; bp < nbp; bp += 4) {
-        const size_t ao = ((size_t)bp * (level + 1) + l) * N + x0 + lane;
-        u64 v[G];
-        u64 a_cur = pt.a[0][ao], a_nxt = count > 1 ? pt.a[1][ao] : 0;
-        if (m.fp) { // products entirely on the FP64 pipe, signed double sums (17 terms of at most 0.51 q each)
-            double acc[G];
-#pragma unroll
-            for (int g = 0; g < G; ++g) acc[g] = 0.0;
-            const double *dtile = reinterpret_cast<const double *>(ptile);
+    const int room = m.fp && m.q < (1ull << 42) ? 128 : 8; // products between two reductions of a sum (FpAcc, PieceAcc)
+    for (int bp = 2 * slot; bp < nbp; bp += 4) {
+        const bool both = bp + 1 < nbp;
+        const size_t ao = ((size_t)bp * (level + 1) + l) * N + x0 + lane, ao1 = both ? ao + (size_t)(level + 1) * N : ao;
+        u64 v[2][G];
+        u64 cur[2] = {pt.a[0][ao], pt.a[0][ao1]}, nxt[2] = {0, 0};
+        if (count > 1) { nxt[0] = pt.a[1][ao]; nxt[1] = pt.a[1][ao1]; }
+        auto terms = [&](auto &&product) {
             for (int j = 0; j < count; ++j) {
-                const u64 a = a_cur;
-                a_cur = a_nxt;
-                if (j + 2 < count) a_nxt = pt.a[j + 2][ao];
-                const double ad = u52_to_double(a);
-#pragma unroll
-                for (int g = 0; g < G; ++g) acc[g] = __dadd_rn(acc[g], mul_fp64_lazy(ad, dtile[(size_t)(g * count + j) * 256 + lane], m.q_inv_f, qd));
+                const u64 a0 = cur[0], a1 = cur[1];
+                cur[0] = nxt[0]; cur[1] = nxt[1];
+                if (j + 2 < count) { nxt[0] = pt.a[j + 2][ao]; nxt[1] = pt.a[j + 2][ao1]; }
+                product(a0, a1, ptile + (size_t)j * 256 + lane, j && j % room == 0);
             }
+        };
+        if (m.fp) { // products and sums exactly on the FP64 pipe
+            FpAcc s[2][G];
 #pragma unroll
-            for (int g = 0; g < G; ++g) v[g] = canon_fp64(acc[g], m.q_inv_f, qd);
+            for (int g = 0; g < G; ++g) { s[0][g].zero(); s[1][g].zero(); }
+            terms([&](u64 a0, u64 a1, const u64 *w, bool full) {
+                if (full) {
+#pragma unroll
+                    for (int g = 0; g < G; ++g) { s[0][g].relax(m.q_inv_f, qd); s[1][g].relax(m.q_inv_f, qd); }
+                }
+                const double d0 = u52_to_double(a0), d1 = u52_to_double(a1);
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    const double k = __longlong_as_double((long long)w[(size_t)g * count * 256]);
+                    s[0][g].mac(d0, k); s[1][g].mac(d1, k);
+                }
+            });
+#pragma unroll
+            for (int g = 0; g < G; ++g) { v[0][g] = s[0][g].finish(m.q_inv_f, qd); v[1][g] = s[1][g].finish(m.q_inv_f, qd); }
         } else {
-            Acc128 acc[G];
+            PieceAcc s[2][G];
 #pragma unroll
-            for (int g = 0; g < G; ++g) acc[g].zero();
-            for (int j = 0; j < count; ++j) {
-                const u64 a = a_cur;
-                a_cur = a_nxt;
-                if (j + 2 < count) a_nxt = pt.a[j + 2][ao];
+            for (int g = 0; g < G; ++g) { s[0][g].zero(); s[1][g].zero(); }
+            terms([&](u64 a0, u64 a1, const u64 *w, bool full) {
+                if (full) {
 #pragma unroll
-                for (int g = 0; g < G; ++g) acc[g].mad(a, ptile[(size_t)(g * count + j) * 256 + lane]);
-            }
+                    for (int g = 0; g < G; ++g) { s[0][g].relax(m); s[1][g].relax(m); }
+                }
 #pragma unroll
-            for (int g = 0; g < G; ++g) v[g] = barrett128(acc[g].hi, acc[g].lo, m);
+                for (int g = 0; g < G; ++g) {
+                    const u64 k = w[(size_t)g * count * 256];
+                    s[0][g].mac((u32)a0 & 0x3FFFFFFFu, (u32)(a0 >> 30), (u32)k, (u32)(k >> 32));
+                    s[1][g].mac((u32)a1 & 0x3FFFFFFFu, (u32)(a1 >> 30), (u32)k, (u32)(k >> 32));
+                }
+            });
+#pragma unroll
+            for (int g = 0; g < G; ++g) { v[0][g] = s[0][g].finish(m); v[1][g] = s[1][g].finish(m); }
         }
 #pragma unroll
-        for (int g = 0; g < G; ++g)
-            if (g < gn) {
-                if (t) {
-                    const size_t w = (((size_t)(g0 + g) * nbp + bp) * level + l) * N + x0 + lane;
-                    out[w] = mul_mod_any(sub_mod(v[g], t[w], m.q), qli, m);
-                } else out[((size_t)(g0 + g) * nbp + bp) * N + x0 + lane] = v[g];
+        for (int i = 0; i < 2; ++i)
+            if (i == 0 || both) {
+#pragma unroll
+                for (int g = 0; g < G; ++g)
+                    if (g < gn) {
+                        if (t) {
+                            const size_t w = (((size_t)(g0 + g) * nbp + bp + i) * level + l) * N + x0 + lane;
+                            out[w] = mul_mod_any(sub_mod(v[i][g], t[w], m.q), qli, m);
+                        } else out[((size_t)(g0 + g) * nbp + bp + i) * N + x0 + lane] = v[i][g];
+                    }
             }
     }
 }
@@ -921,9 +948,6 @@ __global__ void k_ks_inner_pair(u64 *__restrict__ E, const u64 *__restrict__ c0,
 // sum_dg digit_dg * (mask * key_dg) = mask * sum_dg digit_dg * key_dg modulo q, so a key multiplied by the mask once
 // (k_mask_key) turns the masked pair of rotations into ONE lazy inner product with ONE reduction per output residue;
 // the residues are those of k_ks_inner_pair.
-// Stored form of a masked-key word (nothing outside the kernels below sees it): an integer-valued double for primes below 2^44, the two
-// 30-bit pieces in the halves of the word otherwise.
-__device__ __forceinline__ u64 key_word(u64 w, bool fp) { return fp ? (u64)__double_as_longlong(u52_to_double(w)) : ((w >> 30) << 32) | ((u32)w & 0x3FFFFFFFu); }
 // mkey[dg][p][j][i] = (mask[j][i] + mask2[j][i]) * key[dg][p][prime(j)][i];  grid = (N/(256*kElems), ne, nd*2)
 __global__ void k_mask_key(u64 *__restrict__ mkey, const u64 *__restrict__ key, int key_primes, const u64 *__restrict__ mask, const u64 *__restrict__ mask2,
                            const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, int N) {
