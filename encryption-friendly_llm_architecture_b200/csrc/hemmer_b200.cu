@@ -874,7 +874,7 @@ hb_ct *do_tensor(hb_ctx *c, const hb_ct *a, const hb_ct *b, hb_ct *acc, int grou
     else r = new_ct(c, a->level, 3, batch, 2);
     const int n = a->level + 1;
     ALG(c, 2 * a->limbs() + (size_t)(acc ? 2 : 1) * batch * 3 * n);
-    LAUNCH(c), launch_pdl(c->st, k_tensor, c->egrid(batch * n), 256, 0, r->d, (const u64 *)a->d, (const u64 *)b->d, n, c->qmap(a->level), c->pc, c->N, acc ? 1 : 0, groups, batch);
+    LAUNCH(c), launch_pdl(c->st, k_tensor, dim3((unsigned)(c->N / 512), (unsigned)(batch * n)), 256, 0, r->d, (const u64 *)a->d, (const u64 *)b->d, n, c->qmap(a->level), c->pc, c->N, acc ? 1 : 0, groups, batch);
     return r;
 }
 hb_ct *do_relin(hb_ctx *c, const hb_ct *a) {

@@ -76,41 +76,77 @@ __global__ void k_mul_pt(u64 *__restrict__ out, const u64 *__restrict__ a, const
 // tensor product, optional accumulation.  grid.y = batch * n; x, y: [groups][batch][2][n][N]; d: [batch][3][n][N]
 //   d[b] (+)= sum over the groups g of tensor(x[g][b], y[g][b])
 // (groups = 1 is the plain tensor product; several groups are several iterations of a product loop in one launch).
-__global__ void k_tensor(u64 *d, const u64 *x, const u64 *y, int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N,
-                         int accumulate, int groups, int batch) {
+// Two coefficients per thread, so that eight loads of a group are in flight, and one reduction per sum: 256 ciphertexts at level 8
+// 1634 -> 1498 us (5.6 TB/s), a launch of the layer's product loop 620 -> 517 us.  grid.x = N/512
+__global__ void __launch_bounds__(256) k_tensor(u64 *d, const u64 *x, const u64 *y, int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N,
+                                                int accumulate, int groups, int batch) {
+    constexpr int EL = 2;
     const int bl = blockIdx.y, b = bl / n, l = bl % n;
-    const size_t gstride = (size_t)batch * 2 * n * N;
+    const size_t gstride = (size_t)batch * 2 * n * N, poly = (size_t)n * N;
+    const PrimeConst m = pc[map.prime[l]];
+    const u32 i0 = blockIdx.x * (256 * EL) + threadIdx.x;
+    const u64 *xp = x + ((size_t)(b * 2) * n + l) * N + i0, *yp = y + ((size_t)(b * 2) * n + l) * N + i0;
+    u64 *dp = d + ((size_t)(b * 3) * n + l) * N + i0;
+    u64 r[3][EL];
     pdl_wait();
+    auto terms = [&](auto &&product) {
+        for (int g = 0; g < groups; ++g, xp += gstride, yp += gstride) {
+            u64 b1[EL], a1[EL], b2[EL], a2[EL];
 #pragma unroll
-    for (int u_ = 0; u_ < kElems; ++u_) {
-        const int i = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
-        if (i >= N) break;
-        const PrimeConst m = pc[map.prime[l]];
-        const size_t x0 = ((size_t)(b * 2) * n + l) * N + i, x1 = x0 + (size_t)n * N;
-        const size_t d0 = ((size_t)(b * 3) * n + l) * N + i, d1 = d0 + (size_t)n * N, d2 = d1 + (size_t)n * N;
-        u64 r0, r1, r2;
-        if (m.fp) { // lazy products below 1.6q; the group count is bounded by the launcher so that the sums stay below 2^52
-            u64 s0 = 0, s1 = 0, s2 = 0;
-            for (int g = 0; g < groups; ++g) {
-                const u64 b1 = x[g * gstride + x0], a1 = x[g * gstride + x1], b2 = y[g * gstride + x0], a2 = y[g * gstride + x1];
-                const double b1d = u52_to_double(b1), a1d = u52_to_double(a1), b2d = u52_to_double(b2), a2d = u52_to_double(a2);
-                s0 += mul_small_lazy_d(b1, b1d, b2, b2d, m.q_inv_f, m.q);
-                s2 += mul_small_lazy_d(a1, a1d, a2, a2d, m.q_inv_f, m.q);
-                s1 += mul_small_lazy_d(a1, a1d, b2, b2d, m.q_inv_f, m.q) + mul_small_lazy_d(a2, a2d, b1, b1d, m.q_inv_f, m.q);
-            }
-            r0 = reduce_fp(s0, m.q_inv_f, m.q); r1 = reduce_fp(s1, m.q_inv_f, m.q); r2 = reduce_fp(s2, m.q_inv_f, m.q);
-        } else {
-            PieceAcc s0, s1, s2; s0.zero(); s1.zero(); s2.zero();
-            for (int g = 0; g < groups; ++g) {
-                if (g && g % 3 == 0) { s0.relax(m); s1.relax(m); s2.relax(m); }
-                const u64 b1 = x[g * gstride + x0], a1 = x[g * gstride + x1], b2 = y[g * gstride + x0], a2 = y[g * gstride + x1];
-                s0.mac(b1, b2); s2.mac(a1, a2); s1.mac(a1, b2); s1.mac(a2, b1);
-            }
-            r0 = s0.finish(m); r1 = s1.finish(m); r2 = s2.finish(m);
+            for (int u = 0; u < EL; ++u) { b1[u] = xp[u * 256]; a1[u] = xp[poly + u * 256]; b2[u] = yp[u * 256]; a2[u] = yp[poly + u * 256]; }
+            product(g, b1, a1, b2, a2);
         }
-        if (accumulate) { r0 = add_mod(r0, d[d0], m.q); r1 = add_mod(r1, d[d1], m.q); r2 = add_mod(r2, d[d2], m.q); }
-        d[d0] = r0; d[d1] = r1; d[d2] = r2;
+    };
+    if (m.fp) { // exact sums; the middle one takes two products per group: 64 groups below 2^42, four below 2^44, before it is reduced
+        const double qd = (double)m.q;
+        const int room = m.q < (1ull << 42) ? 64 : 4;
+        FpAcc s[3][EL];
+#pragma unroll
+        for (int u = 0; u < EL; ++u) { s[0][u].zero(); s[1][u].zero(); s[2][u].zero(); }
+        terms([&](int g, const u64 (&b1)[EL], const u64 (&a1)[EL], const u64 (&b2)[EL], const u64 (&a2)[EL]) {
+            if (g && g % room == 0) {
+#pragma unroll
+                for (int u = 0; u < EL; ++u)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) s[k][u].relax(m.q_inv_f, qd);
+            }
+#pragma unroll
+            for (int u = 0; u < EL; ++u) {
+                const double b1d = u52_to_double(b1[u]), a1d = u52_to_double(a1[u]), b2d = u52_to_double(b2[u]), a2d = u52_to_double(a2[u]);
+                s[0][u].mac(b1d, b2d); s[2][u].mac(a1d, a2d);
+                s[1][u].mac(a1d, b2d); s[1][u].mac(a2d, b1d);
+            }
+        });
+#pragma unroll
+        for (int u = 0; u < EL; ++u)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) r[k][u] = s[k][u].finish(m.q_inv_f, qd);
+    } else {
+        PieceAcc s[3][EL];
+#pragma unroll
+        for (int u = 0; u < EL; ++u) { s[0][u].zero(); s[1][u].zero(); s[2][u].zero(); }
+        terms([&](int g, const u64 (&b1)[EL], const u64 (&a1)[EL], const u64 (&b2)[EL], const u64 (&a2)[EL]) {
+            if (g && g % 4 == 0) {
+#pragma unroll
+                for (int u = 0; u < EL; ++u)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) s[k][u].relax(m);
+            }
+#pragma unroll
+            for (int u = 0; u < EL; ++u) { s[0][u].mac(b1[u], b2[u]); s[2][u].mac(a1[u], a2[u]); s[1][u].mac(a1[u], b2[u]); s[1][u].mac(a2[u], b1[u]); }
+        });
+#pragma unroll
+        for (int u = 0; u < EL; ++u)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) r[k][u] = s[k][u].finish(m);
     }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int u = 0; u < EL; ++u) {
+            u64 *o = dp + k * poly + u * 256;
+            *o = accumulate ? add_mod(r[k][u], *o, m.q) : r[k][u];
+        }
 }
 // out[li][i] = in[li][perm_g(i)]
 __global__ void k_permute(u64 *__restrict__ out, const u64 *__restrict__ in, u32 g, int logn, int N) {
