@@ -671,8 +671,8 @@ hb_ct *do_assemble_mk(hb_ctx *c, const hb_ct *a, const u64 *dt, const hb_mkey *c
     for (int g = 0; g < groups; ++g) ALG(c, (size_t)mrl.r[g].count * ((size_t)d.nd * 2 * ne + n) + (size_t)batch * 2 * (n - 1));
     ALG(c, (size_t)batch * (2 * n + d.dt_count));
     if (d.nd <= 2) {
-        const int per = members_per_cta(batch, N / 512 * ne * groups), chunks = (batch + per - 1) / per;
-        LAUNCH(c), launch_pdl(c->st, d.nd == 1 ? k_ks_inner_mkr<1> : k_ks_inner_mkr<2>, dim3((unsigned)(N / 512), (unsigned)(groups * chunks), (unsigned)ne), 256, 0, E.p, (const u64 *)a->d,
+        const int per = members_per_cta(batch, N / (256 * 1) * ne * groups), chunks = (batch + per - 1) / per;
+        LAUNCH(c), launch_pdl(c->st, d.nd == 1 ? k_ks_inner_mkr<1> : k_ks_inner_mkr<2>, dim3((unsigned)(N / (256 * 1)), (unsigned)(groups * chunks), (unsigned)ne), 256, 0, E.p, (const u64 *)a->d,
                               (const u64 *)a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch, per, pl, c->pc, c->logn, N);
     } else {
         LAUNCH(c), launch_pdl(c->st, k_ks_inner_mk, dim3((unsigned)((N + 1023) / 1024), groups * batch, ne), 256, 0, E.p, (const u64 *)a->d, (const u64 *)a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch, pl,

@@ -1112,15 +1112,17 @@ __global__ void __launch_bounds__(256, 2) k_ks_inner_mk(u64 *E, const u64 *c0, c
 #pragma unroll
     for (int u = 0; u < EL; ++u) { o0[u * blockDim.x] = r0[u]; o1[u * blockDim.x] = r1[u]; }
 }
-// At most two digits: a thread keeps the words of the one or two masked keys for its two coefficients in registers and walks over `per`
+// At most two digits: a thread keeps the words of the one or two masked keys for its coefficient in registers and walks over `per`
 // input members with the next member's words in flight.  Up to eleven masked-key words meet six words per member and coefficient;
 // staging both in shared memory by bulk copies for three members at a time took 1.6 times as long (they crossed L2 for every
-// third member, and a CTA's copies, sums and stores did not overlap).
-// grid = (N/512, groups * ceil(batch/per), ne)
+// third member, and a CTA's copies, sums and stores did not overlap).  Two coefficients per thread and two CTAs per SM: 869 us a launch
+// for 168 outputs at level 6; one coefficient and three CTAs 837 us, four CTAs 776 us (64 registers): the integer chains of
+// the 60-bit limbs want warps more than they want independent work in a thread.
+// grid = (N/256, groups * ceil(batch/per), ne)
 template <int ND, int CNT>
 __device__ __forceinline__ void ks_inner_mkr_body(u64 *o, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const MaskedRot &mr, int b0, int b1, const KsPlan *__restrict__ pl,
                                                   const PrimeConst &m, int j, u32 x0, int logn, int N) {
-    constexpr int EL = 2;
+    constexpr int EL = 1;
     const int ne = pl->ne;
     const bool has_c0 = j < pl->n;
     const size_t kpoly = (size_t)ne * N;
@@ -1206,13 +1208,13 @@ __device__ __forceinline__ void ks_inner_mkr_body(u64 *o, const u64 *c0, const u
     }
 }
 template <int ND>
-__global__ void __launch_bounds__(256, 2) k_ks_inner_mkr(u64 *E, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const __grid_constant__ MaskedRotList mrl, int batch, int per,
+__global__ void __launch_bounds__(256, 4) k_ks_inner_mkr(u64 *E, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const __grid_constant__ MaskedRotList mrl, int batch, int per,
                                                          const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, int logn, int N) {
     const int chunks = (batch + per - 1) / per, grp = blockIdx.y / chunks, b0 = (blockIdx.y % chunks) * per, b1 = min(batch, b0 + per);
     const int j = blockIdx.z; // limb-major block order: the digits of one limb stay in L2 across the copies
     const MaskedRot &mr = mrl.r[grp];
     const PrimeConst m = pc[pl->ext_prime[j]];
-    const u32 x0 = blockIdx.x * 512 + threadIdx.x;
+    const u32 x0 = blockIdx.x * (256 * 1) + threadIdx.x;
     u64 *o = E + (((size_t)(grp * batch + b0) * 2) * pl->ne + j) * N + x0;
     pdl_wait();
     if (mr.count == 1) ks_inner_mkr_body<ND, 1>(o, c0, a_ntt, a_outer, dt, mr, b0, b1, pl, m, j, x0, logn, N);
