@@ -470,17 +470,23 @@ void ks_apply(hb_ctx *c, const SwitchList &sl, size_t a_outer, int level, int ba
     const PlanDims d = plan_dims(c, level);
     const int N = c->N, n = d.n, ne = d.ne, total = sl.count * batch;
     Tmp acc(c, (size_t)total * 2 * ne), t(c, (size_t)total * 2 * n);
-    const int per = members_per_cta(batch, N / 512 * ne * sl.count), chunks = (batch + per - 1) / per;
-    auto inner = [&](auto *kernel) { LAUNCH(c), launch_pdl(c->st, kernel, dim3((unsigned)(N / 512), sl.count * chunks, ne), 256, 0, acc.p, sl, batch, per, a_outer, c->nprimes, pl, c->pc, c->logn, N); };
+    // Many members and up to four digits: one coefficient per thread, four CTAs per SM (256 members at level 8 1620 -> 1471 us, 42
+    // members 513 -> 492).  Few members: two coefficients, whose loads cover the latency of a short walk (two digits of two
+    // members 40 us, with one coefficient 51).
+    const int el = batch >= 32 && d.nd <= 4 ? 1 : 2;
+    const int per = members_per_cta(batch, N / (256 * el) * ne * sl.count), chunks = (batch + per - 1) / per;
+    auto inner = [&](auto *kernel) {
+        LAUNCH(c), launch_pdl(c->st, kernel, dim3((unsigned)(N / (256 * el)), sl.count * chunks, ne), 256, 0, acc.p, sl, batch, per, a_outer, c->nprimes, pl, c->pc, c->logn, N);
+    };
     switch (d.nd) {
-    case 1: inner(k_ks_inner<1>); break;
-    case 2: inner(k_ks_inner<2>); break;
-    case 3: inner(k_ks_inner<3>); break;
-    case 4: inner(k_ks_inner<4>); break;
-    case 5: inner(k_ks_inner<5>); break;
-    case 6: inner(k_ks_inner<6>); break;
-    case 7: inner(k_ks_inner<7>); break;
-    default: inner(k_ks_inner<8>); break;
+    case 1: inner(el == 1 ? k_ks_inner<1, 1> : k_ks_inner<1, 2>); break;
+    case 2: inner(el == 1 ? k_ks_inner<2, 1> : k_ks_inner<2, 2>); break;
+    case 3: inner(el == 1 ? k_ks_inner<3, 1> : k_ks_inner<3, 2>); break;
+    case 4: inner(el == 1 ? k_ks_inner<4, 1> : k_ks_inner<4, 2>); break;
+    case 5: inner(k_ks_inner<5, 2>); break;
+    case 6: inner(k_ks_inner<6, 2>); break;
+    case 7: inner(k_ks_inner<7, 2>); break;
+    default: inner(k_ks_inner<8, 2>); break;
     }
     moddown(c, acc.p, t.p, level, total, out, out_outer, sl, batch, add_outer);
 }

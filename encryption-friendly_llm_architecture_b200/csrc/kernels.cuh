@@ -368,7 +368,7 @@ __global__ void k_last_prod_parts(u64 *last, const __grid_constant__ PartTerms p
 // two members, the a_j of a member are read by the ceil(parts / G) CTAs of the chunk (from L2 after the first), and every
 // thread has the next two a_j of both members in flight while it works on the current ones.  1024 threads with one member each and
 // 128-bit sums on the 60-bit limbs: 639 us a launch for one two-tile product, 2876 us in the layer pass; now 607 and 2859 us.
-// Bound by HBM: a_j, t and the parts are 14 GB a launch in the layer pass.
+// Bound by the FP64 pipe: four instructions for each of the count x parts products of a coefficient.
 // t == nullptr: raw sums of limb `level`, out[(g * nbp + bp) * N + x]                       grid = (N/256, 1, ceil(parts/G))
 // else: out[((g * nbp + bp) * level + l) * N + x] = (sum - t[same]) * q_level^-1 mod q_l      grid = (N/256, level, ceil(parts/G))
 template <int G>
@@ -562,15 +562,14 @@ constexpr int kMaxSwitchGroups = 16;
 struct SwitchList { SwitchGroup s[kMaxSwitchGroups]; int count; };
 // Inner product with the switching key over Q_level u P.
 //   acc[ob][p][j][i] = sum_dg digit_dg[j][perm_g(i)] * key[dg][p][prime(j)][i],   member ob = group * batch + b
-// digit_dg[j] is a_ntt[j] for own limbs and dt[...] otherwise.  A CTA owns 512 coefficients of one limb for `per` members of a group:
-// a thread keeps the key words of its two coefficients in registers (as doubles, or cut into pieces) and walks over the
+// digit_dg[j] is a_ntt[j] for own limbs and dt[...] otherwise.  A CTA owns 256 * EL coefficients of one limb for `per` members of a group:
+// a thread keeps the key words of its EL coefficients in registers (as doubles, or cut into pieces) and walks over the
 // members with the next member's digits in flight, so the keys -- two thirds of the words a member needs -- are read once.
 // One member per CTA read and converted them every time: 517 us for 64 members at level 6.
-// grid = (N/512, groups * ceil(batch/per), ne); ND = digits in use
-template <int ND>
-__global__ void __launch_bounds__(256, ND <= 2 ? 3 : 2) k_ks_inner(u64 *acc, const __grid_constant__ SwitchList sl, int batch, int per, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl,
+// grid = (N/(256*EL), groups * ceil(batch/per), ne); ND = digits in use
+template <int ND, int EL>
+__global__ void __launch_bounds__(256, EL == 1 ? 4 : ND <= 2 ? 3 : 2) k_ks_inner(u64 *acc, const __grid_constant__ SwitchList sl, int batch, int per, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl,
                                                                    const PrimeConst *__restrict__ pc, int logn, int N) {
-    constexpr int EL = 2;
     const int chunks = (batch + per - 1) / per, grp = blockIdx.y / chunks, b0 = (blockIdx.y % chunks) * per, b1 = min(batch, b0 + per);
     const int j = blockIdx.z; // limb-major block order
     const SwitchGroup &sg = sl.s[grp];
