@@ -999,8 +999,8 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             p.fp = q < ((u64)1 << 44) ? 1 : 0;
             // lazy FP64-assisted products are below 1.6 q; reduce_fp takes sums below 2^52.  Every fixed-length lazy sum in
             // the kernels has at most 128 terms (16 rotated terms x 8 digits), which any prime below 2^44 allows (>= 160).
-            p.lazy_terms = (u64)((((unsigned __int128)1 << 52) * 5) / ((unsigned __int128)q * 8));
-            if (p.fp && p.lazy_terms < 160) throw std::invalid_argument("prime too large for the lazy FP64-assisted sums");
+            const u64 lazy_terms = (u64)((((unsigned __int128)1 << 52) * 5) / ((unsigned __int128)q * 8)); // how many may be summed
+            if (p.fp && lazy_terms < 160) throw std::invalid_argument("prime too large for the lazy FP64-assisted sums");
             // primes of 45 bits and more: values are folded with shifts by the bit length b, which needs q close below 2^b; the
             // primes of a context are the first ones below a power of two, at most a few hundred 2N-steps away from it
             int bits = 0;

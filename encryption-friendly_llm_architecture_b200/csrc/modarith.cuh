@@ -26,7 +26,6 @@ struct PrimeConst {
     double q_inv_f;     // 1/q
     double n_inv_f;     // n_inv / q
     u64 fp;             // 1 when q < 2^44: element-wise kernels take quotients from the FP64 pipe
-    u64 lazy_terms;     // how many lazy products (each below 1.6 q) may be summed before the sum reaches 2^52
     u32 fold_shift;     // primes of b >= 45 bits: b - 32 (every such prime of a context lies within 2^(b-12) below 2^b)
     u32 fold_d;         //   and 2^b - q
     u32 d60;            // 2^60 - q when that is positive and below 2^26, else 0
@@ -203,16 +202,6 @@ struct FpAcc {
         double r = reduced(q_inv, qd);
         if (r < 0.0) r = __dadd_rn(r, qd);
         return mantissa52(__dadd_rn(r, kTwo52));
-    }
-};
-
-// 128-bit accumulator for lazy sums of products
-struct Acc128 {
-    u64 lo, hi;
-    __device__ __forceinline__ void zero() { lo = 0; hi = 0; }
-    __device__ __forceinline__ void mad(u64 a, u64 b) {
-        u64 pl = a * b, ph = mul_hi(a, b);
-        lo += pl; hi += ph + (lo < pl);
     }
 };
 
