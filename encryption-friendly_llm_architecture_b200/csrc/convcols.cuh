@@ -119,9 +119,12 @@ __device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *s
 }
 
 // a0 + a1 * 2^26 modulo a prime below 2^44 (a1 < 2^52, a0 < 2^61) as an integer-valued double within 2q of zero.  The quotient
-// comes from the FP64 pipe (both sums enter through the 2^52 exponent without a conversion, the offsets are folded into `base`,
-// off by at most 1.6), the remainder is exact in the low 64 bits.
-struct SmallFinish { double k1, k0, base; u32 n0, n1, hi0; };
+// comes from the FP64 pipe (both sums enter through the 2^52 exponent without a conversion, the offsets are folded into `base`),
+// the remainder is exact in the low 64 bits.  The quotient is off by its two roundings, by the low word of a0 that it leaves out
+// (up to 2^32 / q) and by the rounding of `base`, whose size is 2^84 / q: 1.7 in all from q = 2^34 on, but 50 at 27 bits.  The
+// forward row pass adds 16 q to outputs that carry coefficient 0 unreduced, so below 2^34 the remainder is reduced once more (it
+// is below 2^36 there, whatever q).
+struct SmallFinish { double k1, k0, base; u32 n0, n1, hi0; bool again; };
 __device__ __forceinline__ SmallFinish small_finish(const PrimeConst &m) {
     SmallFinish f;
     f.k1 = 0x1p26 * m.q_inv_f; f.k0 = 0x1p32 * m.q_inv_f;
@@ -129,6 +132,7 @@ __device__ __forceinline__ SmallFinish small_finish(const PrimeConst &m) {
     const u64 nq = 0ull - m.q;
     f.n0 = (u32)nq; f.n1 = (u32)(nq >> 32);
     f.hi0 = 0x43380000u - 0x43380000u * f.n0; // exponent word of the result, minus what the exponent word of the quotient contributes
+    f.again = m.q < (1ull << 34);
     return f;
 }
 __device__ __forceinline__ double finish_small(u64 a0, u64 a1, const SmallFinish &f) {
@@ -178,6 +182,7 @@ template <int COLS>
 __device__ __forceinline__ void convert_target_small(u64 *sm, const u64 *ysm, const uint4 *__restrict__ cst, int ns, const PrimeConst &m, int sub, int lane) {
     using I = StripIndex<COLS>;
     const SmallFinish f = small_finish(m);
+    const DsConst ds = ds_const(m);
 #pragma unroll 1
     for (int e0 = 0; e0 < 16; e0 += 4) {
         u64 a0[4], a1[4];
@@ -194,7 +199,11 @@ __device__ __forceinline__ void convert_target_small(u64 *sm, const u64 *ysm, co
             }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) sm[I::a(e0 + u, sub, lane)] = (u64)__double_as_longlong(finish_small(a0[u], a1[u], f));
+        for (int u = 0; u < 4; ++u) {
+            double v = finish_small(a0[u], a1[u], f);
+            if (f.again) v = ds_reduce(v, ds);
+            sm[I::a(e0 + u, sub, lane)] = (u64)__double_as_longlong(v);
+        }
     }
 }
 template <int COLS>

@@ -73,6 +73,31 @@ def test_other_parameter_sets_of_2_16_points(pkg, oracle_so, name):
         assert np.array_equal(g.ct_export(folded), res[0][3]), f"{name}: masked keys at level {level}"
 
 
+@pytest.mark.parametrize("q_bits", [26, 27, 28, 34])
+def test_short_scaling_primes_of_2_16_points(pkg, oracle_so, q_bits):
+    """Digits of six and seven limbs convert to scaling primes of 26 to 34 bits on the integer pipe, where the quotient of the first
+    reduction is least exact (off by up to 2^32 / q).  A transform carries coefficient 0 into every output without reducing it, so
+    the members have that coefficient zero, random, and at its largest."""
+    prm = dict(log_n=16, max_level=12, dnum=2, num_special=4, hamming_weight=64, q_bits=q_bits)
+    g, o = pkg.open_gpu(pkg.make_params(**prm)), open_oracle(pkg, oracle_so, **prm)
+    level = int(g.L)
+    data = rand_ct_residues(g, level, 2, 3, seed=80 + q_bits)
+    for l in range(level + 1):
+        q = int(g.primes[l])
+        for p in range(2):
+            mean = int(data[0, p, l].astype(object).sum()) * pow(g.N, -1, q) % q  # coefficient 0 of the polynomial
+            data[0, p, l] = (data[0, p, l] + np.uint64(q - mean)) % np.uint64(q)
+        data[2, :, l] = np.uint64(q - 1)
+    res = []
+    for lib in (g, o):
+        lib.keygen()
+        lib.gen_rot_keys([3])
+        x = _ct(lib, data)
+        res.append([lib.ct_export(c) for c in (lib.rotate(x, 3), lib.relin(lib.tensor(x, x)))])
+    for k, (a, b) in enumerate(zip(*res)):
+        assert np.array_equal(a, b), f"operation {k}"
+
+
 @pytest.mark.parametrize("batch", [1, 2, 3, 4, 5])
 @pytest.mark.parametrize("q_bits", [42, 44])
 def test_rotated_and_masked_sums_at_their_longest(pkg, oracle_so, q_bits, batch):
