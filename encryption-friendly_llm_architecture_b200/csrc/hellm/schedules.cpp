@@ -543,11 +543,19 @@ Ciphertext multPackedMatMatPreRot(Env &e, const CtxtTensor &in, int target_level
 CtxtTensor multPackedMatMatPreRev(Env &e, const CtxtTensor &b, int target_level) {
     return packedDiagonalToRow(e, CtxtTensor(b.getShape(), e.ev.levelDown(b.get(), target_level + 2)));
 }
+// Shifted copies in `pre` for every member of tb.  One right operand meets whatever copies there are; several need the full set of a
+// tile, `copies`, for each of them (copy k of input j at k * batch + j), since a shorter or longer batch does not say whose a copy is.
+static int copies_per_member(const Ciphertext &pre, const CtxtTensor &tb, i64 copies) {
+    const int batch = tb.get().getBatch();
+    if (batch == 1) return pre.getBatch();
+    if (pre.getBatch() != copies * batch) throw std::invalid_argument("[CCReuse] the left operand's copies do not match the batch of the right operand");
+    return (int)copies;
+}
 // multPackedMatMatCCReuse -- MatrixUtils.cpp:1276-1305 (relinearised and rescaled)
 CtxtTensor multPackedMatMatCCReuse(Env &e, const Ciphertext &pre, const CtxtTensor &tb) {
     const i64 width = tb.getBlockWidth();
     Ciphertext b = tb.get(), acc;
-    const int count = pre.getBatch() / tb.get().getBatch();
+    const int count = copies_per_member(pre, tb, tb.getHeight() / 2);
     if (e.mode >= kDirect) {
         const Hoisted h = e.ev.decompose(tb.get());
         const i64 group = loop_group(tb.get());
@@ -612,7 +620,7 @@ CtxtTensor multMatMatPreRev(Env &e, const CtxtTensor &b, int target_level) {
 CtxtTensor multMatMatCCReUse(Env &e, const Ciphertext &pre, const CtxtTensor &tb) {
     const i64 width = tb.getBlockWidth();
     Ciphertext b = tb.get(), acc;
-    const int count = pre.getBatch() / tb.get().getBatch();
+    const int count = copies_per_member(pre, tb, tb.getHeight());
     if (e.mode >= kDirect) {
         const Hoisted h = e.ev.decompose(tb.get());
         const i64 group = loop_group(tb.get());

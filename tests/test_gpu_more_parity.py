@@ -270,3 +270,57 @@ def test_tile_batched_accumulate_many_terms_with_44_bit_primes(pkg):
             q = int(g.primes[l])
             want = np.array([(copies * (q - 1) * (int(a) + int(b))) % q for a, b in zip(w[0][l], w[1][l])], dtype=np.uint64)
             assert np.array_equal(got[0, 0, l], want) and np.array_equal(got[0, 1, l], want), f"tile {t} limb {l}"
+
+
+def _reuse(H, packed):
+    """(copies of the left operand, right operand made ready, product) of the two reuse families, at target level 2"""
+    if packed:
+        return lambda a: H.packed_matmul_pre_rot(H.packed_matmul_pre(a, 2), 2), lambda b: H.packed_matmul_pre_rev(b, 2), H.packed_matmul_cc_reuse
+    return lambda a: H.matmul_pre(a, 2), lambda b: H.matmul_pre_rev(b, 2), H.matmul_cc_reuse
+
+
+def _operands(pkg, g, H, packed, count, base):
+    d = cases.tile_dim(g)
+    rng = np.random.default_rng(base)
+    out = []
+    for k in range(count):
+        t = H.encrypt2(rng.uniform(-1, 1, (d, d)), rng.uniform(-1, 1, (d, d)), nonce=base + k)
+        if packed:
+            (H.complex_packing_row_inplace if base % 2 else H.complex_packing_inplace)(t)
+        out.append(t)
+    return out, lambda ts: pkg.CtxtTensor(g.batch_concat([t.ct for t in ts]), *ts[0].shape)
+
+
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("schedule", [0, 1, 2])
+def test_reused_copies_of_a_batch_equal_single_calls(pkg, gpu_small, schedule, packed):
+    """Three left operands copied together meet three right operands: member by member the products of single calls.  Copies that are
+    not the full set of every right operand are refused."""
+    g = gpu_small
+    H = pkg.open_hemmer(g)
+    H.set_schedule(schedule)
+    pre, rev, product = _reuse(H, packed)
+    left, join = _operands(pkg, g, H, packed, 3, 500)
+    right, _ = _operands(pkg, g, H, packed, 3, 601)
+    copies, tb = pre(join(left)), rev(join(right))
+    got = g.ct_export(product(copies, tb).ct)
+    single = [pre(a) for a in left]
+    for k in range(3):
+        want = g.ct_export(product(single[k], rev(right[k])).ct)
+        _same(got[k:k + 1], want, f"member {k}")
+    for lone, many in ((single[0], rev(join(right[:2]))), (single[0], tb), (copies, rev(join(right[:2])))):
+        with pytest.raises(pkg.HBError):
+            product(lone, many)
+
+
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("schedule", [0, 1])
+def test_reused_copies_refuse_more_right_operands_than_copies(pkg, gpu_small, schedule, packed):
+    g = gpu_small
+    H = pkg.open_hemmer(g)
+    H.set_schedule(schedule)
+    _, rev, product = _reuse(H, packed)
+    right, join = _operands(pkg, g, H, packed, 3, 701)
+    tb = rev(join(right))
+    with pytest.raises(pkg.HBError):
+        product(g.batch_slice(tb.ct, 0, 2), tb)
