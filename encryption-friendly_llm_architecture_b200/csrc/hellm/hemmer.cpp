@@ -175,18 +175,23 @@ static Ciphertext row_sums(HEMMer &h, Ciphertext x, const std::vector<int> &dir,
     for (i64 rot = 1; rot < out_end; rot <<= 1) x = ev.add(x, ev.leftRotateGroups(x, steps(-rot)));
     return x;
 }
+// (the operands are replaced at the end: an error on the way leaves them as they are)
 static void row_sums_pair(HEMMer &h, CtxtTensor &a, CtxtTensor &b, i64 in_end, i64 out_end) {
     const Evaluator &ev = h.eval();
+    auto whole = [&](const CtxtTensor &t) { return ev.view(t.get(), 0, t.get().getBatch()); };
+    Ciphertext sa, sb;
     if (a.getLevel() != b.getLevel() || a.get().getBatch() != b.get().getBatch()) {
-        a.get() = row_sums(h, std::move(a.get()), {1}, in_end, out_end);
-        b.get() = row_sums(h, std::move(b.get()), {-1}, in_end, out_end);
-        return;
+        sa = row_sums(h, whole(a), {1}, in_end, out_end);
+        sb = row_sums(h, whole(b), {-1}, in_end, out_end);
+    } else {
+        std::vector<Ciphertext> two;
+        two.push_back(whole(a)); two.push_back(whole(b));
+        const Ciphertext x = row_sums(h, ev.concat(two), {1, -1}, in_end, out_end);
+        sa = ev.copyGroup(x, 0, 2);
+        sb = ev.copyGroup(x, 1, 2);
     }
-    std::vector<Ciphertext> two;
-    two.push_back(std::move(a.get())); two.push_back(std::move(b.get()));
-    const Ciphertext x = row_sums(h, ev.concat(two), {1, -1}, in_end, out_end);
-    a.get() = ev.copyGroup(x, 0, 2);
-    b.get() = ev.copyGroup(x, 1, 2);
+    a.get() = std::move(sa);
+    b.get() = std::move(sb);
 }
 // HEMMer::oneMatRotSumInplace -- HEMMer.cpp:882-919 with ModelArgs::HEAD_DIM equal to the tile side
 void HEMMer::oneMatRotSumInplace(CtxtTensor &a, CtxtTensor &b) { row_sums_pair(*this, a, b, tile_ / 2, tile_); }

@@ -91,13 +91,22 @@ def test_files_round_trip(pkg, gpu_mid, tmp_path):
         g.ct_load(tmp_path / "missing.bin")
 
 
+def _compiled(name, tmp_path):
+    exe = tmp_path / name
+    subprocess.check_call(["g++", "-O1", "-std=c++17", os.path.join(ROOT, "tests", "integration", name + ".cpp"), "-I", os.path.join(ROOT, "include"),
+                           "-I", os.path.join(PKG_DIR, "csrc", "hellm"), "-L", PKG_DIR, "-lhellm_b200", "-lhemmer_b200", f"-Wl,-rpath,{PKG_DIR}", "-o", str(exe)])
+    return exe
+
+
+def test_operands_of_the_row_sums_survive_an_error(tmp_path):
+    r = subprocess.run([str(_compiled("operands_after_error", tmp_path))], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 def test_cpp_class_from_a_separately_compiled_program(pkg, tmp_path):
     """tests/integration/hemmer_snippet.cpp (the example of INTEGRATION.md) built with g++ against the two shared
     libraries, run, and compared with the same calls through ctypes: equal residues, correct products."""
-    exe, out = tmp_path / "snippet", tmp_path / "snippet.bin"
-    cmd = ["g++", "-O1", "-std=c++17", os.path.join(ROOT, "tests", "integration", "hemmer_snippet.cpp"), "-I", os.path.join(ROOT, "include"),
-           "-I", os.path.join(PKG_DIR, "csrc", "hellm"), "-L", PKG_DIR, "-lhellm_b200", "-lhemmer_b200", f"-Wl,-rpath,{PKG_DIR}", "-o", str(exe)]
-    subprocess.check_call(cmd)
+    exe, out = _compiled("hemmer_snippet", tmp_path), tmp_path / "snippet.bin"
     r = subprocess.run([str(exe), str(out)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     raw = out.read_bytes()
