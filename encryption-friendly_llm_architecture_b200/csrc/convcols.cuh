@@ -411,15 +411,15 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
 // Single passes, for the fused sequences.  A grid of one or two CTAs per SM takes the kernels that may use 128 registers and
 // fetch the twiddles of the second round (which nobody shares) before anything else, under the tail of the predecessor.
 constexpr int kSmallGrid = 2 * 148;
-inline void launch_inv_rows16(cudaStream_t st, const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
-    launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_inv_rows<2> : ntt16v2_inv_rows<4>, dim3(16, count), 256, 0, src, LimbAddr16{src_outer}, dst, LimbAddr16{dst_outer}, map, pc, tb);
+inline cudaError_t launch_inv_rows16(cudaStream_t st, const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
+    return launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_inv_rows<2> : ntt16v2_inv_rows<4>, dim3(16, count), 256, 0, src, LimbAddr16{src_outer}, dst, LimbAddr16{dst_outer}, map, pc, tb);
 }
-inline void launch_fwd_rows16(cudaStream_t st, u64 *d, size_t outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
-    launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_fwd_rows<2> : ntt16v2_fwd_rows<4>, dim3(16, count), 256, 0, d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb);
+inline cudaError_t launch_fwd_rows16(cudaStream_t st, u64 *d, size_t outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
+    return launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_fwd_rows<2> : ntt16v2_fwd_rows<4>, dim3(16, count), 256, 0, d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb);
 }
 template <class ADD>
-inline void launch_fwd_rows_fin16(cudaStream_t st, const u64 *t, size_t t_outer, int n, int instances, const RowsFin &f, const InvScale &sc, const ADD &add, const PrimeConst *pc, const Ntt16Tables &tb) {
-    launch_pdl(st, 16 * n * instances <= kSmallGrid ? ntt16v2_fwd_rows_fin<2, ADD> : ntt16v2_fwd_rows_fin<4, ADD>, dim3(16, n, instances), 256, 0, t, t_outer, f, sc, add, pc, tb);
+inline cudaError_t launch_fwd_rows_fin16(cudaStream_t st, const u64 *t, size_t t_outer, int n, int instances, const RowsFin &f, const InvScale &sc, const ADD &add, const PrimeConst *pc, const Ntt16Tables &tb) {
+    return launch_pdl(st, 16 * n * instances <= kSmallGrid ? ntt16v2_fwd_rows_fin<2, ADD> : ntt16v2_fwd_rows_fin<4, ADD>, dim3(16, n, instances), 256, 0, t, t_outer, f, sc, add, pc, tb);
 }
 
 } // namespace hb

@@ -192,6 +192,11 @@ void ntt(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int count, 
     c->launches += (count == 0) ? 0 : (c->logn == 16 ? 2 : 1);
     CK(launch_ntt(c->st, src, so, dst, dof, count, m, c->pc, c->tb, c->logn, inv));
 }
+// a launch under programmatic dependence; a configuration that the device refuses ends the call here
+template <class K, class... A> void launch(hb_ctx *c, K *kernel, dim3 grid, dim3 block, size_t smem, A &&...args) {
+    c->launches++;
+    CK(launch_pdl(c->st, kernel, grid, block, smem, std::forward<A>(args)...));
+}
 // a constant v mod q in the form the 2^16 kernels multiply by: the value as a double and v / q, or the value and its Shoup companion
 void scale_words(u64 v, u64 q, u64 &w, u64 &comp) {
     if (q >> 44) { w = v; comp = hbhost::shoup(v, q); return; }
@@ -361,9 +366,8 @@ StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? 
 // `plans` conversions (the largest with max_ns sources) of `instances` polynomials in one launch
 void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int instances) {
     conv_opt_in(c);
-    LAUNCH(c);
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
-        launch_pdl(c->st, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
+        launch(c, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
     };
     switch (conv_shape(instances * count)) {
     case kStrip8x4: go(conv_cols<8, 4, 1>, 8, 4, strip_bytes<8>(max_ns + 4)); break;
@@ -374,9 +378,8 @@ void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, con
 // half-inverse limbs of prime `level` (one per instance) -> half-forward lifts to the limbs below
 void launch_lift(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int level, int instances) {
     conv_opt_in(c);
-    LAUNCH(c);
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
-        launch_pdl(c->st, kernel, dim3(256 / cols, instances), cols * 16 * groups, smem, src, so, dst, dof, level, c->pc, c->tb.t16);
+        launch(c, kernel, dim3(256 / cols, instances), cols * 16 * groups, smem, src, so, dst, dof, level, c->pc, c->tb.t16);
     };
     switch (lift_shape(instances)) {
     case kStrip4x8: go(lift_cols<4, 8, 1>, 4, 8, strip_bytes<4>(9)); break;
@@ -385,10 +388,10 @@ void launch_lift(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int
     }
 }
 void inv_rows(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int count, const LimbMap &m) {
-    LAUNCH(c), launch_inv_rows16(c->st, src, so, dst, dof, count, m, c->pc, c->tb.t16);
+    LAUNCH(c); CK(launch_inv_rows16(c->st, src, so, dst, dof, count, m, c->pc, c->tb.t16));
 }
 void fwd_rows(hb_ctx *c, u64 *d, size_t outer, int count, const LimbMap &m) {
-    LAUNCH(c), launch_fwd_rows16(c->st, d, outer, count, m, c->pc, c->tb.t16);
+    LAUNCH(c); CK(launch_fwd_rows16(c->st, d, outer, count, m, c->pc, c->tb.t16));
 }
 LimbMap one_limb(int prime) { LimbMap m{}; m.n = 1; m.prime[0] = (unsigned char)prime; return m; }
 
@@ -446,7 +449,7 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, siz
         inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, total * 2 * K, pm);
         launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, total * 2);
         const RowsFin f{acc, (size_t)ne * N, out, out_outer, 2, batch, add_outer};
-        LAUNCH(c), launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, total * 2, f, c->p_inv_scale, sl, c->pc, c->tb.t16);
+        LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, total * 2, f, c->p_inv_scale, sl, c->pc, c->tb.t16));
         CK(cudaGetLastError());
         return;
     }
@@ -476,7 +479,7 @@ void ks_apply(hb_ctx *c, const SwitchList &sl, size_t a_outer, int level, int ba
     const int el = batch >= 32 && d.nd <= 4 ? 1 : 2;
     const int per = members_per_cta(batch, N / (256 * el) * ne * sl.count), chunks = (batch + per - 1) / per;
     auto inner = [&](auto *kernel) {
-        LAUNCH(c), launch_pdl(c->st, kernel, dim3((unsigned)(N / (256 * el)), sl.count * chunks, ne), 256, 0, acc.p, sl, batch, per, a_outer, c->nprimes, pl, c->pc, c->logn, N);
+        launch(c, kernel, dim3((unsigned)(N / (256 * el)), sl.count * chunks, ne), 256, 0, acc.p, sl, batch, per, a_outer, c->nprimes, pl, c->pc, c->logn, N);
     };
     switch (d.nd) {
     case 1: inner(el == 1 ? k_ks_inner<1, 1> : k_ks_inner<1, 2>); break;
@@ -612,7 +615,7 @@ hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch) {
             inv_rows(c, src, (size_t)ne * N, src, (size_t)ne * N, batch * 2 * ns, sm);
             launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, batch * 2);
             const RowsFin f{E, (size_t)ne * N, r->d, (size_t)2 * level * N, 2, 1, 0};
-            LAUNCH(c), launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], NoAddends{}, c->pc, c->tb.t16);
+            LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], NoAddends{}, c->pc, c->tb.t16));
             CK(cudaGetLastError());
             return r;
         }
@@ -678,10 +681,10 @@ hb_ct *do_assemble_mk(hb_ctx *c, const hb_ct *a, const u64 *dt, const hb_mkey *c
     ALG(c, (size_t)batch * (2 * n + d.dt_count));
     if (d.nd <= 2) {
         const int per = members_per_cta(batch, N / (256 * 1) * ne * groups), chunks = (batch + per - 1) / per;
-        LAUNCH(c), launch_pdl(c->st, d.nd == 1 ? k_ks_inner_mkr<1> : k_ks_inner_mkr<2>, dim3((unsigned)(N / (256 * 1)), (unsigned)(groups * chunks), (unsigned)ne), 256, 0, E.p, (const u64 *)a->d,
+        launch(c, d.nd == 1 ? k_ks_inner_mkr<1> : k_ks_inner_mkr<2>, dim3((unsigned)(N / (256 * 1)), (unsigned)(groups * chunks), (unsigned)ne), 256, 0, E.p, (const u64 *)a->d,
                               (const u64 *)a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch, per, pl, c->pc, c->logn, N);
     } else {
-        LAUNCH(c), launch_pdl(c->st, k_ks_inner_mk, dim3((unsigned)((N + 1023) / 1024), groups * batch, ne), 256, 0, E.p, (const u64 *)a->d, (const u64 *)a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch, pl,
+        launch(c, k_ks_inner_mk, dim3((unsigned)((N + 1023) / 1024), groups * batch, ne), 256, 0, E.p, (const u64 *)a->d, (const u64 *)a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch, pl,
                               c->pc, c->logn, N);
     }
     CK(cudaGetLastError());
@@ -703,7 +706,7 @@ void rescale_core(hb_ctx *c, const u64 *x, u64 *out, int l, int np, int nbp, u64
         inv_rows(c, x + (size_t)l * N, (size_t)(l + 1) * N, last, (size_t)N, nbp, lm);
         launch_lift(c, last, (size_t)N, t, (size_t)l * N, l, nbp);
         const RowsFin f{x, (size_t)(l + 1) * N, out, (size_t)np * l * N, np, 1, 0};
-        LAUNCH(c), launch_fwd_rows_fin16(c->st, t, (size_t)l * N, l, nbp, f, sc, NoAddends{}, c->pc, c->tb.t16);
+        LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, t, (size_t)l * N, l, nbp, f, sc, NoAddends{}, c->pc, c->tb.t16));
     } else {
         ntt(c, x + (size_t)l * N, (size_t)(l + 1) * N, last, (size_t)N, nbp, lm, true);
         LAUNCH(c), k_rescale_prep<<<c->egrid(nbp * l), 256, 0, c->st>>>(t, last, l, c->pc, N);
@@ -762,11 +765,11 @@ hb_ct *do_prod_rescale(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, 
     ALG(c, (size_t)count * sums * ((size_t)nbp * (l + 1) + (l + 1)) + (size_t)total * l);
     try {
         Tmp last(c, (size_t)groups * total), t(c, (size_t)total * l);
-        LAUNCH(c), launch_pdl(c->st, k_last_prod, dim3(gx, total, groups), 256, 0, last.p, tl, separate ? 1 : 0, l, nbp, c->pc, N);
+        launch(c, k_last_prod, dim3(gx, total, groups), 256, 0, last.p, tl, separate ? 1 : 0, l, nbp, c->pc, N);
         lift_last(c, last.p, 1, groups, total, l, t.p);
         Scalars qi{};
         for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
-        LAUNCH(c), launch_pdl(c->st, k_prod_rescale_fin, c->egrid(total * l), 256, 0, r->d, tl, t.p, l, nbp, c->pc, N, qi);
+        launch(c, k_prod_rescale_fin, c->egrid(total * l), 256, 0, r->d, tl, t.p, l, nbp, c->pc, N, qi);
         CK(cudaGetLastError());
     } catch (...) { hb_ct_free(r); throw; }
     return r;
@@ -813,7 +816,7 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
         if (!c->smem_opt_in_parts) { CK(cudaFuncSetAttribute(k_prod_parts<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, G * kMaxPartTerms * 2048)); c->smem_opt_in_parts = true; }
         Scalars qi{};
         for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
-        if (separate) LAUNCH(c), launch_pdl(c->st, k_last_prod_parts, dim3(c->gx(), nbp, parts * count), 256, 0, last.p, pt, l, nbp, c->pc, N);
+        if (separate) launch(c, k_last_prod_parts, dim3(c->gx(), nbp, parts * count), 256, 0, last.p, pt, l, nbp, c->pc, N);
         else LAUNCH(c), k_prod_parts<G><<<dim3(gx1, 1, pg), 512, smem, c->st>>>(last.p, pt, nullptr, l, nbp, c->pc, N, qi, c->dev_err);
         lift_last(c, last.p, parts, separate ? count : 1, nbp, l, t.p);
         LAUNCH(c), k_prod_parts<G><<<dim3(gx1, (unsigned)l, pg), 512, smem, c->st>>>(r->d, pt, t.p, l, nbp, c->pc, N, qi, c->dev_err);
@@ -880,7 +883,9 @@ hb_ct *do_tensor(hb_ctx *c, const hb_ct *a, const hb_ct *b, hb_ct *acc, int grou
     else r = new_ct(c, a->level, 3, batch, 2);
     const int n = a->level + 1;
     ALG(c, 2 * a->limbs() + (size_t)(acc ? 2 : 1) * batch * 3 * n);
-    LAUNCH(c), launch_pdl(c->st, k_tensor, dim3((unsigned)(c->N / 512), (unsigned)(batch * n)), 256, 0, r->d, (const u64 *)a->d, (const u64 *)b->d, n, c->qmap(a->level), c->pc, c->N, acc ? 1 : 0, groups, batch);
+    try {
+        launch(c, k_tensor, dim3((unsigned)(c->N / 512), (unsigned)(batch * n)), 256, 0, r->d, (const u64 *)a->d, (const u64 *)b->d, n, c->qmap(a->level), c->pc, c->N, acc ? 1 : 0, groups, batch);
+    } catch (...) { if (!acc) hb_ct_free(r); throw; }
     return r;
 }
 hb_ct *do_relin(hb_ctx *c, const hb_ct *a) {
@@ -951,7 +956,7 @@ int host_workers(const hb_ctx *c, int tasks) {
 template <class F> int guard(hb_ctx *c, F &&f) {
     try { CK(cudaSetDevice(c->device)); f(); return HB_OK; }
     catch (const ArgFail &e) { c->err = e.msg; return e.code; }
-    catch (const CudaFail &e) { c->err = std::string(e.where) + ": " + cudaGetErrorString(e.e); return HB_E_CUDA; }
+    catch (const CudaFail &e) { cudaGetLastError(); c->err = std::string(e.where) + ": " + cudaGetErrorString(e.e); return HB_E_CUDA; }
     catch (const std::invalid_argument &e) { c->err = e.what(); return HB_E_ARG; }
     catch (const std::exception &e) { c->err = e.what(); return HB_E_CUDA; }
 }

@@ -521,14 +521,9 @@ inline cudaError_t launch_ntt16(cudaStream_t st, const u64 *src, size_t src_oute
     if (count == 0) return cudaSuccess;
     LimbAddr16 sa{src_outer}, da{dst_outer};
     dim3 grid(16, count);
-    if (!inverse) {
-        launch_pdl(st, ntt16v2_fwd_cols<MINB>, grid, 256, 0, src, sa, dst, da, map, pc, tb);
-        launch_pdl(st, ntt16v2_fwd_rows<MINB>, grid, 256, 0, dst, da, dst, da, map, pc, tb);
-    } else {
-        launch_pdl(st, ntt16v2_inv_rows<MINB>, grid, 256, 0, src, sa, dst, da, map, pc, tb);
-        launch_pdl(st, ntt16v2_inv_cols<MINB>, grid, 256, 0, dst, da, dst, da, map, pc, tb);
-    }
-    return cudaGetLastError();
+    const cudaError_t e = inverse ? launch_pdl(st, ntt16v2_inv_rows<MINB>, grid, 256, 0, src, sa, dst, da, map, pc, tb) : launch_pdl(st, ntt16v2_fwd_cols<MINB>, grid, 256, 0, src, sa, dst, da, map, pc, tb);
+    if (e != cudaSuccess) return e;
+    return inverse ? launch_pdl(st, ntt16v2_inv_cols<MINB>, grid, 256, 0, dst, da, dst, da, map, pc, tb) : launch_pdl(st, ntt16v2_fwd_rows<MINB>, grid, 256, 0, dst, da, dst, da, map, pc, tb);
 }
 
 } // namespace hb

@@ -18,15 +18,18 @@ __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// the error is returned and not left for the next cudaGetLastError, which would blame another call
 template <class... P, class... A>
-inline void launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
+inline cudaError_t launch_pdl(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cfg.attrs = at; cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 } // namespace hb

@@ -153,3 +153,16 @@ def test_release_cached_returns_idle_buffers(pkg):
     g.dll.hb_mem_info(g.ctx, C.byref(pool), C.byref(used))
     assert pool.value < before and pool.value >= used.value
     assert np.abs(g.decrypt(ct).real - z).max() < 2.0 ** -14
+
+
+def test_a_refused_launch_is_reported_by_its_own_call(pkg):
+    """713 ciphertexts with 92 lifted limbs each are more limb instances (65 596) than a grid has room for: hb_decompose says so
+    instead of handing out digits that were never finished, and the next call is not blamed for it."""
+    g = pkg.open_gpu(pkg.make_params(log_n=16, max_level=12, dnum=7, num_special=2, hamming_weight=64))
+    with pytest.raises(pkg.HBError):
+        g.decompose(g.ct_create(12, 2, 713))
+    x = g.ct_create(12, 2, 1)
+    g.ct_import(x, rand_ct_residues(g, 12, 2, 1, seed=3))
+    g.decompose(x)
+    assert g.dll.hb_sync(g.ctx) == 0
+    g.close()
