@@ -1436,13 +1436,13 @@ int hb_batch_concat(hb_ctx *c, const hb_ct *const *parts, int n, hb_ct **out) {
 int hb_batch_view(hb_ctx *c, const hb_ct *src, int start, int count, hb_ct **out) {
     return guard(c, [&] {
         own(c, src);
-        if (start < 0 || count < 1 || start + count > src->batch) fail(HB_E_ARG, "batch_view: bad range");
+        if (start < 0 || count < 1 || count > src->batch || start > src->batch - count) fail(HB_E_ARG, "batch_view: bad range");
         *out = new hb_ct{c, src->level, src->np, count, src->spow, src->d + (size_t)start * src->np * (src->level + 1) * c->N, true};
     });
 }
 int hb_batch_slice(hb_ctx *c, const hb_ct *src, int start, int count, hb_ct **out) {
     return guard(c, [&] {
-        if (start < 0 || count < 1 || start + count > src->batch) fail(HB_E_ARG, "batch_slice: bad range");
+        if (start < 0 || count < 1 || count > src->batch || start > src->batch - count) fail(HB_E_ARG, "batch_slice: bad range");
         hb_ct *r = new_ct(c, src->level, src->np, count, src->spow);
         const size_t per = (size_t)src->np * (src->level + 1) * c->N;
         CK(cudaMemcpyAsync(r->d, src->d + per * start, per * count * 8, cudaMemcpyDeviceToDevice, c->st));
@@ -1773,6 +1773,7 @@ static std::vector<hb_ct> group_views(hb_ctx *c, const hb_ct *x, int groups) {
 int hb_sum_mul_pt_rescale_grouped(hb_ctx *c, const hb_ct *x, const hb_pt *const *p, int count, int sums, hb_ct **out) {
     return guard(c, [&] {
         if (!x || !p || count < 1 || sums < 1) fail(HB_E_ARG, "product sums: bad arguments");
+        if (count > kMaxTerms || sums > kMaxTerms) fail(HB_E_LIMIT, "product sum: between 1 and " + std::to_string(kMaxTerms) + " terms");
         const std::vector<hb_ct> v = group_views(c, x, count * sums);
         std::vector<const hb_ct *> a;
         for (const hb_ct &y : v) a.push_back(&y);
@@ -1794,7 +1795,7 @@ int hb_mul2_add_rescale(hb_ctx *c, const hb_ct *a, const hb_pt *pa, const hb_ct 
 }
 int hb_matmul_acc_multi(hb_ctx *c, const hb_ct *pre, int btotal, int b0, const hb_pt *const *pts, int bcount, int64_t row_step, hb_ct **out) {
     return guard(c, [&] {
-        if (btotal < 1 || pre->batch % btotal || b0 < 0 || bcount < 1 || b0 + bcount > btotal || bcount > 16) fail(HB_E_SHAPE, "matmul_acc: group selection");
+        if (btotal < 1 || pre->batch % btotal || b0 < 0 || bcount < 1 || bcount > 16 || bcount > btotal || b0 > btotal - bcount) fail(HB_E_SHAPE, "matmul_acc: group selection");
         if (pre->np != 2 || pre->spow != 1) fail(HB_E_SHAPE, "matmul_acc: operands");
         own(c, pre);
         for (int b = 0; b < bcount; ++b) {
@@ -1814,7 +1815,7 @@ int hb_matmul_acc_multi(hb_ctx *c, const hb_ct *pre, int btotal, int b0, const h
 int hb_matmul_acc_tiles(hb_ctx *c, const hb_ct *pre, int btotal, int b0, const hb_pt *const *pts, int bcount, int tiles, int64_t row_step, hb_ct **out) {
     return guard(c, [&] {
         if (!pre || !pts || !out || tiles < 1) fail(HB_E_ARG, "matmul_acc: null argument");
-        if (btotal < 1 || pre->batch % btotal || b0 < 0 || bcount < 1 || b0 + bcount > btotal || bcount > 16) fail(HB_E_SHAPE, "matmul_acc: group selection");
+        if (btotal < 1 || pre->batch % btotal || b0 < 0 || bcount < 1 || bcount > 16 || bcount > btotal || b0 > btotal - bcount) fail(HB_E_SHAPE, "matmul_acc: group selection");
         if (pre->np != 2 || pre->spow != 1) fail(HB_E_SHAPE, "matmul_acc: operands");
         own(c, pre);
         for (int i = 0; i < tiles * bcount; ++i) {
