@@ -41,7 +41,7 @@ struct Pool {
         if (!v.empty()) { p = v.back(); v.pop_back(); }
         else {
             cudaError_t e = cudaMalloc(&p, bytes);
-            if (e != cudaSuccess) { release_cached(); e = cudaMalloc(&p, bytes); }
+            if (e != cudaSuccess) { cudaGetLastError(); release_cached(); e = cudaMalloc(&p, bytes); } // the first failure must not stay behind as the last error
             if (e != cudaSuccess) { cudaGetLastError(); fail(HB_E_OOM, "device allocation of " + std::to_string(bytes) + " bytes failed"); }
             total += bytes;
         }

@@ -166,3 +166,21 @@ def test_a_refused_launch_is_reported_by_its_own_call(pkg):
     g.decompose(x)
     assert g.dll.hb_sync(g.ctx) == 0
     g.close()
+
+
+def test_a_full_pool_makes_room_for_another_size(pkg):
+    """Idle buffers fill more than half of the device, then a larger one is asked for: the allocation that fails at first is tried again
+    without them, and the failure is not held against the next call."""
+    import torch
+    g = pkg.open_gpu(pkg.make_params(log_n=16, max_level=12, hamming_weight=64))
+    x = g.ct_create(1, 2, 1, 2)
+    g.ct_import(x, rand_ct_residues(g, 1, 2, 1, seed=6))
+    want = g.ct_export(g.rescale(x))
+    member = 2 * 13 * g.N * 8
+    free = torch.cuda.mem_get_info()[0]
+    g.ct_create(12, 2, int(0.55 * free / member))  # freed at once: stays in the pool
+    large = g.ct_create(12, 2, int(0.6 * free / member))
+    got = g.ct_export(g.rescale(x))
+    _same(got, want, "rescale after the pool made room")
+    del large
+    g.close()
