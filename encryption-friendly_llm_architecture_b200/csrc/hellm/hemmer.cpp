@@ -175,12 +175,15 @@ static Ciphertext row_sums(HEMMer &h, Ciphertext x, const std::vector<int> &dir,
     for (i64 rot = 1; rot < out_end; rot <<= 1) x = ev.add(x, ev.leftRotateGroups(x, steps(-rot)));
     return x;
 }
+// two ciphertexts go through one launch sequence while they are few: the sequence gains nothing once its members fill the GPU, and
+// twice the members are twice the scratch and half the batch that a grid has room for
+static bool rows_together(const Ciphertext &a, const Ciphertext &b) { return a.getLevel() == b.getLevel() && a.getBatch() == b.getBatch() && a.getBatch() <= 84; }
 // (the operands are replaced at the end: an error on the way leaves them as they are)
 static void row_sums_pair(HEMMer &h, CtxtTensor &a, CtxtTensor &b, i64 in_end, i64 out_end) {
     const Evaluator &ev = h.eval();
     auto whole = [&](const CtxtTensor &t) { return ev.view(t.get(), 0, t.get().getBatch()); };
     Ciphertext sa, sb;
-    if (a.getLevel() != b.getLevel() || a.get().getBatch() != b.get().getBatch()) {
+    if (!rows_together(a.get(), b.get())) {
         sa = row_sums(h, whole(a), {1}, in_end, out_end);
         sb = row_sums(h, whole(b), {-1}, in_end, out_end);
     } else {
@@ -232,33 +235,54 @@ void HEMMer::maskRightLeft(const CtxtTensor &t, CtxtTensor &left, CtxtTensor &ri
     right = CtxtTensor(t.getShape(), eval_.mult(t.get(), hemmer_mask(*this, kHeadRight, t.getLevel())));
 }
 // Gaussian-kernel score assembly -- TransformerBlock.cpp:2420-2482 (one query / key pair; the reference loops over three).  The two heads
-// go through the same operations, so they travel as the two member groups [left | right] of one ciphertext.
+// go through the same operations, so small batches of them travel as the two member groups [left | right] of one ciphertext.  The
+// giant steps of a transform hold up to 17 parts of every member at once and lift up to 96 limbs of each in one grid of at most
+// 65535, which forty members never exceed: beyond twenty pairs the heads go one after the other, so that stacking costs no batch its
+// place.  Nothing is lost there: together / one after the other 508 / 509 ms for 21 pairs and 688 / 670 ms for 28 (schedule 2).
+constexpr int kHeadsTogether = 20;
 std::vector<CtxtTensor> HEMMer::gaussianKernelScores(const CtxtTensor &query, const CtxtTensor &key, int target_level) {
-    auto heads = [&](const CtxtTensor &t) { // maskRightLeft
-        return CtxtTensor(t.getShape(), eval_.multSumParts({&t.get()}, {{&hemmer_mask(*this, kHeadLeft, t.getLevel())}, {&hemmer_mask(*this, kHeadRight, t.getLevel())}}, false));
+    struct Head { int mask, direction; };
+    auto scores = [&](const std::vector<Head> &heads) { // one member group per head
+        std::vector<int> dir;
+        for (const Head &h : heads) dir.push_back(h.direction);
+        auto masked = [&](const CtxtTensor &t) { // maskRightLeft
+            std::vector<std::vector<const Plaintext *>> rows;
+            for (const Head &h : heads) rows.push_back({&hemmer_mask(*this, h.mask, t.getLevel())});
+            return CtxtTensor(t.getShape(), eval_.multSumParts({&t.get()}, rows, false));
+        };
+        CtxtTensor mq = masked(query), mk = masked(key);
+        Ciphertext oq = eval_.square(mq.get()), ok = eval_.square(mk.get());
+        if (rows_together(oq, ok)) {
+            std::vector<Ciphertext> both;
+            both.push_back(std::move(oq)); both.push_back(std::move(ok));
+            std::vector<int> twice = dir;
+            twice.insert(twice.end(), dir.begin(), dir.end());
+            const Ciphertext x = row_sums(*this, eval_.concat(both), twice, tile_ / 2, tile_);
+            oq = eval_.copyGroup(x, 0, 2);
+            ok = eval_.copyGroup(x, 1, 2);
+        } else {
+            oq = row_sums(*this, std::move(oq), dir, tile_ / 2, tile_);
+            ok = row_sums(*this, std::move(ok), dir, tile_ / 2, tile_);
+        }
+        CtxtTensor okt(key.getShape(), std::move(ok));
+        transposeInplace(okt, target_level);
+        complexPackingInplace(mq);
+        transposeInplace(mk);
+        complexPackingRowInplace(mk);
+        CtxtTensor s = repackCC(packedMatMul(mq, mk, target_level));
+        s.get() = eval_.multInteger(s.get(), -2);
+        s.get() = eval_.add(s.get(), oq);
+        s.get() = eval_.add(s.get(), okt.get());
+        return s;
     };
-    CtxtTensor mq = heads(query), mk = heads(key);
-    Ciphertext oq = eval_.square(mq.get()), ok = eval_.square(mk.get());
-    if (oq.getLevel() == ok.getLevel() && oq.getBatch() == ok.getBatch()) {
-        std::vector<Ciphertext> both;
-        both.push_back(std::move(oq)); both.push_back(std::move(ok));
-        const Ciphertext x = row_sums(*this, eval_.concat(both), {1, -1, 1, -1}, tile_ / 2, tile_);
-        oq = eval_.copyGroup(x, 0, 2);
-        ok = eval_.copyGroup(x, 1, 2);
-    } else {
-        oq = row_sums(*this, std::move(oq), {1, -1}, tile_ / 2, tile_);
-        ok = row_sums(*this, std::move(ok), {1, -1}, tile_ / 2, tile_);
-    }
-    CtxtTensor okt(key.getShape(), std::move(ok));
-    transposeInplace(okt, target_level);
-    complexPackingInplace(mq);
-    transposeInplace(mk);
-    complexPackingRowInplace(mk);
-    CtxtTensor s = repackCC(packedMatMul(mq, mk, target_level));
-    s.get() = eval_.multInteger(s.get(), -2);
-    s.get() = eval_.add(s.get(), oq);
-    s.get() = eval_.add(s.get(), okt.get());
+    const Head left{kHeadLeft, 1}, right{kHeadRight, -1};
     std::vector<CtxtTensor> out;
+    if (std::max(query.get().getBatch(), key.get().getBatch()) > kHeadsTogether) {
+        out.push_back(scores({left}));
+        out.push_back(scores({right}));
+        return out;
+    }
+    const CtxtTensor s = scores({left, right});
     for (int j = 0; j < 2; ++j) out.emplace_back(s.getShape(), eval_.copyGroup(s.get(), j, 2));
     return out;
 }

@@ -324,3 +324,37 @@ def test_reused_copies_refuse_more_right_operands_than_copies(pkg, gpu_small, sc
     tb = rev(join(right))
     with pytest.raises(pkg.HBError):
         product(g.batch_slice(tb.ct, 0, 2), tb)
+
+
+@pytest.mark.parametrize("schedule", [0, 1, 2])
+def test_gaussian_scores_of_a_batch_equal_single_calls(pkg, gpu_small, schedule):
+    """Both heads as one ciphertext up to twenty members, one after the other beyond."""
+    g = gpu_small
+    H = pkg.open_hemmer(g)
+    H.set_schedule(schedule)
+    query, join = _operands(pkg, g, H, False, 21, 800)
+    key, _ = _operands(pkg, g, H, False, 21, 900)
+    singles = {k: [g.ct_export(t.ct) for t in H.gaussian_kernel_scores(query[k], key[k], 2)] for k in (0, 1, 19, 20)}
+    for batch in (2, 20, 21):
+        got = [g.ct_export(t.ct) for t in H.gaussian_kernel_scores(join(query[:batch]), join(key[:batch]), 2)]
+        for k in {0, 1, batch - 1}:
+            for head in range(2):
+                _same(got[head][k:k + 1], singles[k][head], f"head {head} of member {k} of {batch}")
+
+
+def test_gaussian_scores_of_a_large_batch(pkg, gpu_full):
+    """72 query / key pairs at full size: sixteen giant-step parts of every member of one head are 35 712 lifted limbs at the level of
+    the transpose; of both heads they would be more than a grid has room for."""
+    g = gpu_full
+    H = pkg.open_hemmer(g)
+    H.set_schedule(2)
+    rng = np.random.default_rng(72)
+    query, key = (H.encrypt2(rng.uniform(-1, 1, (128, 128)), rng.uniform(-1, 1, (128, 128)), nonce=n) for n in (1000, 1001))
+    many = lambda t: pkg.CtxtTensor(g.batch_concat([t.ct] * 72), *t.shape)
+    want = [g.ct_export(t.ct) for t in H.gaussian_kernel_scores(query, key, 4)]
+    got = H.gaussian_kernel_scores(many(query), many(key), 4)
+    for head in range(2):
+        for k in (0, 71):
+            _same(g.ct_export(g.batch_slice(got[head].ct, k, 1)), want[head], f"head {head} of member {k}")
+    del got
+    g._chk(g.dll.hb_release_cached(g.ctx))
