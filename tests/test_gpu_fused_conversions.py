@@ -1,6 +1,6 @@
 """The kernels that join base conversions to the transforms of 2^16 points, and the inner products that walk over batch members,
 at the edges of their launch rules: every strip shape, partly filled member chunks, one and two rotations, one to seven conversion
-sources, and primes of every class (doubles, 45 to 59 bits, 60 bits).  Residues are whole numbers, so every comparison is exact."""
+sources, and primes of every class (below 2^34, below 2^44, 45 to 59 bits, 60 bits).  Residues are whole numbers, so every comparison is exact."""
 import ctypes as C
 
 import numpy as np
@@ -17,12 +17,18 @@ def _ct(lib, data):
     return ct
 
 
-@pytest.mark.parametrize("level", [7, 3])  # two digits and one
-@pytest.mark.parametrize("batch", [1, 2, 3, 5, 17, 33, 47])
-def test_members_of_a_batch_equal_single_calls(gpu_full, level, batch):
-    """Strip shapes change at 2, 4 and 32 polynomials, the inner products split 47 members into uneven chunks; a batch of one takes
-    the narrow shapes, whose residues the full-size oracle tests pin."""
-    g = gpu_full
+SIZES = [("full", 12, (5, 33)), ("full", 7, (1, 2, 3, 5, 17, 33, 47)), ("full", 3, (1, 2, 3, 5, 17, 33, 47)), ("full", 2, (2, 5, 33)),
+         ("mid", 7, (17, 33, 47)), ("mid", 3, (17, 33, 47)), ("mid", 2, (17, 33, 47))]
+
+
+@pytest.mark.parametrize("size,level,batch", [(s, l, b) for s, l, batches in SIZES for b in batches])
+def test_members_of_a_batch_equal_single_calls(request, size, level, batch):
+    """Four, three, two and one digits (levels 12, 7, 3, 2), on either side of the 32 members from which the inner products hold one
+    coefficient per thread.  At 2^16 points the strip shapes change at 2, 4 and 32 polynomials, and one chunk holds all members
+    except at two and one digits with few of them (two chunks).  At 2^12 points a chunk holds two to seven members and the last
+    one fewer, in the masked sums of one and two digits as well.  A batch of one takes the narrow shapes, whose residues the oracle
+    tests pin."""
+    g = request.getfixturevalue(f"gpu_{size}")
     g.gen_rot_keys([1, 128, -3])
     data = rand_ct_residues(g, level, 2, batch, seed=900 + batch)
     data[-1, :, 0] = np.uint64(int(g.primes[0]) - 1)
