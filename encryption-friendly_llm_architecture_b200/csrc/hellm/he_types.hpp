@@ -151,12 +151,8 @@ class Evaluator {
         hb_ct *o = nullptr; check(c_, hb_rotate(c_, a.raw(), steps, &o)); return Ciphertext(c_, o);
     }
     Ciphertext rightRotate(const Ciphertext &a, i64 steps) const { return leftRotate(a, -steps); }
-    // many rotations of one ciphertext: decompose once, then one cheap call per step (same bits as leftRotate)
+    // many rotations of one ciphertext: decompose once, then leftRotateMulti (same bits as leftRotate)
     Hoisted decompose(const Ciphertext &a) const { hb_digits *d = nullptr; check(c_, hb_decompose(c_, a.raw(), &d)); return Hoisted(d); }
-    Ciphertext leftRotate(const Ciphertext &a, const Hoisted &h, i64 steps) const {
-        check(c_, hb_gen_rot_keys(c_, &steps, 1));
-        hb_ct *o = nullptr; check(c_, hb_rotate_hoisted(c_, a.raw(), h.raw(), steps, &o)); return Ciphertext(c_, o);
-    }
     // all rotations of one ciphertext by `steps` in one launch sequence: member k * batch + b = rotation k of member b
     Ciphertext leftRotateMulti(const Ciphertext &a, const Hoisted &h, const std::vector<i64> &steps) const {
         check(c_, hb_gen_rot_keys(c_, steps.data(), (int)steps.size()));
@@ -210,26 +206,13 @@ class Evaluator {
     Plaintext mult(const Plaintext &a, const Plaintext &b) const { hb_pt *o = nullptr; check(c_, hb_pt_mul(c_, a.raw(), b.raw(), &o)); return Plaintext(o); }
     Plaintext add(const Plaintext &a, const Plaintext &b) const { hb_pt *o = nullptr; check(c_, hb_pt_add(c_, a.raw(), b.raw(), &o)); return Plaintext(o); }
     Plaintext leftRotate(const Plaintext &p, i64 steps) const { hb_pt *o = nullptr; check(c_, hb_pt_rotate(c_, p.raw(), steps, &o)); return Plaintext(o); }
-    // rescale(a (.) pa + b (.) pb): the "assemble" step of the matmul loops in one pass
-    Ciphertext assemble(const Ciphertext &a, const Plaintext &pa, const Ciphertext &b, const Plaintext &pb) const {
-        hb_ct *o = nullptr; check(c_, hb_mul2_add_rescale(c_, a.raw(), pa.raw(), b.raw(), pb.raw(), &o)); return Ciphertext(c_, o);
-    }
-    // pa (.) rot(a, sa) + pb (.) rot(a, sb), one level down: both key switches stay in the extended basis and share
-    // one division by P * q_level (pa, pb from encodeExtended)
-    Ciphertext assembleRotations(const Ciphertext &a, const Hoisted &h, i64 sa, const Plaintext &pa, i64 sb, const Plaintext &pb) const {
-        const i64 steps[2] = {sa, sb};
-        check(c_, hb_gen_rot_keys(c_, steps, 2));
-        hb_ct *o = nullptr; check(c_, hb_assemble_hoisted(c_, a.raw(), h.raw(), sa, pa.raw(), sb, pb.raw(), &o)); return Ciphertext(c_, o);
-    }
-    // the same from rotation keys that already carry the masks; kb may be empty (one masked rotation)
+    // the rotation key of `steps` with a mask (or the sum of two) multiplied into it
     MaskedKey maskedKey(i64 steps, const Plaintext &m1, const Plaintext *m2 = nullptr) const {
         check(c_, hb_gen_rot_keys(c_, &steps, 1));
         hb_mkey *k = nullptr; check(c_, hb_masked_key_create(c_, steps, m1.raw(), m2 ? m2->raw() : nullptr, &k)); return MaskedKey(k);
     }
-    Ciphertext assembleRotations(const Ciphertext &a, const Hoisted &h, const MaskedKey &ka, const MaskedKey &kb) const {
-        hb_ct *o = nullptr; check(c_, hb_assemble_masked(c_, a.raw(), h.raw(), ka.raw(), kb.raw(), &o)); return Ciphertext(c_, o);
-    }
-    // several wrapped copies of the same input in one launch sequence; member g * batch + b of the result is copy g of input b
+    // wrapped copies of the same input, pa (.) rot(a, sa) + pb (.) rot(a, sb) one level down: the key switches stay in the extended basis and share one
+    // division by P * q_level.  One launch sequence for all copies; member g * batch + b of the result is copy g of input b; kb[g] may be null (one rotation)
     Ciphertext assembleRotationsMulti(const Ciphertext &a, const Hoisted &h, const std::vector<const MaskedKey *> &ka, const std::vector<const MaskedKey *> &kb) const {
         std::vector<const hb_mkey *> k1, k2;
         for (size_t g = 0; g < ka.size(); ++g) { k1.push_back(ka[g]->raw()); k2.push_back(kb[g] ? kb[g]->raw() : nullptr); }
@@ -299,7 +282,6 @@ class Evaluator {
         for (size_t k = 0; k < v.size(); ++k) check(c_, hb_batch_set(c_, o, (int)k, v[k].raw()));
         return out;
     }
-    Ciphertext slice(const Ciphertext &b, int k) const { hb_ct *o = nullptr; check(c_, hb_batch_get(c_, b.raw(), k, &o)); return Ciphertext(c_, o); }
   private:
     hb_ctx *c_;
 };

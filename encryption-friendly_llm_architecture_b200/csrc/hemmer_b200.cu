@@ -1002,10 +1002,10 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             p.q_inv_f = 1.0 / (double)q;
             p.n_inv_f = (double)p.n_inv / (double)q;
             p.fp = q < ((u64)1 << 44) ? 1 : 0;
-            // lazy FP64-assisted products are below 1.6 q; reduce_fp takes sums below 2^52.  Every fixed-length lazy sum in
-            // the kernels has at most 128 terms (16 rotated terms x 8 digits), which any prime below 2^44 allows (>= 160).
+            // lazy FP64-assisted products are below 1.6 q; reduce_fp takes sums below 2^52.  The lazy sums that are left have at most
+            // kMaxTerms terms (k_last_prod, k_prod_rescale_fin; eight digits in k_ks_inner_pair); any prime below 2^44 allows 160.
             const u64 lazy_terms = (u64)((((unsigned __int128)1 << 52) * 5) / ((unsigned __int128)q * 8)); // how many may be summed
-            if (p.fp && lazy_terms < 160) throw std::invalid_argument("prime too large for the lazy FP64-assisted sums");
+            if (p.fp && lazy_terms < (u64)kMaxTerms) throw std::invalid_argument("prime too large for the lazy FP64-assisted sums");
             // primes of 45 bits and more: values are folded with shifts by the bit length b, which needs q close below 2^b; the
             // primes of a context are the first ones below a power of two, at most a few hundred 2N-steps away from it
             int bits = 0;
@@ -1823,13 +1823,6 @@ int hb_matmul_acc_tiles(hb_ctx *c, const hb_ct *pre, int btotal, int b0, const h
             own(c, pts[i]);
             if (pre->level != pts[i]->level) fail(HB_E_LEVEL, "matmul_acc: plaintext level differs from the ciphertexts'");
             if (pts[i]->spow != 1) fail(HB_E_SHAPE, "matmul_acc: operands");
-        }
-        if (c->N % 512) { // small rings: tile by tile
-            for (int t = 0; t < tiles; ++t) {
-                int rc = hb_matmul_acc_multi(c, pre, btotal, b0, pts + (size_t)t * bcount, bcount, row_step, &out[t]);
-                if (rc != HB_OK) { for (int u = 0; u < t; ++u) { hb_ct_free(out[u]); out[u] = nullptr; } throw ArgFail{rc, c->err}; }
-            }
-            return;
         }
         const int n = pre->level + 1, kc = pre->batch / btotal;
         const u32 *dg = galois_table(c, kc, row_step);
