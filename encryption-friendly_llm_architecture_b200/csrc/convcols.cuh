@@ -8,8 +8,11 @@
 //     inverse row pass (ntt16v2_inv_rows)  ->  conv_cols / lift_cols  ->  forward row pass (ntt16v2_fwd_rows*)
 //
 // replaces inverse columns, conversion and forward columns as three kernels: for a conversion of S limbs to T, S reads + T
-// writes instead of 3 S + S + 3 T limb transfers, and one launch instead of three.  Measured at S = 4, T = 6 (the division by
-// P * q_l at level 6) and 336 polynomials: see the launcher.
+// writes instead of 3 S + S + 3 T limb transfers, and one launch instead of three.  At S = 4, T = 6 (the division by P * q_l at
+// level 6) conv_cols<8, 4, 1> takes 585 us for 128 polynomials and 1225 us for 336.  Nothing in it is near its limit: 48 % of the
+// issue slots, FP64 pipe 29 %, multiply-add pipe 36 %, DRAM 13 %.  Sixteen warps per SM (128 registers; 64 make the radix-16 rounds
+// spill) do not cover their own latencies: dependent instructions, loads, and the barrier between sources and targets, which all
+// groups of the only CTA on the SM reach together.
 //
 // A CTA is G groups of COLS * 16 threads.  Sources are dealt to the groups, then (one CTA barrier later) targets; inside a
 // group a radix-16 round exchanges through shared memory behind a named barrier of that group only, so one group's loads,
@@ -82,7 +85,7 @@ __device__ __forceinline__ void strip_inverse(u64 (&v)[16], const u64 *p /* limb
         for (int e = 0; e < 16; ++e) v[e] = canon_q(mul_shoup4(v[e], sw, sc, c.nq), c.q, c.f);
     }
 }
-// Forward column pass of one limb strip that lies in sm (words of this thread at I::a; double bits below 2^44, |v| < 2q; otherwise below 4q).
+// Forward column pass of one limb strip that lies in sm (words of this thread at I::a; double bits below 2^44, |v| < 2q; otherwise below 3q).
 template <int COLS>
 __device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, int g, int sub, int lane) {
     using I = StripIndex<COLS>;
@@ -314,7 +317,9 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) lift_cols(const u64 *src,
 // ---- forward row pass with the last step of a division ----
 //   out[b][p][l] = (x[b][p][l] - t[b][p][l]) * inv_l  (+ add_p[b][l] o perm_g, ADD: addends and g of the member's group)
 // t arrives half-forward (conv_cols / lift_cols).  grid = (16, n, instances), instance bp = b * np + p.  The operands of the last
-// step are read after the barrier of the final exchange, when the registers of the transform are free.
+// step are read after the barrier of the final exchange, when the registers of the transform are free.  Without addends bound by DRAM
+// and the FP64 pipe together: 128 polynomials of six limbs 226 us, 5.4 TB/s of DRAM traffic (0.83 of a copy), FP64 pipe 50 % busy; with
+// addends 424 us for 96 of nine limbs, 4.5 TB/s.  64 registers for four CTAs per SM spill 8 to 16 bytes a thread.
 struct RowsFin {
     const u64 *x; size_t x_outer;            // instance stride of x; limb l at l * N
     u64 *out; size_t out_outer;              // ciphertext stride; polynomial p at p * n * N

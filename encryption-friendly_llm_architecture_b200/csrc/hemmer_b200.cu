@@ -475,7 +475,9 @@ void ks_apply(hb_ctx *c, const SwitchList &sl, size_t a_outer, int level, int ba
     Tmp acc(c, (size_t)total * 2 * ne), t(c, (size_t)total * 2 * n);
     // Many members and up to four digits: one coefficient per thread, four CTAs per SM (256 members at level 8 1620 -> 1471 us, 42
     // members 513 -> 492).  Few members: two coefficients, whose loads cover the latency of a short walk (two digits of two
-    // members 40 us, with one coefficient 51).
+    // members 40 us, with one coefficient 51).  The line between them matters little: hoisted rotations (this kernel and ModDown), one /
+    // two coefficients, us: three digits (level 8) 2 members 84.9 / 84.7, 8 242 / 245, 24 653 / 665, 48 1241 / 1266; two digits
+    // (level 5) 2 70.7 / 70.7, 8 184 / 181, 24 488 / 484, 48 916 / 909.
     const int el = batch >= 32 && d.nd <= 4 ? 1 : 2;
     const int per = members_per_cta(batch, N / (256 * el) * ne * sl.count), chunks = (batch + per - 1) / per;
     auto inner = [&](auto *kernel) {

@@ -77,7 +77,8 @@ __global__ void k_mul_pt(u64 *__restrict__ out, const u64 *__restrict__ a, const
 //   d[b] (+)= sum over the groups g of tensor(x[g][b], y[g][b])
 // (groups = 1 is the plain tensor product; several groups are several iterations of a product loop in one launch).
 // Two coefficients per thread, so that eight loads of a group are in flight, and one reduction per sum: 256 ciphertexts at level 8
-// 1634 -> 1498 us (5.6 TB/s), a launch of the layer's product loop 620 -> 517 us.  grid.x = N/512
+// 1634 -> 1498 us (5.6 TB/s), a launch of the layer's product loop 620 -> 517 us.  48 ciphertexts at level 8: 253 us, DRAM 4.3 TB/s,
+// 54 % of the issue slots.  grid.x = N/512
 __global__ void __launch_bounds__(256) k_tensor(u64 *d, const u64 *x, const u64 *y, int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N,
                                                 int accumulate, int groups, int batch) {
     constexpr int EL = 2;
@@ -368,7 +369,8 @@ __global__ void k_last_prod_parts(u64 *last, const __grid_constant__ PartTerms p
 // two members, the a_j of a member are read by the ceil(parts / G) CTAs of the chunk (from L2 after the first), and every
 // thread has the next two a_j of both members in flight while it works on the current ones.  1024 threads with one member each and
 // 128-bit sums on the 60-bit limbs: 639 us a launch for one two-tile product, 2876 us in the layer pass; now 607 and 2859 us.
-// Bound by the FP64 pipe: four instructions for each of the count x parts products of a coefficient.
+// Bound by the latency of the a_j loads: sixteen warps per SM (128 registers, 16 bytes a thread spilled) with two loads ahead leave 60 % of
+// the issue slots empty, FP64 pipe 18 %, wide multiply-adds 38 %, DRAM 1.9 TB/s (sixteen terms, twelve parts, 48 polynomials, level 7).
 // t == nullptr: raw sums of limb `level`, out[(g * nbp + bp) * N + x]                       grid = (N/256, 1, ceil(parts/G))
 // else: out[((g * nbp + bp) * level + l) * N + x] = (sum - t[same]) * q_level^-1 mod q_l      grid = (N/256, level, ceil(parts/G))
 template <int G>
@@ -565,7 +567,8 @@ struct SwitchList { SwitchGroup s[kMaxSwitchGroups]; int count; };
 // digit_dg[j] is a_ntt[j] for own limbs and dt[...] otherwise.  A CTA owns 256 * EL coefficients of one limb for `per` members of a group:
 // a thread keeps the key words of its EL coefficients in registers (as doubles, or cut into pieces) and walks over the
 // members with the next member's digits in flight, so the keys -- two thirds of the words a member needs -- are read once.
-// One member per CTA read and converted them every time: 517 us for 64 members at level 6.
+// One member per CTA read and converted them every time: 517 us for 64 members at level 6.  Bound by DRAM: 48 members at level 8 take
+// 285 us at 5.3 TB/s (0.82 of a copy), 43 % of the issue slots.  Eight digits spill (132 bytes a thread), seven 12, fewer none.
 // grid = (N/(256*EL), groups * ceil(batch/per), ne); ND = digits in use
 template <int ND, int EL>
 __global__ void __launch_bounds__(256, EL == 1 ? 4 : ND <= 2 ? 3 : 2) k_ks_inner(u64 *acc, const __grid_constant__ SwitchList sl, int batch, int per, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl,
@@ -1115,8 +1118,9 @@ __global__ void __launch_bounds__(256, 2) k_ks_inner_mk(u64 *E, const u64 *c0, c
 // input members with the next member's words in flight.  Up to eleven masked-key words meet six words per member and coefficient;
 // staging both in shared memory by bulk copies for three members at a time took 1.6 times as long (they crossed L2 for every
 // third member, and a CTA's copies, sums and stores did not overlap).  Two coefficients per thread and two CTAs per SM: 869 us a launch
-// for 168 outputs at level 6; one coefficient and three CTAs 837 us, four CTAs 776 us (64 registers): the integer chains of
-// the 60-bit limbs want warps more than they want independent work in a thread.
+// for 168 outputs at level 6; one coefficient and three CTAs 837 us, four CTAs 776 us (64 registers, of which two digits spill 24
+// bytes a thread): the integer chains of the 60-bit limbs want warps more than they want independent work in a thread.  Bound by
+// instruction issue: 65 % of the slots and 52 % of the wide multiply-adds for 64 outputs (367 us), DRAM 3.1 TB/s.
 // grid = (N/256, groups * ceil(batch/per), ne)
 template <int ND, int CNT>
 __device__ __forceinline__ void ks_inner_mkr_body(u64 *o, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const MaskedRot &mr, int b0, int b1, const KsPlan *__restrict__ pl,
@@ -1380,8 +1384,8 @@ __global__ void k_keygen(u64 *__restrict__ b, const u64 *__restrict__ a, const u
 // (scale Delta^2, no rescale) for T output tiles t that share the shifted copies, which are stored k-major; the sum over b adds the
 // partial products of several K-groups in the same pass.  A thread works on E coefficients of both polynomials: a copy word is
 // read once for T tiles and a weight word once (and converted or cut once) for two polynomials.  Four tiles a launch in the layer
-// pass: one polynomial per thread with every product reduced 840 us, this 675 us; bound by the 60-bit limb's integer products and
-// by HBM on the copies.  grid = (N/(256*E), n)
+// pass: one polynomial per thread with every product reduced 840 us, this 675 us.  Bound by the latency of its loads: 16 warps
+// per SM (128 registers, of which two and four tiles spill 8 to 16 bytes) issue in 45 % of the slots, DRAM 2.1 TB/s, FP64 pipe 23 %.  grid = (N/(256*E), n)
 template <int T> struct TilePts { const u64 *p[T][16]; u64 *out[T]; };
 template <int T, int E>
 __global__ void __launch_bounds__(256, 2) k_matmul_acc(const __grid_constant__ TilePts<T> tp, const u64 *__restrict__ pre, int kcount, int btotal, int b0, int bcount, const u32 *__restrict__ gal,

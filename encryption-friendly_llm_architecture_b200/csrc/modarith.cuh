@@ -215,7 +215,7 @@ __device__ __forceinline__ u64 mad_wide(u32 a, u32 b, u64 c) {
     asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;" : "+r"(l), "+r"(h) : "r"(a), "r"(b));
     return ((u64)h << 32) | l;
 }
-// a0 + a1 * 2^30 + a2 * 2^60 modulo a prime of 45 to 60 bits (a0, a1 + 2^34, a2 + 2^34 < 2^64): below 4q
+// a0 + a1 * 2^30 + a2 * 2^60 modulo a prime of 45 to 60 bits (a0, a1 + 2^34, a2 + 2^34 < 2^64): below 3q
 __device__ __forceinline__ u64 finish_wide(u64 a0, u64 a1, u64 a2, const PrimeConst &m) {
     const u32 m30 = 0x3FFFFFFFu;
     if (m.d60) { // 2^60 = d60 modulo q
