@@ -376,6 +376,7 @@ def run_gpu(args):
     pb, iu = C.c_uint64(), C.c_uint64()
     lib.dll.hb_mem_info(lib.ctx, C.byref(pb), C.byref(iu))
     pool_gb = round(pb.value / 2 ** 30, 1)   # what the timed passes of the default schedule hold
+    timed_as = "cuda_graph_replay" if graph is not None else "host_launched"
     graph = graph_out = None
     gc.collect()
     lib.dll.hb_release_cached(lib.ctx)
@@ -492,7 +493,7 @@ def run_gpu(args):
             "config": {"workload": "bert_base_layer_matmuls_fwd_plus_lora_bwd", "units": len(wl.units), "batched_calls": True, "schedule": {0: "reference_sequence", 1: "direct_hoisted", 2: "direct_hoisted_one_division_per_copy"}[args.schedule], "ring_degree": 65536, "levels": 12, "tile": 128,
                        "l2": "working set per step is tens of GB, far above the 126 MB L2", "max_abs_err_vs_float64": err,
                        "bit_exact_units": bit_exact, "bit_exact_units_reference_sequence": faithful_exact, "outputs_sha256": outputs_sha, "outputs_missing": len(missing),
-                       "timed_as": "cuda_graph_replay" if graph is not None else "host_launched", "host_launched_ms": ms_eager,
+                       "timed_as": timed_as, "host_launched_ms": ms_eager,
                        "reference_sequence_ms": ms_faithful, "device_pool_gb": pool_gb},
             "schedule_roofline_ms": alg_bytes / (hbm * 1e6), "algorithmic_bytes_per_step": alg_bytes,
             "comm_ms": comm_ms, "exposed_comm_frac": comm_ms / ms_step if ms_step else None,
