@@ -168,9 +168,13 @@ class Lib:
         n = len(items)
         if not self.has("decrypt_many"):  # a library without the batched entry point: one call per member
             return np.stack([self.decrypt(ct, k) for ct, k in items])
-        re = np.zeros((n, self.slots)); im = np.zeros((n, self.slots))
         cts = (C.c_void_p * n)(*[ct.ptr.value for ct, _ in items])
         idx = (C.c_int * n)(*[int(k) for _, k in items])
+        if self.has("decrypt_many_complex"):
+            z = np.empty((n, self.slots), dtype=np.complex128)
+            self._chk(self._fn("decrypt_many_complex")(self.ctx, cts, idx, C.c_int(n), z.ctypes.data_as(C.POINTER(C.c_double))))
+            return z
+        re = np.zeros((n, self.slots)); im = np.zeros((n, self.slots))
         self._chk(self._fn("decrypt_many")(self.ctx, cts, idx, C.c_int(n), _f64(re), _f64(im)))
         return re + 1j * im
 

@@ -7,12 +7,14 @@
 #include "kernels.cuh"
 #include "ntt.cuh"
 #include "convcols.cuh"
+#include "embed.cuh"
 
 #include <cstdio>
 #include <dlfcn.h>
 #include <map>
 #include <thread>
 #include <memory>
+#include <system_error>
 #include <mutex>
 #include <nccl.h> // types only: the library is resolved at run time, see nccl_api()
 #include <unordered_map>
@@ -123,10 +125,16 @@ struct hb_ctx {
     InvScale p_inv_scale{};               // 2^16 rings: P^-1 mod q_l
     std::map<int, InvScale> div_scale;    // (P * q_level)^-1 mod q_l per level
     bool smem_opt_in_conv = false;
-    u64 *pinned = nullptr; size_t pinned_bytes = 0; // host staging buffer of hb_decrypt_many
+    // slot values on their way between the caller's memory and the device: two pinned buffers, each with the event of its last copy
+    double *stage[2] = {nullptr, nullptr};
+    cudaEvent_t staged[2] = {nullptr, nullptr};
+    double2 *emb = nullptr;               // twiddles of the embedding, inverse then forward
+    u64 *cdt = nullptr;                   // table of the discrete Gaussian
+    EmbedTables emb_tb{};
+    CentreConst centre{};
     ChaChaKey ckey{};
     std::map<std::pair<int, long long>, u32 *> gal_tables; // (copies, row_step) -> Galois elements of hb_matmul_acc, on the device
-    int host_threads = 0;                                 // cap for the host-side encode / decode workers (0: all cores, at most 32)
+    int host_threads = 0;                                 // cap for the threads that move slot values in host memory (0: no cap beyond kCopyThreads)
     bool capturing = false;                               // between hb_graph_begin and hb_graph_end
     unsigned long long launches_at_capture = 0, alg_at_capture = 0;
     int N = 0, logn = 0, L = 0, K = 0, nprimes = 0;
@@ -525,6 +533,14 @@ const u32 *galois_table(hb_ctx *c, int copies, i64 row_step) {
     return d;
 }
 
+// out [count][limbs of map][N]: coef (null: none) plus a discrete Gaussian polynomial from the streams `ids`, coefficient form
+void error_residues(hb_ctx *c, u64 *out, const i64 *coef, const StreamIds &ids, int count, const LimbMap &map) {
+    launch(c, coef ? k_residues<true, true> : k_residues<false, true>, dim3((unsigned)((c->N / 8 + 127) / 128), (unsigned)count), 128, 0, out, coef, ids, (const u64 *)c->cdt,
+           (int)c->h->gauss_cdt.size(), map, c->pc, c->N);
+}
+void message_residues(hb_ctx *c, u64 *out, const i64 *coef, int count, const LimbMap &map) {
+    launch(c, k_residues<true, false>, dim3((unsigned)((c->N / 8 + 127) / 128), (unsigned)count), 128, 0, out, coef, StreamIds{}, (const u64 *)nullptr, 0, map, c->pc, c->N);
+}
 // switching key for secret s' (g == 0: s^2, else s o perm_g); stream ids kid*64 + digit
 Evk make_key(hb_ctx *c, u64 kid, u32 g) {
     if (!c->have_sk) fail(HB_E_NOKEY, "secret key not generated");
@@ -532,24 +548,17 @@ Evk make_key(hb_ctx *c, u64 kid, u32 g) {
     const HostCtx &h = *c->h;
     const int N = c->N, np = c->nprimes, nd = h.digit_of(h.L) + 1;
     Evk k; k.nd = nd; k.d = c->alloc_limbs((size_t)nd * 2 * np);
-    const LimbMap am = c->allmap();
-    Tmp e(c, (size_t)np);
-    TmpBytes ecoef_buf(c, (size_t)N * 8);
-    i64 *ecoef = (i64 *)ecoef_buf.p;
-    Scalars pmod{};
-    for (int pi = 0; pi <= h.L; ++pi) { u64 v = 1; for (int j = 0; j < h.K; ++j) v = hbhost::mulmod(v, h.q[h.L + 1 + j] % h.q[pi], h.q[pi]); pmod.v[pi] = v; }
-    std::vector<i64> ev;
-    for (int dg = 0; dg < nd; ++dg) {
-        u64 *b = k.d + ((size_t)dg * 2) * np * N, *a = b + (size_t)np * N;
-        LAUNCH(c), k_uniform<<<dim3((unsigned)((N / 4 + 255) / 256), np), 256, 0, c->st>>>(a, am, c->pc, N, c->ckey, hbhost::STREAM_KEY_A, kid * 64 + dg);
-        h.sample_gauss(hbhost::STREAM_KEY_E, kid * 64 + dg, ev);
-        CK(cudaMemcpyAsync(ecoef, ev.data(), (size_t)N * 8, cudaMemcpyHostToDevice, c->st));
-        LAUNCH(c), k_reduce_i64<<<c->egrid(np), 256, 0, c->st>>>(e.p, ecoef, am, c->pc, N);
-        CK(cudaStreamSynchronize(c->st)); // ev is reused by the next digit
-        ntt_inplace(c, e.p, np, am, false);
-        LAUNCH(c), k_keygen<<<c->egrid(np), 256, 0, c->st>>>(b, a, e.p, c->sk, c->pc, N, c->logn, g, h.digit_lo(dg), h.digit_hi(dg, h.L + 1), pmod);
-    }
-    CK(cudaGetLastError());
+    try {
+        const LimbMap am = c->allmap();
+        Tmp e(c, (size_t)nd * np);
+        Scalars pmod{};
+        for (int pi = 0; pi <= h.L; ++pi) { u64 v = 1; for (int j = 0; j < h.K; ++j) v = hbhost::mulmod(v, h.q[h.L + 1 + j] % h.q[pi], h.q[pi]); pmod.v[pi] = v; }
+        error_residues(c, e.p, nullptr, StreamIds{c->ckey, hbhost::STREAM_KEY_E, nullptr, kid * 64}, nd, am);
+        ntt_inplace(c, e.p, nd * np, am, false);
+        LAUNCH(c), k_keygen<<<dim3((unsigned)((N / 4 + 255) / 256), np, nd), 256, 0, c->st>>>(k.d, e.p, c->sk, StreamIds{c->ckey, hbhost::STREAM_KEY_A, nullptr, kid * 64}, c->pc, N, c->logn, g,
+                                                                                             h.L + 1, h.alpha, pmod);
+        CK(cudaGetLastError());
+    } catch (...) { c->pool.put(k.d); throw; }
     return k;
 }
 const Evk &galois_key(hb_ctx *c, u64 g) {
@@ -949,10 +958,102 @@ u64 *noalloc_scratch(int device) {
     return g_noalloc_ptr[device];
 }
 
-// host threads for the encode / decode halves of hb_encrypt_many / hb_decrypt_many
-int host_workers(const hb_ctx *c, int tasks) {
-    const int cap = c->host_threads > 0 ? c->host_threads : std::min(32, std::max(1, (int)std::thread::hardware_concurrency()));
-    return std::max(1, std::min(tasks, cap));
+// ---- slot values between the caller's memory and the device ----
+// Messages travel in chunks of kStageMembers through two pinned buffers, so that moving one chunk in host memory overlaps the copy and
+// the transforms of the other.  The caller's pages are often new ones, whose first touch costs more than the bytes: several threads.
+constexpr int kStageMembers = 8, kCopyThreads = 4;
+size_t stage_words(const hb_ctx *c) { return (size_t)kStageMembers * c->N; } // two doubles per slot
+void stage_open(hb_ctx *c) {
+    if (c->stage[0]) return;
+    for (int i = 0; i < 2; ++i) if (!c->staged[i]) CK(cudaEventCreateWithFlags(&c->staged[i], cudaEventDisableTiming));
+    double *p = nullptr;
+    CK(cudaMallocHost(&p, 2 * stage_words(c) * sizeof(double)));
+    c->stage[0] = p; c->stage[1] = p + stage_words(c);
+}
+void host_copy(const hb_ctx *c, double *dst, const double *src, size_t words) {
+    const size_t per = (size_t)1 << 16; // words that are worth a thread
+    const int cap = c->host_threads > 0 ? std::min(c->host_threads, kCopyThreads) : kCopyThreads;
+    const int n = (int)std::max<size_t>(1, std::min<size_t>((size_t)cap, words / per));
+    const size_t step = (words + n - 1) / n;
+    auto part = [=](int t) { std::memcpy(dst + t * step, src + t * step, std::min(step, words - t * step) * sizeof(double)); };
+    std::thread pool[kCopyThreads];
+    int started = 1;
+    try { for (; started < n; ++started) pool[started] = std::thread(part, started); } catch (const std::system_error &) {} // no more threads: the rest here
+    part(0);
+    for (int t = started; t < n; ++t) part(t);
+    for (int t = 1; t < started; ++t) pool[t].join();
+}
+// coef [count][N] = rounded coefficients at scale sc of the messages re / im [count][n] on the device (im may be null)
+void embed_inverse(hb_ctx *c, i64 *coef, const double *re, const double *im, int n, int count, double sc) {
+    if (c->logn == 16) {
+        Tmp v(c, (size_t)count);
+        launch(c, k_embed_inv_cols, dim3(16, (unsigned)count), kEmbThreads, 0, (double2 *)v.p, re, im, n, c->emb_tb);
+        launch(c, k_embed_inv_rows, dim3(16, (unsigned)count), kEmbThreads, 0, coef, (const double2 *)v.p, sc, c->emb_tb);
+    } else launch(c, k_embed_inv_small, dim3((unsigned)count), 256, 0, coef, re, im, n, c->logn - 1, sc, c->emb_tb);
+}
+// slot values of the residues t [count][2][N]: member b, slot s at re[(b * slots + s) * stride], im likewise
+void embed_forward(hb_ctx *c, double *re, double *im, int stride, const u64 *t, const DecItem *items, int count) {
+    if (c->logn == 16) {
+        Tmp v(c, (size_t)count);
+        launch(c, k_embed_fwd_rows, dim3(16, (unsigned)count), kEmbThreads, 0, (double2 *)v.p, t, items, c->centre, c->pc, c->emb_tb);
+        launch(c, k_embed_fwd_cols, dim3(16, (unsigned)count), kEmbThreads, 0, re, im, stride, (const double2 *)v.p, c->emb_tb);
+    } else launch(c, k_embed_fwd_small, dim3((unsigned)count), 256, 0, re, im, stride, t, items, c->logn - 1, c->centre, c->pc, c->emb_tb);
+}
+// Messages re / im [count][n] in host memory, chunk by chunk: use(first member, members, coefficients on the device, stream).  Every chunk's
+// values have left the caller's memory when this returns; the device may still be at work.
+template <class F> void encode_chunks(hb_ctx *c, const double *re, const double *im, size_t n, int count, double sc, F &&use) {
+    stage_open(c);
+    for (int first = 0, slot = 0; first < count; first += kStageMembers, slot ^= 1) {
+        const int m = std::min(kStageMembers, count - first);
+        const size_t words = (size_t)m * n;
+        CK(cudaEventSynchronize(c->staged[slot])); // its last copy has been made
+        double *h = c->stage[slot];
+        host_copy(c, h, re + (size_t)first * n, words);
+        if (im) host_copy(c, h + words, im + (size_t)first * n, words);
+        TmpBytes d(c, std::max<size_t>(1, words * (im ? 2 : 1)) * sizeof(double)), coef(c, (size_t)m * c->N * sizeof(i64));
+        double *dr = (double *)d.p;
+        CK(cudaMemcpyAsync(dr, h, words * (im ? 2 : 1) * sizeof(double), cudaMemcpyHostToDevice, c->st));
+        CK(cudaEventRecord(c->staged[slot], c->st));
+        embed_inverse(c, (i64 *)coef.p, dr, im ? dr + words : nullptr, (int)n, m, sc);
+        use(first, m, (const i64 *)coef.p);
+    }
+}
+// Decrypts and decodes `count` items into host memory: member i at re[i * slots], im likewise (im may be null); or, z, as complex values
+// at re[2 * i * slots].
+void decrypt_items(hb_ctx *c, const std::vector<DecItem> &items, bool z, double *re, double *im) {
+    stage_open(c);
+    const int count = (int)items.size(), N = c->N, slots = N / 2;
+    TmpBytes list(c, items.size() * sizeof(DecItem));
+    CK(cudaMemcpyAsync(list.p, items.data(), items.size() * sizeof(DecItem), cudaMemcpyHostToDevice, c->st));
+    auto collect = [&](int first, int slot) {
+        const int m = std::min(kStageMembers, count - first);
+        const size_t words = (size_t)m * slots;
+        CK(cudaEventSynchronize(c->staged[slot]));
+        const double *h = c->stage[slot];
+        if (z) { host_copy(c, re + (size_t)first * N, h, 2 * words); return; }
+        host_copy(c, re + (size_t)first * slots, h, words);
+        if (im) host_copy(c, im + (size_t)first * slots, h + words, words);
+    };
+    int slot = 0;
+    for (int first = 0; first < count; first += kStageMembers, slot ^= 1) {
+        const int m = std::min(kStageMembers, count - first);
+        const size_t words = (size_t)m * slots;
+        const DecItem *it = (const DecItem *)list.p + first;
+        Tmp t(c, (size_t)m * 2), v(c, (size_t)m);
+        launch(c, k_decrypt, dim3(c->gx(), 2, (unsigned)m), 256, 0, t.p, it, (const u64 *)c->sk, c->pc, N);
+        ntt_inplace(c, t.p, m * 2, c->qmap(1), true);
+        double *d = (double *)v.p;
+        embed_forward(c, d, z ? d + 1 : d + words, z ? 2 : 1, t.p, it, m);
+        CK(cudaMemcpyAsync(c->stage[slot], d, words * (z || im ? 2 : 1) * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaEventRecord(c->staged[slot], c->st));
+        if (first) collect(first - kStageMembers, slot ^ 1);
+    }
+    collect((count - 1) / kStageMembers * kStageMembers, slot ^ 1);
+}
+double scale_of(const hb_ctx *c, int level, int spow) { return spow == 2 ? c->h->scale[level] * c->h->scale[level] : c->h->scale[level]; }
+DecItem dec_item(const hb_ctx *c, const hb_ct *ct, int index) {
+    const int n = ct->level + 1;
+    return DecItem{ct->d + (size_t)index * ct->np * n * c->N, n, ct->np, scale_of(c, ct->level, ct->spow)};
 }
 
 template <class F> int guard(hb_ctx *c, F &&f) {
@@ -1056,6 +1157,19 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             c->tb.psi = c->tw; c->tb.psi_sh = c->tw + (size_t)np * N; c->tb.ipsi = c->tw + (size_t)2 * np * N; c->tb.ipsi_sh = c->tw + (size_t)3 * np * N;
         }
         CK(cudaMalloc(&c->sk, (size_t)np * N * 8));
+        std::vector<hbhost::Cpx> ei, ef;
+        c->h->embed_twiddles(ei, ef);
+        static_assert(sizeof(hbhost::Cpx) == sizeof(double2), "complex values");
+        const size_t slots = ei.size();
+        CK(cudaMalloc(&c->emb, 2 * slots * sizeof(double2)));
+        CK(cudaMemcpy(c->emb, ei.data(), slots * sizeof(double2), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(c->emb + slots, ef.data(), slots * sizeof(double2), cudaMemcpyHostToDevice));
+        c->emb_tb = EmbedTables{c->emb, c->emb + slots};
+        const std::vector<hbhost::u64> &cdt = c->h->gauss_cdt;
+        CK(cudaMalloc(&c->cdt, std::max<size_t>(1, cdt.size()) * 8));
+        CK(cudaMemcpy(c->cdt, cdt.data(), cdt.size() * 8, cudaMemcpyHostToDevice));
+        const unsigned __int128 Q = (unsigned __int128)c->h->q[0] * c->h->q[1];
+        c->centre = CentreConst{c->h->q[0], c->h->q[0] / 2, (u64)(Q >> 64), (u64)Q, (u64)((Q / 2) >> 64), (u64)(Q / 2), hbhost::invmod(c->h->q[0] % c->h->q[1], c->h->q[1])};
     } catch (const CudaFail &) { hb_ctx_destroy(c); return HB_E_CUDA; }
     catch (const ArgFail &e) { int code = e.code; hb_ctx_destroy(c); return code; }
     catch (...) { hb_ctx_destroy(c); return HB_E_ARG; }
@@ -1070,7 +1184,10 @@ void hb_ctx_destroy(hb_ctx *c) {
     for (auto &kv : c->div_plans) cudaFree(kv.second);
     for (auto &kv : c->conv_plans) cudaFree(kv.second);
     for (auto &kv : c->gal_tables) cudaFree(kv.second);
-    if (c->pinned) cudaFreeHost(c->pinned);
+    if (c->stage[0]) cudaFreeHost(c->stage[0]);
+    for (cudaEvent_t e : c->staged) if (e) cudaEventDestroy(e);
+    if (c->emb) cudaFree(c->emb);
+    if (c->cdt) cudaFree(c->cdt);
     if (c->pc) cudaFree(c->pc);
     if (c->tw) cudaFree(c->tw);
     if (c->sk) cudaFree(c->sk);
@@ -1134,7 +1251,7 @@ int hb_keygen(hb_ctx *c) {
         i64 *sc = (i64 *)sc_buf.p;
         CK(cudaMemcpyAsync(sc, s.data(), (size_t)c->N * 8, cudaMemcpyHostToDevice, c->st));
         const LimbMap am = c->allmap();
-        LAUNCH(c), k_reduce_i64<<<c->egrid(c->nprimes), 256, 0, c->st>>>(c->sk, sc, am, c->pc, c->N);
+        message_residues(c, c->sk, sc, 1, am);
         ntt_inplace(c, c->sk, c->nprimes, am, false);
         CK(cudaStreamSynchronize(c->st));
         c->have_sk = true;
@@ -1163,23 +1280,20 @@ int hb_evk_export(hb_ctx *c, uint64_t g, uint64_t *host, int *digits) {
     });
 }
 
+static void encode_into(hb_ctx *c, hb_pt *p, const double *re, const double *im, size_t n, const LimbMap &map) {
+    try {
+        encode_chunks(c, re, im, n, 1, c->h->scale[p->level], [&](int, int, const i64 *coef) { message_residues(c, p->d, coef, 1, map); });
+        ntt_inplace(c, p->d, map.n, map, false);
+        CK(cudaStreamSynchronize(c->st));
+    } catch (...) { hb_pt_free(p); throw; }
+}
 int hb_encode(hb_ctx *c, const double *re, const double *im, size_t n, int level, hb_pt **out) {
     return guard(c, [&] {
         no_capture(c, "encode");
         if (!re || !out || n > (size_t)c->h->slots) fail(HB_E_ARG, "encode: bad message");
         if (level < 0 || level > c->L) fail(HB_E_LEVEL, "encode: bad level");
-        std::vector<i64> coef;
-        c->h->encode_coeffs(re, im, n, c->h->scale[level], coef);
         hb_pt *p = new_pt(c, level, 1);
-        try {
-            TmpBytes dcb(c, (size_t)c->N * 8);
-            i64 *dc = (i64 *)dcb.p;
-            CK(cudaMemcpyAsync(dc, coef.data(), (size_t)c->N * 8, cudaMemcpyHostToDevice, c->st));
-            const LimbMap qm = c->qmap(level);
-            LAUNCH(c), k_reduce_i64<<<c->egrid(level + 1), 256, 0, c->st>>>(p->d, dc, qm, c->pc, c->N);
-            ntt_inplace(c, p->d, level + 1, qm, false);
-            CK(cudaStreamSynchronize(c->st)); // coef goes out of scope
-        } catch (...) { hb_pt_free(p); throw; }
+        encode_into(c, p, re, im, n, c->qmap(level));
         *out = p;
     });
 }
@@ -1188,42 +1302,20 @@ int hb_encode_ext(hb_ctx *c, const double *re, const double *im, size_t n, int l
         no_capture(c, "encode_ext");
         if (!re || !out || n > (size_t)c->h->slots) fail(HB_E_ARG, "encode: bad message");
         if (level < 0 || level > c->L) fail(HB_E_LEVEL, "encode: bad level");
-        std::vector<i64> coef;
-        c->h->encode_coeffs(re, im, n, c->h->scale[level], coef);
         const int ne = level + 1 + c->K;
         hb_pt *p = new hb_pt{c, level, 1, nullptr};
         p->ext = 1;
         try { p->d = c->alloc_limbs((size_t)ne); } catch (...) { delete p; throw; }
-        try {
-            TmpBytes dcb(c, (size_t)c->N * 8);
-            i64 *dc = (i64 *)dcb.p;
-            CK(cudaMemcpyAsync(dc, coef.data(), (size_t)c->N * 8, cudaMemcpyHostToDevice, c->st));
-            LimbMap em{}; em.n = ne;
-            for (int j = 0; j < ne; ++j) em.prime[j] = (unsigned char)(j <= level ? j : c->L + 1 + (j - level - 1));
-            LAUNCH(c), k_reduce_i64<<<c->egrid(ne), 256, 0, c->st>>>(p->d, dc, em, c->pc, c->N);
-            ntt_inplace(c, p->d, ne, em, false);
-            CK(cudaStreamSynchronize(c->st)); // coef goes out of scope
-        } catch (...) { hb_pt_free(p); throw; }
+        LimbMap em{}; em.n = ne;
+        for (int j = 0; j < ne; ++j) em.prime[j] = (unsigned char)(j <= level ? j : c->L + 1 + (j - level - 1));
+        encode_into(c, p, re, im, n, em);
         *out = p;
     });
-}
-static void decode_limbs(hb_ctx *c, const u64 *dev_coef, int level, int spow, double *re, double *im) {
-    const int nl = level >= 1 ? 2 : 1, N = c->N;
-    std::vector<u64> hc((size_t)nl * N);
-    CK(cudaMemcpyAsync(hc.data(), dev_coef, hc.size() * 8, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    std::vector<double> val;
-    c->h->centre(hc.data(), nl == 2 ? hc.data() + N : nullptr, val);
-    const double sc = spow == 2 ? c->h->scale[level] * c->h->scale[level] : c->h->scale[level];
-    c->h->decode_values(val, sc, re, im);
 }
 int hb_decode(hb_ctx *c, const hb_pt *p, double *re, double *im) {
     return guard(c, [&] {
         no_capture(c, "decode");
-        const int nl = p->level >= 1 ? 2 : 1;
-        Tmp t(c, (size_t)nl);
-        ntt(c, p->d, (size_t)nl * c->N, t.p, (size_t)nl * c->N, nl, c->qmap(nl - 1), true);
-        decode_limbs(c, t.p, p->level, p->spow, re, im);
+        decrypt_items(c, {DecItem{p->d, p->level + 1, 1, scale_of(c, p->level, p->spow)}}, false, re, im);
     });
 }
 int hb_encrypt(hb_ctx *c, const hb_pt *p, uint64_t nonce, hb_ct **out) {
@@ -1234,16 +1326,11 @@ int hb_encrypt(hb_ctx *c, const hb_pt *p, uint64_t nonce, hb_ct **out) {
         hb_ct *r = new_ct(c, p->level, 2, 1, p->spow);
         try {
             const LimbMap qm = c->qmap(p->level);
-            u64 *b = r->d, *a = r->d + (size_t)n * N;
-            LAUNCH(c), k_uniform<<<dim3((unsigned)((N / 4 + 255) / 256), n), 256, 0, c->st>>>(a, qm, c->pc, N, c->ckey, hbhost::STREAM_ENC_A, nonce);
-            std::vector<i64> ev; c->h->sample_gauss(hbhost::STREAM_ENC_E, nonce, ev);
-            TmpBytes ecb(c, (size_t)N * 8);
-            i64 *ec = (i64 *)ecb.p;
             Tmp e(c, (size_t)n);
-            CK(cudaMemcpyAsync(ec, ev.data(), (size_t)N * 8, cudaMemcpyHostToDevice, c->st));
-            LAUNCH(c), k_reduce_i64<<<c->egrid(n), 256, 0, c->st>>>(e.p, ec, qm, c->pc, N);
+            error_residues(c, e.p, nullptr, StreamIds{c->ckey, hbhost::STREAM_ENC_E, nullptr, nonce}, 1, qm);
             ntt_inplace(c, e.p, n, qm, false);
-            LAUNCH(c), k_encrypt<<<c->egrid(n), 256, 0, c->st>>>(b, a, e.p, c->sk, p->d, qm, c->pc, N);
+            launch(c, k_encrypt, dim3((unsigned)((N / 4 + 255) / 256), (unsigned)n), 256, 0, r->d, (const u64 *)e.p, (const u64 *)p->d, (const u64 *)c->sk,
+                   StreamIds{c->ckey, hbhost::STREAM_ENC_A, nullptr, nonce}, c->pc, N);
             CK(cudaStreamSynchronize(c->st));
         } catch (...) { hb_ct_free(r); throw; }
         *out = r;
@@ -1257,46 +1344,20 @@ int hb_encrypt_many(hb_ctx *c, const double *re, const double *im, size_t n_slot
         if (!re || !nonces || !out || count < 1 || n_slots > (size_t)c->h->slots) fail(HB_E_ARG, "encrypt_many: bad message");
         if (level < 0 || level > c->L) fail(HB_E_LEVEL, "encrypt_many: bad level");
         const int n = level + 1, N = c->N;
-        const HostCtx &h = *c->h;
-        // host part, one member per task: inverse embedding + rounding, and the error polynomial
-        const size_t words = (size_t)count * 2 * N;
-        if (c->pinned_bytes < words * 8) {
-            if (c->pinned) CK(cudaFreeHost(c->pinned));
-            c->pinned = nullptr; c->pinned_bytes = 0;
-            CK(cudaMallocHost(&c->pinned, words * 8));
-            c->pinned_bytes = words * 8;
-        }
-        i64 *host = (i64 *)c->pinned; // [count][2][N]: message coefficients, error coefficients
-        const int workers = host_workers(c, count);
-        std::vector<std::thread> pool;
-        for (int w = 0; w < workers; ++w)
-            pool.emplace_back([&, w] {
-                std::vector<i64> v;
-                for (int i = w; i < count; i += workers) {
-                    h.encode_coeffs(re + (size_t)i * n_slots, im ? im + (size_t)i * n_slots : nullptr, n_slots, h.scale[level], v);
-                    std::memcpy(host + (size_t)i * 2 * N, v.data(), (size_t)N * 8);
-                    h.sample_gauss(hbhost::STREAM_ENC_E, nonces[i], v);
-                    std::memcpy(host + ((size_t)i * 2 + 1) * N, v.data(), (size_t)N * 8);
-                }
-            });
-        for (auto &th : pool) th.join();
         hb_ct *r = new_ct(c, level, 2, count, 1);
         try {
             const LimbMap qm = c->qmap(level);
-            TmpBytes dcb(c, words * 8);
-            i64 *dc = (i64 *)dcb.p;
-            Tmp me(c, (size_t)count * 2 * n); // [count][message | error][n][N]
-            CK(cudaMemcpyAsync(dc, host, words * 8, cudaMemcpyHostToDevice, c->st));
-            for (int i = 0; i < count * 2; ++i)
-                LAUNCH(c), k_reduce_i64<<<c->egrid(n), 256, 0, c->st>>>(me.p + (size_t)i * n * N, dc + (size_t)i * N, qm, c->pc, N);
-            ntt_inplace(c, me.p, count * 2 * n, qm, false);
-            for (int i = 0; i < count; ++i) {
-                u64 *b = r->d + (size_t)i * 2 * n * N, *a = b + (size_t)n * N;
-                LAUNCH(c), k_uniform<<<dim3((unsigned)((N / 4 + 255) / 256), n), 256, 0, c->st>>>(a, qm, c->pc, N, c->ckey, hbhost::STREAM_ENC_A, nonces[i]);
-                LAUNCH(c), k_encrypt<<<c->egrid(n), 256, 0, c->st>>>(b, a, me.p + ((size_t)i * 2 + 1) * n * N, c->sk, me.p + (size_t)i * 2 * n * N, qm, c->pc, N);
-            }
-            CK(cudaGetLastError());
-            CK(cudaStreamSynchronize(c->st)); // the staging buffer is reused by the next call
+            TmpBytes ids(c, (size_t)count * 8);
+            CK(cudaMemcpyAsync(ids.p, nonces, (size_t)count * 8, cudaMemcpyHostToDevice, c->st));
+            Tmp me(c, (size_t)std::min(count, kStageMembers) * n); // message + error; NTT form is linear, one transform serves both
+            encode_chunks(c, re, im, n_slots, count, c->h->scale[level], [&](int first, int m, const i64 *coef) {
+                const u64 *id = (const u64 *)ids.p + first;
+                error_residues(c, me.p, coef, StreamIds{c->ckey, hbhost::STREAM_ENC_E, id, 0}, m, qm);
+                ntt_inplace(c, me.p, m * n, qm, false);
+                launch(c, k_encrypt, dim3((unsigned)((N / 4 + 255) / 256), (unsigned)n, (unsigned)m), 256, 0, r->d + (size_t)first * 2 * n * N, (const u64 *)me.p, (const u64 *)nullptr,
+                       (const u64 *)c->sk, StreamIds{c->ckey, hbhost::STREAM_ENC_A, id, 0}, c->pc, N);
+            });
+            CK(cudaStreamSynchronize(c->st)); // the nonces are the caller's memory
         } catch (...) { hb_ct_free(r); throw; }
         *out = r;
     });
@@ -1306,71 +1367,25 @@ int hb_decrypt(hb_ctx *c, const hb_ct *ct, int index, double *re, double *im) {
         no_capture(c, "decrypt");
         if (!c->have_sk) fail(HB_E_NOKEY, "secret key not generated");
         if (index < 0 || index >= ct->batch) fail(HB_E_ARG, "decrypt: bad batch index");
-        const int n = ct->level + 1, N = c->N, nl = ct->level >= 1 ? 2 : 1;
-        Tmp t(c, (size_t)nl);
-        LAUNCH(c), k_decrypt<<<c->egrid(nl), 256, 0, c->st>>>(t.p, ct->d + (size_t)index * ct->np * n * N, n, ct->np, c->sk, c->pc, N);
-        ntt_inplace(c, t.p, nl, c->qmap(nl - 1), true);
-        decode_limbs(c, t.p, ct->level, ct->spow, re, im);
+        decrypt_items(c, {dec_item(c, ct, index)}, false, re, im);
     });
 }
-
-int hb_decrypt_many(hb_ctx *c, const hb_ct *const *cts, const int *index, int count, double *re, double *im) {
+static int decrypt_list(hb_ctx *c, const hb_ct *const *cts, const int *index, int count, bool z, double *re, double *im) {
     return guard(c, [&] {
         no_capture(c, "decrypt_many");
         if (!c->have_sk) fail(HB_E_NOKEY, "secret key not generated");
         if (count < 1 || !cts || !re) fail(HB_E_ARG, "decrypt_many: nothing to decrypt");
-        const int N = c->N, slots = c->h->slots;
-        bool two = true;
+        std::vector<DecItem> items((size_t)count);
         for (int i = 0; i < count; ++i) {
             const int idx = index ? index[i] : 0;
             if (!cts[i] || idx < 0 || idx >= cts[i]->batch) fail(HB_E_ARG, "decrypt_many: bad batch index");
-            if (cts[i]->level < 1) two = false;
+            items[(size_t)i] = dec_item(c, cts[i], idx);
         }
-        if (!two) { // a level-0 member has one limb only: take the members one by one
-            for (int i = 0; i < count; ++i) {
-                const hb_ct *ct = cts[i];
-                const int n = ct->level + 1, nl = ct->level >= 1 ? 2 : 1;
-                Tmp t(c, (size_t)nl);
-                LAUNCH(c), k_decrypt<<<c->egrid(nl), 256, 0, c->st>>>(t.p, ct->d + (size_t)(index ? index[i] : 0) * ct->np * n * N, n, ct->np, c->sk, c->pc, N);
-                ntt_inplace(c, t.p, nl, c->qmap(nl - 1), true);
-                decode_limbs(c, t.p, ct->level, ct->spow, re + (size_t)i * slots, im ? im + (size_t)i * slots : nullptr);
-            }
-            return;
-        }
-        const size_t bytes = (size_t)count * 2 * N * 8;
-        if (c->pinned_bytes < bytes) {
-            if (c->pinned) CK(cudaFreeHost(c->pinned));
-            c->pinned = nullptr; c->pinned_bytes = 0;
-            CK(cudaMallocHost(&c->pinned, bytes));
-            c->pinned_bytes = bytes;
-        }
-        Tmp t(c, (size_t)count * 2);
-        for (int i = 0; i < count; ++i) {
-            const hb_ct *ct = cts[i];
-            const int n = ct->level + 1;
-            LAUNCH(c), k_decrypt<<<c->egrid(2), 256, 0, c->st>>>(t.p + (size_t)i * 2 * N, ct->d + (size_t)(index ? index[i] : 0) * ct->np * n * N, n, ct->np, c->sk, c->pc, N);
-        }
-        ntt_inplace(c, t.p, count * 2, c->qmap(1), true);
-        CK(cudaMemcpyAsync(c->pinned, t.p, bytes, cudaMemcpyDeviceToHost, c->st));
-        CK(cudaStreamSynchronize(c->st));
-        // CRT lift and inverse embedding on the host cores, one member per task
-        const int workers = host_workers(c, count);
-        std::vector<std::thread> pool;
-        const HostCtx &h = *c->h;
-        const u64 *host = c->pinned;
-        for (int w = 0; w < workers; ++w)
-            pool.emplace_back([&, w] {
-                std::vector<double> val;
-                for (int i = w; i < count; i += workers) {
-                    const hb_ct *ct = cts[i];
-                    h.centre(host + (size_t)i * 2 * N, host + ((size_t)i * 2 + 1) * N, val);
-                    const double sc = ct->spow == 2 ? h.scale[ct->level] * h.scale[ct->level] : h.scale[ct->level];
-                    h.decode_values(val, sc, re + (size_t)i * slots, im ? im + (size_t)i * slots : nullptr);
-                }
-            });
-        for (auto &th : pool) th.join();
+        decrypt_items(c, items, z, re, im);
     });
 }
+int hb_decrypt_many(hb_ctx *c, const hb_ct *const *cts, const int *index, int count, double *re, double *im) { return decrypt_list(c, cts, index, count, false, re, im); }
+int hb_decrypt_many_complex(hb_ctx *c, const hb_ct *const *cts, const int *index, int count, double *z) { return decrypt_list(c, cts, index, count, true, z, nullptr); }
 
 int hb_ct_create(hb_ctx *c, int level, int np, int batch, int spow, hb_ct **out) { return guard(c, [&] { *out = new_ct(c, level, np, batch, spow); }); }
 int hb_ct_clone(hb_ctx *c, const hb_ct *s, hb_ct **out) {

@@ -1,7 +1,6 @@
 // Host-side parameter set of the CUDA library: prime chain, NTT twiddles, scale ladder,
-// canonical-embedding FFT, key-switch constants and the small host samplers.
-// Everything heavy runs on the device; this file only prepares tables and does the
-// float64 encode/decode transform (a 2^15-point FFT per plaintext).
+// embedding twiddles, the table of the discrete Gaussian and the sampler of the secret.
+// This file only prepares tables; the transforms and the other samplers run on the device.
 //
 // Parameter rules (shared with any party that must reproduce the same ciphertext bits):
 //   * primes are congruent to 1 modulo 2N.  q_0 is the largest such prime below 2^q0_bits; the K
@@ -65,7 +64,7 @@ struct HostParams {
     u64 seed[4];
 };
 
-// ChaCha20 block function (RFC 8439), host copy for the small sequential samplers.
+// ChaCha20 block function (RFC 8439), host copy for the secret.
 struct HostChaCha {
     u32 key[8];
     static u32 rol(u32 v, int c) { return (v << c) | (v >> (32 - c)); }
@@ -213,84 +212,21 @@ struct HostCtx {
     u64 galois_rot(i64 left) const { i64 r = left % slots; if (r < 0) r += slots; return orbit5[(size_t)r]; }
     u64 galois_conj() const { return (u64)2 * N - 1; }
 
-    // ----- special FFT over the orbit of 5 (in place, size = slots) -----
-    static void bit_reverse_permute(std::vector<Cpx> &v) {
-        const size_t n = v.size();
-        for (size_t i = 1, j = 0; i < n; ++i) {
-            size_t bit = n >> 1;
-            while (j >= bit) { j -= bit; bit >>= 1; }
-            j += bit;
-            if (i < j) std::swap(v[i], v[j]);
-        }
-    }
-    void embed_inverse(std::vector<Cpx> &v) const { // slot values -> (re, im) halves of the coefficient vector
-        const size_t n = v.size(); const u64 M = (u64)2 * N;
-        for (size_t len = n; len >= 2; len >>= 1) {
-            const size_t h = len >> 1, quad = len << 2; const u64 stride = M / quad;
-            for (size_t base = 0; base < n; base += len)
-                for (size_t j = 0; j < h; ++j) {
-                    const Cpx w = unit[(quad - orbit5[j] % quad) * stride];
-                    Cpx a = v[base + j], b = v[base + j + h];
-                    Cpx s = {a.re + b.re, a.im + b.im}, d = {a.re - b.re, a.im - b.im};
-                    v[base + j] = s;
-                    v[base + j + h] = Cpx{d.re * w.re - d.im * w.im, d.re * w.im + d.im * w.re};
-                }
-        }
-        bit_reverse_permute(v);
-        const double inv = 1.0 / (double)n;
-        for (Cpx &x : v) { x.re = x.re * inv; x.im = x.im * inv; }
-    }
-    void embed_forward(std::vector<Cpx> &v) const {
-        const size_t n = v.size(); const u64 M = (u64)2 * N;
-        bit_reverse_permute(v);
-        for (size_t len = 2; len <= n; len <<= 1) {
-            const size_t h = len >> 1, quad = len << 2; const u64 stride = M / quad;
-            for (size_t base = 0; base < n; base += len)
-                for (size_t j = 0; j < h; ++j) {
-                    const Cpx w = unit[(orbit5[j] % quad) * stride];
-                    Cpx a = v[base + j], b = v[base + j + h];
-                    Cpx t = {b.re * w.re - b.im * w.im, b.re * w.im + b.im * w.re};
-                    v[base + j] = Cpx{a.re + t.re, a.im + t.im};
-                    v[base + j + h] = Cpx{a.re - t.re, a.im - t.im};
-                }
-        }
-    }
-    // message -> rounded integer coefficients at scale sc
-    void encode_coeffs(const double *re, const double *im, size_t n, double sc, std::vector<i64> &coef) const {
-        std::vector<Cpx> v((size_t)slots, Cpx{0.0, 0.0});
-        for (size_t i = 0; i < n; ++i) { v[i].re = re[i]; v[i].im = im ? im[i] : 0.0; }
-        embed_inverse(v);
-        coef.resize(N);
-        for (int i = 0; i < slots; ++i) {
-            coef[i] = (i64)std::rint(v[i].re * sc);
-            coef[i + slots] = (i64)std::rint(v[i].im * sc);
-        }
-    }
-    // centred coefficient values (as doubles) -> message
-    void decode_values(const std::vector<double> &val, double sc, double *re, double *im) const {
-        std::vector<Cpx> v((size_t)slots);
-        for (int i = 0; i < slots; ++i) { v[i].re = val[i] / sc; v[i].im = val[i + slots] / sc; }
-        embed_forward(v);
-        for (int i = 0; i < slots; ++i) { re[i] = v[i].re; if (im) im[i] = v[i].im; }
-    }
-    // residues of limb 0 (and 1) in coefficient form -> centred doubles
-    void centre(const u64 *c0, const u64 *c1, std::vector<double> &val) const {
-        val.resize(N);
-        if (!c1) {
-            for (int i = 0; i < N; ++i) val[i] = c0[i] > q[0] / 2 ? -(double)(q[0] - c0[i]) : (double)c0[i];
-            return;
-        }
-        const u64 q0 = q[0], q1 = q[1], q0inv = invmod(q0 % q1, q1);
-        const u128 Q = (u128)q0 * q1;
-        for (int i = 0; i < N; ++i) {
-            u64 r0 = c0[i], r1 = c1[i], r0m = r0 % q1;
-            u64 diff = r1 >= r0m ? r1 - r0m : r1 + q1 - r0m;
-            u128 x = (u128)r0 + (u128)q0 * mulmod(diff, q0inv, q1);
-            val[i] = x > Q / 2 ? -(double)(__int128)(Q - x) : (double)(__int128)x;
+    // Twiddles of the embedding for butterflies of distance h, position j < h, at [h + j]: the transform itself runs on the device
+    // (embed.cuh).  Encoding multiplies by exp(-2 pi i 5^j / 8h), decoding by exp(+2 pi i 5^j / 8h).
+    void embed_twiddles(std::vector<Cpx> &inv, std::vector<Cpx> &fwd) const {
+        const u64 M = (u64)2 * N;
+        inv.assign(slots, Cpx{0.0, 0.0}); fwd = inv;
+        for (size_t h = 1; h < (size_t)slots; h <<= 1) {
+            const u64 quad = 8 * h, stride = M / quad;
+            for (size_t j = 0; j < h; ++j) {
+                inv[h + j] = unit[(quad - orbit5[j] % quad) * stride];
+                fwd[h + j] = unit[(orbit5[j] % quad) * stride];
+            }
         }
     }
 
-    // ----- host samplers (sequential, small) -----
+    // ----- the secret: rejection sampling, sequential -----
     void sample_secret(std::vector<i64> &s) const {
         s.assign(N, 0);
         HostChaCha::Reader rd(&cha, STREAM_SK, 0);
@@ -299,17 +235,6 @@ struct HostCtx {
             size_t pos = (size_t)(r & (u64)(N - 1));
             if (s[pos]) continue;
             s[pos] = (r >> 63) ? -1 : 1; ++placed;
-        }
-    }
-    void sample_gauss(u32 domain, u64 id, std::vector<i64> &e) const {
-        e.resize(N);
-        HostChaCha::Reader rd(&cha, domain, id);
-        for (int c = 0; c < N; ++c) {
-            // magnitude = number of table entries <= u; the table is increasing, so stop at the first larger one
-            u64 r = rd.next(), u = r >> 1; i64 mag = 0;
-            const size_t J = gauss_cdt.size();
-            while ((size_t)mag < J && gauss_cdt[(size_t)mag] <= u) ++mag;
-            e[c] = (r & 1) ? -mag : mag;
         }
     }
 };

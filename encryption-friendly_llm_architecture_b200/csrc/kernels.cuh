@@ -1,4 +1,4 @@
-// Element-wise, base-conversion, automorphism, sampling and accumulate kernels (sm_100a).
+// Element-wise, base-conversion, automorphism and accumulate kernels (sm_100a).
 // Arrays are dense [instances][N] uint64 unless a stride is named; instance li uses prime
 // map.prime[li % map.n].  One thread handles one coefficient of one limb instance; a warp
 // touches 256 contiguous bytes per array, so every stream is fully coalesced.  Gathers through
@@ -157,18 +157,6 @@ __global__ void k_permute(u64 *__restrict__ out, const u64 *__restrict__ in, u32
         const int i = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
         if (i >= N) break;
         out[(size_t)li * N + i] = in[(size_t)li * N + ntt_perm((u32)i, g, logn)];
-    }
-}
-// int64 coefficients -> residues of every limb instance (coefficient form)
-__global__ void k_reduce_i64(u64 *__restrict__ out, const i64 *__restrict__ coef, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N) {
-    const int li = blockIdx.y;
-#pragma unroll
-    for (int u_ = 0; u_ < kElems; ++u_) {
-        const int i = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
-        if (i >= N) break;
-        const PrimeConst m = pc[map.prime[li % map.n]];
-        const size_t off = (size_t)li * N + i;
-        out[off] = reduce_i64(coef[i], m);
     }
 }
 // x mod q for lazily summed residues
@@ -1288,94 +1276,6 @@ __global__ void k_div_fin(u64 *__restrict__ out, const u64 *__restrict__ E, cons
         if (i >= N) break;
         const u64 v = sub_mod(E[((size_t)bp * ne + l) * N + i], t[((size_t)bp * nl + l) * N + i], m.q);
         out[((size_t)bp * nl + l) * N + i] = mul_mod_any(v, dinv, m);
-    }
-}
-
-// ---------------- ChaCha20 ----------------
-__device__ __forceinline__ u32 rotl32(u32 v, int c) { return __funnelshift_l(v, v, c); }
-#define HB_QR(a, b, c, d)                                   \
-    a += b; d ^= a; d = rotl32(d, 16); c += d; b ^= c; b = rotl32(b, 12); \
-    a += b; d ^= a; d = rotl32(d, 8);  c += d; b ^= c; b = rotl32(b, 7);
-struct ChaChaKey { u32 k[8]; };
-__device__ __forceinline__ void chacha_block(const ChaChaKey &key, u32 domain, u64 id, u32 counter, u32 (&o)[16]) {
-    u32 in[16] = {0x61707865u, 0x3320646eu, 0x79622d32u, 0x6b206574u, key.k[0], key.k[1], key.k[2], key.k[3], key.k[4], key.k[5], key.k[6], key.k[7],
-                  counter, domain, (u32)id, (u32)(id >> 32)};
-    u32 x0 = in[0], x1 = in[1], x2 = in[2], x3 = in[3], x4 = in[4], x5 = in[5], x6 = in[6], x7 = in[7];
-    u32 x8 = in[8], x9 = in[9], x10 = in[10], x11 = in[11], x12 = in[12], x13 = in[13], x14 = in[14], x15 = in[15];
-#pragma unroll
-    for (int r = 0; r < 10; ++r) {
-        HB_QR(x0, x4, x8, x12) HB_QR(x1, x5, x9, x13) HB_QR(x2, x6, x10, x14) HB_QR(x3, x7, x11, x15)
-        HB_QR(x0, x5, x10, x15) HB_QR(x1, x6, x11, x12) HB_QR(x2, x7, x8, x13) HB_QR(x3, x4, x9, x14)
-    }
-    o[0] = x0 + in[0]; o[1] = x1 + in[1]; o[2] = x2 + in[2]; o[3] = x3 + in[3]; o[4] = x4 + in[4]; o[5] = x5 + in[5]; o[6] = x6 + in[6]; o[7] = x7 + in[7];
-    o[8] = x8 + in[8]; o[9] = x9 + in[9]; o[10] = x10 + in[10]; o[11] = x11 + in[11]; o[12] = x12 + in[12]; o[13] = x13 + in[13]; o[14] = x14 + in[14]; o[15] = x15 + in[15];
-}
-// uniform residues: limb instance li (prime pi = map.prime[li]) coefficient c = (128-bit word (pi*N + c) of the stream) mod q.
-// One thread produces the four coefficients of one ChaCha block.  grid = (N/4/256, count)
-__global__ void k_uniform(u64 *__restrict__ out, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int N, ChaChaKey key, u32 domain, u64 id) {
-    const int li = blockIdx.y;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t * 4 >= N) return;
-    const int pi = map.prime[li % map.n];
-    const PrimeConst m = pc[pi];
-    u32 o[16];
-    chacha_block(key, domain, id, (u32)(((u64)pi * N + (u64)t * 4) >> 2), o);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        u64 lo = (u64)o[4 * k] | ((u64)o[4 * k + 1] << 32), hi = (u64)o[4 * k + 2] | ((u64)o[4 * k + 3] << 32);
-        out[(size_t)li * N + t * 4 + k] = barrett128(hi, lo, m);
-    }
-}
-
-// ---------------- encrypt / decrypt / key generation ----------------
-// b = e - a*s + msg   (all NTT form).  grid.y = n limbs
-__global__ void k_encrypt(u64 *__restrict__ b, const u64 *__restrict__ a, const u64 *__restrict__ e, const u64 *__restrict__ s, const u64 *__restrict__ msg, const __grid_constant__ LimbMap map,
-                          const PrimeConst *__restrict__ pc, int N) {
-    const int li = blockIdx.y;
-#pragma unroll
-    for (int u_ = 0; u_ < kElems; ++u_) {
-        const int i = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
-        if (i >= N) break;
-        const PrimeConst m = pc[map.prime[li % map.n]];
-        const size_t off = (size_t)li * N + i;
-        const size_t so = (size_t)map.prime[li % map.n] * N + i;
-        u64 v = sub_mod(e[off], mul_mod(a[off], s[so], m), m.q);
-        b[off] = add_mod(v, msg[off], m.q);
-    }
-}
-// out[l] = b + a*s (+ d2*s^2) for limbs l < nl of entry `index`
-__global__ void k_decrypt(u64 *__restrict__ out, const u64 *__restrict__ ct, int n, int np, const u64 *__restrict__ s, const PrimeConst *__restrict__ pc, int N) {
-    const int l = blockIdx.y;
-#pragma unroll
-    for (int u_ = 0; u_ < kElems; ++u_) {
-        const int i = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
-        if (i >= N) break;
-        const PrimeConst m = pc[l];
-        const u64 sv = s[(size_t)l * N + i];
-        u64 v = add_mod(ct[(size_t)l * N + i], mul_mod(ct[((size_t)n + l) * N + i], sv, m), m.q);
-        if (np == 3) v = add_mod(v, mul_mod(ct[((size_t)2 * n + l) * N + i], mul_mod(sv, sv, m), m), m.q);
-        out[(size_t)l * N + i] = v;
-    }
-}
-// switching-key body: b = e - a*s + [prime in digit] * (P mod q) * s',  s' = s^2 (g == 0) or s o perm_g.
-// grid.y = nprimes; one digit per launch.
-__global__ void k_keygen(u64 *__restrict__ b, const u64 *__restrict__ a, const u64 *__restrict__ e, const u64 *__restrict__ s, const PrimeConst *__restrict__ pc, int N,
-                         int logn, u32 g, int dig_lo, int dig_hi, const __grid_constant__ Scalars pmod) {
-    const int pi = blockIdx.y;
-#pragma unroll
-    for (int u_ = 0; u_ < kElems; ++u_) {
-        const int i = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
-        if (i >= N) break;
-        const PrimeConst m = pc[pi];
-        const size_t off = (size_t)pi * N + i;
-        u64 v = sub_mod(e[off], mul_mod(a[off], s[off], m), m.q);
-        if (pi >= dig_lo && pi < dig_hi) {
-            u64 sp;
-            if (g == 0) sp = mul_mod(s[off], s[off], m);
-            else sp = s[(size_t)pi * N + ntt_perm((u32)i, g, logn)];
-            v = add_mod(v, mul_mod(sp, pmod.v[pi], m), m.q);
-        }
-        b[off] = v;
     }
 }
 

@@ -243,7 +243,7 @@ class LayerWorkload:
     def _encrypt_all(self, nonce0):
         """Encode + encrypt every operand of this rank's units, one batched call per group of operands."""
         H, lib = self.H, self.lib
-        per_ct = 2 * lib.N * 8  # rounded message coefficients + error polynomial uploaded per encryption
+        per_ct = lib.slots * 8  # the slot values of a real message
         groups = {"full": [], "half": []}      # pcmm: (unit index, [(pair, nonce)])
         ccmm = {False: [], True: [], "left": []}
         for i in self.mine:
@@ -399,7 +399,7 @@ class LayerWorkload:
     def _decrypt_all(self, out, check=False):
         """Decrypt every result this rank holds to host matrices (one batched call); returns the max-abs error when `check`."""
         err = 0.0
-        per = 2 * self.lib.N * 8
+        per = self.lib.slots * 16  # complex slot values
         held = self.held_outputs(out)
         if not held:
             return err

@@ -101,17 +101,18 @@ int hb_encode_ext(hb_ctx *ctx, const double *re, const double *im, size_t n_slot
 /* Encryptor::encrypt(ptxt, sk, ctxt) -- Encryptor.hpp:84; `nonce` selects the random streams */
 int hb_encrypt(hb_ctx *ctx, const hb_pt *pt, uint64_t nonce, hb_ct **out);
 /* encode + encrypt `count` messages (message i at re + i * n_slots, im likewise or NULL) into ONE handle of batch
- * `count`: the inverse embeddings and error polynomials are made on the host cores in parallel, uploaded in one
- * copy, and the device part runs over the whole batch.  Member i is bit for bit hb_encrypt(hb_encode(message i,
- * level), nonces[i]). */
+ * `count`: the messages are uploaded in chunks, everything from the inverse embedding and the error polynomials on is
+ * done by the device.  Member i is bit for bit hb_encrypt(hb_encode(message i, level), nonces[i]). */
 int hb_encrypt_many(hb_ctx *ctx, const double *re, const double *im, size_t n_slots, int count, int level, const uint64_t *nonces,
                     hb_ct **out);
 /* Decryptor::decrypt -- Decryptor.hpp:36; decrypts entry `index` of the batch */
 int hb_decrypt(hb_ctx *ctx, const hb_ct *ct, int index, double *re, double *im);
 /* the same for `count` ciphertexts at once (member index[i] of batch handle cts[i]; index may be NULL for all zero):
- * one device pass and one copy for all, the CRT lift and the inverse embedding spread over the host cores.
- * re / im receive count * slots doubles; each member's values are exactly those hb_decrypt gives. */
+ * decryption, CRT lift and embedding on the device, copies in chunks.  re / im receive count * slots doubles (im may be
+ * NULL); each member's values are exactly those hb_decrypt gives. */
 int hb_decrypt_many(hb_ctx *ctx, const hb_ct *const *cts, const int *index, int count, double *re, double *im);
+/* the same as complex values: slot s of item i at z[2 * (i * slots + s)] (real part) and the word after it */
+int hb_decrypt_many_complex(hb_ctx *ctx, const hb_ct *const *cts, const int *index, int count, double *z);
 
 /* Ciphertext construction / metadata / raw residues -- Ciphertext.hpp:83-131 */
 int hb_ct_create(hb_ctx *ctx, int level, int n_poly, int batch, int scale_pow, hb_ct **out);
@@ -295,7 +296,7 @@ int hb_send(hb_ctx *ctx, const hb_ct *a, int peer, void *nccl_comm);
 int hb_recv(hb_ctx *ctx, hb_ct *a, int peer, void *nccl_comm);
 int hb_sum_mod_reduce(hb_ctx *ctx, const hb_ct *const *parts, int count, hb_ct **out);
 
-/* Host threads used by the encode / decode halves of hb_encrypt_many / hb_decrypt_many (0: every core, at most 32).
+/* Host threads that move slot values between the caller's memory and the pinned buffers (0: up to four).
  * Several ranks on one host each take cores / ranks.  No counterpart in the reference (one process per GPU under mpirun). */
 int hb_set_host_threads(hb_ctx *ctx, int n);
 

@@ -1,0 +1,76 @@
+"""Encoding, sampling, encryption and decryption on the device against the oracle, whose embedding, error polynomials and CRT lift are
+host code with the same sequence of IEEE operations: residues and decoded values are compared bit for bit.  Members travel in chunks
+of eight through two buffers, so batches lie on both sides of one, two and three chunks."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _pair(request, size):
+    return request.getfixturevalue(f"gpu_{size}"), request.getfixturevalue(f"orc_{size}")
+
+
+def _messages(rng, count, slots, cplx):
+    z = rng.uniform(-1, 1, (count, slots))
+    return z + 1j * rng.uniform(-1, 1, (count, slots)) if cplx else z
+
+
+@pytest.mark.parametrize("size,level,count,slots,cplx", [
+    ("small", 0, 1, 1, False), ("small", 8, 9, 511, True), ("mid", 3, 17, 2048, True), ("mid", 1, 8, 0, False),
+    ("full", 12, 9, 32768, False), ("full", 0, 2, 32767, True), ("full", 1, 17, 129, True), ("full", 4, 8, 20000, False)])
+def test_encrypt_and_decrypt_equal_the_oracle(request, size, level, count, slots, cplx):
+    g, o = _pair(request, size)
+    msgs = _messages(np.random.default_rng(level * 100 + count), count, slots, cplx)
+    nonces = [2**63 + 5 * k for k in range(count)]
+    ct = g.encrypt_many(msgs, level, nonces)
+    got = g.ct_export(ct)
+    values = g.decrypt_many([(ct, k) for k in reversed(range(count))])[::-1]
+    for k in sorted({0, min(7, count - 1), min(8, count - 1), count - 1}):
+        ref = o.encrypt(o.encode(msgs[k], level), nonces[k])
+        assert np.array_equal(got[k:k + 1], o.ct_export(ref)), f"ciphertext {k}"
+        assert np.array_equal(values[k], o.decrypt(ref)), f"values {k}"
+        assert np.array_equal(values[k], g.decrypt(ct, k))
+
+
+@pytest.mark.parametrize("size", ["small", "full"])
+@pytest.mark.parametrize("scale", [1e-300, 2.0**-20, 2.0**20, 1e30])
+def test_rounding_at_the_ends_of_the_range(request, size, scale):
+    """Coefficients that vanish, that leave the 51 bits of the short reduction, and that do not fit 64 bits (which saturate as on the host)."""
+    g, o = _pair(request, size)
+    z = _messages(np.random.default_rng(3), 1, g.slots, True)[0] * scale
+    z[1] = -0.0
+    for level in (1, g.L):
+        assert np.array_equal(g.pt_export(g.encode(z, level)), o.pt_export(o.encode(z, level)))
+        p, q = g.encode(z, level), o.encode(z, level)
+        assert np.array_equal(g.decode(p), o.decode(q))
+
+
+def test_not_a_number_and_infinity_encode_as_on_the_host(gpu_small, orc_small):
+    z = np.zeros(gpu_small.slots)
+    for bad in (np.nan, np.inf, -np.inf):
+        z[3] = bad
+        assert np.array_equal(gpu_small.pt_export(gpu_small.encode(z, 2)), orc_small.pt_export(orc_small.encode(z, 2)))
+
+
+@pytest.mark.parametrize("size", ["small", "full"])
+def test_decoding_of_uniform_residues(request, size):
+    """Every value of the lift is met: both halves of q_0 and of q_0 q_1, one to three polynomials, one and two factors of the scale."""
+    from conftest import rand_ct_residues
+    g, o = _pair(request, size)
+    for level, polys, power in ((0, 2, 1), (1, 3, 2), (3, 2, 2)):
+        data = rand_ct_residues(g, level, polys, 1, seed=level + 7)
+        cts = []
+        for lib in (g, o):
+            ct = lib.ct_create(level, polys, 1, power)
+            lib.ct_import(ct, data)
+            cts.append(ct)
+        assert np.array_equal(g.decrypt(cts[0]), o.decrypt(cts[1])), (level, polys, power)
+
+
+@pytest.mark.parametrize("size", ["small", "full"])
+def test_switching_keys_equal_the_oracle(request, size):
+    g, o = _pair(request, size)
+    for galois in (0, g.galois(3)):
+        g.gen_rot_keys([3]); o.gen_rot_keys([3])
+        assert np.array_equal(g.evk_export(galois), o.evk_export(galois))
