@@ -163,6 +163,22 @@ class Lib:
         self._chk(self._fn("encrypt_many")(self.ctx, _f64(re), _f64(im), C.c_size_t(msgs.shape[1]), C.c_int(n), C.c_int(level), nn, C.byref(out)))
         return Handle(self, out, "ct")
 
+    def encrypt_tiles(self, groups, level, nonces):
+        """encrypt_many for messages given as lists of real tiles that lie side by side."""
+        tiles = [[np.ascontiguousarray(np.asarray(t).real, dtype=np.float64) for t in g] for g in groups]
+        rows, cols = tiles[0][0].shape
+        if not self.has("encrypt_tiles") or rows * cols == 0 or any(t.shape != (rows, cols) for g in tiles for t in g):
+            msgs = np.zeros((len(tiles), self.slots))
+            for m, g in zip(msgs, tiles):
+                np.concatenate(g, axis=1, out=m[: sum(t.size for t in g)].reshape(g[0].shape[0], sum(t.shape[1] for t in g)))
+            return self.encrypt_many(msgs, level, nonces)
+        n, across = len(tiles), len(tiles[0])
+        ptr = (C.c_void_p * (n * across))(*[t.ctypes.data for g in tiles for t in g])
+        nn = (C.c_uint64 * n)(*[int(k) for k in nonces])
+        out = C.c_void_p()
+        self._chk(self._fn("encrypt_tiles")(self.ctx, ptr, C.c_int(across), C.c_int(rows), C.c_int(cols), C.c_int(n), C.c_int(level), nn, C.byref(out)))
+        return Handle(self, out, "ct")
+
     def decrypt_many(self, items):
         """Decrypt a list of (ciphertext handle, batch index) pairs in one call; returns complex [len(items)][slots]."""
         n = len(items)

@@ -125,9 +125,9 @@ struct hb_ctx {
     InvScale p_inv_scale{};               // 2^16 rings: P^-1 mod q_l
     std::map<int, InvScale> div_scale;    // (P * q_level)^-1 mod q_l per level
     bool smem_opt_in_conv = false;
-    // slot values on their way between the caller's memory and the device: two pinned buffers, each with the event of its last copy
-    double *stage[2] = {nullptr, nullptr};
-    cudaEvent_t staged[2] = {nullptr, nullptr};
+    // slot values on their way between the caller's memory and the device: two pinned buffers a direction, with the events of their last copies
+    double *up[2] = {nullptr, nullptr}, *down[2] = {nullptr, nullptr};
+    cudaEvent_t went_up[2] = {nullptr, nullptr}, came_down[2] = {nullptr, nullptr};
     double2 *emb = nullptr;               // twiddles of the embedding, inverse then forward
     u64 *cdt = nullptr;                   // table of the discrete Gaussian
     EmbedTables emb_tb{};
@@ -963,25 +963,29 @@ u64 *noalloc_scratch(int device) {
 // the transforms of the other.  The caller's pages are often new ones, whose first touch costs more than the bytes: several threads.
 constexpr int kStageMembers = 8, kCopyThreads = 4;
 size_t stage_words(const hb_ctx *c) { return (size_t)kStageMembers * c->N; } // two doubles per slot
-void stage_open(hb_ctx *c) {
-    if (c->stage[0]) return;
-    for (int i = 0; i < 2; ++i) if (!c->staged[i]) CK(cudaEventCreateWithFlags(&c->staged[i], cudaEventDisableTiming));
+// Two buffers and their events.  Those of messages are write-combined: the host only writes them, and the copy engine need not ask its caches.
+void stage_open(hb_ctx *c, double *(&buf)[2], cudaEvent_t (&ev)[2], unsigned flags) {
+    if (buf[0]) return;
+    for (cudaEvent_t &e : ev) if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     double *p = nullptr;
-    CK(cudaMallocHost(&p, 2 * stage_words(c) * sizeof(double)));
-    c->stage[0] = p; c->stage[1] = p + stage_words(c);
+    CK(cudaHostAlloc(&p, 2 * stage_words(c) * sizeof(double), flags));
+    buf[0] = p; buf[1] = p + stage_words(c);
 }
-void host_copy(const hb_ctx *c, double *dst, const double *src, size_t words) {
+// work(begin, end) over [0, n) on up to kCopyThreads threads, `words` doubles moved in all
+template <class F> void in_threads(const hb_ctx *c, size_t n, size_t words, F &&work) {
     const size_t per = (size_t)1 << 16; // words that are worth a thread
     const int cap = c->host_threads > 0 ? std::min(c->host_threads, kCopyThreads) : kCopyThreads;
-    const int n = (int)std::max<size_t>(1, std::min<size_t>((size_t)cap, words / per));
-    const size_t step = (words + n - 1) / n;
-    auto part = [=](int t) { std::memcpy(dst + t * step, src + t * step, std::min(step, words - t * step) * sizeof(double)); };
+    const int k = (int)std::max<size_t>(1, std::min<size_t>({(size_t)cap, words / per, n}));
+    auto part = [&](int t) { work(n * t / k, n * (t + 1) / k); };
     std::thread pool[kCopyThreads];
     int started = 1;
-    try { for (; started < n; ++started) pool[started] = std::thread(part, started); } catch (const std::system_error &) {} // no more threads: the rest here
+    try { for (; started < k; ++started) pool[started] = std::thread(part, started); } catch (const std::system_error &) {} // no more threads: the rest here
     part(0);
-    for (int t = started; t < n; ++t) part(t);
+    for (int t = started; t < k; ++t) part(t);
     for (int t = 1; t < started; ++t) pool[t].join();
+}
+void host_copy(const hb_ctx *c, double *dst, const double *src, size_t words) {
+    in_threads(c, words, words, [&](size_t a, size_t b) { std::memcpy(dst + a, src + a, (b - a) * sizeof(double)); });
 }
 // coef [count][N] = rounded coefficients at scale sc of the messages re / im [count][n] on the device (im may be null)
 void embed_inverse(hb_ctx *c, i64 *coef, const double *re, const double *im, int n, int count, double sc) {
@@ -999,37 +1003,43 @@ void embed_forward(hb_ctx *c, double *re, double *im, int stride, const u64 *t, 
         launch(c, k_embed_fwd_cols, dim3(16, (unsigned)count), kEmbThreads, 0, re, im, stride, (const double2 *)v.p, c->emb_tb);
     } else launch(c, k_embed_fwd_small, dim3((unsigned)count), 256, 0, re, im, stride, t, items, c->logn - 1, c->centre, c->pc, c->emb_tb);
 }
-// Messages re / im [count][n] in host memory, chunk by chunk: use(first member, members, coefficients on the device, stream).  Every chunk's
-// values have left the caller's memory when this returns; the device may still be at work.
-template <class F> void encode_chunks(hb_ctx *c, const double *re, const double *im, size_t n, int count, double sc, F &&use) {
-    stage_open(c);
+// `count` messages of n slots, chunk by chunk: fill(first member, members, buffer) writes their real parts and, cplx, their imaginary parts
+// after all of those; use(first member, members, coefficients on the device) takes them on.  Nothing of the caller's memory is needed
+// once this has returned; the device may still be at work.
+template <class FILL, class USE> void encode_chunks(hb_ctx *c, size_t n, bool cplx, int count, double sc, FILL &&fill, USE &&use) {
+    stage_open(c, c->up, c->went_up, cudaHostAllocWriteCombined);
     for (int first = 0, slot = 0; first < count; first += kStageMembers, slot ^= 1) {
         const int m = std::min(kStageMembers, count - first);
-        const size_t words = (size_t)m * n;
-        CK(cudaEventSynchronize(c->staged[slot])); // its last copy has been made
-        double *h = c->stage[slot];
-        host_copy(c, h, re + (size_t)first * n, words);
-        if (im) host_copy(c, h + words, im + (size_t)first * n, words);
-        TmpBytes d(c, std::max<size_t>(1, words * (im ? 2 : 1)) * sizeof(double)), coef(c, (size_t)m * c->N * sizeof(i64));
+        const size_t words = (size_t)m * n, bytes = words * (cplx ? 2 : 1) * sizeof(double);
+        CK(cudaEventSynchronize(c->went_up[slot])); // its last copy has been made
+        fill(first, m, c->up[slot]);
+        TmpBytes d(c, std::max<size_t>(1, bytes)), coef(c, (size_t)m * c->N * sizeof(i64));
         double *dr = (double *)d.p;
-        CK(cudaMemcpyAsync(dr, h, words * (im ? 2 : 1) * sizeof(double), cudaMemcpyHostToDevice, c->st));
-        CK(cudaEventRecord(c->staged[slot], c->st));
-        embed_inverse(c, (i64 *)coef.p, dr, im ? dr + words : nullptr, (int)n, m, sc);
+        CK(cudaMemcpyAsync(dr, c->up[slot], bytes, cudaMemcpyHostToDevice, c->st));
+        CK(cudaEventRecord(c->went_up[slot], c->st));
+        embed_inverse(c, (i64 *)coef.p, dr, cplx ? dr + words : nullptr, (int)n, m, sc);
         use(first, m, (const i64 *)coef.p);
     }
+}
+// fill() for messages re / im [count][n]
+auto from_arrays(hb_ctx *c, const double *re, const double *im, size_t n) {
+    return [=](int first, int m, double *h) {
+        host_copy(c, h, re + (size_t)first * n, (size_t)m * n);
+        if (im) host_copy(c, h + (size_t)m * n, im + (size_t)first * n, (size_t)m * n);
+    };
 }
 // Decrypts and decodes `count` items into host memory: member i at re[i * slots], im likewise (im may be null); or, z, as complex values
 // at re[2 * i * slots].
 void decrypt_items(hb_ctx *c, const std::vector<DecItem> &items, bool z, double *re, double *im) {
-    stage_open(c);
+    stage_open(c, c->down, c->came_down, cudaHostAllocDefault);
     const int count = (int)items.size(), N = c->N, slots = N / 2;
     TmpBytes list(c, items.size() * sizeof(DecItem));
     CK(cudaMemcpyAsync(list.p, items.data(), items.size() * sizeof(DecItem), cudaMemcpyHostToDevice, c->st));
     auto collect = [&](int first, int slot) {
         const int m = std::min(kStageMembers, count - first);
         const size_t words = (size_t)m * slots;
-        CK(cudaEventSynchronize(c->staged[slot]));
-        const double *h = c->stage[slot];
+        CK(cudaEventSynchronize(c->came_down[slot]));
+        const double *h = c->down[slot];
         if (z) { host_copy(c, re + (size_t)first * N, h, 2 * words); return; }
         host_copy(c, re + (size_t)first * slots, h, words);
         if (im) host_copy(c, im + (size_t)first * slots, h + words, words);
@@ -1044,11 +1054,32 @@ void decrypt_items(hb_ctx *c, const std::vector<DecItem> &items, bool z, double 
         ntt_inplace(c, t.p, m * 2, c->qmap(1), true);
         double *d = (double *)v.p;
         embed_forward(c, d, z ? d + 1 : d + words, z ? 2 : 1, t.p, it, m);
-        CK(cudaMemcpyAsync(c->stage[slot], d, words * (z || im ? 2 : 1) * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-        CK(cudaEventRecord(c->staged[slot], c->st));
+        CK(cudaMemcpyAsync(c->down[slot], d, words * (z || im ? 2 : 1) * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaEventRecord(c->came_down[slot], c->st));
         if (first) collect(first - kStageMembers, slot ^ 1);
     }
     collect((count - 1) / kStageMembers * kStageMembers, slot ^ 1);
+}
+// encode + encrypt `count` messages into one batched handle; member i is bit for bit hb_encrypt(hb_encode(message i), nonces[i])
+template <class FILL> hb_ct *encrypt_messages(hb_ctx *c, size_t n_slots, bool cplx, int count, int level, const uint64_t *nonces, FILL &&fill) {
+    if (level < 0 || level > c->L) fail(HB_E_LEVEL, "encrypt_many: bad level");
+    const int n = level + 1, N = c->N;
+    hb_ct *r = new_ct(c, level, 2, count, 1);
+    try {
+        const LimbMap qm = c->qmap(level);
+        TmpBytes ids(c, (size_t)count * 8);
+        CK(cudaMemcpyAsync(ids.p, nonces, (size_t)count * 8, cudaMemcpyHostToDevice, c->st));
+        Tmp me(c, (size_t)std::min(count, kStageMembers) * n); // message + error; NTT form is linear, one transform serves both
+        encode_chunks(c, n_slots, cplx, count, c->h->scale[level], fill, [&](int first, int m, const i64 *coef) {
+            const u64 *id = (const u64 *)ids.p + first;
+            error_residues(c, me.p, coef, StreamIds{c->ckey, hbhost::STREAM_ENC_E, id, 0}, m, qm);
+            ntt_inplace(c, me.p, m * n, qm, false);
+            launch(c, k_encrypt, dim3((unsigned)((N / 4 + 255) / 256), (unsigned)n, (unsigned)m), 256, 0, r->d + (size_t)first * 2 * n * N, (const u64 *)me.p, (const u64 *)nullptr,
+                   (const u64 *)c->sk, StreamIds{c->ckey, hbhost::STREAM_ENC_A, id, 0}, c->pc, N);
+        });
+        CK(cudaStreamSynchronize(c->st)); // the nonces are the caller's memory
+    } catch (...) { hb_ct_free(r); throw; }
+    return r;
 }
 double scale_of(const hb_ctx *c, int level, int spow) { return spow == 2 ? c->h->scale[level] * c->h->scale[level] : c->h->scale[level]; }
 DecItem dec_item(const hb_ctx *c, const hb_ct *ct, int index) {
@@ -1184,8 +1215,8 @@ void hb_ctx_destroy(hb_ctx *c) {
     for (auto &kv : c->div_plans) cudaFree(kv.second);
     for (auto &kv : c->conv_plans) cudaFree(kv.second);
     for (auto &kv : c->gal_tables) cudaFree(kv.second);
-    if (c->stage[0]) cudaFreeHost(c->stage[0]);
-    for (cudaEvent_t e : c->staged) if (e) cudaEventDestroy(e);
+    for (double *p : {c->up[0], c->down[0]}) if (p) cudaFreeHost(p);
+    for (cudaEvent_t e : {c->went_up[0], c->went_up[1], c->came_down[0], c->came_down[1]}) if (e) cudaEventDestroy(e);
     if (c->emb) cudaFree(c->emb);
     if (c->cdt) cudaFree(c->cdt);
     if (c->pc) cudaFree(c->pc);
@@ -1282,7 +1313,7 @@ int hb_evk_export(hb_ctx *c, uint64_t g, uint64_t *host, int *digits) {
 
 static void encode_into(hb_ctx *c, hb_pt *p, const double *re, const double *im, size_t n, const LimbMap &map) {
     try {
-        encode_chunks(c, re, im, n, 1, c->h->scale[p->level], [&](int, int, const i64 *coef) { message_residues(c, p->d, coef, 1, map); });
+        encode_chunks(c, n, im != nullptr, 1, c->h->scale[p->level], from_arrays(c, re, im, n), [&](int, int, const i64 *coef) { message_residues(c, p->d, coef, 1, map); });
         ntt_inplace(c, p->d, map.n, map, false);
         CK(cudaStreamSynchronize(c->st));
     } catch (...) { hb_pt_free(p); throw; }
@@ -1336,30 +1367,29 @@ int hb_encrypt(hb_ctx *c, const hb_pt *p, uint64_t nonce, hb_ct **out) {
         *out = r;
     });
 }
-// encode + encrypt `count` messages into one batched handle; member i is bit for bit hb_encrypt(hb_encode(message i), nonces[i])
 int hb_encrypt_many(hb_ctx *c, const double *re, const double *im, size_t n_slots, int count, int level, const uint64_t *nonces, hb_ct **out) {
     return guard(c, [&] {
         no_capture(c, "encrypt_many");
         if (!c->have_sk) fail(HB_E_NOKEY, "secret key not generated");
         if (!re || !nonces || !out || count < 1 || n_slots > (size_t)c->h->slots) fail(HB_E_ARG, "encrypt_many: bad message");
-        if (level < 0 || level > c->L) fail(HB_E_LEVEL, "encrypt_many: bad level");
-        const int n = level + 1, N = c->N;
-        hb_ct *r = new_ct(c, level, 2, count, 1);
-        try {
-            const LimbMap qm = c->qmap(level);
-            TmpBytes ids(c, (size_t)count * 8);
-            CK(cudaMemcpyAsync(ids.p, nonces, (size_t)count * 8, cudaMemcpyHostToDevice, c->st));
-            Tmp me(c, (size_t)std::min(count, kStageMembers) * n); // message + error; NTT form is linear, one transform serves both
-            encode_chunks(c, re, im, n_slots, count, c->h->scale[level], [&](int first, int m, const i64 *coef) {
-                const u64 *id = (const u64 *)ids.p + first;
-                error_residues(c, me.p, coef, StreamIds{c->ckey, hbhost::STREAM_ENC_E, id, 0}, m, qm);
-                ntt_inplace(c, me.p, m * n, qm, false);
-                launch(c, k_encrypt, dim3((unsigned)((N / 4 + 255) / 256), (unsigned)n, (unsigned)m), 256, 0, r->d + (size_t)first * 2 * n * N, (const u64 *)me.p, (const u64 *)nullptr,
-                       (const u64 *)c->sk, StreamIds{c->ckey, hbhost::STREAM_ENC_A, id, 0}, c->pc, N);
+        *out = encrypt_messages(c, n_slots, im != nullptr, count, level, nonces, from_arrays(c, re, im, n_slots));
+    });
+}
+int hb_encrypt_tiles(hb_ctx *c, const double *const *tiles, int across, int rows, int cols, int count, int level, const uint64_t *nonces, hb_ct **out) {
+    return guard(c, [&] {
+        no_capture(c, "encrypt_tiles");
+        if (!c->have_sk) fail(HB_E_NOKEY, "secret key not generated");
+        if (!tiles || !nonces || !out || count < 1 || across < 1 || rows < 1 || cols < 1) fail(HB_E_ARG, "encrypt_tiles: nothing to encrypt");
+        const size_t slots = (size_t)c->h->slots, row = (size_t)across * (size_t)cols, n = row * (size_t)rows;
+        if (row > slots || n > slots) fail(HB_E_ARG, "encrypt_tiles: the tiles do not fit the slots");
+        for (size_t i = 0; i < (size_t)count * across; ++i) if (!tiles[i]) fail(HB_E_ARG, "encrypt_tiles: missing tile");
+        *out = encrypt_messages(c, n, false, count, level, nonces, [&](int first, int m, double *h) {
+            in_threads(c, (size_t)m * rows, (size_t)m * n, [&](size_t a, size_t b) {
+                for (size_t k = a; k < b; ++k)
+                    for (int t = 0; t < across; ++t)
+                        std::memcpy(h + k * row + (size_t)t * cols, tiles[((size_t)first + k / rows) * across + t] + (k % rows) * cols, (size_t)cols * sizeof(double));
             });
-            CK(cudaStreamSynchronize(c->st)); // the nonces are the caller's memory
-        } catch (...) { hb_ct_free(r); throw; }
-        *out = r;
+        });
     });
 }
 int hb_decrypt(hb_ctx *c, const hb_ct *ct, int index, double *re, double *im) {

@@ -168,12 +168,8 @@ class Hemmer:
 
     def encrypt2_many(self, pairs, nonces):
         """encrypt2 for a list of (left, right) tile pairs: one batched CtxtTensor, member i = encrypt2(*pairs[i], nonces[i])."""
-        msgs = np.zeros((len(pairs), self.lib.slots))
-        for m, (a, b) in zip(msgs, pairs):   # the layout of message2, written once
-            a, b = np.asarray(a).real, np.asarray(b).real
-            np.concatenate([a, b], axis=1, out=m[: a.size + b.size].reshape(a.shape[0], -1))
         d = pairs[0][0].shape
-        return CtxtTensor(self.lib.encrypt_many(msgs, self.lib.L, nonces), d[0], d[1], 2 * d[1])
+        return CtxtTensor(self.lib.encrypt_tiles(pairs, self.lib.L, nonces), d[0], d[1], 2 * d[1])
 
     def decrypt(self, t):
         fn = self._native("decrypt")

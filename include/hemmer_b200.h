@@ -105,6 +105,10 @@ int hb_encrypt(hb_ctx *ctx, const hb_pt *pt, uint64_t nonce, hb_ct **out);
  * done by the device.  Member i is bit for bit hb_encrypt(hb_encode(message i, level), nonces[i]). */
 int hb_encrypt_many(hb_ctx *ctx, const double *re, const double *im, size_t n_slots, int count, int level, const uint64_t *nonces,
                     hb_ct **out);
+/* the same for real messages that lie in memory as tiles: message i is the `across` row-major rows x cols tiles
+ * tiles[i * across ...] side by side (HEMMer::encrypt2 for across = 2) */
+int hb_encrypt_tiles(hb_ctx *ctx, const double *const *tiles, int across, int rows, int cols, int count, int level, const uint64_t *nonces,
+                     hb_ct **out);
 /* Decryptor::decrypt -- Decryptor.hpp:36; decrypts entry `index` of the batch */
 int hb_decrypt(hb_ctx *ctx, const hb_ct *ct, int index, double *re, double *im);
 /* the same for `count` ciphertexts at once (member index[i] of batch handle cts[i]; index may be NULL for all zero):

@@ -74,3 +74,25 @@ def test_switching_keys_equal_the_oracle(request, size):
     for galois in (0, g.galois(3)):
         g.gen_rot_keys([3]); o.gen_rot_keys([3])
         assert np.array_equal(g.evk_export(galois), o.evk_export(galois))
+
+
+@pytest.mark.parametrize("size,count,across,rows,cols", [("small", 1, 1, 1, 1), ("mid", 9, 2, 8, 4), ("full", 17, 2, 128, 128), ("full", 3, 3, 5, 7), ("full", 8, 1, 181, 181)])
+def test_tiles_side_by_side_equal_their_messages(request, size, count, across, rows, cols):
+    g = request.getfixturevalue(f"gpu_{size}")
+    rng = np.random.default_rng(count)
+    tiles = [[rng.uniform(-1, 1, (rows, cols)) for _ in range(across)] for _ in range(count)]
+    tiles[0][0] = np.asfortranarray(tiles[0][0])  # not in row-major order: copied first
+    msgs = np.stack([np.concatenate(t, axis=1).reshape(-1) for t in tiles])
+    nonces = list(range(50, 50 + count))
+    assert np.array_equal(g.ct_export(g.encrypt_tiles(tiles, 2, nonces)), g.ct_export(g.encrypt_many(msgs, 2, nonces)))
+
+
+def test_tiles_that_are_refused_or_take_the_general_path(pkg, gpu_small):
+    g = gpu_small
+    wide = np.ones((2, g.slots // 2 + 1))
+    for bad in ([[wide]], [[wide, wide]]):
+        with pytest.raises((pkg.HBError, ValueError)):
+            g.encrypt_tiles(bad, 2, [1])
+    a, b = np.ones((4, 3)), np.ones((4, 5))
+    assert np.array_equal(g.ct_export(g.encrypt_tiles([[a, b]], 2, [9])), g.ct_export(g.encrypt_many(np.ones((1, 32)), 2, [9])))
+    assert np.array_equal(g.ct_export(g.encrypt_tiles([[np.zeros((0, 4))]], 2, [9])), g.ct_export(g.encrypt_many(np.zeros((1, 4)), 2, [9])))
