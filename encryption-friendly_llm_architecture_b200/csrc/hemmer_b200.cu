@@ -816,21 +816,26 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
         if (!terms) fail(HB_E_ARG, "product sums: a part without terms");
     }
     const int l = a0->level, N = c->N, nbp = a0->batch * a0->np, gnbp = parts * nbp;
-    const unsigned gx1 = (unsigned)((N + 255) / 256);
     hb_ct *r = new_ct(c, l - 1, a0->np, parts * a0->batch, 1);
     ALG(c, (size_t)count * nbp * (l + 1) + used * (l + 1) + (size_t)gnbp * l);
     try {
         Tmp last(c, (size_t)gnbp * (separate ? count : 1)), t(c, (size_t)gnbp * l);
-        constexpr int G = 6; // parts per CTA: 6 x 17 mask chunks of 2 KB = 204 KB of shared memory
-        const size_t smem = (size_t)G * count * 2048;
+        constexpr int G = 6; // parts per CTA: more accumulators than that do not fit the registers
         const unsigned pg = (unsigned)((parts + G - 1) / G);
-        if (!c->smem_opt_in_parts) { CK(cudaFuncSetAttribute(k_prod_parts<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, G * kMaxPartTerms * 2048)); c->smem_opt_in_parts = true; }
+        if (!c->smem_opt_in_parts) { CK(cudaFuncSetAttribute(k_prod_parts<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)part_smem(G, kMaxPartTerms))); c->smem_opt_in_parts = true; }
         Scalars qi{};
         for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
+        // Up to ten polynomials the masks are streamed once per pair, beyond that they are kept.  A call with sixteen terms and twelve parts at
+        // level 7, us, streamed / kept: 4 polynomials 848 / 1305, 8 1536 / 1665, 10 1880 / 2039, 12 2223 / 2215.
+        auto sums = [&](u64 *o, const u64 *tt) {
+            const unsigned limbs = (unsigned)(tt ? l : 1);
+            if (nbp <= 10) LAUNCH(c), k_prod_parts_few<<<dim3((unsigned)(N / 256 * ((nbp + 1) / 2)), limbs), 256, 0, c->st>>>(o, pt, tt, l, nbp, c->pc, N, qi);
+            else LAUNCH(c), k_prod_parts<G><<<dim3(pg, (unsigned)(N / kPartLanes), limbs), 512, part_smem(G, count), c->st>>>(o, pt, tt, l, nbp, c->pc, N, qi, c->dev_err);
+        };
         if (separate) launch(c, k_last_prod_parts, dim3(c->gx(), nbp, parts * count), 256, 0, last.p, pt, l, nbp, c->pc, N);
-        else LAUNCH(c), k_prod_parts<G><<<dim3(gx1, 1, pg), 512, smem, c->st>>>(last.p, pt, nullptr, l, nbp, c->pc, N, qi, c->dev_err);
+        else sums(last.p, nullptr);
         lift_last(c, last.p, parts, separate ? count : 1, nbp, l, t.p);
-        LAUNCH(c), k_prod_parts<G><<<dim3(gx1, (unsigned)l, pg), 512, smem, c->st>>>(r->d, pt, t.p, l, nbp, c->pc, N, qi, c->dev_err);
+        sums(r->d, t.p);
         CK(cudaGetLastError());
     } catch (...) { hb_ct_free(r); throw; }
     return r;

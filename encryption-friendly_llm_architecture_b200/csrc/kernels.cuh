@@ -351,40 +351,67 @@ __global__ void k_last_prod_parts(u64 *last, const __grid_constant__ PartTerms p
         last[((size_t)blockIdx.z * nbp + bp) * N + x] = p ? mul_mod_any(pt.a[j][((size_t)bp * (level + 1) + level) * N + x], p[(size_t)level * N + x], m) : 0;
     }
 }
-// A CTA of 512 threads keeps the mask chunks of G parts for its 256 coefficients of one limb in shared memory (bulk
-// copies, up to G * 17 chunks of 2 KB, one mbarrier, bounded wait) and walks over the batch members, four at a time
-// (thread = coefficient + 256 * member pair): the masks cross L2 once per CTA instead of once per member and shared memory once per
-// two members, the a_j of a member are read by the ceil(parts / G) CTAs of the chunk (from L2 after the first), and every
-// thread has the next two a_j of both members in flight while it works on the current ones.  1024 threads with one member each and
-// 128-bit sums on the 60-bit limbs: 639 us a launch for one two-tile product, 2876 us in the layer pass; now 607 and 2859 us.
-// Bound by the latency of the a_j loads: sixteen warps per SM (128 registers, 16 bytes a thread spilled) with two loads ahead leave 60 % of
-// the issue slots empty, FP64 pipe 18 %, wide multiply-adds 38 %, DRAM 1.9 TB/s (sixteen terms, twelve parts, 48 polynomials, level 7).
-// t == nullptr: raw sums of limb `level`, out[(g * nbp + bp) * N + x]                       grid = (N/256, 1, ceil(parts/G))
-// else: out[((g * nbp + bp) * level + l) * N + x] = (sum - t[same]) * q_level^-1 mod q_l      grid = (N/256, level, ceil(parts/G))
+// A CTA of 512 threads keeps the mask chunks of G parts for its kPartLanes coefficients of one limb in shared memory (bulk copies, up to
+// G * 17 chunks of 1 KB, one mbarrier, bounded wait) and walks over the polynomials, eight at a time (thread = coefficient +
+// kPartLanes * pair of polynomials): the masks cross L2 once per CTA and shared memory once per two polynomials.  The words a_j, and the words of
+// t that a sum is subtracted from, come through a ring of kPartRing stages in shared memory that runs on across terms and polynomials, each
+// thread copying its own (cp.async, no barrier).  With two loads ahead in registers and t loaded when it was needed, 6.1 ms for 48
+// polynomials, sixteen terms, twelve parts at level 7 (both launches); with the ring for the a_j 5.5, with t in it as well and two terms per
+// turn of the loop (the sums change registers with every product, so a single one ends in moves) 4.1 ms.  Bound by instruction
+// issue now: 57 % of the slots with sixteen warps, FP64 40 % of the time on a short limb.
+// t == nullptr: raw sums of limb `level`, out[(g * nbp + bp) * N + x]                       grid = (ceil(parts/G), N/kPartLanes, 1)
+// else: out[((g * nbp + bp) * level + l) * N + x] = (sum - t[same]) * q_level^-1 mod q_l      grid = (ceil(parts/G), N/kPartLanes, level)
+// (parts first, so that the CTAs that read the same words run together)
+constexpr int kPartLanes = 128, kPartRing = 8;
+constexpr size_t part_smem(int g, int count) { return ((size_t)g * count * kPartLanes + (size_t)kPartRing * 2 * 512) * 8; }
 template <int G>
 __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, const __grid_constant__ PartTerms pt, const u64 *__restrict__ t, int level, int nbp,
                                                        const PrimeConst *__restrict__ pc, int N, const __grid_constant__ Scalars qlinv, int *__restrict__ err) {
+    constexpr int M = 2, kSlots = 512 / kPartLanes, kStage = M * 512; // members of a thread
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) u64 bar;
-    u64 *ptile = reinterpret_cast<u64 *>(smem_raw); // [G][count][256]
-    const int tid = threadIdx.x, lane = tid & 255, slot = tid >> 8;
-    const int l = t ? (int)blockIdx.y : level, g0 = blockIdx.z * G, count = pt.count;
+    const int count = pt.count;
+    const u64 *ring = reinterpret_cast<u64 *>(smem_raw) + threadIdx.x;   // [kPartRing][2][512]
+    u64 *ptile = reinterpret_cast<u64 *>(smem_raw) + kPartRing * kStage; // [count][G][kPartLanes]
+    const u32 ring_at = smem_u32(ring);
+    const int tid = threadIdx.x, lane = tid & (kPartLanes - 1), slot = tid / kPartLanes;
+    const int l = t ? (int)blockIdx.z : level, g0 = blockIdx.x * G;
     const int gn = min(G, pt.parts - g0);
-    const u32 x0 = blockIdx.x * 256;
+    const u32 x0 = blockIdx.y * kPartLanes;
     if (tid == 0) { mbar_init(&bar, 1); mbar_fence_init(); }
     __syncthreads();
     if (tid < 32) {
         if (tid == 0) {
             u32 present = 0;
             for (int ci = 0; ci < gn * count; ++ci) present += pt.p[g0 + ci / count][ci % count] != nullptr;
-            mbar_arrive_expect_tx(&bar, present * 2048u);
+            mbar_arrive_expect_tx(&bar, present * (kPartLanes * 8u));
         }
         __syncwarp();
         for (int ci = tid; ci < gn * count; ci += 32) {
             const u64 *src = pt.p[g0 + ci / count][ci % count];
-            if (src) bulk_load(ptile + (size_t)ci * 256, src + (size_t)l * N + x0, 2048u, &bar);
+            if (src) bulk_load(ptile + (size_t)((ci % count) * G + ci / count) * kPartLanes, src + (size_t)l * N + x0, kPartLanes * 8u, &bar);
         }
     }
+    // The words of this thread: members slot * M .., then kSlots * M further on; of each the terms a_j, then the words of t that its parts
+    // are subtracted from.
+    const size_t member = (size_t)(level + 1) * N, t_part = (size_t)nbp * level * N;
+    const size_t first = (size_t)l * N + x0 + lane;
+    const int words = count + (t ? gn : 0);
+    int fj = 0, fb = M * slot;
+    u32 to = 0; // byte offset of the stage that is filled next
+    auto fetch = [&] {
+        if (fb < nbp) {
+            const bool term = fj < count;
+            const u64 *p = term ? pt.a[fj] + first + (size_t)fb * member : t + first + (size_t)fb * level * N + (size_t)(g0 + fj - count) * t_part;
+            cp_async8(ring_at + to, p);
+            cp_async8(ring_at + to + 4096, fb + 1 < nbp ? p + (term ? member : (size_t)level * N) : p);
+            if (++fj == words) { fj = 0; fb += kSlots * M; }
+        }
+        cp_async_commit();
+        to = (to + kStage * 8) & (kPartRing * kStage * 8 - 1);
+    };
+#pragma unroll 1
+    for (int k = 0; k < kPartRing - 1; ++k) fetch();
     u32 have[G]; // bit j: part g0 + g has term j
 #pragma unroll
     for (int g = 0; g < G; ++g) {
@@ -400,74 +427,147 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
     // independent chains of the G parts interleave); the masks become doubles or pairs of pieces once.
 #pragma unroll
     for (int g = 0; g < G; ++g)
-        for (int j = slot; j < count; j += 2) {
-            u64 *w = ptile + (size_t)(g * count + j) * 256 + lane;
+        for (int j = slot; j < count; j += kSlots) {
+            u64 *w = ptile + (size_t)(j * G + g) * kPartLanes + lane;
             *w = ((have[g] >> j) & 1u) ? key_word(*w, m.fp) : 0;
         }
     __syncthreads();
-    const int room = m.fp && m.q < (1ull << 42) ? 128 : 8; // products between two reductions of a sum (FpAcc, PieceAcc)
-    for (int bp = 2 * slot; bp < nbp; bp += 4) {
-        const bool both = bp + 1 < nbp;
-        const size_t ao = ((size_t)bp * (level + 1) + l) * N + x0 + lane, ao1 = both ? ao + (size_t)(level + 1) * N : ao;
-        u64 v[2][G];
-        u64 cur[2] = {pt.a[0][ao], pt.a[0][ao1]}, nxt[2] = {0, 0};
-        if (count > 1) { nxt[0] = pt.a[1][ao]; nxt[1] = pt.a[1][ao1]; }
+    const bool eight = !(m.fp && m.q < (1ull << 42)); // at most eight products between two reductions of a sum, else 128 (FpAcc, PieceAcc)
+    int use = 0; // word offset of the stage that is read next
+    auto next = [&](u64 (&a)[M]) {
+        cp_async_wait<kPartRing - 2>();
+#pragma unroll
+        for (int i = 0; i < M; ++i) a[i] = ring[use + i * 512];
+        use = (use + kStage) & (kPartRing * kStage - 1);
+        fetch();
+    };
+    for (int bp = M * slot; bp < nbp; bp += kSlots * M) {
+        u64 v[M][G];
         auto terms = [&](auto &&product) {
-            for (int j = 0; j < count; ++j) {
-                const u64 a0 = cur[0], a1 = cur[1];
-                cur[0] = nxt[0]; cur[1] = nxt[1];
-                if (j + 2 < count) { nxt[0] = pt.a[j + 2][ao]; nxt[1] = pt.a[j + 2][ao1]; }
-                product(a0, a1, ptile + (size_t)j * 256 + lane, j && j % room == 0);
+            const u64 *w = ptile + lane;
+#pragma unroll 2
+            for (int j = 0; j < count; ++j, w += G * kPartLanes) {
+                u64 a[M];
+                next(a);
+                product(a, w, eight && j && j % 8 == 0);
             }
         };
         if (m.fp) { // products and sums exactly on the FP64 pipe
-            FpAcc s[2][G];
+            FpAcc s[M][G];
 #pragma unroll
-            for (int g = 0; g < G; ++g) { s[0][g].zero(); s[1][g].zero(); }
-            terms([&](u64 a0, u64 a1, const u64 *w, bool full) {
+            for (int i = 0; i < M; ++i)
+#pragma unroll
+                for (int g = 0; g < G; ++g) s[i][g].zero();
+            terms([&](const u64 (&a)[M], const u64 *w, bool full) {
                 if (full) {
 #pragma unroll
-                    for (int g = 0; g < G; ++g) { s[0][g].relax(m.q_inv_f, qd); s[1][g].relax(m.q_inv_f, qd); }
+                    for (int i = 0; i < M; ++i)
+#pragma unroll
+                        for (int g = 0; g < G; ++g) s[i][g].relax(m.q_inv_f, qd);
                 }
-                const double d0 = u52_to_double(a0), d1 = u52_to_double(a1);
+                double d[M];
+#pragma unroll
+                for (int i = 0; i < M; ++i) d[i] = u52_to_double(a[i]);
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
-                    const double k = __longlong_as_double((long long)w[(size_t)g * count * 256]);
-                    s[0][g].mac(d0, k); s[1][g].mac(d1, k);
+                    const double k = __longlong_as_double((long long)w[g * kPartLanes]);
+#pragma unroll
+                    for (int i = 0; i < M; ++i) s[i][g].mac(d[i], k);
                 }
             });
 #pragma unroll
-            for (int g = 0; g < G; ++g) { v[0][g] = s[0][g].finish(m.q_inv_f, qd); v[1][g] = s[1][g].finish(m.q_inv_f, qd); }
+            for (int i = 0; i < M; ++i)
+#pragma unroll
+                for (int g = 0; g < G; ++g) v[i][g] = s[i][g].finish(m.q_inv_f, qd);
         } else {
-            PieceAcc s[2][G];
+            PieceAcc s[M][G];
 #pragma unroll
-            for (int g = 0; g < G; ++g) { s[0][g].zero(); s[1][g].zero(); }
-            terms([&](u64 a0, u64 a1, const u64 *w, bool full) {
+            for (int i = 0; i < M; ++i)
+#pragma unroll
+                for (int g = 0; g < G; ++g) s[i][g].zero();
+            terms([&](const u64 (&a)[M], const u64 *w, bool full) {
                 if (full) {
 #pragma unroll
-                    for (int g = 0; g < G; ++g) { s[0][g].relax(m); s[1][g].relax(m); }
+                    for (int i = 0; i < M; ++i)
+#pragma unroll
+                        for (int g = 0; g < G; ++g) s[i][g].relax(m);
                 }
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
-                    const u64 k = w[(size_t)g * count * 256];
-                    s[0][g].mac((u32)a0 & 0x3FFFFFFFu, (u32)(a0 >> 30), (u32)k, (u32)(k >> 32));
-                    s[1][g].mac((u32)a1 & 0x3FFFFFFFu, (u32)(a1 >> 30), (u32)k, (u32)(k >> 32));
+                    const u64 k = w[g * kPartLanes];
+#pragma unroll
+                    for (int i = 0; i < M; ++i) s[i][g].mac((u32)a[i] & 0x3FFFFFFFu, (u32)(a[i] >> 30), (u32)k, (u32)(k >> 32));
                 }
             });
 #pragma unroll
-            for (int g = 0; g < G; ++g) { v[0][g] = s[0][g].finish(m); v[1][g] = s[1][g].finish(m); }
+            for (int i = 0; i < M; ++i)
+#pragma unroll
+                for (int g = 0; g < G; ++g) v[i][g] = s[i][g].finish(m);
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+            if (g < gn) {
+                u64 a[M];
+                if (t) next(a);
+#pragma unroll
+                for (int i = 0; i < M; ++i)
+                    if (bp + i < nbp) {
+                        if (t) out[(size_t)(g0 + g) * t_part + (size_t)(bp + i) * level * N + first] = mul_mod_any(sub_mod(v[i][g], a[i], m.q), qli, m);
+                        else out[((size_t)(g0 + g) * nbp + bp + i) * N + x0 + lane] = v[i][g];
+                    }
+            }
+    }
+}
+// The same for a few polynomials: the masks are then most of the bytes, so they are streamed instead of kept.  A thread holds the words a_j of
+// its coefficient in two polynomials and walks over the parts, with the masks of a part in flight together.  A launch for one two-tile
+// product 604 -> 215 us (2.5 TB/s of masks).  grid = (N/256 * pairs of polynomials, 1 or level), arguments as above
+__global__ void __launch_bounds__(256, 2) k_prod_parts_few(u64 *__restrict__ out, const __grid_constant__ PartTerms pt, const u64 *__restrict__ t, int level, int nbp, const PrimeConst *__restrict__ pc, int N,
+                                                           const __grid_constant__ Scalars qlinv) {
+    const int pairs = (nbp + 1) / 2, bp = blockIdx.x % pairs * 2; // the pairs that read the same masks run together
+    const int l = t ? (int)blockIdx.y : level, count = pt.count, x = blockIdx.x / pairs * 256 + threadIdx.x;
+    const bool both = bp + 1 < nbp;
+    const PrimeConst m = pc[l];
+    const u64 qli = t ? qlinv.v[l] : 0;
+    const double qd = (double)m.q;
+    const size_t po = (size_t)l * N + x, ao = po + (size_t)bp * (level + 1) * N, ao1 = both ? ao + (size_t)(level + 1) * N : ao;
+    u64 a[2][kMaxPartTerms];
+#pragma unroll
+    for (int j = 0; j < kMaxPartTerms; ++j) {
+        a[0][j] = j < count ? key_word(pt.a[j][ao], m.fp) : 0;
+        a[1][j] = j < count ? key_word(pt.a[j][ao1], m.fp) : 0;
+    }
+    const bool eight = !(m.fp && m.q < (1ull << 42));
+#pragma unroll 1
+    for (int g = 0; g < pt.parts; ++g) {
+        u64 w[kMaxPartTerms], v[2];
+#pragma unroll
+        for (int j = 0; j < kMaxPartTerms; ++j) w[j] = j < count && pt.p[g][j] ? pt.p[g][j][po] : 0;
+        if (m.fp) {
+            FpAcc s[2]; s[0].zero(); s[1].zero();
+#pragma unroll
+            for (int j = 0; j < kMaxPartTerms; ++j) {
+                if (j && j % 8 == 0 && eight) { s[0].relax(m.q_inv_f, qd); s[1].relax(m.q_inv_f, qd); }
+                const double k = u52_to_double(w[j]);
+                s[0].mac(__longlong_as_double((long long)a[0][j]), k); s[1].mac(__longlong_as_double((long long)a[1][j]), k);
+            }
+            v[0] = s[0].finish(m.q_inv_f, qd); v[1] = s[1].finish(m.q_inv_f, qd);
+        } else {
+            PieceAcc s[2]; s[0].zero(); s[1].zero();
+#pragma unroll
+            for (int j = 0; j < kMaxPartTerms; ++j) {
+                if (j && j % 8 == 0) { s[0].relax(m); s[1].relax(m); }
+                const u32 k0 = (u32)w[j] & 0x3FFFFFFFu, k1 = (u32)(w[j] >> 30);
+                s[0].mac((u32)a[0][j], (u32)(a[0][j] >> 32), k0, k1); s[1].mac((u32)a[1][j], (u32)(a[1][j] >> 32), k0, k1);
+            }
+            v[0] = s[0].finish(m); v[1] = s[1].finish(m);
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i)
             if (i == 0 || both) {
-#pragma unroll
-                for (int g = 0; g < G; ++g)
-                    if (g < gn) {
-                        if (t) {
-                            const size_t w = (((size_t)(g0 + g) * nbp + bp + i) * level + l) * N + x0 + lane;
-                            out[w] = mul_mod_any(sub_mod(v[i][g], t[w], m.q), qli, m);
-                        } else out[((size_t)(g0 + g) * nbp + bp + i) * N + x0 + lane] = v[i][g];
-                    }
+                if (t) {
+                    const size_t o = (((size_t)g * nbp + bp + i) * level + l) * N + x;
+                    out[o] = mul_mod_any(sub_mod(v[i], t[o], m.q), qli, m);
+                } else out[((size_t)g * nbp + bp + i) * N + x] = v[i];
             }
     }
 }

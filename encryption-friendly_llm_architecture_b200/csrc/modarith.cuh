@@ -207,7 +207,7 @@ struct FpAcc {
 
 // ---- sums of products modulo the primes of 45 to 60 bits ---------------------------------------------------------
 // A full 64 x 64 -> 128-bit product with its carries costs about 34 cycles here.  For sums of a few products the operands are cut
-// into two pieces of 30 bits instead: a product is four 32 x 32 -> 64-bit multiply-adds into three carry-free accumulators (16
+// into two pieces of 30 bits instead: a product is three 32 x 32 -> 64-bit multiply-adds into three carry-free accumulators (12
 // cycles, 4 more per operand that is cut), and the sum  a0 + a1 * 2^30 + a2 * 2^60  is reduced once per output residue with
 // 2^60 = d60 modulo q (a 128-bit Barrett reduction takes 65 cycles).  Eight products fit the accumulators.
 __device__ __forceinline__ u64 mad_wide(u32 a, u32 b, u64 c) {
@@ -232,20 +232,22 @@ __device__ __forceinline__ u64 finish_wide(u64 a0, u64 a1, u64 a2, const PrimeCo
     lo += x; hi += (a2 >> 4) + (lo < x);
     return barrett128(hi, lo, m);
 }
+// Karatsuba: the middle products come from one product of the sums of the pieces, from which the outer two are taken off at the end (modulo
+// 2^64, which the true sum a1 does not reach): three multiply-adds and two 32-bit additions, of which the compiler makes one per factor.
 struct PieceAcc {
-    u64 a0, a1, a2; // weights 1, 2^30, 2^60
-    __device__ __forceinline__ void zero() { a0 = a1 = a2 = 0; }
+    u64 a0, am, a2; // weights 1 and 2^60 of the outer products; am = a0 + a1 + a2 modulo 2^64, a1 of weight 2^30
+    __device__ __forceinline__ void zero() { a0 = am = a2 = 0; }
     __device__ __forceinline__ void mac(u32 v0, u32 v1, u32 k0, u32 k1) { // 30-bit pieces of the factors
-        a0 = mad_wide(v0, k0, a0); a1 = mad_wide(v0, k1, a1); a1 = mad_wide(v1, k0, a1); a2 = mad_wide(v1, k1, a2);
+        a0 = mad_wide(v0, k0, a0); am = mad_wide(v0 + v1, k0 + k1, am); a2 = mad_wide(v1, k1, a2);
     }
     __device__ __forceinline__ void mac(u64 v, u64 k) { mac((u32)v & 0x3FFFFFFFu, (u32)(v >> 30), (u32)k & 0x3FFFFFFFu, (u32)(k >> 30)); } // v, k < 2^60
     // after at most eight products: makes room for eight more
     __device__ __forceinline__ void relax(const PrimeConst &m) {
-        const u64 r = finish_wide(a0, a1, a2, m);
-        a0 = r & 0x3FFFFFFFu; a1 = r >> 30; a2 = 0;
+        const u64 r = finish_wide(a0, am - a0 - a2, a2, m);
+        a0 = r & 0x3FFFFFFFu; am = a0 + (r >> 30); a2 = 0;
     }
     __device__ __forceinline__ u64 finish(const PrimeConst &m) const { // canonical
-        const u64 r = finish_wide(a0, a1, a2, m);
+        const u64 r = finish_wide(a0, am - a0 - a2, a2, m);
         return canon_q(r, m.q, FoldQ{m.fold_shift, (1u << m.fold_shift) - 1u, m.fold_d});
     }
 };

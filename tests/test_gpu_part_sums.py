@@ -1,6 +1,6 @@
 """Part sums of the baby-step / giant-step transforms and the plaintext products with shared copies at the edges of their kernels: one
-and two polynomials (masks streamed), more (masks kept, member pairs dealt to four slots, odd and missing pairs, several turns of the
-ring), one to seventeen terms and parts, absent terms, and primes of 42 and 44 bits (128 and 8 products between two reductions).
+to ten polynomials (masks streamed for pairs of them), more (masks kept, pairs dealt to four slots, odd and missing pairs, several turns of
+the ring), one to seventeen terms and parts, absent terms, and primes of 42 and 44 bits (128 and 8 products between two reductions).
 Residues are whole numbers: every comparison is exact."""
 import ctypes as C
 
@@ -34,7 +34,7 @@ def _ptrs(handles):
     return (C.c_void_p * len(handles))(*[h.ptr.value if h else None for h in handles])
 
 
-@pytest.mark.parametrize("terms,parts,polys,batch", [(1, 1, 1, 1), (17, 17, 2, 1), (9, 2, 1, 2), (8, 6, 3, 1), (17, 7, 2, 2), (16, 5, 1, 5), (2, 13, 2, 4), (17, 12, 3, 3), (3, 6, 2, 9), (10, 1, 1, 17)])
+@pytest.mark.parametrize("terms,parts,polys,batch", [(1, 1, 1, 1), (17, 17, 2, 1), (9, 2, 1, 2), (8, 6, 3, 1), (17, 7, 2, 2), (16, 5, 1, 5), (2, 13, 2, 4), (17, 12, 3, 3), (3, 6, 2, 9), (10, 1, 1, 17), (17, 17, 1, 11), (16, 16, 2, 6), (1, 1, 3, 4), (9, 13, 1, 13)])
 @pytest.mark.parametrize("top", [False, True])
 def test_part_sums_equal_their_sums_one_by_one(pkg, g, terms, parts, polys, batch, top):
     rng = np.random.default_rng(terms * 100 + parts)
