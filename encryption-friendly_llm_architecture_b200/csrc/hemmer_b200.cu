@@ -124,7 +124,7 @@ struct hb_ctx {
     std::map<int, ConvPlan *> conv_plans; // 2^16 rings, per level: one per key-switch digit, then ModDown, then the division by P * q_level (level >= 1)
     InvScale p_inv_scale{};               // 2^16 rings: P^-1 mod q_l
     std::map<int, InvScale> div_scale;    // (P * q_level)^-1 mod q_l per level
-    bool smem_opt_in_conv = false;
+    bool smem_opt_in_conv = false, smem_opt_in_acc = false;
     // slot values on their way between the caller's memory and the device: two pinned buffers a direction, with the events of their last copies
     double *up[2] = {nullptr, nullptr}, *down[2] = {nullptr, nullptr};
     cudaEvent_t went_up[2] = {nullptr, nullptr}, came_down[2] = {nullptr, nullptr};
@@ -840,6 +840,12 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
     } catch (...) { hb_ct_free(r); throw; }
     return r;
 }
+void acc_opt_in(hb_ctx *c) {
+    if (c->smem_opt_in_acc) return;
+    auto allow = [](auto *kernel, size_t bytes) { CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); };
+    allow(k_matmul_acc<1>, acc_smem(1)); allow(k_matmul_acc<2>, acc_smem(2)); allow(k_matmul_acc<3>, acc_smem(3)); allow(k_matmul_acc<4>, acc_smem(4));
+    c->smem_opt_in_acc = true;
+}
 template <int T>
 void launch_matmul_tiles(hb_ctx *c, const hb_ct *pre, int btotal, int b0, const hb_pt *const *pts, int bcount, int kc, const u32 *dg, hb_ct *const *outs) {
     TilePts<T> tp{};
@@ -848,8 +854,8 @@ void launch_matmul_tiles(hb_ctx *c, const hb_ct *pre, int btotal, int b0, const 
         tp.out[t] = outs[t]->d;
     }
     const int n = pre->level + 1;
-    constexpr int E = T >= 3 ? 1 : 2;
-    LAUNCH(c), k_matmul_acc<T, E><<<dim3((unsigned)(c->N / (256 * E)), (unsigned)n), 256, 0, c->st>>>(tp, pre->d, kc, btotal, b0, bcount, dg, n, c->qmap(pre->level), c->pc, c->logn, c->N);
+    acc_opt_in(c);
+    LAUNCH(c), k_matmul_acc<T><<<dim3((unsigned)(c->N / 256), (unsigned)n), 256, acc_smem(T), c->st>>>(tp, pre->d, kc, btotal, b0, bcount, dg, n, c->qmap(pre->level), c->pc, c->logn, c->N);
 }
 hb_ct *do_level_down(hb_ctx *c, const hb_ct *a, int target) {
     own(c, a);

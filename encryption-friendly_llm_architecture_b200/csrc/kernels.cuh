@@ -1382,104 +1382,108 @@ __global__ void k_div_fin(u64 *__restrict__ out, const u64 *__restrict__ E, cons
 // ---------------- fused plaintext-matmul accumulate ----------------
 // out_t[p][l][i] = sum_{b < bcount} sum_{k < kcount} pre[k * btotal + b0 + b][p][l][i] * pt_tb[l][perm_{g_k}(i)]
 // (scale Delta^2, no rescale) for T output tiles t that share the shifted copies, which are stored k-major; the sum over b adds the
-// partial products of several K-groups in the same pass.  A thread works on E coefficients of both polynomials: a copy word is
-// read once for T tiles and a weight word once (and converted or cut once) for two polynomials.  Four tiles a launch in the layer
-// pass: one polynomial per thread with every product reduced 840 us, this 675 us.  Bound by the latency of its loads: 16 warps
-// per SM (128 registers, of which two and four tiles spill 8 to 16 bytes) issue in 45 % of the slots, DRAM 2.1 TB/s, FP64 pipe 23 %.  grid = (N/(256*E), n)
+// partial products of several K-groups in the same pass.  A thread works on one coefficient of both polynomials: a copy word is
+// read once for T tiles and a weight word once (and converted or cut once) for two polynomials.  Both come through a ring of kAccRing stages
+// in shared memory that every thread fills for itself (cp.async), so a dozen loads of each of its 16 warps per SM are in flight without
+// registers for them; two terms a turn, because the sums change registers with every product.  Four tiles, two polynomials from
+// registers with one or two terms ahead: 675 us a launch in the layer pass, 611 in the Q/K/V projections; now 398 and 324.
+// grid = (N/256, n)
 template <int T> struct TilePts { const u64 *p[T][16]; u64 *out[T]; };
-template <int T, int E>
+constexpr int kAccRing = 8;
+constexpr size_t acc_smem(int T) { return (size_t)kAccRing * (2 + T) * 256 * 8; }
+template <int T>
 __global__ void __launch_bounds__(256, 2) k_matmul_acc(const __grid_constant__ TilePts<T> tp, const u64 *__restrict__ pre, int kcount, int btotal, int b0, int bcount, const u32 *__restrict__ gal,
                                                        int n, const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, int logn, int N) {
+    extern __shared__ __align__(16) u64 words[]; // [kAccRing][2 + T][256]
+    constexpr int kStage = (2 + T) * 256;
     const int l = blockIdx.y;
     const PrimeConst m = pc[map.prime[l]];
     const size_t poly = (size_t)n * N, limb = (size_t)l * N;
-    const u32 x0 = blockIdx.x * (256 * E) + threadIdx.x;
-    u64 r[T][2][E];
+    const u32 x0 = blockIdx.x * 256 + threadIdx.x;
+    const u64 *ring = words + threadIdx.x;
+    const u32 ring_at = smem_u32(ring);
+    // what is fetched next: copy k of input b, and the weights' words that meet it
+    int fk = 0, fb = 0, to = 0;
+    u32 src = 0;
+    const u64 *fa = pre + (size_t)b0 * 2 * poly + limb + x0;
+    auto fetch = [&] {
+        if (fk < kcount) {
+            if (fb == 0) { const u32 g = __ldg(gal + fk); src = g == 1 ? x0 : ntt_perm(x0, g, logn); }
+            const u32 r = ring_at + to * (kStage * 8);
+            const u64 *a = fa + (size_t)fb * 2 * poly;
+            cp_async8(r, a); cp_async8(r + 2048, a + poly);
+#pragma unroll
+            for (int t = 0; t < T; ++t) cp_async8(r + (2 + t) * 2048, tp.p[t][fb] + limb + src);
+            if (++fb == bcount) { fb = 0; ++fk; fa += (size_t)btotal * 2 * poly; }
+        }
+        cp_async_commit();
+        to = (to + 1) % kAccRing;
+    };
+#pragma unroll 1
+    for (int k = 0; k < kAccRing - 1; ++k) fetch();
+    u64 r[T][2];
     auto terms = [&](auto &&product) {
-        for (int k = 0; k < kcount; ++k) {
-            const u32 g = __ldg(gal + k);
-            u32 src[E];
-#pragma unroll
-            for (int u = 0; u < E; ++u) src[u] = g == 1 ? x0 + u * 256 : ntt_perm(x0 + u * 256, g, logn);
-            const u64 *a = pre + ((size_t)k * btotal + b0) * 2 * poly + limb + x0;
+        const int total = kcount * bcount;
+        int from = 0;
 #pragma unroll 2
-            for (int b = 0; b < bcount; ++b, a += 2 * poly) {
-                u64 v[2][E], w[T][E];
+        for (int k = 0; k < total; ++k) {
+            cp_async_wait<kAccRing - 2>();
+            const u64 *q = ring + from * kStage;
+            u64 v[2] = {q[0], q[256]}, w[T];
 #pragma unroll
-                for (int u = 0; u < E; ++u) {
-                    v[0][u] = a[u * 256]; v[1][u] = a[poly + u * 256];
-#pragma unroll
-                    for (int t = 0; t < T; ++t) w[t][u] = (tp.p[t][b] + limb)[src[u]];
-                }
-                product(v, w);
-            }
+            for (int t = 0; t < T; ++t) w[t] = q[(2 + t) * 256];
+            from = (from + 1) % kAccRing;
+            fetch();
+            product(v, w);
         }
     };
     if (m.fp) { // exact sums (see FpAcc): 128 products of primes below 2^42, eight below 2^44, before they are reduced
         const double qd = (double)m.q;
         const int room = m.q < (1ull << 42) ? 128 : 8;
-        FpAcc s[T][2][E];
+        FpAcc s[T][2];
         int held = 0;
 #pragma unroll
-        for (int t = 0; t < T; ++t)
-#pragma unroll
-            for (int u = 0; u < E; ++u) { s[t][0][u].zero(); s[t][1][u].zero(); }
-        terms([&](const u64 (&v)[2][E], const u64 (&w)[T][E]) {
+        for (int t = 0; t < T; ++t) { s[t][0].zero(); s[t][1].zero(); }
+        terms([&](const u64 (&v)[2], const u64 (&w)[T]) {
             if (++held > room) {
                 held = 1;
 #pragma unroll
-                for (int t = 0; t < T; ++t)
-#pragma unroll
-                    for (int u = 0; u < E; ++u) { s[t][0][u].relax(m.q_inv_f, qd); s[t][1][u].relax(m.q_inv_f, qd); }
+                for (int t = 0; t < T; ++t) { s[t][0].relax(m.q_inv_f, qd); s[t][1].relax(m.q_inv_f, qd); }
             }
+            const double v0 = u52_to_double(v[0]), v1 = u52_to_double(v[1]);
 #pragma unroll
-            for (int u = 0; u < E; ++u) {
-                const double v0 = u52_to_double(v[0][u]), v1 = u52_to_double(v[1][u]);
-#pragma unroll
-                for (int t = 0; t < T; ++t) {
-                    const double wd = u52_to_double(w[t][u]);
-                    s[t][0][u].mac(v0, wd);
-                    s[t][1][u].mac(v1, wd);
-                }
+            for (int t = 0; t < T; ++t) {
+                const double wd = u52_to_double(w[t]);
+                s[t][0].mac(v0, wd);
+                s[t][1].mac(v1, wd);
             }
         });
 #pragma unroll
-        for (int t = 0; t < T; ++t)
-#pragma unroll
-            for (int u = 0; u < E; ++u) { r[t][0][u] = s[t][0][u].finish(m.q_inv_f, qd); r[t][1][u] = s[t][1][u].finish(m.q_inv_f, qd); }
+        for (int t = 0; t < T; ++t) { r[t][0] = s[t][0].finish(m.q_inv_f, qd); r[t][1] = s[t][1].finish(m.q_inv_f, qd); }
     } else {
-        PieceAcc s[T][2][E];
+        PieceAcc s[T][2];
         int held = 0; // products in the accumulators
 #pragma unroll
-        for (int t = 0; t < T; ++t)
-#pragma unroll
-            for (int u = 0; u < E; ++u) { s[t][0][u].zero(); s[t][1][u].zero(); }
-        terms([&](const u64 (&v)[2][E], const u64 (&w)[T][E]) {
+        for (int t = 0; t < T; ++t) { s[t][0].zero(); s[t][1].zero(); }
+        terms([&](const u64 (&v)[2], const u64 (&w)[T]) {
             if (++held > 8) {
                 held = 1;
 #pragma unroll
-                for (int t = 0; t < T; ++t)
-#pragma unroll
-                    for (int u = 0; u < E; ++u) { s[t][0][u].relax(m); s[t][1][u].relax(m); }
+                for (int t = 0; t < T; ++t) { s[t][0].relax(m); s[t][1].relax(m); }
             }
 #pragma unroll
-            for (int u = 0; u < E; ++u)
-#pragma unroll
-                for (int t = 0; t < T; ++t) {
-                    s[t][0][u].mac(v[0][u], w[t][u]);
-                    s[t][1][u].mac(v[1][u], w[t][u]);
-                }
+            for (int t = 0; t < T; ++t) {
+                s[t][0].mac(v[0], w[t]);
+                s[t][1].mac(v[1], w[t]);
+            }
         });
 #pragma unroll
-        for (int t = 0; t < T; ++t)
-#pragma unroll
-            for (int u = 0; u < E; ++u) { r[t][0][u] = s[t][0][u].finish(m); r[t][1][u] = s[t][1][u].finish(m); }
+        for (int t = 0; t < T; ++t) { r[t][0] = s[t][0].finish(m); r[t][1] = s[t][1].finish(m); }
     }
 #pragma unroll
     for (int t = 0; t < T; ++t) {
         u64 *o = tp.out[t] + limb + x0;
-#pragma unroll
-        for (int u = 0; u < E; ++u) { o[u * 256] = r[t][0][u]; o[poly + u * 256] = r[t][1][u]; }
+        o[0] = r[t][0]; o[poly] = r[t][1];
     }
 }
 
