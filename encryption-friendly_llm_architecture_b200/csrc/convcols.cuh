@@ -8,11 +8,13 @@
 //     inverse row pass (ntt16v2_inv_rows)  ->  conv_cols / lift_cols  ->  forward row pass (ntt16v2_fwd_rows*)
 //
 // replaces inverse columns, conversion and forward columns as three kernels: for a conversion of S limbs to T, S reads + T
-// writes instead of 3 S + S + 3 T limb transfers, and one launch instead of three.  At S = 4, T = 6 (the division by P * q_l at
-// level 6) conv_cols<8, 4, 1> takes 585 us for 128 polynomials and 1225 us for 336.  Nothing in it is near its limit: 48 % of the
-// issue slots, FP64 pipe 29 %, multiply-add pipe 36 %, DRAM 13 %.  Sixteen warps per SM (128 registers; 64 make the radix-16 rounds
-// spill) do not cover their own latencies: dependent instructions, loads, and the barrier between sources and targets, which all
-// groups of the only CTA on the SM reach together.
+// writes instead of 3 S + S + 3 T limb transfers, and one launch instead of three.  The constants of a conversion carry the scale of the
+// inverse transforms, the twiddle of their last stage and that of the first forward stage, which so cost no products of their own.
+//
+// At S = 4, T = 6 (the division by P * q_level at level 6) 96 polynomials took 887 us with one CTA of four groups per SM; with two CTAs of
+// two groups 833, with the folded twiddles 815.  The instructions it cannot do without take about three quarters of that: FP64 and
+// integer products issue at half rate and do not overlap on a scheduler (a persistent version in which some groups transform the next
+// strip's sources while others convert targets, so that both kinds are always at hand, took 956 us).
 //
 // A CTA is G groups of COLS * 16 threads.  Sources are dealt to the groups, then (one CTA barrier later) targets; inside a
 // group a radix-16 round exchanges through shared memory behind a named barrier of that group only, so one group's loads,
@@ -34,11 +36,12 @@ struct ConvPlan {
     int src_limb, dst_limb;             // first limb of the sources / targets inside one instance of the arrays
     unsigned char src_prime[8], dst_prime[kMaxPrimes];
     unsigned char order[kMaxPrimes];    // targets in the order they are taken: those of the long primes, which take twice the time, first
-    u64 scale_w[8], scale_c[8];         // (ds_twiddle_word, w / q as a double) below 2^44, (w, Shoup companion) otherwise
+    u64 scale_w[8][2], scale_c[8][2];   // (ds_twiddle_word, w / q as a double) below 2^44, (w, Shoup companion) otherwise; [1]: times psi^(-N/2), the
+                                        // twiddle of the last inverse stage
     unsigned char fp[kMaxPrimes];       // target t converts on the FP64 pipe (see ConvFp)
-    uint4 c[kMaxPrimes][8];             // [target][source]: C = D / d_s mod target.  Target below 2^44: the 26-bit pieces of C
-                                        // and of C * 2^30; otherwise the 30-bit pieces of C, 0, 0
-    double d[kMaxPrimes][8][4];         // fp targets: C = d1 + d0 with d1 a multiple of 2^21, |d0| <= 2^20, C taken within q/2 of zero; the
+    uint4 c[kMaxPrimes][2][8];          // [target][half of the rows][source], the second half times psi^(N/2), the twiddle of the first forward stage: C = D / d_s mod target.  Target below 2^44: the 26-bit pieces of C
+                                        // and of C * 2^30; otherwise the 30-bit pieces of C, their sum, 0
+    double d[kMaxPrimes][2][8][4];      // fp targets: C = d1 + d0 with d1 a multiple of 2^21, |d0| <= 2^20, C taken within q/2 of zero; the
                                         // same for C * 2^30.  Set when every sum of the products is exact in a double
 };
 
@@ -49,10 +52,11 @@ template <int COLS> struct StripIndex { // [256 rows][COLS] words in shared memo
 };
 template <int THREADS> __device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(THREADS) : "memory"); }
 
-// Inverse column pass of one limb strip into the registers of a group: on return v[e] is row e * 16 + sub, times the scale, canonical.
-template <int COLS>
-__device__ __forceinline__ void strip_inverse(u64 (&v)[16], const u64 *p /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, u64 sw, u64 sc,
-                                              int g, int sub, int lane) {
+// Inverse column pass of one limb strip: word(canonical value times the scale) goes to sm at I::a, where this thread has read its own words.
+// sw, sc: the scale, and the scale times the twiddle of the last stage.
+template <int COLS, class WORD>
+__device__ __forceinline__ void strip_inverse(const u64 *p /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, const u64 (&sw)[2], const u64 (&sc)[2],
+                                              int g, int sub, int lane, WORD &&word) {
     using I = StripIndex<COLS>;
     if (m.small) {
         const DsConst c = ds_const(m);
@@ -66,12 +70,11 @@ __device__ __forceinline__ void strip_inverse(u64 (&v)[16], const u64 *p /* limb
         group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) d[e] = smd[I::a(e, sub, lane)];
-        inv16_ds(d, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
-        const double qinv_up = c.qinv * (1.0 + 0x1p-50), sf = __longlong_as_double((long long)sc);
-#pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = ds_store(ds_mul(d[e], sw, sf, c), c, c.qd, qinv_up);
+        inv16_ds<1>(d, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
+        inv16_ds_last(d, sw, sc, c, [&](int e, u64 w) { sm[I::a(e, sub, lane)] = word(w); });
     } else {
         const IntConst c = int_const(m);
+        u64 v[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = p[(sub * 16 + e) * 256];
         inv16_int(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
@@ -80,13 +83,13 @@ __device__ __forceinline__ void strip_inverse(u64 (&v)[16], const u64 *p /* limb
         group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[I::a(e, sub, lane)];
-        inv16_int(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
-#pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = canon_q(mul_shoup4(v[e], sw, sc, c.nq), c.q, c.f);
+        inv16_int<1>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
+        inv16_int_last(v, sw, sc, c, [&](int e, u64 w) { sm[I::a(e, sub, lane)] = word(w); });
     }
 }
 // Forward column pass of one limb strip that lies in sm (words of this thread at I::a; double bits below 2^44, |v| < 2q; otherwise below 3q).
-template <int COLS>
+// MADE: the rows from 128 on already carry the twiddle of the first stage.
+template <int COLS, bool MADE>
 __device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, int g, int sub, int lane) {
     using I = StripIndex<COLS>;
     if (m.small) {
@@ -95,7 +98,7 @@ __device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *s
         double d[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) d[e] = smd[I::a(e, sub, lane)];
-        fwd16_ds(d, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
+        fwd16_ds<MADE>(d, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[I::a(e, sub, lane)] = d[e];
         group_sync<COLS * 16>(g);
@@ -109,7 +112,7 @@ __device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *s
         u64 v[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[I::a(e, sub, lane)];
-        fwd16_int<kFoldColsA>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
+        fwd16_int<kFoldColsA, MADE>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[I::a(e, sub, lane)] = v[e];
         group_sync<COLS * 16>(g);
@@ -155,7 +158,7 @@ __device__ __forceinline__ double finish_small(u64 a0, u64 a1, const SmallFinish
 // units of 2^21), remainder of a1 + a0.  Sixteen fused multiply-adds and eight conversions for four sources, 58 FP64 cycles per warp
 // coefficient; the integer sums take 100 on the integer pipes.
 template <int COLS>
-__device__ __forceinline__ void convert_target_fp(u64 *sm, const u64 *ysm, const double (*__restrict__ cst)[4], int ns, const PrimeConst &m, int sub, int lane) {
+__device__ __forceinline__ void convert_target_fp(u64 *sm, const u64 *ysm, const double (*__restrict__ cst)[8][4], int ns, const PrimeConst &m, int sub, int lane) {
     using I = StripIndex<COLS>;
     const double qinv = m.q_inv_f, qd = (double)m.q;
 #pragma unroll 1
@@ -165,7 +168,7 @@ __device__ __forceinline__ void convert_target_fp(u64 *sm, const u64 *ysm, const
         for (int u = 0; u < 4; ++u) { a0[u] = 0.0; a1[u] = 0.0; }
 #pragma unroll 2
         for (int s = 0; s < ns; ++s) {
-            const double2 k0 = __ldg(reinterpret_cast<const double2 *>(cst[s])), k1 = __ldg(reinterpret_cast<const double2 *>(cst[s]) + 1);
+            const double2 *k = reinterpret_cast<const double2 *>(cst[e0 >> 3][s]), k0 = __ldg(k), k1 = __ldg(k + 1);
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
@@ -182,7 +185,7 @@ __device__ __forceinline__ void convert_target_fp(u64 *sm, const u64 *ysm, const
     }
 }
 template <int COLS>
-__device__ __forceinline__ void convert_target_small(u64 *sm, const u64 *ysm, const uint4 *__restrict__ cst, int ns, const PrimeConst &m, int sub, int lane) {
+__device__ __forceinline__ void convert_target_small(u64 *sm, const u64 *ysm, const uint4 (*__restrict__ cst)[8], int ns, const PrimeConst &m, int sub, int lane) {
     using I = StripIndex<COLS>;
     const SmallFinish f = small_finish(m);
     const DsConst ds = ds_const(m);
@@ -193,7 +196,7 @@ __device__ __forceinline__ void convert_target_small(u64 *sm, const u64 *ysm, co
         for (int u = 0; u < 4; ++u) { a0[u] = 0; a1[u] = 0; }
 #pragma unroll 1
         for (int s = 0; s < ns; ++s) {
-            const uint4 c = __ldg(cst + s);
+            const uint4 c = __ldg(cst[e0 >> 3] + s);
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
@@ -210,25 +213,25 @@ __device__ __forceinline__ void convert_target_small(u64 *sm, const u64 *ysm, co
     }
 }
 template <int COLS>
-__device__ __forceinline__ void convert_target_wide(u64 *sm, const u64 *ysm, const uint4 *__restrict__ cst, int ns, const PrimeConst &m, int sub, int lane) {
+__device__ __forceinline__ void convert_target_wide(u64 *sm, const u64 *ysm, const uint4 (*__restrict__ cst)[8], int ns, const PrimeConst &m, int sub, int lane) {
     using I = StripIndex<COLS>;
 #pragma unroll 1
     for (int e0 = 0; e0 < 16; e0 += 4) {
-        u64 a0[4], a1[4], a2[4];
+        u64 a0[4], am[4], a2[4]; // as in PieceAcc
 #pragma unroll
-        for (int u = 0; u < 4; ++u) { a0[u] = 0; a1[u] = 0; a2[u] = 0; }
+        for (int u = 0; u < 4; ++u) { a0[u] = 0; am[u] = 0; a2[u] = 0; }
 #pragma unroll 2
         for (int s = 0; s < ns; ++s) {
-            const uint4 c = __ldg(cst + s);
+            const uint4 c = __ldg(cst[e0 >> 3] + s);
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
-                a0[u] = mad_wide((u32)y, c.x, a0[u]); a1[u] = mad_wide((u32)y, c.y, a1[u]);
-                a1[u] = mad_wide((u32)(y >> 32), c.x, a1[u]); a2[u] = mad_wide((u32)(y >> 32), c.y, a2[u]);
+                const u32 y0 = (u32)y, y1 = (u32)(y >> 32);
+                a0[u] = mad_wide(y0, c.x, a0[u]); am[u] = mad_wide(y0 + y1, c.z, am[u]); a2[u] = mad_wide(y1, c.y, a2[u]);
             }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) sm[I::a(e0 + u, sub, lane)] = finish_wide(a0[u], a1[u], a2[u], m);
+        for (int u = 0; u < 4; ++u) sm[I::a(e0 + u, sub, lane)] = finish_wide(a0[u], am[u] - a0[u] - a2[u], a2[u], m);
     }
 }
 
@@ -247,14 +250,12 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
     const int col = blockIdx.x * COLS + lane;
     const u64 *sp = src + (size_t)blockIdx.z * src_outer + (size_t)pl->src_limb * kN16 + col;
     u64 *dp = dst + (size_t)blockIdx.z * dst_outer + (size_t)pl->dst_limb * kN16 + col;
-    u64 v[16];
     pdl_wait();
     for (int s = g; s < ns; s += G) {
         const int pi = pl->src_prime[s];
         u64 *sm = strips + s * I::kWords;
-        strip_inverse<COLS>(v, sp + (size_t)s * kN16, sm, pc[pi], tb.inv + (size_t)pi * Ntt16Layout::kEntries, pl->scale_w[s], pl->scale_c[s], g, sub, lane);
-#pragma unroll
-        for (int e = 0; e < 16; ++e) sm[I::a(e, sub, lane)] = ((v[e] >> 30) << 32) | ((u32)v[e] & 0x3FFFFFFFu); // the words this thread read itself
+        strip_inverse<COLS>(sp + (size_t)s * kN16, sm, pc[pi], tb.inv + (size_t)pi * Ntt16Layout::kEntries, pl->scale_w[s], pl->scale_c[s], g, sub, lane,
+                            [](u64 v) { return ((v >> 30) << 32) | ((u32)v & 0x3FFFFFFFu); });
     }
     __syncthreads();
     u64 *ex = strips + (ns + g) * I::kWords;
@@ -267,12 +268,12 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
         const int t = pl->order[k];
         const int pi = pl->dst_prime[t];
         const PrimeConst m = pc[pi];
-        const uint4 *cst = pl->c[t];
+        const uint4 (*cst)[8] = pl->c[t];
         const bool fp = pl->fp[t];
         if (fp) convert_target_fp<COLS>(ex, strips, pl->d[t], ns, m, sub, lane);
         else if (m.small) convert_target_small<COLS>(ex, strips, cst, ns, m, sub, lane);
         else convert_target_wide<COLS>(ex, strips, cst, ns, m, sub, lane);
-        strip_forward<COLS>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)pi * Ntt16Layout::kEntries, g, sub, lane);
+        strip_forward<COLS, true>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)pi * Ntt16Layout::kEntries, g, sub, lane);
     }
 }
 
@@ -287,14 +288,11 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) lift_cols(const u64 *src,
     const int col = blockIdx.x * COLS + lane;
     const u64 ql = pc[level].q;
     const bool src_small = pc[level].small;
-    u64 v[16];
     pdl_wait();
     if (g == 0) {
         const PrimeConst m = pc[level];
-        const u64 sw = m.small ? ds_twiddle_word(m.n_inv) : m.n_inv, sc = m.small ? (u64)__double_as_longlong(m.n_inv_f) : m.n_inv_sh;
-        strip_inverse<COLS>(v, src + (size_t)blockIdx.y * src_outer + col, strips, m, tb.inv + (size_t)level * Ntt16Layout::kEntries, sw, sc, g, sub, lane);
-#pragma unroll
-        for (int e = 0; e < 16; ++e) strips[I::a(e, sub, lane)] = v[e] > (ql >> 1) ? v[e] - ql : v[e]; // signed
+        strip_inverse<COLS>(src + (size_t)blockIdx.y * src_outer + col, strips, m, tb.inv + (size_t)level * Ntt16Layout::kEntries, m.n_inv_w, m.n_inv_c, g, sub, lane,
+                            [&](u64 v) { return v > (ql >> 1) ? v - ql : v; }); // signed
     }
     __syncthreads();
     u64 *dp = dst + (size_t)blockIdx.y * dst_outer + col, *ex = strips + (1 + g) * I::kWords;
@@ -310,7 +308,7 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) lift_cols(const u64 *src,
             else if ((ql >> 1) < m.q) w = y < 0 ? (u64)(y + (i64)m.q) : (u64)y;
             else w = reduce_i64(y, m);
         }
-        strip_forward<COLS>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)t * Ntt16Layout::kEntries, g, sub, lane);
+        strip_forward<COLS, false>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)t * Ntt16Layout::kEntries, g, sub, lane);
     }
 }
 
@@ -416,14 +414,24 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
 // Single passes, for the fused sequences.  A grid of one or two CTAs per SM takes the kernels that may use 128 registers and
 // fetch the twiddles of the second round (which nobody shares) before anything else, under the tail of the predecessor.
 constexpr int kSmallGrid = 2 * 148;
+// From this many CTAs on, the passes that follow a conversion are launched the ordinary way: under programmatic dependence their CTAs would
+// move onto SMs that the conversion still holds at its 208 KB of shared memory, and the SMs would keep that split, with the smallest L1, for
+// all kernels of the sequence (forward row passes with the last step 255 -> 312 us, tensor products 201 -> 229, masked inner products 484 -> 537).
+constexpr int kPlainGrid = 4 * 4 * 148;
+template <class... P, class... A> inline cudaError_t launch_plain(cudaStream_t st, void (*kernel)(P...), dim3 grid, dim3 block, A &&...args) {
+    kernel<<<grid, block, 0, st>>>(P(std::forward<A>(args))...);
+    return cudaPeekAtLastError();
+}
 inline cudaError_t launch_inv_rows16(cudaStream_t st, const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
     return launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_inv_rows<2> : ntt16v2_inv_rows<4>, dim3(16, count), 256, 0, src, LimbAddr16{src_outer}, dst, LimbAddr16{dst_outer}, map, pc, tb);
 }
 inline cudaError_t launch_fwd_rows16(cudaStream_t st, u64 *d, size_t outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
+    if (16 * count >= kPlainGrid) return launch_plain(st, ntt16v2_fwd_rows<4>, dim3(16, count), 256, d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb);
     return launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_fwd_rows<2> : ntt16v2_fwd_rows<4>, dim3(16, count), 256, 0, d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb);
 }
 template <class ADD>
 inline cudaError_t launch_fwd_rows_fin16(cudaStream_t st, const u64 *t, size_t t_outer, int n, int instances, const RowsFin &f, const InvScale &sc, const ADD &add, const PrimeConst *pc, const Ntt16Tables &tb) {
+    if (16 * n * instances >= kPlainGrid) return launch_plain(st, ntt16v2_fwd_rows_fin<4, ADD>, dim3(16, n, instances), 256, t, t_outer, f, sc, add, pc, tb);
     return launch_pdl(st, 16 * n * instances <= kSmallGrid ? ntt16v2_fwd_rows_fin<2, ADD> : ntt16v2_fwd_rows_fin<4, ADD>, dim3(16, n, instances), 256, 0, t, t_outer, f, sc, add, pc, tb);
 }
 

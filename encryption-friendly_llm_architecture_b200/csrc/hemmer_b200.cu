@@ -284,32 +284,38 @@ const KsPlan *get_plan(hb_ctx *c, int level) {
 void fill_conv(const HostCtx &h, ConvPlan &p, const std::vector<int> &src, const std::vector<int> &dst, int src_limb, int dst_limb) {
     p.ns = (int)src.size(); p.nt = (int)dst.size(); p.src_limb = src_limb; p.dst_limb = dst_limb;
     auto hat = [&](size_t s, u64 q) { u64 v = 1; for (size_t t = 0; t < src.size(); ++t) if (t != s) v = hbhost::mulmod(v, h.q[src[t]] % q, q); return v; };
+    auto half_turn = [&](int prime) { return hbhost::powmod(h.psi_root[(size_t)prime], (u64)h.N / 2, h.q[(size_t)prime]); }; // psi^(N/2)
     for (size_t s = 0; s < src.size(); ++s) {
-        const u64 q = h.q[src[s]];
+        const u64 q = h.q[src[s]], v = hbhost::mulmod(hbhost::invmod((u64)h.N % q, q), hbhost::invmod(hat(s, q), q), q);
         p.src_prime[s] = (unsigned char)src[s];
-        scale_words(hbhost::mulmod(hbhost::invmod((u64)h.N % q, q), hbhost::invmod(hat(s, q), q), q), q, p.scale_w[s], p.scale_c[s]);
+        scale_words(v, q, p.scale_w[s][0], p.scale_c[s][0]);
+        scale_words(hbhost::mulmod(v, q - half_turn(src[s]), q), q, p.scale_w[s][1], p.scale_c[s][1]); // its inverse is its negative
     }
     for (size_t t = 0; t < dst.size(); ++t) {
-        const u64 q = h.q[dst[t]];
+        const u64 q = h.q[dst[t]], m26 = ((u64)1 << 26) - 1, m30 = ((u64)1 << 30) - 1;
         p.dst_prime[t] = (unsigned char)dst[t];
-        double low = 0, high = 0; // largest sums of the FP64 form, in units of 1 and 2^21
-        for (size_t s = 0; s < src.size(); ++s) {
-            const u64 v = hat(s, q), v30 = hbhost::mulmod(v, ((u64)1 << 30) % q, q), m26 = ((u64)1 << 26) - 1, m30 = ((u64)1 << 30) - 1;
-            if (!(q >> 44)) {
-                auto split = [&](u64 w, double *d) { // |w - q * [w > q / 2]| = d[1] + d[0]
-                    const i64 c = w > q / 2 ? (i64)w - (i64)q : (i64)w, hi = (c + ((i64)1 << 20)) >> 21;
-                    d[0] = (double)(c - hi * ((i64)1 << 21)); d[1] = (double)(hi * ((i64)1 << 21));
-                };
-                split(v, p.d[t][s]); split(v30, p.d[t][s] + 2);
-            }
-            p.c[t][s] = (q >> 44) ? make_uint4((u32)(v & m30), (u32)(v >> 30), 0, 0) : make_uint4((u32)(v & m26), (u32)(v >> 26), (u32)(v30 & m26), (u32)(v30 >> 26));
-            const double y0 = 0x1p30, y1 = (double)((h.q[src[s]] >> 30) + 1);
-            low += y0 * std::fabs(p.d[t][s][0]) + y1 * std::fabs(p.d[t][s][2]);
-            high += (y0 * std::fabs(p.d[t][s][1]) + y1 * std::fabs(p.d[t][s][3])) * 0x1p-21;
-        }
-        // a1 - qh * q is formed exactly when |a0| + 2q stays below 2^53; the quotient must be exact to well below one
         p.order[t] = (unsigned char)t;
-        p.fp[t] = !(q >> 44) && src.size() <= 4 && low + 2.0 * (double)q < 0x1p53 && high < 0x1p53;
+        p.fp[t] = !(q >> 44) && src.size() <= 4;
+        for (int half = 0; half < 2; ++half) {
+            double low = 0, high = 0; // largest sums of the FP64 form, in units of 1 and 2^21
+            for (size_t s = 0; s < src.size(); ++s) {
+                const u64 v = half ? hbhost::mulmod(hat(s, q), half_turn(dst[t]), q) : hat(s, q), v30 = hbhost::mulmod(v, ((u64)1 << 30) % q, q);
+                double *d = p.d[t][half][s];
+                if (!(q >> 44)) {
+                    auto split = [&](u64 w, double *o) { // |w - q * [w > q / 2]| = o[1] + o[0]
+                        const i64 c = w > q / 2 ? (i64)w - (i64)q : (i64)w, hi = (c + ((i64)1 << 20)) >> 21;
+                        o[0] = (double)(c - hi * ((i64)1 << 21)); o[1] = (double)(hi * ((i64)1 << 21));
+                    };
+                    split(v, d); split(v30, d + 2);
+                }
+                p.c[t][half][s] = (q >> 44) ? make_uint4((u32)(v & m30), (u32)(v >> 30), (u32)(v & m30) + (u32)(v >> 30), 0) : make_uint4((u32)(v & m26), (u32)(v >> 26), (u32)(v30 & m26), (u32)(v30 >> 26));
+                const double y0 = 0x1p30, y1 = (double)((h.q[src[s]] >> 30) + 1);
+                low += y0 * std::fabs(d[0]) + y1 * std::fabs(d[2]);
+                high += (y0 * std::fabs(d[1]) + y1 * std::fabs(d[3])) * 0x1p-21;
+            }
+            // a1 - qh * q is formed exactly when |a0| + 2q stays below 2^53; the quotient must be exact to well below one
+            if (!(low + 2.0 * (double)q < 0x1p53 && high < 0x1p53)) p.fp[t] = 0;
+        }
     }
     std::stable_sort(p.order, p.order + p.nt, [&](int x, int y) { return (h.q[p.dst_prime[x]] >> 44) && !(h.q[p.dst_prime[y]] >> 44); });
 }
@@ -361,15 +367,18 @@ void conv_opt_in(hb_ctx *c) {
     if (c->smem_opt_in_conv) return;
     auto allow = [](auto *kernel, size_t bytes) { CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); };
     allow(conv_cols<8, 4, 1>, strip_bytes<8>(12)); allow(conv_cols<4, 4, 2>, strip_bytes<4>(12)); allow(conv_cols<4, 8, 1>, strip_bytes<4>(16));
-    allow(lift_cols<8, 2, 2>, strip_bytes<8>(3)); allow(lift_cols<4, 4, 2>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1>, strip_bytes<4>(9));
+    allow(conv_cols<8, 2, 2>, strip_bytes<8>(6)); allow(lift_cols<8, 2, 2>, strip_bytes<8>(3)); allow(lift_cols<4, 4, 2>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1>, strip_bytes<4>(9));
     c->smem_opt_in_conv = true;
 }
 // Strip width and groups of a launch over `units` (polynomial, conversion) pairs.  At most two units: narrow strips and many groups, so that
-// all sources and all targets of a unit are worked on at once.  Up to 32: narrow strips, two CTAs per SM, for the last wave.
-// Beyond: strips of eight columns (64-byte runs).  Rotations at level 6, us, (4 cols x 8 groups) / (4 x 4) / (8 x 4): one ciphertext
-// 88 / 103 / 98, eight 397 / 363 / 378, 64 2773 / 2524 / 2494.
+// all sources and all targets of a unit are worked on at once.  Up to twelve: narrow strips, two CTAs per SM, for the last wave.
+// Beyond: strips of eight columns (64-byte runs) and two groups, two CTAs per SM, whose barriers and loads cover each other, as long as their
+// strips fit (four sources); otherwise four groups and one CTA.  Rotations at level 6, us, (4 cols x 8 groups) / (4 x 4) / (8 x 4): one
+// ciphertext 88 / 103 / 98, eight 397 / 363 / 378, 64 2773 / 2524 / 2494.  Launches, us, (8 x 4) / (8 x 2): 96 polynomials of the division at level 6
+// 858 / 815, the conversions of 256 products at level 8 3093 / 2863; (4 x 4) / (8 x 2): 32 polynomials of the division 142 / 147, but the call
+// sequence of one product 10.87 / 10.74 ms; eight units 44.5 / 66.8.
 enum StripShape { kStrip8x2, kStrip8x4, kStrip4x4, kStrip4x8 };
-StripShape conv_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 32 ? kStrip4x4 : kStrip8x4; }
+StripShape conv_shape(int units, int max_ns) { return units <= 2 ? kStrip4x8 : units <= 12 ? kStrip4x4 : max_ns <= 4 ? kStrip8x2 : units <= 32 ? kStrip4x4 : kStrip8x4; }
 StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : kStrip8x2; }
 // `plans` conversions (the largest with max_ns sources) of `instances` polynomials in one launch
 void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int instances) {
@@ -377,7 +386,8 @@ void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, con
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
         launch(c, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
     };
-    switch (conv_shape(instances * count)) {
+    switch (conv_shape(instances * count, max_ns)) {
+    case kStrip8x2: go(conv_cols<8, 2, 2>, 8, 2, strip_bytes<8>(max_ns + 2)); break;
     case kStrip8x4: go(conv_cols<8, 4, 1>, 8, 4, strip_bytes<8>(max_ns + 4)); break;
     case kStrip4x4: go(conv_cols<4, 4, 2>, 4, 4, strip_bytes<4>(max_ns + 4)); break;
     default: go(conv_cols<4, 8, 1>, 4, 8, strip_bytes<4>(max_ns + 8)); break;
@@ -1142,10 +1152,11 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             p.mu_lo = (u64)(((two64 % q) << 64) / q);
             p.n_inv = hbhost::invmod((u64)N, q); p.n_inv_sh = hbhost::shoup(p.n_inv, q);
             p.iu = hbhost::powmod(c->h->psi_root[i], (u64)N / 2, q); p.iu_sh = hbhost::shoup(p.iu, q);
+            scale_words(p.n_inv, q, p.n_inv_w[0], p.n_inv_c[0]);
+            scale_words(hbhost::mulmod(p.n_inv, q - p.iu, q), q, p.n_inv_w[1], p.n_inv_c[1]); // psi^(-N/2) = -psi^(N/2)
             // the 2^16 transform carries the residues of primes below 2^44 as integer-valued doubles (ntt16.cuh)
             p.small = (big && q < ((u64)1 << 44)) ? 1 : 0;
             p.q_inv_f = 1.0 / (double)q;
-            p.n_inv_f = (double)p.n_inv / (double)q;
             p.fp = q < ((u64)1 << 44) ? 1 : 0;
             // lazy FP64-assisted products are below 1.6 q; reduce_fp takes sums below 2^52.  The lazy sums that are left have at most
             // kMaxTerms terms (k_last_prod, k_prod_rescale_fin; eight digits in k_ks_inner_pair); any prime below 2^44 allows 160.

@@ -21,10 +21,10 @@ struct PrimeConst {
     u64 q;
     u64 mu_hi, mu_lo;   // floor(2^128 / q)
     u64 n_inv, n_inv_sh; // N^-1 mod q and its Shoup companion
+    u64 n_inv_w[2], n_inv_c[2]; // N^-1 and N^-1 psi^(-N/2) in the form the 2^16 transforms multiply by: (w, companion)
     u64 iu, iu_sh;      // psi^(N/2): the image of the imaginary unit
     u64 small;          // 1 when q < 2^44 and N = 2^16: the transforms carry its residues as doubles
     double q_inv_f;     // 1/q
-    double n_inv_f;     // n_inv / q
     u64 fp;             // 1 when q < 2^44: element-wise kernels take quotients from the FP64 pipe
     u32 fold_shift;     // primes of b >= 45 bits: b - 32 (every such prime of a context lies within 2^(b-12) below 2^b)
     u32 fold_d;         //   and 2^b - q

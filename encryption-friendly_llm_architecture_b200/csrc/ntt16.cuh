@@ -140,7 +140,8 @@ __device__ __forceinline__ IntConst int_const(const PrimeConst &m) {
 // Products are below 4q (mul_shoup4), so a stage adds 4q to the bound B of the values; x is folded below ~2^b before the
 // additions of the stages named by the bit mask FOLD.  The words hold 16 q: in units of q the four rounds of a transform
 // (masks 8, 4, 2, 9) run 3-7-11-15|5, 5-9-13|5-9, 9-13|5-9-13, 13|5-9-13|5 (| = a fold).
-template <int FOLD, class TW> __device__ __forceinline__ void fwd16_int(u64 (&v)[16], const TW &tp, const IntConst &c) {
+// MADE: the upper half already carries the twiddle of the first stage (values below 4q)
+template <int FOLD, bool MADE = false, class TW> __device__ __forceinline__ void fwd16_int(u64 (&v)[16], const TW &tp, const IntConst &c) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         const int half = 8 >> s;
@@ -150,7 +151,7 @@ template <int FOLD, class TW> __device__ __forceinline__ void fwd16_int(u64 (&v)
 #pragma unroll
             for (int j = 0; j < half; ++j) {
                 u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
-                const u64 t = mul_shoup4(y, tw.x, tw.y, c.nq);
+                const u64 t = MADE && s == 0 ? y : mul_shoup4(y, tw.x, tw.y, c.nq);
                 if ((FOLD >> s) & 1) x = fold_q(x, c.f);
                 y = x + c.q4 - t;
                 x = x + t;
@@ -161,9 +162,10 @@ template <int FOLD, class TW> __device__ __forceinline__ void fwd16_int(u64 (&v)
 constexpr int kFoldColsA = 8, kFoldColsB = 4, kFoldRowsA = 2, kFoldRowsB = 9;
 // Four Gentleman-Sande stages, the mirror image.  Values enter and leave below 4q: sums reach 8q, then 16q, and are folded at
 // every second stage.
-template <class TW> __device__ __forceinline__ void inv16_int(u64 (&v)[16], const TW &tp, const IntConst &c) {
+// LAST: the stage to end with
+template <int LAST = 0, class TW> __device__ __forceinline__ void inv16_int(u64 (&v)[16], const TW &tp, const IntConst &c) {
 #pragma unroll
-    for (int s = 3; s >= 0; --s) {
+    for (int s = 3; s >= LAST; --s) {
         const int half = 8 >> s;
 #pragma unroll
         for (int g = 0; g < (1 << s); ++g) {
@@ -176,6 +178,17 @@ template <class TW> __device__ __forceinline__ void inv16_int(u64 (&v)[16], cons
                 y = mul_shoup4(d, tw.x, tw.y, c.nq);
             }
         }
+    }
+}
+
+// The last stage of an inverse transform together with the multiplication by N^-1 (or another constant): its only twiddle goes into the
+// constant of the differences, so that the stage costs no products of its own.  sw, sc: constant, constant * twiddle.  store(e, canonical).
+template <class STORE> __device__ __forceinline__ void inv16_int_last(const u64 (&v)[16], const u64 (&sw)[2], const u64 (&sc)[2], const IntConst &c, STORE &&store) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { // below 8q before, sums and differences below 16q
+        const u64 a = v[j] + v[j + 8], d = v[j] + c.q8 - v[j + 8];
+        store(j, canon_q(mul_shoup4(a, sw[0], sc[0], c.nq), c.q, c.f));
+        store(j + 8, canon_q(mul_shoup4(d, sw[1], sc[1], c.nq), c.q, c.f));
     }
 }
 
@@ -229,7 +242,8 @@ __device__ __forceinline__ u64 ds_store(double v, const DsConst &c, double shift
     const double rb = __fma_rn(-k, c.qd, v2 + kTwo52);                   // 2^52 + (v2 - k q), exact
     return (u64)__double_as_longlong(rb) & 0x000FFFFFFFFFFFFFull;
 }
-template <class TW> __device__ __forceinline__ void fwd16_ds(double (&v)[16], const TW &tp, const DsConst &c) {
+// MADE: as in fwd16_int
+template <bool MADE = false, class TW> __device__ __forceinline__ void fwd16_ds(double (&v)[16], const TW &tp, const DsConst &c) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         const int half = 8 >> s;
@@ -240,7 +254,7 @@ template <class TW> __device__ __forceinline__ void fwd16_ds(double (&v)[16], co
 #pragma unroll
             for (int j = 0; j < half; ++j) {
                 double &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
-                const double t = ds_mul(y, tw.x, wf, c);
+                const double t = MADE && s == 0 ? y : ds_mul(y, tw.x, wf, c);
                 y = x - t;
                 x = x + t;
             }
@@ -285,9 +299,9 @@ template <class TW> __device__ __forceinline__ void inv16_ds8(double (&v)[16], c
 // Gentleman-Sande round.  The sum path doubles per stage; only v[0] takes the sum at all four stages (16 x its
 // inputs), v[1] ends below 4.2 q whatever came in, the others lower: the caller reduces v[0] after each round, so
 // every round starts from values below 4.2 q and stays below 68 q.
-template <class TW> __device__ __forceinline__ void inv16_ds(double (&v)[16], const TW &tp, const DsConst &c) {
+template <int LAST = 0, class TW> __device__ __forceinline__ void inv16_ds(double (&v)[16], const TW &tp, const DsConst &c) {
 #pragma unroll
-    for (int s = 3; s >= 0; --s) {
+    for (int s = 3; s >= LAST; --s) {
         const int half = 8 >> s;
 #pragma unroll
         for (int g = 0; g < (1 << s); ++g) {
@@ -302,7 +316,16 @@ template <class TW> __device__ __forceinline__ void inv16_ds(double (&v)[16], co
             }
         }
     }
-    v[0] = ds_reduce(v[0], c);
+    if (LAST == 0) v[0] = ds_reduce(v[0], c);
+}
+// as inv16_int_last; the values come from three stages without a reduction (below 34 q, sums below 68 q), the products lie within 0.7 q of zero
+template <class STORE> __device__ __forceinline__ void inv16_ds_last(const double (&v)[16], const u64 (&sw)[2], const u64 (&sc)[2], const DsConst &c, STORE &&store) {
+    const double s0 = __longlong_as_double((long long)sc[0]), s1 = __longlong_as_double((long long)sc[1]), qinv_up = c.qinv * (1.0 + 0x1p-50);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        store(j, ds_store(ds_mul(v[j] + v[j + 8], sw[0], s0, c), c, c.qd, qinv_up));
+        store(j + 8, ds_store(ds_mul(v[j] - v[j + 8], sw[1], s1, c), c, c.qd, qinv_up));
+    }
 }
 
 // ---- forward, column pass: stages 1..8 ----
@@ -486,14 +509,8 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *src, Li
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smd[(e * 16 + sub) * 16 + lane];
-        inv16_ds(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
-        const double qinv_up = c.qinv * (1.0 + 0x1p-50);
-        const u64 sw = ds_twiddle_word(m.n_inv);
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            const double t = ds_mul(v[e], sw, m.n_inv_f, c); // x * N^-1 in (-0.52 q, 0.52 q)
-            o[(e * 16 + sub) * 256] = ds_store(t, c, c.qd, qinv_up);
-        }
+        inv16_ds<1>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
+        inv16_ds_last(v, m.n_inv_w, m.n_inv_c, c, [&](int e, u64 w) { o[(e * 16 + sub) * 256] = w; });
     } else {
         u64 v[16];
         pdl_wait();
@@ -506,9 +523,8 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *src, Li
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[(e * 16 + sub) * 16 + lane];
-        inv16_int(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
-#pragma unroll
-        for (int e = 0; e < 16; ++e) o[(e * 16 + sub) * 256] = canon_q(mul_shoup4(v[e], m.n_inv, m.n_inv_sh, c.nq), c.q, c.f);
+        inv16_int<1>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
+        inv16_int_last(v, m.n_inv_w, m.n_inv_c, c, [&](int e, u64 w) { o[(e * 16 + sub) * 256] = w; });
     }
 }
 
