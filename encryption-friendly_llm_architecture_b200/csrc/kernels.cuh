@@ -356,9 +356,9 @@ __global__ void k_last_prod_parts(u64 *last, const __grid_constant__ PartTerms p
 // kPartLanes * pair of polynomials): the masks cross L2 once per CTA and shared memory once per two polynomials.  The words a_j, and the words of
 // t that a sum is subtracted from, come through a ring of kPartRing stages in shared memory that runs on across terms and polynomials, each
 // thread copying its own (cp.async, no barrier).  With two loads ahead in registers and t loaded when it was needed, 6.1 ms for 48
-// polynomials, sixteen terms, twelve parts at level 7 (both launches); with the ring for the a_j 5.5, with t in it as well and two terms per
-// turn of the loop (the sums change registers with every product, so a single one ends in moves) 4.1 ms.  Bound by instruction
-// issue now: 57 % of the slots with sixteen warps, FP64 40 % of the time on a short limb.
+// polynomials, sixteen terms, twelve parts at level 7 (both launches); with the ring for the a_j 5.5, with t in it as well 4.1, with addresses
+// from a table instead of branches and one instruction per wide multiply-add 3.7 ms.  Bound by instruction issue now: 57 % of the slots with
+// sixteen warps, on a short limb FP64 45 % of the time.
 // t == nullptr: raw sums of limb `level`, out[(g * nbp + bp) * N + x]                       grid = (ceil(parts/G), N/kPartLanes, 1)
 // else: out[((g * nbp + bp) * level + l) * N + x] = (sum - t[same]) * q_level^-1 mod q_l      grid = (ceil(parts/G), N/kPartLanes, level)
 // (parts first, so that the CTAs that read the same words run together)
@@ -378,6 +378,12 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
     const int l = t ? (int)blockIdx.z : level, g0 = blockIdx.x * G;
     const int gn = min(G, pt.parts - g0);
     const u32 x0 = blockIdx.y * kPartLanes;
+    // What a member needs, in order: its terms a_j, then the words of t that its parts are subtracted from.  (address at member 0, bytes per member)
+    __shared__ ulonglong2 table[kMaxPartTerms + G];
+    const u32 words = (u32)(count + (t ? gn : 0));
+    const size_t member = (size_t)(level + 1) * N, t_member = (size_t)level * N, t_part = (size_t)nbp * t_member, first = (size_t)l * N + x0;
+    if ((u32)tid < words)
+        table[tid] = tid < count ? make_ulonglong2((u64)(size_t)(pt.a[tid] + first), member * 8) : make_ulonglong2((u64)(size_t)(t + (size_t)(g0 + tid - count) * t_part + first), t_member * 8);
     if (tid == 0) { mbar_init(&bar, 1); mbar_fence_init(); }
     __syncthreads();
     if (tid < 32) {
@@ -392,22 +398,19 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
             if (src) bulk_load(ptile + (size_t)((ci % count) * G + ci / count) * kPartLanes, src + (size_t)l * N + x0, kPartLanes * 8u, &bar);
         }
     }
-    // The words of this thread: members slot * M .., then kSlots * M further on; of each the terms a_j, then the words of t that its parts
-    // are subtracted from.
-    const size_t member = (size_t)(level + 1) * N, t_part = (size_t)nbp * level * N;
-    const size_t first = (size_t)l * N + x0 + lane;
-    const int words = count + (t ? gn : 0);
-    int fj = 0, fb = M * slot;
-    u32 to = 0; // byte offset of the stage that is filled next
+    // The words of this thread: members slot * M .., then kSlots * M further on, by the table's rows for each.  Past the last member the
+    // last one is fetched again, and not used.
+    const u32 lane_at = (u32)lane * 8u, last_member = (u32)nbp - 1u;
+    u32 row = 0, fb = (u32)(M * slot), to = 0; // what is fetched next; byte offset of the stage that it goes to
     auto fetch = [&] {
-        if (fb < nbp) {
-            const bool term = fj < count;
-            const u64 *p = term ? pt.a[fj] + first + (size_t)fb * member : t + first + (size_t)fb * level * N + (size_t)(g0 + fj - count) * t_part;
-            cp_async8(ring_at + to, p);
-            cp_async8(ring_at + to + 4096, fb + 1 < nbp ? p + (term ? member : (size_t)level * N) : p);
-            if (++fj == words) { fj = 0; fb += kSlots * M; }
-        }
+        const ulonglong2 r = table[row];
+        const u64 p = r.x + lane_at;
+        cp_async8(ring_at + to, reinterpret_cast<const void *>(p + (u64)min(fb, last_member) * (u32)r.y));
+        cp_async8(ring_at + to + 4096, reinterpret_cast<const void *>(p + (u64)min(fb + 1u, last_member) * (u32)r.y));
         cp_async_commit();
+        const bool wrap = row + 1u == words;
+        row = wrap ? 0u : row + 1u;
+        fb += wrap ? (u32)(kSlots * M) : 0u;
         to = (to + kStage * 8) & (kPartRing * kStage * 8 - 1);
     };
 #pragma unroll 1
@@ -443,14 +446,12 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
     };
     for (int bp = M * slot; bp < nbp; bp += kSlots * M) {
         u64 v[M][G];
-        auto terms = [&](auto &&product) {
-            const u64 *w = ptile + lane;
-#pragma unroll 2
-            for (int j = 0; j < count; ++j, w += G * kPartLanes) {
-                u64 a[M];
-                next(a);
-                product(a, w, eight && j && j % 8 == 0);
-            }
+        const u64 *w = ptile + lane;
+        auto term = [&](int j, auto &&product) {
+            u64 a[M];
+            next(a);
+            product(a, w, eight && j && j % 8 == 0);
+            w += G * kPartLanes;
         };
         if (m.fp) { // products and sums exactly on the FP64 pipe
             FpAcc s[M][G];
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
             for (int i = 0; i < M; ++i)
 #pragma unroll
                 for (int g = 0; g < G; ++g) s[i][g].zero();
-            terms([&](const u64 (&a)[M], const u64 *w, bool full) {
+            auto product = [&](const u64 (&a)[M], const u64 *w, bool full) {
                 if (full) {
 #pragma unroll
                     for (int i = 0; i < M; ++i)
@@ -474,7 +475,9 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
 #pragma unroll
                     for (int i = 0; i < M; ++i) s[i][g].mac(d[i], k);
                 }
-            });
+            };
+#pragma unroll 2
+            for (int j = 0; j < count; ++j) term(j, product);
 #pragma unroll
             for (int i = 0; i < M; ++i)
 #pragma unroll
@@ -485,7 +488,7 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
             for (int i = 0; i < M; ++i)
 #pragma unroll
                 for (int g = 0; g < G; ++g) s[i][g].zero();
-            terms([&](const u64 (&a)[M], const u64 *w, bool full) {
+            auto product = [&](const u64 (&a)[M], const u64 *w, bool full) {
                 if (full) {
 #pragma unroll
                     for (int i = 0; i < M; ++i)
@@ -498,25 +501,27 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
 #pragma unroll
                     for (int i = 0; i < M; ++i) s[i][g].mac((u32)a[i] & 0x3FFFFFFFu, (u32)(a[i] >> 30), (u32)k, (u32)(k >> 32));
                 }
-            });
+            };
+#pragma unroll 1
+            for (int j = 0; j < count; ++j) term(j, product);
 #pragma unroll
             for (int i = 0; i < M; ++i)
 #pragma unroll
                 for (int g = 0; g < G; ++g) v[i][g] = s[i][g].finish(m);
         }
+        u64 *o = out + (t ? (size_t)g0 * t_part + (size_t)bp * t_member + first : ((size_t)g0 * nbp + bp) * N + x0) + lane;
+        const size_t o_part = t ? t_part : (size_t)nbp * N, o_member = t ? t_member : (size_t)N;
 #pragma unroll
-        for (int g = 0; g < G; ++g)
+        for (int g = 0; g < G; ++g, o += o_part)
             if (g < gn) {
                 u64 a[M];
                 if (t) next(a);
 #pragma unroll
                 for (int i = 0; i < M; ++i)
-                    if (bp + i < nbp) {
-                        if (t) out[(size_t)(g0 + g) * t_part + (size_t)(bp + i) * level * N + first] = mul_mod_any(sub_mod(v[i][g], a[i], m.q), qli, m);
-                        else out[((size_t)(g0 + g) * nbp + bp + i) * N + x0 + lane] = v[i][g];
-                    }
+                    if (bp + i < nbp) o[i * o_member] = t ? mul_mod_any(sub_mod(v[i][g], a[i], m.q), qli, m) : v[i][g];
             }
     }
+    cp_async_wait<0>(); // what was fetched past the end
 }
 // The same for a few polynomials: the masks are then most of the bytes, so they are streamed instead of kept.  A thread holds the words a_j of
 // its coefficient in two polynomials and walks over the parts, with the masks of a part in flight together.  A launch for one two-tile
@@ -1385,8 +1390,8 @@ __global__ void k_div_fin(u64 *__restrict__ out, const u64 *__restrict__ E, cons
 // partial products of several K-groups in the same pass.  A thread works on one coefficient of both polynomials: a copy word is
 // read once for T tiles and a weight word once (and converted or cut once) for two polynomials.  Both come through a ring of kAccRing stages
 // in shared memory that every thread fills for itself (cp.async), so a dozen loads of each of its 16 warps per SM are in flight without
-// registers for them; two terms a turn, because the sums change registers with every product.  Four tiles, two polynomials from
-// registers with one or two terms ahead: 675 us a launch in the layer pass, 611 in the Q/K/V projections; now 398 and 324.
+// registers for them.  Four tiles, words loaded to registers one or two terms ahead: 675 us a launch in the layer pass, 611 in the Q/K/V
+// projections; now 380 and 305.
 // grid = (N/256, n)
 template <int T> struct TilePts { const u64 *p[T][16]; u64 *out[T]; };
 constexpr int kAccRing = 8;
@@ -1402,22 +1407,25 @@ __global__ void __launch_bounds__(256, 2) k_matmul_acc(const __grid_constant__ T
     const u32 x0 = blockIdx.x * 256 + threadIdx.x;
     const u64 *ring = words + threadIdx.x;
     const u32 ring_at = smem_u32(ring);
-    // what is fetched next: copy k of input b, and the weights' words that meet it
-    int fk = 0, fb = 0, to = 0;
-    u32 src = 0;
+    // what is fetched next: copy fk of input fb, and the weights' words that meet it (past the end the last copy again, which is not used)
+    int fk = 0, fb = 0;
+    u32 to = 0, g = __ldg(gal), src = g == 1 ? x0 : ntt_perm(x0, g, logn);
     const u64 *fa = pre + (size_t)b0 * 2 * poly + limb + x0;
+    const size_t to_next_copy = (size_t)(btotal - bcount + 1) * 2 * poly;
     auto fetch = [&] {
-        if (fk < kcount) {
-            if (fb == 0) { const u32 g = __ldg(gal + fk); src = g == 1 ? x0 : ntt_perm(x0, g, logn); }
-            const u32 r = ring_at + to * (kStage * 8);
-            const u64 *a = fa + (size_t)fb * 2 * poly;
-            cp_async8(r, a); cp_async8(r + 2048, a + poly);
+        const u32 r = ring_at + to;
+        cp_async8(r, fa); cp_async8(r + 2048, fa + poly);
 #pragma unroll
-            for (int t = 0; t < T; ++t) cp_async8(r + (2 + t) * 2048, tp.p[t][fb] + limb + src);
-            if (++fb == bcount) { fb = 0; ++fk; fa += (size_t)btotal * 2 * poly; }
-        }
+        for (int t = 0; t < T; ++t) cp_async8(r + (2 + t) * 2048, tp.p[t][fb] + limb + src);
         cp_async_commit();
-        to = (to + 1) % kAccRing;
+        if (++fb < bcount) fa += 2 * poly;
+        else if (fk + 1 < kcount) {
+            fb = 0; ++fk; fa += to_next_copy;
+            g = __ldg(gal + fk);
+            src = g == 1 ? x0 : ntt_perm(x0, g, logn);
+        } else fb = bcount - 1;
+        to += kStage * 8;
+        if (to == kAccRing * kStage * 8) to = 0; // a stage is no power of two
     };
 #pragma unroll 1
     for (int k = 0; k < kAccRing - 1; ++k) fetch();
@@ -1428,11 +1436,12 @@ __global__ void __launch_bounds__(256, 2) k_matmul_acc(const __grid_constant__ T
 #pragma unroll 2
         for (int k = 0; k < total; ++k) {
             cp_async_wait<kAccRing - 2>();
-            const u64 *q = ring + from * kStage;
+            const u64 *q = ring + from;
             u64 v[2] = {q[0], q[256]}, w[T];
 #pragma unroll
             for (int t = 0; t < T; ++t) w[t] = q[(2 + t) * 256];
-            from = (from + 1) % kAccRing;
+            from += kStage;
+            if (from == kAccRing * kStage) from = 0;
             fetch();
             product(v, w);
         }
@@ -1480,6 +1489,7 @@ __global__ void __launch_bounds__(256, 2) k_matmul_acc(const __grid_constant__ T
 #pragma unroll
         for (int t = 0; t < T; ++t) { r[t][0] = s[t][0].finish(m); r[t][1] = s[t][1].finish(m); }
     }
+    cp_async_wait<0>(); // what was fetched past the end
 #pragma unroll
     for (int t = 0; t < T; ++t) {
         u64 *o = tp.out[t] + limb + x0;
