@@ -218,6 +218,19 @@ class Evaluator {
         for (size_t g = 0; g < ka.size(); ++g) { k1.push_back(ka[g]->raw()); k2.push_back(kb[g] ? kb[g]->raw() : nullptr); }
         hb_ct *o = nullptr; check(c_, hb_assemble_masked_multi(c_, a.raw(), h.raw(), k1.data(), k2.data(), (int)k1.size(), &o)); return Ciphertext(c_, o);
     }
+    // the same into the members first .. of dst
+    void assembleRotationsInto(const Ciphertext &a, const Hoisted &h, const std::vector<const MaskedKey *> &ka, const std::vector<const MaskedKey *> &kb, Ciphertext &dst, int first) const {
+        std::vector<const hb_mkey *> k1, k2;
+        for (size_t g = 0; g < ka.size(); ++g) { k1.push_back(ka[g]->raw()); k2.push_back(kb[g] ? kb[g]->raw() : nullptr); }
+        check(c_, hb_assemble_masked_into(c_, a.raw(), h.raw(), k1.data(), k2.data(), (int)k1.size(), dst.raw(), first));
+    }
+    // members to be written one after the other, and x into the first of them
+    Ciphertext room(int level, int members, const Ciphertext &x) const {
+        hb_ct *o = nullptr; check(c_, hb_ct_create(c_, level, 2, members, 1, &o));
+        Ciphertext r(c_, o);
+        check(c_, hb_batch_set(c_, o, 0, x.raw()));
+        return r;
+    }
     // acc += sum_g tensor(a[g], b[g]) for group-major batches of `groups` groups
     void tensorAccumulateGroups(Ciphertext &acc, const Ciphertext &a, const Ciphertext &b, int groups) const {
         hb_ct *p = acc.release();

@@ -579,18 +579,23 @@ Ciphertext multMatMatPre(Env &e, const CtxtTensor &in, int target_level) {
     const i64 num_rows = in.getHeight();
     const int lvl = target_level + 2;
     CtxtTensor s = diagonalToColumn(e, CtxtTensor(in.getShape(), e.ev.levelDown(in.get(), target_level + 3)));
+    if (e.mode == kLazy) { // a group of copies comes out copy-major, as stack() lays them, so each goes straight to its place
+        const Hoisted h = e.ev.decompose(s.get());
+        const int batch = s.get().getBatch();
+        Ciphertext pre = e.ev.room(s.get().getLevel() - 1, (int)num_rows * batch, e.ev.levelDownOne(s.get()));
+        const i64 group = loop_group(s.get());
+        for (i64 i0 = 1; i0 < num_rows; i0 += group) {
+            std::vector<const MaskedKey *> ka, kb;
+            for (i64 i = i0; i < std::min(num_rows, i0 + group); ++i) {
+                const WrappedCopy w = wrapped_copy(e, false, s.getShape(), i, lvl, i, i - num_rows);
+                ka.push_back(w.main); kb.push_back(w.wrapped);
+            }
+            e.ev.assembleRotationsInto(s.get(), h, ka, kb, pre, (int)i0 * batch);
+        }
+        return pre;
+    }
     std::vector<Ciphertext> copies;
     copies.push_back(e.ev.levelDownOne(s.get()));
-    if (e.mode == kLazy) {
-        const Hoisted h = e.ev.decompose(s.get());
-        const i64 group = loop_group(s.get());
-        for (i64 i0 = 1; i0 < num_rows; i0 += group) { // a group of copies is already laid out copy-major, as stack() lays them
-            std::vector<WrappedCopy> w;
-            for (i64 i = i0; i < std::min(num_rows, i0 + group); ++i) w.push_back(wrapped_copy(e, false, s.getShape(), i, lvl, i, i - num_rows));
-            copies.push_back(assemble_lazy(e, s.get(), h, w));
-        }
-        return e.ev.concat(copies);
-    }
     const TileTensorShape shp = s.getShape();
     if (e.mode >= kDirect) {
         const Hoisted h = e.ev.decompose(s.get());

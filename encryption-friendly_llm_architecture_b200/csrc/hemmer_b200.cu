@@ -620,12 +620,14 @@ const DivPlan *get_div_plan(hb_ctx *c, int level) {
     c->div_plans[level] = d;
     return d;
 }
-// E [batch][2][ne][N] over Q_level u P  ->  new ciphertext at level - 1:  (E - lift(E mod P*q_level)) / (P*q_level)
-hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch) {
+// E [batch][2][ne][N] over Q_level u P  ->  ciphertext at level - 1:  (E - lift(E mod P*q_level)) / (P*q_level), a new one or (dst) the
+// members `first` .. of one that is there
+hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch, hb_ct *dst = nullptr, int first = 0) {
     const DivPlan *dv = get_div_plan(c, level);
     const PlanDims d = plan_dims(c, level);
     const int N = c->N, n = d.n, ne = d.ne, ns = d.K + 1;
-    hb_ct *r = new_ct(c, level - 1, 2, batch, 1);
+    hb_ct *r = dst ? dst : new_ct(c, level - 1, 2, batch, 1);
+    u64 *out = r->d + (size_t)first * 2 * level * N;
     try {
         const unsigned gx1 = (unsigned)((N + 255) / 256), gx = c->gx();
         Tmp t(c, (size_t)batch * 2 * level);
@@ -635,7 +637,7 @@ hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch) {
             const ConvPlan *cv = get_conv_plans(c, level);
             inv_rows(c, src, (size_t)ne * N, src, (size_t)ne * N, batch * 2 * ns, sm);
             launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, batch * 2);
-            const RowsFin f{E, (size_t)ne * N, r->d, (size_t)2 * level * N, 2, 1, 0};
+            const RowsFin f{E, (size_t)ne * N, out, (size_t)2 * level * N, 2, 1, 0};
             LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], NoAddends{}, c->pc, c->tb.t16));
             CK(cudaGetLastError());
             return r;
@@ -644,9 +646,9 @@ hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch) {
         ntt(c, src, (size_t)ne * N, sc.p, (size_t)ns * N, batch * 2 * ns, sm, true);
         LAUNCH(c), k_div_conv<<<dim3(gx1, 1, batch * 2), 256, 0, c->st>>>(t.p, sc.p, dv, c->pc, N);
         ntt_inplace(c, t.p, batch * 2 * level, c->qmap(level - 1), false);
-        LAUNCH(c), k_div_fin<<<dim3(gx, level, batch * 2), 256, 0, c->st>>>(r->d, E, t.p, ne, dv, c->pc, N);
+        LAUNCH(c), k_div_fin<<<dim3(gx, level, batch * 2), 256, 0, c->st>>>(out, E, t.p, ne, dv, c->pc, N);
         CK(cudaGetLastError());
-    } catch (...) { hb_ct_free(r); throw; }
+    } catch (...) { if (!dst) hb_ct_free(r); throw; }
     return r;
 }
 // rescale(p1 (.) rot(a, s1) + p2 (.) rot(a, s2)) from the lifted digits `dt` of a: both inner products stay in
@@ -676,11 +678,14 @@ hb_ct *do_assemble_rot(hb_ctx *c, const hb_ct *a, const u64 *dt, int64_t s1, con
 }
 // the same from keys that already carry the masks (hb_masked_key_create).  `groups` wrapped copies of the same input
 // (each with its own one or two keys: k1s[g], k2s[g] or null) come out of one launch sequence, group-major.
-hb_ct *do_assemble_mk(hb_ctx *c, const hb_ct *a, const u64 *dt, const hb_mkey *const *k1s, const hb_mkey *const *k2s, int groups) {
-    own(c, a);
+hb_ct *do_assemble_mk(hb_ctx *c, const hb_ct *a, const u64 *dt, const hb_mkey *const *k1s, const hb_mkey *const *k2s, int groups, hb_ct *dst = nullptr, int first = 0) {
+    own(c, a, (const hb_ct *)dst);
     if (a->np != 2 || a->spow != 1) fail(HB_E_SHAPE, "assemble: needs a rescaled 2-poly ciphertext");
     if (a->level < 1) fail(HB_E_LEVEL, "assemble: level 0");
     if (groups < 1 || groups > kMaxRotGroups) fail(HB_E_LIMIT, "assemble: 1 to 16 wrapped copies per call");
+    if (dst && (dst->level != a->level - 1 || dst->np != 2 || dst->spow != 1)) fail(HB_E_SHAPE, "assemble: destination of another shape");
+    if (dst && (first < 0 || first > dst->batch || (i64)groups * a->batch > dst->batch - first)) fail(HB_E_SHAPE, "assemble: the destination has no room for the copies");
+    if (dst && a->d < dst->d + dst->limbs() * c->N && dst->d < a->d + a->limbs() * c->N) fail(HB_E_ARG, "assemble: destination and input share memory");
     MaskedRotList mrl{};
     for (int g = 0; g < groups; ++g) {
         MaskedRot &mr = mrl.r[g];
@@ -709,7 +714,7 @@ hb_ct *do_assemble_mk(hb_ctx *c, const hb_ct *a, const u64 *dt, const hb_mkey *c
                               c->pc, c->logn, N);
     }
     CK(cudaGetLastError());
-    return divide_by_p_ql(c, E.p, level, groups * batch);
+    return divide_by_p_ql(c, E.p, level, groups * batch, dst, first);
 }
 
 void check_same(const hb_ct *a, const hb_ct *b, const char *what) {
@@ -1726,6 +1731,13 @@ int hb_assemble_masked_multi(hb_ctx *c, const hb_ct *a, const hb_digits *dg, con
         if (a->np != 2 || dg->level != a->level || dg->batch != a->batch) fail(HB_E_SHAPE, "assemble_masked: digits do not belong to this ciphertext");
         if (!k1s) fail(HB_E_ARG, "assemble_masked: no keys");
         *out = do_assemble_mk(c, a, dg->d, k1s, k2s, groups);
+    });
+}
+int hb_assemble_masked_into(hb_ctx *c, const hb_ct *a, const hb_digits *dg, const hb_mkey *const *k1s, const hb_mkey *const *k2s, int groups, hb_ct *dst, int first) {
+    return guard(c, [&] {
+        if (a->np != 2 || dg->level != a->level || dg->batch != a->batch) fail(HB_E_SHAPE, "assemble_masked: digits do not belong to this ciphertext");
+        if (!k1s || !dst) fail(HB_E_ARG, "assemble_masked: no keys or no destination");
+        do_assemble_mk(c, a, dg->d, k1s, k2s, groups, dst, first);
     });
 }
 int hb_tensor_acc_groups(hb_ctx *c, const hb_ct *a, const hb_ct *b, int groups, hb_ct **acc) { return guard(c, [&] { *acc = do_tensor(c, a, b, *acc, groups); }); }

@@ -228,6 +228,9 @@ int hb_assemble_masked(hb_ctx *ctx, const hb_ct *a, const hb_digits *digits, con
  * for batches too small to fill the GPU on their own. */
 int hb_assemble_masked_multi(hb_ctx *ctx, const hb_ct *a, const hb_digits *digits, const hb_mkey *const *k1s, const hb_mkey *const *k2s,
                              int groups, hb_ct **out);
+/* the same into the members first .. first + groups * batch(a) - 1 of a ciphertext that is there (two polynomials, level(a) - 1) */
+int hb_assemble_masked_into(hb_ctx *ctx, const hb_ct *a, const hb_digits *digits, const hb_mkey *const *k1s, const hb_mkey *const *k2s,
+                            int groups, hb_ct *dst, int first);
 /* raw forward / inverse NTT of every limb of the batch, in place (primitive sweep) */
 int hb_ntt(hb_ctx *ctx, hb_ct *a, int inverse);
 

@@ -142,3 +142,26 @@ def test_tensor_of_halves(pkg, g, batch):
     _same(g.ct_export(pkg.capi.Handle(g, got, "ct")), g.ct_export(pkg.capi.Handle(g, want, "ct")), "accumulated")
     odd, out = _ct(g, 3, 5), C.c_void_p()
     assert g.dll.hb_tensor_acc_halves(g.ctx, odd.ptr, C.byref(out)) != 0 and not out.value
+
+
+@pytest.mark.parametrize("groups,batch,first", [(1, 1, 0), (3, 2, 1), (16, 1, 4)])
+def test_wrapped_copies_into_a_ciphertext_that_is_there(pkg, g, groups, batch, first):
+    """The members asked for get what the call with a result of its own gives; the others stay as they were."""
+    x = _ct(g, batch, 61)
+    digits = g.decompose(x)
+    m = (np.random.default_rng(3).uniform(0, 1, g.slots) > 0.5).astype(np.float64)
+    g.gen_rot_keys([1, -2])
+    k1, k2 = g.masked_key(1, g.encode_ext(m, LEVEL)), g.masked_key(-2, g.encode_ext(1 - m, LEVEL))
+    keys, wrapped = _ptrs([k1] * groups), _ptrs([k2 if k % 2 else None for k in range(groups)])
+    want = g.ct_export(_call(pkg, g, "assemble_masked_multi", x, digits, keys, wrapped, C.c_int(groups)))
+    dst = _ct(g, first + groups * batch + 1, 62, level=LEVEL - 1)
+    before = g.ct_export(dst)
+    into = lambda d, at, n=groups: g._chk(g._fn("assemble_masked_into")(g.ctx, x.ptr, digits.ptr, keys, wrapped, C.c_int(n), d.ptr, C.c_int(at)))
+    into(dst, first)
+    after = g.ct_export(dst)
+    _same(after[first:first + groups * batch], want, "the copies")
+    _same(after[:first], before[:first], "members before")
+    _same(after[first + groups * batch:], before[first + groups * batch:], "members after")
+    for bad in (lambda: into(dst, first + 2), lambda: into(dst, -1), lambda: into(dst, 2**31 - 1), lambda: into(x, 0), lambda: into(dst, 0, 0), lambda: into(dst, 0, 17)):
+        with pytest.raises(pkg.HBError):
+            bad()
