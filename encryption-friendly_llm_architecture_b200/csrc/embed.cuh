@@ -14,7 +14,7 @@
 // takes the sixteen rows that agree in their low four bits, whose images are runs of sixteen coefficients.
 // Bound by latency (16 CTAs of 128 threads a member): for eight members 7 and 14 us to encode, 40 and 35 us to decode, where the
 // host cores took 2.0 and 1.8 ms a member for the same transforms and 2.8 and 1.4 ms for sampling and CRT lift.  Thirteen messages
-// from host memory to ciphertexts 7.1 -> 1.8 ms, thirteen ciphertexts to host memory 5.6 -> 0.8 ms, of which the copies are a half.
+// from host memory to ciphertexts 7.1 -> 0.68 ms, thirteen ciphertexts to host memory 5.6 -> 0.6 ms; the copies are most of both.
 #pragma once
 #include "modarith.cuh"
 #include "kernels.cuh"

@@ -125,9 +125,11 @@ struct hb_ctx {
     InvScale p_inv_scale{};               // 2^16 rings: P^-1 mod q_l
     std::map<int, InvScale> div_scale;    // (P * q_level)^-1 mod q_l per level
     bool smem_opt_in_conv = false, smem_opt_in_acc = false;
-    // slot values on their way between the caller's memory and the device: two pinned buffers a direction, with the events of their last copies
-    double *up[2] = {nullptr, nullptr}, *down[2] = {nullptr, nullptr};
-    cudaEvent_t went_up[2] = {nullptr, nullptr}, came_down[2] = {nullptr, nullptr};
+    // slot values on their way between the caller's memory and the device: two pinned buffers a direction, with the events of their last
+    // copies.  Messages go up on a stream of their own, beside the kernels of the chunk before, into two buffers on the device.
+    double *up[2] = {nullptr, nullptr}, *down[2] = {nullptr, nullptr}, *up_dev[2] = {nullptr, nullptr};
+    cudaEvent_t went_up[2] = {nullptr, nullptr}, up_read[2] = {nullptr, nullptr}, came_down[2] = {nullptr, nullptr};
+    cudaStream_t up_st = nullptr;
     double2 *emb = nullptr;               // twiddles of the embedding, inverse then forward
     u64 *cdt = nullptr;                   // table of the discrete Gaussian
     EmbedTables emb_tb{};
@@ -985,17 +987,28 @@ u64 *noalloc_scratch(int device) {
 }
 
 // ---- slot values between the caller's memory and the device ----
-// Messages travel in chunks of kStageMembers through two pinned buffers, so that moving one chunk in host memory overlaps the copy and
-// the transforms of the other.  The caller's pages are often new ones, whose first touch costs more than the bytes: several threads.
-constexpr int kStageMembers = 8, kCopyThreads = 4;
-size_t stage_words(const hb_ctx *c) { return (size_t)kStageMembers * c->N; } // two doubles per slot
+// Values travel in chunks through two pinned buffers a direction, so that moving one chunk in host memory overlaps the copy and the
+// transforms of the other.  The caller's pages are often new ones, whose first touch costs more than the bytes: several threads.
+// Going up, chunks of four members: the copies (6 to 8 GB/s here) take as long as the kernels, and only that of the first is not covered
+// (thirteen messages 1.03 ms with chunks of eight on the kernels' stream, 0.93 with a stream of their own, 0.68 in chunks of four).
+// Coming down, eight: the kernels are short, and neither a stream of its own nor chunks of four made a difference.
+constexpr int kStageMembers = 8, kUpMembers = 4, kCopyThreads = 4;
+size_t stage_words(const hb_ctx *c, int members) { return (size_t)members * c->N; } // two doubles per slot
 // Two buffers and their events.  Those of messages are write-combined: the host only writes them, and the copy engine need not ask its caches.
-void stage_open(hb_ctx *c, double *(&buf)[2], cudaEvent_t (&ev)[2], unsigned flags) {
+void stage_open(hb_ctx *c, double *(&buf)[2], cudaEvent_t (&ev)[2], int members, unsigned flags) {
     if (buf[0]) return;
     for (cudaEvent_t &e : ev) if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     double *p = nullptr;
-    CK(cudaHostAlloc(&p, 2 * stage_words(c) * sizeof(double), flags));
-    buf[0] = p; buf[1] = p + stage_words(c);
+    CK(cudaHostAlloc(&p, 2 * stage_words(c, members) * sizeof(double), flags));
+    buf[0] = p; buf[1] = p + stage_words(c, members);
+}
+void up_open(hb_ctx *c) {
+    if (!c->up_st) CK(cudaStreamCreateWithFlags(&c->up_st, cudaStreamNonBlocking));
+    for (int i = 0; i < 2; ++i) {
+        if (!c->up_read[i]) CK(cudaEventCreateWithFlags(&c->up_read[i], cudaEventDisableTiming));
+        if (!c->up_dev[i]) CK(cudaMalloc(&c->up_dev[i], stage_words(c, kUpMembers) * sizeof(double)));
+    }
+    stage_open(c, c->up, c->went_up, kUpMembers, cudaHostAllocWriteCombined);
 }
 // work(begin, end) over [0, n) on up to kCopyThreads threads, `words` doubles moved in all
 template <class F> void in_threads(const hb_ctx *c, size_t n, size_t words, F &&work) {
@@ -1017,9 +1030,13 @@ void host_copy(const hb_ctx *c, double *dst, const double *src, size_t words) {
 void embed_inverse(hb_ctx *c, i64 *coef, const double *re, const double *im, int n, int count, double sc) {
     if (c->logn == 16) {
         Tmp v(c, (size_t)count);
-        launch(c, k_embed_inv_cols, dim3(16, (unsigned)count), kEmbThreads, 0, (double2 *)v.p, re, im, n, c->emb_tb);
+        LAUNCH(c), k_embed_inv_cols<<<dim3(16, (unsigned)count), kEmbThreads, 0, c->st>>>((double2 *)v.p, re, im, n, c->emb_tb); // comes after a copy, not after a kernel
+        CK(cudaPeekAtLastError());
         launch(c, k_embed_inv_rows, dim3(16, (unsigned)count), kEmbThreads, 0, coef, (const double2 *)v.p, sc, c->emb_tb);
-    } else launch(c, k_embed_inv_small, dim3((unsigned)count), 256, 0, coef, re, im, n, c->logn - 1, sc, c->emb_tb);
+    } else {
+        LAUNCH(c), k_embed_inv_small<<<dim3((unsigned)count), 256, 0, c->st>>>(coef, re, im, n, c->logn - 1, sc, c->emb_tb);
+        CK(cudaPeekAtLastError());
+    }
 }
 // slot values of the residues t [count][2][N]: member b, slot s at re[(b * slots + s) * stride], im likewise
 void embed_forward(hb_ctx *c, double *re, double *im, int stride, const u64 *t, const DecItem *items, int count) {
@@ -1033,17 +1050,20 @@ void embed_forward(hb_ctx *c, double *re, double *im, int stride, const u64 *t, 
 // after all of those; use(first member, members, coefficients on the device) takes them on.  Nothing of the caller's memory is needed
 // once this has returned; the device may still be at work.
 template <class FILL, class USE> void encode_chunks(hb_ctx *c, size_t n, bool cplx, int count, double sc, FILL &&fill, USE &&use) {
-    stage_open(c, c->up, c->went_up, cudaHostAllocWriteCombined);
-    for (int first = 0, slot = 0; first < count; first += kStageMembers, slot ^= 1) {
-        const int m = std::min(kStageMembers, count - first);
+    up_open(c);
+    for (int first = 0, slot = 0; first < count; first += kUpMembers, slot ^= 1) {
+        const int m = std::min(kUpMembers, count - first);
         const size_t words = (size_t)m * n, bytes = words * (cplx ? 2 : 1) * sizeof(double);
-        CK(cudaEventSynchronize(c->went_up[slot])); // its last copy has been made
+        CK(cudaEventSynchronize(c->went_up[slot])); // the pinned buffer's last copy has been made
         fill(first, m, c->up[slot]);
-        TmpBytes d(c, std::max<size_t>(1, bytes)), coef(c, (size_t)m * c->N * sizeof(i64));
-        double *dr = (double *)d.p;
-        CK(cudaMemcpyAsync(dr, c->up[slot], bytes, cudaMemcpyHostToDevice, c->st));
-        CK(cudaEventRecord(c->went_up[slot], c->st));
-        embed_inverse(c, (i64 *)coef.p, dr, cplx ? dr + words : nullptr, (int)n, m, sc);
+        double *d = c->up_dev[slot];
+        CK(cudaStreamWaitEvent(c->up_st, c->up_read[slot], 0)); // and its counterpart's last contents have been read
+        CK(cudaMemcpyAsync(d, c->up[slot], bytes, cudaMemcpyHostToDevice, c->up_st));
+        CK(cudaEventRecord(c->went_up[slot], c->up_st));
+        CK(cudaStreamWaitEvent(c->st, c->went_up[slot], 0));
+        TmpBytes coef(c, (size_t)m * c->N * sizeof(i64));
+        embed_inverse(c, (i64 *)coef.p, d, cplx ? d + words : nullptr, (int)n, m, sc);
+        CK(cudaEventRecord(c->up_read[slot], c->st));
         use(first, m, (const i64 *)coef.p);
     }
 }
@@ -1057,7 +1077,7 @@ auto from_arrays(hb_ctx *c, const double *re, const double *im, size_t n) {
 // Decrypts and decodes `count` items into host memory: member i at re[i * slots], im likewise (im may be null); or, z, as complex values
 // at re[2 * i * slots].
 void decrypt_items(hb_ctx *c, const std::vector<DecItem> &items, bool z, double *re, double *im) {
-    stage_open(c, c->down, c->came_down, cudaHostAllocDefault);
+    stage_open(c, c->down, c->came_down, kStageMembers, cudaHostAllocDefault);
     const int count = (int)items.size(), N = c->N, slots = N / 2;
     TmpBytes list(c, items.size() * sizeof(DecItem));
     CK(cudaMemcpyAsync(list.p, items.data(), items.size() * sizeof(DecItem), cudaMemcpyHostToDevice, c->st));
@@ -1095,7 +1115,7 @@ template <class FILL> hb_ct *encrypt_messages(hb_ctx *c, size_t n_slots, bool cp
         const LimbMap qm = c->qmap(level);
         TmpBytes ids(c, (size_t)count * 8);
         CK(cudaMemcpyAsync(ids.p, nonces, (size_t)count * 8, cudaMemcpyHostToDevice, c->st));
-        Tmp me(c, (size_t)std::min(count, kStageMembers) * n); // message + error; NTT form is linear, one transform serves both
+        Tmp me(c, (size_t)std::min(count, kUpMembers) * n); // message + error; NTT form is linear, one transform serves both
         encode_chunks(c, n_slots, cplx, count, c->h->scale[level], fill, [&](int first, int m, const i64 *coef) {
             const u64 *id = (const u64 *)ids.p + first;
             error_residues(c, me.p, coef, StreamIds{c->ckey, hbhost::STREAM_ENC_E, id, 0}, m, qm);
@@ -1237,13 +1257,16 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
 void hb_ctx_destroy(hb_ctx *c) {
     if (!c) return;
     cudaSetDevice(c->device);
+    if (c->up_st) cudaStreamSynchronize(c->up_st);
     if (c->st) cudaStreamSynchronize(c->st);
     for (auto &kv : c->plans) cudaFree(kv.second);
     for (auto &kv : c->div_plans) cudaFree(kv.second);
     for (auto &kv : c->conv_plans) cudaFree(kv.second);
     for (auto &kv : c->gal_tables) cudaFree(kv.second);
     for (double *p : {c->up[0], c->down[0]}) if (p) cudaFreeHost(p);
-    for (cudaEvent_t e : {c->went_up[0], c->went_up[1], c->came_down[0], c->came_down[1]}) if (e) cudaEventDestroy(e);
+    for (double *p : c->up_dev) if (p) cudaFree(p);
+    for (cudaEvent_t e : {c->went_up[0], c->went_up[1], c->up_read[0], c->up_read[1], c->came_down[0], c->came_down[1]}) if (e) cudaEventDestroy(e);
+    if (c->up_st) cudaStreamDestroy(c->up_st);
     if (c->emb) cudaFree(c->emb);
     if (c->cdt) cudaFree(c->cdt);
     if (c->pc) cudaFree(c->pc);

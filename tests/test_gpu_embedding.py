@@ -1,6 +1,6 @@
 """Encoding, sampling, encryption and decryption on the device against the oracle, whose embedding, error polynomials and CRT lift are
-host code with the same sequence of IEEE operations: residues and decoded values are compared bit for bit.  Members travel in chunks
-of eight through two buffers, so batches lie on both sides of one, two and three chunks."""
+host code with the same sequence of IEEE operations: residues and decoded values are compared bit for bit.  Messages go up in
+chunks of four and values come down in chunks of eight, through two buffers each, so batches lie on both sides of one to five chunks."""
 import numpy as np
 import pytest
 
