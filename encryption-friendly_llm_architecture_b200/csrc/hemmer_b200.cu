@@ -1006,7 +1006,12 @@ void up_open(hb_ctx *c) {
     if (!c->up_st) CK(cudaStreamCreateWithFlags(&c->up_st, cudaStreamNonBlocking));
     for (int i = 0; i < 2; ++i) {
         if (!c->up_read[i]) CK(cudaEventCreateWithFlags(&c->up_read[i], cudaEventDisableTiming));
-        if (!c->up_dev[i]) CK(cudaMalloc(&c->up_dev[i], stage_words(c, kUpMembers) * sizeof(double)));
+        if (c->up_dev[i]) continue;
+        const size_t bytes = stage_words(c, kUpMembers) * sizeof(double);
+        if (cudaMalloc(&c->up_dev[i], bytes) == cudaSuccess) continue;
+        cudaGetLastError();
+        c->pool.release_cached(); // the pool's idle buffers may hold what is left of the memory
+        CK(cudaMalloc(&c->up_dev[i], bytes));
     }
     stage_open(c, c->up, c->went_up, kUpMembers, cudaHostAllocWriteCombined);
 }
