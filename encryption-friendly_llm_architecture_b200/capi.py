@@ -167,7 +167,7 @@ class Lib:
         """encrypt_many for messages given as lists of real tiles that lie side by side."""
         tiles = [[np.ascontiguousarray(np.asarray(t).real, dtype=np.float64) for t in g] for g in groups]
         rows, cols = tiles[0][0].shape
-        if not self.has("encrypt_tiles") or rows * cols == 0 or any(t.shape != (rows, cols) for g in tiles for t in g):
+        if not self.has("encrypt_tiles") or rows * cols == 0 or any(len(g) != len(tiles[0]) or any(t.shape != (rows, cols) for t in g) for g in tiles):
             msgs = np.zeros((len(tiles), self.slots))
             for m, g in zip(msgs, tiles):
                 np.concatenate(g, axis=1, out=m[: sum(t.size for t in g)].reshape(g[0].shape[0], sum(t.shape[1] for t in g)))

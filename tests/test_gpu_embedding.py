@@ -96,3 +96,9 @@ def test_tiles_that_are_refused_or_take_the_general_path(pkg, gpu_small):
     a, b = np.ones((4, 3)), np.ones((4, 5))
     assert np.array_equal(g.ct_export(g.encrypt_tiles([[a, b]], 2, [9])), g.ct_export(g.encrypt_many(np.ones((1, 32)), 2, [9])))
     assert np.array_equal(g.ct_export(g.encrypt_tiles([[np.zeros((0, 4))]], 2, [9])), g.ct_export(g.encrypt_many(np.zeros((1, 4)), 2, [9])))
+    rng = np.random.default_rng(6)
+    uneven = [[rng.uniform(-1, 1, (8, 8)) for _ in range(k)] for k in (2, 1, 3)]  # as many tiles as three messages of two
+    msgs = np.zeros((3, g.slots))
+    for m, t in zip(msgs, uneven):
+        m[:64 * len(t)] = np.concatenate(t, axis=1).reshape(-1)
+    assert np.array_equal(g.ct_export(g.encrypt_tiles(uneven, 2, [4, 5, 6])), g.ct_export(g.encrypt_many(msgs, 2, [4, 5, 6])))

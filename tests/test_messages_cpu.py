@@ -1,0 +1,54 @@
+"""How messages that are given as tiles reach the native library, on the CPU: a stand-in for its entry points that keeps what each call hands
+over, and the oracle's library, which has no entry point for tiles."""
+import ctypes as C
+import importlib
+
+import numpy as np
+import pytest
+
+SLOTS = 64
+
+
+class Recorder:
+    """Entry points encrypt_tiles and encrypt_many of a library, as the messages [count][SLOTS] that the call would encrypt."""
+
+    def __init__(self, capi):
+        self.lib = capi.Lib.__new__(capi.Lib)
+        self.lib.slots, self.lib.L, self.lib.ctx = SLOTS, 3, None
+        self.lib.has = lambda name: True
+        self.lib._fn = lambda name: getattr(self, name, lambda *a: 0)
+        self.called = self.messages = None
+
+    @staticmethod
+    def _row(parts):
+        m = np.zeros(SLOTS)
+        flat = np.concatenate(parts, axis=1).reshape(-1)
+        m[:flat.size] = flat
+        return m
+
+    def encrypt_tiles(self, ctx, ptr, across, rows, cols, count, level, nonces, out):
+        across, rows, cols = across.value, rows.value, cols.value
+        tile = lambda p: np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_double)), (rows, cols)).copy()
+        self.called = "encrypt_tiles"
+        self.messages = np.stack([self._row([tile(ptr[i * across + t]) for t in range(across)]) for i in range(count.value)])
+        return 0
+
+    def encrypt_many(self, ctx, re, im, n, count, level, nonces, out):
+        self.called = "encrypt_many"
+        self.messages = np.ctypeslib.as_array(C.cast(re, C.POINTER(C.c_double)), (count.value, n.value)).copy()
+        return 0
+
+
+@pytest.fixture
+def rec(pkg):
+    return Recorder(importlib.import_module(pkg.__name__ + ".capi"))
+
+
+@pytest.mark.parametrize("groups", [(2, 2), (2, 1, 3), (1, 2), (2, 1), (3, 1, 2)])
+def test_every_message_keeps_its_own_tiles(rec, groups):
+    """Groups of as many tiles each go to the tile entry point, uneven ones are laid out: two tiles, one, three."""
+    rng = np.random.default_rng(len(groups))
+    tiles = [[rng.uniform(-1, 1, (3, 4)) for _ in range(n)] for n in groups]
+    rec.lib.encrypt_tiles(tiles, 2, range(len(groups)))
+    assert np.array_equal(rec.messages, np.stack([Recorder._row(g) for g in tiles]))
+    assert rec.called == ("encrypt_tiles" if len(set(groups)) == 1 else "encrypt_many")
