@@ -166,13 +166,14 @@ class Lib:
     def encrypt_tiles(self, groups, level, nonces):
         """encrypt_many for messages given as lists of real tiles that lie side by side."""
         tiles = [[np.ascontiguousarray(np.asarray(t).real, dtype=np.float64) for t in g] for g in groups]
-        rows, cols = tiles[0][0].shape
-        if not self.has("encrypt_tiles") or rows * cols == 0 or any(len(g) != len(tiles[0]) or any(t.shape != (rows, cols) for t in g) for g in tiles):
+        shape = tiles[0][0].shape
+        if not self.has("encrypt_tiles") or len(shape) != 2 or 0 in shape or any(len(g) != len(tiles[0]) or any(t.shape != shape for t in g) for g in tiles):
             msgs = np.zeros((len(tiles), self.slots))
             for m, g in zip(msgs, tiles):
-                np.concatenate(g, axis=1, out=m[: sum(t.size for t in g)].reshape(g[0].shape[0], sum(t.shape[1] for t in g)))
+                flat = np.concatenate(g, axis=1).reshape(-1)
+                m[: flat.size] = flat
             return self.encrypt_many(msgs, level, nonces)
-        n, across = len(tiles), len(tiles[0])
+        (rows, cols), n, across = shape, len(tiles), len(tiles[0])
         ptr = (C.c_void_p * (n * across))(*[t.ctypes.data for g in tiles for t in g])
         nn = (C.c_uint64 * n)(*[int(k) for k in nonces])
         out = C.c_void_p()

@@ -52,3 +52,15 @@ def test_every_message_keeps_its_own_tiles(rec, groups):
     rec.lib.encrypt_tiles(tiles, 2, range(len(groups)))
     assert np.array_equal(rec.messages, np.stack([Recorder._row(g) for g in tiles]))
     assert rec.called == ("encrypt_tiles" if len(set(groups)) == 1 else "encrypt_many")
+
+
+def test_tiles_of_other_forms_are_laid_out(rec):
+    """Tiles of unequal width, and stacks of matrices, whose second axis they are joined on."""
+    a, b, c = np.ones((4, 3)), np.full((4, 5), 2.0), np.arange(24.0).reshape(2, 3, 4)
+    rec.lib.encrypt_tiles([[a, b]], 2, [1])
+    assert np.array_equal(rec.messages, Recorder._row([a, b])[None])
+    rec.lib.encrypt_tiles([[c, -c]], 2, [1])
+    assert np.array_equal(rec.messages, Recorder._row([c, -c])[None])
+    for bad in ([[]], [[a], []], [[np.ones(4)]], [[a, np.ones((3, 3))]], [[np.ones((8, 5)), np.ones((8, 4))]]):
+        with pytest.raises((ValueError, IndexError)):
+            rec.lib.encrypt_tiles(bad, 2, range(len(bad)))
