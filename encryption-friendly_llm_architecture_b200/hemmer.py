@@ -169,7 +169,7 @@ class Hemmer:
     def encrypt2_many(self, pairs, nonces):
         """encrypt2 for a list of (left, right) tile pairs: one batched CtxtTensor, member i = encrypt2(*pairs[i], nonces[i])."""
         d = pairs[0][0].shape
-        return CtxtTensor(self.lib.encrypt_tiles(pairs, self.lib.L, nonces), d[0], d[1], 2 * d[1])
+        return CtxtTensor(self.lib.encrypt_tiles([(a, b) for a, b in pairs], self.lib.L, nonces), d[0], d[1], 2 * d[1])
 
     def decrypt(self, t):
         fn = self._native("decrypt")

@@ -64,3 +64,22 @@ def test_tiles_of_other_forms_are_laid_out(rec):
     for bad in ([[]], [[a], []], [[np.ones(4)]], [[a, np.ones((3, 3))]], [[np.ones((8, 5)), np.ones((8, 4))]]):
         with pytest.raises((ValueError, IndexError)):
             rec.lib.encrypt_tiles(bad, 2, range(len(bad)))
+
+
+def test_encrypt2_many_takes_pairs_only(pkg, rec):
+    """Lists, tuples, arrays and iterators of two tiles; three or one are refused before anything is encrypted."""
+    hemmer = importlib.import_module(pkg.__name__ + ".hemmer")
+    H = hemmer.Hemmer.__new__(hemmer.Hemmer)
+    H.lib = rec.lib
+    rng = np.random.default_rng(4)
+    a = [rng.uniform(-1, 1, (3, 4)) for _ in range(6)]
+    got = H.encrypt2_many([(a[0], a[1]), [a[2], a[3]], iter((a[4], a[5]))], [1, 2, 3])
+    assert got.shape == (3, 4, 8)
+    assert np.array_equal(rec.messages, np.stack([Recorder._row([a[k], a[k + 1]]) for k in (0, 2, 4)]))
+    H.encrypt2_many(np.stack(a[:2])[None], [1])
+    assert np.array_equal(rec.messages, Recorder._row(a[:2])[None])
+    rec.called = None
+    for bad in ([a[:3]], [a[:1]], [a[:2], a[:3]], [a[:2], a[2:3], a[3:6]]):
+        with pytest.raises(ValueError):
+            H.encrypt2_many(bad, range(len(bad)))
+    assert rec.called is None
