@@ -39,6 +39,13 @@ class HBError(RuntimeError):
         self.code = code
 
 
+def _nonces(nonces, count):
+    nonces = [int(k) for k in nonces]
+    if len(nonces) != count:
+        raise ValueError(f"{count} messages, {len(nonces)} nonces")
+    return nonces
+
+
 def _f64(a):
     return None if a is None else a.ctypes.data_as(c_f64p)
 
@@ -153,12 +160,12 @@ class Lib:
     def encrypt_many(self, msgs, level, nonces):
         """Encode + encrypt the rows of `msgs` ([count][slots], real or complex) into one batched handle."""
         msgs = np.asarray(msgs)
-        n = msgs.shape[0]
+        n, nonces = msgs.shape[0], _nonces(nonces, msgs.shape[0])
         if not self.has("encrypt_many"):  # a library without the batched entry point: one call per member
             return self.batch_concat([self.encrypt(self.encode(m, level), k) for m, k in zip(msgs, nonces)])
         re = np.ascontiguousarray(msgs.real, dtype=np.float64)
         im = np.ascontiguousarray(msgs.imag, dtype=np.float64) if np.iscomplexobj(msgs) else None
-        nn = (C.c_uint64 * n)(*[int(k) for k in nonces])
+        nn = (C.c_uint64 * n)(*nonces)
         out = C.c_void_p()
         self._chk(self._fn("encrypt_many")(self.ctx, _f64(re), _f64(im), C.c_size_t(msgs.shape[1]), C.c_int(n), C.c_int(level), nn, C.byref(out)))
         return Handle(self, out, "ct")
@@ -166,6 +173,7 @@ class Lib:
     def encrypt_tiles(self, groups, level, nonces):
         """encrypt_many for messages given as lists of real tiles that lie side by side."""
         tiles = [[np.ascontiguousarray(np.asarray(t).real, dtype=np.float64) for t in g] for g in groups]
+        nonces = _nonces(nonces, len(tiles))
         shape = tiles[0][0].shape
         if not self.has("encrypt_tiles") or len(shape) != 2 or 0 in shape or any(len(g) != len(tiles[0]) or any(t.shape != shape for t in g) for g in tiles):
             msgs = np.zeros((len(tiles), self.slots))
@@ -175,7 +183,7 @@ class Lib:
             return self.encrypt_many(msgs, level, nonces)
         (rows, cols), n, across = shape, len(tiles), len(tiles[0])
         ptr = (C.c_void_p * (n * across))(*[t.ctypes.data for g in tiles for t in g])
-        nn = (C.c_uint64 * n)(*[int(k) for k in nonces])
+        nn = (C.c_uint64 * n)(*nonces)
         out = C.c_void_p()
         self._chk(self._fn("encrypt_tiles")(self.ctx, ptr, C.c_int(across), C.c_int(rows), C.c_int(cols), C.c_int(n), C.c_int(level), nn, C.byref(out)))
         return Handle(self, out, "ct")

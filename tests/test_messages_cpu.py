@@ -83,3 +83,19 @@ def test_encrypt2_many_takes_pairs_only(pkg, rec):
         with pytest.raises(ValueError):
             H.encrypt2_many(bad, range(len(bad)))
     assert rec.called is None
+
+
+def test_one_nonce_a_message(rec, orc_small):
+    """Missing nonces were zeros: messages under one nonce share their randomness, and the difference of the ciphertexts gives that of the messages."""
+    msgs = np.random.default_rng(5).uniform(-1, 1, (3, 16))
+    tiles = [[m.reshape(4, 4)] for m in msgs]
+    for lib in (rec.lib, orc_small):
+        for nonces in ([], [7, 8], [7, 8, 9, 10], range(2)):
+            with pytest.raises(ValueError):
+                lib.encrypt_many(msgs, 2, nonces)
+            with pytest.raises(ValueError):
+                lib.encrypt_tiles(tiles, 2, nonces)
+    assert rec.called is None
+    want = [orc_small.ct_export(orc_small.encrypt(orc_small.encode(m, 2), k)) for m, k in zip(msgs, (7, 8, 9))]
+    for got in (orc_small.encrypt_many(msgs, 2, iter((7, 8, 9))), orc_small.encrypt_tiles(tiles, 2, np.arange(7, 10))):
+        assert np.array_equal(orc_small.ct_export(got), np.concatenate(want))
