@@ -8,6 +8,7 @@
 #include "ntt.cuh"
 #include "convcols.cuh"
 #include "embed.cuh"
+#include "pool.hpp"
 
 #include <cstdio>
 #include <dlfcn.h>
@@ -27,41 +28,6 @@ namespace {
 
 struct CudaFail { cudaError_t e; const char *where; };
 #define CK(x) do { cudaError_t e__ = (x); if (e__ != cudaSuccess) throw CudaFail{e__, #x}; } while (0)
-struct ArgFail { int code; std::string msg; };
-[[noreturn]] void fail(int code, const std::string &m) { throw ArgFail{code, m}; }
-
-// Size-bucketed caching allocator: the matmul schedules allocate and free the same few buffer
-// sizes thousands of times; cudaMalloc is reached only the first time a size is seen.
-struct Pool {
-    std::unordered_map<size_t, std::vector<void *>> free_;
-    std::unordered_map<void *, size_t> live_;
-    size_t total = 0, in_use = 0;
-    void *get(size_t bytes) {
-        bytes = (bytes + 255) & ~(size_t)255;
-        auto &v = free_[bytes];
-        void *p = nullptr;
-        if (!v.empty()) { p = v.back(); v.pop_back(); }
-        else {
-            cudaError_t e = cudaMalloc(&p, bytes);
-            if (e != cudaSuccess) { cudaGetLastError(); release_cached(); e = cudaMalloc(&p, bytes); } // the first failure must not stay behind as the last error
-            if (e != cudaSuccess) { cudaGetLastError(); fail(HB_E_OOM, "device allocation of " + std::to_string(bytes) + " bytes failed"); }
-            total += bytes;
-        }
-        live_[p] = bytes; in_use += bytes;
-        return p;
-    }
-    void put(void *p) {
-        if (!p) return;
-        auto it = live_.find(p);
-        if (it == live_.end()) return;
-        free_[it->second].push_back(p); in_use -= it->second; live_.erase(it);
-    }
-    void release_cached() {
-        for (auto &kv : free_) { for (void *p : kv.second) { cudaFree(p); total -= kv.first; } kv.second.clear(); }
-    }
-    ~Pool() { release_cached(); for (auto &kv : live_) cudaFree(kv.first); }
-};
-
 struct Evk { u64 *d = nullptr; int nd = 0; };
 
 // NCCL is bound at first use instead of at link time: a process that also loads PyTorch must use the
@@ -138,6 +104,7 @@ struct hb_ctx {
     std::map<std::pair<int, long long>, u32 *> gal_tables; // (copies, row_step) -> Galois elements of hb_matmul_acc, on the device
     int host_threads = 0;                                 // cap for the threads that move slot values in host memory (0: no cap beyond kCopyThreads)
     bool capturing = false;                               // between hb_graph_begin and hb_graph_end
+    Pool::Buffers recorded;                               // what the pool handed out in between
     unsigned long long launches_at_capture = 0, alg_at_capture = 0;
     int N = 0, logn = 0, L = 0, K = 0, nprimes = 0;
     unsigned long long launches = 0; // kernels launched by this context
@@ -1006,12 +973,7 @@ void up_open(hb_ctx *c) {
     if (!c->up_st) CK(cudaStreamCreateWithFlags(&c->up_st, cudaStreamNonBlocking));
     for (int i = 0; i < 2; ++i) {
         if (!c->up_read[i]) CK(cudaEventCreateWithFlags(&c->up_read[i], cudaEventDisableTiming));
-        if (c->up_dev[i]) continue;
-        const size_t bytes = stage_words(c, kUpMembers) * sizeof(double);
-        if (cudaMalloc(&c->up_dev[i], bytes) == cudaSuccess) continue;
-        cudaGetLastError();
-        c->pool.release_cached(); // the pool's idle buffers may hold what is left of the memory
-        CK(cudaMalloc(&c->up_dev[i], bytes));
+        if (!c->up_dev[i]) c->up_dev[i] = (double *)c->pool.raw(stage_words(c, kUpMembers) * sizeof(double));
     }
     stage_open(c, c->up, c->went_up, kUpMembers, cudaHostAllocWriteCombined);
 }
@@ -2240,12 +2202,15 @@ int hb_set_host_threads(hb_ctx *c, int n) { if (!c || n < 0) return HB_E_ARG; c-
 // it replays the graph (every replay writes the results into those same buffers).  Everything the pass needs that is
 // made on first use -- rotation keys, plans, masks, masked keys, Galois tables, pool buffers -- must exist already:
 // run the pass once before recording it.  Calls that copy to or from the host are refused while recording.
-struct hb_graph { hb_ctx *ctx; cudaGraph_t g; cudaGraphExec_t e; unsigned long long kernels, alg_limbs; };
+// The buffers that were handed out meanwhile stay allocated as long as the graph, whatever asks the pool for its idle ones.
+struct hb_graph { hb_ctx *ctx; cudaGraph_t g; cudaGraphExec_t e; unsigned long long kernels, alg_limbs; Pool::Buffers buffers; };
 int hb_graph_begin(hb_ctx *c) {
     return guard(c, [&] {
         if (c->capturing) fail(HB_E_ARG, "graph: already recording");
         CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeRelaxed));
         c->capturing = true;
+        c->recorded.clear();
+        c->pool.recording = &c->recorded;
         c->launches_at_capture = c->launches;
         c->alg_at_capture = c->alg_limbs;
     });
@@ -2254,12 +2219,17 @@ int hb_graph_end(hb_ctx *c, hb_graph **out) {
     return guard(c, [&] {
         if (!c->capturing) fail(HB_E_ARG, "graph: not recording");
         c->capturing = false;
-        cudaGraph_t g = nullptr;
-        CK(cudaStreamEndCapture(c->st, &g));
-        cudaGraphExec_t e = nullptr;
-        cudaError_t rc = cudaGraphInstantiate(&e, g, 0);
-        if (rc != cudaSuccess) { cudaGraphDestroy(g); throw CudaFail{rc, "cudaGraphInstantiate"}; }
-        *out = new hb_graph{c, g, e, c->launches - c->launches_at_capture, c->alg_limbs - c->alg_at_capture};
+        c->pool.recording = nullptr;
+        Pool::Buffers buffers;
+        buffers.swap(c->recorded);
+        try {
+            cudaGraph_t g = nullptr;
+            CK(cudaStreamEndCapture(c->st, &g));
+            cudaGraphExec_t e = nullptr;
+            cudaError_t rc = cudaGraphInstantiate(&e, g, 0);
+            if (rc != cudaSuccess) { cudaGraphDestroy(g); throw CudaFail{rc, "cudaGraphInstantiate"}; }
+            *out = new hb_graph{c, g, e, c->launches - c->launches_at_capture, c->alg_limbs - c->alg_at_capture, buffers};
+        } catch (...) { c->pool.unhold(buffers); throw; }
     });
 }
 int hb_graph_launch(hb_ctx *c, hb_graph *g) {
@@ -2275,6 +2245,7 @@ void hb_graph_free(hb_graph *g) {
     if (!g) return;
     cudaSetDevice(g->ctx->device);
     cudaGraphExecDestroy(g->e); cudaGraphDestroy(g->g);
+    g->ctx->pool.unhold(g->buffers);
     delete g;
 }
 

@@ -71,7 +71,7 @@ int hb_mem_info(const hb_ctx *ctx, uint64_t *pool_bytes, uint64_t *in_use_bytes)
  * returns, and the next hb_sync reports HB_E_TIMEOUT once; the context stays usable.  Exercises the path every bounded
  * device-side wait of the library takes when a copy does not land. */
 int hb_selftest_bounded_wait(hb_ctx *ctx);
-/* hands the pool's idle device buffers back to the driver (the buffers of live handles stay); refused while a graph records */
+/* hands the pool's idle device buffers back to the driver (those of live handles and of recorded graphs stay); refused while a graph records */
 int hb_release_cached(hb_ctx *ctx);
 /* the CUDA stream all kernels of this context run on (as a void* cudaStream_t) */
 void *hb_stream(const hb_ctx *ctx);

@@ -1,6 +1,7 @@
 """Full-size parity of the benchmarked path: the units of the encoder-layer workload, computed through the batched
 calls the layer driver makes (shared launch sequences, grouped loop iterations), must carry the residues the CPU
 oracle produced for the same units one at a time (digests in tests/golden/golden.json, made by make_golden.py)."""
+import ctypes as C
 import importlib
 import json
 import os
@@ -79,3 +80,35 @@ def test_graph_replay_reproduces_the_pass(pkg, gpu_full):
     with pytest.raises(pkg.HBError):
         g.ct_export(out["ccmm"]["all"][1].ct)
     g.graph_end()
+
+
+def test_recorded_buffers_outlive_a_release_of_the_pool(pkg):
+    """A replay after the pool gave its idle buffers back: those that the graph addresses are still there (looked at before the replay),
+    and go once the graph has gone."""
+    g = pkg.open_gpu(pkg.make_params(log_n=10, max_level=4, dnum=2, num_special=3, hamming_weight=32))
+    g.keygen()
+    g.gen_rot_keys([1, 5])
+    x = g.encrypt(g.encode(np.random.default_rng(3).uniform(-1, 1, g.slots), 3), 1)
+    step = lambda: g.rescale(g.mul_pt_norescale(g.rotate(g.rotate(x, 1), 5), w))
+    w = g.encode(np.full(g.slots, 0.5), 3)
+    want = g.ct_export(step())
+
+    def idle():
+        total, used = C.c_uint64(), C.c_uint64()
+        g._chk(g._fn("mem_info")(g.ctx, C.byref(total), C.byref(used)))
+        return total.value - used.value
+
+    g.graph_begin()
+    out = step()
+    graph = g.graph_end()
+    before = idle()
+    g._chk(g._fn("release_cached")(g.ctx))
+    assert 0 < idle() <= before
+    for _ in range(2):
+        g.graph_launch(graph)
+    g.sync()
+    assert np.array_equal(g.ct_export(out), want)
+    assert np.array_equal(g.ct_export(step()), want)
+    del graph
+    g._chk(g._fn("release_cached")(g.ctx))
+    assert idle() == 0

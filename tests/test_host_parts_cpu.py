@@ -1,0 +1,17 @@
+"""Host-side parts of the CUDA library that need no device, built with g++ against stand-ins for what they call."""
+import os
+import subprocess
+
+from conftest import PKG_NAME, ROOT
+
+
+def _run(tmp_path, name, *flags):
+    exe = str(tmp_path / name)
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-Wall", os.path.join(ROOT, "tests", "integration", name + ".cpp"), "-I", os.path.join(ROOT, PKG_NAME, "csrc"),
+                           "-I", "/usr/local/cuda/include", *flags, "-o", exe])
+    done = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert done.returncode == 0, done.stdout + done.stderr
+
+
+def test_pool_keeps_what_a_recorded_graph_addresses(tmp_path):
+    _run(tmp_path, "pool")
