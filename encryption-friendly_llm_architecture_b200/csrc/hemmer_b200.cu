@@ -8,14 +8,13 @@
 #include "ntt.cuh"
 #include "convcols.cuh"
 #include "embed.cuh"
+#include "host_threads.hpp"
 #include "pool.hpp"
 
 #include <cstdio>
 #include <dlfcn.h>
 #include <map>
-#include <thread>
 #include <memory>
-#include <system_error>
 #include <mutex>
 #include <nccl.h> // types only: the library is resolved at run time, see nccl_api()
 #include <unordered_map>
@@ -959,7 +958,7 @@ u64 *noalloc_scratch(int device) {
 // Going up, chunks of four members: the copies (6 to 8 GB/s here) take as long as the kernels, and only that of the first is not covered
 // (thirteen messages 1.03 ms with chunks of eight on the kernels' stream, 0.93 with a stream of their own, 0.68 in chunks of four).
 // Coming down, eight: the kernels are short, and neither a stream of its own nor chunks of four made a difference.
-constexpr int kStageMembers = 8, kUpMembers = 4, kCopyThreads = 4;
+constexpr int kStageMembers = 8, kUpMembers = 4;
 size_t stage_words(const hb_ctx *c, int members) { return (size_t)members * c->N; } // two doubles per slot
 // Two buffers and their events.  Those of messages are write-combined: the host only writes them, and the copy engine need not ask its caches.
 void stage_open(hb_ctx *c, double *(&buf)[2], cudaEvent_t (&ev)[2], int members, unsigned flags) {
@@ -977,21 +976,9 @@ void up_open(hb_ctx *c) {
     }
     stage_open(c, c->up, c->went_up, kUpMembers, cudaHostAllocWriteCombined);
 }
-// work(begin, end) over [0, n) on up to kCopyThreads threads, `words` doubles moved in all
-template <class F> void in_threads(const hb_ctx *c, size_t n, size_t words, F &&work) {
-    const size_t per = (size_t)1 << 16; // words that are worth a thread
-    const int cap = c->host_threads > 0 ? std::min(c->host_threads, kCopyThreads) : kCopyThreads;
-    const int k = (int)std::max<size_t>(1, std::min<size_t>({(size_t)cap, words / per, n}));
-    auto part = [&](int t) { work(n * t / k, n * (t + 1) / k); };
-    std::thread pool[kCopyThreads];
-    int started = 1;
-    try { for (; started < k; ++started) pool[started] = std::thread(part, started); } catch (const std::system_error &) {} // no more threads: the rest here
-    part(0);
-    for (int t = started; t < k; ++t) part(t);
-    for (int t = 1; t < started; ++t) pool[t].join();
-}
+int copy_threads(const hb_ctx *c) { return c->host_threads > 0 ? c->host_threads : kCopyThreads; }
 void host_copy(const hb_ctx *c, double *dst, const double *src, size_t words) {
-    in_threads(c, words, words, [&](size_t a, size_t b) { std::memcpy(dst + a, src + a, (b - a) * sizeof(double)); });
+    in_threads(copy_threads(c), words, words, [&](size_t a, size_t b) { std::memcpy(dst + a, src + a, (b - a) * sizeof(double)); });
 }
 // coef [count][N] = rounded coefficients at scale sc of the messages re / im [count][n] on the device (im may be null)
 void embed_inverse(hb_ctx *c, i64 *coef, const double *re, const double *im, int n, int count, double sc) {
@@ -1401,7 +1388,7 @@ int hb_encrypt_tiles(hb_ctx *c, const double *const *tiles, int across, int rows
         if (row > slots || n > slots) fail(HB_E_ARG, "encrypt_tiles: the tiles do not fit the slots");
         for (size_t i = 0; i < (size_t)count * across; ++i) if (!tiles[i]) fail(HB_E_ARG, "encrypt_tiles: missing tile");
         *out = encrypt_messages(c, n, false, count, level, nonces, [&](int first, int m, double *h) {
-            in_threads(c, (size_t)m * rows, (size_t)m * n, [&](size_t a, size_t b) {
+            in_threads(copy_threads(c), (size_t)m * rows, (size_t)m * n, [&](size_t a, size_t b) {
                 for (size_t k = a; k < b; ++k)
                     for (int t = 0; t < across; ++t)
                         std::memcpy(h + k * row + (size_t)t * cols, tiles[((size_t)first + k / rows) * across + t] + (k % rows) * cols, (size_t)cols * sizeof(double));

@@ -15,3 +15,7 @@ def _run(tmp_path, name, *flags):
 
 def test_pool_keeps_what_a_recorded_graph_addresses(tmp_path):
     _run(tmp_path, "pool")
+
+
+def test_threads_that_cannot_be_started_leave_their_share(tmp_path):
+    _run(tmp_path, "host_threads", "-pthread")
