@@ -375,20 +375,21 @@ __global__ void __launch_bounds__(256) k_keygen(u64 *key, const u64 *e, const u6
     store4(o, r);
     store4(o + (size_t)np * N, a);
 }
-// out [count][2][N]: b + a s (+ d2 s^2) of the first one or two limbs of every member (one polynomial: b alone).  grid = (gx, 2, count)
+// out [count][2][N]: b + a s (+ d2 s^2) of the first one or two limbs of every member (one polynomial: b alone; a limb that the member does
+// not have: 0).  grid = (gx, 1 or 2, count)
 __global__ void k_decrypt(u64 *out, const DecItem *items, const u64 *s, const PrimeConst *__restrict__ pc, int N) {
     const int l = blockIdx.y;
     pdl_wait();
     const DecItem it = items[blockIdx.z];
     const int np = it.np;
     const size_t poly = (size_t)it.n * N;
-    if (l >= it.n) return;
     const PrimeConst m = pc[l];
 #pragma unroll
     for (int u_ = 0; u_ < kElems; ++u_) {
         const int i = (blockIdx.x * kElems + u_) * blockDim.x + threadIdx.x;
         if (i >= N) break;
         const size_t off = (size_t)l * N + i;
+        if (l >= it.n) { out[(size_t)blockIdx.z * 2 * N + off] = 0; continue; }
         const u64 sv = s[off];
         u64 v = it.ct[off];
         if (np > 1) v = add_mod(v, mul_mod_any(it.ct[poly + off], sv, m), m.q);

@@ -1050,8 +1050,10 @@ void decrypt_items(hb_ctx *c, const std::vector<DecItem> &items, bool z, double 
         const size_t words = (size_t)m * slots;
         const DecItem *it = (const DecItem *)list.p + first;
         Tmp t(c, (size_t)m * 2), v(c, (size_t)m);
-        launch(c, k_decrypt, dim3(c->gx(), 2, (unsigned)m), 256, 0, t.p, it, (const u64 *)c->sk, c->pc, N);
-        ntt_inplace(c, t.p, m * 2, c->qmap(1), true);
+        int limbs = 1; // a second one if any member has it
+        for (int i = 0; i < m; ++i) limbs = std::max(limbs, std::min(2, items[(size_t)(first + i)].n));
+        launch(c, k_decrypt, dim3(c->gx(), (unsigned)limbs, (unsigned)m), 256, 0, t.p, it, (const u64 *)c->sk, c->pc, N);
+        ntt(c, t.p, (size_t)2 * N, t.p, (size_t)2 * N, m * limbs, c->qmap(limbs - 1), true);
         double *d = (double *)v.p;
         embed_forward(c, d, z ? d + 1 : d + words, z ? 2 : 1, t.p, it, m);
         CK(cudaMemcpyAsync(c->down[slot], d, words * (z || im ? 2 : 1) * sizeof(double), cudaMemcpyDeviceToHost, c->st));

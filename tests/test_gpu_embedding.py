@@ -69,6 +69,25 @@ def test_decoding_of_uniform_residues(request, size):
 
 
 @pytest.mark.parametrize("size", ["small", "full"])
+def test_members_with_one_limb_among_others(request, size):
+    """Chunks of eight whose members have one limb each, some two, one polynomial or three."""
+    g, o = _pair(request, size)
+    from conftest import rand_ct_residues
+    cts = []
+    for lib in (g, o):
+        cts.append([])
+        for k, (level, polys) in enumerate([(0, 2), (3, 2), (0, 3), (1, 2)]):
+            ct = lib.ct_create(level, polys, 1)
+            lib.ct_import(ct, rand_ct_residues(g, level, polys, 1, seed=30 + k))
+            cts[-1].append(ct)
+    want = [o.decrypt(ct) for ct in cts[1]]
+    order = [0, 2] * 4 + [0, 1, 2, 3] * 2 + [0, 3, 2]
+    got = g.decrypt_many([(cts[0][k], 0) for k in order])
+    for row, k in zip(got, order):
+        assert np.array_equal(row, want[k])
+
+
+@pytest.mark.parametrize("size", ["small", "full"])
 def test_switching_keys_equal_the_oracle(request, size):
     g, o = _pair(request, size)
     for galois in (0, g.galois(3)):
