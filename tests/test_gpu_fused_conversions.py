@@ -1,5 +1,5 @@
 """The kernels that join base conversions to the transforms of 2^16 points, and the inner products that walk over batch members,
-at the edges of their launch rules: every strip shape, partly filled member chunks, one and two rotations, one to seven conversion
+at the edges of their launch rules: every strip shape (those of more than four sources with batches of their own), partly filled member chunks, one and two rotations, one to seven conversion
 sources, and primes of every class (below 2^34, below 2^44, 45 to 59 bits, 60 bits).  Residues are whole numbers, so every comparison is exact."""
 import ctypes as C
 
@@ -18,14 +18,15 @@ def _ct(lib, data):
 
 
 SIZES = [("full", 12, (5, 33)), ("full", 7, (1, 2, 3, 5, 17, 33, 47)), ("full", 3, (1, 2, 3, 5, 17, 33, 47)), ("full", 2, (2, 5, 33)),
-         ("mid", 7, (17, 33, 47)), ("mid", 3, (17, 33, 47)), ("mid", 2, (17, 33, 47))]
+         ("full", 3, (6, 7, 12, 13)), ("mid", 7, (17, 33, 47)), ("mid", 3, (17, 33, 47)), ("mid", 2, (17, 33, 47))]
 
 
 @pytest.mark.parametrize("size,level,batch", [(s, l, b) for s, l, batches in SIZES for b in batches])
 def test_members_of_a_batch_equal_single_calls(request, size, level, batch):
     """Four, three, two and one digits (levels 12, 7, 3, 2), on either side of the 32 members from which the inner products hold one
-    coefficient per thread.  At 2^16 points the strip shapes change at 2, 4 and 32 polynomials, and one chunk holds all members
-    except at two and one digits with few of them (two chunks).  At 2^12 points a chunk holds two to seven members and the last
+    coefficient per thread.  At 2^16 points the strip shapes of these conversions (up to four sources) change at 2 and 12 units, polynomials
+    times digits, those of the rescale at 2 and 4 polynomials; one chunk holds all members except at two and one digits with few of them (two
+    chunks).  At 2^12 points a chunk holds two to seven members and the last
     one fewer, in the masked sums of one and two digits as well.  A batch of one takes the narrow shapes, whose residues the oracle
     tests pin."""
     g = request.getfixturevalue(f"gpu_{size}")
@@ -77,6 +78,32 @@ def test_other_parameter_sets_of_2_16_points(pkg, oracle_so, name):
         x = _ct(g, data)
         folded = g.assemble_masked(x, g.decompose(x), g.masked_key(3, g.encode_ext(m1, level)), g.masked_key(-5, g.encode_ext(1.0 - m1, level)))
         assert np.array_equal(g.ct_export(folded), res[0][3]), f"{name}: masked keys at level {level}"
+
+
+@pytest.fixture(scope="module", params=["all primes below 2^44", "one digit of seven limbs"])
+def many_sources(request, pkg):
+    g = pkg.open_gpu(pkg.make_params(log_n=16, hamming_weight=64, **PARAMS[request.param]))
+    g.keygen()
+    g.gen_rot_keys([3])
+    return g
+
+
+@pytest.mark.parametrize("batch", [6, 7, 12, 13, 16, 17, 33])
+def test_batches_of_conversions_with_more_than_four_sources(many_sources, batch):
+    """Divisions of five and seven sources, ModDown of six, a digit of seven: on either side of twelve units, from which conversions of up to
+    four sources take other strips, and of 32, from which the others do.  Units are members (decomposition) or pairs of polynomials."""
+    g = many_sources
+    level = int(g.L)
+    data = rand_ct_residues(g, level, 2, batch, seed=300 + batch)
+    data[-1, :, level] = np.uint64(int(g.primes[level]) - 1)
+    m = (np.random.default_rng(9).uniform(0, 1, g.slots) > 0.5).astype(np.float64)
+    key = g.masked_key(3, g.encode_ext(m, level))
+    ops = [lambda x: g.rotate(x, 3), lambda x: g.assemble_masked(x, g.decompose(x), key)]
+    whole = _ct(g, data)
+    for n, op in enumerate(ops):
+        got = g.ct_export(op(whole))
+        for k in sorted({0, batch // 2, batch - 1}):
+            assert np.array_equal(got[k:k + 1], g.ct_export(op(_ct(g, data[k:k + 1])))), f"operation {n}, member {k} of {batch}"
 
 
 @pytest.mark.parametrize("q_bits", [26, 27, 28, 34])
