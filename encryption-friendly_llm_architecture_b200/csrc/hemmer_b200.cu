@@ -808,11 +808,13 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
         if (!c->smem_opt_in_parts) { CK(cudaFuncSetAttribute(k_prod_parts<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)part_smem(G, kMaxPartTerms))); c->smem_opt_in_parts = true; }
         Scalars qi{};
         for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
-        // Up to ten polynomials the masks are streamed once per pair, beyond that they are kept.  A call with sixteen terms and twelve parts at
-        // level 7, us, streamed / kept: 4 polynomials 848 / 1305, 8 1536 / 1665, 10 1880 / 2039, 12 2223 / 2215.
+        // Up to ten polynomials, and for one or two parts, the masks are streamed once per pair of polynomials; otherwise they are kept.  Calls at
+        // level 7, us, streamed / kept: sixteen terms and twelve parts, 4 polynomials 647 / 1220, 10 1505 / 1920, 12 1804 / 2090, 24 3526 / 3338; nine
+        // terms and six parts, 10 818 / 832, 12 970 / 903; one term and one part, 12 149 / 269, 48 473 / 645; sixteen and two, 24 791 / 1063.
         auto sums = [&](u64 *o, const u64 *tt) {
             const unsigned limbs = (unsigned)(tt ? l : 1);
-            if (nbp <= 10) LAUNCH(c), k_prod_parts_few<<<dim3((unsigned)(N / 256 * ((nbp + 1) / 2)), limbs), 256, 0, c->st>>>(o, pt, tt, l, nbp, c->pc, N, qi);
+            auto few = [&](auto *kernel) { LAUNCH(c), kernel<<<dim3((unsigned)(N / 256 * ((nbp + 1) / 2)), limbs), 256, 0, c->st>>>(o, pt, tt, l, nbp, c->pc, N, qi); };
+            if (nbp <= 10 || parts <= 2) few(count <= 2 ? k_prod_parts_few<2> : count <= 4 ? k_prod_parts_few<4> : count <= 8 ? k_prod_parts_few<8> : k_prod_parts_few<kMaxPartTerms>);
             else LAUNCH(c), k_prod_parts<G><<<dim3(pg, (unsigned)(N / kPartLanes), limbs), 512, part_smem(G, count), c->st>>>(o, pt, tt, l, nbp, c->pc, N, qi, c->dev_err);
         };
         if (separate) launch(c, k_last_prod_parts, dim3(c->gx(), nbp, parts * count), 256, 0, last.p, pt, l, nbp, c->pc, N);

@@ -523,11 +523,14 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
     }
     cp_async_wait<0>(); // what was fetched past the end
 }
-// The same for a few polynomials: the masks are then most of the bytes, so they are streamed instead of kept.  A thread holds the words a_j of
-// its coefficient in two polynomials and walks over the parts, with the masks of a part in flight together.  A launch for one two-tile
-// product 604 -> 215 us (2.5 TB/s of masks).  grid = (N/256 * pairs of polynomials, 1 or level), arguments as above
-__global__ void __launch_bounds__(256, 2) k_prod_parts_few(u64 *__restrict__ out, const __grid_constant__ PartTerms pt, const u64 *__restrict__ t, int level, int nbp, const PrimeConst *__restrict__ pc, int N,
-                                                           const __grid_constant__ Scalars qlinv) {
+// The same for a few polynomials or parts: the masks are then most of the bytes, so they are streamed instead of kept.  A thread holds the words
+// a_j of its coefficient in two polynomials and walks over the parts, with the masks of a part in flight together.  A launch for one two-tile
+// product 604 -> 215 us (2.5 TB/s of masks).  TERMS: the most terms there can be; all of them are multiplied, and what a call does not have is
+// zero.  With seventeen for every call, one term and eight parts of eight polynomials took 871 us at level 7 (kept masks 739);
+// with two 523.  grid = (N/256 * pairs of polynomials, 1 or level), arguments as above
+template <int TERMS>
+__global__ void __launch_bounds__(256, TERMS <= 4 ? 4 : TERMS <= 8 ? 3 : 2) k_prod_parts_few(u64 *__restrict__ out, const __grid_constant__ PartTerms pt, const u64 *__restrict__ t, int level, int nbp,
+                                                                                            const PrimeConst *__restrict__ pc, int N, const __grid_constant__ Scalars qlinv) {
     const int pairs = (nbp + 1) / 2, bp = blockIdx.x % pairs * 2; // the pairs that read the same masks run together
     const int l = t ? (int)blockIdx.y : level, count = pt.count, x = blockIdx.x / pairs * 256 + threadIdx.x;
     const bool both = bp + 1 < nbp;
@@ -535,22 +538,22 @@ __global__ void __launch_bounds__(256, 2) k_prod_parts_few(u64 *__restrict__ out
     const u64 qli = t ? qlinv.v[l] : 0;
     const double qd = (double)m.q;
     const size_t po = (size_t)l * N + x, ao = po + (size_t)bp * (level + 1) * N, ao1 = both ? ao + (size_t)(level + 1) * N : ao;
-    u64 a[2][kMaxPartTerms];
+    u64 a[2][TERMS];
 #pragma unroll
-    for (int j = 0; j < kMaxPartTerms; ++j) {
+    for (int j = 0; j < TERMS; ++j) {
         a[0][j] = j < count ? key_word(pt.a[j][ao], m.fp) : 0;
         a[1][j] = j < count ? key_word(pt.a[j][ao1], m.fp) : 0;
     }
     const bool eight = !(m.fp && m.q < (1ull << 42));
 #pragma unroll 1
     for (int g = 0; g < pt.parts; ++g) {
-        u64 w[kMaxPartTerms], v[2];
+        u64 w[TERMS], v[2];
 #pragma unroll
-        for (int j = 0; j < kMaxPartTerms; ++j) w[j] = j < count && pt.p[g][j] ? pt.p[g][j][po] : 0;
+        for (int j = 0; j < TERMS; ++j) w[j] = j < count && pt.p[g][j] ? pt.p[g][j][po] : 0;
         if (m.fp) {
             FpAcc s[2]; s[0].zero(); s[1].zero();
 #pragma unroll
-            for (int j = 0; j < kMaxPartTerms; ++j) {
+            for (int j = 0; j < TERMS; ++j) {
                 if (j && j % 8 == 0 && eight) { s[0].relax(m.q_inv_f, qd); s[1].relax(m.q_inv_f, qd); }
                 const double k = u52_to_double(w[j]);
                 s[0].mac(__longlong_as_double((long long)a[0][j]), k); s[1].mac(__longlong_as_double((long long)a[1][j]), k);
@@ -559,7 +562,7 @@ __global__ void __launch_bounds__(256, 2) k_prod_parts_few(u64 *__restrict__ out
         } else {
             PieceAcc s[2]; s[0].zero(); s[1].zero();
 #pragma unroll
-            for (int j = 0; j < kMaxPartTerms; ++j) {
+            for (int j = 0; j < TERMS; ++j) {
                 if (j && j % 8 == 0) { s[0].relax(m); s[1].relax(m); }
                 const u32 k0 = (u32)w[j] & 0x3FFFFFFFu, k1 = (u32)(w[j] >> 30);
                 s[0].mac((u32)a[0][j], (u32)(a[0][j] >> 32), k0, k1); s[1].mac((u32)a[1][j], (u32)(a[1][j] >> 32), k0, k1);

@@ -1,5 +1,5 @@
 """Part sums of the baby-step / giant-step transforms and the plaintext products with shared copies at the edges of their kernels: one
-to ten polynomials (masks streamed for pairs of them), more (masks kept, pairs dealt to four slots, odd and missing pairs, several turns of
+to ten polynomials and one or two parts (masks streamed for pairs of polynomials), more (masks kept, pairs dealt to four slots, odd and missing pairs, several turns of
 the ring), one to seventeen terms and parts, absent terms, and primes of 42 and 44 bits (128 and 8 products between two reductions).
 Residues are whole numbers: every comparison is exact."""
 import ctypes as C
@@ -37,6 +37,16 @@ def _ptrs(handles):
 @pytest.mark.parametrize("terms,parts,polys,batch", [(1, 1, 1, 1), (17, 17, 2, 1), (9, 2, 1, 2), (8, 6, 3, 1), (17, 7, 2, 2), (16, 5, 1, 5), (2, 13, 2, 4), (17, 12, 3, 3), (3, 6, 2, 9), (10, 1, 1, 17), (17, 17, 1, 11), (16, 16, 2, 6), (1, 1, 3, 4), (9, 13, 1, 13)])
 @pytest.mark.parametrize("top", [False, True])
 def test_part_sums_equal_their_sums_one_by_one(pkg, g, terms, parts, polys, batch, top):
+    _compare_part_sums(pkg, g, terms, parts, polys, batch, top)
+
+
+@pytest.mark.parametrize("terms,parts,polys,batch", [(t, p, *s) for t in (2, 3, 4, 5, 8, 9) for p, s in ((3, (2, 5)), (2, (1, 11)), (3, (1, 11)))])
+def test_part_sums_on_either_side_of_the_term_counts_of_their_kernels(pkg, g, terms, parts, polys, batch):
+    """Streamed masks have a kernel for up to two, four, eight and seventeen terms, taken up to ten polynomials or two parts."""
+    _compare_part_sums(pkg, g, terms, parts, polys, batch, True)
+
+
+def _compare_part_sums(pkg, g, terms, parts, polys, batch, top):
     rng = np.random.default_rng(terms * 100 + parts)
     xs = [_ct(g, polys, batch, 40 + j, top) for j in range(terms)]
     pool = [g.encode(rng.uniform(-1, 1, g.slots), LEVEL) for _ in range(5)]
