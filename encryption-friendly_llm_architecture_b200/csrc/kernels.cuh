@@ -1394,7 +1394,8 @@ __global__ void k_div_fin(u64 *__restrict__ out, const u64 *__restrict__ E, cons
 // read once for T tiles and a weight word once (and converted or cut once) for two polynomials.  Both come through a ring of kAccRing stages
 // in shared memory that every thread fills for itself (cp.async), so a dozen loads of each of its 16 warps per SM are in flight without
 // registers for them.  Four tiles, words loaded to registers one or two terms ahead: 675 us a launch in the layer pass, 611 in the Q/K/V
-// projections; now 380 and 305.
+// projections; then 380 and 305.  Nothing is fetched past the last term, in a loop of its own: with the last word fetched again into every
+// stage one copy and one tile took 15.7 us (12.1 before there was a ring), now 12.3; 128 copies of two inputs and four tiles 580, now 566.
 // grid = (N/256, n)
 template <int T> struct TilePts { const u64 *p[T][16]; u64 *out[T]; };
 constexpr int kAccRing = 8;
@@ -1410,7 +1411,8 @@ __global__ void __launch_bounds__(256, 2) k_matmul_acc(const __grid_constant__ T
     const u32 x0 = blockIdx.x * 256 + threadIdx.x;
     const u64 *ring = words + threadIdx.x;
     const u32 ring_at = smem_u32(ring);
-    // what is fetched next: copy fk of input fb, and the weights' words that meet it (past the end the last copy again, which is not used)
+    // what is fetched next: copy fk of input fb, and the weights' words that meet it (nothing past the end, where the stages stay empty)
+    const int total = kcount * bcount;
     int fk = 0, fb = 0;
     u32 to = 0, g = __ldg(gal), src = g == 1 ? x0 : ntt_perm(x0, g, logn);
     const u64 *fa = pre + (size_t)b0 * 2 * poly + limb + x0;
@@ -1426,18 +1428,19 @@ __global__ void __launch_bounds__(256, 2) k_matmul_acc(const __grid_constant__ T
             fb = 0; ++fk; fa += to_next_copy;
             g = __ldg(gal + fk);
             src = g == 1 ? x0 : ntt_perm(x0, g, logn);
-        } else fb = bcount - 1;
+        }
         to += kStage * 8;
         if (to == kAccRing * kStage * 8) to = 0; // a stage is no power of two
     };
 #pragma unroll 1
-    for (int k = 0; k < kAccRing - 1; ++k) fetch();
+    for (int k = 0; k < kAccRing - 1; ++k) {
+        if (k < total) fetch();
+        else cp_async_commit();
+    }
     u64 r[T][2];
     auto terms = [&](auto &&product) {
-        const int total = kcount * bcount;
         int from = 0;
-#pragma unroll 2
-        for (int k = 0; k < total; ++k) {
+        auto term = [&](auto &&then) {
             cp_async_wait<kAccRing - 2>();
             const u64 *q = ring + from;
             u64 v[2] = {q[0], q[256]}, w[T];
@@ -1445,9 +1448,14 @@ __global__ void __launch_bounds__(256, 2) k_matmul_acc(const __grid_constant__ T
             for (int t = 0; t < T; ++t) w[t] = q[(2 + t) * 256];
             from += kStage;
             if (from == kAccRing * kStage) from = 0;
-            fetch();
+            then();
             product(v, w);
-        }
+        };
+        const int fetching = max(0, total - (kAccRing - 1));
+#pragma unroll 2
+        for (int k = 0; k < fetching; ++k) term(fetch);
+#pragma unroll 1
+        for (int k = fetching; k < total; ++k) term([] { cp_async_commit(); });
     };
     if (m.fp) { // exact sums (see FpAcc): 128 products of primes below 2^42, eight below 2^44, before they are reduced
         const double qd = (double)m.q;
@@ -1492,7 +1500,6 @@ __global__ void __launch_bounds__(256, 2) k_matmul_acc(const __grid_constant__ T
 #pragma unroll
         for (int t = 0; t < T; ++t) { r[t][0] = s[t][0].finish(m); r[t][1] = s[t][1].finish(m); }
     }
-    cp_async_wait<0>(); // what was fetched past the end
 #pragma unroll
     for (int t = 0; t < T; ++t) {
         u64 *o = tp.out[t] + limb + x0;
