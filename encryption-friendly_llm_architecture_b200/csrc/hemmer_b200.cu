@@ -517,7 +517,7 @@ void error_residues(hb_ctx *c, u64 *out, const i64 *coef, const StreamIds &ids, 
            (int)c->h->gauss_cdt.size(), map, c->pc, c->N);
 }
 void message_residues(hb_ctx *c, u64 *out, const i64 *coef, int count, const LimbMap &map) {
-    launch(c, k_residues<true, false>, dim3((unsigned)((c->N / 8 + 127) / 128), (unsigned)count), 128, 0, out, coef, StreamIds{}, (const u64 *)nullptr, 0, map, c->pc, c->N);
+    launch(c, k_residues<true, false>, dim3((unsigned)((c->N / 8 + 127) / 128), (unsigned)count, (unsigned)map.n), 128, 0, out, coef, StreamIds{}, (const u64 *)nullptr, 0, map, c->pc, c->N);
 }
 // switching key for secret s' (g == 0: s^2, else s o perm_g); stream ids kid*64 + digit
 Evk make_key(hb_ctx *c, u64 kid, u32 g) {
