@@ -341,20 +341,30 @@ void conv_opt_in(hb_ctx *c) {
 // Strip width and groups of a launch over `units` (polynomial, conversion) pairs.  At most two units: narrow strips and many groups, so that
 // all sources and all targets of a unit are worked on at once.  Up to twelve: narrow strips, two CTAs per SM, for the last wave.
 // Beyond: strips of eight columns (64-byte runs) and two groups, two CTAs per SM, whose barriers and loads cover each other, as long as their
-// strips fit (four sources); otherwise four groups and one CTA.  Rotations at level 6, us, (4 cols x 8 groups) / (4 x 4) / (8 x 4): one
-// ciphertext 88 / 103 / 98, eight 397 / 363 / 378, 64 2773 / 2524 / 2494.  Launches, us, (8 x 4) / (8 x 2): 96 polynomials of the division at level 6
-// 858 / 815, the conversions of 256 products at level 8 3093 / 2863; (4 x 4) / (8 x 2): 32 polynomials of the division 142 / 147, but the call
-// sequence of one product 10.87 / 10.74 ms; eight units 44.5 / 66.8.
+// strips fit (four sources); otherwise four groups and one CTA.  Calls, us, before the wide strips / (4 x 4) / (8 x 2), the shape of the launches
+// over the units named: products of level 8, 18 units (six members) 501 / 497 / 488; rotations of level 2, 16 units 208 / 203 / 192, 40 units 427 /
+// 424 / 389.  Launches, (8 x 4) / (8 x 2): 96 polynomials of the division at level 6 858 / 815, the conversions of 256 products at level 8 3093 / 2863.
+// The wide strips lose where few SMs have one CTA more than the others: 15, 16, 19 and 20 units leave a tenth to a half of the SMs with it,
+// and a CTA with four sources and many targets is long.  Calls, us, before / (4 x 4) / (8 x 2): rotations of five members at level 7 (15 units) 299 /
+// 299 / 310, products of eight at level 6 (16 units) 459 / 453 / 465; divisions of level 7, 16 units 257 / 254 / 261, 20 units 317 / 312 / 325.  Up to five
+// targets it does not show (division of level 3, 16 units 157 / 151 / 141; level 5, 20 units 219 / 212 / 214), nor with the three sources of
+// a ModDown (products of eight members at level 7, 16 units 586 / 577 / 567).
 enum StripShape { kStrip8x2, kStrip8x4, kStrip4x4, kStrip4x8 };
-StripShape conv_shape(int units, int max_ns) { return units <= 2 ? kStrip4x8 : units <= 12 ? kStrip4x4 : max_ns <= 4 ? kStrip8x2 : units <= 32 ? kStrip4x4 : kStrip8x4; }
+StripShape conv_shape(int units, int max_ns, int targets) {
+    if (units <= 2) return kStrip4x8;
+    if (units <= 12) return kStrip4x4;
+    if (max_ns > 4) return units <= 32 ? kStrip4x4 : kStrip8x4;
+    const int more = units * 32 % 148; // SMs with one CTA more
+    return units <= 20 && max_ns == 4 && targets > 5 && more >= 148 / 10 && more < 148 / 2 ? kStrip4x4 : kStrip8x2;
+}
 StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : kStrip8x2; }
-// `plans` conversions (the largest with max_ns sources) of `instances` polynomials in one launch
-void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int instances) {
+// `plans` conversions (the largest with max_ns sources, `targets` each on average) of `instances` polynomials in one launch
+void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int targets, int instances) {
     conv_opt_in(c);
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
         launch(c, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
     };
-    switch (conv_shape(instances * count, max_ns)) {
+    switch (conv_shape(instances * count, max_ns, targets)) {
     case kStrip8x2: go(conv_cols<8, 2, 2>, 8, 2, strip_bytes<8>(max_ns + 2)); break;
     case kStrip8x4: go(conv_cols<8, 4, 1>, 8, 4, strip_bytes<8>(max_ns + 4)); break;
     case kStrip4x4: go(conv_cols<4, 4, 2>, 4, 4, strip_bytes<4>(max_ns + 4)); break;
@@ -413,7 +423,7 @@ void ks_decompose(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch,
     Tmp acoef(c, (size_t)batch * n);
     if (c->logn == 16) {
         inv_rows(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level));
-        launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), batch);
+        launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.dt_count / d.nd, batch);
         fwd_rows(c, dt, (size_t)d.dt_count * N, batch * d.dt_count, d.dtmap);
         return;
     }
@@ -433,7 +443,7 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, siz
         const ConvPlan *cv = get_conv_plans(c, level);
         u64 *sp = acc + (size_t)n * N;
         inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, total * 2 * K, pm);
-        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, total * 2);
+        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, n, total * 2);
         const RowsFin f{acc, (size_t)ne * N, out, out_outer, 2, batch, add_outer};
         LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, total * 2, f, c->p_inv_scale, sl, c->pc, c->tb.t16));
         CK(cudaGetLastError());
@@ -604,7 +614,7 @@ hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch, hb_ct *dst = null
         if (c->logn == 16) {
             const ConvPlan *cv = get_conv_plans(c, level);
             inv_rows(c, src, (size_t)ne * N, src, (size_t)ne * N, batch * 2 * ns, sm);
-            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, batch * 2);
+            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, level, batch * 2);
             const RowsFin f{E, (size_t)ne * N, out, (size_t)2 * level * N, 2, 1, 0};
             LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], NoAddends{}, c->pc, c->tb.t16));
             CK(cudaGetLastError());

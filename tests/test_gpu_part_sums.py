@@ -1,7 +1,7 @@
 """Part sums of the baby-step / giant-step transforms and the plaintext products with shared copies at the edges of their kernels: one
-to ten polynomials and one or two parts (masks streamed for pairs of polynomials), more (masks kept, pairs dealt to four slots, odd and missing pairs, several turns of
-the ring), one to seventeen terms and parts, absent terms, and primes of 42 and 44 bits (128 and 8 products between two reductions).
-Residues are whole numbers: every comparison is exact."""
+to ten polynomials and one or two parts (masks streamed for pairs of polynomials), more (masks kept, pairs dealt to four slots, odd and
+missing pairs, several turns of the ring), one to seventeen terms and parts, absent terms, and primes of 42 and 44 bits (128 and 8 products
+between two reductions).  Residues are whole numbers: every comparison is exact."""
 import ctypes as C
 
 import numpy as np
