@@ -14,7 +14,8 @@
 // takes the sixteen rows that agree in their low four bits, whose images are runs of sixteen coefficients.
 // Bound by latency (16 CTAs of 128 threads a member): for eight members 7 and 14 us to encode, 40 and 35 us to decode, where the
 // host cores took 2.0 and 1.8 ms a member for the same transforms and 2.8 and 1.4 ms for sampling and CRT lift.  Thirteen messages
-// from host memory to ciphertexts 7.1 -> 0.68 ms, thirteen ciphertexts to host memory 5.6 -> 0.6 ms; the copies are most of both.
+// of two tiles from host memory to ciphertexts 7.3 -> 0.85 ms, thirteen ciphertexts to host memory 5.5 -> 0.80 ms, each pass through the Python
+// call on other buffers; the library call on the same buffers again takes 0.60 and 0.57.  The copies are most of all of these.
 #pragma once
 #include "modarith.cuh"
 #include "kernels.cuh"

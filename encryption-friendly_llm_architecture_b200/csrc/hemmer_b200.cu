@@ -968,7 +968,8 @@ u64 *noalloc_scratch(int device) {
 // Values travel in chunks through two pinned buffers a direction, so that moving one chunk in host memory overlaps the copy and the
 // transforms of the other.  The caller's pages are often new ones, whose first touch costs more than the bytes: several threads.
 // Going up, chunks of four members: the copies (6 to 8 GB/s here) take as long as the kernels, and only that of the first is not covered
-// (thirteen messages 1.03 ms with chunks of eight on the kernels' stream, 0.93 with a stream of their own, 0.68 in chunks of four).
+// (thirteen messages, the same buffers again: 1.03 ms with chunks of eight on the kernels' stream, 0.93 with a stream of their own, 0.68 in chunks of
+// four).
 // Coming down, eight: the kernels are short, and neither a stream of its own nor chunks of four made a difference.
 constexpr int kStageMembers = 8, kUpMembers = 4;
 size_t stage_words(const hb_ctx *c, int members) { return (size_t)members * c->N; } // two doubles per slot

@@ -357,8 +357,9 @@ __global__ void k_last_prod_parts(u64 *last, const __grid_constant__ PartTerms p
 // t that a sum is subtracted from, come through a ring of kPartRing stages in shared memory that runs on across terms and polynomials, each
 // thread copying its own (cp.async, no barrier).  With two loads ahead in registers and t loaded when it was needed, 6.1 ms for 48
 // polynomials, sixteen terms, twelve parts at level 7 (both launches); with the ring for the a_j 5.5, with t in it as well 4.1, with addresses
-// from a table instead of branches and one instruction per wide multiply-add 3.7 ms.  Bound by instruction issue now: 57 % of the slots with
-// sixteen warps, on a short limb FP64 45 % of the time.
+// from a table instead of branches and one instruction per wide multiply-add 3.7 ms.  Memory hardly shows any more (DRAM 16 %, half a
+// warp waiting for loads): four warps a scheduler issue in 57 % of the slots, between fixed latencies and their turns at the math pipes (FP64 45 % of
+// the time on a short limb, wide multiply-adds 37 % over all).
 // t == nullptr: raw sums of limb `level`, out[(g * nbp + bp) * N + x]                       grid = (ceil(parts/G), N/kPartLanes, 1)
 // else: out[((g * nbp + bp) * level + l) * N + x] = (sum - t[same]) * q_level^-1 mod q_l      grid = (ceil(parts/G), N/kPartLanes, level)
 // (parts first, so that the CTAs that read the same words run together)
@@ -1396,6 +1397,7 @@ __global__ void k_div_fin(u64 *__restrict__ out, const u64 *__restrict__ E, cons
 // registers for them.  Four tiles, words loaded to registers one or two terms ahead: 675 us a launch in the layer pass, 611 in the Q/K/V
 // projections; then 380 and 305.  Nothing is fetched past the last term, in a loop of its own: with the last word fetched again into every
 // stage one copy and one tile took 15.7 us (12.1 before there was a ring), now 12.3; 128 copies of two inputs and four tiles 580, now 566.
+// These issue in 66 % of the slots with sixteen warps per SM, DRAM 35 %, FP64 34 %.
 // grid = (N/256, n)
 template <int T> struct TilePts { const u64 *p[T][16]; u64 *out[T]; };
 constexpr int kAccRing = 8;

@@ -210,8 +210,8 @@ struct FpAcc {
 // into two pieces of 30 bits instead: a product is three 32 x 32 -> 64-bit multiply-adds into three carry-free accumulators (12
 // cycles, 4 more per operand that is cut), and the sum  a0 + a1 * 2^30 + a2 * 2^60  is reduced once per output residue with
 // 2^60 = d60 modulo q (a 128-bit Barrett reduction takes 65 cycles).  Eight products fit the accumulators.
-// One instruction.  The pair mad.lo.cc / madc.hi is a little cheaper in a chain of its own (4.1 against 5.0 cycles), but inside the kernels
-// it came out as seven instructions, with moves: part sums of 48 polynomials 6.5 against 5.9 ms, one limb of them 1.3 against 0.9 ms.
+// The pair mad.lo.cc / madc.hi is a little cheaper in a chain of its own (4.1 against 5.0 cycles), but not inside the kernels: part sums of 48
+// polynomials 6.5 against 5.9 ms, one limb of them 1.3 against 0.9 ms.
 __device__ __forceinline__ u64 mad_wide(u32 a, u32 b, u64 c) {
     u64 r;
     asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
