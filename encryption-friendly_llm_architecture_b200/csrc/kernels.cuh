@@ -1216,8 +1216,8 @@ __global__ void __launch_bounds__(256, 2) k_ks_inner_mk(u64 *E, const u64 *c0, c
 // staging both in shared memory by bulk copies for three members at a time took 1.6 times as long (they crossed L2 for every
 // third member, and a CTA's copies, sums and stores did not overlap).  Two coefficients per thread and two CTAs per SM: 869 us a launch
 // for 168 outputs at level 6; one coefficient and three CTAs 837 us, four CTAs 776 us (64 registers, of which two digits spill 24
-// bytes a thread): the integer chains of the 60-bit limbs want warps more than they want independent work in a thread.  Bound by
-// instruction issue: 65 % of the slots and 52 % of the wide multiply-adds for 64 outputs (367 us), DRAM 3.1 TB/s.
+// bytes a thread): the integer chains of the 60-bit limbs want warps more than they want independent work in a thread.  65 % of the
+// issue slots and 52 % of the wide multiply-adds for 64 outputs (367 us), DRAM 3.1 TB/s; in a third of the cycles it waits for loads.
 // grid = (N/256, groups * ceil(batch/per), ne)
 template <int ND, int CNT>
 __device__ __forceinline__ void ks_inner_mkr_body(u64 *o, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const MaskedRot &mr, int b0, int b1, const KsPlan *__restrict__ pl,
