@@ -312,7 +312,8 @@ int hb_set_host_threads(hb_ctx *ctx, int n);
  * hb_graph_launch replays them on the context's stream.  Device buffers come from the context's pool exactly as in
  * an unrecorded pass, so the recorded kernels use fixed addresses: keep the operand handles alive and update them
  * in place only, and keep the result handles of the recorded pass while the graph is in use -- every replay writes
- * its results there.  Whatever is made on first use (rotation keys, masks, masked keys, per-level plans) must exist
+ * its results there.  The temporaries of the recorded pass are idle buffers between replays: a handle made after recording may
+ * lie in one of them and is overwritten by the next replay, so make what has to outlive replays before recording.  Whatever is made on first use (rotation keys, masks, masked keys, per-level plans) must exist
  * before recording: run the sequence once first.  Calls that wait for the stream or copy to / from the host
  * (encode, encrypt, decrypt, import, export, sync) return HB_E_ARG while recording. */
 typedef struct hb_graph hb_graph;
