@@ -22,6 +22,8 @@ __device__ __forceinline__ void bulk_load(void *dst_smem, const void *src_gmem, 
 }
 // eight bytes global -> shared memory, asynchronously; groups of them complete in order, for the thread that issued them
 __device__ __forceinline__ void cp_async8(u32 dst_smem, const void *src_gmem) { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst_smem), "l"(src_gmem) : "memory"); }
+// sixteen bytes, past L1; both addresses 16-byte aligned
+__device__ __forceinline__ void cp_async16(u32 dst_smem, const void *src_gmem) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src_gmem) : "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int PENDING> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 // asks for `bytes` (a multiple of 16) at a 16-byte aligned global address to be brought into L2

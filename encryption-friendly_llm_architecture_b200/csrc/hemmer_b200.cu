@@ -331,11 +331,13 @@ const ConvPlan *get_conv_plans(hb_ctx *c, int level) {
     return d;
 }
 template <int COLS> size_t strip_bytes(int strips) { return (size_t)strips * StripIndex<COLS>::kWords * 8; }
+size_t conv_const_bytes(int ns, int nt) { return (size_t)2 * ns * nt * sizeof(ConvConst); }
 void conv_opt_in(hb_ctx *c) {
     if (c->smem_opt_in_conv) return;
     auto allow = [](auto *kernel, size_t bytes) { CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); };
-    allow(conv_cols<8, 4, 1>, strip_bytes<8>(12)); allow(conv_cols<4, 4, 2>, strip_bytes<4>(12)); allow(conv_cols<4, 8, 1>, strip_bytes<4>(16));
-    allow(conv_cols<8, 2, 2>, strip_bytes<8>(6)); allow(lift_cols<8, 2, 2>, strip_bytes<8>(3)); allow(lift_cols<4, 4, 2>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1>, strip_bytes<4>(9));
+    const size_t consts = conv_const_bytes(8, kMaxPrimes);
+    allow(conv_cols<8, 4, 1>, strip_bytes<8>(12) + consts); allow(conv_cols<4, 4, 2>, strip_bytes<4>(12) + consts); allow(conv_cols<4, 8, 1>, strip_bytes<4>(16) + consts);
+    allow(conv_cols<8, 2, 2>, strip_bytes<8>(6) + conv_const_bytes(4, kMaxPrimes)); allow(lift_cols<8, 2, 2>, strip_bytes<8>(3)); allow(lift_cols<4, 4, 2>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1>, strip_bytes<4>(9));
     c->smem_opt_in_conv = true;
 }
 // Strip width and groups of a launch over `units` (polynomial, conversion) pairs.  At most two units: narrow strips and many groups, so that
@@ -358,17 +360,18 @@ StripShape conv_shape(int units, int max_ns, int targets) {
     return units <= 20 && max_ns == 4 && targets > 5 && more >= 148 / 10 && more < 148 / 2 ? kStrip4x4 : kStrip8x2;
 }
 StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : kStrip8x2; }
-// `plans` conversions (the largest with max_ns sources, `targets` each on average) of `instances` polynomials in one launch
-void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int targets, int instances) {
+// `plans` conversions (the largest with max_ns sources, `targets` each on average, max_nt at most) of `instances` polynomials in one launch
+void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int targets, int max_nt, int instances) {
     conv_opt_in(c);
+    const size_t consts = conv_const_bytes(max_ns, max_nt);
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
         launch(c, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
     };
     switch (conv_shape(instances * count, max_ns, targets)) {
-    case kStrip8x2: go(conv_cols<8, 2, 2>, 8, 2, strip_bytes<8>(max_ns + 2)); break;
-    case kStrip8x4: go(conv_cols<8, 4, 1>, 8, 4, strip_bytes<8>(max_ns + 4)); break;
-    case kStrip4x4: go(conv_cols<4, 4, 2>, 4, 4, strip_bytes<4>(max_ns + 4)); break;
-    default: go(conv_cols<4, 8, 1>, 4, 8, strip_bytes<4>(max_ns + 8)); break;
+    case kStrip8x2: go(conv_cols<8, 2, 2>, 8, 2, strip_bytes<8>(max_ns + 2) + consts); break;
+    case kStrip8x4: go(conv_cols<8, 4, 1>, 8, 4, strip_bytes<8>(max_ns + 4) + consts); break;
+    case kStrip4x4: go(conv_cols<4, 4, 2>, 4, 4, strip_bytes<4>(max_ns + 4) + consts); break;
+    default: go(conv_cols<4, 8, 1>, 4, 8, strip_bytes<4>(max_ns + 8) + consts); break;
     }
 }
 // half-inverse limbs of prime `level` (one per instance) -> half-forward lifts to the limbs below
@@ -423,7 +426,7 @@ void ks_decompose(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch,
     Tmp acoef(c, (size_t)batch * n);
     if (c->logn == 16) {
         inv_rows(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level));
-        launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.dt_count / d.nd, batch);
+        launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.dt_count / d.nd, d.ne, batch);
         fwd_rows(c, dt, (size_t)d.dt_count * N, batch * d.dt_count, d.dtmap);
         return;
     }
@@ -443,7 +446,7 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, siz
         const ConvPlan *cv = get_conv_plans(c, level);
         u64 *sp = acc + (size_t)n * N;
         inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, total * 2 * K, pm);
-        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, n, total * 2);
+        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, n, n, total * 2);
         const RowsFin f{acc, (size_t)ne * N, out, out_outer, 2, batch, add_outer};
         LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, total * 2, f, c->p_inv_scale, sl, c->pc, c->tb.t16));
         CK(cudaGetLastError());
@@ -614,7 +617,7 @@ hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch, hb_ct *dst = null
         if (c->logn == 16) {
             const ConvPlan *cv = get_conv_plans(c, level);
             inv_rows(c, src, (size_t)ne * N, src, (size_t)ne * N, batch * 2 * ns, sm);
-            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, level, batch * 2);
+            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, level, level, batch * 2);
             const RowsFin f{E, (size_t)ne * N, out, (size_t)2 * level * N, 2, 1, 0};
             LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], NoAddends{}, c->pc, c->tb.t16));
             CK(cudaGetLastError());
