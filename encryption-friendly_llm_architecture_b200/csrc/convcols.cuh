@@ -36,8 +36,7 @@ struct ConvPlan {
     int src_limb, dst_limb;             // first limb of the sources / targets inside one instance of the arrays
     unsigned char src_prime[8], dst_prime[kMaxPrimes];
     unsigned char order[kMaxPrimes];    // targets in the order they are taken: those of the long primes, which take twice the time, first
-    u64 scale_w[8][2], scale_c[8][2];   // (ds_twiddle_word, w / q as a double) below 2^44, (w, Shoup companion) otherwise; [1]: times psi^(-N/2), the
-                                        // twiddle of the last inverse stage
+    u64 scale_w[8][2], scale_c[8][2];   // as scale_words makes them; [1]: times psi^(-N/2), the twiddle of the last inverse stage
     unsigned char fp[kMaxPrimes];       // target t converts on the FP64 pipe (see ConvFp)
     uint4 c[kMaxPrimes][2][8];          // [target][half of the rows][source], the second half times psi^(N/2), the twiddle of the first forward stage: C = D / d_s mod target.  Target below 2^44: the 26-bit pieces of C
                                         // and of C * 2^30; otherwise the 30-bit pieces of C, their sum, 0
@@ -68,7 +67,7 @@ template <int COLS> __device__ __forceinline__ void strip_fetch(const u64 *p /* 
 }
 // Inverse column pass of one limb strip, whose words of the rows sub * 16 + e are in(e): word(canonical value times the scale) goes to sm at I::a,
 // where this thread has read its own words.  sw, sc: the scale, and the scale times the twiddle of the last stage.
-template <int COLS, class IN, class WORD>
+template <int COLS, class LONG, class IN, class WORD>
 __device__ __forceinline__ void strip_inverse(IN &&in, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, const u64 (&sw)[2], const u64 (&sc)[2],
                                               int g, int sub, int lane, WORD &&word) {
     using I = StripIndex<COLS>;
@@ -87,23 +86,23 @@ __device__ __forceinline__ void strip_inverse(IN &&in, u64 *sm, const PrimeConst
         inv16_ds<1>(d, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
         inv16_ds_last(d, sw, sc, c, [&](int e, u64 w) { sm[I::a(e, sub, lane)] = word(w); });
     } else {
-        const IntConst c = int_const(m);
+        const typename LONG::Const c = LONG::make(m);
         u64 v[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = in(e);
-        inv16_int(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
+        LONG::inv16(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[I::b(e, sub, lane)] = v[e];
         group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[I::a(e, sub, lane)];
-        inv16_int<1>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
-        inv16_int_last(v, sw, sc, c, [&](int e, u64 w) { sm[I::a(e, sub, lane)] = word(w); });
+        LONG::template inv16<1>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
+        inv16_int_last<LONG>(v, sw, sc, c, [&](int e, u64 w) { sm[I::a(e, sub, lane)] = word(w); });
     }
 }
 // Forward column pass of one limb strip that lies in sm (words of this thread at I::a; double bits below 2^44, |v| < 2q; otherwise below 3q).
 // MADE: the rows from 128 on already carry the twiddle of the first stage.
-template <int COLS, bool MADE>
+template <int COLS, class LONG, bool MADE>
 __device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, int g, int sub, int lane) {
     using I = StripIndex<COLS>;
     if (m.small) {
@@ -122,17 +121,17 @@ __device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *s
 #pragma unroll
         for (int e = 0; e < 16; ++e) reinterpret_cast<double *>(o)[(sub * 16 + e) * 256] = d[e];
     } else {
-        const IntConst c = int_const(m);
+        const typename LONG::Const c = LONG::make(m);
         u64 v[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[I::a(e, sub, lane)];
-        fwd16_int<kFoldColsA, MADE>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
+        LONG::template fwd16<0, MADE>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[I::a(e, sub, lane)] = v[e];
         group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[I::b(e, sub, lane)];
-        fwd16_int<kFoldColsB>(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
+        LONG::template fwd16<1>(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) o[(sub * 16 + e) * 256] = v[e];
     }
@@ -255,7 +254,7 @@ __device__ __forceinline__ void convert_target_wide(u64 *sm, const u64 *ysm, con
 // every few products, and what L1 is left beside the strips holds no more than the twiddles.  All sources are on their way
 // from the start instead of behind one another.  The two together: 139 -> 129 ms
 // of the layer's conversions, products of 256 members at level 8 5.69 -> 5.33 ms.
-template <int COLS, int G, int MINB>
+template <int COLS, int G, int MINB, class LONG>
 __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, const ConvPlan *__restrict__ plans,
                                                                          const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     extern __shared__ __align__(16) u64 strips[];
@@ -281,7 +280,7 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
         group_sync<COLS * 16>(g);
         const int pi = pl->src_prime[s];
         u64 *sm = strips + s * I::kWords;
-        strip_inverse<COLS>([&](int e) { return sm[I::b(e, sub, lane)]; }, sm, pc[pi], tb.inv + (size_t)pi * Ntt16Layout::kEntries, pl->scale_w[s], pl->scale_c[s], g, sub, lane,
+        strip_inverse<COLS, LONG>([&](int e) { return sm[I::b(e, sub, lane)]; }, sm, pc[pi], tb.inv + (size_t)pi * Ntt16Layout::kEntries, pl->scale_w[s], pl->scale_c[s], g, sub, lane,
                             [](u64 v) { return ((v >> 30) << 32) | ((u32)v & 0x3FFFFFFFu); });
     }
     __syncthreads();
@@ -300,13 +299,13 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
         if (fp) convert_target_fp<COLS>(ex, strips, cst, ns, m, sub, lane);
         else if (m.small) convert_target_small<COLS>(ex, strips, cst, ns, m, sub, lane);
         else convert_target_wide<COLS>(ex, strips, cst, ns, m, sub, lane);
-        strip_forward<COLS, true>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)pi * Ntt16Layout::kEntries, g, sub, lane);
+        strip_forward<COLS, LONG, true>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)pi * Ntt16Layout::kEntries, g, sub, lane);
     }
 }
 
 // Rescale: one source limb (prime index `level`), lifted centred to the limbs 0 .. level - 1.
 // grid = (256 / COLS, instances); dynamic shared memory: 1 + G strips.
-template <int COLS, int G, int MINB>
+template <int COLS, int G, int MINB, class LONG>
 __global__ void __launch_bounds__(COLS * 16 * G, MINB) lift_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int level,
                                                                          const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     extern __shared__ __align__(16) u64 strips[];
@@ -319,7 +318,7 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) lift_cols(const u64 *src,
     if (g == 0) {
         const PrimeConst m = pc[level];
         const u64 *sp = src + (size_t)blockIdx.y * src_outer + col;
-        strip_inverse<COLS>([&](int e) { return sp[(sub * 16 + e) * 256]; }, strips, m, tb.inv + (size_t)level * Ntt16Layout::kEntries, m.n_inv_w, m.n_inv_c, g, sub, lane,
+        strip_inverse<COLS, LONG>([&](int e) { return sp[(sub * 16 + e) * 256]; }, strips, m, tb.inv + (size_t)level * Ntt16Layout::kEntries, m.n_inv_w, m.n_inv_c, g, sub, lane,
                             [&](u64 v) { return v > (ql >> 1) ? v - ql : v; }); // signed
     }
     __syncthreads();
@@ -336,7 +335,7 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) lift_cols(const u64 *src,
             else if ((ql >> 1) < m.q) w = y < 0 ? (u64)(y + (i64)m.q) : (u64)y;
             else w = reduce_i64(y, m);
         }
-        strip_forward<COLS, false>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)t * Ntt16Layout::kEntries, g, sub, lane);
+        strip_forward<COLS, LONG, false>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)t * Ntt16Layout::kEntries, g, sub, lane);
     }
 }
 
@@ -351,9 +350,9 @@ struct RowsFin {
     u64 *out; size_t out_outer;              // ciphertext stride; polynomial p at p * n * N
     int np, batch; size_t add_outer;         // ciphertexts per group, ciphertext stride of the addends
 };
-struct InvScale { u64 w[kMaxPrimes], c[kMaxPrimes]; }; // per limb: (ds_twiddle_word, w / q as a double) below 2^44, (w, Shoup companion) otherwise
+struct InvScale { u64 w[kMaxPrimes], c[kMaxPrimes]; }; // per limb, as scale_words makes them
 struct NoAddends {};
-template <int MINB, class ADD /* SwitchList or NoAddends */>
+template <int MINB, class ADD /* SwitchList or NoAddends */, class LONG>
 __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, size_t t_outer, const __grid_constant__ RowsFin f, const __grid_constant__ InvScale sc, const __grid_constant__ ADD add,
                                                             const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     __shared__ u64 sm[16 * kRowStride];
@@ -410,19 +409,19 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
             o[e * 16] = ds_store(r, c, c.qd, qinv_up);
         }
     } else {
-        const IntConst c = int_const(m);
+        const typename LONG::Const c = LONG::make(m);
         u64 v[16];
         const TwiddlesB<ulonglong2, MINB <= 2> tw(tab + Ntt16Layout::rowsB(row, 0, clo));
         pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = tp[e * 16];
-        fwd16_int<kFoldRowsA>(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
+        LONG::template fwd16<2>(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
-        fwd16_int<kFoldRowsB>(v, tw, c); // below 5q
+        LONG::template fwd16<3>(v, tw, c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = v[e];
         u64 x[16];
@@ -432,9 +431,9 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
         const u64 sw = sc.w[l], ss = sc.c[l];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-            u64 r = mul_shoup4(x[e] + c.q8 - smr[e * 17 + clo], sw, ss, c.nq); // below 4q
+            u64 r = LONG::mul(x[e] + LONG::above(c) - smr[e * 17 + clo], sw, ss, c); // below 7q
             if (ap) r += ap[g ? ntt_perm((u32)(pos + e * 16), g, 16) : (u32)(pos + e * 16)];
-            o[e * 16] = canon_q(r, c.q, c.f);
+            o[e * 16] = LONG::canon(r, c);
         }
     }
 }
@@ -451,16 +450,23 @@ template <class... P, class... A> inline cudaError_t launch_plain(cudaStream_t s
     return cudaPeekAtLastError();
 }
 inline cudaError_t launch_inv_rows16(cudaStream_t st, const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
-    return launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_inv_rows<2> : ntt16v2_inv_rows<4>, dim3(16, count), 256, 0, src, LimbAddr16{src_outer}, dst, LimbAddr16{dst_outer}, map, pc, tb);
+    auto go = [&](auto *small, auto *kernel) { return launch_pdl(st, 16 * count <= kSmallGrid ? small : kernel, dim3(16, count), 256, 0, src, LimbAddr16{src_outer}, dst, LimbAddr16{dst_outer}, map, pc, tb); };
+    return tb.pm ? go(ntt16v2_inv_rows<2, LongPm>, ntt16v2_inv_rows<4, LongPm>) : go(ntt16v2_inv_rows<2, LongShoup>, ntt16v2_inv_rows<4, LongShoup>);
 }
 inline cudaError_t launch_fwd_rows16(cudaStream_t st, u64 *d, size_t outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
-    if (16 * count >= kPlainGrid) return launch_plain(st, ntt16v2_fwd_rows<4>, dim3(16, count), 256, d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb);
-    return launch_pdl(st, 16 * count <= kSmallGrid ? ntt16v2_fwd_rows<2> : ntt16v2_fwd_rows<4>, dim3(16, count), 256, 0, d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb);
+    auto go = [&](auto *small, auto *kernel) {
+        if (16 * count >= kPlainGrid) return launch_plain(st, kernel, dim3(16, count), 256, d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb);
+        return launch_pdl(st, 16 * count <= kSmallGrid ? small : kernel, dim3(16, count), 256, 0, d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb);
+    };
+    return tb.pm ? go(ntt16v2_fwd_rows<2, LongPm>, ntt16v2_fwd_rows<4, LongPm>) : go(ntt16v2_fwd_rows<2, LongShoup>, ntt16v2_fwd_rows<4, LongShoup>);
 }
 template <class ADD>
 inline cudaError_t launch_fwd_rows_fin16(cudaStream_t st, const u64 *t, size_t t_outer, int n, int instances, const RowsFin &f, const InvScale &sc, const ADD &add, const PrimeConst *pc, const Ntt16Tables &tb) {
-    if (16 * n * instances >= kPlainGrid) return launch_plain(st, ntt16v2_fwd_rows_fin<4, ADD>, dim3(16, n, instances), 256, t, t_outer, f, sc, add, pc, tb);
-    return launch_pdl(st, 16 * n * instances <= kSmallGrid ? ntt16v2_fwd_rows_fin<2, ADD> : ntt16v2_fwd_rows_fin<4, ADD>, dim3(16, n, instances), 256, 0, t, t_outer, f, sc, add, pc, tb);
+    auto go = [&](auto *small, auto *kernel) {
+        if (16 * n * instances >= kPlainGrid) return launch_plain(st, kernel, dim3(16, n, instances), 256, t, t_outer, f, sc, add, pc, tb);
+        return launch_pdl(st, 16 * n * instances <= kSmallGrid ? small : kernel, dim3(16, n, instances), 256, 0, t, t_outer, f, sc, add, pc, tb);
+    };
+    return tb.pm ? go(ntt16v2_fwd_rows_fin<2, ADD, LongPm>, ntt16v2_fwd_rows_fin<4, ADD, LongPm>) : go(ntt16v2_fwd_rows_fin<2, ADD, LongShoup>, ntt16v2_fwd_rows_fin<4, ADD, LongShoup>);
 }
 
 } // namespace hb

@@ -173,9 +173,15 @@ template <class K, class... A> void launch(hb_ctx *c, K *kernel, dim3 grid, dim3
     c->launches++;
     CK(launch_pdl(c->st, kernel, grid, block, smem, std::forward<A>(args)...));
 }
-// a constant v mod q in the form the 2^16 kernels multiply by: the value as a double and v / q, or the value and its Shoup companion
-void scale_words(u64 v, u64 q, u64 &w, u64 &comp) {
-    if (q >> 44) { w = v; comp = hbhost::shoup(v, q); return; }
+// a constant v mod q in the form the 2^16 kernels multiply by: the value as a double and v / q; for long primes the pieces of LongPm, or the value and its
+// Shoup companion
+void scale_words(u64 v, u64 q, bool pm, u64 &w, u64 &comp) {
+    if (q >> 44) {
+        auto pieces = [](u64 x) { return (x & 0x1FFFFFFFu) | (x >> 29 << 32); };
+        w = pm ? pieces(v) : v;
+        comp = pm ? pieces(hbhost::mulmod(v, ((u64)1 << 32) % q, q)) : hbhost::shoup(v, q);
+        return;
+    }
     w = ds_twiddle_word(v);
     const double f = (double)v / (double)q;
     std::memcpy(&comp, &f, 8);
@@ -249,15 +255,15 @@ const KsPlan *get_plan(hb_ctx *c, int level) {
     return d;
 }
 // ---- conversions between the column passes (2^16 rings) ----
-void fill_conv(const HostCtx &h, ConvPlan &p, const std::vector<int> &src, const std::vector<int> &dst, int src_limb, int dst_limb) {
+void fill_conv(const HostCtx &h, bool pm, ConvPlan &p, const std::vector<int> &src, const std::vector<int> &dst, int src_limb, int dst_limb) {
     p.ns = (int)src.size(); p.nt = (int)dst.size(); p.src_limb = src_limb; p.dst_limb = dst_limb;
     auto hat = [&](size_t s, u64 q) { u64 v = 1; for (size_t t = 0; t < src.size(); ++t) if (t != s) v = hbhost::mulmod(v, h.q[src[t]] % q, q); return v; };
     auto half_turn = [&](int prime) { return hbhost::powmod(h.psi_root[(size_t)prime], (u64)h.N / 2, h.q[(size_t)prime]); }; // psi^(N/2)
     for (size_t s = 0; s < src.size(); ++s) {
         const u64 q = h.q[src[s]], v = hbhost::mulmod(hbhost::invmod((u64)h.N % q, q), hbhost::invmod(hat(s, q), q), q);
         p.src_prime[s] = (unsigned char)src[s];
-        scale_words(v, q, p.scale_w[s][0], p.scale_c[s][0]);
-        scale_words(hbhost::mulmod(v, q - half_turn(src[s]), q), q, p.scale_w[s][1], p.scale_c[s][1]); // its inverse is its negative
+        scale_words(v, q, pm, p.scale_w[s][0], p.scale_c[s][0]);
+        scale_words(hbhost::mulmod(v, q - half_turn(src[s]), q), q, pm, p.scale_w[s][1], p.scale_c[s][1]); // its inverse is its negative
     }
     for (size_t t = 0; t < dst.size(); ++t) {
         const u64 q = h.q[dst[t]], m26 = ((u64)1 << 26) - 1, m30 = ((u64)1 << 30) - 1;
@@ -292,6 +298,7 @@ const ConvPlan *get_conv_plans(hb_ctx *c, int level) {
     if (it != c->conv_plans.end()) return it->second;
     no_capture(c, "first key switch at this level");
     const HostCtx &h = *c->h;
+    const bool pm = c->tb.t16.pm;
     const int n = level + 1, K = h.K, ne = n + K, nd = h.digit_of(level) + 1;
     auto prime_of = [&](int j) { return j < n ? j : h.L + 1 + (j - n); };
     std::vector<ConvPlan> v((size_t)nd + 2);
@@ -303,25 +310,25 @@ const ConvPlan *get_conv_plans(hb_ctx *c, int level) {
     for (int dg = 0; dg < nd; ++dg) {
         std::vector<int> src, dst;
         for (int j = 0; j < ne; ++j) (j >= h.digit_lo(dg) && j < h.digit_hi(dg, n) ? src : dst).push_back(prime_of(j));
-        fill_conv(h, v[(size_t)dg], src, dst, h.digit_lo(dg), entry);
+        fill_conv(h, pm, v[(size_t)dg], src, dst, h.digit_lo(dg), entry);
         entry += (int)dst.size();
     }
-    fill_conv(h, v[(size_t)nd], special, q_all, 0, 0);
+    fill_conv(h, pm, v[(size_t)nd], special, q_all, 0, 0);
     if (level >= 1 && K < 8) {
         std::vector<int> src{level};
         src.insert(src.end(), special.begin(), special.end());
-        fill_conv(h, v[(size_t)nd + 1], src, q_low, 0, 0);
+        fill_conv(h, pm, v[(size_t)nd + 1], src, q_low, 0, 0);
         InvScale &sc = c->div_scale[level];
         for (int l = 0; l < level; ++l) {
             u64 d = h.q[level] % h.q[l];
             for (int p : special) d = hbhost::mulmod(d, h.q[p] % h.q[l], h.q[l]);
-            scale_words(hbhost::invmod(d, h.q[l]), h.q[l], sc.w[l], sc.c[l]);
+            scale_words(hbhost::invmod(d, h.q[l]), h.q[l], pm, sc.w[l], sc.c[l]);
         }
     }
     for (int l = 0; l < n; ++l) {
         u64 d = 1;
         for (int p : special) d = hbhost::mulmod(d, h.q[p] % h.q[l], h.q[l]);
-        scale_words(hbhost::invmod(d, h.q[l]), h.q[l], c->p_inv_scale.w[l], c->p_inv_scale.c[l]);
+        scale_words(hbhost::invmod(d, h.q[l]), h.q[l], pm, c->p_inv_scale.w[l], c->p_inv_scale.c[l]);
     }
     ConvPlan *d = nullptr;
     CK(cudaMalloc(&d, v.size() * sizeof(ConvPlan)));
@@ -336,8 +343,13 @@ void conv_opt_in(hb_ctx *c) {
     if (c->smem_opt_in_conv) return;
     auto allow = [](auto *kernel, size_t bytes) { CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); };
     const size_t consts = conv_const_bytes(8, kMaxPrimes);
-    allow(conv_cols<8, 4, 1>, strip_bytes<8>(12) + consts); allow(conv_cols<4, 4, 2>, strip_bytes<4>(12) + consts); allow(conv_cols<4, 8, 1>, strip_bytes<4>(16) + consts);
-    allow(conv_cols<8, 2, 2>, strip_bytes<8>(6) + conv_const_bytes(4, kMaxPrimes)); allow(lift_cols<8, 2, 2>, strip_bytes<8>(3)); allow(lift_cols<4, 4, 2>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1>, strip_bytes<4>(9));
+    auto all = [&](auto arithmetic) {
+        using LONG = decltype(arithmetic);
+        allow(conv_cols<8, 4, 1, LONG>, strip_bytes<8>(12) + consts); allow(conv_cols<4, 4, 2, LONG>, strip_bytes<4>(12) + consts); allow(conv_cols<4, 8, 1, LONG>, strip_bytes<4>(16) + consts);
+        allow(conv_cols<8, 2, 2, LONG>, strip_bytes<8>(6) + conv_const_bytes(4, kMaxPrimes));
+        allow(lift_cols<8, 2, 2, LONG>, strip_bytes<8>(3)); allow(lift_cols<4, 4, 2, LONG>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1, LONG>, strip_bytes<4>(9));
+    };
+    if (c->tb.t16.pm) all(LongPm{}); else all(LongShoup{});
     c->smem_opt_in_conv = true;
 }
 // Strip width and groups of a launch over `units` (polynomial, conversion) pairs.  At most two units: narrow strips and many groups, so that
@@ -367,12 +379,16 @@ void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, con
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
         launch(c, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
     };
-    switch (conv_shape(instances * count, max_ns, targets)) {
-    case kStrip8x2: go(conv_cols<8, 2, 2>, 8, 2, strip_bytes<8>(max_ns + 2) + consts); break;
-    case kStrip8x4: go(conv_cols<8, 4, 1>, 8, 4, strip_bytes<8>(max_ns + 4) + consts); break;
-    case kStrip4x4: go(conv_cols<4, 4, 2>, 4, 4, strip_bytes<4>(max_ns + 4) + consts); break;
-    default: go(conv_cols<4, 8, 1>, 4, 8, strip_bytes<4>(max_ns + 8) + consts); break;
-    }
+    auto shapes = [&](auto arithmetic) {
+        using LONG = decltype(arithmetic);
+        switch (conv_shape(instances * count, max_ns, targets)) {
+        case kStrip8x2: go(conv_cols<8, 2, 2, LONG>, 8, 2, strip_bytes<8>(max_ns + 2) + consts); break;
+        case kStrip8x4: go(conv_cols<8, 4, 1, LONG>, 8, 4, strip_bytes<8>(max_ns + 4) + consts); break;
+        case kStrip4x4: go(conv_cols<4, 4, 2, LONG>, 4, 4, strip_bytes<4>(max_ns + 4) + consts); break;
+        default: go(conv_cols<4, 8, 1, LONG>, 4, 8, strip_bytes<4>(max_ns + 8) + consts); break;
+        }
+    };
+    if (c->tb.t16.pm) shapes(LongPm{}); else shapes(LongShoup{});
 }
 // half-inverse limbs of prime `level` (one per instance) -> half-forward lifts to the limbs below
 void launch_lift(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int level, int instances) {
@@ -380,11 +396,15 @@ void launch_lift(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
         launch(c, kernel, dim3(256 / cols, instances), cols * 16 * groups, smem, src, so, dst, dof, level, c->pc, c->tb.t16);
     };
-    switch (lift_shape(instances)) {
-    case kStrip4x8: go(lift_cols<4, 8, 1>, 4, 8, strip_bytes<4>(9)); break;
-    case kStrip4x4: go(lift_cols<4, 4, 2>, 4, 4, strip_bytes<4>(5)); break;
-    default: go(lift_cols<8, 2, 2>, 8, 2, strip_bytes<8>(3)); break;
-    }
+    auto shapes = [&](auto arithmetic) {
+        using LONG = decltype(arithmetic);
+        switch (lift_shape(instances)) {
+        case kStrip4x8: go(lift_cols<4, 8, 1, LONG>, 4, 8, strip_bytes<4>(9)); break;
+        case kStrip4x4: go(lift_cols<4, 4, 2, LONG>, 4, 4, strip_bytes<4>(5)); break;
+        default: go(lift_cols<8, 2, 2, LONG>, 8, 2, strip_bytes<8>(3)); break;
+        }
+    };
+    if (c->tb.t16.pm) shapes(LongPm{}); else shapes(LongShoup{});
 }
 void inv_rows(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int count, const LimbMap &m) {
     LAUNCH(c); CK(launch_inv_rows16(c->st, src, so, dst, dof, count, m, c->pc, c->tb.t16));
@@ -709,7 +729,7 @@ void rescale_core(hb_ctx *c, const u64 *x, u64 *out, int l, int np, int nbp, u64
     const LimbMap lm = one_limb(l);
     if (c->logn == 16) {
         InvScale sc{};
-        for (int i = 0; i < l; ++i) scale_words(hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]), c->h->q[i], sc.w[i], sc.c[i]);
+        for (int i = 0; i < l; ++i) scale_words(hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]), c->h->q[i], c->tb.t16.pm, sc.w[i], sc.c[i]);
         inv_rows(c, x + (size_t)l * N, (size_t)(l + 1) * N, last, (size_t)N, nbp, lm);
         launch_lift(c, last, (size_t)N, t, (size_t)l * N, l, nbp);
         const RowsFin f{x, (size_t)(l + 1) * N, out, (size_t)np * l * N, np, 1, 0};
@@ -1140,6 +1160,8 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
         std::vector<u64> tw(big ? 0 : (size_t)4 * np * N);
         std::vector<ulonglong2> t16(big ? (size_t)2 * np * Ntt16Layout::kEntries : 0);
         std::vector<double> b8(big ? (size_t)2 * np * kRowsB8 : 0);
+        bool pm = big; // every long prime lies within 2^26 below 2^60 (LongPm)
+        for (int i = 0; i < np; ++i) pm = pm && (c->h->q[i] < ((u64)1 << 44) || ((u64)1 << 60) - c->h->q[i] < ((u64)1 << 26));
         for (int i = 0; i < np; ++i) {
             const u64 q = c->h->q[i];
             PrimeConst &p = pcs[i];
@@ -1149,8 +1171,8 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             p.mu_lo = (u64)(((two64 % q) << 64) / q);
             p.n_inv = hbhost::invmod((u64)N, q); p.n_inv_sh = hbhost::shoup(p.n_inv, q);
             p.iu = hbhost::powmod(c->h->psi_root[i], (u64)N / 2, q); p.iu_sh = hbhost::shoup(p.iu, q);
-            scale_words(p.n_inv, q, p.n_inv_w[0], p.n_inv_c[0]);
-            scale_words(hbhost::mulmod(p.n_inv, q - p.iu, q), q, p.n_inv_w[1], p.n_inv_c[1]); // psi^(-N/2) = -psi^(N/2)
+            scale_words(p.n_inv, q, pm, p.n_inv_w[0], p.n_inv_c[0]);
+            scale_words(hbhost::mulmod(p.n_inv, q - p.iu, q), q, pm, p.n_inv_w[1], p.n_inv_c[1]); // psi^(-N/2) = -psi^(N/2)
             // the 2^16 transform carries the residues of primes below 2^44 as integer-valued doubles (ntt16.cuh)
             p.small = (big && q < ((u64)1 << 44)) ? 1 : 0;
             p.q_inv_f = 1.0 / (double)q;
@@ -1170,16 +1192,10 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             p.d60 = below60 < ((u64)1 << 26) ? (u32)below60 : 0;
             std::vector<u64> f, fs, iv, ivs;
             c->h->twiddles(i, f, fs, iv, ivs);
-            if (p.small) { // companion words hold w/q as doubles instead of Shoup quotients
-                for (int k = 0; k < N; ++k) {
-                    double a = (double)f[k] / (double)q, b = (double)iv[k] / (double)q;
-                    std::memcpy(&fs[k], &a, 8); std::memcpy(&ivs[k], &b, 8);
-                }
-            }
             if (big) {
-                auto word = [&](u64 w) { return p.small ? ds_twiddle_word(w) : w; };
-                ntt16_fill_table(&t16[(size_t)i * Ntt16Layout::kEntries], [&](unsigned k) { return make_ulonglong2(word(f[k]), fs[k]); });
-                ntt16_fill_table(&t16[((size_t)np + i) * Ntt16Layout::kEntries], [&](unsigned k) { return make_ulonglong2(word(iv[k]), ivs[k]); });
+                auto entry = [&](u64 w) { ulonglong2 e; scale_words(w, q, pm, e.x, e.y); return e; };
+                ntt16_fill_table(&t16[(size_t)i * Ntt16Layout::kEntries], [&](unsigned k) { return entry(f[k]); });
+                ntt16_fill_table(&t16[((size_t)np + i) * Ntt16Layout::kEntries], [&](unsigned k) { return entry(iv[k]); });
                 if (p.small) {
                     ntt16_fill_rows_b8(&b8[(size_t)i * kRowsB8], [&](unsigned k) { return (double)f[k]; });
                     ntt16_fill_rows_b8(&b8[((size_t)np + i) * kRowsB8], [&](unsigned k) { return (double)iv[k]; });
@@ -1200,7 +1216,7 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             CK(cudaMemcpy(reinterpret_cast<char *>(c->tw) + t16_bytes, b8.data(), b8.size() * sizeof(double), cudaMemcpyHostToDevice));
             const ulonglong2 *t = reinterpret_cast<const ulonglong2 *>(c->tw);
             const double *tb8 = reinterpret_cast<const double *>(reinterpret_cast<const char *>(c->tw) + t16_bytes);
-            c->tb.t16 = Ntt16Tables{t, t + (size_t)np * Ntt16Layout::kEntries, tb8, tb8 + (size_t)np * kRowsB8};
+            c->tb.t16 = Ntt16Tables{t, t + (size_t)np * Ntt16Layout::kEntries, tb8, tb8 + (size_t)np * kRowsB8, pm};
         } else {
             CK(cudaMalloc(&c->tw, tw.size() * 8));
             CK(cudaMemcpy(c->tw, tw.data(), tw.size() * 8, cudaMemcpyHostToDevice));

@@ -48,12 +48,12 @@ __device__ __forceinline__ u64 mul_shoup(u64 x, u64 w, u64 wsh, u64 q) {
     return r >= q ? r - q : r;
 }
 // ---- cheaper lazy forms for the primes of 45 to 60 bits --------------------------------------------------------
-// Measured here (cycles per warp instruction and SM sub-partition): a 32 x 32 -> 64 product 2.1, a low product with a 32-bit addend
-// 2.0, a high word 4.0, the product with a 64-bit addend 5.0 (4.1 as mad.lo.cc + madc.hi), a 64-bit add 2.1; products and shifts
-// overlap, products and adds do not.  The quotient of a Shoup product does not need the exact high product:
-// h = x1 s1 + hi(x0 s1) + hi(x1 s0) is low by less than three, so x*w - h*q lies in [0, 4q) for any x < 2^64.  A radix-16 round of
-// butterflies with it takes 35 (Cooley-Tukey) and 36 (Gentleman-Sande) cycles per warp butterfly; with the exact high
-// product and a conditional subtraction per butterfly 49.
+// Measured here (cycles per warp instruction and SM sub-partition, chains that use both words of a product): a low product with a 32-bit addend 2, a
+// 32 x 32 -> 64 product 4, with a 64-bit addend 5 to 6, a high word 4, a 64-bit add 2; products overlap with separate adds, shifts and FP64
+// instructions (product and FMA 4.4 together), those with a 64-bit addend hardly (7.2).  The quotient of a Shoup product does not need the exact high
+// product: h = x1 s1 + hi(x0 s1) + hi(x1 s0) is low by less than three, so x*w - h*q lies in [0, 4q) for any x < 2^64.  A radix-16 round of
+// butterflies with it takes 37 (Cooley-Tukey) and 39 (Gentleman-Sande) cycles per warp butterfly; with the exact high
+// product and a conditional subtraction per butterfly 49.  Primes next to 2^60 have a cheaper form (LongPm in ntt16.cuh).
 __device__ __forceinline__ u64 mul_shoup4(u64 x, u64 w, u64 wsh, u64 nq /* 2^64 - q */) {
     const u32 x0 = (u32)x, x1 = (u32)(x >> 32), s0 = (u32)wsh, s1 = (u32)(wsh >> 32), w0 = (u32)w, w1 = (u32)(w >> 32), n0 = (u32)nq, n1 = (u32)(nq >> 32);
     const u64 h = (u64)x1 * s1 + (u64)__umulhi(x0, s1) + __umulhi(x1, s0);

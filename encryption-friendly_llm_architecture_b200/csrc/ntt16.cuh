@@ -24,7 +24,7 @@
 //    forward stage (|x| < 9.4 q after 16 stages from a canonical start, far below 2^51).
 //    The pass boundary stores the doubles as they are (the intermediate array is private to the transform); the last
 //    store reduces to the canonical residue, so the bits that reach memory are those of any other exact method.
-//    Primes of 44 bits and more use Shoup butterflies on integers below 16 q.
+//    Primes of 44 bits and more use butterflies on integers below 16 q (LongPm, LongShoup).
 #pragma once
 #include "modarith.cuh"
 #include "pdl.cuh"
@@ -47,13 +47,14 @@ struct Ntt16Layout {
     static __host__ __device__ constexpr int rowsA(int row, int j) { return kRowsA + row * 16 + j; }
     static __host__ __device__ constexpr int rowsB(int row, int j, int clo) { return kRowsB + (row * 15 + j) * 16 + clo; }
 };
-// entry: x = w, y = companion (bits of the double w/q for primes below 2^44, Shoup quotient otherwise)
+// entry: x = w, y = companion, as scale_words makes them: below 2^44 the bits of the doubles w and w/q, otherwise what LongPm or LongShoup multiply by
 struct Ntt16Tables {
     const ulonglong2 *fwd, *inv; // each [nprimes][Ntt16Layout::kEntries]
     // the last round of the row pass for primes below 2^44: the twiddle alone as a double, [nprimes][kRowsB8], entry j of
     // lane clo of row `row` at (row * 15 + j) * 16 + clo -- half the bytes of the 16-byte entries, and in that round every
     // thread reads 15 twiddles nobody else uses (more bytes than the coefficients themselves)
     const double *fwdB8, *invB8;
+    bool pm; // the constants of the primes of 45 bits and more are those of LongPm
 };
 constexpr int kRowsB8 = 256 * 15 * 16;
 
@@ -126,69 +127,141 @@ __device__ __forceinline__ void gs_bfly(u64 &x, u64 &y, u64 w, u64 ws, u64 q, u6
     x = s >= q2 ? s - q2 : s;
     y = mul_shoup_lazy(d, w, ws, q);
 }
-struct IntConst {
-    u64 q, nq, q4, q8;
-    FoldQ f;
+// The arithmetic of the primes of 45 bits and more in these kernels, as a policy: LongPm where every such prime of the context lies within 2^26 below
+// 2^60, as the first primes below it do, otherwise LongShoup.  Both keep values below 16 q in 64 bits and multiply by constants that come as two words.
+struct LongShoup {
+    struct Const { u64 q, nq, q4, q8; FoldQ f; };
+    static __device__ __forceinline__ Const make(const PrimeConst &m) {
+        Const c;
+        c.q = m.q; c.nq = 0ull - m.q; c.q4 = m.q << 2; c.q8 = m.q << 3;
+        c.f.shift = m.fold_shift; c.f.mask = (1u << m.fold_shift) - 1u; c.f.d = m.fold_d;
+        return c;
+    }
+    static __device__ __forceinline__ u64 mul(u64 x, u64 w, u64 comp, const Const &c) { return mul_shoup4(x, w, comp, c.nq); } // any x -> below 4q
+    static __device__ __forceinline__ u64 canon(u64 x, const Const &c) { return canon_q(x, c.q, c.f); }
+    static __device__ __forceinline__ u64 above(const Const &c) { return c.q8; } // a multiple of q above what a forward transform leaves (5q)
+    // Four Cooley-Tukey stages on 16 register values; twiddles tp[j].
+    // A stage adds 4q to the bound B of the values; x is folded below ~2^b before the additions of the stages named by the bit mask FOLD.
+    // The words hold 16 q: in units of q the four rounds of a transform (masks 8, 4, 2, 9) run 3-7-11-15|5, 5-9-13|5-9, 9-13|5-9-13, 13|5-9-13|5 (| = a fold).
+    // MADE: the upper half already carries the twiddle of the first stage (values below 4q)
+    template <int ROUND, bool MADE = false, class TW> static __device__ __forceinline__ void fwd16(u64 (&v)[16], const TW &tp, const Const &c) {
+        constexpr int FOLD = ROUND == 0 ? 8 : ROUND == 1 ? 4 : ROUND == 2 ? 2 : 9;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const int half = 8 >> s;
+#pragma unroll
+            for (int g = 0; g < (1 << s); ++g) {
+                const ulonglong2 tw = tp[(1 << s) - 1 + g];
+#pragma unroll
+                for (int j = 0; j < half; ++j) {
+                    u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
+                    const u64 t = MADE && s == 0 ? y : mul(y, tw.x, tw.y, c);
+                    if ((FOLD >> s) & 1) x = fold_q(x, c.f);
+                    y = x + c.q4 - t;
+                    x = x + t;
+                }
+            }
+        }
+    }
+    // Four Gentleman-Sande stages, the mirror image.  Values enter and leave below 4q: sums reach 8q, then 16q, and are folded at
+    // every second stage.  LAST: the stage to end with
+    template <int LAST = 0, class TW> static __device__ __forceinline__ void inv16(u64 (&v)[16], const TW &tp, const Const &c) {
+#pragma unroll
+        for (int s = 3; s >= LAST; --s) {
+            const int half = 8 >> s;
+#pragma unroll
+            for (int g = 0; g < (1 << s); ++g) {
+                const ulonglong2 tw = tp[(1 << s) - 1 + g];
+#pragma unroll
+                for (int j = 0; j < half; ++j) {
+                    u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
+                    const u64 d = x + ((s & 1) ? c.q4 : c.q8) - y, a = x + y;
+                    x = (s & 1) ? a : fold_q(a, c.f);
+                    y = mul(d, tw.x, tw.y, c);
+                }
+            }
+        }
+    }
 };
-__device__ __forceinline__ IntConst int_const(const PrimeConst &m) {
-    IntConst c;
-    c.q = m.q; c.nq = 0ull - m.q; c.q4 = m.q << 2; c.q8 = m.q << 3;
-    c.f.shift = m.fold_shift; c.f.mask = (1u << m.fold_shift) - 1u; c.f.d = m.fold_d;
-    return c;
-}
-// Four Cooley-Tukey stages on 16 register values; twiddles tp[j].
-// Products are below 4q (mul_shoup4), so a stage adds 4q to the bound B of the values; x is folded below ~2^b before the
-// additions of the stages named by the bit mask FOLD.  The words hold 16 q: in units of q the four rounds of a transform
-// (masks 8, 4, 2, 9) run 3-7-11-15|5, 5-9-13|5-9, 9-13|5-9-13, 13|5-9-13|5 (| = a fold).
-// MADE: the upper half already carries the twiddle of the first stage (values below 4q)
-template <int FOLD, bool MADE = false, class TW> __device__ __forceinline__ void fwd16_int(u64 (&v)[16], const TW &tp, const IntConst &c) {
+// Primes q = 2^60 - d, d < 2^26.  A constant w comes as its two pieces and those of w' = w * 2^32 mod q (29 low and 31 high bits in the words of a u64), so
+// that x * w = x0 w + x1 w' = A + B * 2^29 takes the words of x as they are, and B = Bl + Bh * 2^32 folds by 2^61 = 2d the same way: A + Bl * 2^29 + Bh * 2d.
+// Six 32 x 32 products instead of the Shoup form's five and four low ones, and no carries in between: 11.5 instructions a butterfly against 21.
+// In units of 2^60, for x below X: A < 2 + X/8, Bl * 2^29 < 2, Bh * 2d < 1/2: below 4.5 + X/8, 6.5 for any x.
+// A radix-16 round, cycles per warp butterfly and scheduler with four warps: 29 against 37 (Cooley-Tukey), 35 against 39 (Gentleman-Sande); half of the warps
+// in FP64 butterflies: 19 on average against 26, as products with 64-bit addends leave FP64 products few issue slots.
+struct LongPm {
+    struct Const { u64 q, q7; u32 d, d2; };
+    static __device__ __forceinline__ Const make(const PrimeConst &m) {
+        Const c;
+        c.q = m.q; c.q7 = m.q * 7; c.d = m.d60; c.d2 = 2 * m.d60;
+        return c;
+    }
+    // separate instructions: the compiler would join most of them to products with 64-bit addends, which take longer than both (33 cycles a butterfly)
+    static __device__ __forceinline__ u64 add(u64 a, u64 b) { u64 r; asm volatile("add.u64 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+    static __device__ __forceinline__ u64 wide(u32 a, u32 b) { u64 r; asm("mul.wide.u32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b)); return r; }
+    static __device__ __forceinline__ u64 mul(u64 x, u64 w, u64 comp, const Const &c) {
+        const u32 x0 = (u32)x, x1 = (u32)(x >> 32);
+        const u64 a = add(wide(x1, (u32)comp), wide(x0, (u32)w)), b = add(wide(x1, (u32)(comp >> 32)), wide(x0, (u32)(w >> 32)));
+        return add(add(a, wide((u32)b, 1u << 29)), wide((u32)(b >> 32), c.d2));
+    }
+    // x < 16 * 2^60 -> congruent value below 2^60 + 2^30
+    static __device__ __forceinline__ u64 fold(u64 x, const Const &c) {
+        const u32 hi = (u32)(x >> 32);
+        return (((u64)(hi & 0x0FFFFFFFu) << 32) | (u32)x) + (hi >> 28) * c.d;
+    }
+    static __device__ __forceinline__ u64 canon(u64 x, const Const &c) {
+        const u64 r = fold(x, c);
+        return r >= c.q ? r - c.q : r;
+    }
+    static __device__ __forceinline__ u64 above(const Const &c) { return c.q7 + 2 * c.q; }
+    // x is folded before the additions of every second stage; differences are taken from 7q, above every product.  Bounds (units of 2^60) alternate: 8.1 behind
+    // a stage with a fold, 15.1 behind one without, whose products are below 4.5 + 15.1 / 8 = 6.4.
+    // MADE: the upper half already carries the twiddle of the first stage (both halves below 3q)
+    template <int ROUND, bool MADE = false, class TW> static __device__ __forceinline__ void fwd16(u64 (&v)[16], const TW &tp, const Const &c) {
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        const int half = 8 >> s;
+        for (int s = 0; s < 4; ++s) {
+            const int half = 8 >> s;
 #pragma unroll
-        for (int g = 0; g < (1 << s); ++g) {
-            const ulonglong2 tw = tp[(1 << s) - 1 + g];
+            for (int g = 0; g < (1 << s); ++g) {
+                const ulonglong2 tw = tp[(1 << s) - 1 + g];
 #pragma unroll
-            for (int j = 0; j < half; ++j) {
-                u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
-                const u64 t = MADE && s == 0 ? y : mul_shoup4(y, tw.x, tw.y, c.nq);
-                if ((FOLD >> s) & 1) x = fold_q(x, c.f);
-                y = x + c.q4 - t;
-                x = x + t;
+                for (int j = 0; j < half; ++j) {
+                    u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
+                    const u64 t = MADE && s == 0 ? y : mul(y, tw.x, tw.y, c);
+                    if (s & 1) x = fold(x, c);
+                    y = x + c.q7 - t;
+                    x = x + t;
+                }
             }
         }
     }
-}
-constexpr int kFoldColsA = 8, kFoldColsB = 4, kFoldRowsA = 2, kFoldRowsB = 9;
-// Four Gentleman-Sande stages, the mirror image.  Values enter and leave below 4q: sums reach 8q, then 16q, and are folded at
-// every second stage.
-// LAST: the stage to end with
-template <int LAST = 0, class TW> __device__ __forceinline__ void inv16_int(u64 (&v)[16], const TW &tp, const IntConst &c) {
+    // Values enter and leave below 6.3: sums (below 12.6) are folded at every stage, products of differences (below 13.3) are below 4.5 + 13.3 / 8.
+    template <int LAST = 0, class TW> static __device__ __forceinline__ void inv16(u64 (&v)[16], const TW &tp, const Const &c) {
 #pragma unroll
-    for (int s = 3; s >= LAST; --s) {
-        const int half = 8 >> s;
+        for (int s = 3; s >= LAST; --s) {
+            const int half = 8 >> s;
 #pragma unroll
-        for (int g = 0; g < (1 << s); ++g) {
-            const ulonglong2 tw = tp[(1 << s) - 1 + g];
+            for (int g = 0; g < (1 << s); ++g) {
+                const ulonglong2 tw = tp[(1 << s) - 1 + g];
 #pragma unroll
-            for (int j = 0; j < half; ++j) {
-                u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
-                const u64 d = x + ((s & 1) ? c.q4 : c.q8) - y, a = x + y;
-                x = (s & 1) ? a : fold_q(a, c.f);
-                y = mul_shoup4(d, tw.x, tw.y, c.nq);
+                for (int j = 0; j < half; ++j) {
+                    u64 &x = v[g * 2 * half + j], &y = v[g * 2 * half + j + half];
+                    const u64 d = x + c.q7 - y, a = x + y;
+                    x = fold(a, c);
+                    y = mul(d, tw.x, tw.y, c);
+                }
             }
         }
     }
-}
-
+};
 // The last stage of an inverse transform together with the multiplication by N^-1 (or another constant): its only twiddle goes into the
 // constant of the differences, so that the stage costs no products of its own.  sw, sc: constant, constant * twiddle.  store(e, canonical).
-template <class STORE> __device__ __forceinline__ void inv16_int_last(const u64 (&v)[16], const u64 (&sw)[2], const u64 (&sc)[2], const IntConst &c, STORE &&store) {
+template <class LONG, class STORE> __device__ __forceinline__ void inv16_int_last(const u64 (&v)[16], const u64 (&sw)[2], const u64 (&sc)[2], const typename LONG::Const &c, STORE &&store) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) { // below 8q before, sums and differences below 16q
-        const u64 a = v[j] + v[j + 8], d = v[j] + c.q8 - v[j + 8];
-        store(j, canon_q(mul_shoup4(a, sw[0], sc[0], c.nq), c.q, c.f));
-        store(j + 8, canon_q(mul_shoup4(d, sw[1], sc[1], c.nq), c.q, c.f));
+        const u64 a = v[j] + v[j + 8], d = v[j] + LONG::above(c) - v[j + 8];
+        store(j, LONG::canon(LONG::mul(a, sw[0], sc[0], c), c));
+        store(j + 8, LONG::canon(LONG::mul(d, sw[1], sc[1], c), c));
     }
 }
 
@@ -329,7 +402,7 @@ template <class STORE> __device__ __forceinline__ void inv16_ds_last(const doubl
 }
 
 // ---- forward, column pass: stages 1..8 ----
-template <int MINB>
+template <int MINB, class LONG>
 __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_cols(const u64 *src, LimbAddr16 sa, u64 *dst, LimbAddr16 da,
                                                         const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     __shared__ u64 sm[4096];
@@ -361,21 +434,21 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_cols(const u64 *src, Li
         pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = p[(e * 16 + sub) * 256];
-        const IntConst c = int_const(m);
-        fwd16_int<kFoldColsA>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
+        const typename LONG::Const c = LONG::make(m);
+        LONG::template fwd16<0>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[(e * 16 + sub) * 16 + lane] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[(sub * 16 + e) * 16 + lane];
-        fwd16_int<kFoldColsB>(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
+        LONG::template fwd16<1>(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) o[(sub * 16 + e) * 256] = v[e];
     }
 }
 
 // ---- forward, row pass: stages 9..16; stores canonical residues ----
-template <int MINB>
+template <int MINB, class LONG>
 __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows(const u64 *src, LimbAddr16 sa, u64 *dst, LimbAddr16 da,
                                                         const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     __shared__ u64 sm[16 * kRowStride];
@@ -407,21 +480,21 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows(const u64 *src, Li
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = ds_store(v[e], c, shift, qinv_up); // the words this thread read itself
     } else {
-        const IntConst c = int_const(m);
+        const typename LONG::Const c = LONG::make(m);
         u64 v[16];
         const TwiddlesB<ulonglong2, MINB <= 2> tw(tab + Ntt16Layout::rowsB(row, 0, clo));
         pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = p[e * 16];
-        fwd16_int<kFoldRowsA>(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
+        LONG::template fwd16<2>(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
-        fwd16_int<kFoldRowsB>(v, tw, c);
+        LONG::template fwd16<3>(v, tw, c);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = canon_q(v[e], c.q, c.f);
+        for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = LONG::canon(v[e], c);
     }
     __syncthreads();
 #pragma unroll
@@ -429,7 +502,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows(const u64 *src, Li
 }
 
 // ---- inverse, row pass: undoes stages 16..9 ----
-template <int MINB>
+template <int MINB, class LONG>
 __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_rows(const u64 *src, LimbAddr16 sa, u64 *dst, LimbAddr16 da,
                                                         const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     __shared__ u64 sm[16 * kRowStride];
@@ -471,21 +544,21 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_rows(const u64 *src, Li
         u64 v[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
-        const IntConst c = int_const(m);
-        inv16_int(v, tw, c);
+        const typename LONG::Const c = LONG::make(m);
+        LONG::inv16(v, tw, c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[e * 17 + clo];
-        inv16_int(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
+        LONG::inv16(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) o[e * 16] = v[e];
     }
 }
 
 // ---- inverse, column pass: undoes stages 8..1, scales by N^-1, stores canonical residues ----
-template <int MINB>
+template <int MINB, class LONG>
 __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *src, LimbAddr16 sa, u64 *dst, LimbAddr16 da,
                                                         const __grid_constant__ LimbMap map, const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     __shared__ u64 sm[4096];
@@ -516,15 +589,15 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *src, Li
         pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = p[(sub * 16 + e) * 256];
-        const IntConst c = int_const(m);
-        inv16_int(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
+        const typename LONG::Const c = LONG::make(m);
+        LONG::inv16(v, TwiddlesA(tab + Ntt16Layout::colsB(sub, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[(sub * 16 + e) * 16 + lane] = v[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[(e * 16 + sub) * 16 + lane];
-        inv16_int<1>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
-        inv16_int_last(v, m.n_inv_w, m.n_inv_c, c, [&](int e, u64 w) { o[(e * 16 + sub) * 256] = w; });
+        LONG::template inv16<1>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
+        inv16_int_last<LONG>(v, m.n_inv_w, m.n_inv_c, c, [&](int e, u64 w) { o[(e * 16 + sub) * 256] = w; });
     }
 }
 
@@ -537,9 +610,12 @@ inline cudaError_t launch_ntt16(cudaStream_t st, const u64 *src, size_t src_oute
     if (count == 0) return cudaSuccess;
     LimbAddr16 sa{src_outer}, da{dst_outer};
     dim3 grid(16, count);
-    const cudaError_t e = inverse ? launch_pdl(st, ntt16v2_inv_rows<MINB>, grid, 256, 0, src, sa, dst, da, map, pc, tb) : launch_pdl(st, ntt16v2_fwd_cols<MINB>, grid, 256, 0, src, sa, dst, da, map, pc, tb);
-    if (e != cudaSuccess) return e;
-    return inverse ? launch_pdl(st, ntt16v2_inv_cols<MINB>, grid, 256, 0, dst, da, dst, da, map, pc, tb) : launch_pdl(st, ntt16v2_fwd_rows<MINB>, grid, 256, 0, dst, da, dst, da, map, pc, tb);
+    auto passes = [&](auto *first, auto *second) {
+        const cudaError_t e = launch_pdl(st, first, grid, 256, 0, src, sa, dst, da, map, pc, tb);
+        return e != cudaSuccess ? e : launch_pdl(st, second, grid, 256, 0, dst, da, dst, da, map, pc, tb);
+    };
+    if (tb.pm) return inverse ? passes(ntt16v2_inv_rows<MINB, LongPm>, ntt16v2_inv_cols<MINB, LongPm>) : passes(ntt16v2_fwd_cols<MINB, LongPm>, ntt16v2_fwd_rows<MINB, LongPm>);
+    return inverse ? passes(ntt16v2_inv_rows<MINB, LongShoup>, ntt16v2_inv_cols<MINB, LongShoup>) : passes(ntt16v2_fwd_cols<MINB, LongShoup>, ntt16v2_fwd_rows<MINB, LongShoup>);
 }
 
 } // namespace hb
