@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(256, EL == 1 ? 4 : ND <= 2 ? 3 : 2) k_ks_inner
             for (int u = 0; u < EL; ++u)
 #pragma unroll
                 for (int p = 0; p < 2; ++p) {
-                    PieceAcc s; s.zero(); // at most eight digits
+                    PieceAccT<true> s; s.zero(); // at most eight digits
 #pragma unroll
                     for (int d = 0; d < ND; ++d) s.mac(v0[d][u], v1[d][u], k0[d][p][u], k1[d][p][u]);
                     o[(size_t)p * opoly + u * 256] = s.finish(m);
@@ -1289,7 +1289,7 @@ __device__ __forceinline__ void ks_inner_mkr_body(u64 *o, const u64 *c0, const u
         } else {
 #pragma unroll
             for (int u = 0; u < EL; ++u) {
-                PieceAcc s0, s1; s0.zero(); s1.zero(); // at most six products
+                PieceAccT<true> s0, s1; s0.zero(); s1.zero(); // at most six products
 #pragma unroll
                 for (int r = 0; r < CNT; ++r) {
 #pragma unroll

@@ -217,6 +217,13 @@ __device__ __forceinline__ u64 mad_wide(u32 a, u32 b, u64 c) {
     asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
     return r;
 }
+// the same as two instructions that the compiler does not join
+__device__ __forceinline__ u64 mul_add_wide(u32 a, u32 b, u64 c) {
+    u64 t, r;
+    asm("mul.wide.u32 %0, %1, %2;" : "=l"(t) : "r"(a), "r"(b));
+    asm volatile("add.u64 %0, %1, %2;" : "=l"(r) : "l"(t), "l"(c));
+    return r;
+}
 // a0 + a1 * 2^30 + a2 * 2^60 modulo a prime of 45 to 60 bits (a0, a1 + 2^34, a2 + 2^34 < 2^64): below 3q
 __device__ __forceinline__ u64 finish_wide(u64 a0, u64 a1, u64 a2, const PrimeConst &m) {
     const u32 m30 = 0x3FFFFFFFu;
@@ -236,11 +243,14 @@ __device__ __forceinline__ u64 finish_wide(u64 a0, u64 a1, u64 a2, const PrimeCo
 }
 // Karatsuba: the middle products come from one product of the sums of the pieces, from which the outer two are taken off at the end (modulo
 // 2^64, which the true sum a1 does not reach): three multiply-adds and two 32-bit additions, of which the compiler makes one per factor.
-struct PieceAcc {
+// SPLIT: products and additions apart, which lets FP64 products of other warps in between (see mul_shoup4) and takes more registers.  Layer pass:
+// masked sums 62.4 -> 57.9 ms, inner products of three digits 8.9 -> 8.7; but part sums (which then spill) 32.3 -> 37.0, rotation sums 7.1 -> 7.6.
+template <bool SPLIT> struct PieceAccT {
     u64 a0, am, a2; // weights 1 and 2^60 of the outer products; am = a0 + a1 + a2 modulo 2^64, a1 of weight 2^30
     __device__ __forceinline__ void zero() { a0 = am = a2 = 0; }
     __device__ __forceinline__ void mac(u32 v0, u32 v1, u32 k0, u32 k1) { // 30-bit pieces of the factors
-        a0 = mad_wide(v0, k0, a0); am = mad_wide(v0 + v1, k0 + k1, am); a2 = mad_wide(v1, k1, a2);
+        if (SPLIT) { a0 = mul_add_wide(v0, k0, a0); am = mul_add_wide(v0 + v1, k0 + k1, am); a2 = mul_add_wide(v1, k1, a2); }
+        else { a0 = mad_wide(v0, k0, a0); am = mad_wide(v0 + v1, k0 + k1, am); a2 = mad_wide(v1, k1, a2); }
     }
     __device__ __forceinline__ void mac(u64 v, u64 k) { mac((u32)v & 0x3FFFFFFFu, (u32)(v >> 30), (u32)k & 0x3FFFFFFFu, (u32)(k >> 30)); } // v, k < 2^60
     // after at most eight products: makes room for eight more
@@ -253,6 +263,7 @@ struct PieceAcc {
         return canon_q(r, m.q, FoldQ{m.fold_shift, (1u << m.fold_shift) - 1u, m.fold_d});
     }
 };
+using PieceAcc = PieceAccT<false>;
 
 // index of the source slot of the automorphism X -> X^g on an NTT-form limb:
 //   out[i] = in[ntt_perm(i)], exponents 2*bitrev(i)+1 multiply by g modulo 2N
