@@ -269,9 +269,9 @@ i64 direct_group(const Ciphertext &x) { return std::max<i64>(1, std::min<i64>(8,
 // In kFaithful every shifted copy is the previous one rotated once more: the chains of one loop (an operand and its wrapped copy,
 // of one or both operands) advance side by side as the member groups of one ciphertext.
 struct Chains {
-    Ciphertext x;
+    std::shared_ptr<const Ciphertext> x;
     std::vector<i64> steps;
-    void advance(Env &e) { x = e.ev.leftRotateGroups(x, steps); }
+    void advance(Env &e) { x = std::make_shared<const Ciphertext>(e.ev.leftRotateGroups(*x, steps)); }
     int count() const { return (int)steps.size(); }
 };
 // operand k: groups 2k (rotated by step[k]) and 2k + 1 (that, rotated by -back[k])
@@ -289,8 +289,59 @@ Chains start_chains(Env &e, const std::vector<const Ciphertext *> &ops, const st
         all.push_back(e.ev.group(main, k, n)); all.push_back(e.ev.group(wrapped, k, n));
         c.steps.push_back(step[(size_t)k]); c.steps.push_back(step[(size_t)k]);
     }
-    c.x = stack(std::move(all));
+    c.x = std::make_shared<const Ciphertext>(stack(std::move(all)));
     return c;
+}
+
+// Only the rotations of a chain wait for one another; the masked sums of several iterations are made by one launch sequence (few members leave
+// most of the GPU idle in each of its five launches): up to 32 polynomials of sums, and what the terms of a call allow.  One product of one
+// tile 42.8 -> 39.3 ms.
+class HeldChains {
+  public:
+    HeldChains(Env &e, const Chains &c) : e_(e), sums_(c.count() / 2), hold_(std::max(1, std::min(Evaluator::kMaxSumTerms / c.count(), 32 * c.count() / (2 * sums_ * c.x->getBatch())))) {}
+    // the chains as they are now, with the masks of their groups
+    void add(const Chains &c, std::vector<const Plaintext *> masks) { x_.push_back(c.x); masks_.push_back(std::move(masks)); }
+    bool full() const { return held() == hold_; }
+    int held() const { return (int)x_.size(); }
+    // sum s (groups 2s and 2s + 1, masked) of held iteration k is member group s * held() + k
+    Ciphertext take() {
+        std::vector<Ciphertext> terms;
+        std::vector<const Plaintext *> masks;
+        for (int s = 0; s < sums_; ++s)
+            for (size_t k = 0; k < x_.size(); ++k)
+                for (int r = 2 * s; r < 2 * s + 2; ++r) { terms.push_back(e_.ev.group(*x_[k], r, 2 * sums_)); masks.push_back(masks_[k][(size_t)r]); }
+        Ciphertext out = e_.ev.multSums(terms, masks, 2);
+        x_.clear(); masks_.clear();
+        return out;
+    }
+  private:
+    Env &e_;
+    int sums_, hold_;
+    std::vector<std::shared_ptr<const Ciphertext>> x_;
+    std::vector<std::vector<const Plaintext *>> masks_;
+};
+// acc += sum over i of tensor(masked chains of the first operand, of the second), i from 1 to `end`; masks(i): those of the four groups
+template <class MASKS> Ciphertext tensor_chains(Env &e, Chains c, i64 end, MASKS &&masks) {
+    Ciphertext acc;
+    HeldChains held(e, c);
+    for (i64 i = 1; i < end; ++i) {
+        if (i > 1) c.advance(e);
+        held.add(c, masks(i));
+        if (!held.full() && i + 1 < end) continue;
+        const int n = held.held();
+        const Ciphertext s = held.take();
+        e.ev.tensorAccumulateGroups(acc, e.ev.group(s, 0, 2), e.ev.group(s, 1, 2), n);
+    }
+    return acc;
+}
+// the masked copies of one chain for i from 1 to `end`, in order, appended to `copies`
+template <class MASKS> void masked_copies(Env &e, Chains c, i64 end, std::vector<Ciphertext> &copies, MASKS &&masks) {
+    HeldChains held(e, c);
+    for (i64 i = 1; i < end; ++i) {
+        if (i > 1) c.advance(e);
+        held.add(c, masks(i));
+        if (held.full() || i + 1 == end) copies.push_back(held.take());
+    }
 }
 
 void require_product_shapes(const CtxtTensor &a, const CtxtTensor &b) {
@@ -424,11 +475,9 @@ CtxtTensor ccmmCore(Env &e, Ciphertext a, Ciphertext b, i64 num_rows, i64 inner,
             e.ev.tensorAccumulateGroups(acc, ak, bk, (int)count);
         }
     } else {
-        Chains c = start_chains(e, {&a, &b}, {1, width}, {cols_tmp, rows_tmp * width});
-        for (i64 i = 1; i < num_k; ++i) {
-            if (i > 1) c.advance(e);
-            e.ev.tensorAccumulateHalves(acc, e.ev.multSumGrouped(c.x, {&col_wrap(e, sa, 2 * i + 1, lvl), &col_wrap(e, sa, 2 * i, lvl), &row_wrap(e, sb, 2 * i + 1, lvl), &row_wrap(e, sb, 2 * i, lvl)}, 2, 2));
-        }
+        acc = tensor_chains(e, start_chains(e, {&a, &b}, {1, width}, {cols_tmp, rows_tmp * width}), num_k, [&](i64 i) {
+            return std::vector<const Plaintext *>{&col_wrap(e, sa, 2 * i + 1, lvl), &col_wrap(e, sa, 2 * i, lvl), &row_wrap(e, sb, 2 * i + 1, lvl), &row_wrap(e, sb, 2 * i, lvl)};
+        });
     }
     res = e.ev.add(res, e.ev.rescale(e.ev.relinearize(acc)));
     return CtxtTensor(TileTensorShape(num_rows, num_cols, width), std::move(res));
@@ -471,7 +520,7 @@ CtxtTensor multMatMatCP(Env &e, const CtxtTensor &op1, const PtxtTensor &op2, in
             c.advance(e);
             b = e.ev.leftRotate(b, width); b_wrap = e.ev.leftRotate(b_wrap, width);
         }
-        Ciphertext ak = e.ev.multSumGrouped(c.x, {&col_wrap(e, sa, 2 * i + 1, lvl), &col_wrap(e, sa, 2 * i, lvl)}, 2, 1);
+        Ciphertext ak = e.ev.multSumGrouped(*c.x, {&col_wrap(e, sa, 2 * i + 1, lvl), &col_wrap(e, sa, 2 * i, lvl)}, 2, 1);
         Plaintext bk = e.ev.add(e.ev.mult(b, row_wrap(e, sb, 2 * i + 1, lvl)), e.ev.mult(b_wrap, row_wrap(e, sb, 2 * i, lvl)));
         Ciphertext term = e.ev.mult(ak, bk);
         acc = acc.empty() ? std::move(term) : e.ev.add(acc, term);
@@ -507,7 +556,7 @@ CtxtTensor multPackedMatMat(Env &e, const CtxtTensor &op1, const CtxtTensor &op2
         b = e.ev.leftRotate(b, 2 * width);
         for (i64 i = 1; i < num_k / 2; ++i) {
             if (i > 1) { c.advance(e); b = e.ev.leftRotate(b, 2 * width); }
-            e.ev.tensorAccumulate(acc, e.ev.multSumGrouped(c.x, {&col_wrap(e, sa, 4 * i + 1, lvl), &col_wrap(e, sa, 4 * i, lvl)}, 2, 1), b);
+            e.ev.tensorAccumulate(acc, e.ev.multSumGrouped(*c.x, {&col_wrap(e, sa, 4 * i + 1, lvl), &col_wrap(e, sa, 4 * i, lvl)}, 2, 1), b);
         }
     }
     res = e.ev.add(res, e.ev.rescale(e.ev.relinearize(acc)));
@@ -532,12 +581,10 @@ Ciphertext multPackedMatMatPreRot(Env &e, const CtxtTensor &in, int target_level
                                            [&](i64 w) -> const Plaintext & { return col_wrap(e, shp, 2 * w - (w % 2), lvl); }));
         return e.ev.concat(copies);
     }
-    Chains c = start_chains(e, {&in.get()}, {2}, {num_rows});
-    for (i64 i = 1; i < num_rows / 2; ++i) {
-        if (i > 1) c.advance(e);
-        copies.push_back(e.ev.multSumGrouped(c.x, {&col_wrap(e, shp, 4 * i + 1, lvl), &col_wrap(e, shp, 4 * i, lvl)}, 2, 1));
-    }
-    return e.ev.stack(copies);
+    masked_copies(e, start_chains(e, {&in.get()}, {2}, {num_rows}), num_rows / 2, copies, [&](i64 i) {
+        return std::vector<const Plaintext *>{&col_wrap(e, shp, 4 * i + 1, lvl), &col_wrap(e, shp, 4 * i, lvl)};
+    });
+    return e.ev.concat(copies);
 }
 // multPackedMatMatPreRev -- MatrixUtils.cpp:1266-1274
 CtxtTensor multPackedMatMatPreRev(Env &e, const CtxtTensor &b, int target_level) {
@@ -579,7 +626,7 @@ Ciphertext multMatMatPre(Env &e, const CtxtTensor &in, int target_level) {
     const i64 num_rows = in.getHeight();
     const int lvl = target_level + 2;
     CtxtTensor s = diagonalToColumn(e, CtxtTensor(in.getShape(), e.ev.levelDown(in.get(), target_level + 3)));
-    if (e.mode == kLazy) { // a group of copies comes out copy-major, as stack() lays them, so each goes straight to its place
+    if (e.mode == kLazy) { // a group of copies comes out copy-major, as concat() would lay them, so each goes straight to its place
         const Hoisted h = e.ev.decompose(s.get());
         const int batch = s.get().getBatch();
         Ciphertext pre = e.ev.room(s.get().getLevel() - 1, (int)num_rows * batch, e.ev.levelDownOne(s.get()));
@@ -605,12 +652,10 @@ Ciphertext multMatMatPre(Env &e, const CtxtTensor &in, int target_level) {
                                            [&](i64 w) -> const Plaintext & { return col_wrap(e, shp, w, lvl); }));
         return e.ev.concat(copies);
     }
-    Chains c = start_chains(e, {&s.get()}, {1}, {num_rows});
-    for (i64 i = 1; i < num_rows; ++i) {
-        if (i > 1) c.advance(e);
-        copies.push_back(e.ev.multSumGrouped(c.x, {&col_wrap(e, shp, 2 * i + 1, lvl), &col_wrap(e, shp, 2 * i, lvl)}, 2, 1));
-    }
-    return e.ev.stack(copies);
+    masked_copies(e, start_chains(e, {&s.get()}, {1}, {num_rows}), num_rows, copies, [&](i64 i) {
+        return std::vector<const Plaintext *>{&col_wrap(e, shp, 2 * i + 1, lvl), &col_wrap(e, shp, 2 * i, lvl)};
+    });
+    return e.ev.concat(copies);
 }
 // multMatMatReUse -- MatrixUtils.cpp:1612-1639: one fused pass over the shifted copies
 CtxtTensor multMatMatReUse(Env &e, const Ciphertext &pre, const PtxtTensor &w) {
@@ -668,12 +713,9 @@ CtxtTensor low_rank_tail(Env &e, Ciphertext a, Ciphertext b, const TileTensorSha
     const i64 num_rows = s1.getNumRows();
     Ciphertext res = e.ev.mult(a, b);
     if (low_dim > 1) {
-        Chains c = start_chains(e, {&a, &b}, {1, width}, {width / 2, num_rows * width});
-        Ciphertext acc;
-        for (i64 i = 1; i < low_dim; ++i) {
-            if (i > 1) c.advance(e);
-            e.ev.tensorAccumulateHalves(acc, e.ev.multSumGrouped(c.x, {&col_wrap(e, s1, 2 * i + 1, lvl), &col_wrap(e, s1, 2 * i, lvl), &row_wrap(e, s2, 2 * i + 1, lvl), &row_wrap(e, s2, 2 * i, lvl)}, 2, 2));
-        }
+        Ciphertext acc = tensor_chains(e, start_chains(e, {&a, &b}, {1, width}, {width / 2, num_rows * width}), low_dim, [&](i64 i) {
+            return std::vector<const Plaintext *>{&col_wrap(e, s1, 2 * i + 1, lvl), &col_wrap(e, s1, 2 * i, lvl), &row_wrap(e, s2, 2 * i + 1, lvl), &row_wrap(e, s2, 2 * i, lvl)};
+        });
         res = e.ev.add(res, e.ev.rescale(e.ev.relinearize(acc)));
     }
     return CtxtTensor(TileTensorShape(s1.getNumRows(), s2.getNumCols(), s2.getBlockWidth()), std::move(res));

@@ -1872,6 +1872,14 @@ int hb_sum_mul_pt_rescale_grouped(hb_ctx *c, const hb_ct *x, const hb_pt *const 
         *out = do_prod_rescale(c, a.data(), p, count, false, sums);
     });
 }
+int hb_sum_mul_pt_rescale_many(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, int count, int sums, hb_ct **out) {
+    return guard(c, [&] {
+        if (!a || !p || !out || count < 1 || sums < 1) fail(HB_E_ARG, "product sums: bad arguments");
+        if (count > kMaxTerms || sums > kMaxTerms || count * sums > kMaxTerms) fail(HB_E_LIMIT, "product sum: between 1 and " + std::to_string(kMaxTerms) + " terms");
+        for (int k = 0; k < count * sums; ++k) if (!a[k] || !p[k]) fail(HB_E_ARG, "product sums: null operand");
+        *out = do_prod_rescale(c, a, p, count, false, sums);
+    });
+}
 int hb_tensor_acc_halves(hb_ctx *c, const hb_ct *x, hb_ct **acc) {
     return guard(c, [&] {
         const std::vector<hb_ct> v = group_views(c, x, 2);

@@ -250,6 +250,8 @@ int hb_mul_pt_sum_parts_each(hb_ctx *ctx, const hb_ct *const *a, const hb_pt *co
 /* out_k = rescale(sum_{j < count} x_{k * count + j} (.) p[k * count + j]) for k < sums, where x_i is member group i of x (count * sums
  * groups, at most 24); out holds sums * batch / (count * sums) members, sum-major */
 int hb_sum_mul_pt_rescale_grouped(hb_ctx *ctx, const hb_ct *x, const hb_pt *const *p, int count, int sums, hb_ct **out);
+/* the same with the operands one by one: out_k = rescale(sum_{j < count} a[k * count + j] (.) p[k * count + j]), batch members per sum */
+int hb_sum_mul_pt_rescale_many(hb_ctx *ctx, const hb_ct *const *a, const hb_pt *const *p, int count, int sums, hb_ct **out);
 /* out = rescale(sum_j a[j] (.) p[j]): the products are added un-rescaled and the sum is rescaled once (one inverse
  * transform of the last limb instead of one per term).  The masked sums of the linear transforms in schedule 2. */
 int hb_sum_mul_pt_rescale(hb_ctx *ctx, const hb_ct *const *a, const hb_pt *const *p, int count, hb_ct **out);
