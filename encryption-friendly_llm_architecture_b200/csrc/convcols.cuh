@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
         const u64 sw = sc.w[l], ss = sc.c[l];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-            u64 r = LONG::mul(x[e] + LONG::above(c) - smr[e * 17 + clo], sw, ss, c); // below 7q
+            u64 r = LONG::mul(x[e] + LONG::above_fwd(c) - smr[e * 17 + clo], sw, ss, c); // below 7q
             if (ap) r += ap[g ? ntt_perm((u32)(pos + e * 16), g, 16) : (u32)(pos + e * 16)];
             o[e * 16] = LONG::canon(r, c);
         }

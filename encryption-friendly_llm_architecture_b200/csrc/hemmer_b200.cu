@@ -1190,6 +1190,7 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             if (!p.fp && (((u64)1 << bits) - q) >> std::min(bits - 12, 32)) throw std::invalid_argument("prime too far below its power of two");
             const u64 below60 = q < ((u64)1 << 60) ? ((u64)1 << 60) - q : 0;
             p.d60 = below60 < ((u64)1 << 26) ? (u32)below60 : 0;
+            p.q7 = p.fp ? 0 : q * 7;
             std::vector<u64> f, fs, iv, ivs;
             c->h->twiddles(i, f, fs, iv, ivs);
             if (big) {

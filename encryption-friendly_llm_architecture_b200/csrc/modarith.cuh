@@ -29,6 +29,7 @@ struct PrimeConst {
     u32 fold_shift;     // primes of b >= 45 bits: b - 32 (every such prime of a context lies within 2^(b-12) below 2^b)
     u32 fold_d;         //   and 2^b - q
     u32 d60;            // 2^60 - q when that is positive and below 2^26, else 0
+    u64 q7;             // 7q of the primes of 45 bits and more
 };
 
 // Limb instances of a launch: instance li (0 <= li < count) uses prime[li % n].

@@ -139,7 +139,8 @@ struct LongShoup {
     }
     static __device__ __forceinline__ u64 mul(u64 x, u64 w, u64 comp, const Const &c) { return mul_shoup4(x, w, comp, c.nq); } // any x -> below 4q
     static __device__ __forceinline__ u64 canon(u64 x, const Const &c) { return canon_q(x, c.q, c.f); }
-    static __device__ __forceinline__ u64 above(const Const &c) { return c.q8; } // a multiple of q above what a forward transform leaves (5q)
+    static __device__ __forceinline__ u64 above_fwd(const Const &c) { return c.q8; } // a multiple of q above what a forward transform leaves (5q)
+    static __device__ __forceinline__ u64 above_inv(const Const &c) { return c.q8; } // and above what three stages of an inverse round leave (8q)
     // Four Cooley-Tukey stages on 16 register values; twiddles tp[j].
     // A stage adds 4q to the bound B of the values; x is folded below ~2^b before the additions of the stages named by the bit mask FOLD.
     // The words hold 16 q: in units of q the four rounds of a transform (masks 8, 4, 2, 9) run 3-7-11-15|5, 5-9-13|5-9, 9-13|5-9-13, 13|5-9-13|5 (| = a fold).
@@ -185,24 +186,26 @@ struct LongShoup {
 };
 // Primes q = 2^60 - d, d < 2^26.  A constant w comes as its two pieces and those of w' = w * 2^32 mod q (29 low and 31 high bits in the words of a u64), so
 // that x * w = x0 w + x1 w' = A + B * 2^29 takes the words of x as they are, and B = Bl + Bh * 2^32 folds by 2^61 = 2d the same way: A + Bl * 2^29 + Bh * 2d.
-// Six 32 x 32 products instead of the Shoup form's five and four low ones, and no carries in between: 11.5 instructions a butterfly against 21.
+// Five 32 x 32 products instead of the Shoup form's five and four low ones, and no carries in between.
 // In units of 2^60, for x below X: A < 2 + X/8, Bl * 2^29 < 2, Bh * 2d < 1/2: below 4.5 + X/8, 6.5 for any x.
-// A radix-16 round, cycles per warp butterfly and scheduler with four warps: 29 against 37 (Cooley-Tukey), 35 against 39 (Gentleman-Sande); half of the warps
-// in FP64 butterflies: 19 on average against 26, as products with 64-bit addends leave FP64 products few issue slots.
+// A radix-16 round, cycles per warp butterfly and scheduler with eight warps: 27 against 38 (Cooley-Tukey), 30 against 39 (Gentleman-Sande); half of the
+// warps in FP64 butterflies: 19 on average against 26, as products with 64-bit addends leave FP64 products few issue slots.  7q comes
+// from memory: where the compiler sees seven times q, it multiplies (35 and 34 cycles).
 struct LongPm {
     struct Const { u64 q, q7; u32 d, d2; };
     static __device__ __forceinline__ Const make(const PrimeConst &m) {
         Const c;
-        c.q = m.q; c.q7 = m.q * 7; c.d = m.d60; c.d2 = 2 * m.d60;
+        c.q = m.q; c.q7 = m.q7; c.d = m.d60; c.d2 = 2 * m.d60;
         return c;
     }
-    // separate instructions: the compiler would join most of them to products with 64-bit addends, which take longer than both (33 cycles a butterfly)
+    // separate instructions: the compiler would join most of them to products with 64-bit addends, which take longer than both
     static __device__ __forceinline__ u64 add(u64 a, u64 b) { u64 r; asm volatile("add.u64 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
     static __device__ __forceinline__ u64 wide(u32 a, u32 b) { u64 r; asm("mul.wide.u32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b)); return r; }
+    static __device__ __forceinline__ u64 shl29(u32 x) { u64 r; asm("{.reg .u32 l, h; shl.b32 l, %1, 29; shr.u32 h, %1, 3; mov.b64 %0, {l, h};}" : "=l"(r) : "r"(x)); return r; }
     static __device__ __forceinline__ u64 mul(u64 x, u64 w, u64 comp, const Const &c) {
         const u32 x0 = (u32)x, x1 = (u32)(x >> 32);
         const u64 a = add(wide(x1, (u32)comp), wide(x0, (u32)w)), b = add(wide(x1, (u32)(comp >> 32)), wide(x0, (u32)(w >> 32)));
-        return add(add(a, wide((u32)b, 1u << 29)), wide((u32)(b >> 32), c.d2));
+        return add(add(a, shl29((u32)b)), wide((u32)(b >> 32), c.d2));
     }
     // x < 16 * 2^60 -> congruent value below 2^60 + 2^30
     static __device__ __forceinline__ u64 fold(u64 x, const Const &c) {
@@ -213,7 +216,8 @@ struct LongPm {
         const u64 r = fold(x, c);
         return r >= c.q ? r - c.q : r;
     }
-    static __device__ __forceinline__ u64 above(const Const &c) { return c.q7 + 2 * c.q; }
+    static __device__ __forceinline__ u64 above_fwd(const Const &c) { return c.q7 << 1; } // a forward transform leaves 8.1
+    static __device__ __forceinline__ u64 above_inv(const Const &c) { return c.q7; }      // an inverse round 6.3
     // x is folded before the additions of every second stage; differences are taken from 7q, above every product.  Bounds (units of 2^60) alternate: 8.1 behind
     // a stage with a fold, 15.1 behind one without, whose products are below 4.5 + 15.1 / 8 = 6.4.
     // MADE: the upper half already carries the twiddle of the first stage (both halves below 3q)
@@ -259,7 +263,7 @@ struct LongPm {
 template <class LONG, class STORE> __device__ __forceinline__ void inv16_int_last(const u64 (&v)[16], const u64 (&sw)[2], const u64 (&sc)[2], const typename LONG::Const &c, STORE &&store) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) { // below 8q before, sums and differences below 16q
-        const u64 a = v[j] + v[j + 8], d = v[j] + LONG::above(c) - v[j + 8];
+        const u64 a = v[j] + v[j + 8], d = v[j] + LONG::above_inv(c) - v[j + 8];
         store(j, LONG::canon(LONG::mul(a, sw[0], sc[0], c), c));
         store(j + 8, LONG::canon(LONG::mul(d, sw[1], sc[1], c), c));
     }
