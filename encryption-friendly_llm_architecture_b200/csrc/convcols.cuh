@@ -39,7 +39,8 @@ struct ConvPlan {
     u64 scale_w[8][2], scale_c[8][2];   // as scale_words makes them; [1]: times psi^(-N/2), the twiddle of the last inverse stage
     unsigned char fp[kMaxPrimes];       // target t converts on the FP64 pipe (see ConvFp)
     uint4 c[kMaxPrimes][2][8];          // [target][half of the rows][source], the second half times psi^(N/2), the twiddle of the first forward stage: C = D / d_s mod target.  Target below 2^44: the 26-bit pieces of C
-                                        // and of C * 2^30; otherwise the 30-bit pieces of C, their sum, 0
+                                        // and of C * 2^30; otherwise the 30-bit pieces of C, their sum, 0, or (kPieceSources) the pieces of 29 and 31
+                                        // bits of C and of C * 2^30
     double d[kMaxPrimes][2][8][4];      // fp targets: C = d1 + d0 with d1 a multiple of 2^21, |d0| <= 2^20, C taken within q/2 of zero; the
                                         // same for C * 2^30.  Set when every sum of the products is exact in a double
 };
@@ -100,7 +101,7 @@ __device__ __forceinline__ void strip_inverse(IN &&in, u64 *sm, const PrimeConst
         inv16_int_last<LONG>(v, sw, sc, c, [&](int e, u64 w) { sm[I::a(e, sub, lane)] = word(w); });
     }
 }
-// Forward column pass of one limb strip that lies in sm (words of this thread at I::a; double bits below 2^44, |v| < 2q; otherwise below 3q).
+// Forward column pass of one limb strip that lies in sm (words of this thread at I::a; double bits below 2^44, |v| < 2q; otherwise below 3q, below 6.5q next to 2^60).
 // MADE: the rows from 128 on already carry the twiddle of the first stage.
 template <int COLS, class LONG, bool MADE>
 __device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, int g, int sub, int lane) {
@@ -163,36 +164,38 @@ __device__ __forceinline__ double finish_small(u64 a0, u64 a1, const SmallFinish
     const u32 hi = q1 * f.n0 + (q0 * f.n1 + (u32)(r >> 32)) + f.hi0;
     return __hiloint2double((int)hi, (int)(u32)r) - kMagic;
 }
-// The conversions of one target for this thread's sixteen coefficients, into sm (at I::a).  Four coefficients at a time in a rolled loop:
-// the constants are fetched four times instead of held, and the straight-line code stays small (warps of a CTA work on
-// different targets, so long code is fetched again and again).
+// The conversions of one target for this thread's sixteen coefficients, into sm (at I::a).  Eight coefficients at a time in a rolled loop:
+// the constants are fetched twice instead of held, and the straight-line code stays small (warps of a CTA work on
+// different targets, so long code is fetched again and again).  NS: the number of sources, 0 for any; three (ModDown) and four
+// (digits, the division by P * q_level) are unrolled.
 //
 // On the FP64 pipe: y = y0 + y1 * 2^30 as two doubles, sums a0 of y * d0 and a1 of y * d1 (both exact: below 2^53, and below 2^53
-// units of 2^21), remainder of a1 + a0.  Sixteen fused multiply-adds and eight conversions for four sources, 58 FP64 cycles per warp
-// coefficient; the integer sums take 100 on the integer pipes.
-template <int COLS>
-__device__ __forceinline__ void convert_target_fp(u64 *sm, const u64 *ysm, const ConvConst *cst, int ns, const PrimeConst &m, int sub, int lane) {
+// units of 2^21), remainder of a1 + a0.  Sixteen products and eight conversions for four sources, 58 FP64 cycles per warp
+// coefficient of the 79 that it takes with four warps a scheduler (four coefficients at a time and a loop over the sources: 88).
+template <int COLS, int NS>
+__device__ __forceinline__ void convert_target_fp(u64 *sm, const u64 *ysm, const ConvConst *cst, int ns_, const PrimeConst &m, int sub, int lane) {
     using I = StripIndex<COLS>;
+    const int ns = NS ? NS : ns_;
     const double qinv = m.q_inv_f, qd = (double)m.q;
 #pragma unroll 1
-    for (int e0 = 0; e0 < 16; e0 += 4) {
-        double a0[4], a1[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) { a0[u] = 0.0; a1[u] = 0.0; }
-#pragma unroll 2
-        for (int s = 0; s < ns; ++s) {
+    for (int e0 = 0; e0 < 16; e0 += 8) {
+        double a0[8], a1[8];
+        auto source = [&](int s, bool first) {
             const ConvConst &k = cst[(e0 >> 3) * ns + s];
             const double2 k0 = k.d[0], k1 = k.d[1];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < 8; ++u) {
                 const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
                 const double y0 = __hiloint2double(0x43300000, (int)(u32)y) - kTwo52, y1 = __hiloint2double(0x43300000, (int)(u32)(y >> 32)) - kTwo52;
-                a0[u] = __fma_rn(y0, k0.x, a0[u]); a1[u] = __fma_rn(y0, k0.y, a1[u]);
+                a0[u] = first ? __dmul_rn(y0, k0.x) : __fma_rn(y0, k0.x, a0[u]); a1[u] = first ? __dmul_rn(y0, k0.y) : __fma_rn(y0, k0.y, a1[u]);
                 a0[u] = __fma_rn(y1, k1.x, a0[u]); a1[u] = __fma_rn(y1, k1.y, a1[u]);
             }
-        }
+        };
+        source(0, true);
+#pragma unroll (NS ? NS : 1)
+        for (int s = 1; s < ns; ++s) source(s, false);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < 8; ++u) {
             const double qh = __fma_rn(a1[u], qinv, __fma_rn(a0[u], qinv, kMagic)) - kMagic;
             sm[I::a(e0 + u, sub, lane)] = (u64)__double_as_longlong(__fma_rn(-qh, qd, a1[u]) + a0[u]); // within 1.1 q of zero
         }
@@ -249,6 +252,38 @@ __device__ __forceinline__ void convert_target_wide(u64 *sm, const u64 *ysm, con
     }
 }
 
+// The same to a prime next to 2^60 from at most four sources: C and C * 2^30 in pieces of 29 and 31 bits, sums A and B of weight 2^29 that stay below 2^63
+// and 2^64, folded as in LongPm::mul: below 6.5 * 2^60.  Four sources take 85 cycles per warp coefficient with four warps a
+// scheduler, three 72; three products a source (convert_target_wide) with their longer reduction 126 and 107.
+template <int COLS, int NS>
+__device__ __forceinline__ void convert_target_pm(u64 *sm, const u64 *ysm, const ConvConst *cst, int ns_, const PrimeConst &m, int sub, int lane) {
+    using I = StripIndex<COLS>;
+    const int ns = NS ? NS : ns_;
+    const u32 d2 = 2 * m.d60;
+#pragma unroll 1
+    for (int e0 = 0; e0 < 16; e0 += 4) {
+        u64 a[4], b[4];
+        auto source = [&](int s, bool first) {
+            const uint4 c = cst[(e0 >> 3) * ns + s].c;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
+                const u32 y0 = (u32)y, y1 = (u32)(y >> 32);
+                const u64 p = LongPm::add(LongPm::wide(y0, c.x), LongPm::wide(y1, c.z)), r = LongPm::add(LongPm::wide(y0, c.y), LongPm::wide(y1, c.w));
+                a[u] = first ? p : LongPm::add(a[u], p);
+                b[u] = first ? r : LongPm::add(b[u], r);
+            }
+        };
+        source(0, true);
+#pragma unroll (NS ? NS : 1)
+        for (int s = 1; s < ns; ++s) source(s, false);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) sm[I::a(e0 + u, sub, lane)] = LongPm::add(LongPm::add(a[u], LongPm::shl29((u32)b[u])), LongPm::wide((u32)(b[u] >> 32), d2));
+    }
+}
+template <class LONG> constexpr int kPieceSources = 0; // up to this many sources the constants of long targets are those of convert_target_pm
+template <> inline constexpr int kPieceSources<LongPm> = 4;
+
 // src: half-inverse limbs (after the inverse row pass), instance b at src + b * src_outer; dst: half-forward limbs.
 // grid = (256 / COLS, plans, instances).  Dynamic shared memory: (largest ns + G) strips, then 2 * nt * ns constants: their loads stand in front of
 // every few products, and what L1 is left beside the strips holds no more than the twiddles.  All sources are on their way
@@ -296,8 +331,15 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
         const PrimeConst m = pc[pi];
         const ConvConst *cst = consts + 2 * t * ns;
         const bool fp = pl->fp[t];
-        if (fp) convert_target_fp<COLS>(ex, strips, cst, ns, m, sub, lane);
-        else if (m.small) convert_target_small<COLS>(ex, strips, cst, ns, m, sub, lane);
+        if (fp) {
+            if (ns == 4) convert_target_fp<COLS, 4>(ex, strips, cst, ns, m, sub, lane);
+            else if (ns == 3) convert_target_fp<COLS, 3>(ex, strips, cst, ns, m, sub, lane);
+            else convert_target_fp<COLS, 0>(ex, strips, cst, ns, m, sub, lane);
+        } else if (!m.small && ns <= kPieceSources<LONG>) {
+            if (ns == 4) convert_target_pm<COLS, 4>(ex, strips, cst, ns, m, sub, lane);
+            else if (ns == 3) convert_target_pm<COLS, 3>(ex, strips, cst, ns, m, sub, lane);
+            else convert_target_pm<COLS, 0>(ex, strips, cst, ns, m, sub, lane);
+        } else if (m.small) convert_target_small<COLS>(ex, strips, cst, ns, m, sub, lane);
         else convert_target_wide<COLS>(ex, strips, cst, ns, m, sub, lane);
         strip_forward<COLS, LONG, true>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)pi * Ntt16Layout::kEntries, g, sub, lane);
     }

@@ -266,7 +266,7 @@ void fill_conv(const HostCtx &h, bool pm, ConvPlan &p, const std::vector<int> &s
         scale_words(hbhost::mulmod(v, q - half_turn(src[s]), q), q, pm, p.scale_w[s][1], p.scale_c[s][1]); // its inverse is its negative
     }
     for (size_t t = 0; t < dst.size(); ++t) {
-        const u64 q = h.q[dst[t]], m26 = ((u64)1 << 26) - 1, m30 = ((u64)1 << 30) - 1;
+        const u64 q = h.q[dst[t]], m26 = ((u64)1 << 26) - 1, m30 = ((u64)1 << 30) - 1, m29 = ((u64)1 << 29) - 1;
         p.dst_prime[t] = (unsigned char)dst[t];
         p.order[t] = (unsigned char)t;
         p.fp[t] = !(q >> 44) && src.size() <= 4;
@@ -282,7 +282,8 @@ void fill_conv(const HostCtx &h, bool pm, ConvPlan &p, const std::vector<int> &s
                     };
                     split(v, d); split(v30, d + 2);
                 }
-                p.c[t][half][s] = (q >> 44) ? make_uint4((u32)(v & m30), (u32)(v >> 30), (u32)(v & m30) + (u32)(v >> 30), 0) : make_uint4((u32)(v & m26), (u32)(v >> 26), (u32)(v30 & m26), (u32)(v30 >> 26));
+                if ((q >> 44) && pm && src.size() <= (size_t)kPieceSources<LongPm>) p.c[t][half][s] = make_uint4((u32)(v & m29), (u32)(v >> 29), (u32)(v30 & m29), (u32)(v30 >> 29));
+                else p.c[t][half][s] = (q >> 44) ? make_uint4((u32)(v & m30), (u32)(v >> 30), (u32)(v & m30) + (u32)(v >> 30), 0) : make_uint4((u32)(v & m26), (u32)(v >> 26), (u32)(v30 & m26), (u32)(v30 >> 26));
                 const double y0 = 0x1p30, y1 = (double)((h.q[src[s]] >> 30) + 1);
                 low += y0 * std::fabs(d[0]) + y1 * std::fabs(d[2]);
                 high += (y0 * std::fabs(d[1]) + y1 * std::fabs(d[3])) * 0x1p-21;

@@ -220,7 +220,7 @@ struct LongPm {
     static __device__ __forceinline__ u64 above_inv(const Const &c) { return c.q7; }      // an inverse round 6.3
     // x is folded before the additions of every second stage; differences are taken from 7q, above every product.  Bounds (units of 2^60) alternate: 8.1 behind
     // a stage with a fold, 15.1 behind one without, whose products are below 4.5 + 15.1 / 8 = 6.4.
-    // MADE: the upper half already carries the twiddle of the first stage (both halves below 3q)
+    // MADE: the upper half already carries the twiddle of the first stage (both halves below 6.5, so sums and differences below 13.6)
     template <int ROUND, bool MADE = false, class TW> static __device__ __forceinline__ void fwd16(u64 (&v)[16], const TW &tp, const Const &c) {
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
