@@ -553,10 +553,21 @@ CtxtTensor multPackedMatMat(Env &e, const CtxtTensor &op1, const CtxtTensor &op2
         }
     } else { // b sits one level below a
         Chains c = start_chains(e, {&a}, {2}, {cols_tmp});
-        b = e.ev.leftRotate(b, 2 * width);
+        HeldChains held(e, c);
+        std::vector<Ciphertext> right; // those of the held iterations, and after a call the last one
+        right.push_back(std::move(b));
         for (i64 i = 1; i < num_k / 2; ++i) {
-            if (i > 1) { c.advance(e); b = e.ev.leftRotate(b, 2 * width); }
-            e.ev.tensorAccumulate(acc, e.ev.multSumGrouped(*c.x, {&col_wrap(e, sa, 4 * i + 1, lvl), &col_wrap(e, sa, 4 * i, lvl)}, 2, 1), b);
+            if (i > 1) c.advance(e);
+            right.push_back(e.ev.leftRotate(right.back(), 2 * width));
+            held.add(c, {&col_wrap(e, sa, 4 * i + 1, lvl), &col_wrap(e, sa, 4 * i, lvl)});
+            if (!held.full() && i + 1 < num_k / 2) continue;
+            const int n = held.held();
+            Ciphertext last = std::move(right.back());
+            right.back() = e.ev.view(last, 0, last.getBatch());
+            right.erase(right.begin());
+            e.ev.tensorAccumulateGroups(acc, held.take(), n == 1 ? std::move(right[0]) : e.ev.concat(right), n);
+            right.clear();
+            right.push_back(std::move(last));
         }
     }
     res = e.ev.add(res, e.ev.rescale(e.ev.relinearize(acc)));
