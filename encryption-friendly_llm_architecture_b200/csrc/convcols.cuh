@@ -103,8 +103,9 @@ __device__ __forceinline__ void strip_inverse(IN &&in, u64 *sm, const PrimeConst
 }
 // Forward column pass of one limb strip that lies in sm (words of this thread at I::a; double bits below 2^44, |v| < 2q; otherwise below 3q, below 6.5q next to 2^60).
 // MADE: the rows from 128 on already carry the twiddle of the first stage.
-template <int COLS, class LONG, bool MADE>
-__device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, int g, int sub, int lane) {
+// between(): done before the barrier between the rounds.
+template <int COLS, class LONG, bool MADE, class BETWEEN>
+__device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *sm, const PrimeConst &m, const ulonglong2 *__restrict__ tab, int g, int sub, int lane, BETWEEN &&between) {
     using I = StripIndex<COLS>;
     if (m.small) {
         const DsConst c = ds_const(m);
@@ -115,6 +116,7 @@ __device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *s
         fwd16_ds<MADE>(d, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[I::a(e, sub, lane)] = d[e];
+        between();
         group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) d[e] = smd[I::b(e, sub, lane)];
@@ -129,6 +131,7 @@ __device__ __forceinline__ void strip_forward(u64 *o /* limb + column */, u64 *s
         LONG::template fwd16<0, MADE>(v, TwiddlesA(tab + Ntt16Layout::colsA(0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) sm[I::a(e, sub, lane)] = v[e];
+        between();
         group_sync<COLS * 16>(g);
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = sm[I::b(e, sub, lane)];
@@ -292,10 +295,10 @@ template <> inline constexpr int kPieceSources<LongPm> = 4;
 template <int COLS, int G, int MINB, class LONG>
 __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, const ConvPlan *__restrict__ plans,
                                                                          const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
-    extern __shared__ __align__(16) u64 strips[];
-    __shared__ int next, turn[G];
+    extern __shared__ __align__(128) u64 strips[]; // rows of 32 bytes at an odd multiple of 16 take 2.4 % longer in all
+    __shared__ int next, turn[2][G];
     using I = StripIndex<COLS>;
-    if (threadIdx.x == 0) next = 0;
+    if (threadIdx.x == 0) next = G <= 2 ? G : 0;
     const ConvPlan *pl = plans + blockIdx.y;
     const int ns = pl->ns, nt = pl->nt;
     const int g = threadIdx.x / (COLS * 16), r = threadIdx.x % (COLS * 16), lane = r % COLS, sub = r / COLS;
@@ -320,12 +323,10 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
     }
     __syncthreads();
     u64 *ex = strips + (ns + g) * I::kWords;
-    while (true) { // the groups take targets from a common counter
-        group_sync<COLS * 16>(g); // the strip of the previous target has been read
-        if (r == 0) turn[g] = atomicAdd(&next, 1);
-        group_sync<COLS * 16>(g);
-        const int k = turn[g];
-        if (k >= nt) break;
+    // The groups take targets from a common counter.  Two groups take their next one in the middle of the present transform, whose barrier makes it known:
+    // asked for at the end it costs a barrier and a round trip, 1000 cycles a target (conversions of 256 products at level 8 4.66 -> 4.50 ms).  More
+    // groups keep the end: there one with a long target would take early what another could begin at once.
+    auto target = [&](int k, auto &&between) {
         const int t = pl->order[k];
         const int pi = pl->dst_prime[t];
         const PrimeConst m = pc[pi];
@@ -341,16 +342,33 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
             else convert_target_pm<COLS, 0>(ex, strips, cst, ns, m, sub, lane);
         } else if (m.small) convert_target_small<COLS>(ex, strips, cst, ns, m, sub, lane);
         else convert_target_wide<COLS>(ex, strips, cst, ns, m, sub, lane);
-        strip_forward<COLS, LONG, true>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)pi * Ntt16Layout::kEntries, g, sub, lane);
+        strip_forward<COLS, LONG, true>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)pi * Ntt16Layout::kEntries, g, sub, lane, between);
+    };
+    if constexpr (G <= 2) {
+        for (int k = g, odd = 0; k < nt; odd ^= 1) {
+            target(k, [&] { if (r == 0) turn[odd][g] = atomicAdd(&next, 1); });
+            k = turn[odd][g];
+            group_sync<COLS * 16>(g); // the strip has been read
+        }
+    } else {
+        while (true) {
+            group_sync<COLS * 16>(g); // the strip of the previous target has been read
+            if (r == 0) turn[0][g] = atomicAdd(&next, 1);
+            group_sync<COLS * 16>(g);
+            const int k = turn[0][g];
+            if (k >= nt) break;
+            target(k, [] {});
+        }
     }
 }
 
-// Rescale: one source limb (prime index `level`), lifted centred to the limbs 0 .. level - 1.
+// Rescale: one source limb (prime index `level`), lifted centred to the limbs 0 .. level - 1.  One group per CTA where there are many
+// instances: a second one would wait for the source.
 // grid = (256 / COLS, instances); dynamic shared memory: 1 + G strips.
 template <int COLS, int G, int MINB, class LONG>
 __global__ void __launch_bounds__(COLS * 16 * G, MINB) lift_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, int level,
                                                                          const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
-    extern __shared__ __align__(16) u64 strips[];
+    extern __shared__ __align__(128) u64 strips[];
     using I = StripIndex<COLS>;
     const int g = threadIdx.x / (COLS * 16), r = threadIdx.x % (COLS * 16), lane = r % COLS, sub = r / COLS;
     const int col = blockIdx.x * COLS + lane;
@@ -377,7 +395,7 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) lift_cols(const u64 *src,
             else if ((ql >> 1) < m.q) w = y < 0 ? (u64)(y + (i64)m.q) : (u64)y;
             else w = reduce_i64(y, m);
         }
-        strip_forward<COLS, LONG, false>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)t * Ntt16Layout::kEntries, g, sub, lane);
+        strip_forward<COLS, LONG, false>(dp + (size_t)t * kN16, ex, m, tb.fwd + (size_t)t * Ntt16Layout::kEntries, g, sub, lane, [] {});
     }
 }
 

@@ -348,7 +348,7 @@ void conv_opt_in(hb_ctx *c) {
         using LONG = decltype(arithmetic);
         allow(conv_cols<8, 4, 1, LONG>, strip_bytes<8>(12) + consts); allow(conv_cols<4, 4, 2, LONG>, strip_bytes<4>(12) + consts); allow(conv_cols<4, 8, 1, LONG>, strip_bytes<4>(16) + consts);
         allow(conv_cols<8, 2, 2, LONG>, strip_bytes<8>(6) + conv_const_bytes(4, kMaxPrimes));
-        allow(lift_cols<8, 2, 2, LONG>, strip_bytes<8>(3)); allow(lift_cols<4, 4, 2, LONG>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1, LONG>, strip_bytes<4>(9));
+        allow(lift_cols<8, 2, 2, LONG>, strip_bytes<8>(3)); allow(lift_cols<8, 1, 4, LONG>, strip_bytes<8>(2)); allow(lift_cols<4, 4, 2, LONG>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1, LONG>, strip_bytes<4>(9));
     };
     if (c->tb.t16.pm) all(LongPm{}); else all(LongShoup{});
     c->smem_opt_in_conv = true;
@@ -364,7 +364,7 @@ void conv_opt_in(hb_ctx *c) {
 // 299 / 310, products of eight at level 6 (16 units) 459 / 453 / 465; divisions of level 7, 16 units 257 / 254 / 261, 20 units 317 / 312 / 325.  Up to five
 // targets it does not show (division of level 3, 16 units 157 / 151 / 141; level 5, 20 units 219 / 212 / 214), nor with the three sources of
 // a ModDown (products of eight members at level 7, 16 units 586 / 577 / 567).
-enum StripShape { kStrip8x2, kStrip8x4, kStrip4x4, kStrip4x8 };
+enum StripShape { kStrip8x1, kStrip8x2, kStrip8x4, kStrip4x4, kStrip4x8 };
 StripShape conv_shape(int units, int max_ns, int targets) {
     if (units <= 2) return kStrip4x8;
     if (units <= 12) return kStrip4x4;
@@ -372,7 +372,9 @@ StripShape conv_shape(int units, int max_ns, int targets) {
     const int more = units * 32 % 148; // SMs with one CTA more
     return units <= 20 && max_ns == 4 && targets > 5 && more >= 148 / 10 && more < 148 / 2 ? kStrip4x4 : kStrip8x2;
 }
-StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : kStrip8x2; }
+// Rescales: from 96 polynomials on (five waves of CTAs) one group per CTA, so that none waits for the source: 512 polynomials at level 8 1.13 -> 1.02 ms.
+// Fewer keep two groups, whose CTAs are half as long, for the last wave.
+StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : units < 96 ? kStrip8x2 : kStrip8x1; }
 // `plans` conversions (the largest with max_ns sources, `targets` each on average, max_nt at most) of `instances` polynomials in one launch
 void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int targets, int max_nt, int instances) {
     conv_opt_in(c);
@@ -402,7 +404,8 @@ void launch_lift(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int
         switch (lift_shape(instances)) {
         case kStrip4x8: go(lift_cols<4, 8, 1, LONG>, 4, 8, strip_bytes<4>(9)); break;
         case kStrip4x4: go(lift_cols<4, 4, 2, LONG>, 4, 4, strip_bytes<4>(5)); break;
-        default: go(lift_cols<8, 2, 2, LONG>, 8, 2, strip_bytes<8>(3)); break;
+        case kStrip8x2: go(lift_cols<8, 2, 2, LONG>, 8, 2, strip_bytes<8>(3)); break;
+        default: go(lift_cols<8, 1, 4, LONG>, 8, 1, strip_bytes<8>(2)); break;
         }
     };
     if (c->tb.t16.pm) shapes(LongPm{}); else shapes(LongShoup{});
