@@ -11,10 +11,10 @@
 // writes instead of 3 S + S + 3 T limb transfers, and one launch instead of three.  The constants of a conversion carry the scale of the
 // inverse transforms, the twiddle of their last stage and that of the first forward stage, which so cost no products of their own.
 //
-// At S = 4, T = 6 (the division by P * q_level at level 6) 96 polynomials took 887 us with one CTA of four groups per SM; with two CTAs of
-// two groups 833, with the folded twiddles 815.  The instructions it cannot do without take about three quarters of that: FP64 and
-// integer products issue at half rate and do not overlap on a scheduler (a persistent version in which some groups transform the next
-// strip's sources while others convert targets, so that both kinds are always at hand, took 956 us).
+// At S = 4, T = 6 (the division by P * q_level at level 6) 96 polynomials took 413 us with Shoup butterflies, 363 with folded pieces (both under the profiler, before
+// convert_target_pm): FP64 a third of the cycles, the wide multiply pipe 40 %, half of the issue slots; four warps a scheduler, whose fixed latencies, shared-memory exchanges and bursts on one pipe are the rest.  FP64 and integer products
+// do overlap on a scheduler, unless the latter carry 64-bit addends.  What did not help: a persistent version in which some groups transform
+// the next strip's sources while others convert targets, more warps with fewer registers, CTAs of an SM started half a turn apart.
 //
 // A CTA is G groups of COLS * 16 threads.  Sources are dealt to the groups, then (one CTA barrier later) targets; inside a
 // group a radix-16 round exchanges through shared memory behind a named barrier of that group only, so one group's loads,
