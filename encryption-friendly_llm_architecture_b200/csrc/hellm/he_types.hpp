@@ -189,6 +189,13 @@ class Evaluator {
         for (auto *q : p) rp.push_back(q->raw());
         hb_ct *o = nullptr; check(c_, hb_sum_mul_pt_rescale_grouped(c_, x.raw(), rp.data(), count, sums, &o)); return Ciphertext(c_, o);
     }
+    // acc += tensor(first half of x's members, second half)
+    void tensorAccumulateHalves(Ciphertext &acc, const Ciphertext &x) const {
+        hb_ct *p = acc.release();
+        int rc = hb_tensor_acc_halves(c_, x.raw(), &p);
+        acc = Ciphertext(c_, p);
+        check(c_, rc);
+    }
     // the same with the operands one by one: sum k from the operands k * count ...
     static constexpr int kMaxSumTerms = 24;
     Ciphertext multSums(const std::vector<Ciphertext> &x, const std::vector<const Plaintext *> &p, int count) const {
@@ -288,6 +295,13 @@ class Evaluator {
     // sum over the K-groups b0 .. b0+pts.size()-1 of a batched set of shifted copies
     Ciphertext matmulGroups(const Ciphertext &pre, int btotal, int b0, const std::vector<const hb_pt *> &pts, i64 row_step) const {
         hb_ct *o = nullptr; check(c_, hb_matmul_acc_multi(c_, pre.raw(), btotal, b0, pts.data(), (int)pts.size(), row_step, &o)); return Ciphertext(c_, o);
+    }
+    Ciphertext stack(const std::vector<Ciphertext> &v) const {
+        int level = 0, np = 0, sp = 0, b = 1; hb_ct_meta(v[0].raw(), &level, &np, &b, &sp);
+        hb_ct *o = nullptr; check(c_, hb_ct_create(c_, level, np, (int)v.size() * b, sp, &o)); // copy k of input j at k*b + j
+        Ciphertext out(c_, o);
+        for (size_t k = 0; k < v.size(); ++k) check(c_, hb_batch_set(c_, o, (int)k, v[k].raw()));
+        return out;
     }
   private:
     hb_ctx *c_;

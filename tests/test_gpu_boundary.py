@@ -103,6 +103,11 @@ def test_operands_of_the_row_sums_survive_an_error(tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
+def test_evaluator_calls_that_the_library_does_not_make(tmp_path):
+    r = subprocess.run([str(_compiled("evaluator_calls", tmp_path))], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 def test_cpp_class_from_a_separately_compiled_program(pkg, tmp_path):
     """tests/integration/hemmer_snippet.cpp (the example of INTEGRATION.md) built with g++ against the two shared
     libraries, run, and compared with the same calls through ctypes: equal residues, correct products."""

@@ -19,3 +19,10 @@ def test_pool_keeps_what_a_recorded_graph_addresses(tmp_path):
 
 def test_threads_that_cannot_be_started_leave_their_share(tmp_path):
     _run(tmp_path, "host_threads", "-pthread")
+
+
+def test_programs_on_the_cpp_headers_compile():
+    """What a separately compiled program may call through HEMMer.hpp, calls that the library does not make itself among them."""
+    for name in ("hemmer_snippet", "operands_after_error", "evaluator_calls"):
+        subprocess.check_call(["g++", "-fsyntax-only", "-std=c++17", "-Wall", os.path.join(ROOT, "tests", "integration", name + ".cpp"), "-I", os.path.join(ROOT, "include"),
+                               "-I", os.path.join(ROOT, PKG_NAME, "csrc", "hellm")])
