@@ -169,8 +169,10 @@ __device__ __forceinline__ double finish_small(u64 a0, u64 a1, const SmallFinish
 }
 // The conversions of one target for this thread's sixteen coefficients, into sm (at I::a).  Eight coefficients at a time in a rolled loop:
 // the constants are fetched twice instead of held, and the straight-line code stays small (warps of a CTA work on
-// different targets, so long code is fetched again and again).  NS: the number of sources, 0 for any; three (ModDown) and four
-// (digits, the division by P * q_level) are unrolled.
+// different targets, so long code is fetched again and again).  NS: the number of sources, 0 for any; in the wide strips three (ModDown) and
+// four (digits, the division by P * q_level) are unrolled.  The narrow ones, whose launches are short, spend more on fetching the unrolled
+// code than it saves: one ciphertext at level 8, its two conversions, us, unrolled / not: with Shoup products 38.3 / 36.4 and 31.6 / 29.7, next to
+// 2^60 29.9 / 30.0 and 22.0 / 22.1.
 //
 // On the FP64 pipe: y = y0 + y1 * 2^30 as two doubles, sums a0 of y * d0 and a1 of y * d1 (both exact: below 2^53, and below 2^53
 // units of 2^21), remainder of a1 + a0.  Sixteen products and eight conversions for four sources, 58 FP64 cycles per warp
@@ -292,7 +294,10 @@ template <> inline constexpr int kPieceSources<LongPm> = 4;
 // every few products, and what L1 is left beside the strips holds no more than the twiddles.  All sources are on their way
 // from the start instead of behind one another.  The two together: 139 -> 129 ms
 // of the layer's conversions, products of 256 members at level 8 5.69 -> 5.33 ms.
-template <int COLS, int G, int MINB, class LONG>
+// ONE: no group has more than one source; its words go straight to registers, since the way through shared memory and the barrier behind it hide
+// nothing then.  One ciphertext at level 8, three digits and ModDown, us, through shared memory / straight: with Shoup products 36.8 / 35.7 and 29.8 / 28.9, next
+// to 2^60 29.9 / 29.2 and 22.3 / 22.5.  Six sources on four groups 59.0 / 62.2: there the second strip arrives behind the first one's work.
+template <int COLS, int G, int MINB, bool ONE, class LONG>
 __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, const ConvPlan *__restrict__ plans,
                                                                          const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     extern __shared__ __align__(128) u64 strips[]; // rows of 32 bytes at an odd multiple of 16 take 2.4 % longer in all
@@ -312,13 +317,16 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
         else consts[i].c = pl->c[t][h][s];
     }
     pdl_wait();
-    for (int s = g; s < ns; s += G) strip_fetch<COLS>(sp + (size_t)s * kN16, strips + s * I::kWords, r);
+    if (!ONE) for (int s = g; s < ns; s += G) strip_fetch<COLS>(sp + (size_t)s * kN16, strips + s * I::kWords, r);
     for (int s = g; s < ns; s += G) {
-        if (s + G < ns) cp_async_wait<1>(); else cp_async_wait<0>(); // at most one more strip of this group may be on its way
-        group_sync<COLS * 16>(g);
+        if (!ONE) {
+            if (s + G < ns) cp_async_wait<1>(); else cp_async_wait<0>(); // at most one more strip of this group may be on its way
+            group_sync<COLS * 16>(g);
+        }
         const int pi = pl->src_prime[s];
         u64 *sm = strips + s * I::kWords;
-        strip_inverse<COLS, LONG>([&](int e) { return sm[I::b(e, sub, lane)]; }, sm, pc[pi], tb.inv + (size_t)pi * Ntt16Layout::kEntries, pl->scale_w[s], pl->scale_c[s], g, sub, lane,
+        const u64 *gm = sp + (size_t)s * kN16 + lane;
+        strip_inverse<COLS, LONG>([&](int e) { return ONE ? gm[(sub * 16 + e) * 256] : sm[I::b(e, sub, lane)]; }, sm, pc[pi], tb.inv + (size_t)pi * Ntt16Layout::kEntries, pl->scale_w[s], pl->scale_c[s], g, sub, lane,
                             [](u64 v) { return ((v >> 30) << 32) | ((u32)v & 0x3FFFFFFFu); });
     }
     __syncthreads();
@@ -332,13 +340,14 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
         const PrimeConst m = pc[pi];
         const ConvConst *cst = consts + 2 * t * ns;
         const bool fp = pl->fp[t];
+        constexpr bool kUnroll = COLS == 8;
         if (fp) {
-            if (ns == 4) convert_target_fp<COLS, 4>(ex, strips, cst, ns, m, sub, lane);
-            else if (ns == 3) convert_target_fp<COLS, 3>(ex, strips, cst, ns, m, sub, lane);
+            if (kUnroll && ns == 4) convert_target_fp<COLS, kUnroll ? 4 : 0>(ex, strips, cst, ns, m, sub, lane);
+            else if (kUnroll && ns == 3) convert_target_fp<COLS, kUnroll ? 3 : 0>(ex, strips, cst, ns, m, sub, lane);
             else convert_target_fp<COLS, 0>(ex, strips, cst, ns, m, sub, lane);
-        } else if (!m.small && ns <= kPieceSources<LONG>) {
-            if (ns == 4) convert_target_pm<COLS, 4>(ex, strips, cst, ns, m, sub, lane);
-            else if (ns == 3) convert_target_pm<COLS, 3>(ex, strips, cst, ns, m, sub, lane);
+        } else if (kPieceSources<LONG> > 0 && !m.small && ns <= kPieceSources<LONG>) {
+            if (kUnroll && ns == 4) convert_target_pm<COLS, kUnroll ? 4 : 0>(ex, strips, cst, ns, m, sub, lane);
+            else if (kUnroll && ns == 3) convert_target_pm<COLS, kUnroll ? 3 : 0>(ex, strips, cst, ns, m, sub, lane);
             else convert_target_pm<COLS, 0>(ex, strips, cst, ns, m, sub, lane);
         } else if (m.small) convert_target_small<COLS>(ex, strips, cst, ns, m, sub, lane);
         else convert_target_wide<COLS>(ex, strips, cst, ns, m, sub, lane);

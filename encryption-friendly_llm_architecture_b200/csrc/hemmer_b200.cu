@@ -346,8 +346,8 @@ void conv_opt_in(hb_ctx *c) {
     const size_t consts = conv_const_bytes(8, kMaxPrimes);
     auto all = [&](auto arithmetic) {
         using LONG = decltype(arithmetic);
-        allow(conv_cols<8, 4, 1, LONG>, strip_bytes<8>(12) + consts); allow(conv_cols<4, 4, 2, LONG>, strip_bytes<4>(12) + consts); allow(conv_cols<4, 8, 1, LONG>, strip_bytes<4>(16) + consts);
-        allow(conv_cols<8, 2, 2, LONG>, strip_bytes<8>(6) + conv_const_bytes(4, kMaxPrimes));
+        allow(conv_cols<8, 4, 1, false, LONG>, strip_bytes<8>(12) + consts); allow(conv_cols<4, 4, 2, false, LONG>, strip_bytes<4>(12) + consts); allow(conv_cols<4, 8, 1, true, LONG>, strip_bytes<4>(16) + consts);
+        allow(conv_cols<4, 4, 2, true, LONG>, strip_bytes<4>(8) + conv_const_bytes(4, kMaxPrimes)); allow(conv_cols<8, 2, 2, false, LONG>, strip_bytes<8>(6) + conv_const_bytes(4, kMaxPrimes));
         allow(lift_cols<8, 2, 2, LONG>, strip_bytes<8>(3)); allow(lift_cols<8, 1, 4, LONG>, strip_bytes<8>(2)); allow(lift_cols<4, 4, 2, LONG>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1, LONG>, strip_bytes<4>(9));
     };
     if (c->tb.t16.pm) all(LongPm{}); else all(LongShoup{});
@@ -385,10 +385,10 @@ void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, con
     auto shapes = [&](auto arithmetic) {
         using LONG = decltype(arithmetic);
         switch (conv_shape(instances * count, max_ns, targets)) {
-        case kStrip8x2: go(conv_cols<8, 2, 2, LONG>, 8, 2, strip_bytes<8>(max_ns + 2) + consts); break;
-        case kStrip8x4: go(conv_cols<8, 4, 1, LONG>, 8, 4, strip_bytes<8>(max_ns + 4) + consts); break;
-        case kStrip4x4: go(conv_cols<4, 4, 2, LONG>, 4, 4, strip_bytes<4>(max_ns + 4) + consts); break;
-        default: go(conv_cols<4, 8, 1, LONG>, 4, 8, strip_bytes<4>(max_ns + 8) + consts); break;
+        case kStrip8x2: go(conv_cols<8, 2, 2, false, LONG>, 8, 2, strip_bytes<8>(max_ns + 2) + consts); break;
+        case kStrip8x4: go(conv_cols<8, 4, 1, false, LONG>, 8, 4, strip_bytes<8>(max_ns + 4) + consts); break;
+        case kStrip4x4: go(max_ns <= 4 ? conv_cols<4, 4, 2, true, LONG> : conv_cols<4, 4, 2, false, LONG>, 4, 4, strip_bytes<4>(max_ns + 4) + consts); break;
+        default: go(conv_cols<4, 8, 1, true, LONG>, 4, 8, strip_bytes<4>(max_ns + 8) + consts); break; // at most eight sources
         }
     };
     if (c->tb.t16.pm) shapes(LongPm{}); else shapes(LongShoup{});

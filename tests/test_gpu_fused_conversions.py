@@ -106,6 +106,56 @@ def test_batches_of_conversions_with_more_than_four_sources(many_sources, batch)
             assert np.array_equal(got[k:k + 1], g.ct_export(op(_ct(g, data[k:k + 1])))), f"operation {n}, member {k} of {batch}"
 
 
+SHOUP = {
+    "q0 of 59 bits": dict(q0_bits=59, max_level=8, dnum=3, num_special=3),
+    "scaling primes of 50 bits": PARAMS["scaling primes of 50 bits"],
+    "one digit of seven limbs, q0 of 59 bits": dict(PARAMS["one digit of seven limbs"], q0_bits=59),
+}
+
+
+@pytest.fixture(scope="module", params=sorted(SHOUP))
+def shoup(request, pkg, oracle_so):
+    prm = dict(log_n=16, hamming_weight=64, **SHOUP[request.param])
+    g, o = pkg.open_gpu(pkg.make_params(**prm)), open_oracle(pkg, oracle_so, **prm)
+    for lib in (g, o):
+        lib.keygen()
+        lib.gen_rot_keys([3])
+    return g, o
+
+
+def test_one_member_with_shoup_products(shoup):
+    """Long primes that are not all next to 2^60: the narrow strips of one member, against the oracle."""
+    g, o = shoup
+    level = int(g.L)
+    data = rand_ct_residues(g, level, 2, 1, seed=500)
+    data[0, :, 0, ::3] = np.uint64(int(g.primes[0]) - 1)
+    m = (np.random.default_rng(11).uniform(0, 1, g.slots) > 0.5).astype(np.float64)
+    res = []
+    for lib in (g, o):
+        x = _ct(lib, data)
+        res.append([lib.ct_export(c) for c in (lib.rotate(x, 3), lib.relin(lib.tensor(x, x)), lib.mul_pt(x, lib.encode(m, level)))])
+    for k, (a, b) in enumerate(zip(*res)):
+        assert np.array_equal(a, b), f"operation {k}"
+
+
+@pytest.mark.parametrize("batch", [2, 4, 5, 13, 17, 33, 48])
+def test_batches_with_shoup_products(shoup, batch):
+    """The same contexts through every strip shape: up to 2, 12 and, with more than four sources, 32 units; rescales of 2, 4 and 96 polynomials."""
+    g, _ = shoup
+    level = int(g.L)
+    data = rand_ct_residues(g, level, 2, batch, seed=600 + batch)
+    data[-1, :, 0] = np.uint64(int(g.primes[0]) - 1)
+    data[-1, :, level] = np.uint64(int(g.primes[level]) - 1)
+    m = (np.random.default_rng(9).uniform(0, 1, g.slots) > 0.5).astype(np.float64)
+    key, w = g.masked_key(3, g.encode_ext(m, level)), g.encode(m - 0.25, level)
+    ops = [lambda x: g.rotate(x, 3), lambda x: g.relin(g.tensor(x, x)), lambda x: g.mul_pt(x, w), lambda x: g.assemble_masked(x, g.decompose(x), key)]
+    whole = _ct(g, data)
+    for n, op in enumerate(ops):
+        got = g.ct_export(op(whole))
+        for k in sorted({0, batch // 2, batch - 1}):
+            assert np.array_equal(got[k:k + 1], g.ct_export(op(_ct(g, data[k:k + 1])))), f"operation {n}, member {k} of {batch}"
+
+
 @pytest.mark.parametrize("q_bits", [26, 27, 28, 34])
 def test_short_scaling_primes_of_2_16_points(pkg, oracle_so, q_bits):
     """Digits of six and seven limbs convert to scaling primes of 26 to 34 bits on the integer pipe, where the quotient of the first
