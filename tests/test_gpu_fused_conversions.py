@@ -17,7 +17,7 @@ def _ct(lib, data):
     return ct
 
 
-SIZES = [("full", 12, (5, 33)), ("full", 7, (1, 2, 3, 5, 17, 33, 47)), ("full", 3, (1, 2, 3, 5, 17, 33, 47)), ("full", 2, (2, 5, 33)),
+SIZES = [("full", 12, (5, 33)), ("full", 7, (1, 2, 3, 5, 17, 33, 47, 48)), ("full", 3, (1, 2, 3, 5, 17, 33, 47, 48)), ("full", 2, (2, 5, 33)),
          ("full", 3, (6, 7, 12, 13)), ("full", 7, (8, 9, 10)), ("mid", 7, (17, 33, 47)), ("mid", 3, (17, 33, 47)), ("mid", 2, (17, 33, 47))]
 
 
@@ -25,7 +25,7 @@ SIZES = [("full", 12, (5, 33)), ("full", 7, (1, 2, 3, 5, 17, 33, 47)), ("full", 
 def test_members_of_a_batch_equal_single_calls(request, size, level, batch):
     """Four, three, two and one digits (levels 12, 7, 3, 2), on either side of the 32 members from which the inner products hold one
     coefficient per thread.  At 2^16 points the strip shapes of these conversions (up to four sources) change at 2 and 12 units, polynomials
-    times digits, and with four sources and many targets at 15, 16, 19 and 20 units, those of the rescale at 2 and 4 polynomials; one chunk
+    times digits, and with four sources and many targets at 15, 16, 19 and 20 units, those of the rescale at 2, 4 and 96 polynomials; one chunk
     holds all members except at two and one digits with few of them (two chunks).  At 2^12 points a chunk holds two to seven members and the
     last one fewer, in the masked sums of one and two digits as well.  A batch of one takes the narrow shapes, whose residues the oracle
     tests pin."""
