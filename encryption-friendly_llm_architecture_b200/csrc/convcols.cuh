@@ -169,10 +169,10 @@ __device__ __forceinline__ double finish_small(u64 a0, u64 a1, const SmallFinish
 }
 // The conversions of one target for this thread's sixteen coefficients, into sm (at I::a).  Eight coefficients at a time in a rolled loop:
 // the constants are fetched twice instead of held, and the straight-line code stays small (warps of a CTA work on
-// different targets, so long code is fetched again and again).  NS: the number of sources, 0 for any; in the wide strips three (ModDown) and
-// four (digits, the division by P * q_level) are unrolled.  The narrow ones, whose launches are short, spend more on fetching the unrolled
-// code than it saves: one ciphertext at level 8, its two conversions, us, unrolled / not: with Shoup products 38.3 / 36.4 and 31.6 / 29.7, next to
-// 2^60 29.9 / 30.0 and 22.0 / 22.1.
+// different targets, so long code is fetched again and again).  NS: the number of sources, 0 for any; three (ModDown) and four (digits, the
+// division by P * q_level) are unrolled.  Not in the narrow strips with Shoup products, whose transforms are the longest code: their short launches
+// spend more on fetching it than the unrolled products save.  One ciphertext at level 8, its two conversions, us, unrolled / not: 38.3 / 36.4 and
+// 31.6 / 29.7.  Next to 2^60 it goes both ways by 2 %: rotations of one ciphertext at level 8 106.1 / 103.5, of four at level 12 354 / 356.
 //
 // On the FP64 pipe: y = y0 + y1 * 2^30 as two doubles, sums a0 of y * d0 and a1 of y * d1 (both exact: below 2^53, and below 2^53
 // units of 2^21), remainder of a1 + a0.  Sixteen products and eight conversions for four sources, 58 FP64 cycles per warp
@@ -294,15 +294,17 @@ template <> inline constexpr int kPieceSources<LongPm> = 4;
 // every few products, and what L1 is left beside the strips holds no more than the twiddles.  All sources are on their way
 // from the start instead of behind one another.  The two together: 139 -> 129 ms
 // of the layer's conversions, products of 256 members at level 8 5.69 -> 5.33 ms.
-// ONE: no group has more than one source; its words go straight to registers, since the way through shared memory and the barrier behind it hide
-// nothing then.  One ciphertext at level 8, three digits and ModDown, us, through shared memory / straight: with Shoup products 36.8 / 35.7 and 29.8 / 28.9, next
-// to 2^60 29.9 / 29.2 and 22.3 / 22.5.  Six sources on four groups 59.0 / 62.2: there the second strip arrives behind the first one's work.
+// ONE: no group has more than one source.  With Shoup products its words go straight to registers: the way through shared memory and the barrier
+// behind it hide nothing then (one ciphertext at level 8, three digits and ModDown, us, through shared memory / straight: 36.8 / 35.7 and 29.8 /
+// 28.9).  Next to 2^60 it is even: divisions of one ciphertext at level 12 78.3 / 79.1, rotations 135.9 / 135.5.  Six sources on four groups 59.0 /
+// 62.2: there the second strip arrives behind the first one's work.
 template <int COLS, int G, int MINB, bool ONE, class LONG>
 __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, const ConvPlan *__restrict__ plans,
                                                                          const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     extern __shared__ __align__(128) u64 strips[]; // rows of 32 bytes at an odd multiple of 16 take 2.4 % longer in all
     __shared__ int next, turn[2][G];
     using I = StripIndex<COLS>;
+    constexpr bool kShoup = kPieceSources<LONG> == 0, kOne = ONE && kShoup;
     if (threadIdx.x == 0) next = G <= 2 ? G : 0;
     const ConvPlan *pl = plans + blockIdx.y;
     const int ns = pl->ns, nt = pl->nt;
@@ -317,16 +319,16 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
         else consts[i].c = pl->c[t][h][s];
     }
     pdl_wait();
-    if (!ONE) for (int s = g; s < ns; s += G) strip_fetch<COLS>(sp + (size_t)s * kN16, strips + s * I::kWords, r);
+    if (!kOne) for (int s = g; s < ns; s += G) strip_fetch<COLS>(sp + (size_t)s * kN16, strips + s * I::kWords, r);
     for (int s = g; s < ns; s += G) {
-        if (!ONE) {
+        if (!kOne) {
             if (s + G < ns) cp_async_wait<1>(); else cp_async_wait<0>(); // at most one more strip of this group may be on its way
             group_sync<COLS * 16>(g);
         }
         const int pi = pl->src_prime[s];
         u64 *sm = strips + s * I::kWords;
         const u64 *gm = sp + (size_t)s * kN16 + lane;
-        strip_inverse<COLS, LONG>([&](int e) { return ONE ? gm[(sub * 16 + e) * 256] : sm[I::b(e, sub, lane)]; }, sm, pc[pi], tb.inv + (size_t)pi * Ntt16Layout::kEntries, pl->scale_w[s], pl->scale_c[s], g, sub, lane,
+        strip_inverse<COLS, LONG>([&](int e) { return kOne ? gm[(sub * 16 + e) * 256] : sm[I::b(e, sub, lane)]; }, sm, pc[pi], tb.inv + (size_t)pi * Ntt16Layout::kEntries, pl->scale_w[s], pl->scale_c[s], g, sub, lane,
                             [](u64 v) { return ((v >> 30) << 32) | ((u32)v & 0x3FFFFFFFu); });
     }
     __syncthreads();
@@ -340,12 +342,12 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
         const PrimeConst m = pc[pi];
         const ConvConst *cst = consts + 2 * t * ns;
         const bool fp = pl->fp[t];
-        constexpr bool kUnroll = COLS == 8;
+        constexpr bool kUnroll = COLS == 8 || !kShoup;
         if (fp) {
             if (kUnroll && ns == 4) convert_target_fp<COLS, kUnroll ? 4 : 0>(ex, strips, cst, ns, m, sub, lane);
             else if (kUnroll && ns == 3) convert_target_fp<COLS, kUnroll ? 3 : 0>(ex, strips, cst, ns, m, sub, lane);
             else convert_target_fp<COLS, 0>(ex, strips, cst, ns, m, sub, lane);
-        } else if (kPieceSources<LONG> > 0 && !m.small && ns <= kPieceSources<LONG>) {
+        } else if (!kShoup && !m.small && ns <= kPieceSources<LONG>) {
             if (kUnroll && ns == 4) convert_target_pm<COLS, kUnroll ? 4 : 0>(ex, strips, cst, ns, m, sub, lane);
             else if (kUnroll && ns == 3) convert_target_pm<COLS, kUnroll ? 3 : 0>(ex, strips, cst, ns, m, sub, lane);
             else convert_target_pm<COLS, 0>(ex, strips, cst, ns, m, sub, lane);
