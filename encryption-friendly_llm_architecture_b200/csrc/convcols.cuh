@@ -26,6 +26,7 @@
 #include "pdl.cuh"
 #include "kernels.cuh"
 #include "ntt16.cuh"
+#include "conv_shared.hpp"
 #include <type_traits>
 
 namespace hb {
@@ -38,17 +39,18 @@ struct ConvPlan {
     unsigned char order[kMaxPrimes];    // targets in the order they are taken: those of the long primes, which take twice the time, first
     u64 scale_w[8][2], scale_c[8][2];   // as scale_words makes them; [1]: times psi^(-N/2), the twiddle of the last inverse stage
     unsigned char fp[kMaxPrimes];       // target t converts on the FP64 pipe (see ConvFp)
-    uint4 c[kMaxPrimes][2][8];          // [target][half of the rows][source], the second half times psi^(N/2), the twiddle of the first forward stage: C = D / d_s mod target.  Target below 2^44: the 26-bit pieces of C
-                                        // and of C * 2^30; otherwise the 30-bit pieces of C, their sum, 0, or (kPieceSources) the pieces of 29 and 31
-                                        // bits of C and of C * 2^30
-    double d[kMaxPrimes][2][8][4];      // fp targets: C = d1 + d0 with d1 a multiple of 2^21, |d0| <= 2^20, C taken within q/2 of zero; the
-                                        // same for C * 2^30.  Set when every sum of the products is exact in a double
+    // The constants as they lie in shared memory: conv_const_words(ns) * 2 * ns words of 16 bytes for each target, in them [half of the rows][source],
+    // the second half times psi^(N/2), the twiddle of the first forward stage: C = D / d_s mod target.
+    //   fp targets, two words each: doubles C = d1 + d0 with d1 a multiple of 2^21, |d0| <= 2^20, C taken within q/2 of zero; the same for C * 2^30.
+    //               Set when every sum of the products is exact in a double
+    //   others, one word each: below 2^44 the 26-bit pieces of C and of C * 2^30; long targets the 30-bit pieces of C, their sum, 0, or (kPieceSources)
+    //               the pieces of 29 and 31 bits of C and of C * 2^30
+    uint4 k[conv_const_bytes(8, kMaxPrimes) / 16];
 };
-
-union ConvConst { double2 d[2]; uint4 c; }; // the constants of one target, half and source while a CTA works: two of d's pairs, or c
+static_assert(conv_const_bytes(kFpSources, kMaxPrimes) <= conv_const_bytes(8, kMaxPrimes), "room for the longer constants");
 
 template <int COLS> struct StripIndex { // [256 rows][COLS] words in shared memory, COLS pad words per 16 rows: both access patterns are conflict-free
-    static constexpr int kWords = 256 * COLS + 16 * COLS;
+    static constexpr int kWords = strip_words(COLS);
     static __device__ __forceinline__ int a(int e, int sub, int lane) { return e * 17 * COLS + sub * COLS + lane; }  // row e * 16 + sub
     static __device__ __forceinline__ int b(int e, int sub, int lane) { return sub * 17 * COLS + e * COLS + lane; }  // row sub * 16 + e
 };
@@ -178,7 +180,7 @@ __device__ __forceinline__ double finish_small(u64 a0, u64 a1, const SmallFinish
 // units of 2^21), remainder of a1 + a0.  Sixteen products and eight conversions for four sources, 58 FP64 cycles per warp
 // coefficient of the 79 that it takes with four warps a scheduler (four coefficients at a time and a loop over the sources: 88).
 template <int COLS, int NS>
-__device__ __forceinline__ void convert_target_fp(u64 *sm, const u64 *ysm, const ConvConst *cst, int ns_, const PrimeConst &m, int sub, int lane) {
+__device__ __forceinline__ void convert_target_fp(u64 *sm, const u64 *ysm, const uint4 *cst, int ns_, const PrimeConst &m, int sub, int lane) {
     using I = StripIndex<COLS>;
     const int ns = NS ? NS : ns_;
     const double qinv = m.q_inv_f, qd = (double)m.q;
@@ -186,8 +188,7 @@ __device__ __forceinline__ void convert_target_fp(u64 *sm, const u64 *ysm, const
     for (int e0 = 0; e0 < 16; e0 += 8) {
         double a0[8], a1[8];
         auto source = [&](int s, bool first) {
-            const ConvConst &k = cst[(e0 >> 3) * ns + s];
-            const double2 k0 = k.d[0], k1 = k.d[1];
+            const double2 *k = reinterpret_cast<const double2 *>(cst + ((e0 >> 3) * ns + s) * 2), k0 = k[0], k1 = k[1];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
@@ -207,7 +208,7 @@ __device__ __forceinline__ void convert_target_fp(u64 *sm, const u64 *ysm, const
     }
 }
 template <int COLS>
-__device__ __forceinline__ void convert_target_small(u64 *sm, const u64 *ysm, const ConvConst *cst, int ns, const PrimeConst &m, int sub, int lane) {
+__device__ __forceinline__ void convert_target_small(u64 *sm, const u64 *ysm, const uint4 *cst, int ns, const PrimeConst &m, int sub, int lane) {
     using I = StripIndex<COLS>;
     const SmallFinish f = small_finish(m);
     const DsConst ds = ds_const(m);
@@ -218,7 +219,7 @@ __device__ __forceinline__ void convert_target_small(u64 *sm, const u64 *ysm, co
         for (int u = 0; u < 4; ++u) { a0[u] = 0; a1[u] = 0; }
 #pragma unroll 1
         for (int s = 0; s < ns; ++s) {
-            const uint4 c = cst[(e0 >> 3) * ns + s].c;
+            const uint4 c = cst[(e0 >> 3) * ns + s];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
@@ -235,7 +236,7 @@ __device__ __forceinline__ void convert_target_small(u64 *sm, const u64 *ysm, co
     }
 }
 template <int COLS>
-__device__ __forceinline__ void convert_target_wide(u64 *sm, const u64 *ysm, const ConvConst *cst, int ns, const PrimeConst &m, int sub, int lane) {
+__device__ __forceinline__ void convert_target_wide(u64 *sm, const u64 *ysm, const uint4 *cst, int ns, const PrimeConst &m, int sub, int lane) {
     using I = StripIndex<COLS>;
 #pragma unroll 1
     for (int e0 = 0; e0 < 16; e0 += 4) {
@@ -244,7 +245,7 @@ __device__ __forceinline__ void convert_target_wide(u64 *sm, const u64 *ysm, con
         for (int u = 0; u < 4; ++u) { a0[u] = 0; am[u] = 0; a2[u] = 0; }
 #pragma unroll 2
         for (int s = 0; s < ns; ++s) {
-            const uint4 c = cst[(e0 >> 3) * ns + s].c;
+            const uint4 c = cst[(e0 >> 3) * ns + s];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
@@ -261,7 +262,7 @@ __device__ __forceinline__ void convert_target_wide(u64 *sm, const u64 *ysm, con
 // and 2^64, folded as in LongPm::mul: below 6.5 * 2^60.  Four sources take 85 cycles per warp coefficient with four warps a
 // scheduler, three 72; three products a source (convert_target_wide) with their longer reduction 126 and 107.
 template <int COLS, int NS>
-__device__ __forceinline__ void convert_target_pm(u64 *sm, const u64 *ysm, const ConvConst *cst, int ns_, const PrimeConst &m, int sub, int lane) {
+__device__ __forceinline__ void convert_target_pm(u64 *sm, const u64 *ysm, const uint4 *cst, int ns_, const PrimeConst &m, int sub, int lane) {
     using I = StripIndex<COLS>;
     const int ns = NS ? NS : ns_;
     const u32 d2 = 2 * m.d60;
@@ -269,7 +270,7 @@ __device__ __forceinline__ void convert_target_pm(u64 *sm, const u64 *ysm, const
     for (int e0 = 0; e0 < 16; e0 += 4) {
         u64 a[4], b[4];
         auto source = [&](int s, bool first) {
-            const uint4 c = cst[(e0 >> 3) * ns + s].c;
+            const uint4 c = cst[(e0 >> 3) * ns + s];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const u64 y = ysm[s * I::kWords + I::a(e0 + u, sub, lane)];
@@ -294,30 +295,28 @@ template <> inline constexpr int kPieceSources<LongPm> = 4;
 // every few products, and what L1 is left beside the strips holds no more than the twiddles.  All sources are on their way
 // from the start instead of behind one another.  The two together: 139 -> 129 ms
 // of the layer's conversions, products of 256 members at level 8 5.69 -> 5.33 ms.
-// ONE: no group has more than one source.  With Shoup products its words go straight to registers: the way through shared memory and the barrier
-// behind it hide nothing then (one ciphertext at level 8, three digits and ModDown, us, through shared memory / straight: 36.8 / 35.7 and 29.8 /
+// The constants take no more room than they need: with eight sources the second CTA of an SM depends on it (conv_shared.hpp).  Divisions of 24 polynomials
+// by P * q_22, eight sources, us: 32 bytes a constant and one CTA 518, 16 bytes and two 421.
+// MAXNS: the most sources a conversion may have.  With no more of them than groups and Shoup products their words go straight to registers:
+// the way through shared memory and the barrier behind it hide nothing then (one ciphertext at level 8, three digits and ModDown, us, through shared memory / straight: 36.8 / 35.7 and 29.8 /
 // 28.9).  Next to 2^60 it is even: divisions of one ciphertext at level 12 78.3 / 79.1, rotations 135.9 / 135.5.  Six sources on four groups 59.0 /
 // 62.2: there the second strip arrives behind the first one's work.
-template <int COLS, int G, int MINB, bool ONE, class LONG>
+template <int COLS, int G, int MINB, int MAXNS, class LONG>
 __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src, size_t src_outer, u64 *dst, size_t dst_outer, const ConvPlan *__restrict__ plans,
                                                                          const PrimeConst *__restrict__ pc, Ntt16Tables tb) {
     extern __shared__ __align__(128) u64 strips[]; // rows of 32 bytes at an odd multiple of 16 take 2.4 % longer in all
     __shared__ int next, turn[2][G];
     using I = StripIndex<COLS>;
-    constexpr bool kShoup = kPieceSources<LONG> == 0, kOne = ONE && kShoup;
+    constexpr bool kShoup = kPieceSources<LONG> == 0, kOne = MAXNS <= G && kShoup;
     if (threadIdx.x == 0) next = G <= 2 ? G : 0;
     const ConvPlan *pl = plans + blockIdx.y;
-    const int ns = pl->ns, nt = pl->nt;
+    const int ns = pl->ns, nt = pl->nt, words = MAXNS <= kFpSources ? 2 : conv_const_words(ns);
     const int g = threadIdx.x / (COLS * 16), r = threadIdx.x % (COLS * 16), lane = r % COLS, sub = r / COLS;
     const int col = blockIdx.x * COLS + lane;
     const u64 *sp = src + (size_t)blockIdx.z * src_outer + (size_t)pl->src_limb * kN16 + blockIdx.x * COLS;
     u64 *dp = dst + (size_t)blockIdx.z * dst_outer + (size_t)pl->dst_limb * kN16 + col;
-    ConvConst *consts = reinterpret_cast<ConvConst *>(strips + (ns + G) * I::kWords);
-    for (int i = threadIdx.x; i < 2 * nt * ns; i += COLS * 16 * G) {
-        const int t = i / (2 * ns), h = i / ns % 2, s = i % ns;
-        if (pl->fp[t]) { const double2 *k = reinterpret_cast<const double2 *>(pl->d[t][h][s]); consts[i].d[0] = k[0]; consts[i].d[1] = k[1]; }
-        else consts[i].c = pl->c[t][h][s];
-    }
+    uint4 *consts = reinterpret_cast<uint4 *>(strips + (ns + G) * I::kWords);
+    for (int i = threadIdx.x; i < 2 * nt * ns * words; i += COLS * 16 * G) consts[i] = pl->k[i];
     pdl_wait();
     if (!kOne) for (int s = g; s < ns; s += G) strip_fetch<COLS>(sp + (size_t)s * kN16, strips + s * I::kWords, r);
     for (int s = g; s < ns; s += G) {
@@ -340,7 +339,7 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) conv_cols(const u64 *src,
         const int t = pl->order[k];
         const int pi = pl->dst_prime[t];
         const PrimeConst m = pc[pi];
-        const ConvConst *cst = consts + 2 * t * ns;
+        const uint4 *cst = consts + 2 * t * ns * words;
         const bool fp = pl->fp[t];
         constexpr bool kUnroll = COLS == 8 || !kShoup;
         if (fp) {

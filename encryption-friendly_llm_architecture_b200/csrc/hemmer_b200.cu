@@ -269,12 +269,14 @@ void fill_conv(const HostCtx &h, bool pm, ConvPlan &p, const std::vector<int> &s
         const u64 q = h.q[dst[t]], m26 = ((u64)1 << 26) - 1, m30 = ((u64)1 << 30) - 1, m29 = ((u64)1 << 29) - 1;
         p.dst_prime[t] = (unsigned char)dst[t];
         p.order[t] = (unsigned char)t;
-        p.fp[t] = !(q >> 44) && src.size() <= 4;
+        p.fp[t] = !(q >> 44) && src.size() <= (size_t)kFpSources;
+        double fp[2][8][4] = {};
+        uint4 pieces[2][8];
         for (int half = 0; half < 2; ++half) {
             double low = 0, high = 0; // largest sums of the FP64 form, in units of 1 and 2^21
             for (size_t s = 0; s < src.size(); ++s) {
                 const u64 v = half ? hbhost::mulmod(hat(s, q), half_turn(dst[t]), q) : hat(s, q), v30 = hbhost::mulmod(v, ((u64)1 << 30) % q, q);
-                double *d = p.d[t][half][s];
+                double *d = fp[half][s];
                 if (!(q >> 44)) {
                     auto split = [&](u64 w, double *o) { // |w - q * [w > q / 2]| = o[1] + o[0]
                         const i64 c = w > q / 2 ? (i64)w - (i64)q : (i64)w, hi = (c + ((i64)1 << 20)) >> 21;
@@ -282,8 +284,8 @@ void fill_conv(const HostCtx &h, bool pm, ConvPlan &p, const std::vector<int> &s
                     };
                     split(v, d); split(v30, d + 2);
                 }
-                if ((q >> 44) && pm && src.size() <= (size_t)kPieceSources<LongPm>) p.c[t][half][s] = make_uint4((u32)(v & m29), (u32)(v >> 29), (u32)(v30 & m29), (u32)(v30 >> 29));
-                else p.c[t][half][s] = (q >> 44) ? make_uint4((u32)(v & m30), (u32)(v >> 30), (u32)(v & m30) + (u32)(v >> 30), 0) : make_uint4((u32)(v & m26), (u32)(v >> 26), (u32)(v30 & m26), (u32)(v30 >> 26));
+                if ((q >> 44) && pm && src.size() <= (size_t)kPieceSources<LongPm>) pieces[half][s] = make_uint4((u32)(v & m29), (u32)(v >> 29), (u32)(v30 & m29), (u32)(v30 >> 29));
+                else pieces[half][s] = (q >> 44) ? make_uint4((u32)(v & m30), (u32)(v >> 30), (u32)(v & m30) + (u32)(v >> 30), 0) : make_uint4((u32)(v & m26), (u32)(v >> 26), (u32)(v30 & m26), (u32)(v30 >> 26));
                 const double y0 = 0x1p30, y1 = (double)((h.q[src[s]] >> 30) + 1);
                 low += y0 * std::fabs(d[0]) + y1 * std::fabs(d[2]);
                 high += (y0 * std::fabs(d[1]) + y1 * std::fabs(d[3])) * 0x1p-21;
@@ -291,6 +293,11 @@ void fill_conv(const HostCtx &h, bool pm, ConvPlan &p, const std::vector<int> &s
             // a1 - qh * q is formed exactly when |a0| + 2q stays below 2^53; the quotient must be exact to well below one
             if (!(low + 2.0 * (double)q < 0x1p53 && high < 0x1p53)) p.fp[t] = 0;
         }
+        for (int half = 0; half < 2; ++half)
+            for (size_t s = 0; s < src.size(); ++s) {
+                uint4 *k = p.k + conv_const_words(p.ns) * 2 * p.ns * t;
+                if (p.fp[t]) std::memcpy(k + 2 * (half * p.ns + s), fp[half][s], sizeof fp[half][s]); else k[half * p.ns + s] = pieces[half][s];
+            }
     }
     std::stable_sort(p.order, p.order + p.nt, [&](int x, int y) { return (h.q[p.dst_prime[x]] >> 44) && !(h.q[p.dst_prime[y]] >> 44); });
 }
@@ -338,17 +345,24 @@ const ConvPlan *get_conv_plans(hb_ctx *c, int level) {
     c->conv_plans[level] = d;
     return d;
 }
-template <int COLS> size_t strip_bytes(int strips) { return (size_t)strips * StripIndex<COLS>::kWords * 8; }
-size_t conv_const_bytes(int ns, int nt) { return (size_t)2 * ns * nt * sizeof(ConvConst); }
+// of the decomposition's conversions, one per digit of `level`, whose own limbs are no targets
+size_t digit_const_bytes(const HostCtx &h, int level) {
+    size_t most = 0;
+    for (int dg = 0; dg <= h.digit_of(level); ++dg) {
+        const int own = h.digit_hi(dg, level + 1) - h.digit_lo(dg);
+        most = std::max(most, conv_const_bytes(own, level + 1 + h.K - own));
+    }
+    return most;
+}
 void conv_opt_in(hb_ctx *c) {
     if (c->smem_opt_in_conv) return;
     auto allow = [](auto *kernel, size_t bytes) { CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); };
     const size_t consts = conv_const_bytes(8, kMaxPrimes);
     auto all = [&](auto arithmetic) {
         using LONG = decltype(arithmetic);
-        allow(conv_cols<8, 4, 1, false, LONG>, strip_bytes<8>(12) + consts); allow(conv_cols<4, 4, 2, false, LONG>, strip_bytes<4>(12) + consts); allow(conv_cols<4, 8, 1, true, LONG>, strip_bytes<4>(16) + consts);
-        allow(conv_cols<4, 4, 2, true, LONG>, strip_bytes<4>(8) + conv_const_bytes(4, kMaxPrimes)); allow(conv_cols<8, 2, 2, false, LONG>, strip_bytes<8>(6) + conv_const_bytes(4, kMaxPrimes));
-        allow(lift_cols<8, 2, 2, LONG>, strip_bytes<8>(3)); allow(lift_cols<8, 1, 4, LONG>, strip_bytes<8>(2)); allow(lift_cols<4, 4, 2, LONG>, strip_bytes<4>(5)); allow(lift_cols<4, 8, 1, LONG>, strip_bytes<4>(9));
+        allow(conv_cols<8, 4, 1, 8, LONG>, strip_bytes(8, 12) + consts); allow(conv_cols<4, 4, 2, 8, LONG>, strip_bytes(4, 12) + consts); allow(conv_cols<4, 8, 1, 8, LONG>, strip_bytes(4, 16) + consts);
+        allow(conv_cols<4, 4, 2, 4, LONG>, strip_bytes(4, 8) + conv_const_bytes(kFpSources, kMaxPrimes)); allow(conv_cols<8, 2, 2, 4, LONG>, strip_bytes(8, 6) + conv_const_bytes(kFpSources, kMaxPrimes));
+        allow(lift_cols<8, 2, 2, LONG>, strip_bytes(8, 3)); allow(lift_cols<8, 1, 4, LONG>, strip_bytes(8, 2)); allow(lift_cols<4, 4, 2, LONG>, strip_bytes(4, 5)); allow(lift_cols<4, 8, 1, LONG>, strip_bytes(4, 9));
     };
     if (c->tb.t16.pm) all(LongPm{}); else all(LongShoup{});
     c->smem_opt_in_conv = true;
@@ -375,20 +389,19 @@ StripShape conv_shape(int units, int max_ns, int targets) {
 // Rescales: from 96 polynomials on (five waves of CTAs) one group per CTA, so that none waits for the source: 512 polynomials at level 8 1.13 -> 1.02 ms.
 // Fewer keep two groups, whose CTAs are half as long, for the last wave.
 StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : units < 96 ? kStrip8x2 : kStrip8x1; }
-// `plans` conversions (the largest with max_ns sources, `targets` each on average, max_nt at most) of `instances` polynomials in one launch
-void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int targets, int max_nt, int instances) {
+// `plans` conversions (the largest with max_ns sources, `targets` each on average, at most `consts` bytes of constants) of `instances` polynomials in one launch
+void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int targets, size_t consts, int instances) {
     conv_opt_in(c);
-    const size_t consts = conv_const_bytes(max_ns, max_nt);
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
         launch(c, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
     };
     auto shapes = [&](auto arithmetic) {
         using LONG = decltype(arithmetic);
         switch (conv_shape(instances * count, max_ns, targets)) {
-        case kStrip8x2: go(conv_cols<8, 2, 2, false, LONG>, 8, 2, strip_bytes<8>(max_ns + 2) + consts); break;
-        case kStrip8x4: go(conv_cols<8, 4, 1, false, LONG>, 8, 4, strip_bytes<8>(max_ns + 4) + consts); break;
-        case kStrip4x4: go(max_ns <= 4 ? conv_cols<4, 4, 2, true, LONG> : conv_cols<4, 4, 2, false, LONG>, 4, 4, strip_bytes<4>(max_ns + 4) + consts); break;
-        default: go(conv_cols<4, 8, 1, true, LONG>, 4, 8, strip_bytes<4>(max_ns + 8) + consts); break; // at most eight sources
+        case kStrip8x2: go(conv_cols<8, 2, 2, 4, LONG>, 8, 2, strip_bytes(8, max_ns + 2) + consts); break;
+        case kStrip8x4: go(conv_cols<8, 4, 1, 8, LONG>, 8, 4, strip_bytes(8, max_ns + 4) + consts); break;
+        case kStrip4x4: go(max_ns <= 4 ? conv_cols<4, 4, 2, 4, LONG> : conv_cols<4, 4, 2, 8, LONG>, 4, 4, strip_bytes(4, max_ns + 4) + consts); break;
+        default: go(conv_cols<4, 8, 1, 8, LONG>, 4, 8, strip_bytes(4, max_ns + 8) + consts); break;
         }
     };
     if (c->tb.t16.pm) shapes(LongPm{}); else shapes(LongShoup{});
@@ -402,10 +415,10 @@ void launch_lift(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, int
     auto shapes = [&](auto arithmetic) {
         using LONG = decltype(arithmetic);
         switch (lift_shape(instances)) {
-        case kStrip4x8: go(lift_cols<4, 8, 1, LONG>, 4, 8, strip_bytes<4>(9)); break;
-        case kStrip4x4: go(lift_cols<4, 4, 2, LONG>, 4, 4, strip_bytes<4>(5)); break;
-        case kStrip8x2: go(lift_cols<8, 2, 2, LONG>, 8, 2, strip_bytes<8>(3)); break;
-        default: go(lift_cols<8, 1, 4, LONG>, 8, 1, strip_bytes<8>(2)); break;
+        case kStrip4x8: go(lift_cols<4, 8, 1, LONG>, 4, 8, strip_bytes(4, 9)); break;
+        case kStrip4x4: go(lift_cols<4, 4, 2, LONG>, 4, 4, strip_bytes(4, 5)); break;
+        case kStrip8x2: go(lift_cols<8, 2, 2, LONG>, 8, 2, strip_bytes(8, 3)); break;
+        default: go(lift_cols<8, 1, 4, LONG>, 8, 1, strip_bytes(8, 2)); break;
         }
     };
     if (c->tb.t16.pm) shapes(LongPm{}); else shapes(LongShoup{});
@@ -450,7 +463,7 @@ void ks_decompose(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch,
     Tmp acoef(c, (size_t)batch * n);
     if (c->logn == 16) {
         inv_rows(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level));
-        launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.dt_count / d.nd, d.ne, batch);
+        launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.dt_count / d.nd, digit_const_bytes(*c->h, level), batch);
         fwd_rows(c, dt, (size_t)d.dt_count * N, batch * d.dt_count, d.dtmap);
         return;
     }
@@ -470,7 +483,7 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, siz
         const ConvPlan *cv = get_conv_plans(c, level);
         u64 *sp = acc + (size_t)n * N;
         inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, total * 2 * K, pm);
-        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, n, n, total * 2);
+        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, n, conv_const_bytes(K, n), total * 2);
         const RowsFin f{acc, (size_t)ne * N, out, out_outer, 2, batch, add_outer};
         LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, total * 2, f, c->p_inv_scale, sl, c->pc, c->tb.t16));
         CK(cudaGetLastError());
@@ -641,7 +654,7 @@ hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch, hb_ct *dst = null
         if (c->logn == 16) {
             const ConvPlan *cv = get_conv_plans(c, level);
             inv_rows(c, src, (size_t)ne * N, src, (size_t)ne * N, batch * 2 * ns, sm);
-            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, level, level, batch * 2);
+            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, level, conv_const_bytes(ns, level), batch * 2);
             const RowsFin f{E, (size_t)ne * N, out, (size_t)2 * level * N, 2, 1, 0};
             LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], NoAddends{}, c->pc, c->tb.t16));
             CK(cudaGetLastError());

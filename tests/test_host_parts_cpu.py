@@ -26,3 +26,7 @@ def test_programs_on_the_cpp_headers_compile():
     for name in ("hemmer_snippet", "operands_after_error", "evaluator_calls"):
         subprocess.check_call(["g++", "-fsyntax-only", "-std=c++17", "-Wall", os.path.join(ROOT, "tests", "integration", name + ".cpp"), "-I", os.path.join(ROOT, "include"),
                                "-I", os.path.join(ROOT, PKG_NAME, "csrc", "hellm")])
+
+
+def test_shared_memory_of_the_conversions(tmp_path):
+    _run(tmp_path, "conv_shared")
