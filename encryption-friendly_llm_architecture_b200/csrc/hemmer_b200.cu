@@ -1208,8 +1208,8 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             const u64 below60 = q < ((u64)1 << 60) ? ((u64)1 << 60) - q : 0;
             p.d60 = below60 < ((u64)1 << 26) ? (u32)below60 : 0;
             p.q7 = p.fp ? 0 : q * 7;
-            std::vector<u64> f, fs, iv, ivs;
-            c->h->twiddles(i, f, fs, iv, ivs);
+            std::vector<u64> f, iv;
+            c->h->twiddles(i, f, iv);
             if (big) {
                 auto entry = [&](u64 w) { ulonglong2 e; scale_words(w, q, pm, e.x, e.y); return e; };
                 ntt16_fill_table(&t16[(size_t)i * Ntt16Layout::kEntries], [&](unsigned k) { return entry(f[k]); });
@@ -1219,10 +1219,10 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
                     ntt16_fill_rows_b8(&b8[((size_t)np + i) * kRowsB8], [&](unsigned k) { return (double)iv[k]; });
                 }
             } else {
-                std::memcpy(&tw[((size_t)0 * np + i) * N], f.data(), (size_t)N * 8);
-                std::memcpy(&tw[((size_t)1 * np + i) * N], fs.data(), (size_t)N * 8);
-                std::memcpy(&tw[((size_t)2 * np + i) * N], iv.data(), (size_t)N * 8);
-                std::memcpy(&tw[((size_t)3 * np + i) * N], ivs.data(), (size_t)N * 8);
+                for (int k = 0; k < N; ++k) { // values and Shoup companions
+                    tw[((size_t)0 * np + i) * N + k] = f[k]; tw[((size_t)1 * np + i) * N + k] = hbhost::shoup(f[k], q);
+                    tw[((size_t)2 * np + i) * N + k] = iv[k]; tw[((size_t)3 * np + i) * N + k] = hbhost::shoup(iv[k], q);
+                }
             }
         }
         CK(cudaMalloc(&c->pc, sizeof(PrimeConst) * np));

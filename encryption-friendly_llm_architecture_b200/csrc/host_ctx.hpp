@@ -167,14 +167,13 @@ struct HostCtx {
         }
     }
     // twiddle tables of prime i: fwd[k] = psi^bitrev(k), inv[k] = psi^-bitrev(k)
-    void twiddles(int i, std::vector<u64> &fwd, std::vector<u64> &fwd_sh, std::vector<u64> &inv, std::vector<u64> &inv_sh) const {
+    void twiddles(int i, std::vector<u64> &fwd, std::vector<u64> &inv) const {
         const u64 m = q[i], r = psi_root[i], ri = invmod(r, m);
-        fwd.resize(N); fwd_sh.resize(N); inv.resize(N); inv_sh.resize(N);
+        fwd.resize(N); inv.resize(N);
         u64 a = 1, b = 1;
         for (int k = 0; k < N; ++k) {
             u32 pos = reverse_bits((u32)k, logn); // power k lands at table slot bitrev(k)
-            fwd[pos] = a; fwd_sh[pos] = shoup(a, m);
-            inv[pos] = b; inv_sh[pos] = shoup(b, m);
+            fwd[pos] = a; inv[pos] = b;
             a = mulmod(a, r, m); b = mulmod(b, ri, m);
         }
     }

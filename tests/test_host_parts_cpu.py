@@ -30,3 +30,7 @@ def test_programs_on_the_cpp_headers_compile():
 
 def test_shared_memory_of_the_conversions(tmp_path):
     _run(tmp_path, "conv_shared")
+
+
+def test_twiddle_values(tmp_path):
+    _run(tmp_path, "twiddles")
