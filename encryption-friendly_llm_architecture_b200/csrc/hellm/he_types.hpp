@@ -199,6 +199,7 @@ class Evaluator {
     // the same with the operands one by one: sum k from the operands k * count ...
     static constexpr int kMaxSumTerms = 24;
     Ciphertext multSums(const std::vector<Ciphertext> &x, const std::vector<const Plaintext *> &p, int count) const {
+        if (count < 1 || x.empty() || x.size() % (size_t)count || p.size() != x.size()) throw std::invalid_argument("[multSums] terms and masks do not make whole sums");
         std::vector<const hb_ct *> rx; std::vector<const hb_pt *> rp;
         for (const auto &y : x) rx.push_back(y.raw());
         for (auto *q : p) rp.push_back(q->raw());

@@ -1,5 +1,6 @@
 // Evaluator calls of a separately compiled program that no part of the library makes itself: stack and tensorAccumulateHalves give the
-// residues of concat and of tensorAccumulate on the two halves.  Returns 0 when they do.
+// residues of concat and of tensorAccumulate on the two halves; multSums refuses terms and masks that do not make whole sums.  Returns 0 when
+// they do.
 #include "HEMMer.hpp"
 
 #include <cstdio>
@@ -34,7 +35,17 @@ int main() {
         ev.tensorAccumulate(plain, ev.view(stacked, 0, 3), ev.view(stacked, 3, 3));
         if (residues(halves) != residues(plain)) ++bad;
     }
+    std::vector<HELLM::Ciphertext> terms;
+    for (int k = 0; k < 3; ++k) terms.push_back(ev.view(stacked, k, 1));
+    const HELLM::Plaintext mask = ev.encode(HELLM::Message((size_t)512), terms[0].getLevel());
+    const std::vector<const HELLM::Plaintext *> three(3, &mask), two(2, &mask);
+    const auto refused = [&](const std::vector<HELLM::Ciphertext> &x, const std::vector<const HELLM::Plaintext *> &p, int count) {
+        try { ev.multSums(x, p, count); } catch (const std::invalid_argument &) { return true; }
+        return false;
+    };
+    if (refused(terms, three, 3) || refused(terms, three, 1)) ++bad;
+    if (!refused(terms, three, 2) || !refused(terms, three, 0) || !refused(terms, three, -1) || !refused(terms, two, 1) || !refused({}, {}, 1)) ++bad;
     delete hemmer;
-    std::printf("%d of 3 results differ\n", bad);
+    std::printf("%d of 5 results differ\n", bad);
     return bad ? 1 : 0;
 }
