@@ -41,3 +41,20 @@ def test_loops_hold_as_many_iterations_as_members_allow(pkg, gpu_small):
             got = g.ct_export(op(join(a[:batch]), join(b[:batch])))
             for k in {0, batch - 1}:
                 _same(np.ascontiguousarray(got[k::batch]), alone[n, k], f"operation {n}, member {k} of {batch}")
+
+
+def test_loops_of_the_full_ring(pkg, gpu_full):
+    """The same where the sums are rescaled and the chains rotated by the kernels of 2^16 points: two held iterations of a product and five of the
+    copies against six and twelve of one operand alone; with packed operands five against twelve."""
+    g = gpu_full
+    H = pkg.open_hemmer(g)
+    H.set_schedule(0)
+    plain = [lambda x, y: H.single_cc_matmul(x, y, 2).ct, lambda x, y: H.matmul_pre(x, 2)]
+    packed = [lambda x, y: H.packed_matmul(x, y, 2).ct, lambda x, y: H.packed_matmul_pre_rot(H.packed_matmul_pre(x, 2), 2)]
+    for pack, ops in ((False, plain), (True, packed)):
+        a, join = _operands(pkg, g, H, pack, 3, 100)
+        b, _ = _operands(pkg, g, H, pack, 3, 201)
+        for n, op in enumerate(ops):
+            got = g.ct_export(op(join(a), join(b)))
+            for k in (0, 2):
+                _same(np.ascontiguousarray(got[k::3]), g.ct_export(op(a[k], b[k])), f"operation {n}, packed {pack}, member {k}")

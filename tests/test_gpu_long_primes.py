@@ -16,8 +16,8 @@ PARAMS = {
 
 @pytest.mark.parametrize("name", sorted(PARAMS))
 def test_long_primes_against_the_oracle(pkg, oracle_so, name):
-    """Residues 0, 1, q - 1, alternating and random: sums of a radix-16 round reach their bounds where all inputs are q - 1.  Levels 0 and 2: one
-    limb alone and beside short ones; rotation and rescale take the long primes through every pass."""
+    """Residues 0, 1, q - 1, alternating and random (the bounds inside a round are far above what canonical residues reach; test_long_primes_cpu.py
+    has those).  Levels 0 and 2: one limb alone and beside short ones; rotation and rescale take the long primes through every pass."""
     prm = dict(log_n=16, max_level=2, dnum=2, num_special=2, hamming_weight=64, **PARAMS[name])
     g, o = pkg.open_gpu(pkg.make_params(**prm)), open_oracle(pkg, oracle_so, **prm)
     for lib in (g, o):
