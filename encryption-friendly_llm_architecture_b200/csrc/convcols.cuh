@@ -11,10 +11,11 @@
 // writes instead of 3 S + S + 3 T limb transfers, and one launch instead of three.  The constants of a conversion carry the scale of the
 // inverse transforms, the twiddle of their last stage and that of the first forward stage, which so cost no products of their own.
 //
-// At S = 4, T = 6 (the division by P * q_level at level 6) 96 polynomials took 413 us with Shoup butterflies, 363 with folded pieces (both under the profiler, before
-// convert_target_pm): FP64 a third of the cycles, the wide multiply pipe 40 %, half of the issue slots; four warps a scheduler, whose fixed latencies, shared-memory exchanges and bursts on one pipe are the rest.  FP64 and integer products
-// do overlap on a scheduler, unless the latter carry 64-bit addends.  What did not help: a persistent version in which some groups transform
-// the next strip's sources while others convert targets, more warps with fewer registers, CTAs of an SM started half a turn apart.
+// At S = 4, T = 6 (the division by P * q_level at level 6) 96 polynomials take 315 us (324 with the counters; 413 with Shoup butterflies, 363 before the
+// targets next to 2^60 were converted by pieces): half of the issue slots, FP64 38 % of the cycles, the wide multiply pipe 37 %.  Four warps a scheduler,
+// whose fixed latencies, shared-memory exchanges and bursts on one pipe are the rest.  FP64 and integer products do overlap on a scheduler, unless the
+// latter carry 64-bit addends.  What did not help: six warps a scheduler (4 x 4 strips, three CTAs at 80 registers, spills of 8 bytes: 364 us), a
+// persistent version in which some groups transform the next strip's sources while others convert targets, CTAs of an SM started half a turn apart.
 //
 // A CTA is G groups of COLS * 16 threads.  Sources are dealt to the groups, then (one CTA barrier later) targets; inside a
 // group a radix-16 round exchanges through shared memory behind a named barrier of that group only, so one group's loads,
@@ -414,7 +415,7 @@ __global__ void __launch_bounds__(COLS * 16 * G, MINB) lift_cols(const u64 *src,
 // t arrives half-forward (conv_cols / lift_cols).  grid = (16, n, instances), instance bp = b * np + p.  The operands of the last
 // step are read after the barrier of the final exchange, when the registers of the transform are free.  Without addends bound by DRAM
 // and the FP64 pipe together: 128 polynomials of six limbs 226 us, 5.4 TB/s of DRAM traffic (0.83 of a copy), FP64 pipe 50 % busy; with
-// addends 424 us for 96 of nine limbs, 4.5 TB/s.  64 registers for four CTAs per SM spill 8 to 16 bytes a thread.
+// addends 424 us for 96 of nine limbs, 4.5 TB/s.  64 registers for four CTAs per SM spill 4 to 16 bytes a thread.
 struct RowsFin {
     const u64 *x; size_t x_outer;            // instance stride of x; limb l at l * N
     u64 *out; size_t out_outer;              // ciphertext stride; polynomial p at p * n * N

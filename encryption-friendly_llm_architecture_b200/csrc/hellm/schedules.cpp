@@ -294,11 +294,13 @@ Chains start_chains(Env &e, const std::vector<const Ciphertext *> &ops, const st
 }
 
 // Only the rotations of a chain wait for one another; the masked sums of several iterations are made by one launch sequence (few members leave
-// most of the GPU idle in each of its five launches): up to 32 polynomials of sums, and what the terms of a call allow.  One product of one
-// tile 42.8 -> 39.3 ms.
+// most of the GPU idle in each of its five launches): up to 32 polynomials of sums, and what the terms of a call allow.  Products / copies of a
+// left operand, ms, one iteration at a time and held, with 1, 2, 4, 5 and 9 operands together: 45.5 / 37.9, 73.5 / 64.7, 132 / 118, 163 / 149, 297 / 273 and
+// 25.9 / 19.7, 39.8 / 32.4, 64.7 / 57.1, 81.4 / 70.5, 136 / 123.  The second of each pair has the faster 60-bit products and conversions too; with nine,
+// where one iteration is held, the gain of 1.09 and 1.10 is theirs alone.
 class HeldChains {
   public:
-    HeldChains(Env &e, const Chains &c) : e_(e), sums_(c.count() / 2), hold_(std::max(1, std::min(Evaluator::kMaxSumTerms / c.count(), 32 * c.count() / (2 * sums_ * c.x->getBatch())))) {}
+    HeldChains(Env &e, const Chains &c) : e_(e), sums_(c.count() / 2), hold_(std::max(1, std::min(Evaluator::kMaxSumTerms / c.count(), 32 / c.x->getBatch()))) {}
     // the chains as they are now, with the masks of their groups
     void add(const Chains &c, std::vector<const Plaintext *> masks) { x_.push_back(c.x); masks_.push_back(std::move(masks)); }
     bool full() const { return held() == hold_; }

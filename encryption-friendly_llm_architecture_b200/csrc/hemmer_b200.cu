@@ -370,14 +370,18 @@ void conv_opt_in(hb_ctx *c) {
 // Strip width and groups of a launch over `units` (polynomial, conversion) pairs.  At most two units: narrow strips and many groups, so that
 // all sources and all targets of a unit are worked on at once.  Up to twelve: narrow strips, two CTAs per SM, for the last wave.
 // Beyond: strips of eight columns (64-byte runs) and two groups, two CTAs per SM, whose barriers and loads cover each other, as long as their
-// strips fit (four sources); otherwise four groups and one CTA.  Calls, us, before the wide strips / (4 x 4) / (8 x 2), the shape of the launches
-// over the units named: products of level 8, 18 units (six members) 501 / 497 / 488; rotations of level 2, 16 units 208 / 203 / 192, 40 units 427 /
-// 424 / 389.  Launches, (8 x 4) / (8 x 2): 96 polynomials of the division at level 6 858 / 815, the conversions of 256 products at level 8 3093 / 2863.
+// strips fit (four sources); otherwise four groups and one CTA.  Calls, us, (4 x 8) / (4 x 4) / (8 x 2): decompositions of level 7, 2 units 47 / 45 / 58,
+// divisions 53 / 59 / 62, 4 units 88 / 81 / 94, 10 units 175 / 163 / 171, 18 units 279 / 260 / 256, 40 units 594 / 546 / 533; decompositions of level 2, 17
+// units 111 / 92 / 83, of level 12, 24 units 280 / 260 / 254.  Launches, us, (8 x 4) / (8 x 2): 192 polynomials of the division at level 6 696 / 604,
+// the conversions of 256 products at level 8 3174 / 2719 and 2079 / 1797.
 // The wide strips lose where few SMs have one CTA more than the others: 15, 16, 19 and 20 units leave a tenth to a half of the SMs with it,
-// and a CTA with four sources and many targets is long.  Calls, us, before / (4 x 4) / (8 x 2): rotations of five members at level 7 (15 units) 299 /
-// 299 / 310, products of eight at level 6 (16 units) 459 / 453 / 465; divisions of level 7, 16 units 257 / 254 / 261, 20 units 317 / 312 / 325.  Up to five
-// targets it does not show (division of level 3, 16 units 157 / 151 / 141; level 5, 20 units 219 / 212 / 214), nor with the three sources of
-// a ModDown (products of eight members at level 7, 16 units 586 / 577 / 567).
+// and a CTA with four sources and many targets is long.  Calls, us, (4 x 4) / (8 x 2): divisions of level 7, 16 units 234 / 238, 20 units 289 / 293, of
+// level 6 169 / 171 and 206 / 208.  Up to five targets it does not show (divisions of level 5, 16 units 157 / 155, 20 units 190 / 188), nor with the
+// three sources of a ModDown (level 7, 206 / 205 and 253 / 252); decompositions of level 12 go either way (179 / 180 and 222 / 221).
+// The line at twelve was drawn when the narrow strips were ahead up to there; now (8 x 2) is from seven units on, except at 10, 14, 16 and 20 of the
+// division (decompositions of level 2, 8 units 56 / 51; divisions of level 3, 8 units 84 / 76, of level 7, 8 units 134 / 131, 14 units 216 / 219).
+// More than four sources, (4 x 4) / (8 x 4): divisions of seven sources 32 units 425 / 434, 40 units 520 / 536; of eight 48 units 1120 / 1140;
+// a digit of seven limbs 40 units 425 / 411.
 enum StripShape { kStrip8x1, kStrip8x2, kStrip8x4, kStrip4x4, kStrip4x8 };
 StripShape conv_shape(int units, int max_ns, int targets) {
     if (units <= 2) return kStrip4x8;
@@ -386,8 +390,10 @@ StripShape conv_shape(int units, int max_ns, int targets) {
     const int more = units * 32 % 148; // SMs with one CTA more
     return units <= 20 && max_ns == 4 && targets > 5 && more >= 148 / 10 && more < 148 / 2 ? kStrip4x4 : kStrip8x2;
 }
-// Rescales: from 96 polynomials on (five waves of CTAs) one group per CTA, so that none waits for the source: 512 polynomials at level 8 1.13 -> 1.02 ms.
-// Fewer keep two groups, whose CTAs are half as long, for the last wave.
+// Rescales: from 96 polynomials on one group per CTA, so that none waits for the source: 512 polynomials at level 8 1.14 -> 1.02 ms.  Calls, us, (4 x 4) / two
+// groups / one: level 8, 4 polynomials 61 / 67 / 69, 8 polynomials 100 / 96 / 115, 16 polynomials 179 / 174 / 174, 48 polynomials 508 / 493 / 485, 94 polynomials
+// 963 / 929 / 912, 96 polynomials 982 / 942 / 926; level 4, 16 polynomials 107 / 102 / 100, 96 polynomials 567 / 533 / 521.  The line lies where the
+// gain was seen first; one group is ahead by 1 to 2 % from 32 polynomials on.
 StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : units < 96 ? kStrip8x2 : kStrip8x1; }
 // `plans` conversions (the largest with max_ns sources, `targets` each on average, at most `consts` bytes of constants) of `instances` polynomials in one launch
 void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int targets, size_t consts, int instances) {

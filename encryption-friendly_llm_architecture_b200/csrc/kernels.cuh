@@ -665,7 +665,7 @@ struct SwitchList { SwitchGroup s[kMaxSwitchGroups]; int count; };
 // a thread keeps the key words of its EL coefficients in registers (as doubles, or cut into pieces) and walks over the
 // members with the next member's digits in flight, so the keys -- two thirds of the words a member needs -- are read once.
 // One member per CTA read and converted them every time: 517 us for 64 members at level 6.  Bound by DRAM: 48 members at level 8 take
-// 285 us at 5.3 TB/s (0.82 of a copy), 43 % of the issue slots.  Eight digits spill (132 bytes a thread), seven 12, fewer none.
+// 285 us at 5.3 TB/s (0.82 of a copy), 43 % of the issue slots.  Eight digits spill (160 bytes a thread), seven 32, fewer none.
 // grid = (N/(256*EL), groups * ceil(batch/per), ne); ND = digits in use
 template <int ND, int EL>
 __global__ void __launch_bounds__(256, EL == 1 ? 4 : ND <= 2 ? 3 : 2) k_ks_inner(u64 *acc, const __grid_constant__ SwitchList sl, int batch, int per, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl,
@@ -1215,9 +1215,9 @@ __global__ void __launch_bounds__(256, 2) k_ks_inner_mk(u64 *E, const u64 *c0, c
 // input members with the next member's words in flight.  Up to eleven masked-key words meet six words per member and coefficient;
 // staging both in shared memory by bulk copies for three members at a time took 1.6 times as long (they crossed L2 for every
 // third member, and a CTA's copies, sums and stores did not overlap).  Two coefficients per thread and two CTAs per SM: 869 us a launch
-// for 168 outputs at level 6; one coefficient and three CTAs 837 us, four CTAs 776 us (64 registers, of which two digits spill 24
-// bytes a thread): the integer chains of the 60-bit limbs want warps more than they want independent work in a thread.  65 % of the
-// issue slots and 52 % of the wide multiply-adds for 64 outputs (367 us), DRAM 3.1 TB/s; in a third of the cycles it waits for loads.
+// for 168 outputs at level 6; one coefficient and three CTAs 837 us, four CTAs 776 us (64 registers), 712 with the
+// products and additions of the 60-bit limbs apart: their integer chains want warps more than they want independent work in a thread.  With joined products
+// 65 % of the issue slots and 52 % of the wide multiply-adds for 64 outputs (367 us), DRAM 3.1 TB/s; in a third of the cycles it waits for loads.
 // grid = (N/256, groups * ceil(batch/per), ne)
 template <int ND, int CNT>
 __device__ __forceinline__ void ks_inner_mkr_body(u64 *o, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const MaskedRot &mr, int b0, int b1, const KsPlan *__restrict__ pl,

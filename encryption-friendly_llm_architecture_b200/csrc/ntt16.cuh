@@ -113,7 +113,7 @@ template <class T> struct TwiddlesB<T, true> {
     __device__ __forceinline__ T operator[](int j) const { return w[j]; }
 };
 
-// ---------------- Shoup butterflies on integers (primes of 44 bits and more) ----------------
+// ---------------- Shoup butterflies on integers (primes of 45 bits and more) ----------------
 // exact quotients, values in [0, 4q) and [0, 2q): the small-ring kernel
 __device__ __forceinline__ void ct_bfly(u64 &x, u64 &y, u64 w, u64 ws, u64 q, u64 q2) {
     x = x >= q2 ? x - q2 : x;
@@ -319,7 +319,7 @@ __device__ __forceinline__ u64 ds_store(double v, const DsConst &c, double shift
     const double rb = __fma_rn(-k, c.qd, v2 + kTwo52);                   // 2^52 + (v2 - k q), exact
     return (u64)__double_as_longlong(rb) & 0x000FFFFFFFFFFFFFull;
 }
-// MADE: as in fwd16_int
+// MADE: as in LongShoup::fwd16
 template <bool MADE = false, class TW> __device__ __forceinline__ void fwd16_ds(double (&v)[16], const TW &tp, const DsConst &c) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) {

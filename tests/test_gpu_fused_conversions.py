@@ -120,7 +120,8 @@ def shoup(request, pkg, oracle_so):
     for lib in (g, o):
         lib.keygen()
         lib.gen_rot_keys([3])
-    return g, o
+    yield g, o
+    g.close()
 
 
 def test_one_member_with_shoup_products(shoup):

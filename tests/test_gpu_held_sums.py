@@ -43,10 +43,11 @@ def test_loops_hold_as_many_iterations_as_members_allow(pkg, gpu_small):
                 _same(np.ascontiguousarray(got[k::batch]), alone[n, k], f"operation {n}, member {k} of {batch}")
 
 
-def test_loops_of_the_full_ring(pkg, gpu_full):
+def test_loops_of_the_full_ring(pkg):
     """The same where the sums are rescaled and the chains rotated by the kernels of 2^16 points: two held iterations of a product and five of the
     copies against six and twelve of one operand alone; with packed operands five against twelve."""
-    g = gpu_full
+    g = pkg.open_gpu(pkg.make_params())
+    g.keygen()
     H = pkg.open_hemmer(g)
     H.set_schedule(0)
     plain = [lambda x, y: H.single_cc_matmul(x, y, 2).ct, lambda x, y: H.matmul_pre(x, 2)]
@@ -58,3 +59,5 @@ def test_loops_of_the_full_ring(pkg, gpu_full):
             got = g.ct_export(op(join(a), join(b)))
             for k in (0, 2):
                 _same(np.ascontiguousarray(got[k::3]), g.ct_export(op(a[k], b[k])), f"operation {n}, packed {pack}, member {k}")
+    H.close()
+    g.close()
