@@ -157,6 +157,28 @@ def test_batches_with_shoup_products(shoup, batch):
             assert np.array_equal(got[k:k + 1], g.ct_export(op(_ct(g, data[k:k + 1])))), f"operation {n}, member {k} of {batch}"
 
 
+def test_eight_sources_and_thirty_limbs(pkg, oracle_so):
+    """Digits of seven, eight and eight limbs, divisions of eight sources, up to 23 targets: the most constants beside the most strips; one member and two."""
+    prm = dict(log_n=16, hamming_weight=64, max_level=22, dnum=3, num_special=7)
+    g, o = pkg.open_gpu(pkg.make_params(**prm)), open_oracle(pkg, oracle_so, **prm)
+    for lib in (g, o):
+        lib.keygen()
+        lib.gen_rot_keys([3, -5])
+    m = (np.random.default_rng(7).uniform(0, 1, g.slots) > 0.5).astype(np.float64)
+    for level in (22, 15):
+        data = rand_ct_residues(g, level, 2, 2, seed=70 + level)
+        for l in range(level + 1):
+            data[1, :, l, ::2] = np.uint64(int(g.primes[l]) - 1)
+        x = _ct(o, data)
+        want = [o.ct_export(c) for c in (o.rotate(x, 3), o.assemble_rot(x, 3, o.encode_ext(m, level), -5, o.encode_ext(1.0 - m, level)))]
+        keys = g.masked_key(3, g.encode_ext(m, level)), g.masked_key(-5, g.encode_ext(1.0 - m, level))
+        for first in (0, 1):  # both members, then the second alone
+            x = _ct(g, data[first:])
+            for k, c in enumerate((g.rotate(x, 3), g.assemble_masked(x, g.decompose(x), *keys))):
+                assert np.array_equal(g.ct_export(c), want[k][first:]), f"operation {k} at level {level}, {2 - first} members"
+    g.close()
+
+
 @pytest.mark.parametrize("q_bits", [26, 27, 28, 34])
 def test_short_scaling_primes_of_2_16_points(pkg, oracle_so, q_bits):
     """Digits of six and seven limbs convert to scaling primes of 26 to 34 bits on the integer pipe, where the quotient of the first
