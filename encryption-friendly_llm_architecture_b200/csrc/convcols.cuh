@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
         fwd16_ds(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[e * 17 + clo] = v[e];
-        __syncthreads();
+        __syncwarp();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smd[clo * 17 + e];
         fwd16_ds8(v, tw, c);
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
         u64 x[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) x[e] = xp[e * 16];
-        __syncthreads();
+        __syncwarp();
         const double sf = __longlong_as_double((long long)sc.c[l]), qinv_up = c.qinv * (1.0 + 0x1p-50);
         const u64 sw = sc.w[l];
 #pragma unroll
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
         LONG::template fwd16<2>(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = v[e];
-        __syncthreads();
+        __syncwarp();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
         LONG::template fwd16<3>(v, tw, c);
@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows_fin(const u64 *t, 
         u64 x[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) x[e] = xp[e * 16];
-        __syncthreads();
+        __syncwarp();
         const u64 sw = sc.w[l], ss = sc.c[l];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {

@@ -5,7 +5,9 @@
 // The limb is a 256 x 256 matrix (index = row*256 + col).  The forward transform is a column pass (stages 1-8,
 // butterfly distance >= 256) followed by a row pass (stages 9-16); the inverse runs the row pass first.  A pass moves
 // a limb through HBM once: a CTA of 256 threads owns 16 columns (or 16 rows), every thread keeps 16 coefficients in
-// registers and performs four butterfly stages at a time (radix 16), exchanging through shared memory once.
+// registers and performs four butterfly stages at a time (radix 16), exchanging through shared memory once.  The threads of a row are half a
+// warp, so the row passes exchange behind a warp barrier: with a barrier of the CTA its warps loaded, computed and stored together (scores of twelve
+// heads: forward row passes 221 -> 191 us a launch, inverse ones 130 -> 122, with the last step of a division 247 -> 233).
 //
 // Two things set these kernels apart from a textbook radix-2 transform:
 //
@@ -476,7 +478,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows(const u64 *src, Li
         fwd16_ds(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[e * 17 + clo] = v[e];
-        __syncthreads();
+        __syncwarp();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smd[clo * 17 + e];
         fwd16_ds8(v, tw, c);
@@ -493,14 +495,14 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_fwd_rows(const u64 *src, Li
         LONG::template fwd16<2>(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = v[e];
-        __syncthreads();
+        __syncwarp();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[clo * 17 + e];
         LONG::template fwd16<3>(v, tw, c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = LONG::canon(v[e], c);
     }
-    __syncthreads();
+    __syncwarp();
 #pragma unroll
     for (int e = 0; e < 16; ++e) o[e * 16] = smr[e * 17 + clo];
 }
@@ -522,7 +524,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_rows(const u64 *src, Li
         pdl_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = p[e * 16];
-        __syncthreads();
+        __syncwarp();
     };
     if (m.small) {
         const TwiddlesB<double, MINB <= 2> tw(tb.invB8 + (size_t)pi * kRowsB8 + (row * 15) * 16 + clo);
@@ -535,7 +537,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_rows(const u64 *src, Li
         inv16_ds8(v, tw, c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smd[clo * 17 + e] = v[e]; // the words this thread read itself
-        __syncthreads();
+        __syncwarp();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smd[e * 17 + clo];
         inv16_ds(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
@@ -552,7 +554,7 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_rows(const u64 *src, Li
         LONG::inv16(v, tw, c);
 #pragma unroll
         for (int e = 0; e < 16; ++e) smr[clo * 17 + e] = v[e];
-        __syncthreads();
+        __syncwarp();
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = smr[e * 17 + clo];
         LONG::inv16(v, TwiddlesA(tab + Ntt16Layout::rowsA(row, 0)), c);
