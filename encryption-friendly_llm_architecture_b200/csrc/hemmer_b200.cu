@@ -7,6 +7,7 @@
 #include "kernels.cuh"
 #include "ntt.cuh"
 #include "convcols.cuh"
+#include "ksrows.cuh"
 #include "embed.cuh"
 #include "host_threads.hpp"
 #include "pool.hpp"
@@ -457,6 +458,16 @@ PlanDims plan_dims(hb_ctx *c, int level) {
 
 size_t key_limbs(hb_ctx *c, int level) { const PlanDims d = plan_dims(c, level); return (size_t)2 * d.nd * d.ne; } // the part of a switching key one key switch reads
 
+// On 2^16 rings: the lifted digits before their forward row pass
+void ks_lift(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch, u64 *dt) {
+    const PlanDims d = plan_dims(c, level);
+    const int N = c->N, n = d.n;
+    Tmp acoef(c, (size_t)batch * n);
+    inv_rows(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level));
+    launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.dt_count / d.nd, digit_const_bytes(*c->h, level), batch);
+}
+// Whether the digits of `members` polynomials that serve one rotation each go through ks_rows (its comment has the times on both sides)
+bool one_use(const hb_ctx *c, const PlanDims &d, int members) { return c->logn == 16 && c->tb.t16.pm && d.nd <= 4 && d.nd >= (members == 1 ? 3 : 2); }
 // Hybrid key switch of polynomial a (NTT form, `n` limbs, per-batch stride a_outer) with key `key`:
 //   out[b][p][l] = ModDown(sum_dg perm_g(lift_dg(a)) (.) key_dg)[p][l] + add_p[b][l] o perm_g
 // Phase 1 of a key switch (shared by every rotation of the same polynomial -- "hoisting"):
@@ -466,20 +477,19 @@ void ks_decompose(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch,
     const PlanDims d = plan_dims(c, level);
     const int N = c->N, n = d.n;
     const unsigned gx1 = (unsigned)((N + 255) / 256); // base-conversion kernels keep one coefficient per thread
-    Tmp acoef(c, (size_t)batch * n);
     if (c->logn == 16) {
-        inv_rows(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level));
-        launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.dt_count / d.nd, digit_const_bytes(*c->h, level), batch);
+        ks_lift(c, a, a_outer, level, batch, dt);
         fwd_rows(c, dt, (size_t)d.dt_count * N, batch * d.dt_count, d.dtmap);
         return;
     }
+    Tmp acoef(c, (size_t)batch * n);
     ntt(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level), true);
     LAUNCH(c), k_modup<<<dim3(gx1, d.nd, batch), 256, 0, c->st>>>(dt, acoef.p, pl, c->pc, N);
     ntt_inplace(c, dt, batch * d.dt_count, d.dtmap, false);
 }
 // ModDown of acc [batch*2][ne][N] into out: conversion of the special limbs, forward transform, final combination
-// (`total` members; addends per group of sl, `batch` members each)
-void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, size_t out_outer, const SwitchList &sl, int batch, size_t add_outer) {
+// (`total` members; addends per group of sl, `batch` members each).  half: the special limbs come behind their inverse row pass (2^16 rings)
+void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, size_t out_outer, const SwitchList &sl, int batch, size_t add_outer, bool half = false) {
     const KsPlan *pl = get_plan(c, level);
     const PlanDims d = plan_dims(c, level);
     const int N = c->N, n = d.n, ne = d.ne, K = d.K;
@@ -488,7 +498,7 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, siz
     if (c->logn == 16) { // the special limbs are transformed in place
         const ConvPlan *cv = get_conv_plans(c, level);
         u64 *sp = acc + (size_t)n * N;
-        inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, total * 2 * K, pm);
+        if (!half) inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, total * 2 * K, pm);
         launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, n, conv_const_bytes(K, n), total * 2);
         const RowsFin f{acc, (size_t)ne * N, out, out_outer, 2, batch, add_outer};
         LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, total * 2, f, c->p_inv_scale, sl, c->pc, c->tb.t16));
@@ -503,6 +513,18 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, siz
     LAUNCH(c), k_moddown_fin<<<dim3(gx, n, total * 2), 256, 0, c->st>>>(out, out_outer, acc, tbuf, sl, batch, add_outer, pl, c->pc, c->logn, N);
     CK(cudaGetLastError());
 }
+void launch_ks_rows(hb_ctx *c, u64 *acc, const SwitchList &sl, int batch, size_t a_outer, const KsPlan *pl, const PlanDims &d) {
+    const int m = batch >= 4 ? 2 : 1;
+    auto go = [&](auto *kernel) {
+        launch(c, kernel, dim3(256 / kKsRows, (unsigned)(sl.count * ((batch + m - 1) / m)), (unsigned)d.ne), 16 * kKsRows * d.nd * m, ks_rows_smem(d.nd, m), acc, sl, batch, a_outer, c->nprimes,
+               pl, c->pc, c->tb.t16);
+    };
+    switch (d.nd) {
+    case 2: go(m == 1 ? ks_rows<2, 1> : ks_rows<2, 2>); break;
+    case 3: go(m == 1 ? ks_rows<3, 1> : ks_rows<3, 2>); break;
+    default: go(m == 1 ? ks_rows<4, 1> : ks_rows<4, 2>); break;
+    }
+}
 // Members that one CTA of a key-stationary kernel walks over: as many as leave about eight CTAs per SM
 int members_per_cta(int batch, int ctas_per_chunk) {
     const int chunks = std::max(1, std::min(batch, (8 * 148 + ctas_per_chunk - 1) / ctas_per_chunk));
@@ -510,11 +532,17 @@ int members_per_cta(int batch, int ctas_per_chunk) {
 }
 // Phase 2: inner products of the (permuted) digits with the keys over Q_level u P, then ModDown, for every group of `sl`:
 //   out[ob][p][l] = ModDown(sum_dg perm_g(digit_dg) (.) key_dg)[p][l] + add_p[b][l] o perm_g,   ob = group * batch + b
-void ks_apply(hb_ctx *c, const SwitchList &sl, size_t a_outer, int level, int batch, u64 *out, size_t out_outer, size_t add_outer) {
+// half: the digits come from ks_lift
+void ks_apply(hb_ctx *c, const SwitchList &sl, size_t a_outer, int level, int batch, u64 *out, size_t out_outer, size_t add_outer, bool half = false) {
     const KsPlan *pl = get_plan(c, level);
     const PlanDims d = plan_dims(c, level);
     const int N = c->N, n = d.n, ne = d.ne, total = sl.count * batch;
     Tmp acc(c, (size_t)total * 2 * ne), t(c, (size_t)total * 2 * n);
+    if (half) {
+        launch_ks_rows(c, acc.p, sl, batch, a_outer, pl, d);
+        moddown(c, acc.p, t.p, level, total, out, out_outer, sl, batch, add_outer, true);
+        return;
+    }
     // Many members and up to four digits: one coefficient per thread, four CTAs per SM (256 members at level 8 1620 -> 1471 us, 42
     // members 513 -> 492).  Few members: two coefficients, whose loads cover the latency of a short walk (two digits of two
     // members 40 us, with one coefficient 51).  The line between them matters little: hoisted rotations (this kernel and ModDown), one /
@@ -542,11 +570,12 @@ void keyswitch(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch, co
                size_t add_outer) {
     const PlanDims d = plan_dims(c, level);
     Tmp dt(c, (size_t)batch * d.dt_count);
-    ks_decompose(c, a, a_outer, level, batch, dt.p);
+    const bool half = one_use(c, d, batch);
+    (half ? ks_lift : ks_decompose)(c, a, a_outer, level, batch, dt.p);
     SwitchList sl{};
     sl.count = 1;
     sl.s[0] = SwitchGroup{a, dt.p, key.d, {add0, add1}, g, 0u};
-    ks_apply(c, sl, a_outer, level, batch, out, out_outer, add_outer);
+    ks_apply(c, sl, a_outer, level, batch, out, out_outer, add_outer, half);
 }
 
 // Galois elements of the row shifts k * row_step, k < copies, kept on the device per (copies, row_step): the fused
@@ -1669,10 +1698,12 @@ int hb_decompose(hb_ctx *c, const hb_ct *a, hb_digits **out) {
     });
 }
 void hb_digits_free(hb_digits *h) { if (h) { h->ctx->pool.put(h->d); delete h; } }
-// rotations of `groups` member groups of x (group k = members k * batch ... ; shared: every group is the whole of x) by their own steps
+// rotations of `groups` member groups of x (group k = members k * batch ... ; shared: every group is the whole of x, and dt its decomposition; otherwise
+// dt comes from ks_lift where one_use says so) by their own steps
 static hb_ct *rotate_groups(hb_ctx *c, const hb_ct *x, const u64 *dt, bool shared, const int64_t *steps, int groups) {
     const int N = c->N, level = x->level, n = level + 1, batch = shared ? x->batch : x->batch / groups;
-    const size_t ct_outer = (size_t)2 * n * N, dt_count = (size_t)plan_dims(c, level).dt_count;
+    const PlanDims d = plan_dims(c, level);
+    const size_t ct_outer = (size_t)2 * n * N, dt_count = (size_t)d.dt_count;
     hb_ct *r = new_ct(c, level, 2, groups * batch, x->spow);
     try {
         for (int k0 = 0; k0 < groups;) { // runs of up to 16 rotated groups; an unrotated group is a copy
@@ -1686,7 +1717,7 @@ static hb_ct *rotate_groups(hb_ctx *c, const hb_ct *x, const u64 *dt, bool share
                 sl.s[sl.count++] = SwitchGroup{a + (size_t)n * N, dt + first * dt_count * N, galois_key(c, g).d, {a, nullptr}, (u32)g, 0u};
             }
             ALG(c, (size_t)sl.count * ((size_t)batch * (4 * n + dt_count) + key_limbs(c, level)));
-            if (sl.count) ks_apply(c, sl, ct_outer, level, batch, r->d + (size_t)k0 * batch * ct_outer, ct_outer, ct_outer);
+            if (sl.count) ks_apply(c, sl, ct_outer, level, batch, r->d + (size_t)k0 * batch * ct_outer, ct_outer, ct_outer, !shared && one_use(c, d, x->batch));
             if (k < groups && sl.count < kMaxSwitchGroups) {
                 CK(cudaMemcpyAsync(r->d + (size_t)k * batch * ct_outer, x->d + (shared ? 0 : (size_t)k * batch * ct_outer), (size_t)batch * ct_outer * 8, cudaMemcpyDeviceToDevice, c->st));
                 ++k;
@@ -1712,7 +1743,7 @@ int hb_rotate_grouped(hb_ctx *c, const hb_ct *x, const int64_t *steps, int group
         if (x->np != 2 || x->batch % groups) fail(HB_E_SHAPE, "rotate: the batch does not split into that many groups");
         const PlanDims d = plan_dims(c, x->level);
         Tmp dt(c, (size_t)x->batch * d.dt_count);
-        ks_decompose(c, x->d + (size_t)d.n * c->N, (size_t)2 * d.n * c->N, x->level, x->batch, dt.p);
+        (one_use(c, d, x->batch) ? ks_lift : ks_decompose)(c, x->d + (size_t)d.n * c->N, (size_t)2 * d.n * c->N, x->level, x->batch, dt.p);
         *out = rotate_groups(c, x, dt.p, false, steps, groups);
     });
 }
