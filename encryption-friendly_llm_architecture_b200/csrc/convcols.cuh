@@ -47,6 +47,9 @@ struct ConvPlan {
     //   others, one word each: below 2^44 the 26-bit pieces of C and of C * 2^30; long targets the 30-bit pieces of C, their sum, 0, or (kPieceSources)
     //               the pieces of 29 and 31 bits of C and of C * 2^30
     uint4 k[conv_const_bytes(8, kMaxPrimes) / 16];
+    // conv_mma (up to four sources, primes of LongPm): the target at position p of `order` has the 512 bytes from 32 p on, in them [half of the rows][block of
+    // sixteen k][byte j][k]: byte j of C_s * 2^(8 i) modulo the target, k = 8 s + i
+    uint4 bytes[kMaxPrimes * 32];
 };
 static_assert(conv_const_bytes(kFpSources, kMaxPrimes) <= conv_const_bytes(8, kMaxPrimes), "room for the longer constants");
 

@@ -7,6 +7,7 @@
 #include "kernels.cuh"
 #include "ntt.cuh"
 #include "convcols.cuh"
+#include "convmma.cuh"
 #include "ksrows.cuh"
 #include "embed.cuh"
 #include "host_threads.hpp"
@@ -301,6 +302,20 @@ void fill_conv(const HostCtx &h, bool pm, ConvPlan &p, const std::vector<int> &s
             }
     }
     std::stable_sort(p.order, p.order + p.nt, [&](int x, int y) { return (h.q[p.dst_prime[x]] >> 44) && !(h.q[p.dst_prime[y]] >> 44); });
+    if (!pm || src.size() > 4) return;
+    unsigned char *bytes = reinterpret_cast<unsigned char *>(p.bytes);
+    for (int pos = 0; pos < p.nt; ++pos) {
+        const int prime = p.dst_prime[p.order[pos]];
+        const u64 q = h.q[prime];
+        for (int half = 0; half < 2; ++half)
+            for (size_t s = 0; s < src.size(); ++s) {
+                u64 v = half ? hbhost::mulmod(hat(s, q), half_turn(prime), q) : hat(s, q);
+                for (size_t i = 0; i < 8; ++i, v = hbhost::mulmod(v, 256 % q, q)) {
+                    const size_t k = 8 * s + i;
+                    for (size_t j = 0; j < 8; ++j) bytes[(size_t)pos * 512 + (size_t)half * 256 + k / 16 * 128 + j * 16 + k % 16] = (unsigned char)(v >> (8 * j));
+                }
+            }
+    }
 }
 const ConvPlan *get_conv_plans(hb_ctx *c, int level) {
     auto it = c->conv_plans.find(level);
@@ -355,6 +370,12 @@ size_t digit_const_bytes(const HostCtx &h, int level) {
     }
     return most;
 }
+// and the most targets of one of them
+int digit_targets(const HostCtx &h, int level) {
+    int most = 0;
+    for (int dg = 0; dg <= h.digit_of(level); ++dg) most = std::max(most, level + 1 + h.K - (h.digit_hi(dg, level + 1) - h.digit_lo(dg)));
+    return most;
+}
 void conv_opt_in(hb_ctx *c) {
     if (c->smem_opt_in_conv) return;
     auto allow = [](auto *kernel, size_t bytes) { CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); };
@@ -366,6 +387,7 @@ void conv_opt_in(hb_ctx *c) {
         allow(lift_cols<8, 2, 2, LONG>, strip_bytes(8, 3)); allow(lift_cols<8, 1, 4, LONG>, strip_bytes(8, 2)); allow(lift_cols<4, 4, 2, LONG>, strip_bytes(4, 5)); allow(lift_cols<4, 8, 1, LONG>, strip_bytes(4, 9));
     };
     if (c->tb.t16.pm) all(LongPm{}); else all(LongShoup{});
+    allow(conv_mma<2, 2>, conv_mma_smem(2, kMaxPrimes)); allow(conv_mma<4, 1>, conv_mma_smem(4, kMaxPrimes));
     c->smem_opt_in_conv = true;
 }
 // Strip width and groups of a launch over `units` (polynomial, conversion) pairs.  At most two units: narrow strips and many groups, so that
@@ -383,8 +405,22 @@ void conv_opt_in(hb_ctx *c) {
 // division (decompositions of level 2, 8 units 56 / 51; divisions of level 3, 8 units 84 / 76, of level 7, 8 units 134 / 131, 14 units 216 / 219).
 // More than four sources, (4 x 4) / (8 x 4): divisions of seven sources 32 units 425 / 434, 40 units 520 / 536; of eight 48 units 1120 / 1140;
 // a digit of seven limbs 40 units 425 / 411.
-enum StripShape { kStrip8x1, kStrip8x2, kStrip8x4, kStrip4x4, kStrip4x8 };
-StripShape conv_shape(int units, int max_ns, int targets) {
+//
+// mma: up to four sources, primes of LongPm, and two CTAs find room with their constants (conv_mma).  Its strips have eight columns, so few units fill the GPU
+// badly: two groups and two CTAs per SM hold nine units at once, four groups and one CTA four and a half.  Calls, us, the strips below / conv_mma
+// with two groups / with four: decompositions of level 6 (two digits), 4 units 39 / 47 / 35, 6 units 53 / 52 / 54, 8 units 65 / 59 / 61, 24 units 161 / 154 /
+// 172, 96 units 541 / 526 / 579, of level 12, 4 units 51 / 68 / 48, 48 units 436 / 420 / 451; masked sums with their divisions of level 6, 4 units 58 / 67 / 57, 8
+// units 97 / 91 / 94, 12 units 132 / 130 / 129, 16 units 162 / 161 / 164, 20 units 198 / 201 / 201, 96 units 803 / 780 / 836, of level 8, 20 units
+// 310 / 304 / 312, 96 units 1313 / 1288 / 1336.  Little is left to convert with fewer sources or targets: divisions of level 1, 96 units 434 / 444 / 483;
+// hoisted rotations with their ModDown of level 4, 96 units 708 / 712 / 765, of level 8 1068 / 1059 / 1133.
+constexpr size_t kTwoCtas = 228 * 1024 / 2 - 2048; // dynamic shared memory of a CTA when an SM takes two
+enum StripShape { kStrip8x1, kStrip8x2, kStrip8x4, kStrip4x4, kStrip4x8, kMma2, kMma4 };
+StripShape conv_shape(int units, int max_ns, int targets, bool mma) {
+    if (mma) {
+        if (units == 3 || units == 4 || units == 12) return kMma4;
+        if (units >= 7 && units <= 9) return kMma2;
+        if ((units == 17 || units == 18 || units >= 24) && targets >= (max_ns == 4 ? 3 : 6)) return kMma2;
+    }
     if (units <= 2) return kStrip4x8;
     if (units <= 12) return kStrip4x4;
     if (max_ns > 4) return units <= 32 ? kStrip4x4 : kStrip8x4;
@@ -396,15 +432,20 @@ StripShape conv_shape(int units, int max_ns, int targets) {
 // 963 / 929 / 912, 96 polynomials 982 / 942 / 926; level 4, 16 polynomials 107 / 102 / 100, 96 polynomials 567 / 533 / 521.  The line lies where the
 // gain was seen first; one group is ahead by 1 to 2 % from 32 polynomials on.
 StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : units < 96 ? kStrip8x2 : kStrip8x1; }
-// `plans` conversions (the largest with max_ns sources, `targets` each on average, at most `consts` bytes of constants) of `instances` polynomials in one launch
-void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int targets, size_t consts, int instances) {
+// `plans` conversions (the largest with max_ns sources, `targets` each on average, `most` at most, at most `consts` bytes of constants) of `instances` polynomials in one launch
+void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int targets, int most, size_t consts, int instances) {
     conv_opt_in(c);
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
         launch(c, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
     };
+    auto products = [&](auto *kernel, int groups) {
+        launch(c, kernel, dim3(32, count, instances), 128 * groups, conv_mma_smem(groups, most), src, so, dst, dof, plans, c->pc, c->tb.t16, c->dev_err);
+    };
     auto shapes = [&](auto arithmetic) {
         using LONG = decltype(arithmetic);
-        switch (conv_shape(instances * count, max_ns, targets)) {
+        switch (conv_shape(instances * count, max_ns, targets, c->tb.t16.pm && max_ns <= 4 && conv_mma_smem(2, most) <= kTwoCtas)) {
+        case kMma2: products(conv_mma<2, 2>, 2); break;
+        case kMma4: products(conv_mma<4, 1>, 4); break;
         case kStrip8x2: go(conv_cols<8, 2, 2, 4, LONG>, 8, 2, strip_bytes(8, max_ns + 2) + consts); break;
         case kStrip8x4: go(conv_cols<8, 4, 1, 8, LONG>, 8, 4, strip_bytes(8, max_ns + 4) + consts); break;
         case kStrip4x4: go(max_ns <= 4 ? conv_cols<4, 4, 2, 4, LONG> : conv_cols<4, 4, 2, 8, LONG>, 4, 4, strip_bytes(4, max_ns + 4) + consts); break;
@@ -464,7 +505,7 @@ void ks_lift(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch, u64 
     const int N = c->N, n = d.n;
     Tmp acoef(c, (size_t)batch * n);
     inv_rows(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level));
-    launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.dt_count / d.nd, digit_const_bytes(*c->h, level), batch);
+    launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.dt_count / d.nd, digit_targets(*c->h, level), digit_const_bytes(*c->h, level), batch);
 }
 // Whether the digits of `members` polynomials that serve one rotation each go through ks_rows (its comment has the times on both sides)
 bool one_use(const hb_ctx *c, const PlanDims &d, int members) { return c->logn == 16 && c->tb.t16.pm && d.nd <= 4 && d.nd >= (members == 1 ? 3 : 2); }
@@ -499,7 +540,7 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, siz
         const ConvPlan *cv = get_conv_plans(c, level);
         u64 *sp = acc + (size_t)n * N;
         if (!half) inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, total * 2 * K, pm);
-        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, n, conv_const_bytes(K, n), total * 2);
+        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, n, n, conv_const_bytes(K, n), total * 2);
         const RowsFin f{acc, (size_t)ne * N, out, out_outer, 2, batch, add_outer};
         LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, total * 2, f, c->p_inv_scale, sl, c->pc, c->tb.t16));
         CK(cudaGetLastError());
@@ -689,7 +730,7 @@ hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch, hb_ct *dst = null
         if (c->logn == 16) {
             const ConvPlan *cv = get_conv_plans(c, level);
             inv_rows(c, src, (size_t)ne * N, src, (size_t)ne * N, batch * 2 * ns, sm);
-            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, level, conv_const_bytes(ns, level), batch * 2);
+            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, level, level, conv_const_bytes(ns, level), batch * 2);
             const RowsFin f{E, (size_t)ne * N, out, (size_t)2 * level * N, 2, 1, 0};
             LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], NoAddends{}, c->pc, c->tb.t16));
             CK(cudaGetLastError());
