@@ -14,8 +14,8 @@
 // takes the sixteen rows that agree in their low four bits, whose images are runs of sixteen coefficients.
 // Bound by latency (16 CTAs of 128 threads a member): for eight members 7 and 14 us to encode, 40 and 35 us to decode, where the
 // host cores took 2.0 and 1.8 ms a member for the same transforms and 2.8 and 1.4 ms for sampling and CRT lift.  Thirteen messages
-// of two tiles from host memory to ciphertexts 7.3 -> 0.85 ms, thirteen ciphertexts to host memory 5.5 -> 0.80 ms, each pass through the Python
-// call on other buffers; the library call on the same buffers again takes 0.60 and 0.57.  The copies are most of all of these.
+// of two tiles from host memory to ciphertexts 7.3 -> 0.82 -> 0.66 ms (0.82 before uniform parts and errors were drawn ahead of the messages), thirteen
+// ciphertexts to host memory 5.5 -> 0.80 ms, each pass through the Python call on other buffers.  The copies are most of all of these.
 #pragma once
 #include "modarith.cuh"
 #include "kernels.cuh"
@@ -268,9 +268,24 @@ __device__ __forceinline__ void chacha_block(const ChaChaKey &key, u32 domain, u
 struct StreamIds { ChaChaKey key; u32 domain; const u64 *ids; u64 first; };
 __device__ __forceinline__ u64 stream_id(const StreamIds &s, int b) { return s.ids ? s.ids[b] : s.first + (u64)b; }
 
+// eight values of a discrete Gaussian from block t of a stream: magnitude = number of the `cdt_n` increasing table entries that are <= the upper 63 bits of
+// the word, sign from its lowest bit
+__device__ __forceinline__ void gauss8(int (&e)[8], const StreamIds &s, u64 id, int t, const u64 *__restrict__ cdt, int cdt_n) {
+    u32 o[16];
+    chacha_block(s.key, s.domain, id, (u32)t, o);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const u64 r = (u64)o[2 * k] | ((u64)o[2 * k + 1] << 32), u = r >> 1;
+        int lo = 0, hi = cdt_n; // entries [0, lo) are <= u, entries [hi, n) above
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (__ldg(cdt + mid) <= u) lo = mid + 1; else hi = mid;
+        }
+        e[k] = (r & 1) ? -lo : lo;
+    }
+}
 // Residues of integer polynomials: out[b][l][i] = (coef[b][i] + error[b][i]) mod prime l, coefficient form.  Either part may be missing.
-// The error is a discrete Gaussian: magnitude = number of the `cdt_n` increasing table entries that are <= the upper 63 bits of the
-// word, sign from its lowest bit; word i of the member's stream.  A thread makes the eight coefficients of one ChaCha block
+// The error is a discrete Gaussian, from word i of the member's stream.  A thread makes the eight coefficients of one ChaCha block
 // for every gridDim.z-th limb: for all limbs where it makes an error, for one otherwise (the limbs one after the other / side by side: key
 // generation, which reduces the secret, 112 / 101 us, 52 / 40 at 2^10 points; one real message at level 12 to a plaintext 92 / 80).
 // grid = (ceil(N/8/128), count, 1 or limbs)
@@ -281,20 +296,7 @@ __global__ void __launch_bounds__(128) k_residues(u64 *out, const i64 *coef, con
     pdl_wait();
     if (t * 8 >= N) return;
     int e[8];
-    if constexpr (ERR) {
-        u32 o[16];
-        chacha_block(ids.key, ids.domain, stream_id(ids, b), (u32)t, o);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const u64 r = (u64)o[2 * k] | ((u64)o[2 * k + 1] << 32), u = r >> 1;
-            int lo = 0, hi = cdt_n; // entries [0, lo) are <= u, entries [hi, n) above
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (__ldg(cdt + mid) <= u) lo = mid + 1; else hi = mid;
-            }
-            e[k] = (r & 1) ? -lo : lo;
-        }
-    }
+    if constexpr (ERR) gauss8(e, ids, stream_id(ids, b), t, cdt, cdt_n);
     i64 m[8];
     if constexpr (MSG) {
         const longlong2 *p = reinterpret_cast<const longlong2 *>(coef + (size_t)b * N) + t * 4;
@@ -330,6 +332,51 @@ __device__ __forceinline__ void load4(u64 (&v)[4], const u64 *p) {
 __device__ __forceinline__ void store4(u64 *p, const u64 (&v)[4]) {
     reinterpret_cast<ulonglong2 *>(p)[0] = make_ulonglong2(v[0], v[1]);
     reinterpret_cast<ulonglong2 *>(p)[1] = make_ulonglong2(v[2], v[3]);
+}
+// What an encryption draws, ahead of the messages (2^16 rings; sampling depends on none of them and so runs while the first ones are on their way):
+// noise[b][i] = coefficient i of the member's error polynomial, below 128 in magnitude.  grid = (N/8/128, count)
+__global__ void __launch_bounds__(128) k_noise(signed char *noise, const __grid_constant__ StreamIds ids, const u64 *__restrict__ cdt, int cdt_n, int N) {
+    const int t = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
+    pdl_wait();
+    int e[8];
+    gauss8(e, ids, stream_id(ids, b), t, cdt, cdt_n);
+    u64 w = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) w |= (u64)(unsigned char)e[k] << (8 * k);
+    reinterpret_cast<u64 *>(noise + (size_t)b * N)[t] = w;
+}
+// -(coef[b][i] + noise[b][i]) modulo prime l, coefficient form: the negative, so that the last step of a division (x - t) finishes an encryption.  A
+// thread has four coefficients of one limb.  grid = (N/4/256, limbs, count)
+__global__ void __launch_bounds__(256) k_noisy_residues(u64 *out, const i64 *coef, const signed char *noise, const PrimeConst *__restrict__ pc, int N) {
+    const int t = blockIdx.x * 256 + threadIdx.x, l = blockIdx.y, b = blockIdx.z;
+    const PrimeConst m = pc[l];
+    pdl_wait();
+    const longlong2 *p = reinterpret_cast<const longlong2 *>(coef + (size_t)b * N) + t * 2;
+    const longlong2 p0 = p[0], p1 = p[1];
+    const char4 e4 = reinterpret_cast<const char4 *>(noise + (size_t)b * N)[t];
+    const i64 v[4] = {p0.x, p0.y, p1.x, p1.y};
+    const int e[4] = {e4.x, e4.y, e4.z, e4.w};
+    u64 r[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const u64 s = add_mod(reduce_i64_any(v[k], m), e[k] < 0 ? m.q - (u64)-e[k] : (u64)e[k], m.q);
+        r[k] = s ? m.q - s : 0;
+    }
+    store4(out + ((size_t)b * gridDim.y + l) * N + t * 4, r);
+}
+// ct [count][2][n][N]: a uniform (second polynomial) and -a s (first one).  One thread per ChaCha block of four coefficients.  grid = (N/4/256, n, count)
+__global__ void __launch_bounds__(256) k_uniform(u64 *ct, const u64 *__restrict__ s, const __grid_constant__ StreamIds ids, const PrimeConst *__restrict__ pc, int N) {
+    const int t = blockIdx.x * 256 + threadIdx.x, l = blockIdx.y, n = gridDim.y, b = blockIdx.z;
+    const PrimeConst m = pc[l];
+    u64 a[4], sv[4], r[4];
+    load4(sv, s + (size_t)l * N + t * 4);
+    pdl_wait();
+    uniform4(a, ids, stream_id(ids, b), l, t, m, N);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { const u64 p = mul_mod_any(a[k], sv[k], m); r[k] = p ? m.q - p : 0; }
+    u64 *o = ct + ((size_t)b * 2 * n + l) * N + t * 4;
+    store4(o, r);
+    store4(o + (size_t)n * N, a);
 }
 // Ciphertexts ct [count][2][n][N]: a uniform, b = e - a s (+ msg), e [count][n][N] (message included, or msg [n][N] apart), all NTT form.
 // One thread per ChaCha block of four coefficients; the generator's additions, exclusive ors and rotations bound it.  grid = (ceil(N/4/256), n, count)

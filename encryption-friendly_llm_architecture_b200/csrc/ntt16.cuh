@@ -607,6 +607,11 @@ __global__ void __launch_bounds__(256, MINB) ntt16v2_inv_cols(const u64 *src, Li
     }
 }
 
+// the column pass of a forward transform alone
+inline cudaError_t launch_fwd_cols16(cudaStream_t st, u64 *d, size_t outer, int count, const LimbMap &map, const PrimeConst *pc, const Ntt16Tables &tb) {
+    auto go = [&](auto *kernel) { return launch_pdl(st, kernel, dim3(16, count), 256, 0, d, LimbAddr16{outer}, d, LimbAddr16{outer}, map, pc, tb); };
+    return tb.pm ? go(ntt16v2_fwd_cols<4, LongPm>) : go(ntt16v2_fwd_cols<4, LongShoup>);
+}
 // Launch a batched transform of `count` limb instances of 2^16 coefficients.  src == dst gives an in-place transform;
 // with distinct buffers `dst` also serves as the intermediate between the two passes.  MINB = CTAs per SM the kernels
 // are compiled for (register budget 65536 / (256 * MINB)); four measured fastest with the FP64 butterflies.

@@ -121,3 +121,28 @@ def test_tiles_that_are_refused_or_take_the_general_path(pkg, gpu_small):
     for m, t in zip(msgs, uneven):
         m[:64 * len(t)] = np.concatenate(t, axis=1).reshape(-1)
     assert np.array_equal(g.ct_export(g.encrypt_tiles(uneven, 2, [4, 5, 6])), g.ct_export(g.encrypt_many(msgs, 2, [4, 5, 6])))
+
+
+@pytest.mark.parametrize("count", [4, 16, 17, 33])
+def test_members_drawn_ahead_equal_single_encryptions(gpu_full, count):
+    """Uniform parts and errors are drawn for up to sixteen members before their messages; messages that saturate and that vanish among them."""
+    g = gpu_full
+    msgs = _messages(np.random.default_rng(count), count, g.slots, True)
+    msgs[0] *= 1e30
+    msgs[-1] *= 1e-300
+    nonces = [2**64 - 1 - 3 * k for k in range(count)]
+    got = g.ct_export(g.encrypt_many(msgs, 2, nonces))
+    for k in range(count):
+        assert np.array_equal(got[k:k + 1], g.ct_export(g.encrypt(g.encode(msgs[k], 2), nonces[k]))), f"member {k}"
+
+
+@pytest.mark.parametrize("sigma", [9.7, 9.8])
+def test_errors_on_either_side_of_a_byte(pkg, sigma):
+    """A table of 127 magnitudes is drawn ahead into bytes, one of 128 is not."""
+    g = pkg.open_gpu(pkg.make_params(log_n=16, max_level=2, dnum=2, num_special=2, hamming_weight=64, sigma=sigma))
+    g.keygen()
+    msgs = _messages(np.random.default_rng(1), 2, g.slots, False)
+    got = g.ct_export(g.encrypt_many(msgs, 1, [5, 6]))
+    for k in range(2):
+        assert np.array_equal(got[k:k + 1], g.ct_export(g.encrypt(g.encode(msgs[k], 1), 5 + k))), f"member {k}"
+    g.close()
