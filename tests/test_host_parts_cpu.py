@@ -21,6 +21,10 @@ def test_threads_that_cannot_be_started_leave_their_share(tmp_path):
     _run(tmp_path, "host_threads", "-pthread")
 
 
+def test_pages_that_are_asked_for_keep_what_they_hold(tmp_path):
+    _run(tmp_path, "pages", "-pthread")
+
+
 def test_programs_on_the_cpp_headers_compile():
     """What a separately compiled program may call through HEMMer.hpp, calls that the library does not make itself among them."""
     for name in ("hemmer_snippet", "operands_after_error", "evaluator_calls"):
