@@ -497,6 +497,15 @@ PlanDims plan_dims(hb_ctx *c, int level) {
     return p;
 }
 
+DigitPlan digit_plan(const hb_ctx *c, const PlanDims &d) {
+    DigitPlan p{};
+    p.n = d.n; p.ne = d.ne; p.dt_count = d.dt_count;
+    int e = 0;
+    for (int j = 0; j < d.ne; ++j) p.prime[j] = (unsigned char)(j < d.n ? j : c->L + 1 + (j - d.n));
+    for (int dg = 0; dg < d.nd; ++dg)
+        for (int j = 0; j < d.ne; ++j) p.entry[dg][j] = j >= c->h->digit_lo(dg) && j < c->h->digit_hi(dg, d.n) ? (short)-1 : (short)e++;
+    return p;
+}
 size_t key_limbs(hb_ctx *c, int level) { const PlanDims d = plan_dims(c, level); return (size_t)2 * d.nd * d.ne; } // the part of a switching key one key switch reads
 
 // On 2^16 rings: the lifted digits before their forward row pass
@@ -592,7 +601,7 @@ void ks_apply(hb_ctx *c, const SwitchList &sl, size_t a_outer, int level, int ba
     const int el = batch >= 32 && d.nd <= 4 ? 1 : 2;
     const int per = members_per_cta(batch, N / (256 * el) * ne * sl.count), chunks = (batch + per - 1) / per;
     auto inner = [&](auto *kernel) {
-        launch(c, kernel, dim3((unsigned)(N / (256 * el)), sl.count * chunks, ne), 256, 0, acc.p, sl, batch, per, a_outer, c->nprimes, pl, c->pc, c->logn, N);
+        launch(c, kernel, dim3((unsigned)(N / (256 * el)), sl.count * chunks, ne), 256, 0, acc.p, sl, batch, per, a_outer, c->nprimes, digit_plan(c, d), c->pc, c->logn, N);
     };
     switch (d.nd) {
     case 1: inner(el == 1 ? k_ks_inner<1, 1> : k_ks_inner<1, 2>); break;
@@ -802,7 +811,7 @@ hb_ct *do_assemble_mk(hb_ctx *c, const hb_ct *a, const u64 *dt, const hb_mkey *c
     if (d.nd <= 2) {
         const int per = members_per_cta(batch, N / (256 * 1) * ne * groups), chunks = (batch + per - 1) / per;
         launch(c, d.nd == 1 ? k_ks_inner_mkr<1> : k_ks_inner_mkr<2>, dim3((unsigned)(N / (256 * 1)), (unsigned)(groups * chunks), (unsigned)ne), 256, 0, E.p, (const u64 *)a->d,
-                              (const u64 *)a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch, per, pl, c->pc, c->logn, N);
+                              (const u64 *)a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch, per, digit_plan(c, d), c->pc, c->logn, N);
     } else {
         launch(c, k_ks_inner_mk, dim3((unsigned)((N + 1023) / 1024), groups * batch, ne), 256, 0, E.p, (const u64 *)a->d, (const u64 *)a->d + (size_t)n * N, (size_t)2 * n * N, dt, mrl, batch, pl,
                               c->pc, c->logn, N);

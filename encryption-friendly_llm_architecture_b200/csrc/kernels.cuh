@@ -654,6 +654,10 @@ __global__ void k_modup(u64 *__restrict__ dt, const u64 *__restrict__ a_coef, co
     }
 }
 
+// What the inner products of many waves of CTAs need of a level's plan before their first loads, as an argument: read from memory it stood in front of them
+// in every CTA (wrapped copies of one member 185 -> 178 us a launch, inner products of fifteen rotations of one member 195 -> 189).  ks_rows, whose
+// launches are short, reads it from memory: arguments come through a cache that every launch finds cold (rotation of one ciphertext 113 -> 117 us).
+struct DigitPlan { int n, ne, dt_count; short entry[8][kMaxPrimes]; unsigned char prime[kMaxPrimes]; }; // as in KsPlan
 // Up to 16 groups of `batch` members, each group with its own key switch: operand (limbs of the switched polynomial in NTT form and
 // its lifted digits), key, Galois element (0: no automorphism) and addends (null: none).
 struct SwitchGroup { const u64 *a_ntt, *dt, *key, *add[2]; u32 g, pad; };
@@ -668,13 +672,13 @@ struct SwitchList { SwitchGroup s[kMaxSwitchGroups]; int count; };
 // 285 us at 5.3 TB/s (0.82 of a copy), 43 % of the issue slots.  Eight digits spill (160 bytes a thread), seven 32, fewer none.
 // grid = (N/(256*EL), groups * ceil(batch/per), ne); ND = digits in use
 template <int ND, int EL>
-__global__ void __launch_bounds__(256, EL == 1 ? 4 : ND <= 2 ? 3 : 2) k_ks_inner(u64 *acc, const __grid_constant__ SwitchList sl, int batch, int per, size_t a_outer, int key_primes, const KsPlan *__restrict__ pl,
+__global__ void __launch_bounds__(256, EL == 1 ? 4 : ND <= 2 ? 3 : 2) k_ks_inner(u64 *acc, const __grid_constant__ SwitchList sl, int batch, int per, size_t a_outer, int key_primes, const __grid_constant__ DigitPlan pl,
                                                                    const PrimeConst *__restrict__ pc, int logn, int N) {
     const int chunks = (batch + per - 1) / per, grp = blockIdx.y / chunks, b0 = (blockIdx.y % chunks) * per, b1 = min(batch, b0 + per);
     const int j = blockIdx.z; // limb-major block order
     const SwitchGroup &sg = sl.s[grp];
     const u32 g = sg.g;
-    const int pj = pl->ext_prime[j], ne = pl->ne;
+    const int pj = pl.prime[j], ne = pl.ne;
     const PrimeConst m = pc[pj];
     const u32 x0 = blockIdx.x * (256 * EL) + threadIdx.x;
     u32 src[EL];
@@ -684,8 +688,8 @@ __global__ void __launch_bounds__(256, EL == 1 ? 4 : ND <= 2 ? 3 : 2) k_ks_inner
     size_t stride[ND];
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
-        const int en = pl->dt_entry[d][j];
-        stride[d] = en < 0 ? a_outer : (size_t)pl->dt_count * N;
+        const int en = pl.entry[d][j];
+        stride[d] = en < 0 ? a_outer : (size_t)pl.dt_count * N;
         sp[d] = (en < 0 ? sg.a_ntt + (size_t)j * N : sg.dt + (size_t)en * N) + (size_t)b0 * stride[d];
     }
     const u64 *kbase = sg.key + (size_t)pj * N + x0;
@@ -1220,11 +1224,11 @@ __global__ void __launch_bounds__(256, 2) k_ks_inner_mk(u64 *E, const u64 *c0, c
 // 65 % of the issue slots and 52 % of the wide multiply-adds for 64 outputs (367 us), DRAM 3.1 TB/s; in a third of the cycles it waits for loads.
 // grid = (N/256, groups * ceil(batch/per), ne)
 template <int ND, int CNT>
-__device__ __forceinline__ void ks_inner_mkr_body(u64 *o, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const MaskedRot &mr, int b0, int b1, const KsPlan *__restrict__ pl,
+__device__ __forceinline__ void ks_inner_mkr_body(u64 *o, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const MaskedRot &mr, int b0, int b1, const DigitPlan &pl,
                                                   const PrimeConst &m, int j, u32 x0, int logn, int N) {
     constexpr int EL = 1;
-    const int ne = pl->ne;
-    const bool has_c0 = j < pl->n;
+    const int ne = pl.ne;
+    const bool has_c0 = j < pl.n;
     const size_t kpoly = (size_t)ne * N;
     u32 src[CNT][EL];
 #pragma unroll
@@ -1235,8 +1239,8 @@ __device__ __forceinline__ void ks_inner_mkr_body(u64 *o, const u64 *c0, const u
     size_t stride[ND];
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
-        const int en = pl->dt_entry[d][j];
-        stride[d] = en < 0 ? a_outer : (size_t)pl->dt_count * N;
+        const int en = pl.entry[d][j];
+        stride[d] = en < 0 ? a_outer : (size_t)pl.dt_count * N;
         sp[d] = (en < 0 ? a_ntt + (size_t)j * N : dt + (size_t)en * N) + (size_t)b0 * stride[d];
     }
     const u64 *cp = c0 + (size_t)b0 * a_outer + (size_t)j * N;
@@ -1309,13 +1313,13 @@ __device__ __forceinline__ void ks_inner_mkr_body(u64 *o, const u64 *c0, const u
 }
 template <int ND>
 __global__ void __launch_bounds__(256, 4) k_ks_inner_mkr(u64 *E, const u64 *c0, const u64 *a_ntt, size_t a_outer, const u64 *dt, const __grid_constant__ MaskedRotList mrl, int batch, int per,
-                                                         const KsPlan *__restrict__ pl, const PrimeConst *__restrict__ pc, int logn, int N) {
+                                                         const __grid_constant__ DigitPlan pl, const PrimeConst *__restrict__ pc, int logn, int N) {
     const int chunks = (batch + per - 1) / per, grp = blockIdx.y / chunks, b0 = (blockIdx.y % chunks) * per, b1 = min(batch, b0 + per);
     const int j = blockIdx.z; // limb-major block order: the digits of one limb stay in L2 across the copies
     const MaskedRot &mr = mrl.r[grp];
-    const PrimeConst m = pc[pl->ext_prime[j]];
+    const PrimeConst m = pc[pl.prime[j]];
     const u32 x0 = blockIdx.x * (256 * 1) + threadIdx.x;
-    u64 *o = E + (((size_t)(grp * batch + b0) * 2) * pl->ne + j) * N + x0;
+    u64 *o = E + (((size_t)(grp * batch + b0) * 2) * pl.ne + j) * N + x0;
     pdl_wait();
     if (mr.count == 1) ks_inner_mkr_body<ND, 1>(o, c0, a_ntt, a_outer, dt, mr, b0, b1, pl, m, j, x0, logn, N);
     else ks_inner_mkr_body<ND, 2>(o, c0, a_ntt, a_outer, dt, mr, b0, b1, pl, m, j, x0, logn, N);
