@@ -1355,7 +1355,9 @@ int hb_ctx_create(const hb_params *prm, int device, hb_ctx **out) {
             CK(cudaMemcpy(reinterpret_cast<char *>(c->tw) + t16_bytes, b8.data(), b8.size() * sizeof(double), cudaMemcpyHostToDevice));
             const ulonglong2 *t = reinterpret_cast<const ulonglong2 *>(c->tw);
             const double *tb8 = reinterpret_cast<const double *>(reinterpret_cast<const char *>(c->tw) + t16_bytes);
-            c->tb.t16 = Ntt16Tables{t, t + (size_t)np * Ntt16Layout::kEntries, tb8, tb8 + (size_t)np * kRowsB8, pm};
+            u32 below44 = 0;
+            for (int i = 0; i < np; ++i) below44 |= (u32)(c->h->q[i] < ((u64)1 << 44)) << i;
+            c->tb.t16 = Ntt16Tables{t, t + (size_t)np * Ntt16Layout::kEntries, tb8, tb8 + (size_t)np * kRowsB8, pm, below44};
         } else {
             CK(cudaMalloc(&c->tw, tw.size() * 8));
             CK(cudaMemcpy(c->tw, tw.data(), tw.size() * 8, cudaMemcpyHostToDevice));

@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(16 * kKsRows * ND * M, 1024 / (16 * kKsRows * 
     const u32 g = sg.g, i0 = blockIdx.x * kTile;
     const int pj = pl->ext_prime[j], ne = pl->ne;
     const PrimeConst m = pc[pj];
+    const bool small = tb.small(pj);
     const u64 *key = sg.key + (size_t)pj * kN16 + i0;
     const size_t kpoly = (size_t)key_primes * kN16;
     if (b0 == 0 && tid < 2 * ND) prefetch_l2(key + tid * kpoly, kTile * 8);
@@ -52,8 +53,8 @@ __global__ void __launch_bounds__(16 * kKsRows * ND * M, 1024 / (16 * kKsRows * 
         pdl_wait();
         if (en < 0) {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = key_word(p[e * 16], m.fp);
-        } else if (m.small) {
+            for (int e = 0; e < 16; ++e) smr[e * 17 + clo] = key_word(p[e * 16], small);
+        } else if (small) {
             const DsConst c = ds_const(m);
             double *smd = reinterpret_cast<double *>(smr);
             double v[16];
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(16 * kKsRows * ND * M, 1024 / (16 * kKsRows * 
 #pragma unroll
             for (int mb = 0; mb < M; ++mb) {
                 u64 r[2], *tile = tiles + mb * TM * kTileWords + w;
-                if (m.fp) {
+                if (small) {
                     const double qd = (double)m.q;
                     FpAcc s[2];
 #pragma unroll
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(16 * kKsRows * ND * M, 1024 / (16 * kKsRows * 
         if (b0 + q / 2 >= batch) break;
         u64 *tile = tiles + (q / 2 * TM + q % 2) * kTileWords, *smr = tile + (source(i0 + rl * 256) >> 8 & (R - 1)) * kRowStride;
         u64 *op = o + (size_t)q * ne * kN16 + rl * 256 + clo;
-        if (m.small) {
+        if (small) {
             const DsConst c = ds_const(m);
             double *smd = reinterpret_cast<double *>(smr);
             double v[16];

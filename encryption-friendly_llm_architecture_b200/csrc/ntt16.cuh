@@ -57,6 +57,8 @@ struct Ntt16Tables {
     // thread reads 15 twiddles nobody else uses (more bytes than the coefficients themselves)
     const double *fwdB8, *invB8;
     bool pm; // the constants of the primes of 45 bits and more are those of LongPm
+    u32 below44; // bit i: prime i is below 2^44.  An argument, so that a kernel knows its branch, and asks for its operands, before PrimeConst has come from memory
+    __device__ __forceinline__ bool small(int prime) const { return below44 >> prime & 1; }
 };
 constexpr int kRowsB8 = 256 * 15 * 16;
 
