@@ -874,6 +874,8 @@ void lift_last(hb_ctx *c, u64 *last, int sums, int groups, int nbp, int l, u64 *
     LAUNCH(c), k_lift_mod<<<c->egrid(total * l), 256, 0, c->st>>>(t, (const i64 *)S.p, l, c->pc, N);
     ntt_inplace(c, t, total * l, c->qmap(l - 1), false);
 }
+// Sums of products are held as a whole before they are rescaled up to this many limbs (8 GB on 2^16 rings), beyond limb by limb
+constexpr size_t kRawLimbs = 16384;
 // sum_j rescale(a_j (.) p_j)  (separate)  or  rescale(sum_j a_j (.) p_j); `sums` such sums of `count` terms each, sum k from the terms
 // k * count ..., one member group of the result per sum
 hb_ct *do_prod_rescale(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, int count, bool separate, int sums = 1) {
@@ -894,6 +896,12 @@ hb_ct *do_prod_rescale(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, 
     ALG(c, (size_t)count * sums * ((size_t)nbp * (l + 1) + (l + 1)) + (size_t)total * l);
     try {
         Tmp last(c, (size_t)groups * total), t(c, (size_t)total * l);
+        if (c->logn == 16 && !separate && (size_t)total * (l + 1) <= kRawLimbs) {
+            Tmp x(c, (size_t)total * (l + 1));
+            launch(c, k_prod_sums, dim3(gx, (unsigned)(total * (l + 1))), 256, 0, x.p, tl, l, nbp, c->pc, N);
+            rescale_core(c, x.p, r->d, l, a0->np, total, last.p, t.p);
+            return r;
+        }
         launch(c, k_last_prod, dim3(gx, total, groups), 256, 0, last.p, tl, separate ? 1 : 0, l, nbp, c->pc, N);
         lift_last(c, last.p, 1, groups, total, l, t.p);
         Scalars qi{};
@@ -946,16 +954,21 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
         // Up to ten polynomials, and for one or two parts, the masks are streamed once per pair of polynomials; otherwise they are kept.  Calls at
         // level 7, us, streamed / kept: sixteen terms and twelve parts, 4 polynomials 647 / 1220, 10 1505 / 1920, 12 1804 / 2090, 24 3526 / 3338; nine
         // terms and six parts, 10 818 / 832, 12 970 / 903; one term and one part, 12 149 / 269, 48 473 / 645; sixteen and two, 24 791 / 1063.
-        auto sums = [&](u64 *o, const u64 *tt) {
-            const unsigned limbs = (unsigned)(tt ? l : 1);
+        auto sums = [&](u64 *o, const u64 *tt, unsigned limbs) {
             auto few = [&](auto *kernel) { LAUNCH(c), kernel<<<dim3((unsigned)(N / 256 * ((nbp + 1) / 2)), limbs), 256, 0, c->st>>>(o, pt, tt, l, nbp, c->pc, N, qi); };
             if (nbp <= 10 || parts <= 2) few(count <= 2 ? k_prod_parts_few<2> : count <= 4 ? k_prod_parts_few<4> : count <= 8 ? k_prod_parts_few<8> : k_prod_parts_few<kMaxPartTerms>);
             else LAUNCH(c), k_prod_parts<G><<<dim3(pg, (unsigned)(N / kPartLanes), limbs), 512, part_smem(G, count), c->st>>>(o, pt, tt, l, nbp, c->pc, N, qi, c->dev_err);
         };
+        if (c->logn == 16 && !separate && (size_t)gnbp * (l + 1) <= kRawLimbs) { // all limbs at once, and a rescale
+            Tmp x(c, (size_t)gnbp * (l + 1));
+            sums(x.p, nullptr, (unsigned)(l + 1));
+            rescale_core(c, x.p, r->d, l, a0->np, gnbp, last.p, t.p);
+            return r;
+        }
         if (separate) launch(c, k_last_prod_parts, dim3(c->gx(), nbp, parts * count), 256, 0, last.p, pt, l, nbp, c->pc, N);
-        else sums(last.p, nullptr);
+        else sums(last.p, nullptr, 1);
         lift_last(c, last.p, parts, separate ? count : 1, nbp, l, t.p);
-        sums(r->d, t.p);
+        sums(r->d, t.p, (unsigned)l);
         CK(cudaGetLastError());
     } catch (...) { hb_ct_free(r); throw; }
     return r;

@@ -327,6 +327,40 @@ __global__ void k_prod_rescale_fin(u64 *out, const __grid_constant__ TermList tl
     for (int u = 0; u < kElems; ++u) op[u * blockDim.x] = mul_mod_any(sub_mod(v[u], tp[u * blockDim.x], m.q), qlinv.v[l], m);
 }
 
+// out[inst][l][x] = sum_j a_j[bp][l][x] * p_j[l][x], canonical, for all limbs up to `level`; instance k * nbp + bp, terms and block order as above.  On 2^16
+// rings the sums of a masked sum go from here through a rescale like any other ciphertext's: last limb to coefficients, lift, forward row pass that ends
+// in the division (k_last_prod and a k_prod_rescale_fin behind whole transforms: five launches instead of four, and the division's product on its own).
+// grid = (N/(256*kElems), instances * (level + 1))
+__global__ void __launch_bounds__(256) k_prod_sums(u64 *out, const __grid_constant__ TermList tl, int level, int nbp, const PrimeConst *__restrict__ pc, int N) {
+    const int total = gridDim.y / (level + 1), l = blockIdx.y / total, inst = blockIdx.y % total, bp = inst % nbp, first = inst / nbp * tl.count;
+    const PrimeConst m = pc[l];
+    pdl_wait();
+    const u32 x0 = blockIdx.x * (256 * kElems) + threadIdx.x;
+    const size_t ao = ((size_t)bp * (level + 1) + l) * N + x0, po = (size_t)l * N + x0;
+    u64 v[kElems];
+    auto sum = [&](auto &s, int room) {
+#pragma unroll
+        for (int u = 0; u < kElems; ++u) s[u].zero();
+#pragma unroll 2
+        for (int j = 0; j < tl.count; ++j) {
+            const u64 *a = tl.a[first + j] + ao, *p = tl.p[first + j] + po;
+            if (j && j % room == 0) {
+#pragma unroll
+                for (int u = 0; u < kElems; ++u) s[u].relax(m);
+            }
+#pragma unroll
+            for (int u = 0; u < kElems; ++u) s[u].product(a[u * 256], p[u * 256]);
+        }
+#pragma unroll
+        for (int u = 0; u < kElems; ++u) v[u] = s[u].canonical(m);
+    };
+    if (m.fp) { FpAcc s[kElems]; sum(s, m.q < (1ull << 42) ? 64 : 7); } // with what relax leaves: 128 products, eight (FpAcc, PieceAcc)
+    else { PieceAcc s[kElems]; sum(s, 7); }
+    u64 *op = out + ((size_t)inst * (level + 1) + l) * N + x0;
+#pragma unroll
+    for (int u = 0; u < kElems; ++u) op[u * 256] = v[u];
+}
+
 // Form of a factor that many products share (masks in shared memory, words of a masked key; nothing outside the kernels sees it): an integer-valued double for primes below 2^44, the two
 // 30-bit pieces in the halves of the word otherwise.
 __device__ __forceinline__ u64 key_word(u64 w, bool fp) { return fp ? (u64)__double_as_longlong(u52_to_double(w)) : ((w >> 30) << 32) | ((u32)w & 0x3FFFFFFFu); }
@@ -360,7 +394,7 @@ __global__ void k_last_prod_parts(u64 *last, const __grid_constant__ PartTerms p
 // from a table instead of branches and one instruction per wide multiply-add 3.7 ms.  Memory hardly shows any more (DRAM 16 %, half a
 // warp waiting for loads): four warps a scheduler issue in 57 % of the slots, between fixed latencies and their turns at the math pipes (FP64 45 % of
 // the time on a short limb, wide multiply-adds 37 % over all).
-// t == nullptr: raw sums of limb `level`, out[(g * nbp + bp) * N + x]                       grid = (ceil(parts/G), N/kPartLanes, 1)
+// t == nullptr: raw sums of the last `limbs` limbs up to `level`, out[((g * nbp + bp) * limbs + k) * N + x]   grid = (ceil(parts/G), N/kPartLanes, limbs)
 // else: out[((g * nbp + bp) * level + l) * N + x] = (sum - t[same]) * q_level^-1 mod q_l      grid = (ceil(parts/G), N/kPartLanes, level)
 // (parts first, so that the CTAs that read the same words run together)
 constexpr int kPartLanes = 128, kPartRing = 8;
@@ -376,7 +410,7 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
     u64 *ptile = reinterpret_cast<u64 *>(smem_raw) + kPartRing * kStage; // [count][G][kPartLanes]
     const u32 ring_at = smem_u32(ring);
     const int tid = threadIdx.x, lane = tid & (kPartLanes - 1), slot = tid / kPartLanes;
-    const int l = t ? (int)blockIdx.z : level, g0 = blockIdx.x * G;
+    const int l = (t ? 0 : level + 1 - (int)gridDim.z) + (int)blockIdx.z, g0 = blockIdx.x * G;
     const int gn = min(G, pt.parts - g0);
     const u32 x0 = blockIdx.y * kPartLanes;
     // What a member needs, in order: its terms a_j, then the words of t that its parts are subtracted from.  (address at member 0, bytes per member)
@@ -510,8 +544,8 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
 #pragma unroll
                 for (int g = 0; g < G; ++g) v[i][g] = s[i][g].finish(m);
         }
-        u64 *o = out + (t ? (size_t)g0 * t_part + (size_t)bp * t_member + first : ((size_t)g0 * nbp + bp) * N + x0) + lane;
-        const size_t o_part = t ? t_part : (size_t)nbp * N, o_member = t ? t_member : (size_t)N;
+        const size_t o_member = (size_t)gridDim.z * N, o_part = (size_t)nbp * o_member;
+        u64 *o = out + (size_t)g0 * o_part + (size_t)bp * o_member + (size_t)blockIdx.z * N + x0 + lane;
 #pragma unroll
         for (int g = 0; g < G; ++g, o += o_part)
             if (g < gn) {
@@ -528,12 +562,12 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
 // a_j of its coefficient in two polynomials and walks over the parts, with the masks of a part in flight together.  A launch for one two-tile
 // product 604 -> 215 us (2.5 TB/s of masks).  TERMS: the most terms there can be; all of them are multiplied, and what a call does not have is
 // zero.  With seventeen for every call, one term and eight parts of eight polynomials took 871 us at level 7 (kept masks 739);
-// with two 523.  grid = (N/256 * pairs of polynomials, 1 or level), arguments as above
+// with two 523.  grid = (N/256 * pairs of polynomials, limbs), arguments as above
 template <int TERMS>
 __global__ void __launch_bounds__(256, TERMS <= 4 ? 4 : TERMS <= 8 ? 3 : 2) k_prod_parts_few(u64 *__restrict__ out, const __grid_constant__ PartTerms pt, const u64 *__restrict__ t, int level, int nbp,
                                                                                             const PrimeConst *__restrict__ pc, int N, const __grid_constant__ Scalars qlinv) {
     const int pairs = (nbp + 1) / 2, bp = blockIdx.x % pairs * 2; // the pairs that read the same masks run together
-    const int l = t ? (int)blockIdx.y : level, count = pt.count, x = blockIdx.x / pairs * 256 + threadIdx.x;
+    const int limbs = gridDim.y, k = blockIdx.y, l = (t ? 0 : level + 1 - limbs) + k, count = pt.count, x = blockIdx.x / pairs * 256 + threadIdx.x;
     const bool both = bp + 1 < nbp;
     const PrimeConst m = pc[l];
     const u64 qli = t ? qlinv.v[l] : 0;
@@ -556,8 +590,8 @@ __global__ void __launch_bounds__(256, TERMS <= 4 ? 4 : TERMS <= 8 ? 3 : 2) k_pr
 #pragma unroll
             for (int j = 0; j < TERMS; ++j) {
                 if (j && j % 8 == 0 && eight) { s[0].relax(m.q_inv_f, qd); s[1].relax(m.q_inv_f, qd); }
-                const double k = u52_to_double(w[j]);
-                s[0].mac(__longlong_as_double((long long)a[0][j]), k); s[1].mac(__longlong_as_double((long long)a[1][j]), k);
+                const double wd = u52_to_double(w[j]);
+                s[0].mac(__longlong_as_double((long long)a[0][j]), wd); s[1].mac(__longlong_as_double((long long)a[1][j]), wd);
             }
             v[0] = s[0].finish(m.q_inv_f, qd); v[1] = s[1].finish(m.q_inv_f, qd);
         } else {
@@ -573,10 +607,8 @@ __global__ void __launch_bounds__(256, TERMS <= 4 ? 4 : TERMS <= 8 ? 3 : 2) k_pr
 #pragma unroll
         for (int i = 0; i < 2; ++i)
             if (i == 0 || both) {
-                if (t) {
-                    const size_t o = (((size_t)g * nbp + bp + i) * level + l) * N + x;
-                    out[o] = mul_mod_any(sub_mod(v[i], t[o], m.q), qli, m);
-                } else out[((size_t)g * nbp + bp + i) * N + x] = v[i];
+                const size_t o = (((size_t)g * nbp + bp + i) * limbs + k) * N + x;
+                out[o] = t ? mul_mod_any(sub_mod(v[i], t[o], m.q), qli, m) : v[i];
             }
     }
 }

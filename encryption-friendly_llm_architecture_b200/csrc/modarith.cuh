@@ -204,6 +204,10 @@ struct FpAcc {
         if (r < 0.0) r = __dadd_rn(r, qd);
         return mantissa52(__dadd_rn(r, kTwo52));
     }
+    // of residues, and with the constants of a prime: the names that PieceAcc has them under
+    __device__ __forceinline__ void product(u64 a, u64 w) { mac(u52_to_double(a), u52_to_double(w)); }
+    __device__ __forceinline__ void relax(const PrimeConst &m) { relax(m.q_inv_f, (double)m.q); }
+    __device__ __forceinline__ u64 canonical(const PrimeConst &m) const { return finish(m.q_inv_f, (double)m.q); }
 };
 
 // ---- sums of products modulo the primes of 45 to 60 bits ---------------------------------------------------------
@@ -263,6 +267,8 @@ template <bool SPLIT> struct PieceAccT {
         const u64 r = finish_wide(a0, am - a0 - a2, a2, m);
         return canon_q(r, m.q, FoldQ{m.fold_shift, (1u << m.fold_shift) - 1u, m.fold_d});
     }
+    __device__ __forceinline__ void product(u64 a, u64 w) { mac(a, w); }
+    __device__ __forceinline__ u64 canonical(const PrimeConst &m) const { return finish(m); }
 };
 using PieceAcc = PieceAccT<false>;
 

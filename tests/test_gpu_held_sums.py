@@ -61,3 +61,35 @@ def test_loops_of_the_full_ring(pkg):
                 _same(np.ascontiguousarray(got[k::3]), g.ct_export(op(a[k], b[k])), f"operation {n}, packed {pack}, member {k}")
     H.close()
     g.close()
+
+
+def _wide(g, batch):
+    """Five members over and over."""
+    few = _ct(g, 5, 90, level=1)
+    return g.batch_slice(g.batch_concat([few] * ((batch + 4) // 5)), 0, batch)
+
+
+@pytest.mark.parametrize("batch", [170, 171])
+def test_sums_on_either_side_of_what_is_held(pkg, gpu_full, batch):
+    """24 sums of one term at level 1: 16 320 limbs are rescaled as a whole, 16 416 limb by limb."""
+    g = gpu_full
+    x, mask = _wide(g, batch), g.encode(np.linspace(-1, 1, g.slots), 1)
+    got = _call(pkg, g, "sum_mul_pt_rescale_many", _ptrs([x] * 24), _ptrs([mask] * 24), C.c_int(1), C.c_int(24))
+    for k in (0, 3, batch - 1):
+        want = g.ct_export(g.mul_pt(g.batch_slice(x, k, 1), mask))
+        for s in (0, 23):
+            _same(g.ct_export(g.batch_slice(got, s * batch + k, 1)), want, f"sum {s}, member {k}")
+
+
+@pytest.mark.parametrize("batch", [240, 241])
+def test_part_sums_on_either_side_of_what_is_held(pkg, gpu_full, batch):
+    """Seventeen parts of two terms at level 1: 16 320 and 16 388 limbs."""
+    g = gpu_full
+    x, masks = _wide(g, batch), [g.encode(np.linspace(-1, k, g.slots), 1) for k in range(2)]
+    got = _call(pkg, g, "mul_pt_sum_parts", _ptrs([x, x]), _ptrs(masks * 17), C.c_int(2), C.c_int(17))
+    for k in (0, 3, batch - 1):
+        one = g.batch_slice(x, k, 1)
+        want = g.ct_export(_call(pkg, g, "sum_mul_pt_rescale", _ptrs([one, one]), _ptrs(masks), C.c_int(2)))
+        for part in (0, 16):
+            _same(g.ct_export(g.batch_slice(got, part * batch + k, 1)), want, f"part {part}, member {k}")
+    g._chk(g._fn("release_cached")(g.ctx))
