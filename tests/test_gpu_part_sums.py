@@ -46,6 +46,13 @@ def test_part_sums_on_either_side_of_the_term_counts_of_their_kernels(pkg, g, te
     _compare_part_sums(pkg, g, terms, parts, polys, batch, True)
 
 
+@pytest.mark.parametrize("terms,parts,polys,batch", [(17, 17, 1, 48), (17, 17, 1, 49), (16, 12, 2, 21), (16, 12, 2, 22), (9, 6, 1, 13), (9, 6, 1, 14), (8, 12, 2, 42), (8, 12, 1, 85), (5, 6, 1, 32),
+                                                     (5, 6, 1, 33), (2, 6, 1, 10), (2, 6, 3, 4), (4, 4, 2, 42), (4, 4, 1, 85), (1, 8, 1, 84), (17, 13, 1, 85), (1, 5, 1, 11)])
+def test_part_sums_on_either_side_of_the_line_between_the_kernels(pkg, g, terms, parts, polys, batch):
+    """Up to how many polynomials the masks are streamed, for full and part-filled kernels of terms and groups of parts."""
+    _compare_part_sums(pkg, g, terms, parts, polys, batch, True)
+
+
 def _compare_part_sums(pkg, g, terms, parts, polys, batch, top):
     rng = np.random.default_rng(terms * 100 + parts)
     xs = [_ct(g, polys, batch, 40 + j, top) for j in range(terms)]
