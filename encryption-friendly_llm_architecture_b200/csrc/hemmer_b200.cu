@@ -825,17 +825,21 @@ void check_same(const hb_ct *a, const hb_ct *b, const char *what) {
     if (a->np != b->np || a->batch != b->batch || a->spow != b->spow) fail(HB_E_SHAPE, std::string(what) + ": shape mismatch");
 }
 
+// the end of a rescale on 2^16 rings: (x - t) / q_l, t behind its forward column pass
+void rescale_rows(hb_ctx *c, const u64 *x, size_t x_outer, const u64 *t, u64 *out, int l, int np, int nbp) {
+    InvScale sc{};
+    for (int i = 0; i < l; ++i) scale_words(hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]), c->h->q[i], c->tb.t16.pm, sc.w[i], sc.c[i]);
+    const RowsFin f{x, x_outer, out, (size_t)np * l * c->N, np, 1, 0};
+    LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, t, (size_t)l * c->N, l, nbp, f, sc, NoAddends{}, c->pc, c->tb.t16));
+}
 // out[bp] = rescale of x[bp] (level + 1 limbs); scratch: nbp * (1 + level) limbs
 void rescale_core(hb_ctx *c, const u64 *x, u64 *out, int l, int np, int nbp, u64 *last, u64 *t) {
     const int N = c->N;
     const LimbMap lm = one_limb(l);
     if (c->logn == 16) {
-        InvScale sc{};
-        for (int i = 0; i < l; ++i) scale_words(hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]), c->h->q[i], c->tb.t16.pm, sc.w[i], sc.c[i]);
         inv_rows(c, x + (size_t)l * N, (size_t)(l + 1) * N, last, (size_t)N, nbp, lm);
         launch_lift(c, last, (size_t)N, t, (size_t)l * N, l, nbp);
-        const RowsFin f{x, (size_t)(l + 1) * N, out, (size_t)np * l * N, np, 1, 0};
-        LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, t, (size_t)l * N, l, nbp, f, sc, NoAddends{}, c->pc, c->tb.t16));
+        rescale_rows(c, x, (size_t)(l + 1) * N, t, out, l, np, nbp);
     } else {
         ntt(c, x + (size_t)l * N, (size_t)(l + 1) * N, last, (size_t)N, nbp, lm, true);
         LAUNCH(c), k_rescale_prep<<<c->egrid(nbp * l), 256, 0, c->st>>>(t, last, l, c->pc, N);
@@ -859,6 +863,14 @@ hb_ct *do_rescale(hb_ctx *c, const hb_ct *a) {
     } catch (...) { hb_ct_free(r); throw; }
     return r;
 }
+// last [sums][groups][nbp][N], residues modulo q_l in NTT form -> t [sums][nbp][l][N], coefficient form: the sum over the groups of the centred lifts
+void lift_sum(hb_ctx *c, u64 *last, int sums, int groups, int nbp, int l, u64 *t) {
+    const int N = c->N, total = sums * nbp;
+    Tmp S(c, (size_t)total);
+    ntt_inplace(c, last, groups * total, one_limb(l), true);
+    LAUNCH(c), k_centre_sum<<<dim3(c->gx(), total), 256, 0, c->st>>>((i64 *)S.p, last, groups, nbp, l, c->pc, N);
+    LAUNCH(c), k_lift_mod<<<c->egrid(total * l), 256, 0, c->st>>>(t, (const i64 *)S.p, l, c->pc, N);
+}
 // last [sums][groups][nbp][N], residues modulo q_l in NTT form -> t [sums][nbp][l][N], NTT form: the sum over the groups of the centred lifts
 void lift_last(hb_ctx *c, u64 *last, int sums, int groups, int nbp, int l, u64 *t) {
     const int N = c->N, total = sums * nbp;
@@ -868,10 +880,7 @@ void lift_last(hb_ctx *c, u64 *last, int sums, int groups, int nbp, int l, u64 *
         fwd_rows(c, t, (size_t)l * N, total * l, c->qmap(l - 1));
         return;
     }
-    Tmp S(c, (size_t)total);
-    ntt_inplace(c, last, groups * total, one_limb(l), true);
-    LAUNCH(c), k_centre_sum<<<dim3(c->gx(), total), 256, 0, c->st>>>((i64 *)S.p, last, groups, nbp, l, c->pc, N);
-    LAUNCH(c), k_lift_mod<<<c->egrid(total * l), 256, 0, c->st>>>(t, (const i64 *)S.p, l, c->pc, N);
+    lift_sum(c, last, sums, groups, nbp, l, t);
     ntt_inplace(c, t, total * l, c->qmap(l - 1), false);
 }
 // Sums of products are held as a whole before they are rescaled up to this many limbs (8 GB on 2^16 rings), beyond limb by limb
@@ -958,21 +967,30 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
         // of parts 4 x 4, 12 377 / 525, 84 2138 / 2256; 2 x 8, 12 553 / 852, 84 3666 / 4158; 1 x 8, 12 569 / 808, 84 3646 / 3899.
         const int groups = (parts + G - 1) / G * G;
         const int streamed = std::max(groups * 4 >= parts * 5 ? 84 : 10, count > 8 ? 48 * count * count / (17 * 17) : count > 4 ? 84 * count * count / 64 : 10);
-        auto sums = [&](u64 *o, const u64 *tt, unsigned limbs) {
-            auto few = [&](auto *kernel) { LAUNCH(c), kernel<<<dim3((unsigned)(N / 256 * ((nbp + 1) / 2)), limbs), 256, 0, c->st>>>(o, pt, tt, l, nbp, c->pc, N, qi); };
+        auto sums = [&](u64 *o, const u64 *tt, int from, unsigned limbs) {
+            auto few = [&](auto *kernel) { LAUNCH(c), kernel<<<dim3((unsigned)(N / 256 * ((nbp + 1) / 2)), limbs), 256, 0, c->st>>>(o, pt, tt, l, from, nbp, c->pc, N, qi); };
             if (nbp <= streamed || parts <= 2) few(count <= 2 ? k_prod_parts_few<2> : count <= 4 ? k_prod_parts_few<4> : count <= 8 ? k_prod_parts_few<8> : k_prod_parts_few<kMaxPartTerms>);
-            else LAUNCH(c), k_prod_parts<G><<<dim3(pg, (unsigned)(N / kPartLanes), limbs), 512, part_smem(G, count), c->st>>>(o, pt, tt, l, nbp, c->pc, N, qi, c->dev_err);
+            else LAUNCH(c), k_prod_parts<G><<<dim3(pg, (unsigned)(N / kPartLanes), limbs), 512, part_smem(G, count), c->st>>>(o, pt, tt, l, from, nbp, c->pc, N, qi, c->dev_err);
         };
         if (c->logn == 16 && !separate && (size_t)gnbp * (l + 1) <= kRawLimbs) { // all limbs at once, and a rescale
             Tmp x(c, (size_t)gnbp * (l + 1));
-            sums(x.p, nullptr, (unsigned)(l + 1));
+            sums(x.p, nullptr, 0, (unsigned)(l + 1));
             rescale_core(c, x.p, r->d, l, a0->np, gnbp, last.p, t.p);
             return r;
         }
         if (separate) launch(c, k_last_prod_parts, dim3(c->gx(), nbp, parts * count), 256, 0, last.p, pt, l, nbp, c->pc, N);
-        else sums(last.p, nullptr, 1);
+        else sums(last.p, nullptr, l, 1);
+        if (separate && c->logn == 16 && (size_t)gnbp * l <= kRawLimbs) { // every product rescaled on its own: the sum of the lifts, raw sums, and the row pass of a rescale
+            Tmp x(c, (size_t)gnbp * l);
+            sums(x.p, nullptr, 0, (unsigned)l);
+            lift_sum(c, last.p, parts, count, nbp, l, t.p);
+            LAUNCH(c); CK(launch_fwd_cols16(c->st, t.p, (size_t)l * N, gnbp * l, c->qmap(l - 1), c->pc, c->tb.t16));
+            rescale_rows(c, x.p, (size_t)l * N, t.p, r->d, l, a0->np, gnbp);
+            CK(cudaGetLastError());
+            return r;
+        }
         lift_last(c, last.p, parts, separate ? count : 1, nbp, l, t.p);
-        sums(r->d, t.p, (unsigned)l);
+        sums(r->d, t.p, 0, (unsigned)l);
         CK(cudaGetLastError());
     } catch (...) { hb_ct_free(r); throw; }
     return r;

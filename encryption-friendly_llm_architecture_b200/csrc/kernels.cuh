@@ -394,13 +394,13 @@ __global__ void k_last_prod_parts(u64 *last, const __grid_constant__ PartTerms p
 // from a table instead of branches and one instruction per wide multiply-add 3.7 ms.  Memory hardly shows any more (DRAM 16 %, half a
 // warp waiting for loads): four warps a scheduler issue in 57 % of the slots, between fixed latencies and their turns at the math pipes (FP64 45 % of
 // the time on a short limb, wide multiply-adds 37 % over all).
-// t == nullptr: raw sums of the last `limbs` limbs up to `level`, out[((g * nbp + bp) * limbs + k) * N + x]   grid = (ceil(parts/G), N/kPartLanes, limbs)
+// t == nullptr: raw sums of the limbs from `from` on, out[((g * nbp + bp) * limbs + k) * N + x] for limb from + k    grid = (ceil(parts/G), N/kPartLanes, limbs)
 // else: out[((g * nbp + bp) * level + l) * N + x] = (sum - t[same]) * q_level^-1 mod q_l      grid = (ceil(parts/G), N/kPartLanes, level)
 // (parts first, so that the CTAs that read the same words run together)
 constexpr int kPartLanes = 128, kPartRing = 8;
 constexpr size_t part_smem(int g, int count) { return ((size_t)g * count * kPartLanes + (size_t)kPartRing * 2 * 512) * 8; }
 template <int G>
-__global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, const __grid_constant__ PartTerms pt, const u64 *__restrict__ t, int level, int nbp,
+__global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, const __grid_constant__ PartTerms pt, const u64 *__restrict__ t, int level, int from, int nbp,
                                                        const PrimeConst *__restrict__ pc, int N, const __grid_constant__ Scalars qlinv, int *__restrict__ err) {
     constexpr int M = 2, kSlots = 512 / kPartLanes, kStage = M * 512; // members of a thread
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
     u64 *ptile = reinterpret_cast<u64 *>(smem_raw) + kPartRing * kStage; // [count][G][kPartLanes]
     const u32 ring_at = smem_u32(ring);
     const int tid = threadIdx.x, lane = tid & (kPartLanes - 1), slot = tid / kPartLanes;
-    const int l = (t ? 0 : level + 1 - (int)gridDim.z) + (int)blockIdx.z, g0 = blockIdx.x * G;
+    const int l = from + (int)blockIdx.z, g0 = blockIdx.x * G;
     const int gn = min(G, pt.parts - g0);
     const u32 x0 = blockIdx.y * kPartLanes;
     // What a member needs, in order: its terms a_j, then the words of t that its parts are subtracted from.  (address at member 0, bytes per member)
@@ -564,10 +564,10 @@ __global__ void __launch_bounds__(512, 1) k_prod_parts(u64 *__restrict__ out, co
 // zero.  With seventeen for every call, one term and eight parts of eight polynomials took 871 us at level 7 (kept masks 739);
 // with two 523.  grid = (N/256 * pairs of polynomials, limbs), arguments as above
 template <int TERMS>
-__global__ void __launch_bounds__(256, TERMS <= 4 ? 4 : TERMS <= 8 ? 3 : 2) k_prod_parts_few(u64 *__restrict__ out, const __grid_constant__ PartTerms pt, const u64 *__restrict__ t, int level, int nbp,
+__global__ void __launch_bounds__(256, TERMS <= 4 ? 4 : TERMS <= 8 ? 3 : 2) k_prod_parts_few(u64 *__restrict__ out, const __grid_constant__ PartTerms pt, const u64 *__restrict__ t, int level, int from, int nbp,
                                                                                             const PrimeConst *__restrict__ pc, int N, const __grid_constant__ Scalars qlinv) {
     const int pairs = (nbp + 1) / 2, bp = blockIdx.x % pairs * 2; // the pairs that read the same masks run together
-    const int limbs = gridDim.y, k = blockIdx.y, l = (t ? 0 : level + 1 - limbs) + k, count = pt.count, x = blockIdx.x / pairs * 256 + threadIdx.x;
+    const int limbs = gridDim.y, k = blockIdx.y, l = from + k, count = pt.count, x = blockIdx.x / pairs * 256 + threadIdx.x;
     const bool both = bp + 1 < nbp;
     const PrimeConst m = pc[l];
     const u64 qli = t ? qlinv.v[l] : 0;
