@@ -1252,13 +1252,14 @@ template <class FILL> hb_ct *encrypt_messages(hb_ctx *c, size_t n_slots, bool cp
         const LimbMap qm = c->qmap(level);
         TmpBytes ids(c, (size_t)count * 8);
         CK(cudaMemcpyAsync(ids.p, nonces, (size_t)count * 8, cudaMemcpyHostToDevice, c->st));
-        Tmp me(c, (size_t)std::min(count, kUpMembers) * n); // message + error; NTT form is linear, one transform serves both
+        const size_t me_limbs = (size_t)std::min(count, kUpMembers) * n;
+        Tmp me(c, me_limbs + ((size_t)count + 7) / 8); // message + error (NTT form is linear, one transform serves both); behind them errors drawn ahead, a byte each
         if (c->logn == 16 && c->h->gauss_cdt.size() < 128) { // errors fit a byte
             // The uniform parts and errors are drawn for up to kAhead members before their messages are there.  Messages at level 12, the
             // Python call, us: 1 141 -> 107, 4 409 -> 314, 13 824 -> 657, 96 3840 -> 3200 (kernels of thirteen 554 -> 415; one residue kernel with the errors in it had 1024
             // warps, and left no place to the generator while the first messages were copied).
             constexpr int kAhead = 4 * kUpMembers;
-            TmpBytes noise(c, (size_t)count * N);
+            signed char *noise = (signed char *)(me.p + me_limbs * (size_t)N);
             InvScale one{};
             for (int l = 0; l < n; ++l) scale_words(1, c->h->q[l], c->tb.t16.pm, one.w[l], one.c[l]);
             auto draw = [&](int first) {
@@ -1267,13 +1268,13 @@ template <class FILL> hb_ct *encrypt_messages(hb_ctx *c, size_t n_slots, bool cp
                 LAUNCH(c), k_uniform<<<dim3((unsigned)(N / 4 / 256), (unsigned)n, m), 256, 0, c->st>>>(r->d + (size_t)first * 2 * n * N, c->sk, StreamIds{c->ckey, hbhost::STREAM_ENC_A, id, 0}, c->pc,
                                                                                                       N); // comes after a copy, the first time
                 CK(cudaPeekAtLastError());
-                launch(c, k_noise, dim3((unsigned)(N / 8 / 128), m), 128, 0, (signed char *)noise.p + (size_t)first * N, StreamIds{c->ckey, hbhost::STREAM_ENC_E, id, 0}, (const u64 *)c->cdt,
+                launch(c, k_noise, dim3((unsigned)(N / 8 / 128), m), 128, 0, noise + (size_t)first * N, StreamIds{c->ckey, hbhost::STREAM_ENC_E, id, 0}, (const u64 *)c->cdt,
                        (int)c->h->gauss_cdt.size(), N);
             };
             draw(0);
             encode_chunks(c, n_slots, cplx, count, c->h->scale[level], fill, [&](int first, int m, const i64 *coef) {
                 u64 *b = r->d + (size_t)first * 2 * n * N; // holds -a s
-                launch(c, k_noisy_residues, dim3((unsigned)(N / 4 / 256), (unsigned)n, (unsigned)m), 256, 0, me.p, coef, (const signed char *)noise.p + (size_t)first * N, c->pc, N);
+                launch(c, k_noisy_residues, dim3((unsigned)(N / 4 / 256), (unsigned)n, (unsigned)m), 256, 0, me.p, coef, (const signed char *)(noise + (size_t)first * N), c->pc, N);
                 LAUNCH(c); CK(launch_fwd_cols16(c->st, me.p, (size_t)n * N, m * n, qm, c->pc, c->tb.t16));
                 const RowsFin f{b, (size_t)2 * n * N, b, (size_t)2 * n * N, 1, 1, 0};
                 LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, me.p, (size_t)n * N, n, m, f, one, NoAddends{}, c->pc, c->tb.t16));
