@@ -177,7 +177,7 @@ __device__ __forceinline__ u64 canon_fp64(double v, double q_inv, double qd) {
 
 // ---- exact sums of a few such products -------------------------------------------------------------------------
 // h collects the products rounded to multiples of 2^40 (it starts at 1.5 * 2^92, whose ulp that is), l the remainders: four FP64
-// instructions per product instead of seven, one quotient for the sum.  a, w >= 0; the products must add up to less than 2^91:
+// instructions per product instead of seven, one quotient for the sum.  a, w >= 0, or a within 0.6 q of zero (ks_rows); the products must add up to less than 2^91 in magnitude:
 // 2^7 of them for primes below 2^42, eight below 2^44.
 constexpr double kGrid40 = 1.5 * 0x1p92;
 struct FpAcc {
