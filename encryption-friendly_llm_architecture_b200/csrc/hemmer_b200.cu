@@ -11,6 +11,7 @@
 #include "ksrows.cuh"
 #include "embed.cuh"
 #include "host_threads.hpp"
+#include "launch_rules.hpp"
 #include "pool.hpp"
 
 #include <cstdio>
@@ -960,16 +961,9 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
         if (!c->smem_opt_in_parts) { CK(cudaFuncSetAttribute(k_prod_parts<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)part_smem(G, kMaxPartTerms))); c->smem_opt_in_parts = true; }
         Scalars qi{};
         for (int i = 0; i < l; ++i) qi.v[i] = hbhost::invmod(c->h->q[l] % c->h->q[i], c->h->q[i]);
-        // For few polynomials, and for one or two parts, the masks are streamed once per pair of polynomials; otherwise they are kept.  Up to how many
-        // polynomials depends on how much of either kernel works for nothing: the streamed one multiplies 2, 4, 8 or 17 terms, the other has six parts a CTA.
-        // Calls at level 7, us, streamed / kept, terms x parts: 16 x 12, 12 polynomials 1397 / 1901, 32 3646 / 3777, 48 5452 / 5305; 12 x 12, 16 polynomials 1820 /
-        // 1997, 24 2712 / 2686; 9 x 6, 12 763 / 806, 16 981 / 931; 8 x 12, 12 987 / 1460, 84 6821 / 7002; 17 x 17, 48 7590 / 8105; with a part-filled last group
-        // of parts 4 x 4, 12 377 / 525, 84 2138 / 2256; 2 x 8, 12 553 / 852, 84 3666 / 4158; 1 x 8, 12 569 / 808, 84 3646 / 3899.
-        const int groups = (parts + G - 1) / G * G;
-        const int streamed = std::max(groups * 4 >= parts * 5 ? 84 : 10, count > 8 ? 48 * count * count / (17 * 17) : count > 4 ? 84 * count * count / 64 : 10);
         auto sums = [&](u64 *o, const u64 *tt, int from, unsigned limbs) {
             auto few = [&](auto *kernel) { LAUNCH(c), kernel<<<dim3((unsigned)(N / 256 * ((nbp + 1) / 2)), limbs), 256, 0, c->st>>>(o, pt, tt, l, from, nbp, c->pc, N, qi); };
-            if (nbp <= streamed || parts <= 2) few(count <= 2 ? k_prod_parts_few<2> : count <= 4 ? k_prod_parts_few<4> : count <= 8 ? k_prod_parts_few<8> : k_prod_parts_few<kMaxPartTerms>);
+            if (parts <= 2 || nbp <= streamed_polynomials(count, parts)) few(count <= 2 ? k_prod_parts_few<2> : count <= 4 ? k_prod_parts_few<4> : count <= 8 ? k_prod_parts_few<8> : k_prod_parts_few<kMaxPartTerms>);
             else LAUNCH(c), k_prod_parts<G><<<dim3(pg, (unsigned)(N / kPartLanes), limbs), 512, part_smem(G, count), c->st>>>(o, pt, tt, l, from, nbp, c->pc, N, qi, c->dev_err);
         };
         if (c->logn == 16 && !separate && (size_t)gnbp * (l + 1) <= kRawLimbs) { // all limbs at once, and a rescale

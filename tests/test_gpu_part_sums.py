@@ -53,6 +53,12 @@ def test_part_sums_on_either_side_of_the_line_between_the_kernels(pkg, g, terms,
     _compare_part_sums(pkg, g, terms, parts, polys, batch, True)
 
 
+@pytest.mark.parametrize("terms,parts,polys,batch", [(4, 4, 2, 48), (4, 4, 1, 97), (3, 6, 2, 12), (3, 6, 1, 25), (8, 6, 3, 4), (8, 6, 1, 13), (5, 7, 2, 24), (5, 7, 1, 49), (8, 12, 2, 8), (8, 12, 1, 17), (9, 4, 1, 10),
+                                                     (9, 4, 1, 11), (17, 13, 2, 8), (17, 13, 1, 17), (16, 12, 2, 6), (16, 12, 1, 13), (9, 8, 1, 12), (9, 8, 1, 13), (11, 17, 1, 10), (11, 17, 1, 11)])
+def test_part_sums_on_either_side_of_every_line_of_the_rule(pkg, g, terms, parts, polys, batch):
+    _compare_part_sums(pkg, g, terms, parts, polys, batch, True)
+
+
 def _compare_part_sums(pkg, g, terms, parts, polys, batch, top):
     rng = np.random.default_rng(terms * 100 + parts)
     xs = [_ct(g, polys, batch, 40 + j, top) for j in range(terms)]

@@ -38,3 +38,7 @@ def test_shared_memory_of_the_conversions(tmp_path):
 
 def test_twiddle_values(tmp_path):
     _run(tmp_path, "twiddles")
+
+
+def test_rules_of_dispatch_take_what_was_measured_quicker(tmp_path):
+    _run(tmp_path, "launch_rules")
