@@ -122,6 +122,7 @@ struct hb_ctx {
     unsigned gx() const { return (unsigned)((N + 256 * kElems - 1) / (256 * kElems)); } // blocks per limb of the element-wise kernels
     dim3 egrid(int count) const { return dim3(gx(), (unsigned)count); }
     u64 *alloc_limbs(size_t limbs) { return (u64 *)pool.get(limbs * (size_t)N * 8); }
+    u64 *spare_limbs(size_t limbs) { return (u64 *)pool.spare(limbs * (size_t)N * 8); }
 };
 
 #define LAUNCH(c) ((c)->launches++, 0)
@@ -158,6 +159,12 @@ struct Tmp { // pool buffer released at scope exit
     Tmp(hb_ctx *cc, size_t limbs) : c(cc), p(cc->alloc_limbs(limbs)) {}
     ~Tmp() { c->pool.put(p); }
     Tmp(const Tmp &) = delete;
+};
+struct Spare { // the same where there is room, null otherwise
+    hb_ctx *c; u64 *p;
+    Spare(hb_ctx *cc, size_t limbs) : c(cc), p(cc->spare_limbs(limbs)) {}
+    ~Spare() { c->pool.put(p); }
+    Spare(const Spare &) = delete;
 };
 
 struct TmpBytes { // the same for a byte count (staging buffers of int64 coefficients)
@@ -884,7 +891,7 @@ void lift_last(hb_ctx *c, u64 *last, int sums, int groups, int nbp, int l, u64 *
     lift_sum(c, last, sums, groups, nbp, l, t);
     ntt_inplace(c, t, total * l, c->qmap(l - 1), false);
 }
-// Sums of products are held as a whole before they are rescaled up to this many limbs (8 GB on 2^16 rings), beyond limb by limb
+// Sums of products are held as a whole before they are rescaled up to this many limbs (8 GB on 2^16 rings) where the device has room for them, else limb by limb
 constexpr size_t kRawLimbs = 16384;
 // sum_j rescale(a_j (.) p_j)  (separate)  or  rescale(sum_j a_j (.) p_j); `sums` such sums of `count` terms each, sum k from the terms
 // k * count ..., one member group of the result per sum
@@ -906,12 +913,12 @@ hb_ct *do_prod_rescale(hb_ctx *c, const hb_ct *const *a, const hb_pt *const *p, 
     ALG(c, (size_t)count * sums * ((size_t)nbp * (l + 1) + (l + 1)) + (size_t)total * l);
     try {
         Tmp last(c, (size_t)groups * total), t(c, (size_t)total * l);
-        if (c->logn == 16 && !separate && (size_t)total * (l + 1) <= kRawLimbs) {
-            Tmp x(c, (size_t)total * (l + 1));
-            launch(c, k_prod_sums, dim3(gx, (unsigned)(total * (l + 1))), 256, 0, x.p, tl, l, nbp, c->pc, N);
-            rescale_core(c, x.p, r->d, l, a0->np, total, last.p, t.p);
-            return r;
-        }
+        if (c->logn == 16 && !separate && (size_t)total * (l + 1) <= kRawLimbs)
+            if (Spare x(c, (size_t)total * (l + 1)); x.p) {
+                launch(c, k_prod_sums, dim3(gx, (unsigned)(total * (l + 1))), 256, 0, x.p, tl, l, nbp, c->pc, N);
+                rescale_core(c, x.p, r->d, l, a0->np, total, last.p, t.p);
+                return r;
+            }
         launch(c, k_last_prod, dim3(gx, total, groups), 256, 0, last.p, tl, separate ? 1 : 0, l, nbp, c->pc, N);
         lift_last(c, last.p, 1, groups, total, l, t.p);
         Scalars qi{};
@@ -951,6 +958,7 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
         }
         if (!terms) fail(HB_E_ARG, "product sums: a part without terms");
     }
+    if (count == 1) separate = false; // a sum of one product
     const int l = a0->level, N = c->N, nbp = a0->batch * a0->np, gnbp = parts * nbp;
     hb_ct *r = new_ct(c, l - 1, a0->np, parts * a0->batch, 1);
     ALG(c, (size_t)count * nbp * (l + 1) + used * (l + 1) + (size_t)gnbp * l);
@@ -966,24 +974,25 @@ hb_ct *do_prod_rescale_parts(hb_ctx *c, const hb_ct *const *a, const hb_pt *cons
             if (parts <= 2 || nbp <= streamed_polynomials(count, parts)) few(count <= 2 ? k_prod_parts_few<2> : count <= 4 ? k_prod_parts_few<4> : count <= 8 ? k_prod_parts_few<8> : k_prod_parts_few<kMaxPartTerms>);
             else LAUNCH(c), k_prod_parts<G><<<dim3(pg, (unsigned)(N / kPartLanes), limbs), 512, part_smem(G, count), c->st>>>(o, pt, tt, l, from, nbp, c->pc, N, qi, c->dev_err);
         };
-        if (c->logn == 16 && !separate && (size_t)gnbp * (l + 1) <= kRawLimbs) { // all limbs at once, and a rescale
-            Tmp x(c, (size_t)gnbp * (l + 1));
-            sums(x.p, nullptr, 0, (unsigned)(l + 1));
-            rescale_core(c, x.p, r->d, l, a0->np, gnbp, last.p, t.p);
-            return r;
-        }
+        if (c->logn == 16 && !separate && (size_t)gnbp * (l + 1) <= kRawLimbs) // all limbs at once, and a rescale
+            if (Spare x(c, (size_t)gnbp * (l + 1)); x.p) {
+                sums(x.p, nullptr, 0, (unsigned)(l + 1));
+                rescale_core(c, x.p, r->d, l, a0->np, gnbp, last.p, t.p);
+                return r;
+            }
         if (separate) launch(c, k_last_prod_parts, dim3(c->gx(), nbp, parts * count), 256, 0, last.p, pt, l, nbp, c->pc, N);
         else sums(last.p, nullptr, l, 1);
         if (separate && c->logn == 16 && (size_t)gnbp * l <= kRawLimbs) { // every product rescaled on its own: the sum of the lifts, raw sums, and the row pass of a rescale
-            Tmp x(c, (size_t)gnbp * l);
-            sums(x.p, nullptr, 0, (unsigned)l);
             lift_sum(c, last.p, parts, count, nbp, l, t.p);
-            LAUNCH(c); CK(launch_fwd_cols16(c->st, t.p, (size_t)l * N, gnbp * l, c->qmap(l - 1), c->pc, c->tb.t16));
-            rescale_rows(c, x.p, (size_t)l * N, t.p, r->d, l, a0->np, gnbp);
-            CK(cudaGetLastError());
-            return r;
-        }
-        lift_last(c, last.p, parts, separate ? count : 1, nbp, l, t.p);
+            if (Spare x(c, (size_t)gnbp * l); x.p) {
+                sums(x.p, nullptr, 0, (unsigned)l);
+                LAUNCH(c); CK(launch_fwd_cols16(c->st, t.p, (size_t)l * N, gnbp * l, c->qmap(l - 1), c->pc, c->tb.t16));
+                rescale_rows(c, x.p, (size_t)l * N, t.p, r->d, l, a0->np, gnbp);
+                CK(cudaGetLastError());
+                return r;
+            }
+            ntt_inplace(c, t.p, gnbp * l, c->qmap(l - 1), false);
+        } else lift_last(c, last.p, parts, separate ? count : 1, nbp, l, t.p);
         sums(r->d, t.p, 0, (unsigned)l);
         CK(cudaGetLastError());
     } catch (...) { hb_ct_free(r); throw; }

@@ -31,13 +31,19 @@ struct Pool {
     }
     void *get(size_t bytes) {
         bytes = (bytes + 255) & ~(size_t)255;
-        auto &v = free_[bytes];
-        void *p = nullptr;
-        if (!v.empty()) { p = v.back(); v.pop_back(); }
-        else { p = raw(bytes); total += bytes; }
-        live_[p] = bytes; in_use += bytes;
-        if (recording && recording->insert(p).second) ++held_[p];
-        return p;
+        void *p = idle(bytes);
+        if (!p) { p = raw(bytes); total += bytes; }
+        return hand_out(p, bytes);
+    }
+    // A buffer that the caller can do without: an idle one or what the driver has left; null otherwise, and no idle buffer goes back to the driver for it.
+    void *spare(size_t bytes) {
+        bytes = (bytes + 255) & ~(size_t)255;
+        void *p = idle(bytes);
+        if (!p) {
+            if (cudaMalloc(&p, bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+            total += bytes;
+        }
+        return hand_out(p, bytes);
     }
     void put(void *p) {
         if (!p) return;
@@ -63,4 +69,18 @@ struct Pool {
         }
     }
     ~Pool() { held_.clear(); release_cached(); for (auto &kv : live_) cudaFree(kv.first); }
+
+private:
+    void *idle(size_t bytes) {
+        auto &v = free_[bytes];
+        if (v.empty()) return nullptr;
+        void *p = v.back();
+        v.pop_back();
+        return p;
+    }
+    void *hand_out(void *p, size_t bytes) {
+        live_[p] = bytes; in_use += bytes;
+        if (recording && recording->insert(p).second) ++held_[p];
+        return p;
+    }
 };

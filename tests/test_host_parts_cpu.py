@@ -42,3 +42,7 @@ def test_twiddle_values(tmp_path):
 
 def test_rules_of_dispatch_take_what_was_measured_quicker(tmp_path):
     _run(tmp_path, "launch_rules")
+
+
+def test_buffers_that_a_call_can_do_without(tmp_path):
+    _run(tmp_path, "pool_spare")
