@@ -104,7 +104,7 @@ struct hb_ctx {
     CentreConst centre{};
     ChaChaKey ckey{};
     std::map<std::pair<int, long long>, u32 *> gal_tables; // (copies, row_step) -> Galois elements of hb_matmul_acc, on the device
-    int host_threads = 0;                                 // cap for the threads that move slot values in host memory (0: no cap beyond kCopyThreads)
+    int host_threads = 0;                                 // cap for the threads of a call that moves slot values in host memory (0: kCopyThreads)
     bool capturing = false;                               // between hb_graph_begin and hb_graph_end
     Pool::Buffers recorded;                               // what the pool handed out in between
     unsigned long long launches_at_capture = 0, alg_at_capture = 0;
@@ -1153,8 +1153,8 @@ void up_open(hb_ctx *c) {
     stage_open(c, c->up, c->went_up, kUpMembers, cudaHostAllocWriteCombined);
 }
 int copy_threads(const hb_ctx *c) { return c->host_threads > 0 ? c->host_threads : kCopyThreads; }
-void host_copy(const hb_ctx *c, double *dst, const double *src, size_t words) {
-    in_threads(copy_threads(c), words, words, [&](size_t a, size_t b) { std::memcpy(dst + a, src + a, (b - a) * sizeof(double)); });
+void host_copy(const hb_ctx *c, double *dst, const double *src, size_t words, int busy = 0) { // busy: threads of the cap that are at work elsewhere
+    in_threads(copy_threads(c) - busy, words, words, [&](size_t a, size_t b) { std::memcpy(dst + a, src + a, (b - a) * sizeof(double)); });
 }
 // coef [count][N] = rounded coefficients at scale sc of the messages re / im [count][n] on the device (im may be null)
 void embed_inverse(hb_ctx *c, i64 *coef, const double *re, const double *im, int n, int count, double sc) {
@@ -1209,7 +1209,7 @@ auto from_arrays(hb_ctx *c, const double *re, const double *im, size_t n) {
 void decrypt_items(hb_ctx *c, const std::vector<DecItem> &items, bool z, double *re, double *im) {
     stage_open(c, c->down, c->came_down, kStageMembers, cudaHostAllocDefault);
     const int count = (int)items.size(), N = c->N, slots = N / 2;
-    Pages pages(copy_threads(c));
+    Pages pages(std::min(copy_threads(c), kCopyThreads) - 1); // and this thread
     TmpBytes list(c, items.size() * sizeof(DecItem));
     CK(cudaMemcpyAsync(list.p, items.data(), items.size() * sizeof(DecItem), cudaMemcpyHostToDevice, c->st));
     auto collect = [&](int first, int slot) {
@@ -1217,9 +1217,9 @@ void decrypt_items(hb_ctx *c, const std::vector<DecItem> &items, bool z, double 
         const size_t words = (size_t)m * slots;
         CK(cudaEventSynchronize(c->came_down[slot]));
         const double *h = c->down[slot];
-        if (z) { host_copy(c, re + (size_t)first * N, h, 2 * words); return; }
-        host_copy(c, re + (size_t)first * slots, h, words);
-        if (im) host_copy(c, im + (size_t)first * slots, h + words, words);
+        if (z) { host_copy(c, re + (size_t)first * N, h, 2 * words, pages.running()); return; }
+        host_copy(c, re + (size_t)first * slots, h, words, pages.running());
+        if (im) host_copy(c, im + (size_t)first * slots, h + words, words, pages.running());
     };
     int slot = 0;
     for (int first = 0; first < count; first += kStageMembers, slot ^= 1) {
@@ -1235,12 +1235,13 @@ void decrypt_items(hb_ctx *c, const std::vector<DecItem> &items, bool z, double 
         embed_forward(c, d, z ? d + 1 : d + words, z ? 2 : 1, t.p, it, m);
         CK(cudaMemcpyAsync(c->down[slot], d, words * (z || im ? 2 : 1) * sizeof(double), cudaMemcpyDeviceToHost, c->st));
         CK(cudaEventRecord(c->came_down[slot], c->st));
-        // For two chunks: later ones are copied while these threads would compete with the copies (96 members 6.0 -> 8.1 ms).  Members to fresh numpy
-        // arrays, us: 2 270 -> 171, 4 530 -> 260, 8 870 -> 400, 13 800 -> 650, 24 1250 -> 780, 48 1400 -> 1400 to 1780, 96 6300 -> 5900.
+        // For two chunks: later ones are copied while these threads would compete with the copies (96 members 6.0 -> 8.1 ms).  Members to pages that are not there
+        // yet, complex values / two arrays, us, without -> with three threads beside the caller: 1 236 / 238 -> 164 / 235, 2 380 / 420 -> 253 / 249, 4 486 / 780 -> 411 / 368,
+        // 8 970 / 860 -> 877 / 644, 13 1314 / 1559 -> 1286 / 1027, 24 2245 / 2407 -> 2159 / 2067, from 48 on within 5 %.  To pages that are there: 2 145 / 138 -> 135 / 139, 13
+        // 436 / 675 -> 370 / 436, 48 1045 / 1085 -> 1041 / 1096 (a thread that has just been at work wakes sooner for the copies).
         if (!first) {
             const size_t early = (size_t)std::min(count, 2 * kStageMembers) * slots;
-            pages.ask(re, early * (z ? 2 : 1));
-            if (!z && im) pages.ask(im, early);
+            pages.ask(re, early * (z ? 2 : 1), z ? nullptr : im);
         }
         if (first) collect(first - kStageMembers, slot ^ 1);
     }

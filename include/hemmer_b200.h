@@ -305,7 +305,8 @@ int hb_send(hb_ctx *ctx, const hb_ct *a, int peer, void *nccl_comm);
 int hb_recv(hb_ctx *ctx, hb_ct *a, int peer, void *nccl_comm);
 int hb_sum_mod_reduce(hb_ctx *ctx, const hb_ct *const *parts, int count, hb_ct **out);
 
-/* Host threads that move slot values between the caller's memory and the pinned buffers (0: up to four).
+/* Host threads of a call that moves slot values between the caller's memory and the pinned buffers, the caller and those that ask for
+ * the pages of results among them (0: up to four).  With 1 a call starts none.
  * Several ranks on one host each take cores / ranks.  No counterpart in the reference (one process per GPU under mpirun). */
 int hb_set_host_threads(hb_ctx *ctx, int n);
 

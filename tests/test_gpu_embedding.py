@@ -146,3 +146,37 @@ def test_errors_on_either_side_of_a_byte(pkg, sigma):
     for k in range(2):
         assert np.array_equal(got[k:k + 1], g.ct_export(g.encrypt(g.encode(msgs[k], 1), 5 + k))), f"member {k}"
     g.close()
+
+
+def test_a_cap_of_one_thread_starts_no_other(gpu_full):
+    """set_host_threads caps all threads of a call: with one, members go to memory that is new, pages and all, by the caller alone."""
+    import os
+    import threading
+
+    from conftest import rand_ct_residues
+    g = gpu_full
+    level, batch = 1, 16
+    x = g.ct_create(level, 2, batch)
+    g.ct_import(x, rand_ct_residues(g, level, 2, batch, seed=3))
+    items = [(x, k) for k in range(batch)]
+    counts, stop = [], threading.Event()
+
+    def watch():
+        while not stop.is_set():
+            counts.append(len(os.listdir("/proc/self/task")))
+
+    g.set_host_threads(1)
+    try:
+        keep = [g.decrypt_many(items)]
+        watcher = threading.Thread(target=watch)
+        watcher.start()
+        while len(counts) < 20:
+            pass
+        before = max(counts[:20])
+        keep += [g.decrypt_many(items) for _ in range(40)]
+        stop.set()
+        watcher.join()
+    finally:
+        g.set_host_threads(0)
+    assert max(counts) == before
+    assert all(np.array_equal(keep[0], z) for z in keep)

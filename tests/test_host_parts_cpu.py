@@ -46,3 +46,7 @@ def test_rules_of_dispatch_take_what_was_measured_quicker(tmp_path):
 
 def test_buffers_that_a_call_can_do_without(tmp_path):
     _run(tmp_path, "pool_spare")
+
+
+def test_threads_that_ask_for_pages_stay_within_their_cap(tmp_path):
+    _run(tmp_path, "page_threads", "-pthread")
