@@ -398,50 +398,15 @@ void conv_opt_in(hb_ctx *c) {
     allow(conv_mma<2, 2>, conv_mma_smem(2, kMaxPrimes)); allow(conv_mma<4, 1>, conv_mma_smem(4, kMaxPrimes));
     c->smem_opt_in_conv = true;
 }
-// Strip width and groups of a launch over `units` (polynomial, conversion) pairs.  At most two units: narrow strips and many groups, so that
-// all sources and all targets of a unit are worked on at once.  Up to twelve: narrow strips, two CTAs per SM, for the last wave.
-// Beyond: strips of eight columns (64-byte runs) and two groups, two CTAs per SM, whose barriers and loads cover each other, as long as their
-// strips fit (four sources); otherwise four groups and one CTA.  Calls, us, (4 x 8) / (4 x 4) / (8 x 2): decompositions of level 7, 2 units 47 / 45 / 58,
-// divisions 53 / 59 / 62, 4 units 88 / 81 / 94, 10 units 175 / 163 / 171, 18 units 279 / 260 / 256, 40 units 594 / 546 / 533; decompositions of level 2, 17
-// units 111 / 92 / 83, of level 12, 24 units 280 / 260 / 254.  Launches, us, (8 x 4) / (8 x 2): 192 polynomials of the division at level 6 696 / 604,
-// the conversions of 256 products at level 8 3174 / 2719 and 2079 / 1797.
-// The wide strips lose where few SMs have one CTA more than the others: 15, 16, 19 and 20 units leave a tenth to a half of the SMs with it,
-// and a CTA with four sources and many targets is long.  Calls, us, (4 x 4) / (8 x 2): divisions of level 7, 16 units 234 / 238, 20 units 289 / 293, of
-// level 6 169 / 171 and 206 / 208.  Up to five targets it does not show (divisions of level 5, 16 units 157 / 155, 20 units 190 / 188), nor with the
-// three sources of a ModDown (level 7, 206 / 205 and 253 / 252); decompositions of level 12 go either way (179 / 180 and 222 / 221).
-// The line at twelve was drawn when the narrow strips were ahead up to there; now (8 x 2) is from seven units on, except at 10, 14, 16 and 20 of the
-// division (decompositions of level 2, 8 units 56 / 51; divisions of level 3, 8 units 84 / 76, of level 7, 8 units 134 / 131, 14 units 216 / 219).
-// More than four sources, (4 x 4) / (8 x 4): divisions of seven sources 32 units 425 / 434, 40 units 520 / 536; of eight 48 units 1120 / 1140;
-// a digit of seven limbs 40 units 425 / 411.
-//
-// mma: up to four sources, primes of LongPm, and two CTAs find room with their constants (conv_mma).  Its strips have eight columns, so few units fill the GPU
-// badly: two groups and two CTAs per SM hold nine units at once, four groups and one CTA four and a half.  Calls, us, the strips below / conv_mma
-// with two groups / with four: decompositions of level 6 (two digits), 4 units 39 / 47 / 35, 6 units 53 / 52 / 54, 8 units 65 / 59 / 61, 24 units 161 / 154 /
-// 172, 96 units 541 / 526 / 579, of level 12, 4 units 51 / 68 / 48, 48 units 436 / 420 / 451; masked sums with their divisions of level 6, 4 units 58 / 67 / 57, 8
-// units 97 / 91 / 94, 12 units 132 / 130 / 129, 16 units 162 / 161 / 164, 20 units 198 / 201 / 201, 96 units 803 / 780 / 836, of level 8, 20 units
-// 310 / 304 / 312, 96 units 1313 / 1288 / 1336.  Little is left to convert with fewer sources or targets: divisions of level 1, 96 units 434 / 444 / 483;
-// hoisted rotations with their ModDown of level 4, 96 units 708 / 712 / 765, of level 8 1068 / 1059 / 1133.
 constexpr size_t kTwoCtas = 228 * 1024 / 2 - 2048; // dynamic shared memory of a CTA when an SM takes two
-enum StripShape { kStrip8x1, kStrip8x2, kStrip8x4, kStrip4x4, kStrip4x8, kMma2, kMma4 };
-StripShape conv_shape(int units, int max_ns, int targets, bool mma) {
-    if (mma) {
-        if (units == 3 || units == 4 || units == 12) return kMma4;
-        if (units >= 7 && units <= 9) return kMma2;
-        if ((units == 17 || units == 18 || units >= 24) && targets >= (max_ns == 4 ? 3 : 6)) return kMma2;
-    }
-    if (units <= 2) return kStrip4x8;
-    if (units <= 12) return kStrip4x4;
-    if (max_ns > 4) return units <= 32 ? kStrip4x4 : kStrip8x4;
-    const int more = units * 32 % 148; // SMs with one CTA more
-    return units <= 20 && max_ns == 4 && targets > 5 && more >= 148 / 10 && more < 148 / 2 ? kStrip4x4 : kStrip8x2;
-}
 // Rescales: from 96 polynomials on one group per CTA, so that none waits for the source: 512 polynomials at level 8 1.14 -> 1.02 ms.  Calls, us, (4 x 4) / two
 // groups / one: level 8, 4 polynomials 61 / 67 / 69, 8 polynomials 100 / 96 / 115, 16 polynomials 179 / 174 / 174, 48 polynomials 508 / 493 / 485, 94 polynomials
 // 963 / 929 / 912, 96 polynomials 982 / 942 / 926; level 4, 16 polynomials 107 / 102 / 100, 96 polynomials 567 / 533 / 521.  The line lies where the
 // gain was seen first; one group is ahead by 1 to 2 % from 32 polynomials on.
 StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : units < 96 ? kStrip8x2 : kStrip8x1; }
-// `plans` conversions (the largest with max_ns sources, `targets` each on average, `most` at most, at most `consts` bytes of constants) of `instances` polynomials in one launch
-void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int targets, int most, size_t consts, int instances) {
+// `plans` conversions (the largest with max_ns sources, `sources` in all, `targets` each on average, `most` at most, at most `consts` bytes of constants) of `instances` polynomials
+// in one launch
+void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int sources, int targets, int most, size_t consts, int instances) {
     conv_opt_in(c);
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
         launch(c, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
@@ -451,7 +416,7 @@ void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, con
     };
     auto shapes = [&](auto arithmetic) {
         using LONG = decltype(arithmetic);
-        switch (conv_shape(instances * count, max_ns, targets, c->tb.t16.pm && max_ns <= 4 && conv_mma_smem(2, most) <= kTwoCtas)) {
+        switch (conv_shape(instances * count, max_ns, targets, count, sources, c->tb.t16.pm && max_ns <= 4 && conv_mma_smem(2, most) <= kTwoCtas)) {
         case kMma2: products(conv_mma<2, 2>, 2); break;
         case kMma4: products(conv_mma<4, 1>, 4); break;
         case kStrip8x2: go(conv_cols<8, 2, 2, 4, LONG>, 8, 2, strip_bytes(8, max_ns + 2) + consts); break;
@@ -522,7 +487,7 @@ void ks_lift(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch, u64 
     const int N = c->N, n = d.n;
     Tmp acoef(c, (size_t)batch * n);
     inv_rows(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level));
-    launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), d.dt_count / d.nd, digit_targets(*c->h, level), digit_const_bytes(*c->h, level), batch);
+    launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), n, d.dt_count / d.nd, digit_targets(*c->h, level), digit_const_bytes(*c->h, level), batch);
 }
 // Whether the digits of `members` polynomials that serve one rotation each go through ks_rows (its comment has the times on both sides)
 bool one_use(const hb_ctx *c, const PlanDims &d, int members) { return c->logn == 16 && c->tb.t16.pm && d.nd <= 4 && d.nd >= (members == 1 ? 3 : 2); }
@@ -557,7 +522,7 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, siz
         const ConvPlan *cv = get_conv_plans(c, level);
         u64 *sp = acc + (size_t)n * N;
         if (!half) inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, total * 2 * K, pm);
-        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, n, n, conv_const_bytes(K, n), total * 2);
+        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, K, n, n, conv_const_bytes(K, n), total * 2);
         const RowsFin f{acc, (size_t)ne * N, out, out_outer, 2, batch, add_outer};
         LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, total * 2, f, c->p_inv_scale, sl, c->pc, c->tb.t16));
         CK(cudaGetLastError());
@@ -747,7 +712,7 @@ hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch, hb_ct *dst = null
         if (c->logn == 16) {
             const ConvPlan *cv = get_conv_plans(c, level);
             inv_rows(c, src, (size_t)ne * N, src, (size_t)ne * N, batch * 2 * ns, sm);
-            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, level, level, conv_const_bytes(ns, level), batch * 2);
+            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, ns, level, level, conv_const_bytes(ns, level), batch * 2);
             const RowsFin f{E, (size_t)ne * N, out, (size_t)2 * level * N, 2, 1, 0};
             LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], NoAddends{}, c->pc, c->tb.t16));
             CK(cudaGetLastError());

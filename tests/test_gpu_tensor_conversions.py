@@ -1,5 +1,5 @@
-"""Base conversions on the tensor cores: the launch rules' edges (3, 4, 7 to 9, 12, 17, 18 and 24 units take them, their neighbours do not), one to four sources, odd and
-even numbers of targets, residues at the ends of their range.  Residues are whole numbers, so every comparison is exact."""
+"""Base conversions on the tensor cores: the launch rules' edges (of 3, 4, 7 to 9, 12, 17, 18 and from 24 units on some or all take them, their neighbours do not), one to
+four sources, odd and even numbers of targets, residues at the ends of their range.  Residues are whole numbers, so every comparison is exact."""
 import numpy as np
 import pytest
 
@@ -47,5 +47,24 @@ def test_members_are_the_same_on_either_side_of_the_rules(gpu_full, level):
     data = _data(g, level, 13)
     want = _pair(g, data, level, masks, (1, -3))
     for batch in (1, 2, 3, 4, 6, 8, 9, 12):
+        for a, b in zip(_pair(g, data[:batch], level, masks, (1, -3)), want):
+            assert np.array_equal(a, b[:batch]), f"{batch} members"
+
+
+@pytest.mark.parametrize("level,batch", [(1, 2), (1, 3), (1, 4), (1, 6), (2, 7), (3, 6), (5, 2), (8, 4), (9, 6), (12, 4)])
+def test_few_units_against_the_oracle(gpu_full, orc_full, level, batch):
+    """One and two targets for four groups, five targets, divisions of 8 and 12 units on either side of the line between two and four groups."""
+    test_against_the_oracle(gpu_full, orc_full, level, batch)
+
+
+@pytest.mark.parametrize("level", [1, 2, 3, 6])
+def test_every_number_of_units_around_the_lines(gpu_full, level):
+    """One digit up to level 2, two up to level 6: 1 to 25 units of decompositions with every count about the lines, even counts of divisions and ModDowns up to 50."""
+    g = gpu_full
+    masks = [np.ones(g.slots), np.full(g.slots, 0.5)]
+    g.gen_rot_keys([1, -3])
+    data = _data(g, level, 25)
+    want = [np.concatenate(x) for x in zip(*[_pair(g, data[k:k + 1], level, masks, (1, -3)) for k in range(25)])]
+    for batch in (2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 16, 17, 18, 19, 23, 24, 25):
         for a, b in zip(_pair(g, data[:batch], level, masks, (1, -3)), want):
             assert np.array_equal(a, b[:batch]), f"{batch} members"
