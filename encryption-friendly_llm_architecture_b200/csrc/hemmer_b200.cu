@@ -489,8 +489,8 @@ void ks_lift(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch, u64 
     inv_rows(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level));
     launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), n, d.dt_count / d.nd, digit_targets(*c->h, level), digit_const_bytes(*c->h, level), batch);
 }
-// Whether the digits of `members` polynomials that serve one rotation each go through ks_rows (its comment has the times on both sides)
-bool one_use(const hb_ctx *c, const PlanDims &d, int members) { return c->logn == 16 && c->tb.t16.pm && d.nd <= 4 && d.nd >= (members == 1 ? 3 : 2); }
+// Whether the digits of `members` polynomials that serve one rotation each go through ks_rows
+bool one_use(const hb_ctx *c, const PlanDims &d, int members) { return c->logn == 16 && c->tb.t16.pm && one_kernel_switch(d.nd, d.ne, members); }
 // Hybrid key switch of polynomial a (NTT form, `n` limbs, per-batch stride a_outer) with key `key`:
 //   out[b][p][l] = ModDown(sum_dg perm_g(lift_dg(a)) (.) key_dg)[p][l] + add_p[b][l] o perm_g
 // Phase 1 of a key switch (shared by every rotation of the same polynomial -- "hoisting"):
@@ -537,7 +537,7 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, siz
     CK(cudaGetLastError());
 }
 void launch_ks_rows(hb_ctx *c, u64 *acc, const SwitchList &sl, int batch, size_t a_outer, const KsPlan *pl, const PlanDims &d) {
-    const int m = batch >= 4 ? 2 : 1;
+    const int m = switch_members(batch);
     auto go = [&](auto *kernel) {
         launch(c, kernel, dim3(256 / kKsRows, (unsigned)(sl.count * ((batch + m - 1) / m)), (unsigned)d.ne), 16 * kKsRows * d.nd * m, ks_rows_smem(d.nd, m), acc, sl, batch, a_outer, c->nprimes,
                pl, c->pc, c->tb.t16);

@@ -12,9 +12,7 @@
 // TB/s).  Blocks of few warps, because their loads, transforms and sums alternate behind barriers: eight rows a CTA 4 to 7 % of a whole rotation
 // slower, four 1 to 2 %.  Two members a CTA share the key words that each coefficient meets: 64 members at level 8 2671 -> 2603 us.  Limbs in the inner order,
 // so that integer and FP64 work meet on an SM: 2729 us, twiddles and keys then come from L2 every time.
-// Rotations, us, three kernels / this one: level 12, 1 member 125 / 117, 4 members 337 / 315, 16 members 1077 / 1057; level 8, 1 member 99.7 / 95.9, 16 members
-// 728 / 713; level 6, 1 member 68 / 81 (left to the three kernels: a single wave of long code), 2 members 101 / 99, 48 members 1403 / 1381; one digit
-// (level 2) 48 / 58 and 261 / 274 (left as well).  256 products at level 8 14.2 / 13.9 ms.
+// Rotations with three kernels and with this one stand at the rule that chooses (one_kernel_switch).  256 products at level 8 14.2 / 13.9 ms.
 #pragma once
 #include "convcols.cuh"
 

@@ -52,6 +52,19 @@ constexpr StripShape conv_shape(int units, int max_ns, int targets, int plans, i
     return units <= 20 && max_ns == 4 && targets > 5 && more >= 148 / 10 && more < 148 / 2 ? kStrip4x4 : kStrip8x2;
 }
 
+// Key switches of digits used once, with limbs of Q and P together: whether their row passes and inner products go through one kernel (ks_rows), and the
+// members a CTA takes there.  Rotations, us, three kernels / ks_rows with one member a CTA / with two:
+//   one member      level 12 (four digits) 121 / 113, level 7 (three) 93 / 91, level 6 (two) 68 / 82; three digits of six limbs in all 65 / 74
+//   two digits      level 6, 2 members 98 / 102 / 104, 3 members 136 / 141 / 144, 12 members 397 / 400 / 394, 17 members 531 / 538 / 535; five limbs in all, 2 members 68 / 80 / 80
+//   three, four     level 12, 2 members 190 / 172 / 171, 24 members 1540 / 1510 / 1494; level 8, 12 members 556 / 561 / 546; level 7, 5 members 254 / 251 / 260
+// Over contexts of two to seven digits and 1 to 33 members no rotation takes over 1.03 of the time with three kernels.
+constexpr bool one_kernel_switch(int digits, int limbs, int members) {
+    if (digits < 2 || digits > 4) return false; // more do not fit the registers
+    if (digits == 2) return limbs >= 7 && members >= 4 && members % 2 == 0;
+    return members > 1 || digits * limbs >= 30;
+}
+constexpr int switch_members(int batch) { return batch >= 4 && (batch % 2 == 0 || batch > 8) ? 2 : 1; } // an odd one leaves half a CTA without work
+
 // Part sums: up to how many polynomials the masks are streamed once per pair of polynomials (k_prod_parts_few); beyond, and never for one or two parts, they
 // are kept (k_prod_parts).  Either kernel works for nothing where its sizes are not filled: the streamed one multiplies 2, 4, 8 or 17 terms, the other has
 // six parts a CTA.  Calls with a mask of its own for every product (the same masks for all parts stay in L2 and make streaming look up to 20 %

@@ -50,3 +50,18 @@ def test_relinearisation_against_the_oracle(gpu_full, orc_full, level):
     for got in res[1:]:
         for k in range(got.shape[0]):
             assert np.array_equal(got[k], res[0][0]), f"member {k} of {got.shape[0]}"
+
+
+@pytest.mark.parametrize("level,batch", [(3, 4), (6, 4), (6, 6), (5, 5), (7, 2), (7, 5), (7, 7), (9, 8), (12, 9), (11, 10), (11, 12)])
+def test_one_and_two_members_a_block(pkg, gpu_full, level, batch):
+    """Two digits from four members on, in pairs; odd numbers up to seven one by one, beyond with half a block."""
+    test_rotations_equal_those_from_kept_digits(pkg, gpu_full, level, batch)
+
+
+def test_few_limbs_in_all(pkg):
+    """Digits of two limbs and two special primes: three digits of six or seven limbs, four of eight, two of five."""
+    g = pkg.open_gpu(pkg.make_params(dnum=7, num_special=2))
+    g.keygen()
+    for level, batch in ((3, 1), (3, 2), (4, 1), (5, 1), (6, 5), (2, 2), (2, 4)):
+        test_rotations_equal_those_from_kept_digits(pkg, g, level, batch)
+    g.close()
