@@ -406,7 +406,7 @@ constexpr size_t kTwoCtas = 228 * 1024 / 2 - 2048; // dynamic shared memory of a
 StripShape lift_shape(int units) { return units <= 2 ? kStrip4x8 : units <= 4 ? kStrip4x4 : units < 96 ? kStrip8x2 : kStrip8x1; }
 // `plans` conversions (the largest with max_ns sources, `sources` in all, `targets` each on average, `most` at most, at most `consts` bytes of constants) of `instances` polynomials
 // in one launch
-void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int sources, int targets, int most, size_t consts, int instances) {
+void launch_conv(hb_ctx *c, Conversion what, const u64 *src, size_t so, u64 *dst, size_t dof, const ConvPlan *plans, int count, int max_ns, int sources, int targets, int most, size_t consts, int instances) {
     conv_opt_in(c);
     auto go = [&](auto *kernel, int cols, int groups, size_t smem) {
         launch(c, kernel, dim3(256 / cols, count, instances), cols * 16 * groups, smem, src, so, dst, dof, plans, c->pc, c->tb.t16);
@@ -416,7 +416,7 @@ void launch_conv(hb_ctx *c, const u64 *src, size_t so, u64 *dst, size_t dof, con
     };
     auto shapes = [&](auto arithmetic) {
         using LONG = decltype(arithmetic);
-        switch (conv_shape(instances * count, max_ns, targets, count, sources, c->tb.t16.pm && max_ns <= 4 && conv_mma_smem(2, most) <= kTwoCtas)) {
+        switch (conv_shape(what, instances * count, max_ns, targets, count, sources, c->tb.t16.pm && max_ns <= 4 && conv_mma_smem(2, most) <= kTwoCtas)) {
         case kMma2: products(conv_mma<2, 2>, 2); break;
         case kMma4: products(conv_mma<4, 1>, 4); break;
         case kStrip8x2: go(conv_cols<8, 2, 2, 4, LONG>, 8, 2, strip_bytes(8, max_ns + 2) + consts); break;
@@ -481,13 +481,13 @@ DigitPlan digit_plan(const hb_ctx *c, const PlanDims &d) {
 }
 size_t key_limbs(hb_ctx *c, int level) { const PlanDims d = plan_dims(c, level); return (size_t)2 * d.nd * d.ne; } // the part of a switching key one key switch reads
 
-// On 2^16 rings: the lifted digits before their forward row pass
-void ks_lift(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch, u64 *dt) {
+// On 2^16 rings: the lifted digits before their forward row pass; once: for ks_rows
+void ks_lift(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch, u64 *dt, bool once) {
     const PlanDims d = plan_dims(c, level);
     const int N = c->N, n = d.n;
     Tmp acoef(c, (size_t)batch * n);
     inv_rows(c, a, a_outer, acoef.p, (size_t)n * N, batch * n, c->qmap(level));
-    launch_conv(c, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), n, d.dt_count / d.nd, digit_targets(*c->h, level), digit_const_bytes(*c->h, level), batch);
+    launch_conv(c, once ? Conversion::kDigitsOnce : Conversion::kDigits, acoef.p, (size_t)n * N, dt, (size_t)d.dt_count * N, get_conv_plans(c, level), d.nd, std::min(n, c->h->alpha), n, d.dt_count / d.nd, digit_targets(*c->h, level), digit_const_bytes(*c->h, level), batch);
 }
 // Whether the digits of `members` polynomials that serve one rotation each go through ks_rows
 bool one_use(const hb_ctx *c, const PlanDims &d, int members) { return c->logn == 16 && c->tb.t16.pm && one_kernel_switch(d.nd, d.ne, members); }
@@ -501,7 +501,7 @@ void ks_decompose(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch,
     const int N = c->N, n = d.n;
     const unsigned gx1 = (unsigned)((N + 255) / 256); // base-conversion kernels keep one coefficient per thread
     if (c->logn == 16) {
-        ks_lift(c, a, a_outer, level, batch, dt);
+        ks_lift(c, a, a_outer, level, batch, dt, false);
         fwd_rows(c, dt, (size_t)d.dt_count * N, batch * d.dt_count, d.dtmap);
         return;
     }
@@ -522,7 +522,7 @@ void moddown(hb_ctx *c, u64 *acc, u64 *tbuf, int level, int total, u64 *out, siz
         const ConvPlan *cv = get_conv_plans(c, level);
         u64 *sp = acc + (size_t)n * N;
         if (!half) inv_rows(c, sp, (size_t)ne * N, sp, (size_t)ne * N, total * 2 * K, pm);
-        launch_conv(c, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, K, n, n, conv_const_bytes(K, n), total * 2);
+        launch_conv(c, Conversion::kModDown, sp, (size_t)ne * N, tbuf, (size_t)n * N, cv + d.nd, 1, K, K, n, n, conv_const_bytes(K, n), total * 2);
         const RowsFin f{acc, (size_t)ne * N, out, out_outer, 2, batch, add_outer};
         LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, tbuf, (size_t)n * N, n, total * 2, f, c->p_inv_scale, sl, c->pc, c->tb.t16));
         CK(cudaGetLastError());
@@ -594,7 +594,8 @@ void keyswitch(hb_ctx *c, const u64 *a, size_t a_outer, int level, int batch, co
     const PlanDims d = plan_dims(c, level);
     Tmp dt(c, (size_t)batch * d.dt_count);
     const bool half = one_use(c, d, batch);
-    (half ? ks_lift : ks_decompose)(c, a, a_outer, level, batch, dt.p);
+    if (half) ks_lift(c, a, a_outer, level, batch, dt.p, true);
+    else ks_decompose(c, a, a_outer, level, batch, dt.p);
     SwitchList sl{};
     sl.count = 1;
     sl.s[0] = SwitchGroup{a, dt.p, key.d, {add0, add1}, g, 0u};
@@ -712,7 +713,7 @@ hb_ct *divide_by_p_ql(hb_ctx *c, u64 *E, int level, int batch, hb_ct *dst = null
         if (c->logn == 16) {
             const ConvPlan *cv = get_conv_plans(c, level);
             inv_rows(c, src, (size_t)ne * N, src, (size_t)ne * N, batch * 2 * ns, sm);
-            launch_conv(c, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, ns, level, level, conv_const_bytes(ns, level), batch * 2);
+            launch_conv(c, Conversion::kDivision, src, (size_t)ne * N, t.p, (size_t)level * N, cv + d.nd + 1, 1, ns, ns, level, level, conv_const_bytes(ns, level), batch * 2);
             const RowsFin f{E, (size_t)ne * N, out, (size_t)2 * level * N, 2, 1, 0};
             LAUNCH(c); CK(launch_fwd_rows_fin16(c->st, t.p, (size_t)level * N, level, batch * 2, f, c->div_scale[level], NoAddends{}, c->pc, c->tb.t16));
             CK(cudaGetLastError());
@@ -1836,7 +1837,9 @@ int hb_rotate_grouped(hb_ctx *c, const hb_ct *x, const int64_t *steps, int group
         if (x->np != 2 || x->batch % groups) fail(HB_E_SHAPE, "rotate: the batch does not split into that many groups");
         const PlanDims d = plan_dims(c, x->level);
         Tmp dt(c, (size_t)x->batch * d.dt_count);
-        (one_use(c, d, x->batch) ? ks_lift : ks_decompose)(c, x->d + (size_t)d.n * c->N, (size_t)2 * d.n * c->N, x->level, x->batch, dt.p);
+        const u64 *a = x->d + (size_t)d.n * c->N;
+        if (one_use(c, d, x->batch)) ks_lift(c, a, (size_t)2 * d.n * c->N, x->level, x->batch, dt.p, true);
+        else ks_decompose(c, a, (size_t)2 * d.n * c->N, x->level, x->batch, dt.p);
         *out = rotate_groups(c, x, dt.p, false, steps, groups);
     });
 }

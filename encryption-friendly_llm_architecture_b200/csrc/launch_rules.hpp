@@ -21,26 +21,29 @@ namespace hb {
 //
 // mma: up to four sources, primes of LongPm, and two CTAs find room with their constants (conv_mma).  Its strips have eight columns, so few units fill the GPU
 // badly: two groups and two CTAs per SM hold nine units at once, four groups and one CTA four and a half; a group without a target waits for the
-// others, and with two sources there is little to multiply.  `plans` conversions of different digits even out, a single one does not: there the number of its
-// targets decides.  Calls, us, the strips / conv_mma with two groups / with four:
-//   3, 4 units       decompositions of level 8, one member 40 / 51 / 37; divisions of level 7 75 / 87 / 73; five targets fill the second round of four
-//                    groups with one (masked sums with their division of level 5 52.0 / 61.1 / 53.0)
+// others, and with two sources there is little to multiply.  Digits of several plans even out, a single conversion does not: there the number of its targets
+// decides; and it matters what runs before and after.  Calls, us, the strips / conv_mma with two groups / with four:
+//   3, 4 units       decompositions of level 8, one member 40 / 51 / 37; divisions of level 7 75 / 87 / 73, of level 5 (five targets fill the second round of
+//                    four groups with one) 52.0 / 61.1 / 53.0
 //   5, 6             decompositions of level 6 53 / 52 / 54, hoisted rotations with their ModDown of level 8 101 / 107 / 107
-//   7 to 9           decompositions of level 12 89 / 83 / 85; divisions of level 1 54 / 49 / 53, of level 12 188 / 193 / 182
-//   12               decompositions of level 12 137 / 124 / 131; divisions of level 4 111 / 108 / 109, of level 12 275 / 288 / 267
+//   7 to 9           decompositions of level 12 89 / 83 / 85; divisions of level 1 54 / 49 / 53, of level 12 188 / 193 / 182; rotations with their ModDown of
+//                    level 8 0.97 / 0.99 of the strips, of level 12 1.02 / 0.99
+//   12               decompositions of level 12 137 / 124 / 131, as part of a rotation (ks_rows follows) 1.00 / 0.98 of the strips; divisions of level 4
+//                    111 / 108 / 109, of level 12 275 / 288 / 267
 //   17, 18           decompositions of level 8 136 / 131 / 144; divisions of level 8 275 / 269 / 260; ModDowns of level 7 208 / 215 / 216
 //   from 24          decompositions of level 12, 48 units 436 / 420 / 451, of level 3 (two sources on average) 148 / 151 / 167; divisions of level 8, 96 units
 //                    1313 / 1288 / 1336, of level 3, 28 units 195 / 201 / 203; ModDowns of level 8, 96 units 1068 / 1059 / 1133, of level 5, 24 units 218 / 222 / 234
 //   two sources      (six or seven digits) decompositions of level 7, 120 units 611 / 636 / 707, 9 units at level 3 45 / 42 / 45
 // Over all levels, 1 to 48 members and contexts of two to four sources no call takes over 1.02 of the time with the strips.
 enum StripShape { kStrip8x1, kStrip8x2, kStrip8x4, kStrip4x4, kStrip4x8, kMma2, kMma4 };
+enum class Conversion { kDigits, kDigitsOnce, kModDown, kDivision }; // kDigitsOnce: of digits that go to ks_rows; kDivision: by P and a prime of Q
 // `plans` conversions of at most max_ns sources, `sources` in all, and `targets` each on average, for units / plans polynomials
-constexpr StripShape conv_shape(int units, int max_ns, int targets, int plans, int sources, bool mma) {
+constexpr StripShape conv_shape(Conversion what, int units, int max_ns, int targets, int plans, int sources, bool mma) {
     if (mma) {
-        const bool one = plans == 1;
-        if ((units == 3 || units == 4) && !(one && targets == 5)) return kMma4;
-        if (units >= 7 && units <= 9) return one && targets >= 7 ? kMma4 : kMma2;
-        if (units == 12) return one && targets >= 5 ? kMma4 : kMma2;
+        const bool one = plans == 1, division = what == Conversion::kDivision, down = what == Conversion::kModDown;
+        if ((units == 3 || units == 4) && !(division && targets == 5)) return kMma4;
+        if (units >= 7 && units <= 9) return (division && targets >= 7) || (down && targets >= (max_ns >= 3 ? 12 : 9)) ? kMma4 : kMma2;
+        if (units == 12) return ((division || down) && targets >= 5) || (what == Conversion::kDigitsOnce && targets >= 6) ? kMma4 : kMma2;
         if (max_ns >= 3 && (units >= 24 || ((units == 17 || units == 18) && !(one && max_ns == 3))) &&
             (one ? targets >= (max_ns == 3 ? 7 : 4) : targets >= 6 || 2 * sources >= 5 * plans))
             return kMma2;

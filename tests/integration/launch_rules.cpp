@@ -16,20 +16,31 @@ static const PartSums part_sums[] = {
     {17, 17, 48, 8062, 8798},
 };
 
-struct Conversion { int units, max_ns, targets, plans, sources; double us[3]; }; // strips, conv_mma with two groups, with four
-static const Conversion conversions[] = {
-    {28, 4, 3, 1, 4, {194.8, 201.2, 203.0}}, {18, 3, 8, 1, 3, {208.4, 214.8, 215.6}}, {18, 3, 7, 1, 3, {178.7, 184.1, 186.2}}, {8, 4, 12, 1, 4, {188.2, 193.1, 181.8}},
-    {8, 4, 11, 1, 4, {178.2, 182.4, 172.0}}, {18, 3, 6, 1, 3, {164.2, 167.9, 172.4}}, {24, 3, 6, 1, 3, {217.5, 222.4, 233.5}}, {12, 4, 9, 3, 10, {113.4, 104.9, 107.6}},
-    {8, 3, 2, 1, 3, {62.9, 56.5, 61.9}}, {30, 4, 10, 3, 11, {257.9, 243.2, 261.3}}, {18, 4, 9, 3, 10, {146.7, 139.0, 152.3}}, {24, 4, 10, 3, 11, {216.0, 202.5, 220.4}},
-    {8, 4, 12, 4, 12, {89.3, 83.2, 84.5}}, {12, 4, 9, 3, 9, {104.2, 97.5, 100.8}}, {3, 4, 9, 3, 9, {40.1, 51.1, 37.4}}, {4, 4, 6, 2, 7, {39.2, 46.9, 35.1}},
-    {18, 3, 7, 1, 3, {263.0, 283.7, 266.3}}, {18, 3, 8, 1, 3, {285.3, 306.2, 286.4}}, {8, 2, 13, 1, 2, {177.4, 189.5, 176.7}}, {18, 2, 6, 1, 2, {160.7, 171.5, 175.1}},
-    {18, 2, 8, 1, 2, {205.8, 218.2, 219.6}}, {8, 3, 12, 1, 3, {216.9, 229.1, 212.3}}, {8, 2, 11, 1, 2, {148.0, 156.3, 146.8}}, {24, 2, 6, 1, 2, {215.3, 227.2, 237.1}},
-    {32, 2, 6, 4, 6, {155.0, 162.6, 173.8}}, {60, 2, 8, 5, 8, {320.2, 333.9, 366.7}}, {120, 2, 8, 5, 8, {610.5, 635.6, 706.8}}, {96, 2, 6, 4, 6, {413.3, 430.2, 482.3}},
-    {240, 2, 8, 5, 8, {1188.5, 1236.3, 1384.3}}, {64, 2, 6, 4, 6, {283.8, 294.9, 329.3}}, {8, 2, 6, 4, 6, {49.9, 47.4, 49.9}}, {8, 3, 2, 1, 3, {58.7, 50.4, 56.7}},
-    {8, 3, 3, 1, 3, {87.0, 81.5, 84.8}}, {12, 2, 3, 2, 3, {53.5, 50.3, 51.9}}, {9, 2, 4, 3, 4, {45.2, 41.8, 44.9}}, {8, 2, 3, 2, 3, {41.3, 38.0, 39.8}},
-    {8, 2, 3, 1, 2, {66.0, 59.6, 64.7}}, {12, 3, 2, 1, 3, {82.5, 77.4, 80.9}}, {32, 4, 3, 1, 4, {224.5, 230.3, 236.7}}, {4, 3, 12, 4, 11, {47.9, 63.0, 45.5}},
-    {8, 3, 12, 4, 11, {91.0, 83.6, 87.9}}, {12, 3, 9, 3, 8, {108.5, 100.3, 104.5}}, {3, 3, 9, 3, 8, {40.8, 51.8, 38.2}}, {9, 3, 9, 3, 8, {80.4, 72.3, 76.1}},
-    {4, 3, 10, 4, 9, {43.3, 56.4, 39.9}}, {8, 3, 6, 2, 4, {56.0, 48.9, 53.5}}, {12, 3, 6, 2, 4, {82.7, 73.5, 79.1}}, {8, 3, 5, 2, 3, {52.8, 46.0, 50.3}},
+struct Call { int units, max_ns, targets, plans, sources; Conversion what; double us[3]; }; // strips, conv_mma with two groups, with four
+constexpr Conversion kDigits = Conversion::kDigits, kDigitsOnce = Conversion::kDigitsOnce, kModDown = Conversion::kModDown, kDivision = Conversion::kDivision;
+static const Call conversions[] = {
+    {18, 3, 7, 1, 3, kDivision, {263.0, 283.7, 266.3}}, {18, 3, 8, 1, 3, kDivision, {285.3, 306.2, 286.4}}, {8, 2, 13, 1, 2, kModDown, {177.4, 189.5, 176.7}},
+    {18, 2, 6, 1, 2, kModDown, {160.7, 171.5, 175.1}}, {18, 2, 8, 1, 2, kModDown, {205.8, 218.2, 219.6}}, {8, 3, 12, 1, 3, kDivision, {216.9, 229.1, 212.3}},
+    {8, 2, 11, 1, 2, kModDown, {148.0, 156.3, 146.8}}, {24, 2, 6, 1, 2, kModDown, {215.3, 227.2, 237.1}}, {32, 2, 6, 4, 6, kDigits, {155.0, 162.6, 173.8}},
+    {60, 2, 8, 5, 8, kDigits, {320.2, 333.9, 366.7}}, {120, 2, 8, 5, 8, kDigits, {610.5, 635.6, 706.8}}, {96, 2, 6, 4, 6, kDigits, {413.3, 430.2, 482.3}},
+    {240, 2, 8, 5, 8, kDigits, {1188.5, 1236.3, 1384.3}}, {64, 2, 6, 4, 6, kDigits, {283.8, 294.9, 329.3}}, {192, 2, 6, 4, 6, kDigits, {795.0, 825.8, 939.8}},
+    {8, 3, 10, 1, 3, kDivision, {182.0, 188.9, 178.7}}, {40, 2, 8, 5, 8, kDigits, {224.6, 232.2, 252.6}}, {28, 4, 3, 1, 4, kDivision, {194.8, 201.2, 203.0}},
+    {240, 2, 9, 5, 9, kDigits, {1302.3, 1343.6, 1502.0}}, {45, 2, 8, 5, 8, kDigits, {247.6, 255.4, 280.5}}, {18, 3, 8, 1, 3, kModDown, {208.4, 214.8, 215.6}},
+    {36, 2, 6, 4, 6, kDigits, {170.2, 175.4, 193.6}}, {18, 3, 7, 1, 3, kModDown, {178.7, 184.1, 186.2}}, {336, 2, 13, 7, 13, kDigits, {2425.6, 2497.0, 2727.4}},
+    {30, 2, 8, 5, 8, kDigits, {177.7, 182.9, 197.8}}, {120, 2, 9, 5, 9, kDigits, {668.7, 688.2, 764.9}}, {80, 2, 8, 5, 8, kDigits, {422.6, 434.9, 482.6}},
+    {60, 2, 9, 5, 9, kDigits, {349.1, 358.9, 394.2}}, {48, 2, 6, 4, 6, kDigits, {223.5, 229.7, 257.5}}, {12, 2, 4, 3, 4, kDigits, {58.4, 56.8, 60.0}},
+    {80, 2, 9, 5, 9, kDigits, {462.8, 475.4, 526.4}}, {84, 2, 13, 7, 13, kDigits, {641.6, 658.9, 716.4}}, {4, 4, 6, 2, 6, kDigits, {37.5, 44.7, 34.2}},
+    {27, 4, 9, 3, 10, kDigits, {212.5, 201.8, 220.8}}, {48, 4, 10, 3, 11, kDigits, {391.4, 369.7, 403.1}}, {3, 4, 9, 3, 10, kDigits, {43.4, 53.8, 38.9}},
+    {96, 4, 12, 4, 13, kDigits, {826.3, 784.0, 851.2}}, {8, 4, 4, 1, 4, kDivision, {81.2, 75.5, 77.9}}, {8, 3, 12, 4, 11, kDigits, {91.0, 83.6, 87.9}},
+    {36, 4, 12, 4, 13, kDigits, {329.7, 313.0, 337.8}}, {4, 3, 12, 4, 11, kDigits, {47.9, 63.0, 45.5}}, {8, 4, 1, 1, 4, kDivision, {54.3, 49.3, 53.2}},
+    {8, 3, 5, 2, 3, kDigits, {52.8, 46.0, 50.3}}, {8, 2, 3, 1, 2, kDigits, {44.5, 38.9, 41.6}}, {8, 4, 12, 4, 13, kDigits, {94.2, 86.0, 88.5}},
+    {72, 4, 10, 3, 11, kDigits, {559.7, 526.6, 581.0}}, {12, 3, 6, 2, 4, kDigits, {82.7, 73.5, 79.1}}, {8, 2, 3, 1, 2, kModDown, {66.0, 59.6, 64.7}},
+    {30, 4, 10, 3, 11, kDigits, {257.9, 243.2, 261.3}}, {3, 3, 9, 3, 8, kDigits, {40.8, 51.8, 38.2}}, {12, 4, 10, 3, 11, kDigitsOnce, {262.4, 258.1, 255.2}},
+    {8, 2, 8, 1, 2, kModDown, {114.7, 115.0, 113.7}}, {8, 3, 9, 1, 3, kModDown, {231.6, 223.9, 229.4}}, {4, 3, 5, 1, 3, kModDown, {58.1, 66.3, 56.9}},
+    {8, 3, 10, 1, 3, kModDown, {134.9, 133.5, 133.2}}, {8, 4, 8, 1, 4, kModDown, {123.7, 121.8, 120.9}}, {8, 3, 7, 1, 3, kModDown, {164.7, 158.2, 161.2}},
+    {12, 4, 6, 2, 6, kDigitsOnce, {207.3, 203.9, 206.1}}, {8, 3, 8, 1, 3, kModDown, {116.0, 114.3, 113.3}}, {12, 4, 8, 3, 8, kDigitsOnce, {213.1, 211.6, 212.5}},
+    {12, 4, 12, 4, 13, kDigitsOnce, {248.9, 249.9, 244.8}}, {8, 3, 10, 1, 3, kModDown, {247.2, 239.3, 244.4}}, {8, 3, 11, 1, 3, kModDown, {142.1, 141.7, 140.1}},
+    {8, 3, 8, 1, 3, kModDown, {215.3, 207.5, 211.7}},
 };
 
 struct Switch { int digits, limbs, members; double us[3]; }; // three kernels, one with a member a CTA, with two
@@ -49,12 +60,12 @@ int main() {
         if (us > c.us[0] * 1.02 || us > 1.05 * std::min({c.us[0], c.us[1], c.us[2]}))
             std::printf("key switch of %d digits, %d limbs, %d members: %.1f us of %.1f / %.1f / %.1f\n", c.digits, c.limbs, c.members, us, c.us[0], c.us[1], c.us[2]), ++bad;
     }
-    for (const Conversion &c : conversions) {
-        const StripShape s = conv_shape(c.units, c.max_ns, c.targets, c.plans, c.sources, true);
+    for (const Call &c : conversions) {
+        const StripShape s = conv_shape(c.what, c.units, c.max_ns, c.targets, c.plans, c.sources, true);
         const double us = c.us[s == kMma2 ? 1 : s == kMma4 ? 2 : 0];
         if (us > c.us[0] * 1.02 || us > 1.06 * std::min({c.us[0], c.us[1], c.us[2]}))
             std::printf("%d units of %d plans, %d sources at most, %d targets: shape %d, %.1f us of %.1f / %.1f / %.1f\n", c.units, c.plans, c.max_ns, c.targets, (int)s, us, c.us[0], c.us[1], c.us[2]), ++bad;
-        if (const StripShape w = conv_shape(c.units, c.max_ns, c.targets, c.plans, c.sources, false); w == kMma2 || w == kMma4) std::printf("conv_mma where it must not be\n"), ++bad;
+        if (const StripShape w = conv_shape(c.what, c.units, c.max_ns, c.targets, c.plans, c.sources, false); w == kMma2 || w == kMma4) std::printf("conv_mma where it must not be\n"), ++bad;
     }
     for (const PartSums &c : part_sums) {
         const bool streamed = c.polys <= streamed_polynomials(c.terms, c.parts);
