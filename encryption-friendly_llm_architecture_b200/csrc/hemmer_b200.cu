@@ -1119,8 +1119,8 @@ void up_open(hb_ctx *c) {
     stage_open(c, c->up, c->went_up, kUpMembers, cudaHostAllocWriteCombined);
 }
 int copy_threads(const hb_ctx *c) { return c->host_threads > 0 ? c->host_threads : kCopyThreads; }
-void host_copy(const hb_ctx *c, double *dst, const double *src, size_t words, int busy = 0) { // busy: threads of the cap that are at work elsewhere
-    in_threads(copy_threads(c) - busy, words, words, [&](size_t a, size_t b) { std::memcpy(dst + a, src + a, (b - a) * sizeof(double)); });
+void host_copy(const hb_ctx *c, double *dst, const double *src, size_t words) {
+    in_threads(copy_threads(c), words, words, [&](size_t a, size_t b) { std::memcpy(dst + a, src + a, (b - a) * sizeof(double)); });
 }
 // coef [count][N] = rounded coefficients at scale sc of the messages re / im [count][n] on the device (im may be null)
 void embed_inverse(hb_ctx *c, i64 *coef, const double *re, const double *im, int n, int count, double sc) {
@@ -1181,11 +1181,16 @@ void decrypt_items(hb_ctx *c, const std::vector<DecItem> &items, bool z, double 
     auto collect = [&](int first, int slot) {
         const int m = std::min(kStageMembers, count - first);
         const size_t words = (size_t)m * slots;
+        while (cudaEventQuery(c->came_down[slot]) == cudaErrorNotReady) {
+            cudaGetLastError(); // which is no error
+            if (!pages.help()) break;
+        }
         CK(cudaEventSynchronize(c->came_down[slot]));
+        pages.stop(); // the copies take all threads of the cap
         const double *h = c->down[slot];
-        if (z) { host_copy(c, re + (size_t)first * N, h, 2 * words, pages.running()); return; }
-        host_copy(c, re + (size_t)first * slots, h, words, pages.running());
-        if (im) host_copy(c, im + (size_t)first * slots, h + words, words, pages.running());
+        if (z) { host_copy(c, re + (size_t)first * N, h, 2 * words); return; }
+        host_copy(c, re + (size_t)first * slots, h, words);
+        if (im) host_copy(c, im + (size_t)first * slots, h + words, words);
     };
     int slot = 0;
     for (int first = 0; first < count; first += kStageMembers, slot ^= 1) {
@@ -1201,10 +1206,11 @@ void decrypt_items(hb_ctx *c, const std::vector<DecItem> &items, bool z, double 
         embed_forward(c, d, z ? d + 1 : d + words, z ? 2 : 1, t.p, it, m);
         CK(cudaMemcpyAsync(c->down[slot], d, words * (z || im ? 2 : 1) * sizeof(double), cudaMemcpyDeviceToHost, c->st));
         CK(cudaEventRecord(c->came_down[slot], c->st));
-        // For two chunks: later ones are copied while these threads would compete with the copies (96 members 6.0 -> 8.1 ms).  Members to pages that are not there
-        // yet, complex values / two arrays, us, without -> with three threads beside the caller: 1 236 / 238 -> 164 / 235, 2 380 / 420 -> 253 / 249, 4 486 / 780 -> 411 / 368,
-        // 8 970 / 860 -> 877 / 644, 13 1314 / 1559 -> 1286 / 1027, 24 2245 / 2407 -> 2159 / 2067, from 48 on within 5 %.  To pages that are there: 2 145 / 138 -> 135 / 139, 13
-        // 436 / 675 -> 370 / 436, 48 1045 / 1085 -> 1041 / 1096 (a thread that has just been at work wakes sooner for the copies).
+        // For two chunks: later ones are copied while these threads would compete with the copies (96 members 6.0 -> 8.1 ms).  Members by the Python call, us, best
+        // of 72, without -> with pages asked for: results kept, so that every page is new, 2 308 -> 188, 4 313 -> 218, 8 577 -> 282, 13 519 -> 382, 24 1046 -> 1207, 48 1205 -> 1076
+        // (medians 451 -> 288, 514 -> 300, 1243 -> 781, 1180 -> 702, 2210 -> 1610, 3479 -> 3230); results dropped, whose pages are there, 2 147 -> 138, 8 472 -> 276, 13 454 -> 368,
+        // 48 1072 -> 1055 (a thread that was at work a moment ago wakes sooner for the copies).  A cap of one, no thread, pages by the caller while it waits: to mapped
+        // memory 1 235 -> 121, 2 407 -> 265, 13 2426 -> 2018, to pages that are there within 3 %.
         if (!first) {
             const size_t early = (size_t)std::min(count, 2 * kStageMembers) * slots;
             pages.ask(re, early * (z ? 2 : 1), z ? nullptr : im);

@@ -1,5 +1,5 @@
-// Pages over a stand-in for the system call: no more threads than the cap, over all calls; each page of one array or of two is asked for once; running() counts
-// the threads at work, so that copies beside them stay within a budget.  Prints what fails; 0 when nothing does.
+// Pages over a stand-in for the system call: no more threads than the cap; each page of one array or of two is asked for once, by threads or by the caller; after
+// stop() no thread is at work, so that copies stay within a budget.  Prints what fails; 0 when nothing does.
 #include "host_threads.hpp"
 
 #include <chrono>
@@ -32,44 +32,49 @@ static int bad = 0;
 #define EXPECT(x) do { if (!(x)) { std::printf("line %d: %s (cap %d, %zu words)\n", __LINE__, #x, cap, words); ++bad; } } while (0)
 
 int main() {
+    const auto self = std::this_thread::get_id();
     for (int cap : {-1, 0, 1, 2, 3, 4, 9})
         for (size_t words : {size_t(512) * 100, size_t(512) * 128 + 511, size_t(512) * 700 + 3, size_t(512) * 5000 + 9})
-            for (int arrays : {1, 2, 3}) { // three: a call for two and a second call
-                double *a = reinterpret_cast<double *>(std::uintptr_t(1) << 40) + 77, *b = a + words + 3000, *c = b + words + 3000;
-                threads.clear(); asked.clear();
-                {
-                    Pages pages(cap);
-                    pages.ask(a, words, arrays > 1 ? b : nullptr);
-                    if (arrays > 2) pages.ask(c, words);
-                    EXPECT(pages.running() >= 0 && pages.running() <= std::max(0, std::min(cap, kCopyThreads)));
-                }
-                EXPECT((int)threads.size() <= std::max(0, std::min(cap, kCopyThreads)));
-                auto whole = [&](const double *x) { return (std::uintptr_t)(x + words) / 4096 - ((std::uintptr_t)x + 4095) / 4096; };
-                const bool first_call = cap > 0 && std::max(whole(a), arrays > 1 ? whole(b) : 0) >= 128, any = first_call || (cap > 0 && arrays > 2 && whole(c) >= 128);
-                EXPECT(threads.empty() == !any);
-                for (const auto &p : asked) EXPECT(p.second == 1);
-                if (first_call)
-                    for (int i = 0; i < std::min(arrays, 2); ++i) {
-                        const std::uintptr_t first = ((std::uintptr_t)(i ? b : a) + 4095) / 4096, last = (std::uintptr_t)((i ? b : a) + words) / 4096;
-                        for (std::uintptr_t p = first; p < last; ++p) EXPECT(asked.count(p));
+            for (int arrays : {1, 2})
+                for (bool helps : {false, true}) {
+                    double *a = reinterpret_cast<double *>(std::uintptr_t(1) << 40) + 77, *b = a + words + 3000;
+                    auto whole = [&](const double *x) { return (std::uintptr_t)(x + words) / 4096 - ((std::uintptr_t)x + 4095) / 4096; };
+                    const int most_threads = std::max(0, std::min(cap, kCopyThreads));
+                    const bool worth = std::max(whole(a), arrays > 1 ? whole(b) : 0) >= 128;
+                    threads.clear(); asked.clear();
+                    {
+                        Pages pages(cap);
+                        EXPECT(!pages.help());
+                        pages.ask(a, words, arrays > 1 ? b : nullptr);
+                        while (helps && pages.help()) {}
                     }
-                size_t inside = 0;
-                for (int i = 0; i < arrays; ++i) inside += whole(i == 0 ? a : i == 1 ? b : c);
-                EXPECT(asked.size() <= inside);
-            }
-    for (int cap : {1, 2, 3, 4, 6}) { // pages and copies together, as a decryption does it
+                    EXPECT((int)threads.size() <= most_threads + helps);
+                    EXPECT(helps || !threads.count(self));
+                    if (!worth) { EXPECT(asked.empty()); continue; }
+                    for (const auto &p : asked) EXPECT(p.second == 1);
+                    if (helps) EXPECT(asked.size() == whole(a) + (arrays > 1 ? whole(b) : 0));
+                    for (const auto &p : asked) EXPECT((p.first * 4096 >= (std::uintptr_t)a && p.first * 4096 + 4096 <= (std::uintptr_t)(a + words)) || (arrays > 1 && p.first * 4096 >= (std::uintptr_t)b && p.first * 4096 + 4096 <= (std::uintptr_t)(b + words)));
+                }
+    for (int cap : {1, 2, 3, 4, 6}) { // pages, then copies, as a decryption does it: twice, with what the first round left
         const size_t words = size_t(512) * 4000;
-        most = 0;
+        most = 0; threads.clear();
         {
             Pages pages(std::min(cap, kCopyThreads) - 1);
-            pages.ask(reinterpret_cast<double *>(std::uintptr_t(1) << 40), words);
-            for (int i = 0; i < 40; ++i) in_threads(cap - pages.running(), 4, words, [](size_t, size_t) { work(50); });
+            for (int i = 0; i < 2; ++i) {
+                pages.ask(reinterpret_cast<double *>(std::uintptr_t(1) << 40), words);
+                for (int k = 0; k < 3; ++k) pages.help();
+                pages.stop();
+                EXPECT(at_work == 0);
+                in_threads(cap, 4, words, [](size_t, size_t) { work(50); });
+                pages.help();
+            }
         }
         EXPECT(most <= cap);
     }
     refuse = true;
-    threads.clear();
+    asked.clear(); threads.clear();
     int cap = 3; size_t words = size_t(512) * 4000;
-    { Pages pages(cap); pages.ask(reinterpret_cast<double *>(std::uintptr_t(1) << 40), words); for (int i = 0; i < 2000 && pages.running(); ++i) std::this_thread::sleep_for(std::chrono::milliseconds(1)); EXPECT(pages.running() == 0); }
+    { Pages pages(cap); pages.ask(reinterpret_cast<double *>(std::uintptr_t(1) << 40), words); while (pages.help()) {} }
+    EXPECT(asked.empty() && threads.size() <= 4);
     return bad != 0;
 }

@@ -149,7 +149,7 @@ def test_errors_on_either_side_of_a_byte(pkg, sigma):
 
 
 def test_a_cap_of_one_thread_starts_no_other(gpu_full):
-    """set_host_threads caps all threads of a call: with one, members go to memory that is new, pages and all, by the caller alone."""
+    """set_host_threads caps all threads of a call: with one, the caller alone asks for pages and copies the values."""
     import os
     import threading
 
