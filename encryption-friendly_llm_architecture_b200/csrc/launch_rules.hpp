@@ -70,20 +70,25 @@ constexpr int switch_members(int batch) { return batch >= 4 && (batch % 2 == 0 |
 
 // Part sums: up to how many polynomials the masks are streamed once per pair of polynomials (k_prod_parts_few); beyond, and never for one or two parts, they
 // are kept (k_prod_parts).  Either kernel works for nothing where its sizes are not filled: the streamed one multiplies 2, 4, 8 or 17 terms, the other has
-// six parts a CTA.  Calls with a mask of its own for every product (the same masks for all parts stay in L2 and make streaming look up to 20 %
-// quicker), level 7, us, streamed / kept, terms x parts:
-//   up to 4 terms   4 x 4, 12 polynomials 382 / 487, 84 2378 / 2368; 4 x 6, 24 0.99 of kept, 48 1.03; 1 x 8, 84 3618 / 3819; 4 x 9, 96 0.95
-//   up to 8         8 x 6, 12 0.93, 16 0.97, 24 1.06; 8 x 12, 12 1116 / 1397, 24 0.98, 48 1.04; 5 x 12, 16 0.96, 24 1.02; 5 x 8, 48 0.95, 84 1.01
-//   more            9 x 6, 12 913 / 796; 9 x 4, 84 4391 / 2964; 16 x 12, 12 1713 / 1884, 16 1.02, 32 4423 / 3791; 9 x 12, 12 1.02; 16 x 8, 16 0.93, 32 1.06;
-//                   9 x 8, 12 0.91, 16 1.02; up to ten polynomials 0.9 to 1.07 in one group of parts
-// No call of 12 to 192 polynomials that it streams takes over 1.02 of the time with kept masks; levels 3 and 12 lie within 0.05 of these ratios.
+// six parts a CTA; from nine terms on the line goes by the products of either.  Calls with a mask of its own for every product (the same masks for all parts
+// stay in L2 and make streaming look up to 20 % quicker; absent masks change nothing), streamed / kept at level 7, us or ratio, terms x parts:
+//   up to 4 terms   4 x 4, 12 polynomials 382 / 487, 84 2378 / 2368; 4 x 6, 24 0.99, 48 1.03; 1 x 8, 84 3618 / 3819; 4 x 9, 96 0.95
+//   up to 8         8 x 6, 12 0.93, 16 0.97, 24 1.06; 5 x 4, 16 1.01; 8 x 12, 12 1116 / 1397, 24 0.98, 48 1.04; 5 x 12, 24 1.02; 5 x 8, 48 1.00, 84 1.01;
+//                   8 x 13, 84 0.94; 8 x 7, 96 0.91; 5 x 9, 48 1.04
+//   more            9 x 6, 12 913 / 796; 9 x 4, 84 4391 / 2964; 9 x 8, 12 0.91, 16 1.02; 12 x 12, 12 0.98, 14 1.04; 16 x 8, 16 0.93, 24 1.01; 16 x 12, 12 1713 / 1884,
+//                   16 1.02, 32 4423 / 3791; 13 x 13, 22 0.97, 28 1.00; 16 x 16, 22 1.01, 24 1.02; 17 x 17, 16 0.90, 24 0.99, 36 1.06, 48 1.10; up to ten
+//                   polynomials 0.9 to 1.07 in one group of parts
+// Over 2200 calls at levels 3 to 12, 12 to 192 polynomials, none that it streams takes over 1.025 of the time with kept masks; all together take 1.002 of what the
+// quicker kernel of each call would.
 constexpr int streamed_polynomials(int terms, int parts) {
-    const int groups = (parts + 5) / 6;
-    const bool room = 2 * parts <= 9 * groups; // a quarter or more of the kept kernel's places for parts are empty
-    if (terms <= 4) return room ? 96 : 24;
-    if (terms <= 8) return groups == 1 ? 12 : room ? 48 : 16;
-    if (groups == 1) return 10;
-    return terms >= 12 ? (room ? 16 : 12) : room ? 12 : 10;
+    const int groups = (parts + 5) / 6, empty = 6 * groups - parts; // empty: places for parts that the kept kernel has and does not need
+    if (terms <= 4) return 2 * empty >= 3 * groups ? 96 : 24;
+    if (terms <= 8) {
+        if (groups == 1) return parts <= 4 ? 16 : 12;
+        return 2 * empty >= 5 * groups ? 96 : 3 * empty >= 5 * groups ? 12 * terms : 2 * empty >= 3 * groups ? 48 : 24;
+    }
+    const int line = groups == 1 ? 10 : (groups == 2 ? 16 : 22) * 6 * groups * terms / (17 * parts);
+    return line > 10 ? line : 10;
 }
 
 } // namespace hb

@@ -54,7 +54,9 @@ def test_part_sums_on_either_side_of_the_line_between_the_kernels(pkg, g, terms,
 
 
 @pytest.mark.parametrize("terms,parts,polys,batch", [(4, 4, 2, 48), (4, 4, 1, 97), (3, 6, 2, 12), (3, 6, 1, 25), (8, 6, 3, 4), (8, 6, 1, 13), (5, 7, 2, 24), (5, 7, 1, 49), (8, 12, 2, 8), (8, 12, 1, 17), (9, 4, 1, 10),
-                                                     (9, 4, 1, 11), (17, 13, 2, 8), (17, 13, 1, 17), (16, 12, 2, 6), (16, 12, 1, 13), (9, 8, 1, 12), (9, 8, 1, 13), (11, 17, 1, 10), (11, 17, 1, 11)])
+                                                     (9, 4, 1, 11), (17, 13, 2, 8), (17, 13, 1, 17), (16, 12, 2, 6), (16, 12, 1, 13), (9, 8, 1, 12), (9, 8, 1, 13), (11, 17, 1, 10), (11, 17, 1, 11),
+                                                     (5, 4, 2, 8), (5, 4, 1, 17), (8, 8, 2, 48), (8, 8, 1, 97), (6, 9, 1, 48), (6, 9, 1, 49), (8, 12, 2, 12), (8, 12, 1, 25), (17, 17, 1, 23), (17, 17, 2, 12), (16, 16, 1, 23),
+                                                     (16, 16, 2, 12), (13, 13, 1, 23), (13, 13, 2, 12), (11, 17, 1, 15), (11, 17, 2, 8)])
 def test_part_sums_on_either_side_of_every_line_of_the_rule(pkg, g, terms, parts, polys, batch):
     _compare_part_sums(pkg, g, terms, parts, polys, batch, True)
 
