@@ -15,7 +15,8 @@
 // Bound by latency (16 CTAs of 128 threads a member): for eight members 7 and 14 us to encode, 40 and 35 us to decode, where the
 // host cores took 2.0 and 1.8 ms a member for the same transforms and 2.8 and 1.4 ms for sampling and CRT lift.  Thirteen messages
 // of two tiles from host memory to ciphertexts 7.3 -> 0.82 -> 0.66 ms (0.82 before uniform parts and errors were drawn ahead of the messages), thirteen
-// ciphertexts to host memory 5.5 -> 0.80 ms, each pass through the Python call on other buffers.  The copies are most of all of these.
+// ciphertexts to host memory 5.5 -> 0.80 -> 0.65 ms (0.80 before their pages were asked for meanwhile), each pass through the Python call on other buffers; the library
+// call on the same buffers again 0.53 and 0.35 ms.  The copies are most of all of these.
 #pragma once
 #include "modarith.cuh"
 #include "kernels.cuh"

@@ -1252,7 +1252,8 @@ __global__ void __launch_bounds__(256, 2) k_ks_inner_mk(u64 *E, const u64 *c0, c
 // staging both in shared memory by bulk copies for three members at a time took 1.6 times as long (they crossed L2 for every
 // third member, and a CTA's copies, sums and stores did not overlap).  Two coefficients per thread and two CTAs per SM: 869 us a launch
 // for 168 outputs at level 6; one coefficient and three CTAs 837 us, four CTAs 776 us (64 registers), 712 with the
-// products and additions of the 60-bit limbs apart: their integer chains want warps more than they want independent work in a thread.  With joined products
+// products and additions of the 60-bit limbs apart: their integer chains want warps more than they want independent work in a thread (each of these with the program
+// of its day; now, with two rotations an output, 824, with one 703).  With joined products
 // 65 % of the issue slots and 52 % of the wide multiply-adds for 64 outputs (367 us), DRAM 3.1 TB/s; in a third of the cycles it waits for loads.
 // grid = (N/256, groups * ceil(batch/per), ne)
 template <int ND, int CNT>

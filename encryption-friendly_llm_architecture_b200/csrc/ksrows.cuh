@@ -8,8 +8,8 @@
 // memory; then all threads form the sums of their coefficients, gathering the digits' words from there.  The lifted limbs are read
 // once and never written back, the special limbs of the result leave half transformed.
 //
-// Bound by instruction issue (48 members at level 8: 631 us, 56 % of the slots, DRAM 2.3 TB/s; the three kernels it replaces 310 + 286 + 86 at 3.5 to 5.3
-// TB/s).  Blocks of few warps, because their loads, transforms and sums alternate behind barriers: eight rows a CTA 4 to 7 % of a whole rotation
+// Bound by instruction issue (48 members at level 8: 640 us, 56 % of the slots, DRAM 2.3 TB/s; the three kernels it replaces 310 + 286 + 86 at 3.5 to 5.3
+// TB/s).  At 64 registers a thread spills 4 to 12 bytes.  Blocks of few warps, because their loads, transforms and sums alternate behind barriers: eight rows a CTA 4 to 7 % of a whole rotation
 // slower, four 1 to 2 %.  Two members a CTA share the key words that each coefficient meets: 64 members at level 8 2671 -> 2603 us.  Limbs in the inner order,
 // so that integer and FP64 work meet on an SM: 2729 us, twiddles and keys then come from L2 every time.
 // Rotations with three kernels and with this one stand at the rule that chooses (one_kernel_switch).  256 products at level 8 14.2 / 13.9 ms.
